@@ -226,17 +226,7 @@ cudaError_t launch_vgemm_mt(const VGemmParams& p, int mt, int k, int hd, int sms
   }
   return cudaErrorInvalidValue;
 }
-constexpr int kTcMaxItems = 256;      // split-K work items whose partial sums the context can hold
-
-// K splits of one verify GEMM: enough (row block, split) items to occupy the GPU, whole groups per split, at most 4
-// partials to add, at most kTcMaxGroups groups per item
-int tc_splits(int rows, int k, int sms) {
-  const int rb = (rows + kTcRowBlock - 1) / kTcRowBlock, G = k / 128;
-  int ns = 1;
-  while (ns < 4 && rb * ns < sms * 3 / 4 && G / (ns * 2) >= 2 && rb * ns * 2 <= kTcMaxItems) ns *= 2;
-  while ((G + ns - 1) / ns > kTcMaxGroups && ns < 64) ns *= 2;
-  return ns;
-}
+constexpr size_t kVsplitFloats = (size_t)256 * 64 * 128;      // K-split partial sums of v_gemm_sub that the context can hold
 
 template <int NT, int EPI>
 cudaError_t launch_vsub_nt(const VsubParams& p, int sms, cudaStream_t st) {
@@ -261,74 +251,55 @@ cudaError_t launch_vsub(const VsubParams& p, int sms, cudaStream_t st) {
   return cudaErrorInvalidValue;
 }
 
-template <int MT, int EPI, bool HZ>
+// K splits (CTAs of a cluster) of one tcgen05 GEMM: matrices with few row blocks are cut in 2 or 4 while every CTA still finds
+// an SM of its own and two groups to multiply
+int tc_splits(int items, int k, int sms) {
+  const int G = k / 128;
+  int ns = 1;
+  while (ns < 4 && items * ns * 2 <= sms && G / (ns * 2) >= 2) ns *= 2;
+  return ns;
+}
+template <int NT, int EPI, bool HZ>
 cudaError_t launch_vtc_hz(VtcParams& p, int sms, cudaStream_t st) {
   static bool configured[64] = {};
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
   if (!configured[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(v_gemm_tc<MT, EPI, HZ>, cudaFuncAttributeMaxDynamicSharedMemorySize, VtcSmem<MT, HZ>::TOTAL);
+    cudaError_t e = cudaFuncSetAttribute(v_gemm_tc<NT, EPI, HZ>, cudaFuncAttributeMaxDynamicSharedMemorySize, VtcSmem<NT, HZ>::TOTAL);
     if (e != cudaSuccess) return e;
     configured[dev] = true;
   }
-  p.nsplit = tc_splits(p.rows, p.K, sms);
-  const int items = ((p.rows + kTcRowBlock - 1) / kTcRowBlock) * p.nsplit;
-  if (p.K % 128 || (p.K / 128 + p.nsplit - 1) / p.nsplit > kTcMaxGroups || (p.nsplit > 1 && items > kTcMaxItems))
-    return cudaErrorInvalidValue;
-  return launch_pdl(v_gemm_tc<MT, EPI, HZ>, dim3(items < sms ? items : sms), dim3(kTcThreads), (size_t)VtcSmem<MT, HZ>::TOTAL, st, p);
+  if (p.K % 128 || p.ntok % 16 || p.ntok > NT || (size_t)p.ntok * p.ntile < (size_t)p.M) return cudaErrorInvalidValue;
+  const int items = ((p.rows + kTcRowBlock - 1) / kTcRowBlock) * p.ntile;
+  p.nsplit = p.ntile == 1 ? tc_splits(items, p.K, sms) : 1;
+  const int grid = p.nsplit > 1 ? items * p.nsplit : (items < sms ? items : sms);
+  return launch_pdl_cluster(v_gemm_tc<NT, EPI, HZ>, dim3(grid), dim3(kTcThreads), (size_t)VtcSmem<NT, HZ>::TOTAL, st,
+                            (unsigned)p.nsplit, p);
 }
-template <int MT, int EPI>
-cudaError_t launch_vtc_mt(VtcParams& p, int sms, cudaStream_t st) {
-  return p.has_zeros ? launch_vtc_hz<MT, EPI, true>(p, sms, st) : launch_vtc_hz<MT, EPI, false>(p, sms, st);
+template <int NT, int EPI>
+cudaError_t launch_vtc_nt(VtcParams& p, int sms, cudaStream_t st, bool hz) {
+  return hz ? launch_vtc_hz<NT, EPI, true>(p, sms, st) : launch_vtc_hz<NT, EPI, false>(p, sms, st);
 }
+// `maps`: the activation buffer as a tensor, one map per token tile height (16, 32, 64, 128)
 template <int EPI>
-cudaError_t launch_vtc(VtcParams& p, int mt, int sms, cudaStream_t st) {
-  switch (mt) {
-    case 16: return launch_vtc_mt<16, EPI>(p, sms, st);
-    case 32: return launch_vtc_mt<32, EPI>(p, sms, st);
-    case 64: return launch_vtc_mt<64, EPI>(p, sms, st);
+cudaError_t launch_vtc(VtcParams& p, const CUtensorMap* maps, int nt, bool hz, int sms, cudaStream_t st) {
+  p.xmap = maps[nt == 16 ? 0 : (nt == 32 ? 1 : (nt == 64 ? 2 : 3))];
+  switch (nt) {
+    case 16: return launch_vtc_nt<16, EPI>(p, sms, st, hz);
+    case 32: return launch_vtc_nt<32, EPI>(p, sms, st, hz);
+    case 64: return launch_vtc_nt<64, EPI>(p, sms, st, hz);
+    case 128: return launch_vtc_hz<128, EPI, false>(p, sms, st);
   }
   return cudaErrorInvalidValue;
 }
 
-template <int MT, bool HZ>
-cudaError_t launch_vchain_hz(VchainParams& p, int sms, cudaStream_t st) {
-  static bool configured[64] = {};
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
-  if (!configured[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(v_chain_tc<MT, HZ>, cudaFuncAttributeMaxDynamicSharedMemorySize, VtcSmem<MT, HZ>::TOTAL);
-    if (e != cudaSuccess) return e;
-    configured[dev] = true;
-  }
-  for (int i = 0; i < p.nph; i++) {
-    VtcPhase& f = p.ph[i];
-    f.nsplit = tc_splits(f.rows, f.K, sms);
-    const int items = ((f.rows + kTcRowBlock - 1) / kTcRowBlock) * f.nsplit;
-    if (f.K % 128 || (f.K / 128 + f.nsplit - 1) / f.nsplit > kTcMaxGroups || (f.nsplit > 1 && items > kTcMaxItems) ||
-        (f.rows + kTcRowBlock - 1) / kTcRowBlock * 4 > 4096)
-      return cudaErrorInvalidValue;
-  }
-  void* args[] = {&p};
-  // every CTA must be resident: the loaders of a phase wait for the epilogue warps of the whole grid
-  return cudaLaunchCooperativeKernel((const void*)v_chain_tc<MT, HZ>, dim3(sms), dim3(kTcThreads), args,
-                                     (size_t)VtcSmem<MT, HZ>::TOTAL, st);
-}
-cudaError_t launch_vchain(VchainParams& p, int mt, bool hz, int sms, cudaStream_t st) {
-  switch (mt) {
-    case 16: return hz ? launch_vchain_hz<16, true>(p, sms, st) : launch_vchain_hz<16, false>(p, sms, st);
-    case 32: return hz ? launch_vchain_hz<32, true>(p, sms, st) : launch_vchain_hz<32, false>(p, sms, st);
-    case 64: return hz ? launch_vchain_hz<64, true>(p, sms, st) : launch_vchain_hz<64, false>(p, sms, st);
-  }
-  return cudaErrorInvalidValue;
-}
-
-cudaError_t launch_vnorm(const uint16_t* h, const uint16_t* w, uint16_t* xn_t, uint16_t* xn_nat, int D, int M, float eps,
-                         cudaStream_t st) {
+cudaError_t launch_vnorm(const uint16_t* h, const uint16_t* w, uint16_t* xn_t, uint16_t* xn_nat, uint16_t* feat, int D, int M,
+                         float eps, cudaStream_t st) {
   if (D % 16 || D > 8 * 256 * 2) return cudaErrorInvalidValue;
-  if (D <= 8 * 256) return launch_pdl(v_rmsnorm<1>, dim3(M), dim3(256), 0, st, h, w, xn_t, xn_nat, D, eps);
-  return launch_pdl(v_rmsnorm<2>, dim3(M), dim3(256), 0, st, h, w, xn_t, xn_nat, D, eps);
+  if (D <= 8 * 256) return launch_pdl(v_rmsnorm<1>, dim3(M), dim3(256), 0, st, h, w, xn_t, xn_nat, feat, D, eps);
+  return launch_pdl(v_rmsnorm<2>, dim3(M), dim3(256), 0, st, h, w, xn_t, xn_nat, feat, D, eps);
 }
+constexpr int kPromptRows = 1024;  // token rows of the activation buffers: a prompt goes through the layers in chunks of at most this
 constexpr int kVSpans = 32;       // most spans of positions a kv head's attention is cut into
 
 cudaError_t launch_vattn(const fb_ctx* c, const uint16_t* q, const uint16_t* kc, const uint16_t* vc, const uint8_t* amask,
@@ -340,21 +311,127 @@ cudaError_t launch_vattn(const fb_ctx* c, const uint16_t* q, const uint16_t* kc,
   int smax = (2 * c->sm_count) / (d.n_kv_head * mgroups);
   if (smax < 1) smax = 1;
   if (smax > kVSpans) smax = kVSpans;
+  if (smax > kVSpans * 64 / M) smax = kVSpans * 64 / M > 0 ? kVSpans * 64 / M : 1;     // the partials' buffer
   int S = (T + 63) / 64;
   if (S > smax) S = smax;
   const int span = ((T + S - 1) / S + 63) / 64 * 64;
   S = (T + span - 1) / span;
+  uint16_t* direct = S == 1 && natural ? ao : nullptr;
 #define FB_VATTN(HD_, R_)                                                                                               \
   if (d.head_dim == HD_ && c->rgqa == R_) {                                                                             \
     cudaError_t e = launch_pdl(v_attn_mma<HD_, R_>, dim3(d.n_kv_head, S, mgroups), dim3(128), 0, st, q, kc, vc, amask, c->vpart,  \
-                               d.n_head, d.n_kv_head, pos, M, d.attn_scale, span);                                      \
-    if (e != cudaSuccess) return e;                                                                                     \
+                               direct, d.n_head, d.n_kv_head, pos, M, d.attn_scale, span);                                      \
+    if (e != cudaSuccess || direct) return e;                                                                           \
     return launch_pdl(v_attn_merge<HD_, R_>, dim3(M, d.n_kv_head), dim3(256), 0, st, (const float*)c->vpart, ao, d.n_head, \
                       d.n_kv_head, M, S, natural);                                                                      \
   }
   FB_VATTN(64, 4) FB_VATTN(80, 4) FB_VATTN(64, 5) FB_VATTN(128, 4)
 #undef FB_VATTN
   return cudaErrorInvalidValue;
+}
+
+typedef CUresult (*EncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
+                             const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
+                             CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+EncodeFn tensor_map_encoder() {
+  void* fn = nullptr;
+  cudaDriverEntryPointQueryResult qres;
+  if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &qres) != cudaSuccess ||
+      qres != cudaDriverEntryPointSuccess)
+    return nullptr;
+  return (EncodeFn)fn;
+}
+
+// The activation buffers of the verify GEMMs as 2-D tensors [rows][K], box 64 columns x a token tile, in the swizzle the MMA reads
+bool make_act_maps(fb_ctx* c) {
+  EncodeFn enc = tensor_map_encoder();
+  if (!enc) return false;
+  const fb_model_desc& d = c->d;
+  void* bases[3] = {c->vxn, c->vao, c->vact};
+  const cuuint64_t widths[3] = {(cuuint64_t)d.dim, (cuuint64_t)d.n_head * d.head_dim, (cuuint64_t)d.ffn};
+  CUtensorMap* maps[3] = {c->m_xn, c->m_ao, c->m_act};
+  for (int i = 0; i < 3; i++)
+    for (int j = 0; j < 4; j++) {
+      const cuuint64_t dims[2] = {widths[i], (cuuint64_t)kPromptRows}, strides[1] = {widths[i] * 2};
+      const cuuint32_t box[2] = {64u, 16u << j}, estr[2] = {1u, 1u};
+      if (enc(&maps[i][j], CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, bases[i], dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+              CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+        return false;
+    }
+  return true;
+}
+
+// The caches as 3-D tensors for the long-cache decode variant: [n_layer * max_seq rows][n_kv heads][HD], box = HD x 1 head x
+// one stage of positions. Returns false where the driver entry point is missing or refuses the shape: the plain variant runs.
+bool make_kv_maps(fb_ctx* c) {
+  EncodeFn fn = tensor_map_encoder();
+  if (!fn) return false;
+  const fb_model_desc& d = c->d;
+  const int HD = d.head_dim, R = d.n_head / d.n_kv_head;
+  int nps = 0;
+  if (HD == 64 && R == 4) nps = AttnCfg<64, 4>::NPS;
+  else if (HD == 80 && R == 4) nps = AttnCfg<80, 4>::NPS;
+  else if (HD == 128 && R == 4) nps = AttnCfg<128, 4>::NPS;
+  else return false;
+  const cuuint64_t dims[3] = {(cuuint64_t)HD, (cuuint64_t)d.n_kv_head, (cuuint64_t)d.n_layer * (cuuint64_t)c->max_seq};
+  const cuuint64_t strides[2] = {(cuuint64_t)HD * 2, (cuuint64_t)d.n_kv_head * HD * 2};
+  const cuuint32_t box[3] = {(cuuint32_t)HD, 1u, (cuuint32_t)nps};
+  const cuuint32_t estr[3] = {1u, 1u, 1u};
+  void* bases[2] = {c->kc, c->vc};
+  CUtensorMap* maps[2] = {&c->kmap, &c->vmap};
+  for (int i = 0; i < 2; i++) {
+    const CUresult r = fn(maps[i], CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, bases[i], dims, strides, box, estr,
+                                      CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                                      CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) return false;
+  }
+  return true;
+}
+
+// One pass of M tokens (1 .. kPromptRows) through the model on the tcgen05 GEMMs: natural-order activations, the matrices in the
+// TC layout. depth / amask NULL: a causal chain (a chunk of a prompt).
+int run_tc_pass(fb_ctx* c, const int32_t* d_tokens, const void* d_h, const int32_t* d_depth, const uint8_t* d_amask, int M,
+                int pos, float* d_logits, void* d_feat, cudaStream_t st) {
+  const fb_model_desc& d = c->d;
+  const int D = d.dim, FF = d.ffn, HD = d.head_dim, QD = d.n_head * HD, QKV = (d.n_head + 2 * d.n_kv_head) * HD, sms = c->sm_count;
+  const bool hz = d.has_zeros != 0;
+  // token tile: the smallest that holds the tokens; more than 64 go in tiles of up to 128 (64 with zero points: their
+  // accumulator takes the tensor memory of the wider tile), cut evenly
+  const int cap = hz ? 64 : 128, nt = M <= 16 ? 16 : (M <= 32 ? 32 : (M <= 64 ? 64 : cap));
+  const size_t tQ = tc_matrix_bytes(QKV, D, hz), tO = tc_matrix_bytes(D, QD, hz), tG = tc_matrix_bytes(2 * FF, D, hz),
+               tF = tc_matrix_bytes(D, FF, hz);
+  FB_CUDA(c, launch_pdl(v_embed, dim3(M), dim3(256), 0, st, d_tokens, (const uint16_t*)c->embed, (const uint16_t*)d_h, c->vh,
+                        D, d.vocab, d.emb_mult, &c->status->code));
+  FB_CUDA(c, launch_pdl(v_rope_table, dim3(M), dim3(64), 0, st, d_depth, (const float*)c->invf, pos, HD / 2, (float2*)c->vrope));
+  VtcParams t;
+  memset(&t, 0, sizeof(t));
+  t.M = M; t.status = c->status; t.spin_limit = c->spin_limit;
+  t.ntile = (M + nt - 1) / nt; t.ntok = ((M + t.ntile - 1) / t.ntile + 15) / 16 * 16;
+  t.rope = (const float2*)c->vrope; t.n_head = d.n_head; t.nkv = d.n_kv_head; t.pos = pos; t.head_dim = HD;
+  t.resid = d.resid_mult; t.logits_scaling = d.logits_scaling; t.h = c->vh; t.q = c->vq; t.act = c->vact; t.logits = d_logits;
+  for (int l = 0; l < d.n_layer; l++) {
+    uint16_t* kcl = (uint16_t*)c->kc + (size_t)l * c->max_seq * d.n_kv_head * HD;
+    uint16_t* vcl = (uint16_t*)c->vc + (size_t)l * c->max_seq * d.n_kv_head * HD;
+    FB_CUDA(c, launch_vnorm(c->vh, (const uint16_t*)c->n1 + (size_t)l * D, nullptr, c->vxn, nullptr, D, M, d.rms_eps, st));
+    t.w = c->t_qkv + l * tQ; t.rows = QKV; t.K = D; t.kc = kcl; t.vc = vcl;
+    FB_CUDA(c, launch_vtc<EPI_QKV>(t, c->m_xn, nt, hz, sms, st));
+    FB_CUDA(c, launch_vattn(c, c->vq, kcl, vcl, d_amask, c->vao, pos, M, 1, st));
+    t.w = c->t_o + l * tO; t.rows = D; t.K = QD; t.out_ld = D;
+    FB_CUDA(c, launch_vtc<EPI_RESID>(t, c->m_ao, nt, hz, sms, st));
+    FB_CUDA(c, launch_vnorm(c->vh, (const uint16_t*)c->n2 + (size_t)l * D, nullptr, c->vxn, nullptr, D, M, d.rms_eps, st));
+    t.w = c->t_gu + l * tG; t.rows = 2 * FF; t.K = D; t.out_ld = FF;
+    FB_CUDA(c, launch_vtc<EPI_SWIGLU>(t, c->m_xn, nt, hz, sms, st));
+    t.w = c->t_d + l * tF; t.rows = D; t.K = FF; t.out_ld = D;
+    FB_CUDA(c, launch_vtc<EPI_RESID>(t, c->m_act, nt, hz, sms, st));
+  }
+  // the feature goes to the caller; the LM head reads the same rows from the context's buffer
+  FB_CUDA(c, launch_vnorm(c->vh, (const uint16_t*)c->nf, nullptr, c->vxn, (uint16_t*)d_feat, D, M, d.rms_eps, st));
+  if (d_logits) {
+    t.w = c->t_lm; t.rows = d.vocab; t.K = D; t.out_ld = d.vocab;
+    FB_CUDA(c, launch_vtc<EPI_LOGITS>(t, c->m_xn, nt, hz, sms, st));
+  }
+  FB_CUDA(c, cudaGetLastError());
+  return FB_OK;
 }
 
 }  // namespace
@@ -451,17 +528,15 @@ int fb_ctx_create_tp(const fb_model_desc* desc, int device, int32_t tp_rank, int
     const size_t rowsz[5] = {(size_t)d.dim, (size_t)d.dim, (size_t)QD, (size_t)QD, (size_t)d.ffn};
     uint16_t** vp[5] = {&c->vh, &c->vxn, &c->vq, &c->vao, &c->vact};
     for (int i = 0; i < 5; i++) {
-      A(dmalloc(vp[i], 64 * rowsz[i] * 2));
-      if (e == cudaSuccess) A(cudaMemset(*vp[i], 0, 64 * rowsz[i] * 2));
+      A(dmalloc(vp[i], kPromptRows * rowsz[i] * 2));
+      if (e == cudaSuccess) A(cudaMemset(*vp[i], 0, kPromptRows * rowsz[i] * 2));
     }
   }
   A(dmalloc(&c->vpart, (size_t)d.n_kv_head * 32 * 64 * c->rgqa * (d.head_dim + 2) * 4));
-  A(dmalloc(&c->vsplit, (size_t)kTcMaxItems * 64 * 128 * 4));
+  A(dmalloc(&c->vsplit, kVsplitFloats * 4));
   A(dmalloc(&c->vcount, kVsCounters * 4));
   if (e == cudaSuccess) A(cudaMemset(c->vcount, 0, kVsCounters * 4));
-  A(cudaMalloc(&c->vrope, (size_t)64 * (d.head_dim / 2) * 8));
-  A(dmalloc(&c->vssq, (size_t)2 * 256 * 64 * 4));
-  A(dmalloc(&c->vgbar, (size_t)(d.n_layer + 2) * 4 * 4));
+  A(cudaMalloc(&c->vrope, (size_t)kPromptRows * (d.head_dim / 2) * 8));
   A(dmalloc(&c->flags, 3 * 256 * 4));
   if (e == cudaSuccess) A(cudaMemset(c->flags, 0, 3 * 256 * 4));
   if (c->sm_count > 256) e = cudaErrorInvalidValue;
@@ -479,6 +554,7 @@ int fb_ctx_create_tp(const fb_model_desc* desc, int device, int32_t tp_rank, int
     if (kDecodeKernels[kid].fn_long)
       A(cudaFuncSetAttribute(kDecodeKernels[kid].fn_long, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes));
   }
+  if (e == cudaSuccess && tp_size == 1 && !make_act_maps(c)) e = cudaErrorInvalidValue;
   if (e != cudaSuccess) {
     fb_ctx_destroy(c);
     return FB_ERR_CUDA;
@@ -495,7 +571,7 @@ int fb_ctx_destroy(fb_ctx* c) {
   void* ptrs[] = {c->w_qkv, c->w_o, c->w_gu, c->w_d, c->w_lm, c->invf,
                   c->status, c->h_ll, c->q_ll, c->k_ll, c->v_ll, c->ao_ll, c->act_ll, c->cand_ll, c->flags,
                   c->part_ll, c->vh, c->vxn, c->vq, c->vao, c->vact, c->vpart, c->inbox,
-                  c->t_qkv, c->t_o, c->t_gu, c->t_d, c->t_lm, c->s_qkv, c->s_o, c->s_gu, c->s_d, c->s_lm, c->vsplit, c->vcount, c->vrope, c->vssq, c->vgbar};
+                  c->t_qkv, c->t_o, c->t_gu, c->t_d, c->t_lm, c->s_qkv, c->s_o, c->s_gu, c->s_d, c->s_lm, c->vsplit, c->vcount, c->vrope};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   delete c;
@@ -664,7 +740,7 @@ int fb_bind_weights(fb_ctx* c, const fb_weight_ptrs* w, void* stream) {
     const int tiles32 = (m.rows + 31) / 32;
     const VsPlan vp = vs_plan(m.k, 1, tiles32);
     if (c->tp_size == 1 && !hz && vp.ok &&
-        (size_t)tiles32 * vp.nkc * 8 * 512 <= (size_t)kTcMaxItems * 64 * 128 * 4) {   // K-split partials fit the shared buffer
+        (size_t)tiles32 * vp.nkc * 8 * 512 <= kVsplitFloats * 4) {   // K-split partials fit the shared buffer
       // the small-tree verify GEMM's copy (symmetric layout only; other shapes keep the bf16 warp-level kernel)
       FB_CUDA(c, dmalloc(m.sdst, (size_t)m.layers * vs_matrix_bytes(m.rows, m.k) + 16));
       vs_repack<<<dim3(tiles32, m.layers), 256, 0, st>>>((const uint32_t*)m.q, (const uint16_t*)m.s, m.rows, m.k, vp.ug, m.order,
@@ -675,39 +751,6 @@ int fb_bind_weights(fb_ctx* c, const fb_weight_ptrs* w, void* stream) {
   c->n1 = w->n1; c->n2 = w->n2; c->nf = w->nf; c->embed = w->embed;
   c->weights_bound = true;
   return FB_OK;
-}
-
-// The caches as 3-D tensors for the long-cache decode variant: [n_layer * max_seq rows][n_kv heads][HD], box = HD x 1 head x
-// one stage of positions. Returns false where the driver entry point is missing or refuses the shape: the plain variant runs.
-static bool make_kv_maps(fb_ctx* c) {
-  typedef CUresult (*EncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
-                               const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
-                               CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-  void* fn = nullptr;
-  cudaDriverEntryPointQueryResult qres;
-  if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &qres) != cudaSuccess || !fn ||
-      qres != cudaDriverEntryPointSuccess)
-    return false;
-  const fb_model_desc& d = c->d;
-  const int HD = d.head_dim, R = d.n_head / d.n_kv_head;
-  int nps = 0;
-  if (HD == 64 && R == 4) nps = AttnCfg<64, 4>::NPS;
-  else if (HD == 80 && R == 4) nps = AttnCfg<80, 4>::NPS;
-  else if (HD == 128 && R == 4) nps = AttnCfg<128, 4>::NPS;
-  else return false;
-  const cuuint64_t dims[3] = {(cuuint64_t)HD, (cuuint64_t)d.n_kv_head, (cuuint64_t)d.n_layer * (cuuint64_t)c->max_seq};
-  const cuuint64_t strides[2] = {(cuuint64_t)HD * 2, (cuuint64_t)d.n_kv_head * HD * 2};
-  const cuuint32_t box[3] = {(cuuint32_t)HD, 1u, (cuuint32_t)nps};
-  const cuuint32_t estr[3] = {1u, 1u, 1u};
-  void* bases[2] = {c->kc, c->vc};
-  CUtensorMap* maps[2] = {&c->kmap, &c->vmap};
-  for (int i = 0; i < 2; i++) {
-    const CUresult r = ((EncodeFn)fn)(maps[i], CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, bases[i], dims, strides, box, estr,
-                                      CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                                      CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) return false;
-  }
-  return true;
 }
 
 int fb_bind_kv(fb_ctx* c, void* d_k, void* d_v, int32_t max_seq) {
@@ -764,6 +807,24 @@ int fb_decode(fb_ctx* c, int32_t token, const int32_t* d_token, void* d_h, int32
   return FB_OK;
 }
 
+int fb_prefill(fb_ctx* c, const int32_t* d_tokens, int32_t n, int32_t pos, float* d_logits, void* d_feat, void* stream) {
+  if (!c || !d_tokens || n < 1) return FB_ERR_ARG;
+  if (!c->weights_bound || !c->kc) return FB_ERR_STATE;
+  if (c->tp_size > 1 || !c->embed) return FB_ERR_STATE;
+  if (pos < 0 || n > c->max_seq - pos) return FB_ERR_RANGE;
+  DeviceGuard g(c->device);
+  const fb_model_desc& d = c->d;
+  const int nchunk = (n + kPromptRows - 1) / kPromptRows;      // chunks of equal length: no short last one
+  for (int i = 0; i < nchunk; i++) {
+    const int t0 = (int)((int64_t)n * i / nchunk), t1 = (int)((int64_t)n * (i + 1) / nchunk);
+    const int rc = run_tc_pass(c, d_tokens + t0, nullptr, nullptr, nullptr, t1 - t0, pos + t0,
+                               d_logits ? d_logits + (size_t)t0 * d.vocab : nullptr,
+                               d_feat ? (uint16_t*)d_feat + (size_t)t0 * d.dim : nullptr, (cudaStream_t)stream);
+    if (rc != FB_OK) return rc;
+  }
+  return FB_OK;
+}
+
 int fb_verify(fb_ctx* c, const int32_t* d_tokens, const void* d_h, const int32_t* d_depth, const uint8_t* d_amask,
               int32_t M, int32_t pos, float* d_logits, void* d_feat, void* stream) {
   if (!c || !d_depth || !d_amask || (!d_tokens && !d_h)) return FB_ERR_ARG;
@@ -778,106 +839,12 @@ int fb_verify(fb_ctx* c, const int32_t* d_tokens, const void* d_h, const int32_t
   const int MT = M <= 16 ? 16 : (M <= 32 ? 32 : 64);
   const int D = d.dim, FF = d.ffn, HD = d.head_dim, QD = d.n_head * HD, QKV = (d.n_head + 2 * d.n_kv_head) * HD;
   const bool hz = d.has_zeros != 0;
+  if (c->verify_path == 2 || c->verify_path == 3 || (c->verify_path == 0 && M > 16) || !vgemm_known(D, QD, FF, HD))
+    return run_tc_pass(c, d_tokens, d_h, d_depth, d_amask, M, pos, d_logits, d_feat, st);
   const size_t strQ = (size_t)pad_rows(QKV, D) * rec_bytes_of(D, hz), strO = (size_t)pad_rows(D, QD) * rec_bytes_of(QD, hz),
                strG = (size_t)pad_rows(2 * FF, D) * rec_bytes_of(D, hz), strF = (size_t)pad_rows(D, FF) * rec_bytes_of(FF, hz);
   FB_CUDA(c, launch_pdl(v_embed, dim3(M), dim3(256), 0, st, d_tokens, (const uint16_t*)c->embed, (const uint16_t*)d_h, c->vh,
                         D, d.vocab, d.emb_mult, &c->status->code));
-  if (c->verify_path == 3) {
-    // ---- tcgen05 GEMM chains: per layer one launch covers O -> gate/up -> down -> the next layer's QKV (or the LM head)
-    const size_t tQ = tc_matrix_bytes(QKV, D, hz), tO = tc_matrix_bytes(D, QD, hz), tG = tc_matrix_bytes(2 * FF, D, hz),
-                 tF = tc_matrix_bytes(D, FF, hz);
-    const int L = d.n_layer, nssq = (D + kTcRowBlock - 1) / kTcRowBlock * 4;
-    float *ssqA = c->vssq, *ssqB = c->vssq + 256 * 64;
-    if (nssq > 256) return FB_ERR_SHAPE;
-    FB_CUDA(c, cudaMemsetAsync(c->vgbar, 0, (size_t)(L + 2) * 16, st));
-    FB_CUDA(c, launch_pdl(v_rope_table, dim3(M), dim3(64), 0, st, d_depth, (const float*)c->invf, (int)pos, HD / 2, (float2*)c->vrope));
-    VchainParams t;
-    memset(&t, 0, sizeof(t));
-    t.M = M; t.part = c->vsplit; t.counters = c->vcount; t.status = c->status; t.spin_limit = c->spin_limit;
-    t.rope = (const float2*)c->vrope; t.n_head = d.n_head; t.nkv = d.n_kv_head; t.pos = pos; t.head_dim = HD; t.dim = D;
-    t.resid = d.resid_mult; t.logits_scaling = d.logits_scaling; t.eps = d.rms_eps;
-    auto kcl = [&](int l) { return (uint16_t*)c->kc + (size_t)l * c->max_seq * d.n_kv_head * HD; };
-    auto vcl = [&](int l) { return (uint16_t*)c->vc + (size_t)l * c->max_seq * d.n_kv_head * HD; };
-    auto qkv_phase = [&](int l, bool normed) {
-      VtcPhase f;
-      memset(&f, 0, sizeof(f));
-      f.w = c->t_qkv + l * tQ; f.rows = QKV; f.K = D; f.epi = EPI_QKV; f.q = c->vq; f.kc = kcl(l); f.vc = vcl(l);
-      if (normed) { f.x = c->vh; f.norm_w = (const uint16_t*)c->n1 + (size_t)l * D; f.ssq_in = ssqB; f.n_ssq = nssq; }
-      else f.x = c->vxn;
-      return f;
-    };
-    // layer 0's QKV reads the embeddings through the stand-alone norm kernel
-    FB_CUDA(c, launch_vnorm(c->vh, (const uint16_t*)c->n1, nullptr, c->vxn, D, M, d.rms_eps, st));
-    t.nph = 1; t.ph[0] = qkv_phase(0, false); t.gbar = c->vgbar;
-    FB_CUDA(c, launch_vchain(t, MT, hz, c->sm_count, st));
-    for (int l = 0; l < L; l++) {
-      FB_CUDA(c, launch_vattn(c, c->vq, kcl(l), vcl(l), d_amask, c->vao, pos, M, 1, st));
-      VtcPhase f;
-      memset(&f, 0, sizeof(f));
-      f.w = c->t_o + l * tO; f.x = c->vao; f.rows = D; f.K = QD; f.epi = EPI_RESID; f.h = c->vh; f.out_ld = D; f.ssq_out = ssqA;
-      t.ph[0] = f;
-      memset(&f, 0, sizeof(f));
-      f.w = c->t_gu + l * tG; f.x = c->vh; f.norm_w = (const uint16_t*)c->n2 + (size_t)l * D; f.ssq_in = ssqA; f.n_ssq = nssq;
-      f.rows = 2 * FF; f.K = D; f.epi = EPI_SWIGLU; f.act = c->vact; f.out_ld = FF;
-      t.ph[1] = f;
-      memset(&f, 0, sizeof(f));
-      f.w = c->t_d + l * tF; f.x = c->vact; f.rows = D; f.K = FF; f.epi = EPI_RESID; f.h = c->vh; f.out_ld = D; f.ssq_out = ssqB;
-      t.ph[2] = f;
-      t.nph = 3;
-      if (l + 1 < L) {
-        t.ph[3] = qkv_phase(l + 1, true);
-        t.nph = 4;
-      } else if (d_logits) {
-        memset(&f, 0, sizeof(f));
-        f.w = c->t_lm; f.x = c->vh; f.norm_w = (const uint16_t*)c->nf; f.ssq_in = ssqB; f.n_ssq = nssq; f.xn_out = (uint16_t*)d_feat;
-        f.rows = d.vocab; f.K = D; f.epi = EPI_LOGITS; f.logits = d_logits; f.out_ld = d.vocab;
-        t.ph[3] = f;
-        t.nph = 4;
-      }
-      t.gbar = c->vgbar + 4 * (l + 1);
-      t.dbg = (c->prof && l == 1) ? c->prof : nullptr;
-      FB_CUDA(c, launch_vchain(t, MT, hz, c->sm_count, st));
-    }
-    if (!d_logits && d_feat)
-      FB_CUDA(c, launch_vnorm(c->vh, (const uint16_t*)c->nf, nullptr, (uint16_t*)d_feat, D, M, d.rms_eps, st));
-    FB_CUDA(c, cudaGetLastError());
-    return FB_OK;
-  }
-  if (c->verify_path == 2 || (c->verify_path == 0 && M > 16) || (c->verify_path != 3 && !vgemm_known(D, QD, FF, HD))) {
-    // ---- tcgen05 path: natural-order activations, the matrices in the TC layout ----
-    const size_t tQ = tc_matrix_bytes(QKV, D, hz), tO = tc_matrix_bytes(D, QD, hz), tG = tc_matrix_bytes(2 * FF, D, hz),
-                 tF = tc_matrix_bytes(D, FF, hz);
-    FB_CUDA(c, launch_pdl(v_rope_table, dim3(M), dim3(64), 0, st, d_depth, (const float*)c->invf, (int)pos, HD / 2, (float2*)c->vrope));
-    VtcParams t;
-    memset(&t, 0, sizeof(t));
-    t.M = M; t.has_zeros = hz; t.part = c->vsplit; t.counters = c->vcount; t.status = c->status; t.spin_limit = c->spin_limit;
-    t.rope = (const float2*)c->vrope; t.n_head = d.n_head; t.nkv = d.n_kv_head; t.pos = pos; t.head_dim = HD;
-    t.resid = d.resid_mult; t.logits_scaling = d.logits_scaling;
-    for (int l = 0; l < d.n_layer; l++) {
-      uint16_t* kcl = (uint16_t*)c->kc + (size_t)l * c->max_seq * d.n_kv_head * HD;
-      uint16_t* vcl = (uint16_t*)c->vc + (size_t)l * c->max_seq * d.n_kv_head * HD;
-      FB_CUDA(c, launch_vnorm(c->vh, (const uint16_t*)c->n1 + (size_t)l * D, nullptr, c->vxn, D, M, d.rms_eps, st));
-      t.w = c->t_qkv + l * tQ; t.x = c->vxn; t.rows = QKV; t.K = D; t.q = c->vq; t.kc = kcl; t.vc = vcl;
-      FB_CUDA(c, launch_vtc<EPI_QKV>(t, MT, c->sm_count, st));
-      FB_CUDA(c, launch_vattn(c, c->vq, kcl, vcl, d_amask, c->vao, pos, M, 1, st));
-      t.w = c->t_o + l * tO; t.x = c->vao; t.rows = D; t.K = QD; t.h = c->vh; t.out_ld = D;
-      FB_CUDA(c, launch_vtc<EPI_RESID>(t, MT, c->sm_count, st));
-      FB_CUDA(c, launch_vnorm(c->vh, (const uint16_t*)c->n2 + (size_t)l * D, nullptr, c->vxn, D, M, d.rms_eps, st));
-      t.w = c->t_gu + l * tG; t.x = c->vxn; t.rows = 2 * FF; t.K = D; t.act = c->vact; t.out_ld = FF;
-      FB_CUDA(c, launch_vtc<EPI_SWIGLU>(t, MT, c->sm_count, st));
-      t.w = c->t_d + l * tF; t.x = c->vact; t.rows = D; t.K = FF; t.out_ld = D;
-      FB_CUDA(c, launch_vtc<EPI_RESID>(t, MT, c->sm_count, st));
-    }
-    // the feature goes to the caller in natural order; the LM head reads the same rows
-    uint16_t* feat = d_feat ? (uint16_t*)d_feat : c->vxn;
-    FB_CUDA(c, launch_vnorm(c->vh, (const uint16_t*)c->nf, nullptr, feat, D, M, d.rms_eps, st));
-    if (d_logits) {
-      t.w = c->t_lm; t.x = feat; t.rows = d.vocab; t.K = D; t.logits = d_logits; t.out_ld = d.vocab;
-      FB_CUDA(c, launch_vtc<EPI_LOGITS>(t, MT, c->sm_count, st));
-    }
-    FB_CUDA(c, cudaGetLastError());
-    return FB_OK;
-  }
   VGemmParams p;
   memset(&p, 0, sizeof(p));
   p.M = M; p.has_zeros = hz; p.depth = d_depth; p.invf = c->invf; p.n_head = d.n_head; p.nkv = d.n_kv_head; p.pos = pos;
@@ -909,13 +876,13 @@ int fb_verify(fb_ctx* c, const int32_t* d_tokens, const void* d_h, const int32_t
     if (sub(c->s_qkv, l, QKV, D)) {
       if (sp.plan.nkc == 1) { sp.x = c->vh; sp.norm_w = (const uint16_t*)c->n1 + (size_t)l * D; }
       else {
-        FB_CUDA(c, launch_vnorm(c->vh, (const uint16_t*)c->n1 + (size_t)l * D, c->vxn, nullptr, D, M, d.rms_eps, st));
+        FB_CUDA(c, launch_vnorm(c->vh, (const uint16_t*)c->n1 + (size_t)l * D, c->vxn, nullptr, nullptr, D, M, d.rms_eps, st));
         sp.x = c->vxn;
       }
       sp.q = c->vq; sp.kc = kcl; sp.vc = vcl;
       FB_CUDA(c, launch_vsub<EPI_QKV>(sp, c->sm_count, st));
     } else {
-      FB_CUDA(c, launch_vnorm(c->vh, (const uint16_t*)c->n1 + (size_t)l * D, c->vxn, nullptr, D, M, d.rms_eps, st));
+      FB_CUDA(c, launch_vnorm(c->vh, (const uint16_t*)c->n1 + (size_t)l * D, c->vxn, nullptr, nullptr, D, M, d.rms_eps, st));
       p.w = c->w_qkv + l * strQ; p.x_t = c->vxn; p.rows = QKV;
       p.q = c->vq; p.kc = kcl; p.vc = vcl;
       FB_CUDA(c, launch_vgemm_mt<EPI_QKV>(p, MT, D, HD, c->sm_count, st));
@@ -931,13 +898,13 @@ int fb_verify(fb_ctx* c, const int32_t* d_tokens, const void* d_h, const int32_t
     if (sub(c->s_gu, l, 2 * FF, D)) {
       if (sp.plan.nkc == 1) { sp.x = c->vh; sp.norm_w = (const uint16_t*)c->n2 + (size_t)l * D; }
       else {
-        FB_CUDA(c, launch_vnorm(c->vh, (const uint16_t*)c->n2 + (size_t)l * D, c->vxn, nullptr, D, M, d.rms_eps, st));
+        FB_CUDA(c, launch_vnorm(c->vh, (const uint16_t*)c->n2 + (size_t)l * D, c->vxn, nullptr, nullptr, D, M, d.rms_eps, st));
         sp.x = c->vxn;
       }
       sp.act_t = c->vact; sp.out_ld = FF;
       FB_CUDA(c, launch_vsub<EPI_SWIGLU>(sp, c->sm_count, st));
     } else {
-      FB_CUDA(c, launch_vnorm(c->vh, (const uint16_t*)c->n2 + (size_t)l * D, c->vxn, nullptr, D, M, d.rms_eps, st));
+      FB_CUDA(c, launch_vnorm(c->vh, (const uint16_t*)c->n2 + (size_t)l * D, c->vxn, nullptr, nullptr, D, M, d.rms_eps, st));
       p.w = c->w_gu + l * strG; p.x_t = c->vxn; p.rows = 2 * FF; p.act_t = c->vact;
       p.out_ld = FF;
       FB_CUDA(c, launch_vgemm_mt<EPI_SWIGLU>(p, MT, D, HD, c->sm_count, st));
@@ -950,7 +917,7 @@ int fb_verify(fb_ctx* c, const int32_t* d_tokens, const void* d_h, const int32_t
       FB_CUDA(c, launch_vgemm_mt<EPI_RESID>(p, MT, FF, HD, c->sm_count, st));
     }
   }
-  FB_CUDA(c, launch_vnorm(c->vh, (const uint16_t*)c->nf, c->vxn, (uint16_t*)d_feat, D, M, d.rms_eps, st));
+  FB_CUDA(c, launch_vnorm(c->vh, (const uint16_t*)c->nf, c->vxn, nullptr, (uint16_t*)d_feat, D, M, d.rms_eps, st));
   if (d_logits) {
     if (sub(c->s_lm, 0, d.vocab, D)) {
       sp.x = c->vxn; sp.logits = d_logits; sp.out_ld = d.vocab;

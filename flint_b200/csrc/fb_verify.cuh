@@ -39,11 +39,11 @@ __global__ void v_embed(const int32_t* tokens, const uint16_t* embed, const uint
     h[(size_t)m * D + i] = h_in ? h_in[(size_t)m * D + i] : f2bf(bf2f(embed[(size_t)tok * D + i]) * mult);
 }
 
-// xn[m] = bf16((float(h) * r) * float(w)) in B order; optionally also in natural order (feature out).
+// xn[m] = bf16((float(h) * r) * float(w)) in B order and / or natural order, and once more for the caller (feature out).
 // One CTA per token; a thread keeps its 8-element pieces in registers between the two passes (D <= 8 * 256 * NV).
 template <int NV>
-__global__ void __launch_bounds__(256) v_rmsnorm(const uint16_t* h, const uint16_t* w, uint16_t* xn_t, uint16_t* xn_nat, int D,
-                                                 float eps) {
+__global__ void __launch_bounds__(256) v_rmsnorm(const uint16_t* h, const uint16_t* w, uint16_t* xn_t, uint16_t* xn_nat,
+                                                 uint16_t* feat, int D, float eps) {
   const int m = blockIdx.x, tid = threadIdx.x;
   const uint4* hm = reinterpret_cast<const uint4*>(h + (size_t)m * D);
   const uint4* wv = reinterpret_cast<const uint4*>(w);
@@ -92,6 +92,7 @@ __global__ void __launch_bounds__(256) v_rmsnorm(const uint16_t* h, const uint16
         for (int e = 0; e < 4; e++) dst[2 * e + (i & 1)] = o[e];
       }
       if (xn_nat) reinterpret_cast<uint4*>(xn_nat + (size_t)m * D)[i] = make_uint4(o[0], o[1], o[2], o[3]);
+      if (feat) reinterpret_cast<uint4*>(feat + (size_t)m * D)[i] = make_uint4(o[0], o[1], o[2], o[3]);
     }
   }
 }
@@ -104,11 +105,13 @@ __global__ void __launch_bounds__(256) v_rmsnorm(const uint16_t* h, const uint16
 // positions at a time the N dimension of Q K^T and the K dimension of P V. Query m sees every cached position
 // t < pos and, among the M new slots pos..pos+M-1, those with amask[m][t - pos] != 0. Probabilities enter P V as a
 // sum of two bf16 values (p = hi + lo), which keeps their fp32 precision to ~2^-17. Every span writes, per query row,
-// an un-normalised partial (acc[HD], running max, denominator); v_attn_merge combines the spans.
+// an un-normalised partial (acc[HD], running max, denominator); v_attn_merge combines the spans. With one span (ao set: long
+// prompts have enough query rows to fill the GPU) the CTA normalises and writes its rows itself, natural order. amask == nullptr is the causal
+// chain (amask[m][j] = j <= m): no CTA looks past its last token.
 template <int HD, int R>
 __global__ void __launch_bounds__(128) v_attn_mma(const uint16_t* q, const uint16_t* kc, const uint16_t* vc,
-                                                  const uint8_t* amask, float* part, int n_head, int nkv, int pos, int M,
-                                                  float scale, int span) {
+                                                  const uint8_t* amask, float* part, uint16_t* ao, int n_head, int nkv, int pos,
+                                                  int M, float scale, int span) {
   constexpr int CH = 64, KSTEPS = HD / 16, NTD = HD / 8, STR = HD * 2 + 16, PW = HD + 2;
   static_assert(HD % 16 == 0 && NTD % 2 == 0, "head_dim must be a multiple of 16");
   __shared__ __align__(16) uint8_t k_s[CH * STR];
@@ -118,7 +121,8 @@ __global__ void __launch_bounds__(128) v_attn_mma(const uint16_t* q, const uint1
   const int T = pos + M, QD = n_head * HD, rows = M * R;
   pdl_trigger();
   pdl_wait();
-  const int t_begin = sp * span, t_end = min(T, t_begin + span);
+  const int m_last = min(M - 1, ((int)blockIdx.z * 64 + 63) / R);      // the CTA's last token
+  const int t_begin = sp * span, t_end = min(amask ? T : pos + m_last + 1, t_begin + span);
   const int ntile = (rows + 15) / 16;
   {
     const int mt = (int)blockIdx.z * 4 + warp;
@@ -175,7 +179,10 @@ __global__ void __launch_bounds__(128) v_attn_mma(const uint16_t* q, const uint1
         for (int e = 0; e < 4; e++) {
           const int tp = c0 + nt * 8 + 2 * t + (e & 1);
           bool ok = tp < T;
-          if (tree && ok && tp >= pos) ok = amask[(e < 2 ? m_lo : m_hi) * M + (tp - pos)] != 0;
+          if (tree && ok && tp >= pos) {
+            const int mq = e < 2 ? m_lo : m_hi;
+            ok = amask ? amask[mq * M + (tp - pos)] != 0 : tp - pos <= mq;
+          }
           const float v = ok ? s[nt][e] * scale : -INFINITY;
           s[nt][e] = v;
           mx[e >> 1] = fmaxf(mx[e >> 1], v);
@@ -229,7 +236,13 @@ __global__ void __launch_bounds__(128) v_attn_mma(const uint16_t* q, const uint1
         lrun[h] += __shfl_xor_sync(0xffffffffu, lrun[h], 1);
         lrun[h] += __shfl_xor_sync(0xffffffffu, lrun[h], 2);
         const int row = mt * 16 + g + 8 * h;
-        if (row < rows) {
+        if (row < rows && ao) {
+          const float inv = 1.0f / lrun[h];
+          uint16_t* dst = ao + (size_t)(row / R) * QD + (size_t)(kvh * R + row % R) * HD;
+#pragma unroll
+          for (int j = 0; j < NTD; j++)
+            *reinterpret_cast<uint32_t*>(dst + j * 8 + 2 * t) = pack_bf16(o[j][2 * h] * inv, o[j][2 * h + 1] * inv);
+        } else if (row < rows) {
           float* pr = part + ((size_t)(kvh * S + sp) * rows + row) * PW;
 #pragma unroll
           for (int j = 0; j < NTD; j++)

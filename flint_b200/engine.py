@@ -180,6 +180,18 @@ class DecodeEngine:
         self._keepalive = (tok, depth, amask)
         return logits, feat
 
+    def prefill(self, tokens, pos: int, want_logits: bool = True):
+        """A causal run of any length at positions pos.. in as few weight passes as fit the activation buffers: returns
+        (logits f32 [n, vocab] or None, feature bf16 [n, dim])."""
+        tok = torch.as_tensor(tokens, device=self.device).to(torch.int32).contiguous()
+        n = tok.numel()
+        logits = torch.empty(n, self.cfg.vocab_size, dtype=torch.float32, device=self.device) if want_logits else None
+        feat = torch.empty(n, self.cfg.dim, dtype=torch.bfloat16, device=self.device)
+        _lib.check(self.lib.fb_prefill(self._ctx, _ptr(tok), n, int(pos), _ptr(logits), _ptr(feat), _stream_ptr(self.device)),
+                   "fb_prefill")
+        self._keepalive = (tok,)
+        return logits, feat
+
     def verify_h(self, h: torch.Tensor, pos: int, depth, amask):
         """Same, from already multiplied embeddings h bf16 [M, dim] (the reference's calling convention)."""
         M = h.shape[0]

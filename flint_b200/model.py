@@ -1,9 +1,9 @@
 """gpt-fast style façade over the decode / verify kernels: `Transformer`, `setup_caches`, `model(idx, input_pos)`.
 
 Keeps the call surface of the reference engine (reference: engine/model.py:100-149) so `generate()`-style loops run
-unchanged: one position -> one decode megakernel launch; several positions -> the M-token verify path with a causal
-mask, in chunks of 64 (which also gives chunked prefill instead of the reference's token-by-token prompt loop,
-reference: chat.py:85-86).
+unchanged: one position -> one decode megakernel launch; up to 64 positions -> the M-token verify path with a causal
+mask; more -> the prompt path, up to 1024 tokens per weight pass (the reference feeds prompts token by token, reference:
+chat.py:85-86).
 """
 from __future__ import annotations
 
@@ -59,12 +59,7 @@ class Transformer:
         if S == 1 and not return_hidden:
             lg = self.engine.decode(int(toks[0]), pos0).clone()
             return lg.view(1, 1, -1)
-        outs, feats = [], []
-        for s in range(0, S, 64):
-            lg, ft = self.engine.verify(toks[s:s + 64], pos0 + s)
-            outs.append(lg)
-            feats.append(ft)
-        logits = torch.cat(outs).unsqueeze(0)
-        return (logits, torch.cat(feats).unsqueeze(0)) if return_hidden else logits
+        logits, feats = self.engine.verify(toks, pos0) if S <= 64 else self.engine.prefill(toks, pos0)
+        return (logits.unsqueeze(0), feats.unsqueeze(0)) if return_hidden else logits.unsqueeze(0)
 
     __call__ = forward

@@ -124,6 +124,13 @@ int fb_decode(fb_ctx* ctx, int32_t token, const int32_t* d_token, void* d_h, int
 int fb_verify(fb_ctx* ctx, const int32_t* d_tokens, const void* d_h, const int32_t* d_depth, const uint8_t* d_amask,
               int32_t M, int32_t pos, float* d_logits, void* d_feat, void* stream);
 
+/* A prompt (or a chunk of one): n tokens at positions pos .. pos+n-1, each seeing everything before it; K/V rows are appended to
+ * the cache. The same computation as fb_verify with a causal mask, for any n >= 1 that fits the cache: the tokens pass the layers
+ * in chunks of up to 1024, so the weights are read once per chunk. The reference feeds prompts token by token (reference:
+ * chat.py:83-87).
+ *   d_tokens : device int32[n];   d_logits : f32 [n, vocab] or NULL;   d_feat : bf16 [n, dim] or NULL (as fb_verify) */
+int fb_prefill(fb_ctx* ctx, const int32_t* d_tokens, int32_t n, int32_t pos, float* d_logits, void* d_feat, void* stream);
+
 /* Tree KV surgery after acceptance: cache row dst[i] <- row src[i] in every layer, in order, for K and V.
  * src/dst are HOST arrays. Replaces `kc[:, dst] = kc[:, src]` (reference: spec_tree.py:126-128). */
 int fb_kv_move(fb_ctx* ctx, const int32_t* src, const int32_t* dst, int32_t n, void* stream);
@@ -232,8 +239,8 @@ int fb_gemv_static(const void* d_q, const void* d_s, const void* d_z, int32_t ro
  *           1 = always (shapes built with it: tiny, 3B-class, 8B-class on one GPU), 2 = never
  *   what 7: GEMMs of fb_verify: 0 = chosen by tree size (default: more than 16 tokens run the tcgen05 kernels with
  *           accumulators in tensor memory; smaller trees, latency-bound, run the warp-level mma.sync kernels: up to
- *           8 tokens on fp16-subnormal operands, 9 to 16 on bf16 operands), 1 = warp-level on bf16 operands, 2 = tcgen05,
- *           3 = tcgen05 with four GEMMs chained per launch, 4 = warp-level on fp16-subnormal operands (the decode
+ *           8 tokens on fp16-subnormal operands, 9 to 16 on bf16 operands), 1 = warp-level on bf16 operands, 2 or 3 =
+ *           tcgen05, 4 = warp-level on fp16-subnormal operands (the decode
  *           kernel's arithmetic; symmetric weights, up to 26 tokens, other cases fall back to 1) */
 int fb_set_option(fb_ctx* ctx, int32_t what, int64_t value);
 
