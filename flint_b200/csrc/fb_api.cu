@@ -288,7 +288,7 @@ cudaError_t launch_vtc(VtcParams& p, const CUtensorMap* maps, int nt, bool hz, i
     case 16: return launch_vtc_nt<16, EPI>(p, sms, st, hz);
     case 32: return launch_vtc_nt<32, EPI>(p, sms, st, hz);
     case 64: return launch_vtc_nt<64, EPI>(p, sms, st, hz);
-    case 128: return launch_vtc_hz<128, EPI, false>(p, sms, st);
+    case 128: return launch_vtc_nt<128, EPI>(p, sms, st, hz);
   }
   return cudaErrorInvalidValue;
 }
@@ -303,7 +303,7 @@ constexpr int kPromptRows = 1024;  // token rows of the activation buffers: a pr
 constexpr int kVSpans = 32;       // most spans of positions a kv head's attention is cut into
 
 cudaError_t launch_vattn(const fb_ctx* c, const uint16_t* q, const uint16_t* kc, const uint16_t* vc, const uint8_t* amask,
-                         uint16_t* ao, int pos, int M, int natural, cudaStream_t st) {
+                         uint16_t* ao, int pos, int M, bool f16, cudaStream_t st) {
   const fb_model_desc& d = c->d;
   const int T = pos + M;
   // a CTA takes 64 query rows (four 16-row tiles); spans of positions are sized so that about two CTAs per SM exist
@@ -316,14 +316,16 @@ cudaError_t launch_vattn(const fb_ctx* c, const uint16_t* q, const uint16_t* kc,
   if (S > smax) S = smax;
   const int span = ((T + S - 1) / S + 63) / 64 * 64;
   S = (T + span - 1) / span;
-  uint16_t* direct = S == 1 && natural ? ao : nullptr;
+  uint16_t* direct = S == 1 && f16 ? ao : nullptr;         // one span: the CTAs write their rows, v_row_f16 converts them
+  unsigned* amax = f16 && !direct ? c->vamax : nullptr;
 #define FB_VATTN(HD_, R_)                                                                                               \
   if (d.head_dim == HD_ && c->rgqa == R_) {                                                                             \
     cudaError_t e = launch_pdl(v_attn_mma<HD_, R_>, dim3(d.n_kv_head, S, mgroups), dim3(128), 0, st, q, kc, vc, amask, c->vpart,  \
-                               direct, d.n_head, d.n_kv_head, pos, M, d.attn_scale, span);                                      \
-    if (e != cudaSuccess || direct) return e;                                                                           \
+                               direct, amax, d.n_head, d.n_kv_head, pos, M, d.attn_scale, span);                                      \
+    if (e != cudaSuccess) return e;                                                                                     \
+    if (direct) return launch_pdl(v_row_f16, dim3(M), dim3(256), 0, st, ao, c->vfao, d.n_head * HD_);                    \
     return launch_pdl(v_attn_merge<HD_, R_>, dim3(M, d.n_kv_head), dim3(256), 0, st, (const float*)c->vpart, ao, d.n_head, \
-                      d.n_kv_head, M, S, natural);                                                                      \
+                      d.n_kv_head, M, S, (const unsigned*)amax, c->vfao);                                                                      \
   }
   FB_VATTN(64, 4) FB_VATTN(80, 4) FB_VATTN(64, 5) FB_VATTN(128, 4)
 #undef FB_VATTN
@@ -354,7 +356,7 @@ bool make_act_maps(fb_ctx* c) {
     for (int j = 0; j < 4; j++) {
       const cuuint64_t dims[2] = {widths[i], (cuuint64_t)kPromptRows}, strides[1] = {widths[i] * 2};
       const cuuint32_t box[2] = {64u, 16u << j}, estr[2] = {1u, 1u};
-      if (enc(&maps[i][j], CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, bases[i], dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+      if (enc(&maps[i][j], CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, bases[i], dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
               CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
         return false;
     }
@@ -395,9 +397,8 @@ int run_tc_pass(fb_ctx* c, const int32_t* d_tokens, const void* d_h, const int32
   const fb_model_desc& d = c->d;
   const int D = d.dim, FF = d.ffn, HD = d.head_dim, QD = d.n_head * HD, QKV = (d.n_head + 2 * d.n_kv_head) * HD, sms = c->sm_count;
   const bool hz = d.has_zeros != 0;
-  // token tile: the smallest that holds the tokens; more than 64 go in tiles of up to 128 (64 with zero points: their
-  // accumulator takes the tensor memory of the wider tile), cut evenly
-  const int cap = hz ? 64 : 128, nt = M <= 16 ? 16 : (M <= 32 ? 32 : (M <= 64 ? 64 : cap));
+  // token tile: the smallest that holds the tokens; prompts go in tiles of up to 128, cut evenly
+  const int nt = M <= 16 ? 16 : (M <= 32 ? 32 : (M <= 64 ? 64 : 128));
   const size_t tQ = tc_matrix_bytes(QKV, D, hz), tO = tc_matrix_bytes(D, QD, hz), tG = tc_matrix_bytes(2 * FF, D, hz),
                tF = tc_matrix_bytes(D, FF, hz);
   FB_CUDA(c, launch_pdl(v_embed, dim3(M), dim3(256), 0, st, d_tokens, (const uint16_t*)c->embed, (const uint16_t*)d_h, c->vh,
@@ -408,26 +409,34 @@ int run_tc_pass(fb_ctx* c, const int32_t* d_tokens, const void* d_h, const int32
   t.M = M; t.status = c->status; t.spin_limit = c->spin_limit;
   t.ntile = (M + nt - 1) / nt; t.ntok = ((M + t.ntile - 1) / t.ntile + 15) / 16 * 16;
   t.rope = (const float2*)c->vrope; t.n_head = d.n_head; t.nkv = d.n_kv_head; t.pos = pos; t.head_dim = HD;
-  t.resid = d.resid_mult; t.logits_scaling = d.logits_scaling; t.h = c->vh; t.q = c->vq; t.act = c->vact; t.logits = d_logits;
+  t.resid = d.resid_mult; t.logits_scaling = d.logits_scaling; t.h = c->vh; t.q = c->vq; t.act = c->vact; t.fa = c->vfa;
+  t.logits = d_logits;
+  auto norm = [&](const void* w, uint16_t* feat, const unsigned* norms) {
+    return D <= 8 * 256 ? launch_pdl(v_norm_f16<1>, dim3(M), dim3(256), 0, st, (const uint16_t*)c->vh, (const uint16_t*)w, c->vxn, feat,
+                                     c->vfx, norms, c->vfa, c->vfa_inv, c->vamax, D, d.rms_eps)
+                        : launch_pdl(v_norm_f16<2>, dim3(M), dim3(256), 0, st, (const uint16_t*)c->vh, (const uint16_t*)w, c->vxn, feat,
+                                     c->vfx, norms, c->vfa, c->vfa_inv, c->vamax, D, d.rms_eps);
+  };
+  if (D > 8 * 256 * 2) return FB_ERR_SHAPE;
   for (int l = 0; l < d.n_layer; l++) {
     uint16_t* kcl = (uint16_t*)c->kc + (size_t)l * c->max_seq * d.n_kv_head * HD;
     uint16_t* vcl = (uint16_t*)c->vc + (size_t)l * c->max_seq * d.n_kv_head * HD;
-    FB_CUDA(c, launch_vnorm(c->vh, (const uint16_t*)c->n1 + (size_t)l * D, nullptr, c->vxn, nullptr, D, M, d.rms_eps, st));
-    t.w = c->t_qkv + l * tQ; t.rows = QKV; t.K = D; t.kc = kcl; t.vc = vcl;
+    FB_CUDA(c, norm((const uint16_t*)c->n1 + (size_t)l * D, nullptr, nullptr));
+    t.w = c->t_qkv + l * tQ; t.rows = QKV; t.K = D; t.kc = kcl; t.vc = vcl; t.fx = c->vfx;
     FB_CUDA(c, launch_vtc<EPI_QKV>(t, c->m_xn, nt, hz, sms, st));
-    FB_CUDA(c, launch_vattn(c, c->vq, kcl, vcl, d_amask, c->vao, pos, M, 1, st));
-    t.w = c->t_o + l * tO; t.rows = D; t.K = QD; t.out_ld = D;
+    FB_CUDA(c, launch_vattn(c, c->vq, kcl, vcl, d_amask, c->vao, pos, M, true, st));
+    t.w = c->t_o + l * tO; t.rows = D; t.K = QD; t.out_ld = D; t.fx = c->vfao;
     FB_CUDA(c, launch_vtc<EPI_RESID>(t, c->m_ao, nt, hz, sms, st));
-    FB_CUDA(c, launch_vnorm(c->vh, (const uint16_t*)c->n2 + (size_t)l * D, nullptr, c->vxn, nullptr, D, M, d.rms_eps, st));
-    t.w = c->t_gu + l * tG; t.rows = 2 * FF; t.K = D; t.out_ld = FF;
+    FB_CUDA(c, norm((const uint16_t*)c->n2 + (size_t)l * D, nullptr, c->gu_norms + 2 * l));
+    t.w = c->t_gu + l * tG; t.rows = 2 * FF; t.K = D; t.out_ld = FF; t.fx = c->vfx;
     FB_CUDA(c, launch_vtc<EPI_SWIGLU>(t, c->m_xn, nt, hz, sms, st));
-    t.w = c->t_d + l * tF; t.rows = D; t.K = FF; t.out_ld = D;
+    t.w = c->t_d + l * tF; t.rows = D; t.K = FF; t.out_ld = D; t.fx = c->vfa_inv;
     FB_CUDA(c, launch_vtc<EPI_RESID>(t, c->m_act, nt, hz, sms, st));
   }
-  // the feature goes to the caller; the LM head reads the same rows from the context's buffer
-  FB_CUDA(c, launch_vnorm(c->vh, (const uint16_t*)c->nf, nullptr, c->vxn, (uint16_t*)d_feat, D, M, d.rms_eps, st));
+  // the feature goes to the caller; the LM head reads the context's copy
+  FB_CUDA(c, norm(c->nf, (uint16_t*)d_feat, nullptr));
   if (d_logits) {
-    t.w = c->t_lm; t.rows = d.vocab; t.K = D; t.out_ld = d.vocab;
+    t.w = c->t_lm; t.rows = d.vocab; t.K = D; t.out_ld = d.vocab; t.fx = c->vfx;
     FB_CUDA(c, launch_vtc<EPI_LOGITS>(t, c->m_xn, nt, hz, sms, st));
   }
   FB_CUDA(c, cudaGetLastError());
@@ -536,6 +545,10 @@ int fb_ctx_create_tp(const fb_model_desc* desc, int device, int32_t tp_rank, int
   A(dmalloc(&c->vsplit, kVsplitFloats * 4));
   A(dmalloc(&c->vcount, kVsCounters * 4));
   if (e == cudaSuccess) A(cudaMemset(c->vcount, 0, kVsCounters * 4));
+  float** fp[4] = {&c->vfx, &c->vfao, &c->vfa, &c->vfa_inv};
+  for (float** p : fp) A(dmalloc(p, kPromptRows * 4));
+  A(dmalloc(&c->vamax, kPromptRows * 4));
+  A(dmalloc(&c->gu_norms, (size_t)d.n_layer * 8));
   A(cudaMalloc(&c->vrope, (size_t)kPromptRows * (d.head_dim / 2) * 8));
   A(dmalloc(&c->flags, 3 * 256 * 4));
   if (e == cudaSuccess) A(cudaMemset(c->flags, 0, 3 * 256 * 4));
@@ -571,7 +584,7 @@ int fb_ctx_destroy(fb_ctx* c) {
   void* ptrs[] = {c->w_qkv, c->w_o, c->w_gu, c->w_d, c->w_lm, c->invf,
                   c->status, c->h_ll, c->q_ll, c->k_ll, c->v_ll, c->ao_ll, c->act_ll, c->cand_ll, c->flags,
                   c->part_ll, c->vh, c->vxn, c->vq, c->vao, c->vact, c->vpart, c->inbox,
-                  c->t_qkv, c->t_o, c->t_gu, c->t_d, c->t_lm, c->s_qkv, c->s_o, c->s_gu, c->s_d, c->s_lm, c->vsplit, c->vcount, c->vrope};
+                  c->t_qkv, c->t_o, c->t_gu, c->t_d, c->t_lm, c->s_qkv, c->s_o, c->s_gu, c->s_d, c->s_lm, c->vsplit, c->vcount, c->vrope, c->vfx, c->vfao, c->vfa, c->vfa_inv, c->vamax, c->gu_norms};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   delete c;
@@ -732,8 +745,9 @@ int fb_bind_weights(fb_ctx* c, const fb_weight_ptrs* w, void* stream) {
     if (c->tp_size == 1) {     // the verify path's own copy, in the layout the tcgen05 GEMM streams
       const int nrb = (m.rows + kTcRowBlock - 1) / kTcRowBlock;
       FB_CUDA(c, dmalloc(m.tdst, (size_t)m.layers * tc_matrix_bytes(m.rows, m.k, hz) + 16));
+      if (m.order == 2) FB_CUDA(c, cudaMemsetAsync(c->gu_norms, 0, (size_t)L * 8, st));
       tc_repack<<<dim3(nrb, m.layers), 256, 0, st>>>((const uint32_t*)m.q, (const uint16_t*)m.s, hz ? (const uint16_t*)m.z : nullptr,
-                                                     m.rows, m.k, m.order, m.arg, m.orows, *m.tdst);
+                                                     m.rows, m.k, m.order, m.arg, m.orows, *m.tdst, m.order == 2 ? c->gu_norms : nullptr);
       FB_CUDA(c, cudaGetLastError());
     }
     if (*m.sdst) { cudaFree(*m.sdst); *m.sdst = nullptr; }
@@ -887,7 +901,7 @@ int fb_verify(fb_ctx* c, const int32_t* d_tokens, const void* d_h, const int32_t
       p.q = c->vq; p.kc = kcl; p.vc = vcl;
       FB_CUDA(c, launch_vgemm_mt<EPI_QKV>(p, MT, D, HD, c->sm_count, st));
     }
-    FB_CUDA(c, launch_vattn(c, c->vq, kcl, vcl, d_amask, c->vao, pos, M, 0, st));
+    FB_CUDA(c, launch_vattn(c, c->vq, kcl, vcl, d_amask, c->vao, pos, M, false, st));
     if (sub(c->s_o, l, D, QD)) {
       sp.x = c->vao; sp.h = c->vh; sp.out_ld = D;
       FB_CUDA(c, launch_vsub<EPI_RESID>(sp, c->sm_count, st));

@@ -36,6 +36,9 @@ struct fb_ctx {
   uint8_t *s_qkv, *s_o, *s_gu, *s_d, *s_lm;                          // verify: the matrices in the R32 layout (small trees); NULL = not built
   float* vsplit;                                                    // verify: split-K partial sums
   unsigned* vcount;                                                 // verify: arrivals per (row block, row quadrant)
+  float *vfx, *vfao, *vfa, *vfa_inv;                                // per token: inverse powers of two of xn / attention output, that of the SwiGLU output and its inverse
+  unsigned* vamax;                                                  // per token: bound on the attention output (float bits)
+  unsigned* gu_norms;                                               // [n_layer][2] largest squared row norms of gate and up (float bits)
   void* vrope;                                                      // verify: (cos, sin) per (token, rotation pair)
   int verify_path;                                                  // 0: by tree size, 1: warp-level MMA GEMMs (bf16), 2 or 3: tcgen05 GEMMs, 4: warp-level MMA GEMMs on fp16 subnormals
   int max_fly, poll_words;

@@ -23,6 +23,13 @@ __host__ __device__ __forceinline__ int k16_pos(int col) {       // where column
   return (col & ~15) + (((c & 7) >> 1) << 2) + ((c >> 3) << 1) + (c & 1);
 }
 
+// the power of two that brings a bound `a` on some magnitudes into [2^14, 2^15), and its inverse (both finite for every a >= 0)
+__device__ __forceinline__ float2 pow2_for(float a) {
+  uint32_t mf = 268u - ((__float_as_uint(a) >> 23) & 255u);
+  mf = mf > 253u ? 253u : (mf < 24u ? 24u : mf);
+  return make_float2(__uint_as_float(mf << 23), __uint_as_float((254u - mf) << 23));
+}
+
 // ------------------------------------------------------------------------------------------------ small kernels
 // h[m] = bf16(float(embed[token[m]]) * mult), or a copy of the caller's residual rows
 __global__ void v_embed(const int32_t* tokens, const uint16_t* embed, const uint16_t* h_in, uint16_t* h, int D, int vocab,
@@ -107,11 +114,12 @@ __global__ void __launch_bounds__(256) v_rmsnorm(const uint16_t* h, const uint16
 // sum of two bf16 values (p = hi + lo), which keeps their fp32 precision to ~2^-17. Every span writes, per query row,
 // an un-normalised partial (acc[HD], running max, denominator); v_attn_merge combines the spans. With one span (ao set: long
 // prompts have enough query rows to fill the GPU) the CTA normalises and writes its rows itself, natural order. amask == nullptr is the causal
-// chain (amask[m][j] = j <= m): no CTA looks past its last token.
+// chain (amask[m][j] = j <= m): no CTA looks past its last token. amax (or nullptr): per token, a bound on the magnitudes of the
+// merged output as float bits -- the largest |acc| / denominator of any span (the merge is a convex combination of those).
 template <int HD, int R>
 __global__ void __launch_bounds__(128) v_attn_mma(const uint16_t* q, const uint16_t* kc, const uint16_t* vc,
-                                                  const uint8_t* amask, float* part, uint16_t* ao, int n_head, int nkv, int pos,
-                                                  int M, float scale, int span) {
+                                                  const uint8_t* amask, float* part, uint16_t* ao, unsigned* amax,
+                                                  int n_head, int nkv, int pos, int M, float scale, int span) {
   constexpr int CH = 64, KSTEPS = HD / 16, NTD = HD / 8, STR = HD * 2 + 16, PW = HD + 2;
   static_assert(HD % 16 == 0 && NTD % 2 == 0, "head_dim must be a multiple of 16");
   __shared__ __align__(16) uint8_t k_s[CH * STR];
@@ -236,6 +244,19 @@ __global__ void __launch_bounds__(128) v_attn_mma(const uint16_t* q, const uint1
         lrun[h] += __shfl_xor_sync(0xffffffffu, lrun[h], 1);
         lrun[h] += __shfl_xor_sync(0xffffffffu, lrun[h], 2);
         const int row = mt * 16 + g + 8 * h;
+        if (amax) {
+          float bm = 0.f;
+#pragma unroll
+          for (int j = 0; j < NTD; j++) bm = fmaxf(bm, fmaxf(fabsf(o[j][2 * h]), fabsf(o[j][2 * h + 1])));
+          bm = fmaxf(bm, __shfl_xor_sync(0xffffffffu, bm, 1));
+          bm = fmaxf(bm, __shfl_xor_sync(0xffffffffu, bm, 2));
+          bm = row < rows && lrun[h] > 0.f ? bm / lrun[h] : 0.f;
+          if (R == 4) {                                   // four consecutive rows are the heads of one token
+            bm = fmaxf(bm, __shfl_xor_sync(0xffffffffu, bm, 4));
+            bm = fmaxf(bm, __shfl_xor_sync(0xffffffffu, bm, 8));
+          }
+          if (row < rows && t == 0 && (R != 4 || (g & 3) == 0)) atomicMax(amax + row / R, __float_as_uint(bm));
+        }
         if (row < rows && ao) {
           const float inv = 1.0f / lrun[h];
           uint16_t* dst = ao + (size_t)(row / R) * QD + (size_t)(kvh * R + row % R) * HD;
@@ -254,14 +275,17 @@ __global__ void __launch_bounds__(128) v_attn_mma(const uint16_t* q, const uint1
   }
 }
 
-// one CTA per (token, kv head): combine the spans' partials, write bf16 in B order or natural order (S <= 32 spans)
+// one CTA per (token, kv head): combine the spans' partials, write bf16 in B order or, with the tokens' bounds amax, fp16 in natural
+// order times the token's power of two, whose inverse goes to fx (S <= 32 spans)
 template <int HD, int R>
 __global__ void __launch_bounds__(256) v_attn_merge(const float* part, uint16_t* ao_t, int n_head, int nkv, int M, int S,
-                                                    int natural) {
+                                                    const unsigned* amax, float* fx) {
   constexpr int PW = HD + 2, MAXS = 32;
   const int m = blockIdx.x, kvh = blockIdx.y, rows = M * R, QD = n_head * HD;
   pdl_trigger();
   pdl_wait();
+  const float2 f = amax ? pow2_for(__uint_as_float(__ldcg(amax + m))) : make_float2(1.f, 1.f);
+  if (amax && kvh == 0 && threadIdx.x == 0) fx[m] = f.y;
   for (int o = threadIdx.x; o < R * HD; o += blockDim.x) {
     const int r = o / HD, d = o % HD, row = m * R + r;
     const float* p0 = part + ((size_t)kvh * S * rows + row) * PW;
@@ -284,7 +308,8 @@ __global__ void __launch_bounds__(256) v_attn_merge(const float* part, uint16_t*
       A = fmaf(pa[s2], e, A);
     }
     const int col = (kvh * R + r) * HD + d;
-    ao_t[(size_t)m * QD + (natural ? col : k16_pos(col))] = f2bf(A / Dn);
+    if (amax) ao_t[(size_t)m * QD + col] = __half_as_ushort(__float2half_rn(rbf(A / Dn) * f.x));
+    else ao_t[(size_t)m * QD + k16_pos(col)] = f2bf(A / Dn);
   }
 }
 

@@ -1,25 +1,30 @@
-// int4 x bf16 GEMM of the M-token verify and prefill paths on the 5th-generation tensor cores (tcgen05): a weight row is
-// read once and multiplied with a tile of up to NT tokens (NT = 16 / 32 / 64 for verify, 128 for prompts).
+// int4 GEMM of the M-token verify and prefill paths on the 5th-generation tensor cores (tcgen05): a weight row is read once and
+// multiplied with a tile of up to NT tokens (NT = 16 / 32 / 64 for verify, 128 for prompts).
 //
-// D[128 weight rows][NT tokens] (fp32, in TENSOR MEMORY) = A[128][128] * B[NT][128]^T per group of 128 columns, issued by
-// one thread as eight tcgen05.mma (K = 16 each). A is the group's weights dequantised to bf16 (nib - 8) / 64 -- exact -- by 128
-// threads, thread = weight row = TMEM lane, and stored with tcgen05.st straight into tensor memory (a ring of four
-// 64-column stages): routing A through shared memory would cost 8 bytes of shared-memory traffic per int4 byte and cap
-// the kernel well below the HBM rate. B is the tokens' activations, fetched by tensor copies (box 64 columns x NT tokens)
-// into the K-major 128-byte-swizzle layout the MMA reads. A group of 128 columns shares one bf16 scale per
-// row, so every group accumulates into its own TMEM accumulator (a ring of them); eight warps read a finished group
-// with tcgen05.ld and fold it into per-thread fp32 sums with the row's scale: the arithmetic is the
-// reference's sum (nib - 8) * s * x with fp32 accumulation (reference: kernels/verify_mega.cu:18-75), only the order of
-// summation differs. The asymmetric layout's zero points ride the same groups as a second MMA with A = z (exact in bf16)
-// into an accumulator of their own.
+// D[128 weight rows][NT tokens] (fp32, in TENSOR MEMORY) += A[128][128] * B[NT][128]^T per group of 128 columns, issued as
+// eight tcgen05.mma (K = 16 each) into ONE accumulator for the whole K range. A is the group's weights with their scale,
+// (nib - 8) * s * 2^er, in fp16: the product of a 4-bit and an 8-bit significand fits fp16's 11 bits, and the row's power of two
+// 2^er (chosen from the row's largest scale) keeps it in range, so it is EXACT (up to group scales 2^29 apart within a row). B is
+// the tokens' bf16-rounded activations as fp16, multiplied by one power of two per token: exact as well for elements down to 2^-31
+// of the token's bound. The powers of two come out in the epilogue. The arithmetic is the reference's sum (nib - 8) * s * x with fp32
+// accumulation (reference: kernels/verify_mega.cu:18-75), only the order of summation differs. The asymmetric layout's zero points
+// are a second MMA per step with A = z * 2^er into the same accumulator.
+// What this replaced: bf16 operands (nib - 8) with one accumulator per group, folded with the scale by eight warps that read every
+// group back from tensor memory. That costs a load and an fma per (row, token, group) and two more barrier hand-overs per group: 1000
+// clocks a group for 128 tokens against 512 for its MMAs.
+//
+// A is dequantised by 128-thread sets, thread = weight row = TMEM lane, and stored with tcgen05.st straight into tensor memory (a
+// ring of 64-column stages): routing A through shared memory would cost 8 bytes of shared-memory traffic per int4 byte. B comes by
+// tensor copies (box 64 columns x NT tokens) in the K-major 128-byte-swizzle layout the MMA reads.
 //
 // Weight layout ("TC layout", a library-owned copy made by tc_repack): per block of 128 rows, one record per group of 128
 // columns: two 4 KB chunks [8 words][128 rows] -- word (w, r) holds columns 8w .. 8w+7 of row r with the nibbles ordered so
-// that the four mask-and-fma conversions yield ADJACENT column pairs -- then the group's scales [128 rows] (and zeros).
-// One 1-D bulk copy brings a record; the dequantising thread of row r reads its words without bank conflicts.
+// that the four mask conversions yield ADJACENT column pairs -- then the group's fp16 scales s * 2^er [128 rows] (and zeros);
+// after the last record the rows' factors 2^-er, fp32 [128]. One 1-D bulk copy brings a record; the dequantising thread of row r
+// reads its words without bank conflicts.
 //
 // Work item = (token tile, row block). Small matrices (QKV, O, down) are split along K over a CLUSTER of 2 or 4 CTAs: every
-// CTA sends the sums of a quarter of the tokens to each CTA of its cluster through distributed shared memory, and each
+// CTA sends the sums of a share of the tokens to each CTA of its cluster through distributed shared memory, and each
 // finishes its own tokens (sum in split order: deterministic), so the split costs one cluster barrier instead of a round
 // trip through global memory and the epilogue is shared out as well. Every wait is bounded.
 #pragma once
@@ -30,47 +35,189 @@
 
 namespace fb {
 
-constexpr int kTcStages = 4;      // operand stages: A (dequantised group, 64 TMEM columns) and B (activations, shared memory)
-constexpr int kTcThreads = 512;   // warps: 0 weights, 1 MMA issue, 2 activations, 4..7 dequantise, 8..15 sums and epilogue
+constexpr int kTcThreads = 640;   // warps: 0 weights, 1 MMA issue, 2 activations, 4..11 dequantise, 12..19 epilogue
 constexpr int kTcRowBlock = 128;
 
 __host__ __device__ constexpr int tc_rec_bytes(int has_zeros) { return 8192 + 256 * (has_zeros ? 2 : 1); }
-__host__ __device__ constexpr size_t tc_block_bytes(int k, int has_zeros) { return (size_t)(k / 128) * tc_rec_bytes(has_zeros); }
+__host__ __device__ constexpr size_t tc_block_bytes(int k, int has_zeros) {
+  return (size_t)(k / 128) * tc_rec_bytes(has_zeros) + kTcRowBlock * 4;
+}
 __host__ __device__ constexpr size_t tc_matrix_bytes(int rows, int k, int has_zeros) {
   return (size_t)((rows + kTcRowBlock - 1) / kTcRowBlock) * tc_block_bytes(k, has_zeros);
 }
 
+__device__ __forceinline__ uint32_t f16x2_scaled(uint32_t bf16_pair, float f) {
+  const __half2 hh = __floats2half2_rn(bflo(bf16_pair) * f, bfhi(bf16_pair) * f);
+  return *reinterpret_cast<const uint32_t*>(&hh);
+}
+
 // caller layout (word c of a row = columns 8c .. 8c+7, column 8c+m in bits [4m, 4m+4)) -> TC layout.
-// grid (row blocks, layers), 256 threads.
-__global__ void tc_repack(const uint32_t* q, const uint16_t* sc, const uint16_t* zr, int rows, int K, int order, int order_arg,
-                          int order_rows, uint8_t* out) {
+// grid (row blocks, layers), 256 threads. norms (gate/up only): [layer][2] largest squared row norm of the gate and the up rows,
+// as the bits of non-negative floats (zero before the launch).
+__global__ void __launch_bounds__(256) tc_repack(const uint32_t* q, const uint16_t* sc, const uint16_t* zr, int rows, int K,
+                                                 int order, int order_arg, int order_rows, uint8_t* out, unsigned* norms) {
   const bool hz = zr != nullptr;
-  const int rb = blockIdx.x, nrb = gridDim.x, G = K / 128, nw = K / 8, rec = tc_rec_bytes(hz);
+  const int rb = blockIdx.x, nrb = gridDim.x, G = K / 128, nw = K / 8, rec = tc_rec_bytes(hz), r = threadIdx.x & 127,
+            part = threadIdx.x >> 7;                            // two threads per row
   uint8_t* blk = out + ((size_t)blockIdx.y * nrb + rb) * tc_block_bytes(K, hz);
-  __shared__ int src_row[128];
-  if (threadIdx.x < 128) {
-    const int j = rb * 128 + threadIdx.x;
-    src_row[threadIdx.x] = j < rows ? (int)blockIdx.y * rows + perm_row(j, order, order_arg, order_rows) : -1;
-  }
+  __shared__ float s_max[256], s_sq[256];
+  const int j = rb * 128 + r;
+  const int row = j < rows ? (int)blockIdx.y * rows + perm_row(j, order, order_arg, order_rows) : -1;
+  float mx = 0.f;
+  if (row >= 0)
+    for (int g = part; g < G; g += 2) {
+      mx = fmaxf(mx, 8.0f * fabsf(bf2f(sc[(size_t)row * G + g])));
+      if (hz) mx = fmaxf(mx, fabsf(bf2f(zr[(size_t)row * G + g])));
+    }
+  s_max[threadIdx.x] = mx;
   __syncthreads();
-  for (int i = threadIdx.x; i < nw * 128; i += blockDim.x) {
-    const int r = i & 127, wq = (i >> 7) & 15, g = i >> 11;      // word wq of the group's 16
+  const float2 f = pow2_for(fmaxf(s_max[r], s_max[r + 128]));
+  float sq = 0.f;
+  for (int wq = part; wq < nw; wq += 2) {                      // word wq of the row
+    const int g = wq >> 4;
     uint32_t d = 0x88888888u;                                  // padding rows: value 0
-    if (src_row[r] >= 0) {
-      const uint32_t s = __ldg(q + (size_t)src_row[r] * nw + g * 16 + wq);
+    if (row >= 0) {
+      const uint32_t s = __ldg(q + (size_t)row * nw + wq);
       // column offset e goes to nibble slot [0, 4, 1, 5, 2, 6, 3, 7][e]: (w & 0x000F000F) is then columns (0, 1),
       // (w & 0x00F000F0) columns (2, 3), and the same two masks on w >> 8 columns (4, 5) and (6, 7)
       d = (s & 0xFu) | ((s >> 4 & 0xFu) << 16) | ((s >> 8 & 0xFu) << 4) | ((s >> 12 & 0xFu) << 20) | ((s >> 16 & 0xFu) << 8) |
           ((s >> 20 & 0xFu) << 24) | ((s >> 24 & 0xFu) << 12) | ((s >> 28 & 0xFu) << 28);
+      if (norms) {
+        const float sv = bf2f(sc[(size_t)row * G + g]), zv = hz ? bf2f(zr[(size_t)row * G + g]) : 0.f;
+        for (int e = 0; e < 8; e++) {
+          const float w = ((float)(s >> (4 * e) & 0xFu) - 8.0f) * sv + zv;
+          sq = fmaf(w, w, sq);
+        }
+      }
     }
-    reinterpret_cast<uint32_t*>(blk + (size_t)g * rec)[wq * 128 + r] = d;
+    reinterpret_cast<uint32_t*>(blk + (size_t)g * rec)[(wq & 15) * 128 + r] = d;
   }
-  for (int i = threadIdx.x; i < G * 128; i += blockDim.x) {
-    const int r = i & 127, g = i >> 7, row = src_row[r];
-    uint16_t* meta = reinterpret_cast<uint16_t*>(blk + (size_t)g * rec + 8192);
-    meta[r] = row >= 0 ? sc[(size_t)row * G + g] : 0;
-    if (hz) meta[128 + r] = row >= 0 ? zr[(size_t)row * G + g] : 0;
+  for (int g = part; g < G; g += 2) {
+    __half* meta = reinterpret_cast<__half*>(blk + (size_t)g * rec + 8192);
+    meta[r] = __float2half_rn(row >= 0 ? bf2f(sc[(size_t)row * G + g]) * f.x : 0.f);
+    if (hz) meta[128 + r] = __float2half_rn(row >= 0 ? bf2f(zr[(size_t)row * G + g]) * f.x : 0.f);
   }
+  if (part == 0) reinterpret_cast<float*>(blk + (size_t)G * rec)[r] = f.y;
+  if (norms) {
+    s_sq[threadIdx.x] = sq;
+    __syncthreads();
+    if (part == 0 && row >= 0)
+      atomicMax(norms + blockIdx.y * 2 + (j & 1), __float_as_uint(s_sq[r] + s_sq[r + 128]));
+  }
+}
+
+// xn[m] = bf16((float(h) * r) * float(w)) of one token, as fp16 times a power of two for the GEMM, and as it is for the caller
+// (feat). Leaves the token's factors: fx[m] = inverse of xn's power of two; with `norms` (the following gate/up matrix' largest
+// squared row norms) also the power of two of the SwiGLU output and its inverse: |silu(g) u| <= |g| |u| <= |xn|^2 |Wg| |Wu|.
+// Clears the token's attention bound. One CTA per token; D <= 8 * 256 * NV.
+template <int NV>
+__global__ void __launch_bounds__(256) v_norm_f16(const uint16_t* h, const uint16_t* w, uint16_t* xn, uint16_t* feat, float* fx,
+                                                  const unsigned* norms, float* fa, float* fa_inv, unsigned* amax, int D, float eps) {
+  const int m = blockIdx.x, tid = threadIdx.x;
+  const uint4* hm = reinterpret_cast<const uint4*>(h + (size_t)m * D);
+  const uint4* wv = reinterpret_cast<const uint4*>(w);
+  const int nvec = D / 8;
+  __shared__ float red[8], red2[8], red3[8];
+  uint4 hv[NV], ww[NV];
+  float ss = 0.f;
+  pdl_trigger();
+#pragma unroll
+  for (int k = 0; k < NV; k++) {       // the norm weights do not depend on the previous kernel
+    const int i = tid + k * 256;
+    ww[k] = make_uint4(0, 0, 0, 0);
+    if (i < nvec) ww[k] = __ldg(wv + i);
+  }
+  pdl_wait();
+#pragma unroll
+  for (int k = 0; k < NV; k++) {
+    const int i = tid + k * 256;
+    hv[k] = make_uint4(0, 0, 0, 0);
+    if (i < nvec) hv[k] = hm[i];
+    const uint32_t p[4] = {hv[k].x, hv[k].y, hv[k].z, hv[k].w};
+#pragma unroll
+    for (int e = 0; e < 4; e++) { ss = fmaf(bflo(p[e]), bflo(p[e]), ss); ss = fmaf(bfhi(p[e]), bfhi(p[e]), ss); }
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+  if ((tid & 31) == 0) red[tid >> 5] = ss;
+  __syncthreads();
+  float tot = 0.f;
+#pragma unroll
+  for (int i = 0; i < 8; i++) tot += red[i];
+  const float r = 1.0f / sqrtf(tot / (float)D + eps);
+  float mx = 0.f, sq = 0.f;
+#pragma unroll
+  for (int k = 0; k < NV; k++) {
+    const uint32_t p[4] = {hv[k].x, hv[k].y, hv[k].z, hv[k].w}, q[4] = {ww[k].x, ww[k].y, ww[k].z, ww[k].w};
+    uint32_t o[4];
+#pragma unroll
+    for (int e = 0; e < 4; e++) {
+      o[e] = (uint32_t)f2bf(bflo(p[e]) * r * bflo(q[e])) | ((uint32_t)f2bf(bfhi(p[e]) * r * bfhi(q[e])) << 16);
+      mx = fmaxf(mx, fmaxf(fabsf(bflo(o[e])), fabsf(bfhi(o[e]))));
+      sq = fmaf(bflo(o[e]), bflo(o[e]), fmaf(bfhi(o[e]), bfhi(o[e]), sq));
+    }
+    hv[k] = make_uint4(o[0], o[1], o[2], o[3]);
+    const int i = tid + k * 256;
+    if (feat && i < nvec) reinterpret_cast<uint4*>(feat + (size_t)m * D)[i] = hv[k];
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    sq += __shfl_xor_sync(0xffffffffu, sq, o);
+  }
+  if ((tid & 31) == 0) { red2[tid >> 5] = mx; red3[tid >> 5] = sq; }
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < 8; i++) mx = fmaxf(mx, red2[i]);
+  const float2 f = pow2_for(mx);
+#pragma unroll
+  for (int k = 0; k < NV; k++) {
+    const int i = tid + k * 256;
+    if (i < nvec)
+      reinterpret_cast<uint4*>(xn + (size_t)m * D)[i] = make_uint4(f16x2_scaled(hv[k].x, f.x), f16x2_scaled(hv[k].y, f.x),
+                                                                  f16x2_scaled(hv[k].z, f.x), f16x2_scaled(hv[k].w, f.x));
+  }
+  if (tid == 0) {
+    fx[m] = f.y;
+    amax[m] = 0u;
+    if (norms) {
+      float n2 = 0.f;
+#pragma unroll
+      for (int i = 0; i < 8; i++) n2 += red3[i];
+      const float2 a = pow2_for(n2 * sqrtf(__uint_as_float(norms[0])) * sqrtf(__uint_as_float(norms[1])));
+      fa[m] = a.x;
+      fa_inv[m] = a.y;
+    }
+  }
+}
+
+// Attention output of one token, bf16 -> fp16 times a power of two, in place (the path where the attention CTAs write their rows
+// themselves; v_attn_merge does it on the way otherwise). One CTA of 256 threads per token.
+__global__ void __launch_bounds__(256) v_row_f16(uint16_t* x, float* fx, int D) {
+  const int m = blockIdx.x, tid = threadIdx.x, nvec = D / 8;
+  __shared__ float red[8];
+  uint4* xm = reinterpret_cast<uint4*>(x + (size_t)m * D);
+  pdl_trigger();
+  pdl_wait();
+  float mx = 0.f;
+  for (int i = tid; i < nvec; i += 256) {
+    const uint4 v = xm[i];
+    const uint32_t p[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int e = 0; e < 4; e++) mx = fmaxf(mx, fmaxf(fabsf(bflo(p[e])), fabsf(bfhi(p[e]))));
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+  if ((tid & 31) == 0) red[tid >> 5] = mx;
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < 8; i++) mx = fmaxf(mx, red[i]);
+  const float2 f = pow2_for(mx);
+  for (int i = tid; i < nvec; i += 256) {
+    const uint4 v = xm[i];
+    xm[i] = make_uint4(f16x2_scaled(v.x, f.x), f16x2_scaled(v.y, f.x), f16x2_scaled(v.z, f.x), f16x2_scaled(v.w, f.x));
+  }
+  if (tid == 0) fx[m] = f.y;
 }
 
 // cos / sin of every (token, rotation pair): the QKV epilogue reads them instead of evaluating sincosf per output.
@@ -87,18 +234,20 @@ __global__ void v_rope_table(const int32_t* depth, const float* invf, int pos, i
 }
 
 struct alignas(64) VtcParams {
-  CUtensorMap xmap;          // activations bf16 [rows >= M][K] as a 2-D tensor, box 64 columns x NT tokens, 128-byte swizzle
+  CUtensorMap xmap;          // activations fp16 [rows >= M][K] as a 2-D tensor, box 64 columns x NT tokens, 128-byte swizzle
   const uint8_t* w;          // TC layout of this matrix
   int rows, K, M;
   int nsplit;                // CTAs of a cluster that share one item's K (1, 2 or 4)
   int ntok, ntile;           // tokens of one tile (a multiple of 16, <= NT; one tile unless this is a prompt) and tiles
   DevStatus* status;
   unsigned spin_limit;
+  const float* fx;           // [M, padded to 8] inverse of the power of two in each token's activations
   // epilogue operands
   uint16_t* h;               // RESID: bf16 [M][out_ld] in/out
   uint16_t* q;               // QKV: bf16 [M][n_head * HD]
   uint16_t *kc, *vc;         // QKV: layer base of the caches [max_seq][nkv][HD]
-  uint16_t* act;             // SWIGLU: bf16 [M][out_ld]
+  uint16_t* act;             // SWIGLU: fp16 [M][out_ld], times the token's fa
+  const float* fa;           // SWIGLU: [M, padded to 8]
   float* logits;             // LOGITS: f32 [M][out_ld]
   const float2* rope;        // QKV: [M][HD / 2] (cos, sin)
   int n_head, nkv, pos, out_ld, head_dim;
@@ -110,17 +259,15 @@ __device__ __forceinline__ uint32_t lds32(uint32_t a) {
   asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a));
   return v;
 }
-// nibble pairs in bits (0..3, 16..19) / (4..7, 20..23) -> bf16 pair ((nib - 8) / 64, ...): the masked bits are the bf16
-// subnormals nib * 2^-133 (16 nib * 2^-133); one bf16x2 fma with 2^127 (2^123) and -1/8
-__device__ __forceinline__ uint32_t tc_cvt_lo(uint32_t w) {
-  uint32_t d;
-  asm("fma.rn.bf16x2 %0, %1, %2, %3;" : "=r"(d) : "r"(w & 0x000F000Fu), "r"(0x7F007F00u), "r"(0xBE00BE00u));
-  return d;
+// nibble pairs in bits (0..3, 16..19) / (4..7, 20..23) -> fp16 pair (nib - 8) * s: OR-ing in the exponent of 1024 makes 1024 + nib
+// (1024 + 16 nib); taking 1032 off (or a sixteenth minus 72) is exact, and so is the product
+__device__ __forceinline__ uint32_t tc_h2(__half2 v) { return *reinterpret_cast<const uint32_t*>(&v); }
+__device__ __forceinline__ __half2 tc_as_h2(uint32_t v) { return *reinterpret_cast<const __half2*>(&v); }
+__device__ __forceinline__ uint32_t tc_cvt_lo(uint32_t w, __half2 s) {
+  return tc_h2(__hmul2(__hsub2(tc_as_h2((w & 0x000F000Fu) | 0x64006400u), tc_as_h2(0x64086408u)), s));
 }
-__device__ __forceinline__ uint32_t tc_cvt_hi(uint32_t w) {
-  uint32_t d;
-  asm("fma.rn.bf16x2 %0, %1, %2, %3;" : "=r"(d) : "r"(w & 0x00F000F0u), "r"(0x7D007D00u), "r"(0xBE00BE00u));
-  return d;
+__device__ __forceinline__ uint32_t tc_cvt_hi(uint32_t w, __half2 s) {
+  return tc_h2(__hmul2(__hfma2(tc_as_h2((w & 0x00F000F0u) | 0x64006400u), tc_as_h2(0x2C002C00u), tc_as_h2(0xD480D480u)), s));
 }
 // shared-memory matrix descriptor: K-major, 128-byte swizzle, 8-row groups 1024 bytes apart
 __device__ __forceinline__ uint64_t tc_desc(uint32_t saddr) {
@@ -152,6 +299,12 @@ __device__ __forceinline__ void tc_mma_ts(uint32_t tmem_d, uint32_t tmem_a, uint
 }
 __device__ __forceinline__ void tc_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
+// one lane of a converged warp; unlike `lane == 0` the compiler knows that the rest of the warp does the same uniform work
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}\n" : "=r"(p));
+  return p != 0;
+}
 __device__ __forceinline__ void tc_st8(uint32_t taddr, uint32_t z) {
   asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%1,%1,%1,%1,%1,%1,%1};" ::"r"(taddr), "r"(z) : "memory");
 }
@@ -172,29 +325,37 @@ __device__ __forceinline__ void st_cluster_f32(uint32_t addr, float v) {
   asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory");
 }
 
-// Shared-memory plan (bytes). The raw ring is what keeps HBM busy; a stage of activations is a group's two 64-column tiles.
+// Shared-memory plan (bytes). The raw ring keeps HBM busy; a stage of activations is a group's two 64-column tiles.
 template <int NT, bool HZ>
 struct VtcSmem {
   static constexpr int REC = tc_rec_bytes(HZ);
-  static constexpr int NS = NT > 64 ? 3 : kTcStages;                // operand stages
-  static constexpr int NRAW = NT > 64 ? 6 : 10;                    // raw int4 groups in flight
+  // A stages (64 columns of tensor memory = a dequantised group) take what two accumulators leave
+  static constexpr int NS = NT <= 32 ? 6 : (NT == 64 ? (HZ ? 5 : 6) : (HZ ? 3 : 4));
+  static constexpr int NB = NT <= 16 ? 16 : (NT == 32 ? 12 : (NT == 64 ? 8 : 5));      // activation stages
+  static constexpr int NRAW = NT <= 32 ? 10 : (NT == 64 ? 7 : 6);                      // raw int4 groups
   static constexpr int BSTAGE = NT * 256;                          // two [NT rows x 128 bytes] swizzled tiles
   static constexpr int B = 0;
-  static constexpr int RAW = B + NS * BSTAGE;
-  static constexpr int NSC = 8;                                    // ring of the groups' row scales (x 64), fp32 [128]
-  static constexpr int SC = RAW + NRAW * REC;
-  static constexpr int YS = SC + NSC * 512;                        // sums on their way to the epilogue, fp32 [tokens][128 rows]
-  static constexpr int BAR = YS + NT * 512;
+  static constexpr int RAW = B + NB * BSTAGE;
+  // Barriers that the MMAs of a group complete (one commit per group): group g's is done[g % ND]. Everybody who waits for a
+  // group to retire (its A stage, its activation stage) waits there; nobody is ND groups behind.
+  static constexpr int ND = 16;
+  static_assert(ND >= NB && ND >= NS, "a retired group must not be overtaken by the next one on its barrier");
+  static constexpr int YS = RAW + NRAW * REC;                      // K splits: the other ranks' sums, fp32 [rank][tokens][128 rows]
+  static constexpr int BAR = YS + (NT <= 64 ? NT * 512 : 0);
   static constexpr int TOTAL = BAR + 512 + 1024;                   // barriers + slack to align the base
   static_assert(TOTAL <= 227 * 1024, "verify GEMM shared memory");
-  // tensor memory columns: group accumulators, zero-point accumulator, A stages (64 columns = 128 bf16 per row), A_z
-  // (8 columns = one k16 step of the row's zero point, the same for every step of the group)
-  static constexpr int NACC = (NT > 64 || (NT == 64 && HZ)) ? 2 : 4;
-  static constexpr int T_ACCZ = NACC * NT, T_A = T_ACCZ + (HZ ? NT : 0), T_AZ = T_A + NS * 64;
+  // tensor memory columns: two accumulators (the epilogue of an item overlaps the MMAs of the next), A stages, A_z (8 columns = one
+  // k16 step of the row's zero point, the same for every step of the group)
+  static constexpr int T_A = 2 * NT, T_AZ = T_A + NS * 64;
   static_assert(T_AZ + (HZ ? NS * 8 : 0) <= 512, "tensor memory columns");
-  // A scale slot of group g is rewritten for group g + NSC. The writer (dequantising group g + NSC) has seen the MMAs of group
-  // g + NSC - NS retire, whose accumulator was free: the sums of group g + NSC - NS - NACC have been read. So:
-  static_assert(NSC >= NS + NACC, "a scale slot must outlive its group's sums");
+};
+
+// position in a ring of N: index and the parity of its current lap
+template <int N>
+struct Ring {
+  int i = 0;
+  uint32_t lap = 0;
+  __device__ __forceinline__ void next() { if (++i == N) { i = 0; lap ^= 1u; } }
 };
 
 // work items of this CTA in order (token tile by token tile: the tile's activations stay in L2); every role walks the same
@@ -216,15 +377,22 @@ struct TcWalk {
   __device__ __forceinline__ void next() { item += step; set(); }
 };
 
-constexpr int kTcChunk = 8;       // tokens whose epilogue operands a thread loads before it uses the first
+constexpr int kTcChunk = 8;       // tokens whose epilogue operands a thread loads together
 
 // What one chunk of the epilogue reads from global memory (issued early: it does not depend on the GEMM)
 struct TcOperands {
+  float fx[kTcChunk], fa[kTcChunk];
   uint16_t h[kTcChunk];
   float2 cs[kTcChunk];
 };
 template <int EPI>
 __device__ __forceinline__ void vtc_fetch(const VtcParams& P, int srow, int t0, int tend, TcOperands& o) {
+#pragma unroll
+  for (int e = 0; e < kTcChunk; e++) {
+    const int t = min(t0 + e, tend - 1);
+    o.fx[e] = __ldcg(P.fx + t);
+    if (EPI == EPI_SWIGLU) o.fa[e] = __ldcg(P.fa + t);
+  }
   if (EPI == EPI_RESID) {
 #pragma unroll
     for (int e = 0; e < kTcChunk; e++)
@@ -237,12 +405,14 @@ __device__ __forceinline__ void vtc_fetch(const VtcParams& P, int srow, int t0, 
       o.cs[e] = (rot && t0 + e < tend) ? __ldg(P.rope + (size_t)(t0 + e) * HP + i) : make_float2(1.f, 0.f);
   }
 }
-// v[e] = the finished sum of (stream row srow, token t0 + e). The whole warp calls this together: lanes 2i, 2i + 1 hold the two
-// rows of a RoPE or gate/up pair.
+// v[e] = accumulator of (stream row srow, token t0 + e), rf = the row's factor. The whole warp calls this together: lanes
+// 2i, 2i + 1 hold the two rows of a RoPE or gate/up pair.
 template <int EPI>
-__device__ __forceinline__ void vtc_epilogue(const VtcParams& P, int srow, int t0, int tend, const float (&v)[kTcChunk],
+__device__ __forceinline__ void vtc_epilogue(const VtcParams& P, int srow, int t0, int tend, float (&v)[kTcChunk], float rf,
                                              const TcOperands& o, int lane) {
   const bool live = srow < P.rows, odd = lane & 1;
+#pragma unroll
+  for (int e = 0; e < kTcChunk; e++) v[e] = v[e] * rf * o.fx[e];
   if (EPI == EPI_RESID) {
 #pragma unroll
     for (int e = 0; e < kTcChunk; e++)
@@ -258,7 +428,8 @@ __device__ __forceinline__ void vtc_epilogue(const VtcParams& P, int srow, int t
       const float got = __shfl_xor_sync(0xffffffffu, odd ? v[e] : v[e + 1], 1);
       const float gg = rbf(odd ? got : v[e]), uu = rbf(odd ? v[e + 1] : got);
       const int t = t0 + e + (odd ? 1 : 0);
-      if (live && t < tend) P.act[(size_t)t * P.out_ld + (srow >> 1)] = f2bf((gg / (1.0f + __expf(-gg))) * uu);
+      const __half a = __float2half_rn(rbf((gg / (1.0f + __expf(-gg))) * uu) * (odd ? o.fa[e + 1] : o.fa[e]));
+      if (live && t < tend) P.act[(size_t)t * P.out_ld + (srow >> 1)] = __half_as_ushort(a);
     }
   } else {
     // QKV: stream rows (2p, 2p+1) of a q / k head are dims (p, p + HD/2); v rows keep their order
@@ -278,7 +449,7 @@ __device__ __forceinline__ void vtc_epilogue(const VtcParams& P, int srow, int t
     for (int e = 0; e < kTcChunk; e++) {
       const float x = rbf(v[e]), y = __shfl_xor_sync(0xffffffffu, x, 1);
       const float r = odd ? x * o.cs[e].x + y * o.cs[e].y : x * o.cs[e].x - y * o.cs[e].y;
-      if (live && t0 + e < tend) base[(size_t)(t0 + e) * ld] = f2bf(rot ? r : x);
+      if (live && t0 + e < tend) base[(size_t)(t0 + e) * ld] = f2bf(rot ? r : (v[e]));
     }
   }
 }
@@ -286,22 +457,23 @@ __device__ __forceinline__ void vtc_epilogue(const VtcParams& P, int srow, int t
 template <int NT, int EPI, bool HZ>
 __global__ void __launch_bounds__(kTcThreads, 1) v_gemm_tc(const __grid_constant__ VtcParams P) {
   using S = VtcSmem<NT, HZ>;
-  constexpr int NRAW = S::NRAW, NS = S::NS, NACC = S::NACC, REC = S::REC, HC = NT / 2;
+  constexpr int NRAW = S::NRAW, NS = S::NS, NB = S::NB, ND = S::ND, REC = S::REC, HC = NT / 2;
   extern __shared__ __align__(1024) uint8_t tsm_raw[];
   // the swizzle pattern is a function of the absolute shared-memory address: tiles must start on 1024-byte boundaries
   uint8_t* tsm = tsm_raw + ((1024u - (smem_u32(tsm_raw) & 1023u)) & 1023u);
   uint64_t* bars = reinterpret_cast<uint64_t*>(tsm + S::BAR);
-  uint64_t *raw_full = bars, *raw_empty = bars + NRAW, *a_full = bars + 2 * NRAW, *b_full = a_full + NS, *s_empty = b_full + NS,
-           *acc_full = s_empty + NS, *acc_empty = acc_full + NACC;
-  uint32_t* s_tmem = reinterpret_cast<uint32_t*>(acc_empty + NACC);
+  uint64_t *raw_full = bars, *raw_empty = bars + NRAW, *a_full = bars + 2 * NRAW, *b_full = a_full + NS, *done = b_full + NB,
+           *acc_full = done + ND, *acc_empty = acc_full + 2;
+  uint32_t* s_tmem = reinterpret_cast<uint32_t*>(acc_empty + 2);
   volatile int* s_abort = reinterpret_cast<volatile int*>(s_tmem + 1);
-  float* scr = reinterpret_cast<float*>(tsm + S::SC);
   float* ys = reinterpret_cast<float*>(tsm + S::YS);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (tid == 0) {
     for (int i = 0; i < NRAW; i++) { mbar_init(&raw_full[i], 1); mbar_init(&raw_empty[i], 4); }
-    for (int i = 0; i < NS; i++) { mbar_init(&a_full[i], 4); mbar_init(&b_full[i], 1); mbar_init(&s_empty[i], 1); }
-    for (int i = 0; i < NACC; i++) { mbar_init(&acc_full[i], 1); mbar_init(&acc_empty[i], 8); }
+    for (int i = 0; i < NS; i++) mbar_init(&a_full[i], 4);
+    for (int i = 0; i < NB; i++) mbar_init(&b_full[i], 1);
+    for (int i = 0; i < ND; i++) mbar_init(&done[i], 1);
+    for (int i = 0; i < 2; i++) { mbar_init(&acc_full[i], 1); mbar_init(&acc_empty[i], 8); }
     *s_abort = 0;
     mbar_fence_init();
   }
@@ -315,29 +487,30 @@ __global__ void __launch_bounds__(kTcThreads, 1) v_gemm_tc(const __grid_constant
   tc_fence_after();
   const uint32_t tmem = *s_tmem;
   WaitCtl wc{P.status, s_abort, P.spin_limit};
-  const bool split = P.nsplit > 1;
+  const bool split = NT <= 64 && P.nsplit > 1;
   if (split) { cluster_arrive(); cluster_wait(); }               // the neighbours' shared memory exists from here on
   pdl_trigger();
-  const int quad = warp & 3, row = quad * 32 + lane;             // warps 4..15: row of the block = TMEM lane
-  const int half = (warp >> 2) & 1;                              // warps 8..15: which half of the token columns
+  const int quad = warp & 3, row = quad * 32 + lane;             // warps 4..19: row of the block = TMEM lane
+  const int half = ((warp >> 2) & 1) ^ 1;                        // warps 4..11: which groups; warps 12..19: which half of the tokens
   // splits: this CTA finishes tokens [rank * TPR, (rank + 1) * TPR) of the item
   const int TPR = NT / P.nsplit, lgT = 31 - __clz(TPR), rank = (int)blockIdx.x % P.nsplit;
   bool ok = true;
   TcOperands pre;
   int e_srow = 0, e_t0 = 0, e_tend = 0;                          // split items: the epilogue's row and first token
+  float e_rf = 0.f;
 
   if (warp == 0) {
     // ---------------- producer: the groups' records (weights do not depend on the previous kernel)
     if (lane == 0) {
       uint32_t gi = 0;
+      Ring<NRAW> r;
       for (TcWalk w(P); w.valid() && ok; w.next()) {
         const uint8_t* blk = P.w + (size_t)w.rb * tc_block_bytes(P.K, HZ);
-        for (int g = w.g0; g < w.g1; g++, gi++) {
-          const int s = gi % NRAW;
-          ok = mbar_wait(&raw_empty[s], ((gi / NRAW) & 1) ^ 1, wc, W_EMPTY, 2);
+        for (int g = w.g0; g < w.g1; g++, gi++, r.next()) {
+          ok = mbar_wait(&raw_empty[r.i], r.lap ^ 1u, wc, W_EMPTY, 2);
           if (!ok) break;
-          mbar_expect_tx(&raw_full[s], REC);
-          bulk_g2s(tsm + S::RAW + s * REC, blk + (size_t)g * REC, REC, &raw_full[s]);
+          mbar_expect_tx(&raw_full[r.i], REC);
+          bulk_g2s(tsm + S::RAW + r.i * REC, blk + (size_t)g * REC, REC, &raw_full[r.i]);
         }
       }
       // every copy issued must have landed before the CTA may exit: the consumers wait for all of them in a clean run;
@@ -353,28 +526,36 @@ __global__ void __launch_bounds__(kTcThreads, 1) v_gemm_tc(const __grid_constant
       }
     }
   } else if (warp == 1) {
-    // ---------------- MMA issue: one thread, eight MMAs per group, two commits
-    if (lane == 0) {
-      const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(P.ntok >> 3) << 17) | ((128u >> 4) << 24);
-      uint32_t gi = 0;
-      for (TcWalk w(P); w.valid() && ok; w.next()) {
-        for (int g = w.g0; g < w.g1 && ok; g++, gi++) {
-          const int a = gi % NACC, s = gi % NS;
-          ok = mbar_wait(&acc_empty[a], ((gi / NACC) & 1) ^ 1, wc, W_EMPTY, 3) && mbar_wait(&a_full[s], (gi / NS) & 1, wc, W_FULL, 4) &&
-               mbar_wait(&b_full[s], (gi / NS) & 1, wc, W_FULL, 4);
-          if (!ok) break;
-          tc_fence_after();
-          const uint32_t ta = tmem + S::T_A + s * 64, tz = tmem + S::T_AZ + s * 8;
-          const uint32_t sb = smem_u32(tsm + S::B + s * S::BSTAGE);
+    // ---------------- MMA issue: the warp waits as one, an elected lane issues eight MMAs per group and one commit. (With the
+    // whole loop under `lane == 0` every operand took a trip through the vector registers: 0.36 us per group on top of the MMAs.)
+    const uint32_t idesc = (1u << 4) | ((uint32_t)(P.ntok >> 3) << 17) | ((128u >> 4) << 24);      // fp16 x fp16 -> fp32
+    Ring<NS> rs;
+    Ring<NB> rb;
+    Ring<ND> rd;
+    Ring<2> ra;
+    for (TcWalk w(P); w.valid() && ok; w.next(), ra.next()) {
+      ok = __all_sync(0xffffffffu, mbar_wait(&acc_empty[ra.i], ra.lap ^ 1u, wc, W_EMPTY, 3));
+      for (int g = w.g0; g < w.g1 && ok; g++, rs.next(), rb.next(), rd.next()) {
+        // both are usually there already: test them side by side, a barrier test is a round trip of its own
+        bool now = mbar_try(&a_full[rs.i], rs.lap);
+        now = mbar_try(&b_full[rb.i], rb.lap) && now;
+        if (!now) ok = mbar_wait(&a_full[rs.i], rs.lap, wc, W_FULL, 4) && mbar_wait(&b_full[rb.i], rb.lap, wc, W_FULL, 4);
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) break;
+        tc_fence_after();
+        if (elect_one()) {
+          const uint32_t ta = tmem + S::T_A + rs.i * 64, tz = tmem + S::T_AZ + rs.i * 8, td = tmem + ra.i * NT;
+          const uint64_t db0 = tc_desc(smem_u32(tsm + S::B + rb.i * S::BSTAGE));
 #pragma unroll
           for (int k = 0; k < 8; k++) {
-            const uint64_t db = tc_desc(sb + (k >> 2) * (NT * 128) + (k & 3) * 32);
-            tc_mma_ts(tmem + a * NT, ta + k * 8, db, idesc, k ? 1u : 0u);
-            if (HZ) tc_mma_ts(tmem + S::T_ACCZ, tz, db, idesc, (g > w.g0 || k) ? 1u : 0u);
+            const uint64_t db = db0 + (uint64_t)(((k >> 2) * (NT * 128) + (k & 3) * 32) >> 4);
+            tc_mma_ts(td, ta + k * 8, db, idesc, (g > w.g0 || k) ? 1u : 0u);
+            if (HZ) tc_mma_ts(td, tz, db, idesc, 1u);
           }
-          tc_commit(&s_empty[s]);
-          tc_commit(&acc_full[a]);
+          tc_commit(&done[rd.i]);
+          if (g == w.g1 - 1) tc_commit(&acc_full[ra.i]);
         }
+        __syncwarp();
       }
     }
   } else if (warp == 2) {
@@ -383,142 +564,126 @@ __global__ void __launch_bounds__(kTcThreads, 1) v_gemm_tc(const __grid_constant
     pdl_wait();
     if (lane == 0) {
       uint32_t gi = 0;
+      Ring<NB> r;
       for (TcWalk w(P); w.valid() && ok; w.next()) {
-        for (int g = w.g0; g < w.g1; g++, gi++) {
-          const int s = gi % NS;
-          ok = mbar_wait(&s_empty[s], ((gi / NS) & 1) ^ 1, wc, W_EMPTY, 8);
+        for (int g = w.g0; g < w.g1; g++, gi++, r.next()) {
+          // group gi - NB has retired
+          ok = gi < NB || mbar_wait(&done[(gi - NB) % ND], ((gi - NB) / ND) & 1, wc, W_EMPTY, 8);
           if (!ok) break;
-          mbar_expect_tx(&b_full[s], S::BSTAGE);
-          uint8_t* dst = tsm + S::B + s * S::BSTAGE;
-          tma_load_2d(dst, &P.xmap, g * 128, w.tt * P.ntok, &b_full[s]);
-          tma_load_2d(dst + NT * 128, &P.xmap, g * 128 + 64, w.tt * P.ntok, &b_full[s]);
+          mbar_expect_tx(&b_full[r.i], S::BSTAGE);
+          uint8_t* dst = tsm + S::B + r.i * S::BSTAGE;
+          tma_load_2d(dst, &P.xmap, g * 128, w.tt * P.ntok, &b_full[r.i]);
+          tma_load_2d(dst + NT * 128, &P.xmap, g * 128 + 64, w.tt * P.ntok, &b_full[r.i]);
         }
       }
       if (*s_abort) {
-        for (int k = 0; k < NS && k < (int)gi; k++) {
+        for (int k = 0; k < NB && k < (int)gi; k++) {
           const uint32_t j = gi - 1 - k;
           for (unsigned i = 0; i < wc.limit; i++) {
-            if (mbar_try(&b_full[j % NS], (j / NS) & 1)) break;
+            if (mbar_try(&b_full[j % NB], (j / NB) & 1)) break;
             if ((i & 1023) == 1023) __nanosleep(64);
           }
         }
       }
     }
-  } else if (warp >= 4 && warp < 8) {
-    // ---------------- dequantise: thread = row of the block = TMEM lane; 16 words -> 64 packed bf16 pairs per group
+  } else if (warp >= 4 && warp < 12) {
+    // ---------------- dequantise: two sets of four warps take the groups in turn; thread = row of the block = TMEM lane; 16 words
+    // -> 64 packed fp16 pairs per group
     const uint32_t tl = tmem + ((uint32_t)(quad * 32) << 16);
     uint32_t gi = 0;
+    Ring<NRAW> rr;
+    Ring<NS> rs;
     for (TcWalk w(P); w.valid() && ok; w.next()) {
-      for (int g = w.g0; g < w.g1; g++, gi++) {
-        const int sr = gi % NRAW, s = gi % NS;
-        ok = mbar_wait(&raw_full[sr], (gi / NRAW) & 1, wc, W_FULL, 5) && mbar_wait(&s_empty[s], ((gi / NS) & 1) ^ 1, wc, W_EMPTY, 6);
+      for (int g = w.g0; g < w.g1; g++, gi++, rr.next(), rs.next()) {
+        if ((int)(gi & 1) != half) continue;
+        uint64_t* freed = &done[(gi - NS) % ND];                 // the stage's previous group has retired
+        const uint32_t fpar = ((gi - NS) / ND) & 1;
+        bool now = mbar_try(&raw_full[rr.i], rr.lap);
+        if (gi >= NS) now = mbar_try(freed, fpar) && now;
+        if (!now) ok = mbar_wait(&raw_full[rr.i], rr.lap, wc, W_FULL, 5) && (gi < NS || mbar_wait(freed, fpar, wc, W_EMPTY, 6));
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
         tc_fence_after();
-        const uint8_t* rec = tsm + S::RAW + sr * REC;
+        const uint8_t* rec = tsm + S::RAW + rr.i * REC;
         const uint32_t raw = smem_u32(rec) + (uint32_t)row * 4;
-        scr[(gi % S::NSC) * 128 + row] = bf2f(reinterpret_cast<const uint16_t*>(rec + 8192)[row]) * 64.0f;
+        const __half2 sc = __half2half2(reinterpret_cast<const __half*>(rec + 8192)[row]);
 #pragma unroll
         for (int c = 0; c < 2; c++) {
           uint32_t v[32];
 #pragma unroll
           for (int q8 = 0; q8 < 8; q8++) {
             const uint32_t wv = lds32(raw + c * 4096 + q8 * 512);
-            v[4 * q8] = tc_cvt_lo(wv); v[4 * q8 + 1] = tc_cvt_hi(wv); v[4 * q8 + 2] = tc_cvt_lo(wv >> 8); v[4 * q8 + 3] = tc_cvt_hi(wv >> 8);
+            v[4 * q8] = tc_cvt_lo(wv, sc); v[4 * q8 + 1] = tc_cvt_hi(wv, sc);
+            v[4 * q8 + 2] = tc_cvt_lo(wv >> 8, sc); v[4 * q8 + 3] = tc_cvt_hi(wv >> 8, sc);
           }
-          tc_st32(tl + S::T_A + s * 64 + c * 32, v);
+          tc_st32(tl + S::T_A + rs.i * 64 + c * 32, v);
         }
         if (HZ) {
           // the group's zero point of this row as one k16 step: A_z = z for every column
           const uint16_t z = reinterpret_cast<const uint16_t*>(rec + 8448)[row];
-          tc_st8(tl + S::T_AZ + s * 8, (uint32_t)z | ((uint32_t)z << 16));
+          tc_st8(tl + S::T_AZ + rs.i * 8, (uint32_t)z | ((uint32_t)z << 16));
         }
         tc_st_wait();
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) { mbar_arrive(&raw_empty[sr]); mbar_arrive(&a_full[s]); }
+        if (lane == 0) { mbar_arrive(&a_full[rs.i]); mbar_arrive(&raw_empty[rr.i]); }
       }
     }
-  } else if (warp >= 8) {
-    // ---------------- sums: thread = (row of the block, half of the tokens), HC fp32 sums in registers
+  } else if (warp >= 12) {
+    // ---------------- epilogue: thread = (row of the block, half of the tokens), eight tokens at a time
     const uint32_t tlane = tmem + ((uint32_t)(quad * 32) << 16) + half * HC;
-    uint32_t gi = 0;
+    Ring<2> ra;
     pdl_wait();
-    for (TcWalk w(P); w.valid() && ok; w.next()) {
-      float y[HC];
-#pragma unroll
-      for (int t = 0; t < HC; t++) y[t] = 0.f;
-      const int tok0 = w.tt * P.ntok, tend = min(P.M, tok0 + P.ntok);
-      if (split) {                                               // one item: fetch what its epilogue needs while the GEMM runs
-        e_srow = w.rb * 128 + row; e_t0 = rank * TPR + half * (TPR / 2); e_tend = min(tend, e_t0 + TPR / 2);
-        vtc_fetch<EPI>(P, e_srow, e_t0, e_tend, pre);
-      }
-      for (int g = w.g0; g < w.g1; g++, gi++) {
-        const int a = gi % NACC;
-        ok = __all_sync(0xffffffffu, mbar_wait(&acc_full[a], (gi / NACC) & 1, wc, W_FULL, 10));
-        if (!ok) break;
-        tc_fence_after();
-        const float s64 = scr[(gi % S::NSC) * 128 + row];
-        constexpr int LB = HC > 32 ? 16 : HC;                    // columns per batch of loads: one wait per batch
-#pragma unroll
-        for (int h0 = 0; h0 < HC; h0 += LB) {
-          uint32_t v[LB / 8][8];
-#pragma unroll
-          for (int c8 = 0; c8 < LB / 8; c8++) tc_ld8(tlane + a * NT + h0 + c8 * 8, v[c8]);
-          tc_ld_wait();
-#pragma unroll
-          for (int c8 = 0; c8 < LB / 8; c8++)
-#pragma unroll
-            for (int e = 0; e < 8; e++) y[h0 + c8 * 8 + e] = fmaf(s64, __uint_as_float(v[c8][e]), y[h0 + c8 * 8 + e]);
-        }
-        if (HZ && g == w.g1 - 1) {                               // the item's zero-point sums: sum_g z_g * sum_k x_k
-#pragma unroll
-          for (int c8 = 0; c8 < HC / 8; c8++) {
-            uint32_t v[8];
-            tc_ld8(tlane + S::T_ACCZ + c8 * 8, v);
-            tc_ld_wait();
-#pragma unroll
-            for (int e = 0; e < 8; e++) y[c8 * 8 + e] += __uint_as_float(v[e]);
-          }
-        }
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&acc_empty[a]);
-      }
+    for (TcWalk w(P); w.valid() && ok; w.next(), ra.next()) {
+      const int tok0 = w.tt * P.ntok, tend = min(P.M, tok0 + P.ntok), srow = w.rb * 128 + row;
+      // the row's factor and the first chunk's operands are fetched while the GEMM runs
+      const float rf = __ldg(reinterpret_cast<const float*>(P.w + (size_t)(w.rb + 1) * tc_block_bytes(P.K, HZ)) - kTcRowBlock + row);
+      const int th0 = split ? rank * TPR + half * (TPR / 2) : tok0 + half * HC;
+      const int the = min(tend, th0 + (split ? TPR / 2 : HC));
+      if (split) { e_srow = srow; e_t0 = th0; e_tend = the; e_rf = rf; }
+      if (th0 < the) vtc_fetch<EPI>(P, srow, th0, the, pre);
+      ok = __all_sync(0xffffffffu, mbar_wait(&acc_full[ra.i], ra.lap, wc, W_FULL, 10));
       if (!ok) break;
+      tc_fence_after();
       if (split) {
         // token t of this half goes to the CTA that finishes it: its ys is [source rank][its tokens][128 rows]
         const uint32_t mine = smem_u32(ys) + (uint32_t)(rank * TPR * 128 + row) * 4;
 #pragma unroll
-        for (int t = 0; t < HC; t++) {
-          const int tk = half * HC + t;
-          st_cluster_f32(map_rank(mine + (uint32_t)(tk & (TPR - 1)) * 512, tk >> lgT), y[t]);
+        for (int c = 0; c < HC; c += 8) {
+          uint32_t v[8];
+          tc_ld8(tlane + ra.i * NT + c, v);
+          tc_ld_wait();
+#pragma unroll
+          for (int e = 0; e < 8; e++) {
+            const int tk = half * HC + c + e;
+            st_cluster_f32(map_rank(mine + (uint32_t)(tk & (TPR - 1)) * 512, tk >> lgT), __uint_as_float(v[e]));
+          }
         }
       } else {
-        // The sums go through shared memory ([token][row], a warp touches only its own rows and tokens) so that the per-token
-        // work is a compact loop: unrolled over all tokens it is tens of KB of straight-line code that runs once per item, one
-        // instruction-cache miss after the other.
-        float* yw = ys + half * HC * 128 + row;
-        __syncwarp();                                            // the previous item's readers are done
-#pragma unroll
-        for (int t = 0; t < HC; t++) yw[t * 128] = y[t];
-        __syncwarp();
-        const int srow = w.rb * 128 + row, th0 = tok0 + half * HC, the = min(tend, th0 + HC);
-        for (int t0 = 0; th0 + t0 < the; t0 += kTcChunk) {
-          vtc_fetch<EPI>(P, srow, th0 + t0, the, pre);
+#pragma unroll 1
+        for (int t0 = th0; t0 < the; t0 += kTcChunk) {
+          uint32_t u[8];
+          tc_ld8(tlane + ra.i * NT + (t0 - th0), u);
+          TcOperands nxt;
+          if (t0 + kTcChunk < the) vtc_fetch<EPI>(P, srow, t0 + kTcChunk, the, nxt);
+          tc_ld_wait();
           float v[kTcChunk];
 #pragma unroll
-          for (int e = 0; e < kTcChunk; e++) v[e] = yw[(t0 + e) * 128];
-          vtc_epilogue<EPI>(P, srow, th0 + t0, the, v, pre, lane);
+          for (int e = 0; e < kTcChunk; e++) v[e] = __uint_as_float(u[e]);
+          vtc_epilogue<EPI>(P, srow, t0, the, v, rf, pre, lane);
+          pre = nxt;
         }
       }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&acc_empty[ra.i]);
     }
   }
   if (split) {
     __syncwarp();
     cluster_arrive();
     cluster_wait();                                              // every rank's sums are in
-    if (warp >= 8 && __all_sync(0xffffffffu, ok && *s_abort == 0)) {
+    if (warp >= 12 && __all_sync(0xffffffffu, ok && *s_abort == 0)) {
       const float* yw = ys + half * (TPR / 2) * 128 + row;
       for (int t0 = 0; e_t0 + t0 < e_tend; t0 += kTcChunk) {
         if (t0) vtc_fetch<EPI>(P, e_srow, e_t0 + t0, e_tend, pre);
@@ -529,7 +694,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) v_gemm_tc(const __grid_constant
           if (t0 + e < TPR / 2)
             for (int r = 0; r < P.nsplit; r++) v[e] += yw[(r * TPR + t0 + e) * 128];
         }
-        vtc_epilogue<EPI>(P, e_srow, e_t0 + t0, e_tend, v, pre, lane);
+        vtc_epilogue<EPI>(P, e_srow, e_t0 + t0, e_tend, v, e_rf, pre, lane);
       }
     }
   }
