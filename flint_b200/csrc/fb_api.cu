@@ -271,7 +271,7 @@ cudaError_t launch_vtc_hz(VtcParams& p, int sms, cudaStream_t st) {
   }
   if (p.K % 128 || p.ntok % 16 || p.ntok > NT || (size_t)p.ntok * p.ntile < (size_t)p.M) return cudaErrorInvalidValue;
   const int items = ((p.rows + kTcRowBlock - 1) / kTcRowBlock) * p.ntile;
-  p.nsplit = p.ntile == 1 ? tc_splits(items, p.K, sms) : 1;
+  p.nsplit = p.ntile == 1 && NT <= 64 ? tc_splits(items, p.K, sms) : 1;
   const int grid = p.nsplit > 1 ? items * p.nsplit : (items < sms ? items : sms);
   return launch_pdl_cluster(v_gemm_tc<NT, EPI, HZ>, dim3(grid), dim3(kTcThreads), (size_t)VtcSmem<NT, HZ>::TOTAL, st,
                             (unsigned)p.nsplit, p);

@@ -377,58 +377,71 @@ struct TcWalk {
   __device__ __forceinline__ void next() { item += step; set(); }
 };
 
-constexpr int kTcChunk = 8;       // tokens whose epilogue operands a thread loads together
-
-// What one chunk of the epilogue reads from global memory (issued early: it does not depend on the GEMM)
-struct TcOperands {
-  float fx[kTcChunk], fa[kTcChunk];
-  uint16_t h[kTcChunk];
-  float2 cs[kTcChunk];
-};
+// Tokens whose accumulators an epilogue thread takes together: 16 where an epilogue reads nothing but factors (more independent
+// exponentials and stores in flight), 8 where every token brings an operand from global memory.
 template <int EPI>
-__device__ __forceinline__ void vtc_fetch(const VtcParams& P, int srow, int t0, int tend, TcOperands& o) {
-#pragma unroll
-  for (int e = 0; e < kTcChunk; e++) {
-    const int t = min(t0 + e, tend - 1);
-    o.fx[e] = __ldcg(P.fx + t);
-    if (EPI == EPI_SWIGLU) o.fa[e] = __ldcg(P.fa + t);
-  }
-  if (EPI == EPI_RESID) {
-#pragma unroll
-    for (int e = 0; e < kTcChunk; e++)
-      o.h[e] = (srow < P.rows && t0 + e < tend) ? ld_cg_u16(P.h + (size_t)(t0 + e) * P.out_ld + srow) : (uint16_t)0;
-  } else if (EPI == EPI_QKV) {
-    const int HP = P.head_dim >> 1, head = srow / P.head_dim, i = (srow % P.head_dim) >> 1;
-    const bool rot = head < P.n_head + P.nkv;
-#pragma unroll
-    for (int e = 0; e < kTcChunk; e++)
-      o.cs[e] = (rot && t0 + e < tend) ? __ldg(P.rope + (size_t)(t0 + e) * HP + i) : make_float2(1.f, 0.f);
-  }
+__host__ __device__ constexpr int tc_chunk(int tokens) {
+  return (EPI == EPI_SWIGLU || EPI == EPI_LOGITS) && tokens % 16 == 0 ? 16 : 8;
 }
-// v[e] = accumulator of (stream row srow, token t0 + e), rf = the row's factor. The whole warp calls this together: lanes
-// 2i, 2i + 1 hold the two rows of a RoPE or gate/up pair.
+// What one chunk of the epilogue reads from global memory (issued early: it does not depend on the GEMM)
+template <int EPI, int CH>
+struct TcOperands {
+  uint16_t h[EPI == EPI_RESID ? CH : 1];
+  float2 cs[EPI == EPI_QKV ? CH : 1];
+  __device__ __forceinline__ void fetch(const VtcParams& P, int srow, int t0, int tend) {
+    if constexpr (EPI == EPI_RESID) {
+#pragma unroll
+      for (int e = 0; e < CH; e++)
+        h[e] = (srow < P.rows && t0 + e < tend) ? ld_cg_u16(P.h + (size_t)(t0 + e) * P.out_ld + srow) : (uint16_t)0;
+    } else if constexpr (EPI == EPI_QKV) {
+      const int HP = P.head_dim >> 1, head = srow / P.head_dim, i = (srow % P.head_dim) >> 1;
+      const bool rot = head < P.n_head + P.nkv;
+#pragma unroll
+      for (int e = 0; e < CH; e++)
+        cs[e] = (rot && t0 + e < tend) ? __ldg(P.rope + (size_t)(t0 + e) * HP + i) : make_float2(1.f, 0.f);
+    }
+  }
+};
+// The token factors of a warp's (up to 64) tokens, spread over its lanes: one load per item instead of an L2 round trip per chunk
 template <int EPI>
-__device__ __forceinline__ void vtc_epilogue(const VtcParams& P, int srow, int t0, int tend, float (&v)[kTcChunk], float rf,
-                                             const TcOperands& o, int lane) {
+struct TcFactors {
+  float fx[2], fa[2];
+  __device__ __forceinline__ void fetch(const VtcParams& P, int t0, int tend, int lane) {
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+      const int t = t0 + 32 * k + lane;
+      fx[k] = t < tend ? __ldcg(P.fx + t) : 0.f;
+      if (EPI == EPI_SWIGLU) fa[k] = t < tend ? __ldcg(P.fa + t) : 0.f;
+    }
+  }
+  __device__ __forceinline__ float x(int i) const { return __shfl_sync(0xffffffffu, i < 32 ? fx[0] : fx[1], i & 31); }
+  __device__ __forceinline__ float a(int i) const { return __shfl_sync(0xffffffffu, i < 32 ? fa[0] : fa[1], i & 31); }
+};
+// v[e] = accumulator of (stream row srow, token t0 + e), the i0 + e-th of the warp's tokens; rf = the row's factor. The whole warp
+// calls this together: lanes 2i, 2i + 1 hold the two rows of a RoPE or gate/up pair.
+template <int EPI, int CH>
+__device__ __forceinline__ void vtc_epilogue(const VtcParams& P, int srow, int t0, int tend, float (&v)[CH], float rf,
+                                             const TcFactors<EPI>& f, int i0, const TcOperands<EPI, CH>& o, int lane) {
   const bool live = srow < P.rows, odd = lane & 1;
 #pragma unroll
-  for (int e = 0; e < kTcChunk; e++) v[e] = v[e] * rf * o.fx[e];
-  if (EPI == EPI_RESID) {
+  for (int e = 0; e < CH; e++) v[e] = v[e] * rf * f.x(i0 + e);
+  if constexpr (EPI == EPI_RESID) {
 #pragma unroll
-    for (int e = 0; e < kTcChunk; e++)
+    for (int e = 0; e < CH; e++)
       if (live && t0 + e < tend) P.h[(size_t)(t0 + e) * P.out_ld + srow] = f2bf(bf2f(o.h[e]) + v[e] * P.resid);
-  } else if (EPI == EPI_LOGITS) {
+  } else if constexpr (EPI == EPI_LOGITS) {
 #pragma unroll
-    for (int e = 0; e < kTcChunk; e++)
+    for (int e = 0; e < CH; e++)
       if (live && t0 + e < tend) P.logits[(size_t)(t0 + e) * P.out_ld + srow] = v[e] / P.logits_scaling;
-  } else if (EPI == EPI_SWIGLU) {
+  } else if constexpr (EPI == EPI_SWIGLU) {
     // stream rows (2i, 2i+1) = (gate_i, up_i): the even lane takes the even tokens of the pair, the odd lane the odd ones
 #pragma unroll
-    for (int e = 0; e < kTcChunk; e += 2) {
+    for (int e = 0; e < CH; e += 2) {
       const float got = __shfl_xor_sync(0xffffffffu, odd ? v[e] : v[e + 1], 1);
       const float gg = rbf(odd ? got : v[e]), uu = rbf(odd ? v[e + 1] : got);
+      const float f0 = f.a(i0 + e), f1 = f.a(i0 + e + 1);
       const int t = t0 + e + (odd ? 1 : 0);
-      const __half a = __float2half_rn(rbf((gg / (1.0f + __expf(-gg))) * uu) * (odd ? o.fa[e + 1] : o.fa[e]));
+      const __half a = __float2half_rn(rbf((gg / (1.0f + __expf(-gg))) * uu) * (odd ? f1 : f0));
       if (live && t < tend) P.act[(size_t)t * P.out_ld + (srow >> 1)] = __half_as_ushort(a);
     }
   } else {
@@ -446,10 +459,10 @@ __device__ __forceinline__ void vtc_epilogue(const VtcParams& P, int srow, int t
       base = (rot ? P.kc : P.vc) + (size_t)P.pos * ld + kvh * HD + (rot ? (within >> 1) + (odd ? HP : 0) : within);
     }
 #pragma unroll
-    for (int e = 0; e < kTcChunk; e++) {
+    for (int e = 0; e < CH; e++) {
       const float x = rbf(v[e]), y = __shfl_xor_sync(0xffffffffu, x, 1);
       const float r = odd ? x * o.cs[e].x + y * o.cs[e].y : x * o.cs[e].x - y * o.cs[e].y;
-      if (live && t0 + e < tend) base[(size_t)(t0 + e) * ld] = f2bf(rot ? r : (v[e]));
+      if (live && t0 + e < tend) base[(size_t)(t0 + e) * ld] = f2bf(rot ? r : v[e]);
     }
   }
 }
@@ -469,8 +482,8 @@ __global__ void __launch_bounds__(kTcThreads, 1) v_gemm_tc(const __grid_constant
   float* ys = reinterpret_cast<float*>(tsm + S::YS);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (tid == 0) {
-    for (int i = 0; i < NRAW; i++) { mbar_init(&raw_full[i], 1); mbar_init(&raw_empty[i], 4); }
-    for (int i = 0; i < NS; i++) mbar_init(&a_full[i], 4);
+    for (int i = 0; i < NRAW; i++) { mbar_init(&raw_full[i], 1); mbar_init(&raw_empty[i], 8); }
+    for (int i = 0; i < NS; i++) mbar_init(&a_full[i], 8);
     for (int i = 0; i < NB; i++) mbar_init(&b_full[i], 1);
     for (int i = 0; i < ND; i++) mbar_init(&done[i], 1);
     for (int i = 0; i < 2; i++) { mbar_init(&acc_full[i], 1); mbar_init(&acc_empty[i], 8); }
@@ -491,11 +504,13 @@ __global__ void __launch_bounds__(kTcThreads, 1) v_gemm_tc(const __grid_constant
   if (split) { cluster_arrive(); cluster_wait(); }               // the neighbours' shared memory exists from here on
   pdl_trigger();
   const int quad = warp & 3, row = quad * 32 + lane;             // warps 4..19: row of the block = TMEM lane
-  const int half = ((warp >> 2) & 1) ^ 1;                        // warps 4..11: which groups; warps 12..19: which half of the tokens
+  const int half = ((warp >> 2) & 1) ^ 1;                        // warps 4..11: half of a group's columns; 12..19: of the tokens
   // splits: this CTA finishes tokens [rank * TPR, (rank + 1) * TPR) of the item
   const int TPR = NT / P.nsplit, lgT = 31 - __clz(TPR), rank = (int)blockIdx.x % P.nsplit;
   bool ok = true;
-  TcOperands pre;
+  constexpr int CH = tc_chunk<EPI>(HC);
+  TcOperands<EPI, CH> pre;
+  TcFactors<EPI> fac;
   int e_srow = 0, e_t0 = 0, e_tend = 0;                          // split items: the epilogue's row and first token
   float e_rf = 0.f;
 
@@ -587,15 +602,15 @@ __global__ void __launch_bounds__(kTcThreads, 1) v_gemm_tc(const __grid_constant
       }
     }
   } else if (warp >= 4 && warp < 12) {
-    // ---------------- dequantise: two sets of four warps take the groups in turn; thread = row of the block = TMEM lane; 16 words
-    // -> 64 packed fp16 pairs per group
-    const uint32_t tl = tmem + ((uint32_t)(quad * 32) << 16);
+    // ---------------- dequantise: thread = (row of the block = TMEM lane, half of the group's columns); 8 words -> 32 packed fp16
+    // pairs per group. (Two warps sharing a group halve the time that a stage is busy; with each warp doing whole groups in turn
+    // the six stages did not cover the round trip to the MMA and back.)
+    const uint32_t tl = tmem + ((uint32_t)(quad * 32) << 16) + half * 32;
     uint32_t gi = 0;
     Ring<NRAW> rr;
     Ring<NS> rs;
     for (TcWalk w(P); w.valid() && ok; w.next()) {
       for (int g = w.g0; g < w.g1; g++, gi++, rr.next(), rs.next()) {
-        if ((int)(gi & 1) != half) continue;
         uint64_t* freed = &done[(gi - NS) % ND];                 // the stage's previous group has retired
         const uint32_t fpar = ((gi - NS) / ND) & 1;
         bool now = mbar_try(&raw_full[rr.i], rr.lap);
@@ -605,20 +620,17 @@ __global__ void __launch_bounds__(kTcThreads, 1) v_gemm_tc(const __grid_constant
         if (!ok) break;
         tc_fence_after();
         const uint8_t* rec = tsm + S::RAW + rr.i * REC;
-        const uint32_t raw = smem_u32(rec) + (uint32_t)row * 4;
+        const uint32_t raw = smem_u32(rec) + (uint32_t)row * 4 + half * 4096;
         const __half2 sc = __half2half2(reinterpret_cast<const __half*>(rec + 8192)[row]);
+        uint32_t v[32];
 #pragma unroll
-        for (int c = 0; c < 2; c++) {
-          uint32_t v[32];
-#pragma unroll
-          for (int q8 = 0; q8 < 8; q8++) {
-            const uint32_t wv = lds32(raw + c * 4096 + q8 * 512);
-            v[4 * q8] = tc_cvt_lo(wv, sc); v[4 * q8 + 1] = tc_cvt_hi(wv, sc);
-            v[4 * q8 + 2] = tc_cvt_lo(wv >> 8, sc); v[4 * q8 + 3] = tc_cvt_hi(wv >> 8, sc);
-          }
-          tc_st32(tl + S::T_A + rs.i * 64 + c * 32, v);
+        for (int q8 = 0; q8 < 8; q8++) {
+          const uint32_t wv = lds32(raw + q8 * 512);
+          v[4 * q8] = tc_cvt_lo(wv, sc); v[4 * q8 + 1] = tc_cvt_hi(wv, sc);
+          v[4 * q8 + 2] = tc_cvt_lo(wv >> 8, sc); v[4 * q8 + 3] = tc_cvt_hi(wv >> 8, sc);
         }
-        if (HZ) {
+        tc_st32(tl + S::T_A + rs.i * 64, v);
+        if (HZ && half == 0) {
           // the group's zero point of this row as one k16 step: A_z = z for every column
           const uint16_t z = reinterpret_cast<const uint16_t*>(rec + 8448)[row];
           tc_st8(tl + S::T_AZ + rs.i * 8, (uint32_t)z | ((uint32_t)z << 16));
@@ -641,7 +653,8 @@ __global__ void __launch_bounds__(kTcThreads, 1) v_gemm_tc(const __grid_constant
       const int th0 = split ? rank * TPR + half * (TPR / 2) : tok0 + half * HC;
       const int the = min(tend, th0 + (split ? TPR / 2 : HC));
       if (split) { e_srow = srow; e_t0 = th0; e_tend = the; e_rf = rf; }
-      if (th0 < the) vtc_fetch<EPI>(P, srow, th0, the, pre);
+      pre.fetch(P, srow, th0, the);
+      fac.fetch(P, th0, the, lane);
       ok = __all_sync(0xffffffffu, mbar_wait(&acc_full[ra.i], ra.lap, wc, W_FULL, 10));
       if (!ok) break;
       tc_fence_after();
@@ -661,16 +674,17 @@ __global__ void __launch_bounds__(kTcThreads, 1) v_gemm_tc(const __grid_constant
         }
       } else {
 #pragma unroll 1
-        for (int t0 = th0; t0 < the; t0 += kTcChunk) {
-          uint32_t u[8];
-          tc_ld8(tlane + ra.i * NT + (t0 - th0), u);
-          TcOperands nxt;
-          if (t0 + kTcChunk < the) vtc_fetch<EPI>(P, srow, t0 + kTcChunk, the, nxt);
-          tc_ld_wait();
-          float v[kTcChunk];
+        for (int t0 = th0; t0 < the; t0 += CH) {
+          uint32_t u[CH / 8][8];
 #pragma unroll
-          for (int e = 0; e < kTcChunk; e++) v[e] = __uint_as_float(u[e]);
-          vtc_epilogue<EPI>(P, srow, t0, the, v, rf, pre, lane);
+          for (int c8 = 0; c8 < CH / 8; c8++) tc_ld8(tlane + ra.i * NT + (t0 - th0) + c8 * 8, u[c8]);
+          TcOperands<EPI, CH> nxt;
+          nxt.fetch(P, srow, t0 + CH, the);
+          tc_ld_wait();
+          float v[CH];
+#pragma unroll
+          for (int e = 0; e < CH; e++) v[e] = __uint_as_float(u[e >> 3][e & 7]);
+          vtc_epilogue<EPI, CH>(P, srow, t0, the, v, rf, fac, t0 - th0, pre, lane);
           pre = nxt;
         }
       }
@@ -685,16 +699,16 @@ __global__ void __launch_bounds__(kTcThreads, 1) v_gemm_tc(const __grid_constant
     cluster_wait();                                              // every rank's sums are in
     if (warp >= 12 && __all_sync(0xffffffffu, ok && *s_abort == 0)) {
       const float* yw = ys + half * (TPR / 2) * 128 + row;
-      for (int t0 = 0; e_t0 + t0 < e_tend; t0 += kTcChunk) {
-        if (t0) vtc_fetch<EPI>(P, e_srow, e_t0 + t0, e_tend, pre);
-        float v[kTcChunk];
+      for (int t0 = 0; e_t0 + t0 < e_tend; t0 += CH) {
+        if (t0) pre.fetch(P, e_srow, e_t0 + t0, e_tend);
+        float v[CH];
 #pragma unroll
-        for (int e = 0; e < kTcChunk; e++) {
+        for (int e = 0; e < CH; e++) {
           v[e] = 0.f;
           if (t0 + e < TPR / 2)
             for (int r = 0; r < P.nsplit; r++) v[e] += yw[(r * TPR + t0 + e) * 128];
         }
-        vtc_epilogue<EPI>(P, e_srow, e_t0 + t0, e_tend, v, e_rf, pre, lane);
+        vtc_epilogue<EPI, CH>(P, e_srow, e_t0 + t0, e_tend, v, e_rf, fac, t0, pre, lane);
       }
     }
   }
