@@ -1,6 +1,7 @@
 // The context object behind the C ABI's opaque `fb_ctx`, shared by the translation units of the library.
 #pragma once
 #include <cuda.h>
+#include <cuda_runtime.h>
 #include <stdint.h>
 
 #include "../../include/flint_b200.h"
@@ -46,3 +47,46 @@ struct fb_ctx {
   bool kv_maps;
   int long_kv;                                                      // 0: long-cache decode variant by cached length, 1: always (where built), 2: never
 };
+
+inline int cuda_fail(fb_ctx* c, cudaError_t e) {
+  if (c) c->last_cuda_error = (int)e;
+  return FB_ERR_CUDA;
+}
+
+#define FB_CUDA(c, call)                                   \
+  do {                                                     \
+    cudaError_t e__ = (call);                              \
+    if (e__ != cudaSuccess) return cuda_fail((c), e__);    \
+  } while (0)
+
+template <class T>
+inline cudaError_t dmalloc(T** p, size_t n) { return cudaMalloc(reinterpret_cast<void**>(p), n); }
+
+struct DeviceGuard {
+  int prev;
+  bool ok;
+  explicit DeviceGuard(int dev) : prev(0), ok(false) {
+    if (cudaGetDevice(&prev) == cudaSuccess && cudaSetDevice(dev) == cudaSuccess) ok = true;
+  }
+  ~DeviceGuard() { if (ok) cudaSetDevice(prev); }
+};
+
+typedef CUresult (*EncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
+                             const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
+                             CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+inline EncodeFn tensor_map_encoder() {
+  void* fn = nullptr;
+  cudaDriverEntryPointQueryResult qres;
+  if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &qres) != cudaSuccess ||
+      qres != cudaDriverEntryPointSuccess)
+    return nullptr;
+  return (EncodeFn)fn;
+}
+
+// ---- the verify / prompt passes (fb_pass.cu)
+constexpr int kPromptRows = 1024;  // token rows of the activation buffers: a prompt goes through the layers in chunks of at most this
+cudaError_t pass_alloc(fb_ctx* c);
+void pass_free(fb_ctx* c);
+// one stacked weight matrix in the layouts the passes read (order / arg / orows as in fb_repack)
+cudaError_t pass_bind_matrix(fb_ctx* c, int which, const void* q, const void* s, const void* z, int layers, int rows, int k, int order,
+                             int arg, int orows, cudaStream_t st);

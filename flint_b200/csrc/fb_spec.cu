@@ -25,18 +25,6 @@ namespace {
 
 constexpr int kMaxHeadRows = 16;
 
-template <class T>
-cudaError_t dmalloc(T** p, size_t n) { return cudaMalloc(reinterpret_cast<void**>(p), n); }
-
-struct DeviceGuard {
-  int prev;
-  bool ok;
-  explicit DeviceGuard(int dev) : prev(0), ok(false) {
-    if (cudaGetDevice(&prev) == cudaSuccess && cudaSetDevice(dev) == cudaSuccess) ok = true;
-  }
-  ~DeviceGuard() { if (ok) cudaSetDevice(prev); }
-};
-
 template <int TT, int MODE>
 cudaError_t launch_linear_tt(const DLin& p, int t0, int sms, cudaStream_t st) {
   static bool configured[64] = {};
