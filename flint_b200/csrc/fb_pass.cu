@@ -7,6 +7,7 @@
 #include "fb_verify.cuh"
 #include "fb_vsub.cuh"
 #include "fb_vtc.cuh"
+#include "fb_vattn.cuh"
 
 using namespace fb;
 
@@ -129,6 +130,7 @@ cudaError_t launch_vtc_hz(VtcParams& p, int sms, cudaStream_t st) {
     if (e != cudaSuccess) return e;
     configured[dev] = true;
   }
+  if (p.xbf && (p.rows + kTcRowBlock - 1) / kTcRowBlock > sms) return cudaErrorInvalidValue;
   if (p.K % 128 || p.ntok % 16 || p.ntok > NT || (size_t)p.ntok * p.ntile < (size_t)p.M) return cudaErrorInvalidValue;
   const int items = ((p.rows + kTcRowBlock - 1) / kTcRowBlock) * p.ntile;
   p.nsplit = p.ntile == 1 && NT <= 64 ? tc_splits(items, p.K, sms) : 1;
@@ -162,7 +164,7 @@ cudaError_t launch_vnorm(const uint16_t* h, const uint16_t* w, uint16_t* xn_t, u
 constexpr int kVSpans = 32;       // most spans of positions a kv head's attention is cut into
 
 cudaError_t launch_vattn(const fb_ctx* c, const uint16_t* q, const uint16_t* kc, const uint16_t* vc, const uint8_t* amask,
-                         uint16_t* ao, int pos, int M, bool f16, cudaStream_t st) {
+                         uint16_t* ao, int pos, int M, cudaStream_t st) {
   const fb_model_desc& d = c->d;
   const int T = pos + M;
   // a CTA takes 64 query rows (four 16-row tiles); spans of positions are sized so that about two CTAs per SM exist
@@ -175,16 +177,13 @@ cudaError_t launch_vattn(const fb_ctx* c, const uint16_t* q, const uint16_t* kc,
   if (S > smax) S = smax;
   const int span = ((T + S - 1) / S + 63) / 64 * 64;
   S = (T + span - 1) / span;
-  uint16_t* direct = S == 1 && f16 ? ao : nullptr;         // one span: the CTAs write their rows, v_row_f16 converts them
-  unsigned* amax = f16 && !direct ? c->vamax : nullptr;
 #define FB_VATTN(HD_, R_)                                                                                               \
   if (d.head_dim == HD_ && c->rgqa == R_) {                                                                             \
     cudaError_t e = launch_pdl(v_attn_mma<HD_, R_>, dim3(d.n_kv_head, S, mgroups), dim3(128), 0, st, q, kc, vc, amask, c->vpart,  \
-                               direct, amax, d.n_head, d.n_kv_head, pos, M, d.attn_scale, span);                                      \
+                               d.n_head, d.n_kv_head, pos, M, d.attn_scale, span);                                      \
     if (e != cudaSuccess) return e;                                                                                     \
-    if (direct) return launch_pdl(v_row_f16, dim3(M), dim3(256), 0, st, ao, c->vfao, d.n_head * HD_);                    \
     return launch_pdl(v_attn_merge<HD_, R_>, dim3(M, d.n_kv_head), dim3(256), 0, st, (const float*)c->vpart, ao, d.n_head, \
-                      d.n_kv_head, M, S, (const unsigned*)amax, c->vfao);                                                                      \
+                      d.n_kv_head, M, S);                                                                      \
   }
   FB_VATTN(64, 4) FB_VATTN(80, 4) FB_VATTN(64, 5) FB_VATTN(128, 4)
 #undef FB_VATTN
@@ -208,6 +207,48 @@ bool make_act_maps(fb_ctx* c) {
         return false;
     }
   return true;
+}
+
+template <int HD, int R, int UP, bool DIRECT>
+cudaError_t launch_vattn_hd(const VattnParams& a, dim3 grid, cudaStream_t st) {
+  static bool configured[64] = {};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
+  auto k = v_attn<HD, R, UP, DIRECT>;
+  if (!configured[dev]) {
+    FB_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, VaSmem<HD>::TOTAL));
+    FB_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    configured[dev] = true;
+  }
+  return launch_pdl_cluster(k, grid, dim3(256), (size_t)VaSmem<HD>::TOTAL, st, grid.x, a);
+}
+// Geometry: enough query rows (prompts) -> 128 rows a CTA, no spans. Otherwise up to four row tiles a CTA and as many spans (a power of
+// two, at most 8; 16 where a long cache meets few rows) as there are 64-position stages.
+cudaError_t launch_vattn_tc(const fb_ctx* c, const uint16_t* kc, const uint16_t* vc, const uint8_t* amask, int pos, int M, bool want_max,
+                            cudaStream_t st) {
+  const fb_model_desc& d = c->d;
+  const int T = pos + M, tiles = (M * c->rgqa + 15) / 16;
+  VattnParams a{c->vq, kc, vc, amask, c->vao, want_max ? c->vamax : nullptr, d.n_head, d.n_kv_head, pos, M, 8, 0, d.attn_scale};
+  const bool direct = !want_max && d.n_kv_head * ((tiles + 7) / 8) >= c->sm_count * 2 / 3;
+  int nspan = 1, mg;
+  if (direct) {
+    mg = (tiles + 7) / 8;
+    a.span = T;
+  } else {
+    a.rt = tiles >= 3 ? 4 : (tiles == 2 ? 2 : 1);
+    mg = (tiles + a.rt - 1) / a.rt;
+    const int stages = (T + kVaPos - 1) / kVaPos, room = 2 * c->sm_count / (d.n_kv_head * mg);
+    const int most = stages > 32 && d.n_kv_head * mg * 16 <= c->sm_count ? 16 : 8;
+    while (nspan < most && nspan * 2 <= stages && nspan * 2 <= room && nspan * 2 <= a.rt * 16) nspan *= 2;
+    a.span = (stages + nspan - 1) / nspan * kVaPos;
+  }
+  const dim3 grid(nspan, d.n_kv_head, mg);
+#define FB_VATTN2(HD_, R_)                                                                                   \
+  if (d.head_dim == HD_ && c->rgqa == R_)                                                                    \
+    return direct ? launch_vattn_hd<HD_, R_, 32, true>(a, grid, st) : launch_vattn_hd<HD_, R_, 16, false>(a, grid, st);
+  FB_VATTN2(64, 4) FB_VATTN2(80, 4) FB_VATTN2(64, 5) FB_VATTN2(128, 4)
+#undef FB_VATTN2
+  return cudaErrorInvalidValue;
 }
 
 // One pass of M tokens (1 .. kPromptRows) through the model on the tcgen05 GEMMs: natural-order activations, the matrices in the
@@ -244,9 +285,14 @@ int run_tc_pass(fb_ctx* c, const int32_t* d_tokens, const void* d_h, const int32
     FB_CUDA(c, norm((const uint16_t*)c->n1 + (size_t)l * D, nullptr, nullptr));
     t.w = c->t_qkv + l * tQ; t.rows = QKV; t.K = D; t.kc = kcl; t.vc = vcl; t.fx = c->vfx;
     FB_CUDA(c, launch_vtc<EPI_QKV>(t, c->m_xn, nt, hz, sms, st));
-    FB_CUDA(c, launch_vattn(c, c->vq, kcl, vcl, d_amask, c->vao, pos, M, true, st));
+    // trees: the O GEMM converts the attention output to fp16 on its way in; prompts, whose activations come by tensor copies, have it
+    // converted in place
+    FB_CUDA(c, launch_vattn_tc(c, kcl, vcl, d_amask, pos, M, nt <= 64, st));
+    if (nt > 64) FB_CUDA(c, launch_pdl(v_row_f16, dim3(M), dim3(256), 0, st, c->vao, c->vfao, QD));
     t.w = c->t_o + l * tO; t.rows = D; t.K = QD; t.out_ld = D; t.fx = c->vfao;
+    t.xbf = nt <= 64 ? c->vao : nullptr; t.amax = nt <= 64 ? c->vamax : nullptr;
     FB_CUDA(c, launch_vtc<EPI_RESID>(t, c->m_ao, nt, hz, sms, st));
+    t.xbf = nullptr; t.amax = nullptr;
     FB_CUDA(c, norm((const uint16_t*)c->n2 + (size_t)l * D, nullptr, c->gu_norms + 2 * l));
     t.w = c->t_gu + l * tG; t.rows = 2 * FF; t.K = D; t.out_ld = FF; t.fx = c->vfx;
     FB_CUDA(c, launch_vtc<EPI_SWIGLU>(t, c->m_xn, nt, hz, sms, st));
@@ -410,7 +456,7 @@ int fb_verify(fb_ctx* c, const int32_t* d_tokens, const void* d_h, const int32_t
       p.q = c->vq; p.kc = kcl; p.vc = vcl;
       FB_CUDA(c, launch_vgemm_mt<EPI_QKV>(p, MT, D, HD, c->sm_count, st));
     }
-    FB_CUDA(c, launch_vattn(c, c->vq, kcl, vcl, d_amask, c->vao, pos, M, false, st));
+    FB_CUDA(c, launch_vattn(c, c->vq, kcl, vcl, d_amask, c->vao, pos, M, st));
     if (sub(c->s_o, l, D, QD)) {
       sp.x = c->vao; sp.h = c->vh; sp.out_ld = D;
       FB_CUDA(c, launch_vsub<EPI_RESID>(sp, c->sm_count, st));

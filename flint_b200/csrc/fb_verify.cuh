@@ -112,14 +112,11 @@ __global__ void __launch_bounds__(256) v_rmsnorm(const uint16_t* h, const uint16
 // positions at a time the N dimension of Q K^T and the K dimension of P V. Query m sees every cached position
 // t < pos and, among the M new slots pos..pos+M-1, those with amask[m][t - pos] != 0. Probabilities enter P V as a
 // sum of two bf16 values (p = hi + lo), which keeps their fp32 precision to ~2^-17. Every span writes, per query row,
-// an un-normalised partial (acc[HD], running max, denominator); v_attn_merge combines the spans. With one span (ao set: long
-// prompts have enough query rows to fill the GPU) the CTA normalises and writes its rows itself, natural order. amask == nullptr is the causal
-// chain (amask[m][j] = j <= m): no CTA looks past its last token. amax (or nullptr): per token, a bound on the magnitudes of the
-// merged output as float bits -- the largest |acc| / denominator of any span (the merge is a convex combination of those).
+// an un-normalised partial (acc[HD], running max, denominator); v_attn_merge combines the spans.
 template <int HD, int R>
 __global__ void __launch_bounds__(128) v_attn_mma(const uint16_t* q, const uint16_t* kc, const uint16_t* vc,
-                                                  const uint8_t* amask, float* part, uint16_t* ao, unsigned* amax,
-                                                  int n_head, int nkv, int pos, int M, float scale, int span) {
+                                                  const uint8_t* amask, float* part, int n_head, int nkv, int pos, int M,
+                                                  float scale, int span) {
   constexpr int CH = 64, KSTEPS = HD / 16, NTD = HD / 8, STR = HD * 2 + 16, PW = HD + 2;
   static_assert(HD % 16 == 0 && NTD % 2 == 0, "head_dim must be a multiple of 16");
   __shared__ __align__(16) uint8_t k_s[CH * STR];
@@ -129,8 +126,7 @@ __global__ void __launch_bounds__(128) v_attn_mma(const uint16_t* q, const uint1
   const int T = pos + M, QD = n_head * HD, rows = M * R;
   pdl_trigger();
   pdl_wait();
-  const int m_last = min(M - 1, ((int)blockIdx.z * 64 + 63) / R);      // the CTA's last token
-  const int t_begin = sp * span, t_end = min(amask ? T : pos + m_last + 1, t_begin + span);
+  const int t_begin = sp * span, t_end = min(T, t_begin + span);
   const int ntile = (rows + 15) / 16;
   {
     const int mt = (int)blockIdx.z * 4 + warp;
@@ -187,10 +183,7 @@ __global__ void __launch_bounds__(128) v_attn_mma(const uint16_t* q, const uint1
         for (int e = 0; e < 4; e++) {
           const int tp = c0 + nt * 8 + 2 * t + (e & 1);
           bool ok = tp < T;
-          if (tree && ok && tp >= pos) {
-            const int mq = e < 2 ? m_lo : m_hi;
-            ok = amask ? amask[mq * M + (tp - pos)] != 0 : tp - pos <= mq;
-          }
+          if (tree && ok && tp >= pos) ok = amask[(e < 2 ? m_lo : m_hi) * M + (tp - pos)] != 0;
           const float v = ok ? s[nt][e] * scale : -INFINITY;
           s[nt][e] = v;
           mx[e >> 1] = fmaxf(mx[e >> 1], v);
@@ -244,26 +237,7 @@ __global__ void __launch_bounds__(128) v_attn_mma(const uint16_t* q, const uint1
         lrun[h] += __shfl_xor_sync(0xffffffffu, lrun[h], 1);
         lrun[h] += __shfl_xor_sync(0xffffffffu, lrun[h], 2);
         const int row = mt * 16 + g + 8 * h;
-        if (amax) {
-          float bm = 0.f;
-#pragma unroll
-          for (int j = 0; j < NTD; j++) bm = fmaxf(bm, fmaxf(fabsf(o[j][2 * h]), fabsf(o[j][2 * h + 1])));
-          bm = fmaxf(bm, __shfl_xor_sync(0xffffffffu, bm, 1));
-          bm = fmaxf(bm, __shfl_xor_sync(0xffffffffu, bm, 2));
-          bm = row < rows && lrun[h] > 0.f ? bm / lrun[h] : 0.f;
-          if (R == 4) {                                   // four consecutive rows are the heads of one token
-            bm = fmaxf(bm, __shfl_xor_sync(0xffffffffu, bm, 4));
-            bm = fmaxf(bm, __shfl_xor_sync(0xffffffffu, bm, 8));
-          }
-          if (row < rows && t == 0 && (R != 4 || (g & 3) == 0)) atomicMax(amax + row / R, __float_as_uint(bm));
-        }
-        if (row < rows && ao) {
-          const float inv = 1.0f / lrun[h];
-          uint16_t* dst = ao + (size_t)(row / R) * QD + (size_t)(kvh * R + row % R) * HD;
-#pragma unroll
-          for (int j = 0; j < NTD; j++)
-            *reinterpret_cast<uint32_t*>(dst + j * 8 + 2 * t) = pack_bf16(o[j][2 * h] * inv, o[j][2 * h + 1] * inv);
-        } else if (row < rows) {
+        if (row < rows) {
           float* pr = part + ((size_t)(kvh * S + sp) * rows + row) * PW;
 #pragma unroll
           for (int j = 0; j < NTD; j++)
@@ -275,17 +249,13 @@ __global__ void __launch_bounds__(128) v_attn_mma(const uint16_t* q, const uint1
   }
 }
 
-// one CTA per (token, kv head): combine the spans' partials, write bf16 in B order or, with the tokens' bounds amax, fp16 in natural
-// order times the token's power of two, whose inverse goes to fx (S <= 32 spans)
+// one CTA per (token, kv head): combine the spans' partials, write bf16 in B order (S <= 32 spans)
 template <int HD, int R>
-__global__ void __launch_bounds__(256) v_attn_merge(const float* part, uint16_t* ao_t, int n_head, int nkv, int M, int S,
-                                                    const unsigned* amax, float* fx) {
+__global__ void __launch_bounds__(256) v_attn_merge(const float* part, uint16_t* ao_t, int n_head, int nkv, int M, int S) {
   constexpr int PW = HD + 2, MAXS = 32;
   const int m = blockIdx.x, kvh = blockIdx.y, rows = M * R, QD = n_head * HD;
   pdl_trigger();
   pdl_wait();
-  const float2 f = amax ? pow2_for(__uint_as_float(__ldcg(amax + m))) : make_float2(1.f, 1.f);
-  if (amax && kvh == 0 && threadIdx.x == 0) fx[m] = f.y;
   for (int o = threadIdx.x; o < R * HD; o += blockDim.x) {
     const int r = o / HD, d = o % HD, row = m * R + r;
     const float* p0 = part + ((size_t)kvh * S * rows + row) * PW;
@@ -308,8 +278,7 @@ __global__ void __launch_bounds__(256) v_attn_merge(const float* part, uint16_t*
       A = fmaf(pa[s2], e, A);
     }
     const int col = (kvh * R + r) * HD + d;
-    if (amax) ao_t[(size_t)m * QD + col] = __half_as_ushort(__float2half_rn(rbf(A / Dn) * f.x));
-    else ao_t[(size_t)m * QD + k16_pos(col)] = f2bf(A / Dn);
+    ao_t[(size_t)m * QD + k16_pos(col)] = f2bf(A / Dn);
   }
 }
 

@@ -37,10 +37,11 @@ namespace fb {
 
 constexpr int kTcThreads = 640;   // warps: 0 weights, 1 MMA issue, 2 activations, 4..11 dequantise, 12..19 epilogue
 constexpr int kTcRowBlock = 128;
+constexpr int kTcTrailer = kTcRowBlock * 4 + 16;      // a block's row factors, then its flag
 
 __host__ __device__ constexpr int tc_rec_bytes(int has_zeros) { return 8192 + 256 * (has_zeros ? 2 : 1); }
 __host__ __device__ constexpr size_t tc_block_bytes(int k, int has_zeros) {
-  return (size_t)(k / 128) * tc_rec_bytes(has_zeros) + kTcRowBlock * 4;
+  return (size_t)(k / 128) * tc_rec_bytes(has_zeros) + kTcTrailer;
 }
 __host__ __device__ constexpr size_t tc_matrix_bytes(int rows, int k, int has_zeros) {
   return (size_t)((rows + kTcRowBlock - 1) / kTcRowBlock) * tc_block_bytes(k, has_zeros);
@@ -60,18 +61,27 @@ __global__ void __launch_bounds__(256) tc_repack(const uint32_t* q, const uint16
   const int rb = blockIdx.x, nrb = gridDim.x, G = K / 128, nw = K / 8, rec = tc_rec_bytes(hz), r = threadIdx.x & 127,
             part = threadIdx.x >> 7;                            // two threads per row
   uint8_t* blk = out + ((size_t)blockIdx.y * nrb + rb) * tc_block_bytes(K, hz);
-  __shared__ float s_max[256], s_sq[256];
+  __shared__ float s_max[256], s_min[256], s_sq[256];
   const int j = rb * 128 + r;
   const int row = j < rows ? (int)blockIdx.y * rows + perm_row(j, order, order_arg, order_rows) : -1;
-  float mx = 0.f;
+  float mx = 0.f, mn = INFINITY;
   if (row >= 0)
     for (int g = part; g < G; g += 2) {
-      mx = fmaxf(mx, 8.0f * fabsf(bf2f(sc[(size_t)row * G + g])));
+      const float a = fabsf(bf2f(sc[(size_t)row * G + g]));
+      mx = fmaxf(mx, 8.0f * a);
+      if (a > 0.f) mn = fminf(mn, a);
       if (hz) mx = fmaxf(mx, fabsf(bf2f(zr[(size_t)row * G + g])));
     }
   s_max[threadIdx.x] = mx;
+  s_min[threadIdx.x] = mn;
   __syncthreads();
-  const float2 f = pow2_for(fmaxf(s_max[r], s_max[r + 128]));
+  const float rmax = fmaxf(s_max[r], s_max[r + 128]);
+  float2 f = rmax > 0.f ? pow2_for(rmax) : make_float2(1.f, 1.f);      // 8 s in [2^14, 2^15)
+  // the block's scales are stored for the one-fma conversion (S = 16 s 2^er, then in [2^15, 2^16), and 2^24 in the factor) when that
+  // is exact in every row: no scale of a row below S = 128
+  const bool fits = fminf(s_min[r], s_min[r + 128]) * f.x * 16.0f >= 128.0f;
+  const bool fast = __syncthreads_and(!hz && fits && f.x < 1e30f && f.y < 1e25f);
+  if (fast) f = make_float2(f.x * 16.0f, f.y * (16777216.0f / 16.0f));
   float sq = 0.f;
   for (int wq = part; wq < nw; wq += 2) {                      // word wq of the row
     const int g = wq >> 4;
@@ -98,6 +108,7 @@ __global__ void __launch_bounds__(256) tc_repack(const uint32_t* q, const uint16
     if (hz) meta[128 + r] = __float2half_rn(row >= 0 ? bf2f(zr[(size_t)row * G + g]) * f.x : 0.f);
   }
   if (part == 0) reinterpret_cast<float*>(blk + (size_t)G * rec)[r] = f.y;
+  if (threadIdx.x < 4) reinterpret_cast<int*>(blk + (size_t)G * rec)[kTcRowBlock + threadIdx.x] = fast;
   if (norms) {
     s_sq[threadIdx.x] = sq;
     __syncthreads();
@@ -241,13 +252,15 @@ struct alignas(64) VtcParams {
   int ntok, ntile;           // tokens of one tile (a multiple of 16, <= NT; one tile unless this is a prompt) and tiles
   DevStatus* status;
   unsigned spin_limit;
-  const float* fx;           // [M, padded to 8] inverse of the power of two in each token's activations
+  const float* fx;           // [M] inverse of the power of two in each token's activations
+  const uint16_t* xbf;       // O of a tree: the attention output as bf16 [M][K]; this kernel converts it on the way in (xmap unused),
+  const unsigned* amax;      // with the power of two of the token's largest magnitude (float bits), fx unused. One item per CTA.
   // epilogue operands
   uint16_t* h;               // RESID: bf16 [M][out_ld] in/out
   uint16_t* q;               // QKV: bf16 [M][n_head * HD]
   uint16_t *kc, *vc;         // QKV: layer base of the caches [max_seq][nkv][HD]
   uint16_t* act;             // SWIGLU: fp16 [M][out_ld], times the token's fa
-  const float* fa;           // SWIGLU: [M, padded to 8]
+  const float* fa;           // SWIGLU: [M]
   float* logits;             // LOGITS: f32 [M][out_ld]
   const float2* rope;        // QKV: [M][HD / 2] (cos, sin)
   int n_head, nkv, pos, out_ld, head_dim;
@@ -269,6 +282,10 @@ __device__ __forceinline__ uint32_t tc_cvt_lo(uint32_t w, __half2 s) {
 __device__ __forceinline__ uint32_t tc_cvt_hi(uint32_t w, __half2 s) {
   return tc_h2(__hmul2(__hfma2(tc_as_h2((w & 0x00F000F0u) | 0x64006400u), tc_as_h2(0x2C002C00u), tc_as_h2(0xD480D480u)), s));
 }
+// The same in one fma, for row blocks whose scales are not more than 2^8 apart in any row (the trailer's flag): the masked bits are
+// the fp16 subnormals nib * 2^-24 (16 nib * 2^-24); times S = s * 2^24 * 2^er (or S / 16) minus 8 S 2^-24 is exact as long as the
+// result's last bit, that of s, is not below 2^-24
+__device__ __forceinline__ uint32_t tc_cvt_fast(uint32_t bits, __half2 s, __half2 c) { return tc_h2(__hfma2(tc_as_h2(bits), s, c)); }
 // shared-memory matrix descriptor: K-major, 128-byte swizzle, 8-row groups 1024 bytes apart
 __device__ __forceinline__ uint64_t tc_desc(uint32_t saddr) {
   return (uint64_t)((saddr & 0x3FFFFu) >> 4) | ((uint64_t)1 << 16) | ((uint64_t)(1024 >> 4) << 32) | ((uint64_t)1 << 46) |
@@ -410,7 +427,7 @@ struct TcFactors {
 #pragma unroll
     for (int k = 0; k < 2; k++) {
       const int t = t0 + 32 * k + lane;
-      fx[k] = t < tend ? __ldcg(P.fx + t) : 0.f;
+      fx[k] = t >= tend ? 0.f : (EPI == EPI_RESID && P.amax) ? pow2_for(__uint_as_float(__ldcg(P.amax + t))).y : __ldcg(P.fx + t);
       if (EPI == EPI_SWIGLU) fa[k] = t < tend ? __ldcg(P.fa + t) : 0.f;
     }
   }
@@ -577,7 +594,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) v_gemm_tc(const __grid_constant
     // ---------------- activations (the previous kernel's output): two tensor copies per group. Token rows past M are whatever
     // the buffer holds: they only feed accumulator columns that nobody reads.
     pdl_wait();
-    if (lane == 0) {
+    if (lane == 0 && !(EPI == EPI_RESID && P.xbf)) {
       uint32_t gi = 0;
       Ring<NB> r;
       for (TcWalk w(P); w.valid() && ok; w.next()) {
@@ -610,6 +627,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) v_gemm_tc(const __grid_constant
     Ring<NRAW> rr;
     Ring<NS> rs;
     for (TcWalk w(P); w.valid() && ok; w.next()) {
+      const bool fast = !HZ && __ldg(reinterpret_cast<const int*>(P.w + (size_t)(w.rb + 1) * tc_block_bytes(P.K, HZ)) - 4) != 0;
       for (int g = w.g0; g < w.g1; g++, gi++, rr.next(), rs.next()) {
         uint64_t* freed = &done[(gi - NS) % ND];                 // the stage's previous group has retired
         const uint32_t fpar = ((gi - NS) / ND) & 1;
@@ -623,11 +641,21 @@ __global__ void __launch_bounds__(kTcThreads, 1) v_gemm_tc(const __grid_constant
         const uint32_t raw = smem_u32(rec) + (uint32_t)row * 4 + half * 4096;
         const __half2 sc = __half2half2(reinterpret_cast<const __half*>(rec + 8192)[row]);
         uint32_t v[32];
+        if (!HZ && fast) {
+          const __half2 sh = __hmul2(sc, tc_as_h2(0x2C002C00u)), off = __hmul2(sc, tc_as_h2(0x80088008u));      // S / 16, -8 S 2^-24
 #pragma unroll
-        for (int q8 = 0; q8 < 8; q8++) {
-          const uint32_t wv = lds32(raw + q8 * 512);
-          v[4 * q8] = tc_cvt_lo(wv, sc); v[4 * q8 + 1] = tc_cvt_hi(wv, sc);
-          v[4 * q8 + 2] = tc_cvt_lo(wv >> 8, sc); v[4 * q8 + 3] = tc_cvt_hi(wv >> 8, sc);
+          for (int q8 = 0; q8 < 8; q8++) {
+            const uint32_t wv = lds32(raw + q8 * 512), wh = wv >> 8;
+            v[4 * q8] = tc_cvt_fast(wv & 0x000F000Fu, sc, off); v[4 * q8 + 1] = tc_cvt_fast(wv & 0x00F000F0u, sh, off);
+            v[4 * q8 + 2] = tc_cvt_fast(wh & 0x000F000Fu, sc, off); v[4 * q8 + 3] = tc_cvt_fast(wh & 0x00F000F0u, sh, off);
+          }
+        } else {
+#pragma unroll
+          for (int q8 = 0; q8 < 8; q8++) {
+            const uint32_t wv = lds32(raw + q8 * 512);
+            v[4 * q8] = tc_cvt_lo(wv, sc); v[4 * q8 + 1] = tc_cvt_hi(wv, sc);
+            v[4 * q8 + 2] = tc_cvt_lo(wv >> 8, sc); v[4 * q8 + 3] = tc_cvt_hi(wv >> 8, sc);
+          }
         }
         tc_st32(tl + S::T_A + rs.i * 64, v);
         if (HZ && half == 0) {
@@ -646,10 +674,46 @@ __global__ void __launch_bounds__(kTcThreads, 1) v_gemm_tc(const __grid_constant
     const uint32_t tlane = tmem + ((uint32_t)(quad * 32) << 16) + half * HC;
     Ring<2> ra;
     pdl_wait();
+    if constexpr (EPI == EPI_RESID && NT <= 64) {
+      if (P.xbf) {
+        // these warps are idle until the sums are there: each brings every eighth group of the attention output, bf16 -> fp16 times
+        // the token's power of two, into the swizzled activation stages
+        float fm[2];
+#pragma unroll
+        for (int k = 0; k < 2; k++) fm[k] = 32 * k + lane < P.M ? pow2_for(__uint_as_float(__ldcg(P.amax + 32 * k + lane))).x : 0.f;
+        const TcWalk w(P);
+        const int c16 = lane & 15, ng = w.valid() ? w.g1 - w.g0 : 0;
+        for (int li = warp - 12; li < ng && ok; li += 8) {
+          ok = li < NB || __all_sync(0xffffffffu, mbar_wait(&done[(li - NB) % ND], ((li - NB) / ND) & 1, wc, W_EMPTY, 8));
+          if (!ok) break;
+          uint8_t* dst = tsm + S::B + (li % NB) * S::BSTAGE + (c16 >> 3) * (NT * 128);
+          const uint16_t* src = P.xbf + (size_t)(w.g0 + li) * 128 + c16 * 8;
+#pragma unroll
+          for (int k0 = 0; k0 < NT / 2; k0 += 8) {
+            uint4 v[8];
+#pragma unroll
+            for (int k = 0; k < 8; k++) {
+              const int m = (lane >> 4) + 2 * (k0 + k);
+              v[k] = m < P.M ? __ldcg(reinterpret_cast<const uint4*>(src + (size_t)m * P.K)) : make_uint4(0, 0, 0, 0);
+            }
+#pragma unroll
+            for (int k = 0; k < 8; k++) {
+              const int m = (lane >> 4) + 2 * (k0 + k);
+              const float f = __shfl_sync(0xffffffffu, k0 + k < 16 ? fm[0] : fm[1], m & 31);
+              *reinterpret_cast<uint4*>(dst + m * 128 + (((c16 & 7) ^ (m & 7)) << 4)) =
+                  make_uint4(f16x2_scaled(v[k].x, f), f16x2_scaled(v[k].y, f), f16x2_scaled(v[k].z, f), f16x2_scaled(v[k].w, f));
+            }
+          }
+          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&b_full[li % NB]);
+        }
+      }
+    }
     for (TcWalk w(P); w.valid() && ok; w.next(), ra.next()) {
       const int tok0 = w.tt * P.ntok, tend = min(P.M, tok0 + P.ntok), srow = w.rb * 128 + row;
       // the row's factor and the first chunk's operands are fetched while the GEMM runs
-      const float rf = __ldg(reinterpret_cast<const float*>(P.w + (size_t)(w.rb + 1) * tc_block_bytes(P.K, HZ)) - kTcRowBlock + row);
+      const float rf = __ldg(reinterpret_cast<const float*>(P.w + (size_t)(w.rb + 1) * tc_block_bytes(P.K, HZ)) - kTcTrailer / 4 + row);
       const int th0 = split ? rank * TPR + half * (TPR / 2) : tok0 + half * HC;
       const int the = min(tend, th0 + (split ? TPR / 2 : HC));
       if (split) { e_srow = srow; e_t0 = th0; e_tend = the; e_rf = rf; }
