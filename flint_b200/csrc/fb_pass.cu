@@ -209,45 +209,40 @@ bool make_act_maps(fb_ctx* c) {
   return true;
 }
 
-template <int HD, int R, int UP, bool DIRECT>
-cudaError_t launch_vattn_hd(const VattnParams& a, dim3 grid, cudaStream_t st) {
+template <int HD, int R, int RT>
+cudaError_t launch_vattn_rt(const VattnParams& a, dim3 grid, cudaStream_t st) {
   static bool configured[64] = {};
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
-  auto k = v_attn<HD, R, UP, DIRECT>;
+  auto k = v_attn<HD, R, RT>;
   if (!configured[dev]) {
-    FB_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, VaSmem<HD>::TOTAL));
-    FB_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    FB_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, VaCfg<HD, RT>::TOTAL));
     configured[dev] = true;
   }
-  return launch_pdl_cluster(k, grid, dim3(256), (size_t)VaSmem<HD>::TOTAL, st, grid.x, a);
+  return launch_pdl_cluster(k, grid, dim3(256), (size_t)VaCfg<HD, RT>::TOTAL, st, grid.x, a);
 }
-// Geometry: enough query rows (prompts) -> 128 rows a CTA, no spans. Otherwise up to four row tiles a CTA and as many spans (a power of
-// two, at most 8; 16 where a long cache meets few rows) as there are 64-position stages.
+template <int HD, int R>
+cudaError_t launch_vattn_hd(const VattnParams& a, int rt, dim3 grid, cudaStream_t st) {
+  return rt == 1 ? launch_vattn_rt<HD, R, 1>(a, grid, st) : (rt == 2 ? launch_vattn_rt<HD, R, 2>(a, grid, st) : launch_vattn_rt<HD, R, 4>(a, grid, st));
+}
+// Geometry. Few row tiles: one or two a CTA, its warps share the span's positions instead; four where that many CTAs would not fit the
+// GPU with four spans each. Spans: a power of two up to 8 while there is a stage for each and all CTAs are resident at once (with one
+// CTA per SM the GPU holds 15 clusters of 8 -- the 16th waited for a second wave, 22 us instead of 12 -- but 36 of 4).
 cudaError_t launch_vattn_tc(const fb_ctx* c, const uint16_t* kc, const uint16_t* vc, const uint8_t* amask, int pos, int M, bool want_max,
                             cudaStream_t st) {
   const fb_model_desc& d = c->d;
-  const int T = pos + M, tiles = (M * c->rgqa + 15) / 16;
-  VattnParams a{c->vq, kc, vc, amask, c->vao, want_max ? c->vamax : nullptr, d.n_head, d.n_kv_head, pos, M, 8, 0, d.attn_scale};
-  const bool direct = !want_max && d.n_kv_head * ((tiles + 7) / 8) >= c->sm_count * 2 / 3;
-  int nspan = 1, mg;
-  if (direct) {
-    mg = (tiles + 7) / 8;
-    a.span = T;
-  } else {
-    a.rt = tiles >= 3 ? 4 : (tiles == 2 ? 2 : 1);
-    mg = (tiles + a.rt - 1) / a.rt;
-    const int stages = (T + kVaPos - 1) / kVaPos, room = 2 * c->sm_count / (d.n_kv_head * mg);
-    const int most = stages > 32 && d.n_kv_head * mg * 16 <= c->sm_count ? 16 : 8;
-    while (nspan < most && nspan * 2 <= stages && nspan * 2 <= room && nspan * 2 <= a.rt * 16) nspan *= 2;
-    a.span = (stages + nspan - 1) / nspan * kVaPos;
-  }
+  const int T = pos + M, tiles = (M * c->rgqa + 15) / 16, per4 = c->sm_count / (4 * d.n_kv_head);
+  VattnParams a{c->vq, kc, vc, amask, c->vao, want_max ? c->vamax : nullptr, d.n_head, d.n_kv_head, pos, M, 0, d.attn_scale * 1.4426950408889634f};
+  const int rt = tiles <= per4 ? 1 : (tiles <= 2 * per4 ? 2 : 4), mg = (tiles + rt - 1) / rt, groups = d.n_kv_head * mg;
+  const int stages = (T + 63) / 64;
+  int nspan = 1;
+  while (nspan < 8 && nspan * 2 <= stages && groups * nspan * 2 <= (nspan == 4 ? c->sm_count * 2 / 3 : c->sm_count)) nspan *= 2;
+  a.span = (stages + nspan - 1) / nspan * 64;
   const dim3 grid(nspan, d.n_kv_head, mg);
-#define FB_VATTN2(HD_, R_)                                                                                   \
-  if (d.head_dim == HD_ && c->rgqa == R_)                                                                    \
-    return direct ? launch_vattn_hd<HD_, R_, 32, true>(a, grid, st) : launch_vattn_hd<HD_, R_, 16, false>(a, grid, st);
-  FB_VATTN2(64, 4) FB_VATTN2(80, 4) FB_VATTN2(64, 5) FB_VATTN2(128, 4)
-#undef FB_VATTN2
+  if (d.head_dim == 64 && c->rgqa == 4) return launch_vattn_hd<64, 4>(a, rt, grid, st);
+  if (d.head_dim == 80 && c->rgqa == 4) return launch_vattn_hd<80, 4>(a, rt, grid, st);
+  if (d.head_dim == 64 && c->rgqa == 5) return launch_vattn_hd<64, 5>(a, rt, grid, st);
+  if (d.head_dim == 128 && c->rgqa == 4) return launch_vattn_hd<128, 4>(a, rt, grid, st);
   return cudaErrorInvalidValue;
 }
 
