@@ -7,6 +7,7 @@
 #include "fb_verify.cuh"
 #include "fb_vsub.cuh"
 #include "fb_vtc.cuh"
+#include "fb_vtl.cuh"
 #include "fb_vattn.cuh"
 
 using namespace fb;
@@ -112,45 +113,51 @@ cudaError_t launch_vsub(const VsubParams& p, int sms, cudaStream_t st) {
   return cudaErrorInvalidValue;
 }
 
-// K splits (CTAs of a cluster) of one tcgen05 GEMM: matrices with few row blocks are cut in 2 or 4 while every CTA still finds
-// an SM of its own and two groups to multiply
-int tc_splits(int items, int k, int sms) {
+// K splits (CTAs of a cluster) of one GEMM over a single token tile: two CTAs share an SM; matrices with few row blocks are cut while
+// all CTAs are resident at once and each keeps two groups to multiply
+int tl_splits(int items, int k, int nt, int sms) {
   const int G = k / 128;
   int ns = 1;
-  while (ns < 4 && items * ns * 2 <= sms && G / (ns * 2) >= 2) ns *= 2;
+  while (ns < 8 && items * ns * 2 <= 2 * sms && G / (ns * 2) >= 2 && nt / (ns * 2) >= 2) ns *= 2;
   return ns;
 }
 template <int NT, int EPI, bool HZ>
+cudaError_t launch_vtl_hz(VtcParams& p, int sms, cudaStream_t st) {
+  static bool configured[64] = {};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
+  if (!configured[dev]) {
+    FB_TRY(cudaFuncSetAttribute(v_gemm_tl<NT, EPI, HZ>, cudaFuncAttributeMaxDynamicSharedMemorySize, VtlSmem<NT, HZ>::TOTAL));
+    configured[dev] = true;
+  }
+  if (p.K % 128 || p.M > NT) return cudaErrorInvalidValue;
+  const int items = (p.rows + kTcRowBlock - 1) / kTcRowBlock;
+  p.nsplit = tl_splits(items, p.K, NT, sms);
+  return launch_pdl_cluster(v_gemm_tl<NT, EPI, HZ>, dim3(items * p.nsplit), dim3(kTlThreads), (size_t)VtlSmem<NT, HZ>::TOTAL, st,
+                            (unsigned)p.nsplit, p);
+}
+template <int EPI, bool HZ>
 cudaError_t launch_vtc_hz(VtcParams& p, int sms, cudaStream_t st) {
   static bool configured[64] = {};
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
   if (!configured[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(v_gemm_tc<NT, EPI, HZ>, cudaFuncAttributeMaxDynamicSharedMemorySize, VtcSmem<NT, HZ>::TOTAL);
-    if (e != cudaSuccess) return e;
+    FB_TRY(cudaFuncSetAttribute(v_gemm_tc<EPI, HZ>, cudaFuncAttributeMaxDynamicSharedMemorySize, VtcSmem<HZ>::TOTAL));
     configured[dev] = true;
   }
-  if (p.xbf && (p.rows + kTcRowBlock - 1) / kTcRowBlock > sms) return cudaErrorInvalidValue;
-  if (p.K % 128 || p.ntok % 16 || p.ntok > NT || (size_t)p.ntok * p.ntile < (size_t)p.M) return cudaErrorInvalidValue;
+  if (p.K % 128 || p.ntok % 16 || p.ntok > kTcTokens || (size_t)p.ntok * p.ntile < (size_t)p.M) return cudaErrorInvalidValue;
   const int items = ((p.rows + kTcRowBlock - 1) / kTcRowBlock) * p.ntile;
-  p.nsplit = p.ntile == 1 && NT <= 64 ? tc_splits(items, p.K, sms) : 1;
-  const int grid = p.nsplit > 1 ? items * p.nsplit : (items < sms ? items : sms);
-  return launch_pdl_cluster(v_gemm_tc<NT, EPI, HZ>, dim3(grid), dim3(kTcThreads), (size_t)VtcSmem<NT, HZ>::TOTAL, st,
-                            (unsigned)p.nsplit, p);
-}
-template <int NT, int EPI>
-cudaError_t launch_vtc_nt(VtcParams& p, int sms, cudaStream_t st, bool hz) {
-  return hz ? launch_vtc_hz<NT, EPI, true>(p, sms, st) : launch_vtc_hz<NT, EPI, false>(p, sms, st);
+  return launch_pdl(v_gemm_tc<EPI, HZ>, dim3(items < sms ? items : sms), dim3(kTcThreads), (size_t)VtcSmem<HZ>::TOTAL, st, p);
 }
 // `maps`: the activation buffer as a tensor, one map per token tile height (16, 32, 64, 128)
 template <int EPI>
 cudaError_t launch_vtc(VtcParams& p, const CUtensorMap* maps, int nt, bool hz, int sms, cudaStream_t st) {
   p.xmap = maps[nt == 16 ? 0 : (nt == 32 ? 1 : (nt == 64 ? 2 : 3))];
   switch (nt) {
-    case 16: return launch_vtc_nt<16, EPI>(p, sms, st, hz);
-    case 32: return launch_vtc_nt<32, EPI>(p, sms, st, hz);
-    case 64: return launch_vtc_nt<64, EPI>(p, sms, st, hz);
-    case 128: return launch_vtc_nt<128, EPI>(p, sms, st, hz);
+    case 16: return hz ? launch_vtl_hz<16, EPI, true>(p, sms, st) : launch_vtl_hz<16, EPI, false>(p, sms, st);
+    case 32: return hz ? launch_vtl_hz<32, EPI, true>(p, sms, st) : launch_vtl_hz<32, EPI, false>(p, sms, st);
+    case 64: return hz ? launch_vtl_hz<64, EPI, true>(p, sms, st) : launch_vtl_hz<64, EPI, false>(p, sms, st);
+    case 128: return hz ? launch_vtc_hz<EPI, true>(p, sms, st) : launch_vtc_hz<EPI, false>(p, sms, st);
   }
   return cudaErrorInvalidValue;
 }
@@ -403,7 +410,7 @@ int fb_verify(fb_ctx* c, const int32_t* d_tokens, const void* d_h, const int32_t
   const int MT = M <= 16 ? 16 : (M <= 32 ? 32 : 64);
   const int D = d.dim, FF = d.ffn, HD = d.head_dim, QD = d.n_head * HD, QKV = (d.n_head + 2 * d.n_kv_head) * HD;
   const bool hz = d.has_zeros != 0;
-  if (c->verify_path == 2 || c->verify_path == 3 || (c->verify_path == 0 && M > 16) || !vgemm_known(D, QD, FF, HD))
+  if (c->verify_path == 2 || c->verify_path == 3 || (c->verify_path == 0 && (M > 8 || hz)) || !vgemm_known(D, QD, FF, HD))
     return run_tc_pass(c, d_tokens, d_h, d_depth, d_amask, M, pos, d_logits, d_feat, st);
   const size_t strQ = (size_t)pad_rows(QKV, D) * rec_bytes_of(D, hz), strO = (size_t)pad_rows(D, QD) * rec_bytes_of(QD, hz),
                strG = (size_t)pad_rows(2 * FF, D) * rec_bytes_of(D, hz), strF = (size_t)pad_rows(D, FF) * rec_bytes_of(FF, hz);

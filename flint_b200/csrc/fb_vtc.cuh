@@ -1,5 +1,6 @@
-// int4 GEMM of the M-token verify and prefill paths on the 5th-generation tensor cores (tcgen05): a weight row is read once and
-// multiplied with a tile of up to NT tokens (NT = 16 / 32 / 64 for verify, 128 for prompts).
+// int4 GEMM of the M-token passes on the 5th-generation tensor cores (tcgen05): a weight row is read once and multiplied with a tile of
+// up to NT tokens. This file: the layout, the arithmetic, the epilogues, and the kernel for prompts (tiles of up to 128 tokens);
+// fb_vtl.cuh: the kernel for trees (one tile of 16 / 32 / 64).
 //
 // D[128 weight rows][NT tokens] (fp32, in TENSOR MEMORY) += A[128][128] * B[NT][128]^T per group of 128 columns, issued as
 // eight tcgen05.mma (K = 16 each) into ONE accumulator for the whole K range. A is the group's weights with their scale,
@@ -23,10 +24,10 @@
 // after the last record the rows' factors 2^-er, fp32 [128]. One 1-D bulk copy brings a record; the dequantising thread of row r
 // reads its words without bank conflicts.
 //
-// Work item = (token tile, row block). Small matrices (QKV, O, down) are split along K over a CLUSTER of 2 or 4 CTAs: every
-// CTA sends the sums of a share of the tokens to each CTA of its cluster through distributed shared memory, and each
-// finishes its own tokens (sum in split order: deterministic), so the split costs one cluster barrier instead of a round
-// trip through global memory and the epilogue is shared out as well. Every wait is bounded.
+// Work item = (token tile, row block), round-robin over persistent CTAs; two accumulators, so an item's epilogue overlaps the MMAs of
+// the next. Trees split K over a CLUSTER instead: every CTA sends the sums of a share of the tokens to each CTA of its cluster
+// through distributed shared memory, and each finishes its own tokens (sum in split order: deterministic), so the split costs one
+// cluster barrier instead of a round trip through global memory. Every wait is bounded.
 #pragma once
 #include <cuda.h>
 
@@ -37,6 +38,7 @@ namespace fb {
 
 constexpr int kTcThreads = 640;   // warps: 0 weights, 1 MMA issue, 2 activations, 4..11 dequantise, 12..19 epilogue
 constexpr int kTcRowBlock = 128;
+constexpr int kTcTokens = 128;    // most tokens of a prompt's tile
 constexpr int kTcTrailer = kTcRowBlock * 4 + 16;      // a block's row factors, then its flag
 
 __host__ __device__ constexpr int tc_rec_bytes(int has_zeros) { return 8192 + 256 * (has_zeros ? 2 : 1); }
@@ -343,13 +345,11 @@ __device__ __forceinline__ void st_cluster_f32(uint32_t addr, float v) {
 }
 
 // Shared-memory plan (bytes). The raw ring keeps HBM busy; a stage of activations is a group's two 64-column tiles.
-template <int NT, bool HZ>
+template <bool HZ>
 struct VtcSmem {
-  static constexpr int REC = tc_rec_bytes(HZ);
-  // A stages (64 columns of tensor memory = a dequantised group) take what two accumulators leave
-  static constexpr int NS = NT <= 32 ? 6 : (NT == 64 ? (HZ ? 5 : 6) : (HZ ? 3 : 4));
-  static constexpr int NB = NT <= 16 ? 16 : (NT == 32 ? 12 : (NT == 64 ? 8 : 5));      // activation stages
-  static constexpr int NRAW = NT <= 32 ? 10 : (NT == 64 ? 7 : 6);                      // raw int4 groups
+  static constexpr int NT = kTcTokens, REC = tc_rec_bytes(HZ);
+  static constexpr int NS = HZ ? 3 : 4;                            // A stages (64 columns): what two accumulators leave
+  static constexpr int NB = 5, NRAW = 6;                           // activation stages, raw int4 groups
   static constexpr int BSTAGE = NT * 256;                          // two [NT rows x 128 bytes] swizzled tiles
   static constexpr int B = 0;
   static constexpr int RAW = B + NB * BSTAGE;
@@ -357,12 +357,11 @@ struct VtcSmem {
   // group to retire (its A stage, its activation stage) waits there; nobody is ND groups behind.
   static constexpr int ND = 16;
   static_assert(ND >= NB && ND >= NS, "a retired group must not be overtaken by the next one on its barrier");
-  static constexpr int YS = RAW + NRAW * REC;                      // K splits: the other ranks' sums, fp32 [rank][tokens][128 rows]
-  static constexpr int BAR = YS + (NT <= 64 ? NT * 512 : 0);
+  static constexpr int BAR = RAW + NRAW * REC;
   static constexpr int TOTAL = BAR + 512 + 1024;                   // barriers + slack to align the base
-  static_assert(TOTAL <= 227 * 1024, "verify GEMM shared memory");
-  // tensor memory columns: two accumulators (the epilogue of an item overlaps the MMAs of the next), A stages, A_z (8 columns = one
-  // k16 step of the row's zero point, the same for every step of the group)
+  static_assert(TOTAL <= 227 * 1024, "prompt GEMM shared memory");
+  // tensor memory columns: two accumulators, A stages, A_z (8 columns = one k16 step of the row's zero point, the same for every
+  // step of the group)
   static constexpr int T_A = 2 * NT, T_AZ = T_A + NS * 64;
   static_assert(T_AZ + (HZ ? NS * 8 : 0) <= 512, "tensor memory columns");
 };
@@ -378,15 +377,13 @@ struct Ring {
 // work items of this CTA in order (token tile by token tile: the tile's activations stay in L2); every role walks the same
 // sequence
 struct TcWalk {
-  int item, nitems, nrb, step, g0, g1, rb, tt;
+  int item, nitems, nrb, step, G, rb, tt;
   __device__ __forceinline__ TcWalk(const VtcParams& P) {
-    const int ns = P.nsplit, G = P.K / 128, sp = (int)blockIdx.x % ns;
+    G = P.K / 128;
     nrb = (P.rows + kTcRowBlock - 1) / kTcRowBlock;
     nitems = nrb * P.ntile;
-    item = (int)blockIdx.x / ns;
-    step = (int)gridDim.x / ns;
-    g0 = G * sp / ns;
-    g1 = G * (sp + 1) / ns;
+    item = (int)blockIdx.x;
+    step = (int)gridDim.x;
     set();
   }
   __device__ __forceinline__ bool valid() const { return item < nitems; }
@@ -484,10 +481,10 @@ __device__ __forceinline__ void vtc_epilogue(const VtcParams& P, int srow, int t
   }
 }
 
-template <int NT, int EPI, bool HZ>
+template <int EPI, bool HZ>
 __global__ void __launch_bounds__(kTcThreads, 1) v_gemm_tc(const __grid_constant__ VtcParams P) {
-  using S = VtcSmem<NT, HZ>;
-  constexpr int NRAW = S::NRAW, NS = S::NS, NB = S::NB, ND = S::ND, REC = S::REC, HC = NT / 2;
+  using S = VtcSmem<HZ>;
+  constexpr int NT = S::NT, NRAW = S::NRAW, NS = S::NS, NB = S::NB, ND = S::ND, REC = S::REC, HC = NT / 2;
   extern __shared__ __align__(1024) uint8_t tsm_raw[];
   // the swizzle pattern is a function of the absolute shared-memory address: tiles must start on 1024-byte boundaries
   uint8_t* tsm = tsm_raw + ((1024u - (smem_u32(tsm_raw) & 1023u)) & 1023u);
@@ -496,7 +493,6 @@ __global__ void __launch_bounds__(kTcThreads, 1) v_gemm_tc(const __grid_constant
            *acc_full = done + ND, *acc_empty = acc_full + 2;
   uint32_t* s_tmem = reinterpret_cast<uint32_t*>(acc_empty + 2);
   volatile int* s_abort = reinterpret_cast<volatile int*>(s_tmem + 1);
-  float* ys = reinterpret_cast<float*>(tsm + S::YS);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (tid == 0) {
     for (int i = 0; i < NRAW; i++) { mbar_init(&raw_full[i], 1); mbar_init(&raw_empty[i], 8); }
@@ -517,19 +513,13 @@ __global__ void __launch_bounds__(kTcThreads, 1) v_gemm_tc(const __grid_constant
   tc_fence_after();
   const uint32_t tmem = *s_tmem;
   WaitCtl wc{P.status, s_abort, P.spin_limit};
-  const bool split = NT <= 64 && P.nsplit > 1;
-  if (split) { cluster_arrive(); cluster_wait(); }               // the neighbours' shared memory exists from here on
   pdl_trigger();
   const int quad = warp & 3, row = quad * 32 + lane;             // warps 4..19: row of the block = TMEM lane
   const int half = ((warp >> 2) & 1) ^ 1;                        // warps 4..11: half of a group's columns; 12..19: of the tokens
-  // splits: this CTA finishes tokens [rank * TPR, (rank + 1) * TPR) of the item
-  const int TPR = NT / P.nsplit, lgT = 31 - __clz(TPR), rank = (int)blockIdx.x % P.nsplit;
   bool ok = true;
   constexpr int CH = tc_chunk<EPI>(HC);
   TcOperands<EPI, CH> pre;
   TcFactors<EPI> fac;
-  int e_srow = 0, e_t0 = 0, e_tend = 0;                          // split items: the epilogue's row and first token
-  float e_rf = 0.f;
 
   if (warp == 0) {
     // ---------------- producer: the groups' records (weights do not depend on the previous kernel)
@@ -538,7 +528,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) v_gemm_tc(const __grid_constant
       Ring<NRAW> r;
       for (TcWalk w(P); w.valid() && ok; w.next()) {
         const uint8_t* blk = P.w + (size_t)w.rb * tc_block_bytes(P.K, HZ);
-        for (int g = w.g0; g < w.g1; g++, gi++, r.next()) {
+        for (int g = 0; g < w.G; g++, gi++, r.next()) {
           ok = mbar_wait(&raw_empty[r.i], r.lap ^ 1u, wc, W_EMPTY, 2);
           if (!ok) break;
           mbar_expect_tx(&raw_full[r.i], REC);
@@ -567,7 +557,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) v_gemm_tc(const __grid_constant
     Ring<2> ra;
     for (TcWalk w(P); w.valid() && ok; w.next(), ra.next()) {
       ok = __all_sync(0xffffffffu, mbar_wait(&acc_empty[ra.i], ra.lap ^ 1u, wc, W_EMPTY, 3));
-      for (int g = w.g0; g < w.g1 && ok; g++, rs.next(), rb.next(), rd.next()) {
+      for (int g = 0; g < w.G && ok; g++, rs.next(), rb.next(), rd.next()) {
         // both are usually there already: test them side by side, a barrier test is a round trip of its own
         bool now = mbar_try(&a_full[rs.i], rs.lap);
         now = mbar_try(&b_full[rb.i], rb.lap) && now;
@@ -581,11 +571,11 @@ __global__ void __launch_bounds__(kTcThreads, 1) v_gemm_tc(const __grid_constant
 #pragma unroll
           for (int k = 0; k < 8; k++) {
             const uint64_t db = db0 + (uint64_t)(((k >> 2) * (NT * 128) + (k & 3) * 32) >> 4);
-            tc_mma_ts(td, ta + k * 8, db, idesc, (g > w.g0 || k) ? 1u : 0u);
+            tc_mma_ts(td, ta + k * 8, db, idesc, (g || k) ? 1u : 0u);
             if (HZ) tc_mma_ts(td, tz, db, idesc, 1u);
           }
           tc_commit(&done[rd.i]);
-          if (g == w.g1 - 1) tc_commit(&acc_full[ra.i]);
+          if (g == w.G - 1) tc_commit(&acc_full[ra.i]);
         }
         __syncwarp();
       }
@@ -594,11 +584,11 @@ __global__ void __launch_bounds__(kTcThreads, 1) v_gemm_tc(const __grid_constant
     // ---------------- activations (the previous kernel's output): two tensor copies per group. Token rows past M are whatever
     // the buffer holds: they only feed accumulator columns that nobody reads.
     pdl_wait();
-    if (lane == 0 && !(EPI == EPI_RESID && P.xbf)) {
+    if (lane == 0) {
       uint32_t gi = 0;
       Ring<NB> r;
       for (TcWalk w(P); w.valid() && ok; w.next()) {
-        for (int g = w.g0; g < w.g1; g++, gi++, r.next()) {
+        for (int g = 0; g < w.G; g++, gi++, r.next()) {
           // group gi - NB has retired
           ok = gi < NB || mbar_wait(&done[(gi - NB) % ND], ((gi - NB) / ND) & 1, wc, W_EMPTY, 8);
           if (!ok) break;
@@ -628,7 +618,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) v_gemm_tc(const __grid_constant
     Ring<NS> rs;
     for (TcWalk w(P); w.valid() && ok; w.next()) {
       const bool fast = !HZ && __ldg(reinterpret_cast<const int*>(P.w + (size_t)(w.rb + 1) * tc_block_bytes(P.K, HZ)) - 4) != 0;
-      for (int g = w.g0; g < w.g1; g++, gi++, rr.next(), rs.next()) {
+      for (int g = 0; g < w.G; g++, gi++, rr.next(), rs.next()) {
         uint64_t* freed = &done[(gi - NS) % ND];                 // the stage's previous group has retired
         const uint32_t fpar = ((gi - NS) / ND) & 1;
         bool now = mbar_try(&raw_full[rr.i], rr.lap);
@@ -674,106 +664,33 @@ __global__ void __launch_bounds__(kTcThreads, 1) v_gemm_tc(const __grid_constant
     const uint32_t tlane = tmem + ((uint32_t)(quad * 32) << 16) + half * HC;
     Ring<2> ra;
     pdl_wait();
-    if constexpr (EPI == EPI_RESID && NT <= 64) {
-      if (P.xbf) {
-        // these warps are idle until the sums are there: each brings every eighth group of the attention output, bf16 -> fp16 times
-        // the token's power of two, into the swizzled activation stages
-        float fm[2];
-#pragma unroll
-        for (int k = 0; k < 2; k++) fm[k] = 32 * k + lane < P.M ? pow2_for(__uint_as_float(__ldcg(P.amax + 32 * k + lane))).x : 0.f;
-        const TcWalk w(P);
-        const int c16 = lane & 15, ng = w.valid() ? w.g1 - w.g0 : 0;
-        for (int li = warp - 12; li < ng && ok; li += 8) {
-          ok = li < NB || __all_sync(0xffffffffu, mbar_wait(&done[(li - NB) % ND], ((li - NB) / ND) & 1, wc, W_EMPTY, 8));
-          if (!ok) break;
-          uint8_t* dst = tsm + S::B + (li % NB) * S::BSTAGE + (c16 >> 3) * (NT * 128);
-          const uint16_t* src = P.xbf + (size_t)(w.g0 + li) * 128 + c16 * 8;
-#pragma unroll
-          for (int k0 = 0; k0 < NT / 2; k0 += 8) {
-            uint4 v[8];
-#pragma unroll
-            for (int k = 0; k < 8; k++) {
-              const int m = (lane >> 4) + 2 * (k0 + k);
-              v[k] = m < P.M ? __ldcg(reinterpret_cast<const uint4*>(src + (size_t)m * P.K)) : make_uint4(0, 0, 0, 0);
-            }
-#pragma unroll
-            for (int k = 0; k < 8; k++) {
-              const int m = (lane >> 4) + 2 * (k0 + k);
-              const float f = __shfl_sync(0xffffffffu, k0 + k < 16 ? fm[0] : fm[1], m & 31);
-              *reinterpret_cast<uint4*>(dst + m * 128 + (((c16 & 7) ^ (m & 7)) << 4)) =
-                  make_uint4(f16x2_scaled(v[k].x, f), f16x2_scaled(v[k].y, f), f16x2_scaled(v[k].z, f), f16x2_scaled(v[k].w, f));
-            }
-          }
-          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-          __syncwarp();
-          if (lane == 0) mbar_arrive(&b_full[li % NB]);
-        }
-      }
-    }
     for (TcWalk w(P); w.valid() && ok; w.next(), ra.next()) {
       const int tok0 = w.tt * P.ntok, tend = min(P.M, tok0 + P.ntok), srow = w.rb * 128 + row;
       // the row's factor and the first chunk's operands are fetched while the GEMM runs
       const float rf = __ldg(reinterpret_cast<const float*>(P.w + (size_t)(w.rb + 1) * tc_block_bytes(P.K, HZ)) - kTcTrailer / 4 + row);
-      const int th0 = split ? rank * TPR + half * (TPR / 2) : tok0 + half * HC;
-      const int the = min(tend, th0 + (split ? TPR / 2 : HC));
-      if (split) { e_srow = srow; e_t0 = th0; e_tend = the; e_rf = rf; }
+      const int th0 = tok0 + half * HC, the = min(tend, th0 + HC);
       pre.fetch(P, srow, th0, the);
       fac.fetch(P, th0, the, lane);
       ok = __all_sync(0xffffffffu, mbar_wait(&acc_full[ra.i], ra.lap, wc, W_FULL, 10));
       if (!ok) break;
       tc_fence_after();
-      if (split) {
-        // token t of this half goes to the CTA that finishes it: its ys is [source rank][its tokens][128 rows]
-        const uint32_t mine = smem_u32(ys) + (uint32_t)(rank * TPR * 128 + row) * 4;
-#pragma unroll
-        for (int c = 0; c < HC; c += 8) {
-          uint32_t v[8];
-          tc_ld8(tlane + ra.i * NT + c, v);
-          tc_ld_wait();
-#pragma unroll
-          for (int e = 0; e < 8; e++) {
-            const int tk = half * HC + c + e;
-            st_cluster_f32(map_rank(mine + (uint32_t)(tk & (TPR - 1)) * 512, tk >> lgT), __uint_as_float(v[e]));
-          }
-        }
-      } else {
 #pragma unroll 1
-        for (int t0 = th0; t0 < the; t0 += CH) {
-          uint32_t u[CH / 8][8];
+      for (int t0 = th0; t0 < the; t0 += CH) {
+        uint32_t u[CH / 8][8];
 #pragma unroll
-          for (int c8 = 0; c8 < CH / 8; c8++) tc_ld8(tlane + ra.i * NT + (t0 - th0) + c8 * 8, u[c8]);
-          TcOperands<EPI, CH> nxt;
-          nxt.fetch(P, srow, t0 + CH, the);
-          tc_ld_wait();
-          float v[CH];
+        for (int c8 = 0; c8 < CH / 8; c8++) tc_ld8(tlane + ra.i * NT + (t0 - th0) + c8 * 8, u[c8]);
+        TcOperands<EPI, CH> nxt;
+        nxt.fetch(P, srow, t0 + CH, the);
+        tc_ld_wait();
+        float v[CH];
 #pragma unroll
-          for (int e = 0; e < CH; e++) v[e] = __uint_as_float(u[e >> 3][e & 7]);
-          vtc_epilogue<EPI, CH>(P, srow, t0, the, v, rf, fac, t0 - th0, pre, lane);
-          pre = nxt;
-        }
+        for (int e = 0; e < CH; e++) v[e] = __uint_as_float(u[e >> 3][e & 7]);
+        vtc_epilogue<EPI, CH>(P, srow, t0, the, v, rf, fac, t0 - th0, pre, lane);
+        pre = nxt;
       }
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&acc_empty[ra.i]);
-    }
-  }
-  if (split) {
-    __syncwarp();
-    cluster_arrive();
-    cluster_wait();                                              // every rank's sums are in
-    if (warp >= 12 && __all_sync(0xffffffffu, ok && *s_abort == 0)) {
-      const float* yw = ys + half * (TPR / 2) * 128 + row;
-      for (int t0 = 0; e_t0 + t0 < e_tend; t0 += CH) {
-        if (t0) pre.fetch(P, e_srow, e_t0 + t0, e_tend);
-        float v[CH];
-#pragma unroll
-        for (int e = 0; e < CH; e++) {
-          v[e] = 0.f;
-          if (t0 + e < TPR / 2)
-            for (int r = 0; r < P.nsplit; r++) v[e] += yw[(r * TPR + t0 + e) * 128];
-        }
-        vtc_epilogue<EPI, CH>(P, e_srow, e_t0 + t0, e_tend, v, e_rf, fac, t0, pre, lane);
-      }
     }
   }
   tc_fence_before();
