@@ -24,7 +24,7 @@ struct VaCfg {
   static constexpr int PW = HD + 4;                     // floats per partial row: acc[HD], max, denominator
   static constexpr int PART = 8 * 16 * PW * 4;          // partials (over the dead stages)
   static constexpr int RING = NSTG * STAGE > PART ? NSTG * STAGE : PART;
-  static constexpr int TOTAL = RING + 2 * 128 * 4;      // + (max, denominator) of the rows that this CTA finishes
+  static constexpr int TOTAL = RING;
   static_assert(SP / UP == PG || RT == 4, "one unit per warp and stage");
 };
 
@@ -236,68 +236,97 @@ __global__ void __launch_bounds__(256) v_attn(const VattnParams P) {
     lrun[h] += __shfl_xor_sync(0xffffffffu, lrun[h], 2);
   }
   __syncthreads();                                              // every warp has left the stages
+  float* part = reinterpret_cast<float*>(va_sm);
   {
-    float* part = reinterpret_cast<float*>(va_sm) + (size_t)warp * 16 * PW;
+    float* mine = part + (size_t)warp * 16 * PW;
 #pragma unroll
     for (int h = 0; h < 2; h++) {
-      float* pr = part + (g + 8 * h) * PW;
+      float* pr = mine + (g + 8 * h) * PW;
 #pragma unroll
       for (int j = 0; j < NTD; j++) *reinterpret_cast<float2*>(pr + j * 8 + 2 * t) = make_float2(o[j][2 * h], o[j][2 * h + 1]);
       if (t == 0) *reinterpret_cast<float2*>(pr + HD) = make_float2(mrun[h], lrun[h]);
     }
   }
-  const bool alone = nspan == 1;
-  if (alone) {
-    __syncthreads();
-  } else {
-    asm volatile("barrier.cluster.arrive.release;" ::: "memory");
-    asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
-  }
-  // this CTA finishes local rows rank, rank + nspan, ...; a row has nspan * PG partials
-  const int nown = RT * 16 / nspan, nsrc = nspan * PG;           // nown * nsrc == 128
-  float* wm = reinterpret_cast<float*>(va_sm + S::RING);
-  float* wl = wm + 128;
-  const uint32_t base = smem_u32(va_sm);
-  auto src_off = [&](int lr, int src) { return base + (uint32_t)((((lr >> 4) + RT * (src % PG)) * 16 + (lr & 15)) * PW) * 4; };
-  if (tid < 128) {
-    const int lr = rank + (tid / nsrc) * nspan, src = tid % nsrc;
-    const uint32_t a = src_off(lr, src) + HD * 4;
-    const float2 ml = alone ? *reinterpret_cast<const float2*>(va_sm + (a - base)) : ld_cluster_f2(cluster_map(a, src / PG));
-    wm[tid] = ml.x;
-    wl[tid] = ml.y;
-  }
   __syncthreads();
-  for (int ri = warp; ri < nown; ri += 8) {
-    const int lr = rank + ri * nspan, row = zg * RT * 16 + lr;
-    const float* pm = wm + ri * nsrc;
-    const float* pl = wl + ri * nsrc;
-    float gm = -1e30f, den = 0.f;
-    for (int s2 = 0; s2 < nsrc; s2++) gm = fmaxf(gm, pm[s2]);
-    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 4
-    for (int s2 = 0; s2 < nsrc; s2++) {
-      const float e = ex2(pm[s2] - gm);
-      den = fmaf(pl[s2], e, den);
-      if (lane < HD / 4) {
-        const uint32_t a = src_off(lr, s2) + lane * 16;
-        const float4 v = alone ? lds128f(a) : ld_cluster_f4(cluster_map(a, s2 / PG));
-        acc.x = fmaf(v.x, e, acc.x); acc.y = fmaf(v.y, e, acc.y); acc.z = fmaf(v.z, e, acc.z); acc.w = fmaf(v.w, e, acc.w);
-      }
-    }
+  const bool alone = nspan == 1;
+  // the position groups of the CTA meet first: a warp merges 2 RT rows (in place of position group 0's partials), so that the cluster
+  // exchanges one partial per row and span
+  auto finish = [&](int lr, float4 acc, float den) {             // local row lr, lane = 4 dims: normalise and write
+    const int row = zg * RT * 16 + lr;
     if (row < rows) {
       const float inv = 1.0f / den;
       const uint32_t w0 = cvt_bf16x2(acc.x * inv, acc.y * inv), w1 = cvt_bf16x2(acc.z * inv, acc.w * inv);
       if (lane < HD / 4)
         *reinterpret_cast<uint2*>(P.ao + (size_t)(row / R) * QD + (size_t)(kvh * R + row % R) * HD + lane * 4) = make_uint2(w0, w1);
       if (P.amax) {
-        float bm = lane < HD / 4 ? fmaxf(fmaxf(fabsf(bflo(w0)), fabsf(bfhi(w0))), fmaxf(fabsf(bflo(w1)), fabsf(bfhi(w1)))) : 0.f;
-#pragma unroll
-        for (int of = 16; of > 0; of >>= 1) bm = fmaxf(bm, __shfl_xor_sync(0xffffffffu, bm, of));
-        if (lane == 0) atomicMax(P.amax + row / R, __float_as_uint(bm));
+        const float bm = lane < HD / 4 ? fmaxf(fmaxf(fabsf(bflo(w0)), fabsf(bfhi(w0))), fmaxf(fabsf(bflo(w1)), fabsf(bfhi(w1)))) : 0.f;
+        const uint32_t bits = __reduce_max_sync(0xffffffffu, __float_as_uint(bm));   // non-negative floats order like their bits
+        if (lane == 0) atomicMax(P.amax + row / R, bits);
       }
+    }
+  };
+#pragma unroll
+  for (int i = 0; i < 2 * RT; i++) {
+    const int lr = warp * 2 * RT + i;
+    float* p0 = part + ((lr >> 4) * 16 + (lr & 15)) * PW;        // position group 0; group k is k * RT tiles further
+    float2 ml[PG];
+    float4 v[PG];
+#pragma unroll
+    for (int k = 0; k < PG; k++) {
+      ml[k] = *reinterpret_cast<const float2*>(p0 + k * RT * 16 * PW + HD);
+      v[k] = lane < HD / 4 ? *reinterpret_cast<const float4*>(p0 + k * RT * 16 * PW + lane * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    float gm = ml[0].x, den = 0.f;
+#pragma unroll
+    for (int k = 1; k < PG; k++) gm = fmaxf(gm, ml[k].x);
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int k = 0; k < PG; k++) {
+      const float e = ex2(ml[k].x - gm);
+      den = fmaf(ml[k].y, e, den);
+      acc.x = fmaf(v[k].x, e, acc.x); acc.y = fmaf(v[k].y, e, acc.y); acc.z = fmaf(v[k].z, e, acc.z); acc.w = fmaf(v[k].w, e, acc.w);
+    }
+    if (alone) {
+      finish(lr, acc, den);
+    } else {
+      __syncwarp();
+      if (lane < HD / 4) *reinterpret_cast<float4*>(p0 + lane * 4) = acc;
+      if (lane == 0) *reinterpret_cast<float2*>(p0 + HD) = make_float2(gm, den);
     }
   }
   if (!alone) {
+    asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+    // this CTA finishes local rows rank, rank + nspan, ...: all spans' partials of a row are requested together
+    const int nown = RT * 16 / nspan;
+    const uint32_t base = smem_u32(va_sm);
+    for (int ri = warp; ri < nown; ri += 8) {
+      const int lr = rank + ri * nspan;
+      const uint32_t a = base + (uint32_t)(((lr >> 4) * 16 + (lr & 15)) * PW) * 4;
+      float2 ml[8];
+      float4 v[8];
+#pragma unroll
+      for (int k = 0; k < 8; k++) {
+        ml[k] = make_float2(-1e30f, 0.f);
+        v[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (k < nspan) {
+          const uint32_t ra = cluster_map(a, k);
+          ml[k] = ld_cluster_f2(ra + HD * 4);
+          if (lane < HD / 4) v[k] = ld_cluster_f4(ra + lane * 16);
+        }
+      }
+      float gm = ml[0].x, den = 0.f;
+#pragma unroll
+      for (int k = 1; k < 8; k++) gm = fmaxf(gm, ml[k].x);
+      float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+      for (int k = 0; k < 8; k++) {
+        const float e = ex2(ml[k].x - gm);
+        den = fmaf(ml[k].y, e, den);
+        acc.x = fmaf(v[k].x, e, acc.x); acc.y = fmaf(v[k].y, e, acc.y); acc.z = fmaf(v[k].z, e, acc.z); acc.w = fmaf(v[k].w, e, acc.w);
+      }
+      finish(lr, acc, den);
+    }
     asm volatile("barrier.cluster.arrive.release;" ::: "memory");
     asm volatile("barrier.cluster.wait.acquire;" ::: "memory");  // nobody leaves while a neighbour reads its shared memory
   }

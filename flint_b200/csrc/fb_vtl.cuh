@@ -5,8 +5,8 @@
 // exist. The 200 KB form left every launch to ramp up after its predecessor had gone: QKV / O / gate-up / down took
 // 9.7 / 9.4 / 11.1 / 12.1 us at 26 tokens of the 3B shape.
 //
-// One work item (row block) per CTA, K split over a cluster of up to eight CTAs. Warps: 0 weight producer, 1 MMA issue, 2..5
-// activations (tensor copies, or the fp16 conversion of the attention output), 6..13 dequantise, then epilogue.
+// One work item (row block) per CTA, K split over a cluster of up to eight CTAs. Warps: 0 weight producer, 1 MMA issue, 2..4
+// activations (tensor copies, or the fp16 conversion of the attention output), 5 code warm-up, 6..13 dequantise, then epilogue.
 #pragma once
 #include "fb_vtc.cuh"
 
@@ -119,16 +119,16 @@ __global__ void __launch_bounds__(kTlThreads, 2) v_gemm_tl(const __grid_constant
       }
       __syncwarp();
     }
-  } else if (warp < 6) {
+  } else if (warp < 5) {
     // ---------------- activations (the previous kernel's output). Token rows past M only feed accumulator columns that nobody reads.
     if (EPI == EPI_RESID && P.xbf) {
-      // the attention output in bf16: each of the four warps converts every fourth group to fp16 times the token's power of two
+      // the attention output in bf16: each of the three warps converts every third group to fp16 times the token's power of two
       pdl_wait();
       float fm[2];
 #pragma unroll
       for (int k = 0; k < 2; k++) fm[k] = 32 * k + lane < P.M ? pow2_for(__uint_as_float(__ldcg(P.amax + 32 * k + lane))).x : 0.f;
       const int c16 = lane & 15;
-      for (int li = warp - 2; li < ng; li += 4) {
+      for (int li = warp - 2; li < ng; li += 3) {
         ok = li < NB || __all_sync(0xffffffffu, mbar_wait(&done[(li - NB) % ND], ((li - NB) / ND) & 1, wc, W_EMPTY, 8));
         if (!ok) break;
         uint8_t* dst = tsm + S::B + (li % NB) * S::BSTAGE + (c16 >> 3) * (NT * 128);
@@ -179,8 +179,10 @@ __global__ void __launch_bounds__(kTlThreads, 2) v_gemm_tl(const __grid_constant
     }
   } else {
     // ---------------- dequantise: thread = (row of the block = TMEM lane, half of the group's columns), then epilogue: thread = (row,
-    // half of the tokens)
-    constexpr int CH = 8;
+    // half of the tokens). Warp 5 walks through the epilogue first, with every store and remote write switched off, so that its
+    // instructions are in the cache when the sums arrive: the code of a dozen kernels passes through that cache every layer, and cold
+    // the QKV epilogue took 3.3 us for what is 0.4 us of work.
+    constexpr int CH = 4;
     const int quad = warp & 3, row = quad * 32 + lane, half = warp >= 10;
     const uint32_t tq = tmem + ((uint32_t)(quad * 32) << 16);
     const int* trailer = reinterpret_cast<const int*>(blk + (size_t)G * REC);
@@ -195,10 +197,19 @@ __global__ void __launch_bounds__(kTlThreads, 2) v_gemm_tl(const __grid_constant
       pre.fetch(P, srow, th0, the);
       fac.fetch(P, th0, the, lane);
     };
+    pre.fetch(P, srow, 0, 0);                                    // nothing: defined values for the walk-through
+    fac.fetch(P, 0, 0, lane);
+    const float rf = __int_as_float(__ldg(trailer + row));
+    const uint32_t tlane = tq + half * HC, mine = smem_u32(ys) + (uint32_t)(rank * TPR * 128 + row) * 4;
+    const float* yw = ys + half * HT * 128 + row;
     Ring<NRAW> rr;
     Ring<NS> rs;
-    for (int gi = 0; gi < ng; gi++, rr.next(), rs.next()) {
-      if (gi == NS) fetch();                                     // the first groups are ready; everything later needs the activations
+    int gi = 0;
+    const bool real = warp > 5;
+    const int gend = real ? ng : 0, tend = real ? the : th0, push_end = real ? P.M : 0;
+#pragma unroll 1
+    for (; gi < gend; gi++, rr.next(), rs.next()) {
+      if (gi == NS) fetch();                                   // the first groups are ready; everything later needs the activations
       uint64_t* freed = &done[(gi - NS) & (ND - 1)];             // the stage's previous group has retired
       const uint32_t fpar = ((gi - NS) / ND) & 1;
       bool now = mbar_try(&raw_full[rr.i], rr.lap);
@@ -237,16 +248,15 @@ __global__ void __launch_bounds__(kTlThreads, 2) v_gemm_tl(const __grid_constant
       __syncwarp();
       if (lane == 0) { mbar_arrive(&a_full[rs.i]); mbar_arrive(&raw_empty[rr.i]); }
     }
-    if (ng <= NS) fetch();
-    const float rf = __int_as_float(__ldg(trailer + row));
-    if (ok) ok = __all_sync(0xffffffffu, mbar_wait(acc_full, 0, wc, W_FULL, 10));
-    if (ok) {
+    if (real) {
+      if (ng <= NS) fetch();
+      if (ok) ok = __all_sync(0xffffffffu, mbar_wait(acc_full, 0, wc, W_FULL, 10));
       tc_fence_after();
-      const uint32_t tlane = tq + half * HC;
-      if (split) {
-        // token t of this half goes to the CTA that finishes it
-        const uint32_t mine = smem_u32(ys) + (uint32_t)(rank * TPR * 128 + row) * 4;
-#pragma unroll
+    }
+    if (split) {
+      // token t of this half goes to the CTA that finishes it
+      if (ok) {
+#pragma unroll 1
         for (int c = 0; c < HC; c += 8) {
           uint32_t u[8];
           tc_ld8(tlane + c, u);
@@ -254,45 +264,39 @@ __global__ void __launch_bounds__(kTlThreads, 2) v_gemm_tl(const __grid_constant
 #pragma unroll
           for (int e = 0; e < 8; e++) {
             const int tk = half * HC + c + e;
-            if (tk < P.M) st_cluster_f32(map_rank(mine + (uint32_t)(tk & (TPR - 1)) * 512, tk >> lgT), __uint_as_float(u[e]));
+            if (tk < push_end) st_cluster_f32(map_rank(mine + (uint32_t)(tk & (TPR - 1)) * 512, tk >> lgT), __uint_as_float(u[e]));
           }
+        }
+      }
+      if (real) {
+        __syncwarp();
+        cluster_arrive();
+        cluster_wait();                                        // every rank's sums are in
+        ok = __all_sync(0xffffffffu, ok && *s_abort == 0);
+      }
+    }
+    int t0 = 0;
+    if (ok) do {
+      float v[CH];
+      if (split) {
+        if (t0) pre.fetch(P, srow, th0 + t0, tend);
+#pragma unroll
+        for (int e = 0; e < CH; e++) {
+          v[e] = 0.f;
+          if (t0 + e < HT)
+            for (int r = 0; r < ns; r++) v[e] += yw[(r * TPR + t0 + e) * 128];
         }
       } else {
-#pragma unroll 1
-        for (int t0 = th0; t0 < the; t0 += CH) {
-          uint32_t u[8];
-          tc_ld8(tlane + (t0 - th0), u);
-          TcOperands<EPI, CH> nxt;
-          nxt.fetch(P, srow, t0 + CH, the);
-          tc_ld_wait();
-          float v[CH];
+        uint32_t u[8];
+        tc_ld8(tlane + t0, u);
+        if (t0) pre.fetch(P, srow, th0 + t0, tend);
+        tc_ld_wait();
 #pragma unroll
-          for (int e = 0; e < CH; e++) v[e] = __uint_as_float(u[e]);
-          vtc_epilogue<EPI, CH>(P, srow, t0, the, v, rf, fac, t0 - th0, pre, lane);
-          pre = nxt;
-        }
+        for (int e = 0; e < CH; e++) v[e] = __uint_as_float(u[e]);
       }
-    }
-    if (split) {
-      __syncwarp();
-      cluster_arrive();
-      cluster_wait();                                            // every rank's sums are in
-      if (__all_sync(0xffffffffu, ok && *s_abort == 0)) {
-        const float* yw = ys + half * HT * 128 + row;
-#pragma unroll 1
-        for (int t0 = 0; th0 + t0 < the; t0 += CH) {
-          if (t0) pre.fetch(P, srow, th0 + t0, the);
-          float v[CH];
-#pragma unroll
-          for (int e = 0; e < CH; e++) {
-            v[e] = 0.f;
-            if (t0 + e < HT)
-              for (int r = 0; r < ns; r++) v[e] += yw[(r * TPR + t0 + e) * 128];
-          }
-          vtc_epilogue<EPI, CH>(P, srow, th0 + t0, the, v, rf, fac, t0, pre, lane);
-        }
-      }
-    }
+      vtc_epilogue<EPI, CH>(P, srow, th0 + t0, tend, v, rf, fac, t0, pre, lane);
+      t0 += CH;
+    } while (th0 + t0 < tend);
   }
   if (split && warp < 6) {
     __syncwarp();
