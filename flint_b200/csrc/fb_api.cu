@@ -296,7 +296,7 @@ int fb_set_option(fb_ctx* c, int32_t what, int64_t value) {
   if (what == 1) { c->force_chunks = (int)value; return FB_OK; }          // attention chunks per kv head (0 = auto)
   if (what == 5) { c->poll_words = value != 0; return FB_OK; }
   if (what == 8) { if (value < 0 || value > 2) return FB_ERR_ARG; c->long_kv = (int)value; return FB_OK; }
-  if (what == 7) { if (value < 0 || value > 4) return FB_ERR_ARG; c->verify_path = (int)value; return FB_OK; }
+  if (what == 7) return value < 0 || value > 4 ? FB_ERR_ARG : FB_OK;     // accepted, without effect: one implementation
   if (what == 4) { if (value < 1 || value > kStages / 2) return FB_ERR_ARG; c->max_fly = (int)value; return FB_OK; }
   if (what == 2) { c->prof = (long long*)(uintptr_t)value; return FB_OK; } // device int64[sm_count * n_layer * 16] phase stamps (ns), 0 = off
   return FB_ERR_ARG;

@@ -32,16 +32,11 @@ struct fb_ctx {
   bool peers_open[8];
   uint16_t *vh, *vxn, *vq, *vao, *vact;                             // verify / prompt activations, kPromptRows token rows each
   CUtensorMap m_xn[4], m_ao[4], m_act[4];                           // vxn, vao, vact as tensors: boxes of 16, 32, 64, 128 token rows
-  float* vpart;                                                     // verify attention: per-span partials
   uint8_t *t_qkv, *t_o, *t_gu, *t_d, *t_lm;                          // verify: the matrices in the tensor-core (TC) layout
-  uint8_t *s_qkv, *s_o, *s_gu, *s_d, *s_lm;                          // verify: the matrices in the R32 layout (small trees); NULL = not built
-  float* vsplit;                                                    // verify: split-K partial sums
-  unsigned* vcount;                                                 // verify: arrivals per (row block, row quadrant)
   float *vfx, *vfao, *vfa, *vfa_inv;                                // per token: inverse powers of two of xn / attention output, that of the SwiGLU output and its inverse
   unsigned* vamax;                                                  // per token: bound on the attention output (float bits)
   unsigned* gu_norms;                                               // [n_layer][2] largest squared row norms of gate and up (float bits)
   void* vrope;                                                      // verify: (cos, sin) per (token, rotation pair)
-  int verify_path;                                                  // 0: by tree size, 1: warp-level MMA GEMMs (bf16), 2 or 3: tcgen05 GEMMs, 4: warp-level MMA GEMMs on fp16 subnormals
   int max_fly, poll_words;
   CUtensorMap kmap, vmap;                                           // the caches as tensors for the long-cache variant
   bool kv_maps;

@@ -5,7 +5,6 @@
 #include "../../include/flint_b200.h"
 #include "fb_ctx.hpp"
 #include "fb_verify.cuh"
-#include "fb_vsub.cuh"
 #include "fb_vtc.cuh"
 #include "fb_vtl.cuh"
 #include "fb_vattn.cuh"
@@ -19,99 +18,6 @@ using namespace fb;
   } while (0)
 
 namespace {
-
-template <int MT, int K, int EPI, int HD, int ROWS>
-cudaError_t launch_vgemm_r(const VGemmParams& p, int sms, cudaStream_t st) {
-  static bool configured[64] = {};        // the attribute belongs to a device's copy of the function: once per device
-  using V = VG<MT, K, ROWS>;
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
-  if (!configured[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(v_gemm<MT, K, EPI, HD, ROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize, V::smem());
-    if (e != cudaSuccess) return e;
-    configured[dev] = true;
-  }
-  const int per_sm = (227 * 1024) / (V::smem() + 1024) >= 2 ? 2 : 1;      // persistent CTAs: as many as are resident
-  const int nrb = (p.rows + V::ROWS - 1) / V::ROWS;
-  const int grid = nrb < sms * per_sm ? nrb : sms * per_sm;
-  return launch_pdl(v_gemm<MT, K, EPI, HD, ROWS>, dim3(grid), dim3(V::NTHR), V::smem(), st, p);
-}
-template <int MT, int K, int EPI, int HD>
-cudaError_t launch_vgemm_k(const VGemmParams& p, int sms, cudaStream_t st) {
-  // tall matrices (gate/up, LM head) with few tokens: 64-row blocks halve the per-chunk overhead per MMA and still
-  // give every SM at least one block
-  if constexpr (MT == 16 && (EPI == EPI_SWIGLU || EPI == EPI_LOGITS)) {
-    if (p.rows >= 64 * sms) return launch_vgemm_r<MT, K, EPI, HD, 64>(p, sms, st);
-  }
-  return launch_vgemm_r<MT, K, EPI, HD, 32>(p, sms, st);
-}
-// the shapes the decode kernel table knows: K = model width for QKV / gate-up / LM head and O, FFN width for down
-// whether the bf16 warp-level verify GEMM is instantiated for a model's widths (the other verify kernels take them at
-// run time)
-bool vgemm_known(int D, int QD, int FF, int HD) {
-  const bool qkv = (D == 512 && HD == 64) || (D == 2560 && (HD == 80 || HD == 64)) || (D == 4096 && HD == 128);
-  const bool kd = D == 512 || D == 2560 || D == 4096, kq = QD == 512 || QD == 2560 || QD == 4096;
-  const bool kf = FF == 1408 || FF == 8192 || FF == 14336 || FF == 512 || FF == 2560 || FF == 4096;
-  return qkv && kd && kq && kf;
-}
-
-template <int MT, int EPI>
-cudaError_t launch_vgemm_shape(const VGemmParams& p, int k, int hd, int sms, cudaStream_t st) {
-  if constexpr (EPI == EPI_QKV) {
-    if (k == 512 && hd == 64) return launch_vgemm_k<MT, 512, EPI, 64>(p, sms, st);
-    if (k == 2560 && hd == 80) return launch_vgemm_k<MT, 2560, EPI, 80>(p, sms, st);
-    if (k == 2560 && hd == 64) return launch_vgemm_k<MT, 2560, EPI, 64>(p, sms, st);
-    if (k == 4096 && hd == 128) return launch_vgemm_k<MT, 4096, EPI, 128>(p, sms, st);
-    return cudaErrorInvalidValue;
-  } else {
-    switch (k) {
-      case 512: return launch_vgemm_k<MT, 512, EPI, 64>(p, sms, st);
-      case 2560: return launch_vgemm_k<MT, 2560, EPI, 64>(p, sms, st);
-      case 4096: return launch_vgemm_k<MT, 4096, EPI, 64>(p, sms, st);
-    }
-    if constexpr (EPI == EPI_RESID) {
-      switch (k) {
-        case 1408: return launch_vgemm_k<MT, 1408, EPI_RESID, 64>(p, sms, st);
-        case 8192: return launch_vgemm_k<MT, 8192, EPI_RESID, 64>(p, sms, st);
-        case 14336: return launch_vgemm_k<MT, 14336, EPI_RESID, 64>(p, sms, st);
-      }
-    }
-    return cudaErrorInvalidValue;
-  }
-}
-template <int EPI>
-cudaError_t launch_vgemm_mt(const VGemmParams& p, int mt, int k, int hd, int sms, cudaStream_t st) {
-  switch (mt) {
-    case 16: return launch_vgemm_shape<16, EPI>(p, k, hd, sms, st);
-    case 32: return launch_vgemm_shape<32, EPI>(p, k, hd, sms, st);
-    case 64: return launch_vgemm_shape<64, EPI>(p, k, hd, sms, st);
-  }
-  return cudaErrorInvalidValue;
-}
-constexpr size_t kVsplitFloats = (size_t)256 * 64 * 128;      // K-split partial sums of v_gemm_sub that the context can hold
-
-template <int NT, int EPI>
-cudaError_t launch_vsub_nt(const VsubParams& p, int sms, cudaStream_t st) {
-  static bool configured[64] = {};
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
-  if (!configured[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(v_gemm_sub<NT, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, kVsSmem);
-    if (e != cudaSuccess) return e;
-    configured[dev] = true;
-  }
-  return launch_pdl(v_gemm_sub<NT, EPI>, dim3(sms), dim3(kVsThreads), (size_t)p.plan.bar_off + 512, st, p);
-}
-template <int EPI>
-cudaError_t launch_vsub(const VsubParams& p, int sms, cudaStream_t st) {
-  switch ((p.M + 7) / 8) {
-    case 1: return launch_vsub_nt<1, EPI>(p, sms, st);
-    case 2: return launch_vsub_nt<2, EPI>(p, sms, st);
-    case 3: return launch_vsub_nt<3, EPI>(p, sms, st);
-    case 4: return launch_vsub_nt<4, EPI>(p, sms, st);
-  }
-  return cudaErrorInvalidValue;
-}
 
 // K splits (CTAs of a cluster) of one GEMM over a single token tile: two CTAs share an SM; matrices with few row blocks are cut while
 // all CTAs are resident at once and each keeps two groups to multiply
@@ -159,41 +65,6 @@ cudaError_t launch_vtc(VtcParams& p, const CUtensorMap* maps, int nt, bool hz, i
     case 64: return hz ? launch_vtl_hz<64, EPI, true>(p, sms, st) : launch_vtl_hz<64, EPI, false>(p, sms, st);
     case 128: return hz ? launch_vtc_hz<EPI, true>(p, sms, st) : launch_vtc_hz<EPI, false>(p, sms, st);
   }
-  return cudaErrorInvalidValue;
-}
-
-cudaError_t launch_vnorm(const uint16_t* h, const uint16_t* w, uint16_t* xn_t, uint16_t* xn_nat, uint16_t* feat, int D, int M,
-                         float eps, cudaStream_t st) {
-  if (D % 16 || D > 8 * 256 * 2) return cudaErrorInvalidValue;
-  if (D <= 8 * 256) return launch_pdl(v_rmsnorm<1>, dim3(M), dim3(256), 0, st, h, w, xn_t, xn_nat, feat, D, eps);
-  return launch_pdl(v_rmsnorm<2>, dim3(M), dim3(256), 0, st, h, w, xn_t, xn_nat, feat, D, eps);
-}
-constexpr int kVSpans = 32;       // most spans of positions a kv head's attention is cut into
-
-cudaError_t launch_vattn(const fb_ctx* c, const uint16_t* q, const uint16_t* kc, const uint16_t* vc, const uint8_t* amask,
-                         uint16_t* ao, int pos, int M, cudaStream_t st) {
-  const fb_model_desc& d = c->d;
-  const int T = pos + M;
-  // a CTA takes 64 query rows (four 16-row tiles); spans of positions are sized so that about two CTAs per SM exist
-  const int mgroups = (M * c->rgqa + 63) / 64;
-  int smax = (2 * c->sm_count) / (d.n_kv_head * mgroups);
-  if (smax < 1) smax = 1;
-  if (smax > kVSpans) smax = kVSpans;
-  if (smax > kVSpans * 64 / M) smax = kVSpans * 64 / M > 0 ? kVSpans * 64 / M : 1;     // the partials' buffer
-  int S = (T + 63) / 64;
-  if (S > smax) S = smax;
-  const int span = ((T + S - 1) / S + 63) / 64 * 64;
-  S = (T + span - 1) / span;
-#define FB_VATTN(HD_, R_)                                                                                               \
-  if (d.head_dim == HD_ && c->rgqa == R_) {                                                                             \
-    cudaError_t e = launch_pdl(v_attn_mma<HD_, R_>, dim3(d.n_kv_head, S, mgroups), dim3(128), 0, st, q, kc, vc, amask, c->vpart,  \
-                               d.n_head, d.n_kv_head, pos, M, d.attn_scale, span);                                      \
-    if (e != cudaSuccess) return e;                                                                                     \
-    return launch_pdl(v_attn_merge<HD_, R_>, dim3(M, d.n_kv_head), dim3(256), 0, st, (const float*)c->vpart, ao, d.n_head, \
-                      d.n_kv_head, M, S);                                                                      \
-  }
-  FB_VATTN(64, 4) FB_VATTN(80, 4) FB_VATTN(64, 5) FB_VATTN(128, 4)
-#undef FB_VATTN
   return cudaErrorInvalidValue;
 }
 
@@ -326,10 +197,6 @@ cudaError_t pass_alloc(fb_ctx* c) {
       if (e == cudaSuccess) A(cudaMemset(*vp[i], 0, kPromptRows * rowsz[i] * 2));
     }
   }
-  A(dmalloc(&c->vpart, (size_t)d.n_kv_head * 32 * 64 * c->rgqa * (d.head_dim + 2) * 4));
-  A(dmalloc(&c->vsplit, kVsplitFloats * 4));
-  A(dmalloc(&c->vcount, kVsCounters * 4));
-  if (e == cudaSuccess) A(cudaMemset(c->vcount, 0, kVsCounters * 4));
   float** fp[4] = {&c->vfx, &c->vfao, &c->vfa, &c->vfa_inv};
   for (float** p : fp) A(dmalloc(p, kPromptRows * 4));
   A(dmalloc(&c->vamax, kPromptRows * 4));
@@ -340,39 +207,23 @@ cudaError_t pass_alloc(fb_ctx* c) {
 }
 
 void pass_free(fb_ctx* c) {
-  void* ptrs[] = {c->vh, c->vxn, c->vq, c->vao, c->vact, c->vpart, c->t_qkv, c->t_o, c->t_gu, c->t_d, c->t_lm, c->s_qkv, c->s_o, c->s_gu,
-                  c->s_d, c->s_lm, c->vsplit, c->vcount, c->vrope, c->vfx, c->vfao, c->vfa, c->vfa_inv, c->vamax, c->gu_norms};
+  void* ptrs[] = {c->vh, c->vxn, c->vq, c->vao, c->vact, c->t_qkv, c->t_o, c->t_gu, c->t_d, c->t_lm, c->vrope,
+                  c->vfx, c->vfao, c->vfa, c->vfa_inv, c->vamax, c->gu_norms};
   for (void* p : ptrs)
     if (p) cudaFree(p);
 }
 
 cudaError_t pass_bind_matrix(fb_ctx* c, int which, const void* q, const void* s, const void* z, int layers, int rows, int k, int order,
                              int arg, int orows, cudaStream_t st) {
-  uint8_t** tdst[] = {&c->t_qkv, &c->t_o, &c->t_gu, &c->t_d, &c->t_lm};
-  uint8_t** sdst[] = {&c->s_qkv, &c->s_o, &c->s_gu, &c->s_d, &c->s_lm};
-  struct M { uint8_t **tdst, **sdst; const void *q, *s, *z; int layers, rows, k, order, arg, orows; } m =
-      {tdst[which], sdst[which], q, s, z, layers, rows, k, order, arg, orows};
-  const bool hz = z != nullptr;
-    if (*m.tdst) { cudaFree(*m.tdst); *m.tdst = nullptr; }
-    if (c->tp_size == 1) {     // the verify path's own copy, in the layout the tcgen05 GEMM streams
-      const int nrb = (m.rows + kTcRowBlock - 1) / kTcRowBlock;
-      FB_TRY(dmalloc(m.tdst, (size_t)m.layers * tc_matrix_bytes(m.rows, m.k, hz) + 16));
-      if (m.order == 2) FB_TRY(cudaMemsetAsync(c->gu_norms, 0, (size_t)m.layers * 8, st));
-      tc_repack<<<dim3(nrb, m.layers), 256, 0, st>>>((const uint32_t*)m.q, (const uint16_t*)m.s, (const uint16_t*)m.z,
-                                                     m.rows, m.k, m.order, m.arg, m.orows, *m.tdst, m.order == 2 ? c->gu_norms : nullptr);
-      FB_TRY(cudaGetLastError());
-    }
-    if (*m.sdst) { cudaFree(*m.sdst); *m.sdst = nullptr; }
-    const int tiles32 = (m.rows + 31) / 32;
-    const VsPlan vp = vs_plan(m.k, 1, tiles32);
-    if (c->tp_size == 1 && !hz && vp.ok &&
-        (size_t)tiles32 * vp.nkc * 8 * 512 <= kVsplitFloats * 4) {   // K-split partials fit the shared buffer
-      // the small-tree verify GEMM's copy (symmetric layout only; other shapes keep the bf16 warp-level kernel)
-      FB_TRY(dmalloc(m.sdst, (size_t)m.layers * vs_matrix_bytes(m.rows, m.k) + 16));
-      vs_repack<<<dim3(tiles32, m.layers), 256, 0, st>>>((const uint32_t*)m.q, (const uint16_t*)m.s, m.rows, m.k, vp.ug, m.order,
-                                                         m.arg, m.orows, *m.sdst);
-      FB_TRY(cudaGetLastError());
-    }
+  uint8_t** dst[] = {&c->t_qkv, &c->t_o, &c->t_gu, &c->t_d, &c->t_lm};
+  uint8_t*& t = *dst[which];
+  if (t) { cudaFree(t); t = nullptr; }
+  if (c->tp_size > 1) return cudaSuccess;          // a tensor-parallel rank decodes only
+  FB_TRY(dmalloc(&t, (size_t)layers * tc_matrix_bytes(rows, k, z != nullptr) + 16));
+  if (order == 2) FB_TRY(cudaMemsetAsync(c->gu_norms, 0, (size_t)layers * 8, st));
+  tc_repack<<<dim3((rows + kTcRowBlock - 1) / kTcRowBlock, layers), 256, 0, st>>>((const uint32_t*)q, (const uint16_t*)s, (const uint16_t*)z, rows, k,
+                                                                                  order, arg, orows, t, order == 2 ? c->gu_norms : nullptr);
+  FB_TRY(cudaGetLastError());
   return cudaSuccess;
 }
 
@@ -404,102 +255,8 @@ int fb_verify(fb_ctx* c, const int32_t* d_tokens, const void* d_h, const int32_t
   if (!d_h && !c->embed) return FB_ERR_STATE;
   if (M < 1 || M > 64) return FB_ERR_RANGE;          /* never fall through to another M (reference: result.md:112-113) */
   if (pos < 0 || pos + M > c->max_seq) return FB_ERR_RANGE;
-  const fb_model_desc& d = c->d;
   DeviceGuard g(c->device);
-  cudaStream_t st = (cudaStream_t)stream;
-  const int MT = M <= 16 ? 16 : (M <= 32 ? 32 : 64);
-  const int D = d.dim, FF = d.ffn, HD = d.head_dim, QD = d.n_head * HD, QKV = (d.n_head + 2 * d.n_kv_head) * HD;
-  const bool hz = d.has_zeros != 0;
-  if (c->verify_path == 2 || c->verify_path == 3 || (c->verify_path == 0 && (M > 8 || hz)) || !vgemm_known(D, QD, FF, HD))
-    return run_tc_pass(c, d_tokens, d_h, d_depth, d_amask, M, pos, d_logits, d_feat, st);
-  const size_t strQ = (size_t)pad_rows(QKV, D) * rec_bytes_of(D, hz), strO = (size_t)pad_rows(D, QD) * rec_bytes_of(QD, hz),
-               strG = (size_t)pad_rows(2 * FF, D) * rec_bytes_of(D, hz), strF = (size_t)pad_rows(D, FF) * rec_bytes_of(FF, hz);
-  FB_CUDA(c, launch_pdl(v_embed, dim3(M), dim3(256), 0, st, d_tokens, (const uint16_t*)c->embed, (const uint16_t*)d_h, c->vh,
-                        D, d.vocab, d.emb_mult, &c->status->code));
-  VGemmParams p;
-  memset(&p, 0, sizeof(p));
-  p.M = M; p.has_zeros = hz; p.depth = d_depth; p.invf = c->invf; p.n_head = d.n_head; p.nkv = d.n_kv_head; p.pos = pos;
-  p.resid = d.resid_mult; p.logits_scaling = d.logits_scaling;
-  // small trees: every GEMM whose matrix has an R32 copy runs on the subnormal-operand kernel. It reads the same
-  // activation buffers; the QKV and gate/up GEMMs read the residual rows and apply the RMSNorm themselves
-  // by tree size: up to 8 tokens (one B tile) this kernel wins (2.07 vs 2.40 ms per pass of the 3B model); above, its
-  // per-CTA conversion of the activations (linear in the tokens) costs more than the dequantisation it saves
-  const bool use_sub = (c->verify_path == 4 || (c->verify_path == 0 && M <= 8)) && M <= kVsMaxTokens && !hz;
-  VsubParams sp;
-  memset(&sp, 0, sizeof(sp));
-  sp.M = M; sp.part = c->vsplit; sp.counters = (int*)c->vcount; sp.status = c->status; sp.spin_limit = c->spin_limit;
-  sp.rope = (const float2*)c->vrope; sp.n_head = d.n_head; sp.nkv = d.n_kv_head; sp.pos = pos; sp.head_dim = HD;
-  sp.resid = d.resid_mult; sp.logits_scaling = d.logits_scaling; sp.eps = d.rms_eps;
-  if (use_sub && c->s_qkv)
-    FB_CUDA(c, launch_pdl(v_rope_table, dim3(M), dim3(64), 0, st, d_depth, (const float*)c->invf, (int)pos, HD / 2, (float2*)c->vrope));
-  int nsub = 0;
-  auto sub = [&](const uint8_t* sw, size_t layer, int rows, int K) -> bool {
-    if (!use_sub || !sw) return false;
-    sp.plan = vs_plan(K, M, (rows + 31) / 32);
-    if (!sp.plan.ok) return false;
-    sp.w = sw + layer * vs_matrix_bytes(rows, K); sp.rows = rows; sp.K = K; sp.norm_w = nullptr;
-    sp.dbg = (c->prof && layer == 1) ? c->prof + 8 * (nsub++ & 7) : nullptr;   // stamps of the second layer's GEMMs
-    return true;
-  };
-  for (int l = 0; l < d.n_layer; l++) {
-    uint16_t* kcl = (uint16_t*)c->kc + (size_t)l * c->max_seq * d.n_kv_head * HD;
-    uint16_t* vcl = (uint16_t*)c->vc + (size_t)l * c->max_seq * d.n_kv_head * HD;
-    if (sub(c->s_qkv, l, QKV, D)) {
-      if (sp.plan.nkc == 1) { sp.x = c->vh; sp.norm_w = (const uint16_t*)c->n1 + (size_t)l * D; }
-      else {
-        FB_CUDA(c, launch_vnorm(c->vh, (const uint16_t*)c->n1 + (size_t)l * D, c->vxn, nullptr, nullptr, D, M, d.rms_eps, st));
-        sp.x = c->vxn;
-      }
-      sp.q = c->vq; sp.kc = kcl; sp.vc = vcl;
-      FB_CUDA(c, launch_vsub<EPI_QKV>(sp, c->sm_count, st));
-    } else {
-      FB_CUDA(c, launch_vnorm(c->vh, (const uint16_t*)c->n1 + (size_t)l * D, c->vxn, nullptr, nullptr, D, M, d.rms_eps, st));
-      p.w = c->w_qkv + l * strQ; p.x_t = c->vxn; p.rows = QKV;
-      p.q = c->vq; p.kc = kcl; p.vc = vcl;
-      FB_CUDA(c, launch_vgemm_mt<EPI_QKV>(p, MT, D, HD, c->sm_count, st));
-    }
-    FB_CUDA(c, launch_vattn(c, c->vq, kcl, vcl, d_amask, c->vao, pos, M, st));
-    if (sub(c->s_o, l, D, QD)) {
-      sp.x = c->vao; sp.h = c->vh; sp.out_ld = D;
-      FB_CUDA(c, launch_vsub<EPI_RESID>(sp, c->sm_count, st));
-    } else {
-      p.w = c->w_o + l * strO; p.x_t = c->vao; p.rows = D; p.h = c->vh; p.out_ld = D;
-      FB_CUDA(c, launch_vgemm_mt<EPI_RESID>(p, MT, QD, HD, c->sm_count, st));
-    }
-    if (sub(c->s_gu, l, 2 * FF, D)) {
-      if (sp.plan.nkc == 1) { sp.x = c->vh; sp.norm_w = (const uint16_t*)c->n2 + (size_t)l * D; }
-      else {
-        FB_CUDA(c, launch_vnorm(c->vh, (const uint16_t*)c->n2 + (size_t)l * D, c->vxn, nullptr, nullptr, D, M, d.rms_eps, st));
-        sp.x = c->vxn;
-      }
-      sp.act_t = c->vact; sp.out_ld = FF;
-      FB_CUDA(c, launch_vsub<EPI_SWIGLU>(sp, c->sm_count, st));
-    } else {
-      FB_CUDA(c, launch_vnorm(c->vh, (const uint16_t*)c->n2 + (size_t)l * D, c->vxn, nullptr, nullptr, D, M, d.rms_eps, st));
-      p.w = c->w_gu + l * strG; p.x_t = c->vxn; p.rows = 2 * FF; p.act_t = c->vact;
-      p.out_ld = FF;
-      FB_CUDA(c, launch_vgemm_mt<EPI_SWIGLU>(p, MT, D, HD, c->sm_count, st));
-    }
-    if (sub(c->s_d, l, D, FF)) {
-      sp.x = c->vact; sp.h = c->vh; sp.out_ld = D;
-      FB_CUDA(c, launch_vsub<EPI_RESID>(sp, c->sm_count, st));
-    } else {
-      p.w = c->w_d + l * strF; p.x_t = c->vact; p.rows = D; p.h = c->vh; p.out_ld = D;
-      FB_CUDA(c, launch_vgemm_mt<EPI_RESID>(p, MT, FF, HD, c->sm_count, st));
-    }
-  }
-  FB_CUDA(c, launch_vnorm(c->vh, (const uint16_t*)c->nf, c->vxn, nullptr, (uint16_t*)d_feat, D, M, d.rms_eps, st));
-  if (d_logits) {
-    if (sub(c->s_lm, 0, d.vocab, D)) {
-      sp.x = c->vxn; sp.logits = d_logits; sp.out_ld = d.vocab;
-      FB_CUDA(c, launch_vsub<EPI_LOGITS>(sp, c->sm_count, st));
-    } else {
-      p.w = c->w_lm; p.x_t = c->vxn; p.rows = d.vocab; p.logits = d_logits; p.out_ld = d.vocab;
-      FB_CUDA(c, launch_vgemm_mt<EPI_LOGITS>(p, MT, D, HD, c->sm_count, st));
-    }
-  }
-  FB_CUDA(c, cudaGetLastError());
-  return FB_OK;
+  return run_tc_pass(c, d_tokens, d_h, d_depth, d_amask, M, pos, d_logits, d_feat, (cudaStream_t)stream);
 }
 
 }  // extern "C"
