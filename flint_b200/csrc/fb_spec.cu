@@ -12,12 +12,13 @@ using namespace fb;
 
 struct fb_draft {
   fb_draft_desc d;
-  int device, sm_count;
+  int device;
   fb_draft_weights w;
   bool bound;
   uint16_t *x, *h, *q, *k, *v, *att, *x2, *act, *hh, *fn;     // [max_tokens] rows of activations
   uint16_t *kc, *vc;                                           // [max_roll, n_kv, hd]
   float* logits;                                               // [max_heads rows, vocab]
+  float* invf;                                                 // [hd / 2] rotation frequencies
   int last_cuda_error;
 };
 
@@ -25,43 +26,34 @@ namespace {
 
 constexpr int kMaxHeadRows = 16;
 
-template <int TT, int MODE>
-cudaError_t launch_linear_tt(const DLin& p, int t0, int sms, cudaStream_t st) {
-  static bool configured[64] = {};
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
-  const size_t smem = (size_t)TT * (p.k0 + p.k1) * 2;
-  if (smem > 200 * 1024) return cudaErrorInvalidValue;
-  if (!configured[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(d_linear<TT, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    if (e != cudaSuccess) return e;
-    configured[dev] = true;
-  }
-  int per_sm = (int)((220 * 1024) / (smem + 1024));
-  per_sm = per_sm < 1 ? 1 : (per_sm > 8 ? 8 : per_sm);
-  int grid = (p.N + 7) / 8;
-  if (grid > sms * per_sm) grid = sms * per_sm;
-  return launch_pdl(d_linear<TT, MODE>, dim3(grid), dim3(256), smem, st, p, t0);
+template <int NT, int MT, int WARPS, int MODE>
+cudaError_t launch_linear_nt(const DLin& p, int t0, cudaStream_t st) {
+  int grid = 0;
+  for (int i = 0; i < (MODE == DL_STORE ? 3 : 1) && p.W[i]; i++) grid += (p.N[i] + 16 * MT - 1) / (16 * MT);
+  if (MODE == DL_STORE && p.x1) return launch_pdl(d_gemm<NT, MT, WARPS, MODE, MODE == DL_STORE>, dim3(grid), dim3(WARPS * 32), 0, st, p, t0);
+  return launch_pdl(d_gemm<NT, MT, WARPS, MODE, false>, dim3(grid), dim3(WARPS * 32), 0, st, p, t0);
 }
-
-// all T tokens, in blocks of up to 16 where two CTAs of 16 input rows still share an SM, else up to 8 (fewer tokens per
-// block where 8 rows of inputs do not fit shared memory): the weights are read once per block
+// All T tokens, up to 32 per pass over the weights. Up to 8 tokens: 16 rows per CTA (the matrices of a layer then give every SM at least
+// one), 32 for the token head, whose 49 000 rows and more do not need it. More tokens: 32 rows per CTA (one matrix) or 16 of each of
+// two, so that a CTA reads about as many bytes of activations from L2 as of weights, and 16 warps to share a long K.
 template <int MODE>
-cudaError_t launch_linear(const DLin& p, int sms, cudaStream_t st) {
-  const int K = p.k0 + p.k1;
-  if (K % 8 || p.k0 % 8 || p.N <= 0 || p.T <= 0) return cudaErrorInvalidValue;
-  const int cap = K * 2 * 8 <= 200 * 1024 ? 8 : (K * 2 * 4 <= 200 * 1024 ? 4 : (K * 2 * 2 <= 200 * 1024 ? 2 : 1));
-  for (int t0 = 0; t0 < p.T;) {
+cudaError_t launch_linear(const DLin& p, cudaStream_t st) {
+  if ((p.k0 + p.k1) % 8 || p.k0 % 8 || p.N[0] <= 0 || p.T <= 0) return cudaErrorInvalidValue;
+  constexpr int MW = MODE == DL_SWIGLU ? 1 : 2;
+  cudaError_t e = cudaSuccess;
+  for (int t0 = 0; t0 < p.T && e == cudaSuccess; t0 += 32) {
     const int left = p.T - t0;
-    cudaError_t e;
-    if (left >= 16 && K * 2 * 16 <= 100 * 1024) { e = launch_linear_tt<16, MODE>(p, t0, sms, st); t0 += 16; }
-    else if (left >= 8 && cap >= 8) { e = launch_linear_tt<8, MODE>(p, t0, sms, st); t0 += 8; }
-    else if (left >= 4 && cap >= 4) { e = launch_linear_tt<4, MODE>(p, t0, sms, st); t0 += 4; }
-    else if (left >= 2 && cap >= 2) { e = launch_linear_tt<2, MODE>(p, t0, sms, st); t0 += 2; }
-    else { e = launch_linear_tt<1, MODE>(p, t0, sms, st); t0 += 1; }
-    if (e != cudaSuccess) return e;
+    if (left <= 8) e = launch_linear_nt<1, MODE == DL_LOGITS ? 2 : 1, 8, MODE>(p, t0, st);
+    else if (left <= 16) e = launch_linear_nt<2, MW, 16, MODE>(p, t0, st);
+    else e = launch_linear_nt<4, MW, 16, MODE>(p, t0, st);
   }
-  return cudaSuccess;
+  return e;
+}
+// CTAs per row of the token choice: slices of at least 4096 values, at most 8 CTAs (the portable cluster)
+int row_ctas(int vocab) {
+  int c = 1;
+  while (c < 8 && vocab >= 4096 * 2 * c) c *= 2;
+  return c;
 }
 
 int dfail(fb_draft* d, cudaError_t e) {
@@ -83,8 +75,10 @@ int fb_sample(const float* d_logits, int32_t vocab, int32_t rows, int64_t row_st
   if (!d_logits || !d_out || vocab <= 0 || rows <= 0 || row_stride < 0) return FB_ERR_ARG;
   SampleParams p{d_logits, (long long)row_stride, vocab, top_k, temperature, (unsigned long long)seed,
                  (unsigned long long)counter, d_out};
-  sample_rows<<<rows, 1024, 0, (cudaStream_t)stream>>>(p);
-  return cudaGetLastError() == cudaSuccess ? FB_OK : FB_ERR_CUDA;
+  const int c = row_ctas(vocab);
+  const bool reg = (vocab + c - 1) / c <= kSampleRegs * 1024;
+  const cudaError_t e = launch_pdl_cluster(reg ? sample_rows<true> : sample_rows<false>, dim3(c, rows), dim3(1024), 0, (cudaStream_t)stream, c, p);
+  return e == cudaSuccess ? FB_OK : FB_ERR_CUDA;
 }
 
 int fb_accept_chain(const int32_t* d_target, const int32_t* d_draft, int32_t k, int32_t* d_out, void* stream) {
@@ -128,7 +122,6 @@ int fb_draft_create(const fb_draft_desc* desc, int device, fb_draft** out) {
   memset(r, 0, sizeof(*r));
   r->d = d;
   r->device = device;
-  if (cudaDeviceGetAttribute(&r->sm_count, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) { delete r; return FB_ERR_CUDA; }
   const size_t T = d.max_tokens, D = d.dim, kvd = (size_t)d.n_kv_head * hd, F = (size_t)d.fuse * d.dim;
   cudaError_t e = cudaSuccess;
   auto A = [&](cudaError_t x) { if (e == cudaSuccess) e = x; };
@@ -138,9 +131,15 @@ int fb_draft_create(const fb_draft_desc* desc, int device, fb_draft** out) {
   A(dmalloc(&r->fn, (size_t)kMaxHeadRows * D * 2));
   A(dmalloc(&r->kc, (size_t)d.max_roll * kvd * 2)); A(dmalloc(&r->vc, (size_t)d.max_roll * kvd * 2));
   A(dmalloc(&r->logits, (size_t)kMaxHeadRows * d.vocab * 4));
+  A(dmalloc(&r->invf, (size_t)hd * 2));
   if (e == cudaSuccess) A(cudaMemset(r->kc, 0, (size_t)d.max_roll * kvd * 2));
   if (e == cudaSuccess) A(cudaMemset(r->vc, 0, (size_t)d.max_roll * kvd * 2));
   (void)F;
+  if (e == cudaSuccess) {
+    d_invf<<<1, 64>>>(r->invf, d.rope_base, hd);
+    A(cudaGetLastError());
+    A(cudaDeviceSynchronize());                    // the streams of the calls do not wait for this one
+  }
   if (e != cudaSuccess) { fb_draft_destroy(r); return FB_ERR_CUDA; }
   *out = r;
   return FB_OK;
@@ -149,7 +148,7 @@ int fb_draft_create(const fb_draft_desc* desc, int device, fb_draft** out) {
 int fb_draft_destroy(fb_draft* r) {
   if (!r) return FB_ERR_ARG;
   DeviceGuard g(r->device);
-  void* ptrs[] = {r->x, r->h, r->q, r->k, r->v, r->att, r->x2, r->act, r->hh, r->fn, r->kc, r->vc, r->logits};
+  void* ptrs[] = {r->x, r->h, r->q, r->k, r->v, r->att, r->x2, r->act, r->hh, r->fn, r->kc, r->vc, r->logits, r->invf};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   delete r;
@@ -175,51 +174,48 @@ int fb_draft_forward(fb_draft* r, const void* d_feat, const void* d_emb, const i
   if (((uintptr_t)d_feat & 15) || ((uintptr_t)d_emb & 15) || ((uintptr_t)d_out & 1)) return FB_ERR_ARG;
   DeviceGuard g(r->device);
   cudaStream_t st = (cudaStream_t)stream;
-  const int D = d.dim, F = d.fuse * d.dim, hd = D / d.n_head, kvd = d.n_kv_head * hd, sms = r->sm_count;
-  const uint16_t* W = nullptr;
+  const int D = d.dim, F = d.fuse * d.dim, hd = D / d.n_head, kvd = d.n_kv_head * hd;
   DLin p;
   // x = merge(cat(feat, emb))
   memset(&p, 0, sizeof(p));
-  p.W = (const uint16_t*)r->w.merge; p.x0 = (const uint16_t*)d_feat; p.ldx0 = F; p.k0 = F;
+  p.W[0] = (const uint16_t*)r->w.merge; p.x0 = (const uint16_t*)d_feat; p.ldx0 = F; p.k0 = F;
   if (d_emb) { p.x1 = (const uint16_t*)d_emb; p.ldx1 = D; }
   else { p.x1 = (const uint16_t*)r->w.embed; p.ldx1 = D; p.x1_tokens = d_tokens; }
-  p.k1 = D; p.N = D; p.T = T; p.y = r->x; p.ldy = D;
-  FB_DCUDA(r, launch_linear<DL_STORE>(p, sms, st));
+  p.k1 = D; p.N[0] = D; p.T = T; p.y[0] = r->x; p.ldy[0] = D;
+  FB_DCUDA(r, launch_linear<DL_STORE>(p, st));
   FB_DCUDA(r, launch_pdl(d_rmsnorm, dim3(T), dim3(256), 0, st, (const uint16_t*)r->x, D, (const uint16_t*)r->w.n1, r->h, D, D, d.rms_eps));
-  // q, k, v
+  // q, k, v in one launch
+  memset(&p, 0, sizeof(p));
   const void* qkvw[3] = {r->w.q, r->w.k, r->w.v};
   uint16_t* qkvo[3] = {r->q, r->k, r->v};
   const int qkvn[3] = {D, kvd, kvd};
-  for (int i = 0; i < 3; i++) {
-    memset(&p, 0, sizeof(p));
-    p.W = (const uint16_t*)qkvw[i]; p.x0 = r->h; p.ldx0 = D; p.k0 = D; p.N = qkvn[i]; p.T = T; p.y = qkvo[i]; p.ldy = qkvn[i];
-    FB_DCUDA(r, launch_linear<DL_STORE>(p, sms, st));
-  }
+  for (int i = 0; i < 3; i++) { p.W[i] = (const uint16_t*)qkvw[i]; p.N[i] = qkvn[i]; p.y[i] = qkvo[i]; p.ldy[i] = qkvn[i]; }
+  p.x0 = r->h; p.ldx0 = D; p.k0 = D; p.T = T;
+  FB_DCUDA(r, launch_linear<DL_STORE>(p, st));
   FB_DCUDA(r, launch_pdl(d_rope_store, dim3(T, d.n_head + d.n_kv_head), dim3(64), 0, st, r->q, (const uint16_t*)r->k, (const uint16_t*)r->v, d_positions,
-                         d_slots, r->kc, r->vc, d.n_head, d.n_kv_head, hd, d.rope_base, d.max_roll));
-  FB_DCUDA(r, launch_pdl(d_attn, dim3(T, d.n_head), dim3(128), (size_t)d.max_roll * 4, st, (const uint16_t*)r->q, d_slots,
+                         d_slots, r->kc, r->vc, d.n_head, d.n_kv_head, hd, (const float*)r->invf, d.max_roll));
+  FB_DCUDA(r, launch_pdl(d_attn, dim3(T, d.n_head), dim3(128), (size_t)(d.max_roll + hd) * 4, st, (const uint16_t*)r->q, d_slots,
                          (const uint16_t*)r->kc, (const uint16_t*)r->vc, r->att, d.n_head, d.n_kv_head, hd, d.max_roll));
   // x2 = x + o(att)
   memset(&p, 0, sizeof(p));
-  p.W = (const uint16_t*)r->w.o; p.x0 = r->att; p.ldx0 = D; p.k0 = D; p.N = D; p.T = T; p.y = r->x2; p.ldy = D;
+  p.W[0] = (const uint16_t*)r->w.o; p.x0 = r->att; p.ldx0 = D; p.k0 = D; p.N[0] = D; p.T = T; p.y[0] = r->x2; p.ldy[0] = D;
   p.resid = r->x; p.ldr = D;
-  FB_DCUDA(r, launch_linear<DL_RESID>(p, sms, st));
+  FB_DCUDA(r, launch_linear<DL_RESID>(p, st));
   FB_DCUDA(r, launch_pdl(d_rmsnorm, dim3(T), dim3(256), 0, st, (const uint16_t*)r->x2, D, (const uint16_t*)r->w.n2, r->h, D, D, d.rms_eps));
   // act = silu(gate h) * up h
   memset(&p, 0, sizeof(p));
-  p.W = (const uint16_t*)r->w.gate; p.W2 = (const uint16_t*)r->w.up; p.x0 = r->h; p.ldx0 = D; p.k0 = D; p.N = d.inter; p.T = T;
-  p.y = r->act; p.ldy = d.inter;
-  FB_DCUDA(r, launch_linear<DL_SWIGLU>(p, sms, st));
+  p.W[0] = (const uint16_t*)r->w.gate; p.W2 = (const uint16_t*)r->w.up; p.x0 = r->h; p.ldx0 = D; p.k0 = D; p.N[0] = d.inter; p.T = T;
+  p.y[0] = r->act; p.ldy[0] = d.inter;
+  FB_DCUDA(r, launch_linear<DL_SWIGLU>(p, st));
   // hh = x2 + down(act)
   memset(&p, 0, sizeof(p));
-  p.W = (const uint16_t*)r->w.down; p.x0 = r->act; p.ldx0 = d.inter; p.k0 = d.inter; p.N = D; p.T = T; p.y = r->hh; p.ldy = D;
+  p.W[0] = (const uint16_t*)r->w.down; p.x0 = r->act; p.ldx0 = d.inter; p.k0 = d.inter; p.N[0] = D; p.T = T; p.y[0] = r->hh; p.ldy[0] = D;
   p.resid = r->x2; p.ldr = D;
-  FB_DCUDA(r, launch_linear<DL_RESID>(p, sms, st));
+  FB_DCUDA(r, launch_linear<DL_RESID>(p, st));
   // out = fout(hh)
   memset(&p, 0, sizeof(p));
-  p.W = (const uint16_t*)r->w.fout; p.x0 = r->hh; p.ldx0 = D; p.k0 = D; p.N = F; p.T = T; p.y = (uint16_t*)d_out; p.ldy = F;
-  FB_DCUDA(r, launch_linear<DL_STORE>(p, sms, st));
-  (void)W;
+  p.W[0] = (const uint16_t*)r->w.fout; p.x0 = r->hh; p.ldx0 = D; p.k0 = D; p.N[0] = F; p.T = T; p.y[0] = (uint16_t*)d_out; p.ldy[0] = F;
+  FB_DCUDA(r, launch_linear<DL_STORE>(p, st));
   FB_DCUDA(r, cudaGetLastError());
   return FB_OK;
 }
@@ -238,11 +234,13 @@ int fb_draft_head(fb_draft* r, const void* d_feat_rows, int32_t n, int32_t top_b
                          d.rms_eps));
   DLin p;
   memset(&p, 0, sizeof(p));
-  p.W = (const uint16_t*)r->w.embed; p.x0 = r->fn; p.ldx0 = D; p.k0 = D; p.N = d.vocab; p.T = n; p.yf = r->logits; p.ldy = d.vocab;
+  p.W[0] = (const uint16_t*)r->w.embed; p.x0 = r->fn; p.ldx0 = D; p.k0 = D; p.N[0] = d.vocab; p.T = n; p.yf = r->logits; p.ldy[0] = d.vocab;
   p.scale = d.logits_scaling;
-  FB_DCUDA(r, launch_linear<DL_LOGITS>(p, r->sm_count, st));
-  FB_DCUDA(r, launch_pdl(topb_rows, dim3(n), dim3(1024), 0, st, (const float*)r->logits, (long long)d.vocab, d.vocab, top_b, d_tokens,
-                         d_scores));
+  FB_DCUDA(r, launch_linear<DL_LOGITS>(p, st));
+  const int nc = row_ctas(d.vocab);
+  const bool reg = (d.vocab + nc - 1) / nc <= kSampleRegs * 1024;
+  FB_DCUDA(r, launch_pdl_cluster(reg ? topb_rows<true> : topb_rows<false>, dim3(nc, n), dim3(1024), 0, st, nc, (const float*)r->logits,
+                                 (long long)d.vocab, d.vocab, top_b, d_tokens, d_scores));
   FB_DCUDA(r, cudaGetLastError());
   return FB_OK;
 }

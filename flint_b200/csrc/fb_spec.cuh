@@ -40,119 +40,227 @@ struct SampleParams {
   int32_t* out;                 // [rows] token ids
 };
 
-// One CTA per row. top-k keeps every entry >= the k-th largest value (ties included, as `logits < v[-1] -> -inf` does,
-// reference: engine/generate.py:41-45); the k-th largest is found exactly by a 4-pass radix select on order-preserving
-// keys. The draw is arg-max of logit / T + Gumbel noise, which is a sample of softmax(logits / T) over the kept
-// entries: the same distribution as arg-max(p / Exponential(1)) (reference: engine/generate.py:37-39).
-__global__ void __launch_bounds__(1024) sample_rows(const SampleParams P) {
-  __shared__ unsigned hist[256];
-  __shared__ unsigned s_bin, s_k;
-  __shared__ float s_v[32];
-  __shared__ int s_i[32];
-  const int tid = threadIdx.x, row = blockIdx.x;
-  const float* lg = P.logits + (long long)row * P.row_stride;
-  const bool draw = P.temperature > 0.f;
-  uint32_t thr = 0u;
-  if (draw && P.top_k > 0 && P.top_k < P.vocab) {
-    uint32_t prefix = 0u, mask = 0u;
-    unsigned k = (unsigned)P.top_k;
-    for (int shift = 24; shift >= 0; shift -= 8) {
-      if (tid < 256) hist[tid] = 0u;
-      __syncthreads();
-      for (int i = tid; i < P.vocab; i += 1024) {
-        const uint32_t key = fkey(lg[i]);
-        if ((key & mask) == prefix) atomicAdd(&hist[(key >> shift) & 255u], 1u);
-      }
-      __syncthreads();
-      if (tid == 0) {
-        unsigned cum = 0u;
-        int b = 255;
-        for (; b > 0; b--) {
-          if (cum + hist[b] >= k) break;
-          cum += hist[b];
-        }
-        s_bin = (unsigned)b;
-        s_k = k - cum;
-      }
-      __syncthreads();
-      prefix |= s_bin << shift;
-      mask |= 0xFFu << shift;
-      k = s_k;
-      __syncthreads();
-    }
-    thr = prefix;                                   // key of the k-th largest value
-  }
-  float bv = -INFINITY;
-  int bi = 0x7fffffff;
-  const float inv_t = draw ? 1.0f / P.temperature : 1.0f;
-  for (int i = tid; i < P.vocab; i += 1024) {
-    const float v = lg[i];
-    if (fkey(v) < thr) continue;
-    const float sc = draw ? v * inv_t + gumbel(mix32(P.seed, P.counter + (unsigned long long)row, (uint32_t)i)) : v;
-    if (sc > bv || (sc == bv && i < bi)) { bv = sc; bi = i; }
-  }
+// One cluster of CTAs per row: a CTA keeps its slice of the row in registers (up to 16 values a thread; longer slices are read again),
+// so a row is read once, by several SMs. top-k keeps every entry >= the k-th largest value (ties included, as `logits < v[-1] -> -inf`
+// does, reference: engine/generate.py:41-45); the k-th largest is found exactly by a radix select on order-preserving keys in three
+// digits of 11, 11 and 10 bits: every CTA counts its own slice and reads the others' counts from their shared memory. The draw is arg-max of logit / T + Gumbel noise,
+// which is a sample of softmax(logits / T) over the kept entries: the same distribution as arg-max(p / Exponential(1)) (reference:
+// engine/generate.py:37-39). Bound by latency: four cluster barriers and three scans. (One CTA per row took 83 us for a row of 128256
+// values and k = 50: five passes of 512 KB through one SM, most of the first digit's atomics on a handful of bins.)
+constexpr int kSampleRegs = 16;
+__device__ __forceinline__ uint32_t sm_map(uint32_t saddr, uint32_t rank) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(saddr), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ void sm_cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+}
+__device__ __forceinline__ void sm_st(uint32_t a, uint32_t v) { asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory"); }
+__device__ __forceinline__ uint2 sm_ld2(uint32_t a) {
+  uint2 v;
+  asm volatile("ld.shared::cluster.v2.u32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(a) : "memory");
+  return v;
+}
+// the better of two (value, index) pairs: larger value, then smaller index
+__device__ __forceinline__ void take_best(float& bv, int& bi, float ov, int oi) {
+  if (ov > bv || (ov == bv && oi < bi)) { bv = ov; bi = oi; }
+}
+__device__ __forceinline__ void warp_best(float& bv, int& bi) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
     const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
     const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-    if (ov > bv || (ov == bv && oi < bi)) { bv = ov; bi = oi; }
-  }
-  if ((tid & 31) == 0) { s_v[tid >> 5] = bv; s_i[tid >> 5] = bi; }
-  __syncthreads();
-  if (tid < 32) {
-    bv = s_v[tid]; bi = s_i[tid];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
-      const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-      if (ov > bv || (ov == bv && oi < bi)) { bv = ov; bi = oi; }
-    }
-    if (tid == 0) P.out[row] = bi == 0x7fffffff ? 0 : bi;
+    take_best(bv, bi, ov, oi);
   }
 }
 
-// the B best entries of every row in order (value descending, first index on ties): B rounds of a block arg-max
+// grid (CTAs per row = cluster, rows), 1024 threads
+template <bool REG>
+__global__ void __launch_bounds__(1024) sample_rows(const SampleParams P) {
+  __shared__ __align__(8) unsigned hist[3][2048];
+  __shared__ unsigned s_warp[32], s_bin, s_k;
+  __shared__ float s_v[32];
+  __shared__ int s_i[32];
+  __shared__ float c_v[16];                       // the CTAs' candidates, in the first CTA
+  __shared__ int c_i[16];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, row = blockIdx.y, C = gridDim.x, rank = blockIdx.x;
+  const float* lg = P.logits + (long long)row * P.row_stride;
+  const int per = (P.vocab + C - 1) / C, i0 = rank * per, i1 = min(P.vocab, i0 + per);
+  const bool draw = P.temperature > 0.f, select = draw && P.top_k > 0 && P.top_k < P.vocab;
+  pdl_trigger();
+  pdl_wait();
+  float v[REG ? kSampleRegs : 1];
+  if constexpr (REG) {
+#pragma unroll
+    for (int j = 0; j < kSampleRegs; j++) v[j] = i0 + tid + j * 1024 < i1 ? lg[i0 + tid + j * 1024] : 0.f;
+  }
+  auto each = [&](auto f) {
+    if constexpr (REG) {
+#pragma unroll
+      for (int j = 0; j < kSampleRegs; j++)
+        if (i0 + tid + j * 1024 < i1) f(i0 + tid + j * 1024, v[j]);
+    } else {
+      for (int i = i0 + tid; i < i1; i += 1024) f(i, lg[i]);
+    }
+  };
+  uint32_t thr = 0u;
+  if (select) {
+    for (int i = tid; i < 2048; i += 1024) { hist[0][i] = hist[1][i] = hist[2][i] = 0u; }
+    __syncthreads();
+    uint32_t prefix = 0u, mask = 0u;
+    unsigned k = (unsigned)P.top_k;
+#pragma unroll 1
+    for (int d = 0; d < 3; d++) {
+      const int shift = d == 0 ? 21 : (d == 1 ? 10 : 0);
+      const uint32_t dmask = d == 2 ? 1023u : 2047u;
+      each([&](int, float x) {
+        const uint32_t key = fkey(x);
+        if ((key & mask) == prefix) atomicAdd(&hist[d][(key >> shift) & dmask], 1u);
+      });
+      sm_cluster_sync();
+      // thread t holds bins 2047 - 2t and 2046 - 2t: an inclusive scan in thread order counts from the largest key down
+      const uint32_t h = (uint32_t)__cvta_generic_to_shared(&hist[d][2046 - 2 * tid]);
+      unsigned b0 = 0u, b1 = 0u;
+#pragma unroll
+      for (int c = 0; c < 8; c++)
+        if (c < C) {
+          const uint2 u = sm_ld2(sm_map(h, c));
+          b0 += u.x;
+          b1 += u.y;
+        }
+      unsigned s = b1 + b0;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const unsigned u = __shfl_up_sync(0xffffffffu, s, o);
+        if (lane >= o) s += u;
+      }
+      if (lane == 31) s_warp[warp] = s;
+      __syncthreads();
+      if (warp == 0) {
+        unsigned w = s_warp[lane];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const unsigned u = __shfl_up_sync(0xffffffffu, w, o);
+          if (lane >= o) w += u;
+        }
+        s_warp[lane] = w;
+      }
+      __syncthreads();
+      const unsigned before = s - b1 - b0 + (warp ? s_warp[warp - 1] : 0u);      // entries in larger bins
+      if (before < k && before + b1 >= k) { s_bin = 2047 - 2 * tid; s_k = k - before; }
+      else if (before + b1 < k && before + b1 + b0 >= k) { s_bin = 2046 - 2 * tid; s_k = k - before - b1; }
+      __syncthreads();
+      prefix |= s_bin << shift;
+      mask |= dmask << shift;
+      k = s_k;
+    }
+    thr = prefix;                                 // key of the k-th largest value
+  }
+  float bv = -INFINITY;
+  int bi = 0x7fffffff;
+  const float inv_t = draw ? 1.0f / P.temperature : 1.0f;
+  each([&](int i, float x) {
+    if (fkey(x) < thr) return;
+    const float sc = draw ? x * inv_t + gumbel(mix32(P.seed, P.counter + (unsigned long long)row, (uint32_t)i)) : x;
+    take_best(bv, bi, sc, i);
+  });
+  warp_best(bv, bi);
+  if (lane == 0) { s_v[warp] = bv; s_i[warp] = bi; }
+  __syncthreads();
+  if (warp == 0) {
+    bv = s_v[lane]; bi = s_i[lane];
+    warp_best(bv, bi);
+    if (lane == 0) {
+      sm_st(sm_map((uint32_t)__cvta_generic_to_shared(c_v + rank), 0), __float_as_uint(bv));
+      sm_st(sm_map((uint32_t)__cvta_generic_to_shared(c_i + rank), 0), (uint32_t)bi);
+    }
+  }
+  sm_cluster_sync();
+  if (rank == 0 && warp == 0) {
+    bv = lane < C ? c_v[lane] : -INFINITY;
+    bi = lane < C ? c_i[lane] : 0x7fffffff;
+    warp_best(bv, bi);
+    if (lane == 0) P.out[row] = bi == 0x7fffffff ? 0 : bi;
+  }
+}
+
+// The B best entries of every row in order (value descending, first index on ties). One cluster per row: every CTA picks the B best of
+// its slice in B rounds of a block arg-max over registers, the first CTA picks the B best of the candidates. grid (cluster, rows)
+template <bool REG>
 __global__ void __launch_bounds__(1024) topb_rows(const float* logits, long long row_stride, int vocab, int B, int32_t* out_idx,
                                                   float* out_val) {
   __shared__ float s_v[32];
-  __shared__ int s_i[32];
-  __shared__ int chosen[16];
-  const int tid = threadIdx.x, row = blockIdx.x;
+  __shared__ int s_i[32], s_pick;
+  __shared__ float c_v[16 * 16];
+  __shared__ int c_i[16 * 16];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, row = blockIdx.y, C = gridDim.x, rank = blockIdx.x;
   const float* lg = logits + (long long)row * row_stride;
+  const int per = (vocab + C - 1) / C, i0 = rank * per, i1 = min(vocab, i0 + per);
   pdl_trigger();
   pdl_wait();
+  float v[REG ? kSampleRegs : 1];
+  unsigned taken = 0u;                            // this thread's entries that were picked already
+  if constexpr (REG) {
+#pragma unroll
+    for (int j = 0; j < kSampleRegs; j++) {
+      const int i = i0 + tid + j * 1024;
+      v[j] = i < i1 ? lg[i] : 0.f;
+      if (i >= i1) taken |= 1u << j;
+    }
+  }
+  float pv = INFINITY;                            // longer slices: the pick of the last round; later picks come after it in order
+  int pi = -1;
   for (int r = 0; r < B; r++) {
     float bv = -INFINITY;
     int bi = 0x7fffffff;
-    for (int i = tid; i < vocab; i += 1024) {
-      bool taken = false;
-      for (int j = 0; j < r; j++) taken = taken || (chosen[j] == i);
-      const float v = lg[i];
-      if (!taken && (v > bv || (v == bv && i < bi))) { bv = v; bi = i; }
-    }
+    if constexpr (REG) {
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
-      const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-      if (ov > bv || (ov == bv && oi < bi)) { bv = ov; bi = oi; }
-    }
-    if ((tid & 31) == 0) { s_v[tid >> 5] = bv; s_i[tid >> 5] = bi; }
-    __syncthreads();
-    if (tid < 32) {
-      bv = s_v[tid]; bi = s_i[tid];
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
-        const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-        if (ov > bv || (ov == bv && oi < bi)) { bv = ov; bi = oi; }
+      for (int j = 0; j < kSampleRegs; j++)
+        if (!(taken >> j & 1u)) take_best(bv, bi, v[j], i0 + tid + j * 1024);
+    } else {
+      for (int i = i0 + tid; i < i1; i += 1024) {
+        const float x = lg[i];
+        if (x < pv || (x == pv && i > pi)) take_best(bv, bi, x, i);
       }
-      if (tid == 0) {
-        chosen[r] = bi;
+    }
+    warp_best(bv, bi);
+    if (lane == 0) { s_v[warp] = bv; s_i[warp] = bi; }
+    __syncthreads();
+    if (warp == 0) {
+      bv = s_v[lane]; bi = s_i[lane];
+      warp_best(bv, bi);
+      if (lane == 0) {
+        s_pick = bi;
+        s_v[0] = bv;
+        sm_st(sm_map((uint32_t)__cvta_generic_to_shared(c_v + rank * B + r), 0), __float_as_uint(bv));
+        sm_st(sm_map((uint32_t)__cvta_generic_to_shared(c_i + rank * B + r), 0), (uint32_t)bi);
+      }
+    }
+    __syncthreads();
+    pi = s_pick;
+    pv = s_v[0];
+    const int loc = pi - i0 - tid;
+    if (REG && pi != 0x7fffffff && loc >= 0 && (loc & 1023) == 0) taken |= 1u << (loc >> 10);
+    __syncthreads();
+  }
+  sm_cluster_sync();
+  if (rank == 0 && warp == 0) {
+    unsigned used = 0u;                           // lane l looks at candidates l, l + 32, ... (at most 256: 8 each)
+    for (int r = 0; r < B; r++) {
+      float bv = -INFINITY;
+      int bi = 0x7fffffff, bc = 0;
+      for (int c = lane, j = 0; c < C * B; c += 32, j++)
+        if (!(used >> j & 1u) && (c_v[c] > bv || (c_v[c] == bv && c_i[c] < bi))) { bv = c_v[c]; bi = c_i[c]; bc = j; }
+      const int own = bi;
+      warp_best(bv, bi);
+      if (own == bi && bi != 0x7fffffff) used |= 1u << bc;
+      if (lane == 0) {
         out_idx[(size_t)row * B + r] = bi == 0x7fffffff ? 0 : bi;
         if (out_val) out_val[(size_t)row * B + r] = bv;
       }
     }
-    __syncthreads();
   }
 }
 
@@ -203,101 +311,158 @@ __global__ void kv_compact(uint16_t* kc, uint16_t* vc, const int32_t* acc, int p
 }
 
 // ------------------------------------------------------------------------------------------------ draft head
-__device__ __forceinline__ float dot8(const uint4& w, const uint4& x, float acc) {
-  acc = fmaf(bflo(w.x), bflo(x.x), acc); acc = fmaf(bfhi(w.x), bfhi(x.x), acc);
-  acc = fmaf(bflo(w.y), bflo(x.y), acc); acc = fmaf(bfhi(w.y), bfhi(x.y), acc);
-  acc = fmaf(bflo(w.z), bflo(x.z), acc); acc = fmaf(bfhi(w.z), bfhi(x.z), acc);
-  acc = fmaf(bflo(w.w), bflo(x.w), acc); acc = fmaf(bfhi(w.w), bfhi(x.w), acc);
-  return acc;
-}
-
 enum { DL_STORE = 0, DL_RESID = 1, DL_SWIGLU = 2, DL_LOGITS = 3 };
 
 struct DLin {
-  const uint16_t* W;            // bf16 [N, K] (torch Linear layout), K = k0 + k1
-  const uint16_t* W2;           // DL_SWIGLU: the `up` matrix, same shape
+  const uint16_t* W[3];         // bf16 [N, K] (torch Linear layout), K = k0 + k1; up to three matrices over the same input (q, k, v)
+  const uint16_t* W2;           // DL_SWIGLU: the `up` matrix, same shape as W[0]
   const uint16_t* x0;           // first input segment: bf16 rows of k0 elements, ldx0 apart
   const uint16_t* x1;           // second segment (k1 elements, ldx1 apart) or nullptr: the input is cat(x0, x1)
   const int32_t* x1_tokens;     // when set, segment 1 of token t is row x1_tokens[t] of x1 (an embedding table); < 0: zeros
   int ldx0, ldx1, k0, k1;
-  int N, T;
-  uint16_t* y;                  // bf16 [T, N] rows ldy apart (STORE / RESID / SWIGLU)
+  int N[3], T;
+  uint16_t* y[3];               // bf16 [T, N] rows ldy apart (STORE / RESID / SWIGLU)
   const uint16_t* resid;        // DL_RESID: y = bf16(resid + bf16(acc)), rows ldr apart
   float* yf;                    // DL_LOGITS: f32 [T, N] = bf16(bf16(acc) / scale), rows ldy apart
-  int ldy, ldr;
+  int ldy[3], ldr;
   float scale;
 };
 
-// y[t, n] = sum_k W[n, k] x[t, k] for TT tokens t0 .. t0+TT-1 at a time: the tokens' inputs sit in shared memory, a warp
-// owns output row n and streams it with 16-byte loads. Weights are read once per TT tokens.
-template <int TT, int MODE>
-__global__ void __launch_bounds__(256) d_linear(const DLin P, int t0) {
-  extern __shared__ __align__(16) uint16_t d_xs[];
-  const int K = P.k0 + P.k1, KV = K >> 3;
-  const int tid = threadIdx.x, lane = tid & 31;
-  pdl_trigger();
-  pdl_wait();
-  for (int idx = tid; idx < TT * KV; idx += 256) {
-    const int t = idx / KV, c = (idx % KV) << 3, tok = t0 + t;
-    uint4 v = make_uint4(0, 0, 0, 0);
-    if (tok < P.T) {
-      if (c < P.k0) {
-        v = *reinterpret_cast<const uint4*>(P.x0 + (size_t)tok * P.ldx0 + c);
-      } else if (P.x1_tokens) {
-        const int id = P.x1_tokens[tok];
-        if (id >= 0) v = *reinterpret_cast<const uint4*>(P.x1 + (size_t)id * P.ldx1 + (c - P.k0));
-      } else {
-        v = *reinterpret_cast<const uint4*>(P.x1 + (size_t)tok * P.ldx1 + (c - P.k0));
-      }
+// y[t, n] = sum_k W[n, k] x[t, k] for up to 8 NT tokens (t0 ...) on the tensor pipe, weights read once. A CTA takes 16 MT rows of W and
+// its WARPS warps share K: warp w takes the 32-column chunks w, w + WARPS, ... A lane loads 16 bytes of row g (and g + 8) straight into
+// the A fragments of two MMA steps -- the order of columns inside a chunk does not matter as long as x is read the same way, 16 bytes of
+// token g at the same columns -- so nothing goes through shared memory but the warps' partial sums. HBM-bound: a warp keeps AH chunks of
+// weights and activations in flight; the first weights are requested before the previous kernel is waited for. (The CUDA-core form
+// read the weights once per 8 or 16 tokens and took 62 us for a 13 to 50 MB matrix at 32 tokens.)
+template <int NT, int MT, int WARPS, int MODE, bool CAT>
+__global__ void __launch_bounds__(WARPS * 32) d_gemm(const DLin P, int t0) {
+  constexpr int NW = MODE == DL_SWIGLU ? 2 : 1, AH = NT == 1 ? 4 : 2, ROWS = 16 * MT * NW;      // weight matrices per row, chunks in flight
+  __shared__ float red[8][ROWS][8 * NT + 1];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+  const int K = P.k0 + P.k1, nch = (K + 31) >> 5;
+  int blk = blockIdx.x, which = 0;
+  if (MODE == DL_STORE) {
+#pragma unroll
+    for (int i = 0; i < 2; i++) {
+      const int nb = (P.N[which] + 16 * MT - 1) / (16 * MT);
+      if (P.W[which + 1] && blk >= nb) { blk -= nb; which++; }
+      else break;
     }
-    *reinterpret_cast<uint4*>(d_xs + (size_t)t * K + c) = v;
   }
-  __syncthreads();
-  const int warp = blockIdx.x * 8 + (tid >> 5), nwarps = gridDim.x * 8;
-  for (int n = warp; n < P.N; n += nwarps) {
-    float acc[TT], acc2[TT];
+  const int N = P.N[which], r0 = blk * 16 * MT;
+  const uint16_t* wr[NW][MT][2];
 #pragma unroll
-    for (int t = 0; t < TT; t++) acc[t] = acc2[t] = 0.f;
-    const uint4* wr = reinterpret_cast<const uint4*>(P.W + (size_t)n * K);
-    const uint4* wr2 = MODE == DL_SWIGLU ? reinterpret_cast<const uint4*>(P.W2 + (size_t)n * K) : nullptr;
-    // few tokens leave registers for more loads in flight per warp: a GEMV of 2560 rows gives an SM only ~17 warps
-    constexpr int UNR = TT <= 2 ? 8 : (TT <= 4 ? 4 : 2);
-#pragma unroll UNR
-    for (int c = lane; c < KV; c += 32) {
-      const uint4 w = __ldg(wr + c);
-      uint4 w2 = make_uint4(0, 0, 0, 0);
-      if (MODE == DL_SWIGLU) w2 = __ldg(wr2 + c);
+  for (int m = 0; m < MT; m++)
 #pragma unroll
-      for (int t = 0; t < TT; t++) {
-        const uint4 xv = *reinterpret_cast<const uint4*>(d_xs + (size_t)t * K + (c << 3));
-        acc[t] = dot8(w, xv, acc[t]);
-        if (MODE == DL_SWIGLU) acc2[t] = dot8(w2, xv, acc2[t]);
-      }
+    for (int h = 0; h < 2; h++) {
+      const size_t row = (size_t)min(r0 + m * 16 + h * 8 + g, N - 1) * K + 8 * t;
+      wr[0][m][h] = P.W[which] + row;
+      if (NW > 1) wr[NW - 1][m][h] = P.W2 + row;
     }
+  uint4 wv[AH][NW][MT][2], xv[AH][NT];
+  auto load_w = [&](int c, uint4 (&d)[NW][MT][2]) {
+    const bool ok = c < nch && c * 32 + 8 * t < K;
 #pragma unroll
-    for (int t = 0; t < TT; t++) {
+    for (int i = 0; i < NW; i++)
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        acc[t] += __shfl_xor_sync(0xffffffffu, acc[t], o);
-        if (MODE == DL_SWIGLU) acc2[t] += __shfl_xor_sync(0xffffffffu, acc2[t], o);
-      }
+      for (int m = 0; m < MT; m++)
+#pragma unroll
+        for (int h = 0; h < 2; h++) d[i][m][h] = ok ? __ldcs(reinterpret_cast<const uint4*>(wr[i][m][h] + c * 32)) : make_uint4(0, 0, 0, 0);
+  };
+  pdl_trigger();
+#pragma unroll
+  for (int a = 0; a < AH; a++) load_w(warp + WARPS * a, wv[a]);
+  pdl_wait();
+  const uint16_t *xp0[NT], *xp1[CAT ? NT : 1];
+#pragma unroll
+  for (int j = 0; j < NT; j++) {
+    const int tok = t0 + j * 8 + g;
+    const bool live = tok < P.T;
+    xp0[j] = live ? P.x0 + (size_t)tok * P.ldx0 + 8 * t : nullptr;
+    if (CAT) {
+      const int id = live ? (P.x1_tokens ? P.x1_tokens[tok] : tok) : -1;
+      xp1[j] = id >= 0 ? P.x1 + (size_t)id * P.ldx1 + 8 * t - P.k0 : nullptr;
     }
-    if (lane == 0) {
+  }
+  auto load_x = [&](int c, uint4 (&d)[NT]) {
+    const int col = c * 32 + 8 * t;
 #pragma unroll
-      for (int t = 0; t < TT; t++) {
-        const int tok = t0 + t;
-        if (tok >= P.T) break;
-        if (MODE == DL_STORE) {
-          P.y[(size_t)tok * P.ldy + n] = f2bf(acc[t]);
-        } else if (MODE == DL_RESID) {
-          P.y[(size_t)tok * P.ldy + n] = f2bf(bf2f(P.resid[(size_t)tok * P.ldr + n]) + rbf(acc[t]));
-        } else if (MODE == DL_SWIGLU) {
-          const float g = rbf(acc[t]), u = rbf(acc2[t]);
-          P.y[(size_t)tok * P.ldy + n] = f2bf(rbf(g / (1.0f + expf(-g))) * u);
-        } else {
-          P.yf[(size_t)tok * P.ldy + n] = rbf(rbf(acc[t]) / P.scale);
+    for (int j = 0; j < NT; j++) {
+      const uint16_t* xp = CAT && col >= P.k0 ? xp1[CAT ? j : 0] : xp0[j];
+      d[j] = xp && col < K ? *reinterpret_cast<const uint4*>(xp + c * 32) : make_uint4(0, 0, 0, 0);
+    }
+  };
+#pragma unroll
+  for (int a = 0; a < AH; a++) load_x(warp + WARPS * a, xv[a]);
+  float acc[NW][MT][NT][4];
+#pragma unroll
+  for (int i = 0; i < NW; i++)
+#pragma unroll
+    for (int m = 0; m < MT; m++)
+#pragma unroll
+      for (int j = 0; j < NT; j++) acc[i][m][j][0] = acc[i][m][j][1] = acc[i][m][j][2] = acc[i][m][j][3] = 0.f;
+  for (int c0 = warp; c0 < nch; c0 += WARPS * AH) {
+#pragma unroll
+    for (int a = 0; a < AH; a++) {                   // chunks past the end multiply zeros
+      const int c = c0 + WARPS * a;
+#pragma unroll
+      for (int i = 0; i < NW; i++)
+#pragma unroll
+        for (int m = 0; m < MT; m++) {
+          const uint4 lo = wv[a][i][m][0], hi = wv[a][i][m][1];
+          const uint32_t a0[4] = {lo.x, hi.x, lo.y, hi.y}, a1[4] = {lo.z, hi.z, lo.w, hi.w};
+#pragma unroll
+          for (int j = 0; j < NT; j++) {
+            mma_bf16(acc[i][m][j], a0, xv[a][j].x, xv[a][j].y);
+            mma_bf16(acc[i][m][j], a1, xv[a][j].z, xv[a][j].w);
+          }
         }
-      }
+      load_w(c + WARPS * AH, wv[a]);
+      load_x(c + WARPS * AH, xv[a]);
+    }
+  }
+  auto at = [&](int i, int m, int j, int e) -> float& {
+    return red[warp & 7][(i * MT + m) * 16 + g + 8 * (e >> 1)][j * 8 + 2 * t + (e & 1)];
+  };
+  auto each_acc = [&](auto f) {
+#pragma unroll
+    for (int i = 0; i < NW; i++)
+#pragma unroll
+      for (int m = 0; m < MT; m++)
+#pragma unroll
+        for (int j = 0; j < NT; j++)
+#pragma unroll
+          for (int e = 0; e < 4; e++) f(i, m, j, e);
+  };
+  if (WARPS > 8) {                                   // the upper eight warps' sums join the lower eight's
+    if (warp >= 8) each_acc([&](int i, int m, int j, int e) { at(i, m, j, e) = acc[i][m][j][e]; });
+    __syncthreads();
+    if (warp < 8) each_acc([&](int i, int m, int j, int e) { acc[i][m][j][e] += at(i, m, j, e); });
+    __syncthreads();
+  }
+  if (warp < 8) each_acc([&](int i, int m, int j, int e) { at(i, m, j, e) = acc[i][m][j][e]; });
+  __syncthreads();
+  for (int o = tid; o < 16 * MT * 8 * NT; o += WARPS * 32) {
+    const int r = o % (16 * MT), tk = o / (16 * MT), n = r0 + r, tok = t0 + tk;
+    if (n >= N || tok >= P.T) continue;
+    float s = 0.f, s2 = 0.f;
+#pragma unroll
+    for (int w = 0; w < 8; w++) {
+      s += red[w][r][tk];
+      if (NW > 1) s2 += red[w][16 * MT * (NW - 1) + r][tk];
+    }
+    if (MODE == DL_LOGITS) {
+      P.yf[(size_t)tok * P.ldy[0] + n] = rbf(rbf(s) / P.scale);
+      continue;
+    }
+    uint16_t* y = P.y[which] + (size_t)tok * P.ldy[which] + n;
+    if (MODE == DL_STORE) {
+      *y = f2bf(s);
+    } else if (MODE == DL_RESID) {
+      *y = f2bf(bf2f(P.resid[(size_t)tok * P.ldr + n]) + rbf(s));
+    } else {
+      const float gg = rbf(s), u = rbf(s2);
+      *y = f2bf(rbf(gg / (1.0f + expf(-gg))) * u);
     }
   }
 }
@@ -329,10 +494,13 @@ __global__ void __launch_bounds__(256) d_rmsnorm(const uint16_t* x, int ldx, con
 
 // Half-split rotation of q and k (bf16 cos / sin tables as the reference casts them, reference:
 // train/draft_model.py:12-22) and the cache write: token t's rotated k and its v go to cache slot slots[t].
-// grid (T, n_head + n_kv), 64 threads: one CTA per (token, head), a thread per rotation pair (the angle's powf / cosf /
-// sinf are the slow part: one per thread). q is rotated in place; a kv-head CTA also copies its v row.
+// grid (T, n_head + n_kv), 64 threads: one CTA per (token, head), a thread per rotation pair (the angle's cosf / sinf are the slow
+// part: one per thread). q is rotated in place; a kv-head CTA also copies its v row. invf: d_invf's table
+__global__ void d_invf(float* invf, float rope_base, int hd) {
+  for (int i = threadIdx.x; i < hd / 2; i += blockDim.x) invf[i] = 1.0f / powf(rope_base, (float)(2 * i) / (float)hd);
+}
 __global__ void d_rope_store(uint16_t* q, const uint16_t* k, const uint16_t* v, const int32_t* positions, const int32_t* slots,
-                             uint16_t* kc, uint16_t* vc, int nh, int nkv, int hd, float rope_base, int max_roll) {
+                             uint16_t* kc, uint16_t* vc, int nh, int nkv, int hd, const float* invf, int max_roll) {
   const int t = blockIdx.x, head = blockIdx.y, half = hd >> 1;
   pdl_trigger();
   pdl_wait();
@@ -340,8 +508,7 @@ __global__ void d_rope_store(uint16_t* q, const uint16_t* k, const uint16_t* v, 
   const int slot = slots ? slots[t] : t;
   if (slot < 0 || slot >= max_roll) return;
   for (int i = threadIdx.x; i < half; i += blockDim.x) {
-    const float inv = 1.0f / powf(rope_base, (float)(2 * i) / (float)hd);
-    const float ang = pos * inv;
+    const float ang = pos * invf[i];
     const float c = rbf(cosf(ang)), s = rbf(sinf(ang));
     if (head < nh) {
       uint16_t* p = q + ((size_t)t * nh + head) * hd;
@@ -368,20 +535,32 @@ __global__ void d_rope_store(uint16_t* q, const uint16_t* k, const uint16_t* v, 
 // train/draft_model.py:43,57-59). grid (T, nh), 128 threads; softmax in fp32, output bf16.
 __global__ void __launch_bounds__(128) d_attn(const uint16_t* q, const int32_t* slots, const uint16_t* kc, const uint16_t* vc,
                                               uint16_t* out, int nh, int nkv, int hd, int max_roll) {
-  extern __shared__ float d_sc[];                  // [max_roll] scores, then [hd] is not needed: threads own dims
+  extern __shared__ float d_sc[];                  // [max_roll] scores, then [hd] the query
   __shared__ float red[4];
+  float* qs = d_sc + max_roll;
   const int t = blockIdx.x, head = blockIdx.y, kh = head / (nh / nkv), tid = threadIdx.x;
   pdl_trigger();
   pdl_wait();
   const int last = min(slots ? slots[t] : t, max_roll - 1);
   if (last < 0) return;
-  const uint16_t* qr = q + ((size_t)t * nh + head) * hd;
+  for (int i = tid; i < hd; i += 128) qs[i] = bf2f(q[((size_t)t * nh + head) * hd + i]);
+  __syncthreads();
   const float scale = rsqrtf((float)hd);
   float mx = -INFINITY;
   for (int s = tid; s <= last; s += 128) {
     const uint16_t* kr = kc + ((size_t)s * nkv + kh) * hd;
     float d = 0.f;
-    for (int i = 0; i < hd; i++) d = fmaf(bf2f(qr[i]), bf2f(kr[i]), d);
+    if (hd % 8 == 0) {                               // rows start on 16-byte boundaries
+#pragma unroll 4
+      for (int i = 0; i < hd; i += 8) {
+        const uint4 kv = *reinterpret_cast<const uint4*>(kr + i);
+        const uint32_t p[4] = {kv.x, kv.y, kv.z, kv.w};
+#pragma unroll
+        for (int e = 0; e < 4; e++) { d = fmaf(qs[i + 2 * e], bflo(p[e]), d); d = fmaf(qs[i + 2 * e + 1], bfhi(p[e]), d); }
+      }
+    } else {
+      for (int i = 0; i < hd; i++) d = fmaf(qs[i], bf2f(kr[i]), d);
+    }
     d *= scale;
     d_sc[s] = d;
     mx = fmaxf(mx, d);
@@ -405,6 +584,7 @@ __global__ void __launch_bounds__(128) d_attn(const uint16_t* q, const int32_t* 
   den = red[0] + red[1] + red[2] + red[3];
   for (int i = tid; i < hd; i += 128) {
     float a = 0.f;
+#pragma unroll 8
     for (int s = 0; s <= last; s++) a = fmaf(d_sc[s], bf2f(vc[((size_t)s * nkv + kh) * hd + i]), a);
     out[((size_t)t * nh + head) * hd + i] = f2bf(a / den);
   }

@@ -17,11 +17,11 @@ from .config import ModelArgs
 
 
 def _ptr(t: Optional[torch.Tensor]):
-    return None if t is None else ctypes.c_void_p(t.data_ptr())
+    return None if t is None else t.data_ptr()          # the prototypes say void*: ctypes takes the integer
 
 
-def _stream_ptr(device) -> ctypes.c_void_p:
-    return ctypes.c_void_p(torch.cuda.current_stream(device).cuda_stream)
+def _stream_ptr(device) -> int:
+    return torch.cuda.current_stream(device).cuda_stream
 
 
 def query(device: int = 0) -> Dict[str, int]:
