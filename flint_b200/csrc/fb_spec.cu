@@ -18,7 +18,6 @@ struct fb_draft {
   uint16_t *x, *h, *q, *k, *v, *att, *x2, *act, *hh, *fn;     // [max_tokens] rows of activations
   uint16_t *kc, *vc;                                           // [max_roll, n_kv, hd]
   float* logits;                                               // [max_heads rows, vocab]
-  float* invf;                                                 // [hd / 2] rotation frequencies
   int last_cuda_error;
 };
 
@@ -34,7 +33,7 @@ cudaError_t launch_linear_nt(const DLin& p, int t0, cudaStream_t st) {
   return launch_pdl(d_gemm<NT, MT, WARPS, MODE, false>, dim3(grid), dim3(WARPS * 32), 0, st, p, t0);
 }
 // All T tokens, up to 32 per pass over the weights. Up to 8 tokens: 16 rows per CTA (the matrices of a layer then give every SM at least
-// one), 32 for the token head, whose 49 000 rows and more do not need it. More tokens: 32 rows per CTA (one matrix) or 16 of each of
+// one) and three CTAs per SM. More tokens: 32 rows per CTA (one matrix) or 16 of each of
 // two, so that a CTA reads about as many bytes of activations from L2 as of weights, and 16 warps to share a long K.
 template <int MODE>
 cudaError_t launch_linear(const DLin& p, cudaStream_t st) {
@@ -43,7 +42,7 @@ cudaError_t launch_linear(const DLin& p, cudaStream_t st) {
   cudaError_t e = cudaSuccess;
   for (int t0 = 0; t0 < p.T && e == cudaSuccess; t0 += 32) {
     const int left = p.T - t0;
-    if (left <= 8) e = launch_linear_nt<1, MODE == DL_LOGITS ? 2 : 1, 8, MODE>(p, t0, st);
+    if (left <= 8) e = launch_linear_nt<1, 1, 8, MODE>(p, t0, st);
     else if (left <= 16) e = launch_linear_nt<2, MW, 16, MODE>(p, t0, st);
     else e = launch_linear_nt<4, MW, 16, MODE>(p, t0, st);
   }
@@ -131,15 +130,9 @@ int fb_draft_create(const fb_draft_desc* desc, int device, fb_draft** out) {
   A(dmalloc(&r->fn, (size_t)kMaxHeadRows * D * 2));
   A(dmalloc(&r->kc, (size_t)d.max_roll * kvd * 2)); A(dmalloc(&r->vc, (size_t)d.max_roll * kvd * 2));
   A(dmalloc(&r->logits, (size_t)kMaxHeadRows * d.vocab * 4));
-  A(dmalloc(&r->invf, (size_t)hd * 2));
   if (e == cudaSuccess) A(cudaMemset(r->kc, 0, (size_t)d.max_roll * kvd * 2));
   if (e == cudaSuccess) A(cudaMemset(r->vc, 0, (size_t)d.max_roll * kvd * 2));
   (void)F;
-  if (e == cudaSuccess) {
-    d_invf<<<1, 64>>>(r->invf, d.rope_base, hd);
-    A(cudaGetLastError());
-    A(cudaDeviceSynchronize());                    // the streams of the calls do not wait for this one
-  }
   if (e != cudaSuccess) { fb_draft_destroy(r); return FB_ERR_CUDA; }
   *out = r;
   return FB_OK;
@@ -148,7 +141,7 @@ int fb_draft_create(const fb_draft_desc* desc, int device, fb_draft** out) {
 int fb_draft_destroy(fb_draft* r) {
   if (!r) return FB_ERR_ARG;
   DeviceGuard g(r->device);
-  void* ptrs[] = {r->x, r->h, r->q, r->k, r->v, r->att, r->x2, r->act, r->hh, r->fn, r->kc, r->vc, r->logits, r->invf};
+  void* ptrs[] = {r->x, r->h, r->q, r->k, r->v, r->att, r->x2, r->act, r->hh, r->fn, r->kc, r->vc, r->logits};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   delete r;
@@ -193,7 +186,7 @@ int fb_draft_forward(fb_draft* r, const void* d_feat, const void* d_emb, const i
   p.x0 = r->h; p.ldx0 = D; p.k0 = D; p.T = T;
   FB_DCUDA(r, launch_linear<DL_STORE>(p, st));
   FB_DCUDA(r, launch_pdl(d_rope_store, dim3(T, d.n_head + d.n_kv_head), dim3(64), 0, st, r->q, (const uint16_t*)r->k, (const uint16_t*)r->v, d_positions,
-                         d_slots, r->kc, r->vc, d.n_head, d.n_kv_head, hd, (const float*)r->invf, d.max_roll));
+                         d_slots, r->kc, r->vc, d.n_head, d.n_kv_head, hd, d.rope_base, d.max_roll));
   FB_DCUDA(r, launch_pdl(d_attn, dim3(T, d.n_head), dim3(128), (size_t)(d.max_roll + hd) * 4, st, (const uint16_t*)r->q, d_slots,
                          (const uint16_t*)r->kc, (const uint16_t*)r->vc, r->att, d.n_head, d.n_kv_head, hd, d.max_roll));
   // x2 = x + o(att)

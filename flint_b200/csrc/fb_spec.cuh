@@ -335,8 +335,8 @@ struct DLin {
 // weights and activations in flight; the first weights are requested before the previous kernel is waited for. (The CUDA-core form
 // read the weights once per 8 or 16 tokens and took 62 us for a 13 to 50 MB matrix at 32 tokens.)
 template <int NT, int MT, int WARPS, int MODE, bool CAT>
-__global__ void __launch_bounds__(WARPS * 32) d_gemm(const DLin P, int t0) {
-  constexpr int NW = MODE == DL_SWIGLU ? 2 : 1, AH = NT == 1 ? 4 : 2, ROWS = 16 * MT * NW;      // weight matrices per row, chunks in flight
+__global__ void __launch_bounds__(WARPS * 32, NT == 1 ? 3 : 1) d_gemm(const DLin P, int t0) {
+  constexpr int NW = MODE == DL_SWIGLU ? 2 : 1, AH = NT == 1 && NW == 1 ? 4 : 2, ROWS = 16 * MT * NW;      // weight matrices per row, chunks in flight
   __shared__ float red[8][ROWS][8 * NT + 1];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
   const int K = P.k0 + P.k1, nch = (K + 31) >> 5;
@@ -494,13 +494,10 @@ __global__ void __launch_bounds__(256) d_rmsnorm(const uint16_t* x, int ldx, con
 
 // Half-split rotation of q and k (bf16 cos / sin tables as the reference casts them, reference:
 // train/draft_model.py:12-22) and the cache write: token t's rotated k and its v go to cache slot slots[t].
-// grid (T, n_head + n_kv), 64 threads: one CTA per (token, head), a thread per rotation pair (the angle's cosf / sinf are the slow
-// part: one per thread). q is rotated in place; a kv-head CTA also copies its v row. invf: d_invf's table
-__global__ void d_invf(float* invf, float rope_base, int hd) {
-  for (int i = threadIdx.x; i < hd / 2; i += blockDim.x) invf[i] = 1.0f / powf(rope_base, (float)(2 * i) / (float)hd);
-}
+// grid (T, n_head + n_kv), 64 threads: one CTA per (token, head), a thread per rotation pair (the angle's powf / cosf / sinf are the
+// slow part: one per thread). q is rotated in place; a kv-head CTA also copies its v row.
 __global__ void d_rope_store(uint16_t* q, const uint16_t* k, const uint16_t* v, const int32_t* positions, const int32_t* slots,
-                             uint16_t* kc, uint16_t* vc, int nh, int nkv, int hd, const float* invf, int max_roll) {
+                             uint16_t* kc, uint16_t* vc, int nh, int nkv, int hd, float rope_base, int max_roll) {
   const int t = blockIdx.x, head = blockIdx.y, half = hd >> 1;
   pdl_trigger();
   pdl_wait();
@@ -508,7 +505,8 @@ __global__ void d_rope_store(uint16_t* q, const uint16_t* k, const uint16_t* v, 
   const int slot = slots ? slots[t] : t;
   if (slot < 0 || slot >= max_roll) return;
   for (int i = threadIdx.x; i < half; i += blockDim.x) {
-    const float ang = pos * invf[i];
+    const float inv = 1.0f / powf(rope_base, (float)(2 * i) / (float)hd);
+    const float ang = pos * inv;
     const float c = rbf(cosf(ang)), s = rbf(sinf(ang));
     if (head < nh) {
       uint16_t* p = q + ((size_t)t * nh + head) * hd;
