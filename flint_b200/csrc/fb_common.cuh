@@ -134,6 +134,18 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* b, uint32_t parity, const Wa
   return false;
 }
 
+// The same out of line, for the decode kernel, whose per-layer code does not fit the instruction cache: what a healthy step
+// never executes stays out of the way.
+inline __device__ __noinline__ void report_fail_far(const WaitCtl c, int where, int layer, int expected, int seen) {
+  report_fail(c, where, layer, expected, seen);
+}
+inline __device__ __noinline__ bool mbar_wait_slow(uint64_t* b, uint32_t parity, const WaitCtl c, int where, int layer) {
+  return mbar_wait(b, parity, c, where, layer);
+}
+__device__ __forceinline__ bool mbar_wait_far(uint64_t* b, uint32_t parity, const WaitCtl& c, int where, int layer) {
+  return mbar_try(b, parity) || mbar_wait_slow(b, parity, c, where, layer);
+}
+
 // ------------------------------------------------------------------------------------------------ streaming layout
 // Weights are stored as TILES of RT consecutive stream rows x all K columns, laid out for the tensor pipe: a tile is
 // a sequence of "steps", 128 bytes each = one 32-bit word per lane of a warp, and a step is exactly the A operand of one
@@ -500,13 +512,14 @@ __device__ __forceinline__ void tile_dot_rolled(const uint8_t* tile, int slice, 
     block(false, left > 4);
     flush(true);
   }
+  if (NB % 4 != 0)
 #pragma unroll 1
   for (; left >= 2; left -= 2) {
     block(true, true);
     block(false, left > 2);
     flush(true);
   }
-  if (left) {                                                    // first half of a round the next slice closes
+  if (NB % 2 != 0 && left) {                                     // first half of a round the next slice closes
     block(true, false);
     flush(false);
   }

@@ -38,9 +38,7 @@ struct fb_ctx {
   unsigned* gu_norms;                                               // [n_layer][2] largest squared row norms of gate and up (float bits)
   void* vrope;                                                      // verify: (cos, sin) per (token, rotation pair)
   int max_fly, poll_words;
-  CUtensorMap kmap, vmap;                                           // the caches as tensors for the long-cache variant
-  bool kv_maps;
-  int long_kv;                                                      // 0: long-cache decode variant by cached length, 1: always (where built), 2: never
+  CUtensorMap kmap, vmap;                                           // the caches as tensors (make_kv_maps)
 };
 
 inline int cuda_fail(fb_ctx* c, cudaError_t e) {

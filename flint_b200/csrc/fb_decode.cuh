@@ -14,27 +14,20 @@
 
 #include "fb_pipe.cuh"
 
-#ifndef FB_ATTN_BATCH
-#define FB_ATTN_BATCH 2      // K/V positions a lane group loads before it uses any of them
-#endif
-#ifndef FB_ATTN_PFD
-#define FB_ATTN_PFD 2        // rounds ahead of its loads that a warp asks L2 for its K/V rows
-#endif
-
 namespace fb {
 
-// GQA flash-decode geometry: a row of K or V (HD bf16) is spread over HD/8 lanes (16 bytes each); a warp handles
-// 32/SEG positions per step. The R query heads of a group share every K/V load.
-template <int HD, int R>
+// K/V rows travel through the weight ring: NPS positions per stage, K rows first, then V rows. Head dimensions that are whole
+// multiples of 64 are cut into column blocks of 64 (128 bytes, the swizzle width), [block][position][64] each, so that the eight
+// rows of an 8x8 matrix load lie in different banks (unswizzled rows of 128 or 256 bytes all start in the same bank: 8 times
+// the shared-memory cycles); other head dimensions keep whole rows (160 bytes for 80: two rows per bank group).
+template <int HD>
 struct AttnCfg {
-  static constexpr int LPR = HD / 8;
-  static constexpr int SEG = LPR <= 8 ? 8 : 16;
-  static constexpr int PPW = 32 / SEG;
-  // long caches: K/V rows travel through the weight ring, NPS positions per stage (K rows, then V rows)
   static constexpr int NPS = 2 * 64 * HD * 2 <= kStageBytes ? 64 : 32;
-  static constexpr int KV_STAGE_BYTES = 2 * NPS * HD * 2;
-  static_assert(HD % 8 == 0 && LPR <= 16, "head_dim must be a multiple of 8 and <= 128");
-  static_assert(KV_STAGE_BYTES <= kStageBytes && (HD * 2) % 16 == 0, "a ring stage holds one sweep of K and V rows");
+  static constexpr int MATRIX_BYTES = NPS * HD * 2, KV_STAGE_BYTES = 2 * MATRIX_BYTES;
+  static constexpr bool SPLIT = HD % 64 == 0;
+  static constexpr int BLKS = SPLIT ? HD / 64 : 1, BCOLS = SPLIT ? 64 : HD, ROWB = BCOLS * 2;
+  static_assert(HD % 8 == 0 && HD <= 128, "head_dim must be a multiple of 8 and <= 128");
+  static_assert(KV_STAGE_BYTES <= kStageBytes && MATRIX_BYTES % 128 == 0, "a ring stage holds one sweep of K and V rows");
 };
 
 // ------------------------------------------------------------------------------------------------ tagged words
@@ -65,13 +58,28 @@ __device__ __forceinline__ void ll_load2_sys(const uint64_t* p, uint64_t& a, uin
 }
 // bounded poll of one word written by another GPU; returns the payload (0 after a failure)
 __device__ __forceinline__ uint32_t ll_poll_sys(const uint64_t* p, uint32_t tag, const WaitCtl& wc, int layer) {
+#pragma unroll 1
   for (unsigned spin = 0;; spin++) {
     const uint64_t v = ll_load_sys(p);
     if ((uint32_t)(v >> 32) == tag) return (uint32_t)v;
     if (*wc.s_abort) return 0;
     if ((spin & 255) == 255 && ld_volatile_s32(&wc.st->abort)) { *wc.s_abort = 1; return 0; }
-    if (spin >= wc.limit) { report_fail(wc, W_FLAG, layer, (int)tag, -3); return 0; }
+    if (spin >= wc.limit) { report_fail_far(wc, W_FLAG, layer, (int)tag, -3); return 0; }
   }
+}
+
+// 16 bytes = two tagged words in one store (each word carries its own tag)
+__device__ __forceinline__ void ll_store2(uint64_t* p, uint32_t pay0, uint32_t pay1, uint32_t tag) {
+  const uint64_t a = ((uint64_t)tag << 32) | pay0, b = ((uint64_t)tag << 32) | pay1;
+  asm volatile("st.relaxed.gpu.global.v2.u64 [%0], {%1, %2};" ::"l"(p), "l"(a), "l"(b) : "memory");
+}
+// one round of a bounded poll went by without the word: true = give up (abort seen or limit reached)
+inline __device__ __noinline__ bool poll_again(unsigned spin, const WaitCtl wc, int layer, int expected, int seen) {
+  if (*wc.s_abort) return true;
+  if (spin > 16) __nanosleep(40);
+  if ((spin & 255) == 255 && ld_volatile_s32(&wc.st->abort)) { *wc.s_abort = 1; return true; }
+  if (spin >= wc.limit) { report_fail_far(wc, W_FLAG, layer, expected, seen); return true; }
+  return false;
 }
 
 // Poll `nwords` (even, 16-byte aligned base) tagged words into 32-bit payloads dst[0..nwords). Threads
@@ -84,6 +92,7 @@ __device__ __forceinline__ void ll_gather(const uint64_t* src, int nwords, uint3
 #pragma unroll
   for (int k = 0; k < MAXP; k++)
     if (tid + k * nthreads < npairs) pending |= 1u << k;
+#pragma unroll 1
   for (unsigned spin = 0; pending; spin++) {
     uint64_t a[MAXP], b[MAXP];
 #pragma unroll
@@ -99,12 +108,7 @@ __device__ __forceinline__ void ll_gather(const uint64_t* src, int nwords, uint3
           pending &= ~(1u << k);
         }
       }
-    if (pending) {
-      if (*wc.s_abort) break;
-      if (spin > 16) __nanosleep(40);
-      if ((spin & 255) == 255 && ld_volatile_s32(&wc.st->abort)) { *wc.s_abort = 1; break; }
-      if (spin >= wc.limit) { report_fail(wc, W_FLAG, layer, (int)tag, -1); break; }
-    }
+    if (pending && poll_again(spin, wc, layer, (int)tag, -1)) break;
   }
 }
 
@@ -128,10 +132,11 @@ __device__ __forceinline__ void st_relaxed_u32(uint32_t* p, uint32_t v) {
 #define FB_FLAG_SETS 1       // poll rounds kept in flight (staggered): a posted flag is seen after ~RTT/2 + RTT/(2 sets)
 #endif
 #ifndef FB_FLAG_SLACK_DIV
-#define FB_FLAG_SLACK_DIV 3  // the gather starts when all but n / 3 producers have posted (0: wait for every flag). The tagged
+#define FB_FLAG_SLACK_DIV 2  // the gather starts when all but n / 2 producers have posted (0: wait for every flag). The tagged
 #endif                       // words of the stragglers are simply polled again by the gather, so the last flags' round trip
-                             // leaves the critical path: measured +2.6 % tokens/s at a third, +1.8 % at a sixth, -0.9 % with
-                             // no flag wait at all (every consumer polling words floods L2)
+                             // leaves the critical path. Microseconds a token at a third / a half / three quarters: 3B-class
+                             // 1060 / 1020 / 1010, 1B 395 / 390 / 386, 40 / 8 heads of 64 1017 / 1020 / 1042; no flag wait at all
+                             // is slower (every consumer polling words floods L2).
 __device__ __forceinline__ void wait_flags(const uint32_t* flags, int n, uint32_t tag, int cw, int lane, const WaitCtl& wc,
                                            int layer) {
   if (cw == 0) {
@@ -161,6 +166,7 @@ __device__ __forceinline__ void wait_flags(const uint32_t* flags, int n, uint32_
       issue(v[s]);
     }
     bool done = false;
+#pragma unroll 1
     for (unsigned spin = 0; !done; spin++) {
 #pragma unroll
       for (int s = 0; s < NS; s++) {
@@ -174,7 +180,7 @@ __device__ __forceinline__ void wait_flags(const uint32_t* flags, int n, uint32_
       if (lane == 0) {
         if (*wc.s_abort) stop = 1;
         else if ((spin & 63) == 63 && ld_volatile_s32(&wc.st->abort)) { *wc.s_abort = 1; stop = 1; }
-        else if (spin >= wc.limit) { report_fail(wc, W_FLAG, layer, (int)tag, n); stop = 1; }
+        else if (spin >= wc.limit) { report_fail_far(wc, W_FLAG, layer, (int)tag, n); stop = 1; }
       }
       if (__shfl_sync(0xffffffffu, stop, 0)) break;
     }
@@ -196,14 +202,23 @@ __device__ __forceinline__ void post_when_cta_done(int* s_done, uint32_t* flag, 
 }
 
 // ------------------------------------------------------------------------------------------------ staging from tagged vectors
-// Both functions leave the phase's activations in sm.xh / sm.xf (fp16 in B-operand order + per-group factors) and end
+// Both are real functions, one instance per kernel, not inlined at their five call sites: the layer loop's code is larger than
+// the instruction cache, and every kilobyte less shortens all phases (inlined copies of one generic staging function 1187 us a token of
+// the 3B-class shape; one shared copy 1051; templated on the widths and shared as here 1001). For the same reason the conversion
+// after the plain gather is a rolled loop and both plain phases share the instance of the wider one. The tile products stay
+// inlined per phase: one shared product costs more in calls than it saves (1125).
+// Both leave the phase's activations in sm.xh / sm.xf (fp16 in B-operand order + per-group factors) and end
 // with a consumer-wide barrier. A thread owns the 4 elements 4*pr .. 4*pr+3 for pr = tid_c, tid_c + kConsumerThreads, ...
 // so a warp owns whole groups of 128 and converts them in place.
 // xn = bf16( (float(h) * r) * float(w) ) from the tagged residual vector (dim/2 words)
 template <int MAXP>
-__device__ __forceinline__ void stage_norm_ll(const uint64_t* hll, const uint32_t* flags, int nflags, uint32_t tag,
-                                              const uint16_t* gw, int D, float eps, const Smem& sm, int tid_c,
-                                              const WaitCtl& wc, int layer, bool have_h, long long* dbg = nullptr) {
+inline __device__ __noinline__ void stage_norm_ll(const uint64_t* hll, const uint32_t* flags, int nflags, uint32_t tag,
+                                                  const uint16_t* gw, int D, float eps, DevStatus* status, unsigned limit, int layer,
+                                                  bool have_h, long long* dbg = nullptr) {
+  extern __shared__ __align__(128) uint8_t smem_raw[];
+  const Smem sm = carve_smem(smem_raw);
+  const WaitCtl wc{status, sm.s_abort, limit};
+  const int tid_c = threadIdx.x;
   uint32_t* xs32 = reinterpret_cast<uint32_t*>(sm.xh);
   float* red = sm.red;
   const int npairs = D / 4, lane = tid_c & 31;
@@ -257,36 +272,35 @@ __device__ __forceinline__ void stage_norm_ll(const uint64_t* hll, const uint32_
 }
 
 template <int MAXP>
-__device__ __forceinline__ void stage_plain_ll(const uint64_t* src, const uint32_t* flags, int nflags, uint32_t tag, int K,
-                                               const Smem& sm, int tid_c, const WaitCtl& wc, int layer) {
+inline __device__ __noinline__ void stage_plain_ll(const uint64_t* src, const uint32_t* flags, int nflags, uint32_t tag, int K,
+                                                   DevStatus* status, unsigned limit, int layer) {
+  extern __shared__ __align__(128) uint8_t smem_raw[];
+  const Smem sm = carve_smem(smem_raw);
+  const WaitCtl wc{status, sm.s_abort, limit};
+  const int tid_c = threadIdx.x;
   uint32_t* xs32 = reinterpret_cast<uint32_t*>(sm.xh);
   const int npairs = K / 4, lane = tid_c & 31;
   if (nflags > 0) wait_flags(flags, nflags, tag, tid_c >> 5, lane, wc, layer);
   else named_bar_sync(kBarConsumers, kConsumerThreads);
   ll_gather<MAXP>(src, K / 2, tag, xs32, tid_c, kConsumerThreads, wc, layer);
   // a thread converts exactly the words it gathered itself
-#pragma unroll
-  for (int k = 0; k < MAXP; k++) {
-    const int pr = tid_c + k * kConsumerThreads;
-    if (pr < npairs) {
-      const uint32_t a = xs32[2 * pr], b = xs32[2 * pr + 1];
-      const int grp = pr >> 5;
-      stage_group_fp16(a, b, sm.xh + grp * 128, sm.xf + grp, lane);
-    }
+#pragma unroll 1
+  for (int pr = tid_c; pr < npairs; pr += kConsumerThreads) {
+    const uint2 v = *reinterpret_cast<const uint2*>(xs32 + 2 * pr);
+    const int grp = pr >> 5;
+    stage_group_fp16(v.x, v.y, sm.xh + grp * 128, sm.xf + grp, lane);
   }
   named_bar_sync(kBarConsumers, kConsumerThreads);
 }
 
 // ------------------------------------------------------------------------------------------------ attention (tagged in/out)
 // q and the new k live in "pair-major" tagged words: word (head*HD/2 + p) = (x[p], x[p + HD/2]), which is what one
-// RoPE thread produces. A lane owns pairs 4*sl .. 4*sl+3, i.e. dims {4sl..4sl+3} and {HD/2+4sl..+3}.
-struct Attn2Args {
+// RoPE thread produces; v words are (v[2w], v[2w+1]).
+struct AttnArgs {
   const uint64_t* q_ll;     // [NH * HD/2]
   const uint64_t* k_ll;     // [NKV * HD/2] new key of this step, pair-major
-  const uint64_t* v_ll;     // [NKV * HD/2] new value, natural order: word w = (v[2w], v[2w+1])
+  const uint64_t* v_ll;     // [NKV * HD/2] new value, natural order
   uint64_t* ao_ll;          // [NH * HD/2] natural order
-  const uint16_t* kc;       // layer base: bf16 [max_seq, NKV, HD]
-  const uint16_t* vc;
   uint64_t* part_ll;        // [NKV][maxchunks][R*HD + 2R] tagged chunk partials (acc, then m, then d per head)
   uint32_t* ao_flags;       // [NKV * nchunks] arrival flags of the attention output, one per (kv head, chunk) CTA
   int nkv, pos, nchunks, maxchunks;
@@ -294,331 +308,217 @@ struct Attn2Args {
   uint32_t tag_in, tag_part, tag_out;
 };
 
-template <int HD, int R, bool LONGKV = false>
-__device__ __forceinline__ void attn2_phase(const Attn2Args& a, uint8_t* scratch, int* misc, int cw, int lane, int tid_c,
-                                            const WaitCtl& wc, int layer, Pipe* pipe = nullptr, int* tdone = nullptr) {
-  using C = AttnCfg<HD, R>;
-  constexpr int HP = HD / 2;
-  float* wacc = reinterpret_cast<float*>(scratch);                 // [CW][R][HD]  (dims in lane order, see below)
+// byte offset of 8-column block `c` of row `row` of a K or V matrix in a ring stage at shared address `base`
+template <int HD>
+__device__ __forceinline__ uint32_t kv_addr(uint32_t base, int row, int c) {
+  using C = AttnCfg<HD>;
+  if constexpr (!C::SPLIT) return base + (uint32_t)(row * C::ROWB + c * 16);
+  const uint32_t a = base + (uint32_t)((c >> 3) * (C::NPS * 128) + row * 128);
+  return a + ((((uint32_t)c & 7) ^ ((a >> 7) & 7)) << 4);       // the tensor copy's 128-byte swizzle: address bits 4..6 ^ 7..9
+}
+__device__ __forceinline__ void ldmatrix_x4(uint32_t (&r)[4], uint32_t addr) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
+}
+__device__ __forceinline__ void ldmatrix_x4_t(uint32_t (&r)[4], uint32_t addr) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
+}
+
+// Flash-decode of this CTA's (kv head, chunk) items on the tensor pipe, K/V from the ring, at every cached length. Warp w takes units
+// of 16 positions w, w + 14, ...: the R query heads of the group are the rows of a 16-row MMA tile, the positions the N dimension of
+// Q K^T and the K dimension of P V. Probabilities enter P V as three bf16 terms (24 bits: fp32 precision). What bounds it is latency:
+// the wait for q, one pass of the warps, the merge of the warps, the round trip of the merge of the chunks. Against dot products on the CUDA cores
+// with K/V loaded by the warps themselves: 40 / 8 heads of 64, 604 positions 1240 -> 1014 us a token (24 us a layer in all), 32 / 8 heads
+// of 64, 22 positions 433 -> 397. Against the earlier ring form (unswizzled 256-byte rows, 8-way bank conflicts on K and V, all 14 warps
+// merged whether they had a unit or not) heads of 128, 1778 positions: attention 9.8 -> 7.9 us a layer.
+template <int HD, int R>
+__device__ __forceinline__ void attention_phase(const AttnArgs& a, uint8_t* scratch, int cw, int lane, int tid_c, const WaitCtl& wc, int layer,
+                                                Pipe& pipe, int* tdone) {
+  using C = AttnCfg<HD>;
+  constexpr int HP = HD / 2, KSTEPS = (HD + 15) / 16, NTD = HD / 8, NPS = C::NPS, UP = 16, SPLIT = NPS / UP, RH = R > 8 ? 2 : 1;
+  static_assert(R <= 16 && NPS % UP == 0, "the query heads of a group are the rows of one MMA tile");
+  static_assert(kConsumerWarps * R * (HD + 2) * 4 + (R + 2) * HD * 2 <= kScratchBytes, "attention scratch");
+  float* wacc = reinterpret_cast<float*>(scratch);                 // [CW][R][HD]
   float* wm = wacc + kConsumerWarps * R * HD;                      // [CW][R]
   float* wd = wm + kConsumerWarps * R;                             // [CW][R]
-  uint32_t* qs = reinterpret_cast<uint32_t*>(wd + kConsumerWarps * R);   // [R*HP] q pairs, then [HP] k pairs, [HP] v words
+  uint32_t* qs = reinterpret_cast<uint32_t*>(wd + kConsumerWarps * R);   // bf16 [R][HD] q, [HD] new k, [HD] new v
   const int T = a.pos + 1;
   const int items = a.nkv * a.nchunks;
   const int chunk_len = (T + a.nchunks - 1) / a.nchunks;
-  const int seg = lane / C::SEG, sl = lane % C::SEG;
-  const bool active = sl < C::LPR;
+  const int g = lane >> 2, t = lane & 3, mat = lane >> 3;
+#pragma unroll 1
   for (int item = blockIdx.x; item < items; item += gridDim.x) {
-    const int kvh = item / a.nchunks, c = item % a.nchunks;
+    const int kvh = item / a.nchunks, c = item - kvh * a.nchunks;
     const int t0 = c * chunk_len, t1 = min(T, t0 + chunk_len);
     const bool has_new = (a.pos >= t0 && a.pos < t1);     // the chunk that contains this step's own position
-    // ---- gather q (R heads) and, for the last chunk, the new k / v ----
+    // ---- gather q (R heads) and, for the last chunk, the new k / v: at most one word pair per thread ----
     {
-      const int nq = R * HP;
-      const int total = nq + (has_new ? 2 * HP : 0);
-      // one pass: every thread owns at most one word pair of each source
-      uint32_t pending = 0;
-      const int pr = tid_c;
-      if (2 * pr < total) pending = 1;
-      for (unsigned spin = 0; pending; spin++) {
-        const int w = 2 * pr;
-        const uint64_t* src = w < nq ? a.q_ll + (size_t)kvh * R * HP + w
-                            : (w < nq + HP ? a.k_ll + (size_t)kvh * HP + (w - nq) : a.v_ll + (size_t)kvh * HP + (w - nq - HP));
-        uint64_t u, v;
-        ll_load2(src, u, v);
-        if ((uint32_t)(u >> 32) == a.tag_in && (uint32_t)(v >> 32) == a.tag_in) {
-          qs[w] = (uint32_t)u; qs[w + 1] = (uint32_t)v;
-          pending = 0;
-        } else {
-          if (*wc.s_abort) break;
-          if (spin > 16) __nanosleep(40);
-          if ((spin & 255) == 255 && ld_volatile_s32(&wc.st->abort)) { *wc.s_abort = 1; break; }
-          if (spin >= wc.limit) { report_fail(wc, W_FLAG, layer, (int)a.tag_in, -2); break; }
+      constexpr int NQ = R * HP;
+      static_assert(NQ + 2 * HP <= 2 * kConsumerThreads, "one word pair per thread");
+      const int w = 2 * tid_c;
+      if (w < NQ + (has_new ? 2 * HP : 0)) {
+        const uint64_t* src = w < NQ ? a.q_ll + (size_t)kvh * NQ + w
+                            : (w < NQ + HP ? a.k_ll + (size_t)kvh * HP + (w - NQ) : a.v_ll + (size_t)kvh * HP + (w - NQ - HP));
+#pragma unroll 1
+        for (unsigned spin = 0;; spin++) {
+          uint64_t u, v;
+          ll_load2(src, u, v);
+          if ((uint32_t)(u >> 32) == a.tag_in && (uint32_t)(v >> 32) == a.tag_in) {
+            const uint32_t x = (uint32_t)u, y = (uint32_t)v;
+            if (w < NQ + HP) {                                     // pairs p, p + 1 -> dims p, p + 1 and HP + p, HP + p + 1
+              const int row = w / HP, p = w - row * HP;
+              qs[row * HP + (p >> 1)] = (x & 0xffffu) | (y << 16);
+              qs[row * HP + (HP >> 1) + (p >> 1)] = (x >> 16) | (y & 0xffff0000u);
+            } else {
+              qs[w] = x; qs[w + 1] = y;
+            }
+            break;
+          }
+          if (poll_again(spin, wc, layer, (int)a.tag_in, -2)) break;
         }
       }
     }
     named_bar_sync(kBarConsumers, kConsumerThreads);
-    if constexpr (LONGKV) {
-      // ---- long caches: K/V stages from the ring, tensor-core flash-decode. Warp w takes units (16 positions of a stage)
-      // w, w + 14, ...: the R query heads are rows 0..R-1 of one 16-row MMA tile, the positions the N dimension of Q K^T and
-      // the K dimension of P V (probabilities as hi + lo bf16 pairs, ~2^-17), running maximum / denominator per row as in the scalar path.
-      constexpr int KSTEPS = HD / 16, NTD = HD / 8, NPS = C::NPS, ROWB = HD * 2;
-      static_assert(HD % 16 == 0 && NPS % 16 == 0 && R <= 8, "MMA flash-decode geometry");
-      const int g = lane >> 2, t = lane & 3;
+    const int nst = t1 > t0 ? (t1 - t0 + NPS - 1) / NPS : 0, units = t1 > t0 ? (t1 - t0 + UP - 1) / UP : 0;
+    if (cw < nst * SPLIT) {
       uint32_t aq[KSTEPS][4];
 #pragma unroll
-      for (int ks = 0; ks < KSTEPS; ks++) {
+      for (int ks = 0; ks < KSTEPS; ks++)
 #pragma unroll
-        for (int hf = 0; hf < 2; hf++) {
-          const int d = 16 * ks + 2 * t + 8 * hf;           // dims d, d + 1 of head g (pair-major words: (x[p], x[p + HP]))
-          uint32_t v = 0;
-          if (g < R) {
-            const uint32_t w0 = qs[g * HP + (d < HP ? d : d - HP)], w1 = qs[g * HP + (d + 1 < HP ? d + 1 : d + 1 - HP)];
-            v = (d < HP ? (w0 & 0xffffu) : (w0 >> 16)) | ((d + 1 < HP ? (w1 & 0xffffu) : (w1 >> 16)) << 16);
-          }
-          aq[ks][2 * hf] = v;
-          aq[ks][2 * hf + 1] = 0u;                           // rows 8..15 of the tile are unused
+        for (int e = 0; e < 4; e++) {                              // rows g, g + 8; columns 2t, 2t + 8
+          const int row = g + 8 * (e & 1), d2 = 8 * ks + t + 4 * (e >> 1);
+          aq[ks][e] = (e & 1) && RH == 1 ? 0u : (row < R && d2 < HP ? qs[row * HP + d2] : 0u);
         }
-      }
       float o[NTD][4];
 #pragma unroll
       for (int j = 0; j < NTD; j++)
 #pragma unroll
         for (int e = 0; e < 4; e++) o[j][e] = 0.f;
-      float mrun = -1e30f, lrun = 0.f;
+      float mrun[RH], lrun[RH];
+#pragma unroll
+      for (int h = 0; h < RH; h++) { mrun[h] = -1e30f; lrun[h] = 0.f; }
       // a stage is cut into units of 16 positions that different warps take: a chunk of a few stages keeps most warps busy
-      constexpr int UP = 16, SPLIT = NPS / UP;
-      const int nst = t1 > t0 ? (t1 - t0 + NPS - 1) / NPS : 0;
+#pragma unroll 1
       for (int u = cw; u < nst * SPLIT; u += kConsumerWarps) {
         const int st = u / SPLIT, part = u % SPLIT;
-        const uint32_t it = pipe->it + st;
+        const uint32_t it = pipe.it + st;
         const int sslot = it % kStages;
-        bool ok = true;
-        if (it >= (uint32_t)kStages) {                     // the stage's previous load must be complete before its phase bit is read
-          ok = false;
-          for (unsigned i = 0; i < wc.limit; i++) {
-            if ((uint32_t)*pipe->landed > it - kStages) { ok = true; break; }
-            if ((i & 63) == 63 && *wc.s_abort) break;
-          }
-          if (!ok && *wc.s_abort == 0) report_fail(wc, W_LANDED, layer, (int)it, *pipe->landed);
-        }
-        if (ok) ok = mbar_wait(&pipe->full[sslot], (it / kStages) & 1, wc, W_FULL, layer);
-        if (!ok) break;
-        uint8_t* k_s = pipe->stages + (size_t)sslot * kStageBytes + (size_t)part * UP * ROWB;
-        uint8_t* v_s = k_s + C::KV_STAGE_BYTES / 2;
-        const int base = t0 + st * NPS + part * UP, nvalid = min(UP, t1 - base);
+        if (!wait_stage(pipe, it, wc, layer)) break;
+        uint8_t* stage = pipe.stages + (size_t)sslot * kStageBytes;
+        const uint32_t k_s = smem_u32(stage), v_s = k_s + C::MATRIX_BYTES;
+        const int row0 = part * UP, base = t0 + st * NPS + row0, nvalid = min(UP, t1 - base);
         if (nvalid > 0) {
-          if (a.pos >= base && a.pos < base + UP) {          // this step's own row: from the tagged words, not the cache
-            const uint32_t* kp = qs + R * HP;
-            const uint32_t* vp = kp + HP;
-            uint16_t* krow = reinterpret_cast<uint16_t*>(k_s + (size_t)(a.pos - base) * ROWB);
-            uint32_t* vrow = reinterpret_cast<uint32_t*>(v_s + (size_t)(a.pos - base) * ROWB);
-            for (int p2 = lane; p2 < HP; p2 += 32) {
-              krow[p2] = (uint16_t)(kp[p2] & 0xffffu);
-              krow[p2 + HP] = (uint16_t)(kp[p2] >> 16);
-              vrow[p2] = vp[p2];
-            }
+          const int own = a.pos - base;
+          if (own >= 0 && own < UP && lane < NTD) {                // this step's own row: from the tagged words, not the cache
+            const uint4 kn = reinterpret_cast<const uint4*>(qs + R * HP)[lane], vn = reinterpret_cast<const uint4*>(qs + (R + 1) * HP)[lane];
+            *reinterpret_cast<uint4*>(stage + (kv_addr<HD>(k_s, row0 + own, lane) - k_s)) = kn;
+            *reinterpret_cast<uint4*>(stage + (kv_addr<HD>(v_s, row0 + own, lane) - k_s)) = vn;
           }
           // rows past the chunk are other cache rows (or never written): their V must not meet a zero probability as NaN
-          for (int i = lane; i < (UP - nvalid) * (ROWB / 16); i += 32)
-            *reinterpret_cast<uint4*>(v_s + (size_t)nvalid * ROWB + (size_t)i * 16) = make_uint4(0, 0, 0, 0);
+#pragma unroll 1
+          for (int i = lane; i < (UP - nvalid) * NTD; i += 32)
+            *reinterpret_cast<uint4*>(stage + (kv_addr<HD>(v_s, row0 + nvalid + i / NTD, i % NTD) - k_s)) = make_uint4(0, 0, 0, 0);
           __syncwarp();
           float sc[2][4];
 #pragma unroll
-          for (int nt = 0; nt < 2; nt++) {
-            sc[nt][0] = sc[nt][1] = sc[nt][2] = sc[nt][3] = 0.f;
+          for (int nt = 0; nt < 2; nt++) sc[nt][0] = sc[nt][1] = sc[nt][2] = sc[nt][3] = 0.f;
 #pragma unroll
-            for (int ks = 0; ks < KSTEPS; ks++) {
-              const uint8_t* kr = k_s + (size_t)(nt * 8 + g) * ROWB + (16 * ks + 2 * t) * 2;
-              mma_bf16(sc[nt], aq[ks], *reinterpret_cast<const uint32_t*>(kr), *reinterpret_cast<const uint32_t*>(kr + 16));
+          for (int ks = 0; ks < KSTEPS; ks++) {
+            uint32_t bk[4];                                        // (positions 0..7, columns 0..7), (.., 8..15), (8..15, 0..7), (8..15, 8..15)
+            ldmatrix_x4(bk, kv_addr<HD>(k_s, row0 + (mat >> 1) * 8 + (lane & 7), min(2 * ks + (mat & 1), NTD - 1)));
+            mma_bf16(sc[0], aq[ks], bk[0], bk[1]);
+            mma_bf16(sc[1], aq[ks], bk[2], bk[3]);
+          }
+          uint32_t ap[3][4];
+#pragma unroll
+          for (int h = 0; h < RH; h++) {                           // rows g + 8h
+            float mx = mrun[h];                                    // finite: the running maximum starts at -1e30
+#pragma unroll
+            for (int nt = 0; nt < 2; nt++)
+#pragma unroll
+              for (int e = 0; e < 2; e++) {
+                float& v = sc[nt][2 * h + e];
+                v = (nt * 8 + 2 * t + e) < nvalid ? v * a.scale : -INFINITY;
+                mx = fmaxf(mx, v);
+              }
+            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+            const float corr = __expf(mrun[h] - mx);
+            mrun[h] = mx;
+            lrun[h] *= corr;
+#pragma unroll
+            for (int j = 0; j < NTD; j++) { o[j][2 * h] *= corr; o[j][2 * h + 1] *= corr; }
+#pragma unroll
+            for (int nt = 0; nt < 2; nt++) {                       // A columns 2t (+ 1) of positions 8 nt ..
+              float p0 = __expf(sc[nt][2 * h] - mx), p1 = __expf(sc[nt][2 * h + 1] - mx);
+              lrun[h] += p0 + p1;                                  // this lane's columns; the quad is summed at the end
+#pragma unroll
+              for (int e = 0; e < 3; e++) {
+                const float h0 = rbf(p0), h1 = rbf(p1);
+                ap[e][2 * nt + h] = pack_bf16(h0, h1);
+                p0 -= h0; p1 -= h1;
+              }
             }
           }
-          float mx = -INFINITY;                              // row g (rows 8..15 of the tile carry nothing)
+          if (RH == 1)
 #pragma unroll
-          for (int nt = 0; nt < 2; nt++)
-#pragma unroll
-            for (int e = 0; e < 2; e++) {
-              const float v = (nt * 8 + 2 * t + e) < nvalid ? sc[nt][e] * a.scale : -INFINITY;
-              sc[nt][e] = v;
-              mx = fmaxf(mx, v);
-            }
-          mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
-          mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
-          const float mn = fmaxf(mrun, mx);                 // finite: the running maximum starts at -1e30
-          const float corr = __expf(mrun - mn);
-          mrun = mn;
-          lrun *= corr;
-#pragma unroll
-          for (int j = 0; j < NTD; j++) { o[j][0] *= corr; o[j][1] *= corr; }
-          uint32_t ah[4], al[4];
-#pragma unroll
-          for (int e = 0; e < 2; e++) {                      // A rows g: positions 2t (+1) and + 8; rows g + 8: zero
-            const float p0 = __expf(sc[e][0] - mrun), p1 = __expf(sc[e][1] - mrun);
-            lrun += p0 + p1;                                 // this lane's columns; the quad is summed at the end
-            const float h0 = rbf(p0), h1 = rbf(p1);
-            ah[2 * e] = pack_bf16(h0, h1);
-            al[2 * e] = pack_bf16(p0 - h0, p1 - h1);
-            ah[2 * e + 1] = 0u;
-            al[2 * e + 1] = 0u;
-          }
+            for (int e = 0; e < 3; e++) ap[e][1] = ap[e][3] = 0u;
 #pragma unroll
           for (int j = 0; j < NTD; j += 2) {
             uint32_t bv[4];
-            const int mat = lane >> 3;
-            ldmatrix_x4_trans(bv, v_s + (size_t)((mat & 1) * 8 + (lane & 7)) * ROWB + (j + (mat >> 1)) * 16);
-            mma_bf16(o[j], ah, bv[0], bv[1]);
-            mma_bf16(o[j], al, bv[0], bv[1]);
-            mma_bf16(o[j + 1], ah, bv[2], bv[3]);
-            mma_bf16(o[j + 1], al, bv[2], bv[3]);
+            ldmatrix_x4_t(bv, kv_addr<HD>(v_s, row0 + (mat & 1) * 8 + (lane & 7), min(j + (mat >> 1), NTD - 1)));
+#pragma unroll
+            for (int e = 0; e < 3; e++) {
+              mma_bf16(o[j], ap[e], bv[0], bv[1]);
+              if (j + 1 < NTD) mma_bf16(o[j + 1 < NTD ? j + 1 : j], ap[e], bv[2], bv[3]);
+            }
           }
         }
         __syncwarp();
-        if (lane == 0) {                                     // the stage's last unit hands it back
-          const int old = atomicAdd(tdone + sslot, 1);
-          if (old == SPLIT - 1) {
-            tdone[sslot] = 0;
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            mbar_arrive(&pipe->empty[sslot]);
-          }
+        if (lane == 0 && atomicAdd(tdone + sslot, 1) == SPLIT - 1) {   // the stage's last unit hands it back
+          tdone[sslot] = 0;
+          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+          mbar_arrive(&pipe.empty[sslot]);
         }
       }
-      pipe->it += (uint32_t)nst;                             // producer and consumers count alike
-      lrun += __shfl_xor_sync(0xffffffffu, lrun, 1);
-      lrun += __shfl_xor_sync(0xffffffffu, lrun, 2);
-      if (g < R) {
-        float* dst = wacc + ((size_t)cw * R + g) * HD;
 #pragma unroll
-        for (int j = 0; j < NTD; j++) { dst[j * 8 + 2 * t] = o[j][0]; dst[j * 8 + 2 * t + 1] = o[j][1]; }
-        if (t == 0) { wm[cw * R + g] = mrun; wd[cw * R + g] = lrun; }
-      }
-    } else {
-      float q[R][8];
+      for (int h = 0; h < RH; h++) {
+        lrun[h] += __shfl_xor_sync(0xffffffffu, lrun[h], 1);
+        lrun[h] += __shfl_xor_sync(0xffffffffu, lrun[h], 2);
+        const int row = g + 8 * h;
+        if (cw < units && row < R) {
+          float* dst = wacc + (cw * R + row) * HD + 2 * t;
 #pragma unroll
-      for (int r = 0; r < R; r++)
-#pragma unroll
-        for (int e = 0; e < 4; e++) {
-          const uint32_t u = active ? qs[r * HP + 4 * sl + e] : 0u;
-          q[r][e] = bflo(u);        // dim 4sl+e
-          q[r][4 + e] = bfhi(u);    // dim HP+4sl+e
-        }
-      float m[R], den[R], acc[R][8];
-#pragma unroll
-      for (int r = 0; r < R; r++) {
-        m[r] = -1e30f; den[r] = 0.f;
-#pragma unroll
-        for (int e = 0; e < 8; e++) acc[r][e] = 0.f;
-      }
-      constexpr int BATCH = FB_ATTN_BATCH;
-      const int stride = kConsumerWarps * C::PPW;
-      for (int tb = t0 + cw * C::PPW; tb < t1; tb += BATCH * stride) {
-        uint2 klo[BATCH], khi[BATCH], vlo[BATCH], vhi[BATCH];
-        bool valid[BATCH];
-#pragma unroll
-        for (int j = 0; j < BATCH; j++) {
-          const int t = tb + j * stride + seg;
-          valid[j] = t < t1;
-          klo[j] = khi[j] = vlo[j] = vhi[j] = make_uint2(0, 0);
-          if (valid[j] && active) {
-            if (t == a.pos) {      // this step's own k / v: from the tagged words (the cache row is for later steps)
-              const uint32_t* kp = qs + R * HP + 4 * sl;
-              const uint32_t* vp = qs + R * HP + HP;
-              klo[j] = make_uint2((kp[0] & 0xffffu) | (kp[1] << 16), (kp[2] & 0xffffu) | (kp[3] << 16));
-              khi[j] = make_uint2((kp[0] >> 16) | (kp[1] & 0xffff0000u), (kp[2] >> 16) | (kp[3] & 0xffff0000u));
-              vlo[j] = make_uint2(vp[2 * sl], vp[2 * sl + 1]);
-              vhi[j] = make_uint2(vp[HP / 2 + 2 * sl], vp[HP / 2 + 2 * sl + 1]);
-            } else {
-              const size_t off = ((size_t)t * a.nkv + kvh) * HD + 4 * sl;
-              klo[j] = __ldcg(reinterpret_cast<const uint2*>(a.kc + off));
-              khi[j] = __ldcg(reinterpret_cast<const uint2*>(a.kc + off + HP));
-              vlo[j] = __ldcg(reinterpret_cast<const uint2*>(a.vc + off));
-              vhi[j] = __ldcg(reinterpret_cast<const uint2*>(a.vc + off + HP));
-            }
-          }
-        }
-        // long chunks: ask L2 for the rows this warp will load two rounds from now (costs no registers)
-        if (sl < (HD * 2 + 63) / 64) {
-#pragma unroll
-          for (int j = 0; j < BATCH; j++) {
-            const int tp = tb + (FB_ATTN_PFD * BATCH + j) * stride + seg;
-            if (tp < t1) {
-              const size_t off = ((size_t)tp * a.nkv + kvh) * HD;
-              asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const char*>(a.kc + off) + sl * 64));
-              asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const char*>(a.vc + off) + sl * 64));
-            }
-          }
-        }
-        // scores of the whole batch first (independent chains), then ONE rescale per head and batch
-        float sc[BATCH][R];
-#pragma unroll
-        for (int j = 0; j < BATCH; j++) {
-          const float kf[8] = {bflo(klo[j].x), bfhi(klo[j].x), bflo(klo[j].y), bfhi(klo[j].y),
-                               bflo(khi[j].x), bfhi(khi[j].x), bflo(khi[j].y), bfhi(khi[j].y)};
-#pragma unroll
-          for (int r = 0; r < R; r++) {
-            float s = 0.f;
-#pragma unroll
-            for (int e = 0; e < 8; e++) s = fmaf(q[r][e], kf[e], s);
-#pragma unroll
-            for (int o = C::SEG / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-            sc[j][r] = valid[j] ? s * a.scale : -INFINITY;
-          }
-        }
-#pragma unroll
-        for (int r = 0; r < R; r++) {
-          float mb = sc[0][r];
-#pragma unroll
-          for (int j = 1; j < BATCH; j++) mb = fmaxf(mb, sc[j][r]);
-          const float m2 = fmaxf(m[r], mb);                 // finite: m starts at -1e30
-          const float corr = __expf(m[r] - m2);
-          den[r] *= corr;
-#pragma unroll
-          for (int e = 0; e < 8; e++) acc[r][e] *= corr;
-          m[r] = m2;
-        }
-#pragma unroll
-        for (int j = 0; j < BATCH; j++) {
-          const float vf[8] = {bflo(vlo[j].x), bfhi(vlo[j].x), bflo(vlo[j].y), bfhi(vlo[j].y),
-                               bflo(vhi[j].x), bfhi(vhi[j].x), bflo(vhi[j].y), bfhi(vhi[j].y)};
-#pragma unroll
-          for (int r = 0; r < R; r++) {
-            const float w = __expf(sc[j][r] - m[r]);        // 0 for a position that does not exist
-            den[r] += w;
-#pragma unroll
-            for (int e = 0; e < 8; e++) acc[r][e] = fmaf(w, vf[e], acc[r][e]);
-          }
-        }
-      }
-      // merge the warp's segments
-#pragma unroll
-      for (int off = C::SEG; off < 32; off <<= 1) {
-#pragma unroll
-        for (int r = 0; r < R; r++) {
-          const float mo = __shfl_xor_sync(0xffffffffu, m[r], off);
-          const float dn = __shfl_xor_sync(0xffffffffu, den[r], off);
-          const float gm = fmaxf(m[r], mo);
-          const float wa = __expf(m[r] - gm), wb = __expf(mo - gm);
-          den[r] = den[r] * wa + dn * wb;
-#pragma unroll
-          for (int e = 0; e < 8; e++) {
-            const float ao_ = __shfl_xor_sync(0xffffffffu, acc[r][e], off);
-            acc[r][e] = acc[r][e] * wa + ao_ * wb;
-          }
-          m[r] = gm;
-        }
-      }
-      if (seg == 0 && active) {
-#pragma unroll
-        for (int r = 0; r < R; r++) {
-          float* dst = wacc + ((size_t)cw * R + r) * HD;
-#pragma unroll
-          for (int e = 0; e < 4; e++) { dst[4 * sl + e] = acc[r][e]; dst[HP + 4 * sl + e] = acc[r][4 + e]; }
-          if (sl == 0) { wm[cw * R + r] = m[r]; wd[cw * R + r] = den[r]; }
+          for (int j = 0; j < NTD; j++) *reinterpret_cast<float2*>(dst + j * 8) = make_float2(o[j][2 * h], o[j][2 * h + 1]);
+          if (t == 0) { wm[cw * R + row] = mrun[h]; wd[cw * R + row] = lrun[h]; }
         }
       }
     }
+    pipe.it += (uint32_t)nst;                                 // producer and consumers count alike
     named_bar_sync(kBarConsumers, kConsumerThreads);
-    // ---- merge the CTA's warps; one thread per (head, dim pair) ----
+    // ---- merge the CTA's warps that had a unit; one thread per (head, dim pair) ----
     constexpr int WPC = R * HD + 2 * R;                       // words of one chunk partial
+    const int nact = min(units, kConsumerWarps);
     uint64_t* mine = a.part_ll + ((size_t)kvh * a.maxchunks + c) * WPC;
+#pragma unroll 1
     for (int o = tid_c; o < R * HP; o += kConsumerThreads) {
-      const int r = o / HP, d = 2 * (o % HP);
+      const int r = o / HP, d = 2 * (o - r * HP);
       float gm = -1e30f;
-#pragma unroll
-      for (int w = 0; w < kConsumerWarps; w++) gm = fmaxf(gm, wm[w * R + r]);
+#pragma unroll 4
+      for (int w = 0; w < nact; w++) gm = fmaxf(gm, wm[w * R + r]);
       float Dn = 0.f, A0 = 0.f, A1 = 0.f;
-#pragma unroll
-      for (int w = 0; w < kConsumerWarps; w++) {
+#pragma unroll 2
+      for (int w = 0; w < nact; w++) {
         const float e = __expf(wm[w * R + r] - gm);
+        const float2 v = *reinterpret_cast<const float2*>(wacc + (w * R + r) * HD + d);
         Dn += wd[w * R + r] * e;
-        A0 += wacc[((size_t)w * R + r) * HD + d] * e;
-        A1 += wacc[((size_t)w * R + r) * HD + d + 1] * e;
+        A0 += v.x * e;
+        A1 += v.y * e;
       }
-      const int qh = kvh * R + r;
       if (a.nchunks == 1) {
-        ll_store(a.ao_ll + (size_t)qh * HP + (d >> 1), (uint32_t)f2bf(A0 / Dn) | ((uint32_t)f2bf(A1 / Dn) << 16), a.tag_out);
+        ll_store(a.ao_ll + (size_t)(kvh * R + r) * HP + (d >> 1), (uint32_t)f2bf(A0 / Dn) | ((uint32_t)f2bf(A1 / Dn) << 16), a.tag_out);
       } else {
-        ll_store(mine + r * HD + d, __float_as_uint(A0), a.tag_part);
-        ll_store(mine + r * HD + d + 1, __float_as_uint(A1), a.tag_part);
+        ll_store2(mine + r * HD + d, __float_as_uint(A0), __float_as_uint(A1), a.tag_part);
         if (d == 0) {
           ll_store(mine + R * HD + r, __float_as_uint(gm), a.tag_part);
           ll_store(mine + R * HD + R + r, __float_as_uint(Dn), a.tag_part);
@@ -630,13 +530,13 @@ __device__ __forceinline__ void attn2_phase(const Attn2Args& a, uint8_t* scratch
       // partial it needs the 2R words (max, denominator) and its own pairs only: one 16-byte tagged load per thread,
       // no counter, no fence, a single round trip.
       named_bar_sync(kBarConsumers, kConsumerThreads);        // wacc / wm / wd are dead: scratch is free
-      const int npairs = R * HP;
+      constexpr int npairs = R * HP;
       const int nown = (npairs - c + a.nchunks - 1) / a.nchunks;
       const int per = R + nown;                                // loads per source chunk
       uint32_t* pg = reinterpret_cast<uint32_t*>(scratch);     // [nchunks][per][2] payloads
       const int total = a.nchunks * per;                       // <= kConsumerThreads (host checks the shape)
       if (tid_c < total) {
-        const int cc = tid_c / per, sl2 = tid_c % per;
+        const int cc = tid_c / per, sl2 = tid_c - cc * per;
         int w;
         if (sl2 < R) {
           w = R * HD + 2 * sl2;
@@ -645,17 +545,15 @@ __device__ __forceinline__ void attn2_phase(const Attn2Args& a, uint8_t* scratch
           w = (o / HP) * HD + 2 * (o % HP);
         }
         const uint64_t* src = a.part_ll + ((size_t)kvh * a.maxchunks + cc) * WPC + w;
+#pragma unroll 1
         for (unsigned spin = 0;; spin++) {
           uint64_t u, v;
           ll_load2(src, u, v);
           if ((uint32_t)(u >> 32) == a.tag_part && (uint32_t)(v >> 32) == a.tag_part) {
-            pg[2 * tid_c] = (uint32_t)u; pg[2 * tid_c + 1] = (uint32_t)v;
+            *reinterpret_cast<uint2*>(pg + 2 * tid_c) = make_uint2((uint32_t)u, (uint32_t)v);
             break;
           }
-          if (*wc.s_abort) break;
-          if (spin > 16) __nanosleep(40);
-          if ((spin & 255) == 255 && ld_volatile_s32(&wc.st->abort)) { *wc.s_abort = 1; break; }
-          if (spin >= wc.limit) { report_fail(wc, W_FLAG, layer, (int)a.tag_part, -4); break; }
+          if (poll_again(spin, wc, layer, (int)a.tag_part, -4)) break;
         }
       }
       named_bar_sync(kBarConsumers, kConsumerThreads);
@@ -664,16 +562,18 @@ __device__ __forceinline__ void attn2_phase(const Attn2Args& a, uint8_t* scratch
         const int o = c + tid_c * a.nchunks, r = o / HP, d = 2 * (o % HP);
         // words 0..R-1 of a chunk's (max, denominator) area are the maxima, R..2R-1 the denominators
         float gm = -1e30f;
+#pragma unroll 4
         for (int cc = 0; cc < a.nchunks; cc++) gm = fmaxf(gm, pf[cc * per * 2 + r]);
         float Dn = 0.f, A0 = 0.f, A1 = 0.f;
+#pragma unroll 4
         for (int cc = 0; cc < a.nchunks; cc++) {
           const float e = __expf(pf[cc * per * 2 + r] - gm);
+          const float2 v = *reinterpret_cast<const float2*>(pf + (cc * per + R + tid_c) * 2);
           Dn += pf[cc * per * 2 + R + r] * e;
-          A0 += pf[(cc * per + R + tid_c) * 2] * e;
-          A1 += pf[(cc * per + R + tid_c) * 2 + 1] * e;
+          A0 += v.x * e;
+          A1 += v.y * e;
         }
-        const int qh = kvh * R + r;
-        ll_store(a.ao_ll + (size_t)qh * HP + (d >> 1), (uint32_t)f2bf(A0 / Dn) | ((uint32_t)f2bf(A1 / Dn) << 16), a.tag_out);
+        ll_store(a.ao_ll + (size_t)(kvh * R + r) * HP + (d >> 1), (uint32_t)f2bf(A0 / Dn) | ((uint32_t)f2bf(A1 / Dn) << 16), a.tag_out);
       }
     }
     named_bar_sync(kBarConsumers, kConsumerThreads);
@@ -681,35 +581,35 @@ __device__ __forceinline__ void attn2_phase(const Attn2Args& a, uint8_t* scratch
   }
 }
 
-// Producer side of the long-cache attention: the K and V rows of this CTA's chunk(s), NPS positions per ring stage. The
-// caches are [layer * max_seq + position][kv head][HD]: one 3-D tensor copy (box HD x 1 head x NPS positions) per
-// matrix and stage brings the strided rows in one request. Rows past the chunk (the last stage) are real cache rows that
+// Producer side of the attention: the K and V rows of this CTA's chunk(s), NPS positions per ring stage. The caches are
+// [layer * max_seq + position][kv head][HD]: 4-D tensors (column, column block, kv head, row), one copy per matrix, stage and
+// column block brings the strided rows in one request. Rows past the chunk (the last stage) are real cache rows that
 // nobody reads; past the end of the cache the copy fills zeros. Called by the producer lane.
-__device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, int x, int y, int z, uint64_t* bar) {
+__device__ __forceinline__ void tma_load_4d(void* dst, const CUtensorMap* map, int x, int y, int z, int w, uint64_t* bar) {
   asm volatile(
-      "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
-      ::"r"(smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(z), "r"(smem_u32(bar)) : "memory");
+      "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];"
+      ::"r"(smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(z), "r"(w), "r"(smem_u32(bar)) : "memory");
 }
-template <int HD, int R>
+template <int HD>
 __device__ __forceinline__ bool produce_kv(Pipe& p, const CUtensorMap* kmap, const CUtensorMap* vmap, int row0, int nkv, int nchunks,
                                            int T, int b, int G, const WaitCtl& wc, int layer) {
-  using C = AttnCfg<HD, R>;
+  using C = AttnCfg<HD>;
   const int items = nkv * nchunks, chunk_len = (T + nchunks - 1) / nchunks;
+#pragma unroll 1
   for (int item = b; item < items; item += G) {
-    const int kvh = item / nchunks, c = item % nchunks, t0 = c * chunk_len, t1 = min(T, t0 + chunk_len);
+    const int kvh = item / nchunks, c = item - kvh * nchunks, t0 = c * chunk_len, t1 = min(T, t0 + chunk_len);
+#pragma unroll 1
     for (int ts = t0; ts < t1; ts += C::NPS) {
+      if (!stage_slot(p, wc, layer)) return false;
       const int s = (int)(p.it % kStages);
-      if (!mbar_wait(&p.empty[s], ((p.it / kStages) & 1) ^ 1, wc, W_EMPTY, layer)) return false;
       mbar_expect_tx(&p.full[s], (uint32_t)C::KV_STAGE_BYTES);
       uint8_t* dst = p.stages + (size_t)s * kStageBytes;
-      tma_load_3d(dst, kmap, 0, kvh, row0 + ts, &p.full[s]);
-      tma_load_3d(dst + C::KV_STAGE_BYTES / 2, vmap, 0, kvh, row0 + ts, &p.full[s]);
-      p.it++;
-      if (p.it > p.max_fly) {                         // same trailing wait as produce_rows: keeps `landed` current
-        const uint32_t j = p.it - 1 - p.max_fly;
-        if (!mbar_wait(&p.full[j % kStages], (j / kStages) & 1, wc, W_FULL, layer)) return false;
-        *p.landed = (int)(j + 1);
+#pragma unroll
+      for (int bl = 0; bl < C::BLKS; bl++) {
+        tma_load_4d(dst + bl * (C::NPS * C::ROWB), kmap, 0, bl, kvh, row0 + ts, &p.full[s]);
+        tma_load_4d(dst + C::MATRIX_BYTES + bl * (C::NPS * C::ROWB), vmap, 0, bl, kvh, row0 + ts, &p.full[s]);
       }
+      if (!stage_issued(p, wc, layer)) return false;
     }
   }
   return true;
@@ -717,7 +617,7 @@ __device__ __forceinline__ bool produce_kv(Pipe& p, const CUtensorMap* kmap, con
 
 // ------------------------------------------------------------------------------------------------ kernel
 struct Decode2Params {
-  CUtensorMap kmap, vmap;     // long-cache variant: the K / V caches as [HD][n_kv][n_layer * max_seq] tensors (else unused)
+  CUtensorMap kmap, vmap;     // the K / V caches as (column, column block, kv head, n_layer * max_seq rows) tensors
   const uint8_t *w_qkv, *w_o, *w_gu, *w_d, *w_lm;
   const uint16_t *n1, *n2, *nf, *embed;
   const float* invf;
@@ -756,8 +656,7 @@ __host__ __device__ constexpr int small_ks(int k) {
 }
 __host__ __device__ constexpr int imax(int a, int b) { return a > b ? a : b; }
 
-// LONGKV: the attention phase reads K/V through the weight ring (produce_kv); chosen by the host for long caches.
-template <int KDIM, int KOUT, int KFFN, int HD, int R, bool HZ, bool LONGKV = false>
+template <int KDIM, int KOUT, int KFFN, int HD, int R, bool HZ>
 __global__ void __launch_bounds__(kThreads, 1) decode_mega2(const __grid_constant__ Decode2Params P) {
   extern __shared__ __align__(128) uint8_t smem_raw[];
   Smem sm = carve_smem(smem_raw);
@@ -798,10 +697,10 @@ __global__ void __launch_bounds__(kThreads, 1) decode_mega2(const __grid_constan
   if (warp == kConsumerWarps) {
     if (lane == 0) {
       bool ok = true;
+#pragma unroll 1
       for (int l = 0; l < L && ok; l++) {
         ok = produce_rows(pipe, P.w_qkv + l * strQ + (size_t)q0 * recD, q1 - q0, CQ::TILE_ROWS, CQ::RT, recD, wc, l);
-        if constexpr (LONGKV)
-          ok = ok && produce_kv<HD, R>(pipe, &P.kmap, &P.vmap, l * P.max_seq, P.n_kv, P.nchunks, P.pos + 1, b, G, wc, l);
+        ok = ok && produce_kv<HD>(pipe, &P.kmap, &P.vmap, l * P.max_seq, P.n_kv, P.nchunks, P.pos + 1, b, G, wc, l);
         ok = ok &&
              produce_rows(pipe, P.w_o + l * strO + (size_t)o0 * recO, o1 - o0, CO::TILE_ROWS, CO::RT, recO, wc, l) &&
              produce_rows(pipe, P.w_gu + l * strG + (size_t)g0 * recD, g1 - g0, CG::TILE_ROWS, CG::RT, recD, wc, l) &&
@@ -837,6 +736,7 @@ __global__ void __launch_bounds__(kThreads, 1) decode_mega2(const __grid_constan
             ll_store2_sys(dst + 2, __float_as_uint(c2), __float_as_uint(c3), tag);
           } else {
             const float cc[4] = {c0, c1, c2, c3};
+#pragma unroll 1
             for (int i = 0; i < nvalid; i++) ll_store_sys(dst + i, __float_as_uint(cc[i]), tag);
           }
         }
@@ -856,9 +756,11 @@ __global__ void __launch_bounds__(kThreads, 1) decode_mega2(const __grid_constan
     float* yin = sm.yin;                                      // [N-1][kMaxOwnRows]
     auto resid_finish = [&](uint32_t tag, int par, int layer) {
       const int npair = (o1 - o0) / 2, nitem = npair * (N - 1);
+#pragma unroll 1
       for (int it = tid_c; it < nitem; it += kConsumerThreads) {
         const int j = it / npair, pr = it % npair, s2 = j >= me ? j + 1 : j;
         const uint64_t* src = P.inbox + ((size_t)(par * N + s2)) * D + o0 + 2 * pr;
+#pragma unroll 1
         for (unsigned spin = 0;; spin++) {
           uint64_t u, v;
           ll_load2_sys(src, u, v);
@@ -869,12 +771,14 @@ __global__ void __launch_bounds__(kThreads, 1) decode_mega2(const __grid_constan
           }
           if (*wc.s_abort) break;
           if ((spin & 255) == 255 && ld_volatile_s32(&wc.st->abort)) { *wc.s_abort = 1; break; }
-          if (spin >= wc.limit) { report_fail(wc, W_FLAG, layer, (int)tag, -3); break; }
+          if (spin >= wc.limit) { report_fail_far(wc, W_FLAG, layer, (int)tag, -3); break; }
         }
       }
       named_bar_sync(kBarConsumers, kConsumerThreads);        // every row's own partial and every peer's are in shared memory
+#pragma unroll 1
       for (int pr = tid_c; pr < npair; pr += kConsumerThreads) {
         float tot0 = 0.f, tot1 = 0.f;
+#pragma unroll 1
         for (int s2 = 0; s2 < N; s2++) {
           const float* src = s2 == me ? ypart : yin + (s2 > me ? s2 - 1 : s2) * kMaxOwnRows;
           tot0 += src[2 * pr]; tot1 += src[2 * pr + 1];
@@ -895,6 +799,7 @@ __global__ void __launch_bounds__(kThreads, 1) decode_mega2(const __grid_constan
         tok = 0;
         if (tid_c == 0 && b == 0) atomicCAS(&P.status->code, 0, 6 /*FB_ERR_RANGE*/);
       }
+#pragma unroll 1
       for (int i = tid_c; i < D; i += kConsumerThreads) {
         const uint16_t v = P.d_h ? ld_cg_u16(P.d_h + i) : f2bf(bf2f(__ldg(P.embed + (size_t)tok * D + i)) * P.emb_mult);
         reinterpret_cast<uint16_t*>(sm.xh)[i] = v;
@@ -903,6 +808,7 @@ __global__ void __launch_bounds__(kThreads, 1) decode_mega2(const __grid_constan
       named_bar_sync(kBarConsumers, kConsumerThreads);
     }
 #define FB_STAMP(i) do { if (P.prof && tid_c == 0) P.prof[((size_t)b * L + l) * 16 + (i)] = (long long)globaltimer_ns(); } while (0)
+#pragma unroll 1
     for (int l = 0; l < L; l++) {
       uint16_t* kcl = P.kc + (size_t)l * P.max_seq * P.n_kv * HD;
       uint16_t* vcl = P.vc + (size_t)l * P.max_seq * P.n_kv * HD;
@@ -911,20 +817,8 @@ __global__ void __launch_bounds__(kThreads, 1) decode_mega2(const __grid_constan
                      tg_dn = mk_tag(P.tag_base, l, PH_DOWN);
       // ================= QKV: norm1 -> GEMV -> RoPE -> tagged q / new k / new v, cache append =================
       FB_STAMP(0);
-      if (b < P.n_kv * P.nchunks) {
-        // the K/V rows this CTA will attend in this layer: pull them into L2 now, they do not depend on anything
-        const int kvh = b / P.nchunks, c = b % P.nchunks;
-        const int T = P.pos + 1, clen = (T + P.nchunks - 1) / P.nchunks;
-        const int t0 = c * clen, t1 = min(min(T, t0 + clen), t0 + 64);
-        constexpr int PER_ROW = (HD * 2 + 63) / 64;
-        for (int i = tid_c; i < (t1 - t0) * PER_ROW * 2; i += kConsumerThreads) {
-          const int t = t0 + (i >> 1) / PER_ROW, seg = (i >> 1) % PER_ROW;
-          const uint16_t* base = ((i & 1) ? vcl : kcl) + ((size_t)t * P.n_kv + kvh) * HD;
-          asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const char*>(base) + seg * 64));
-        }
-      }
       stage_norm_ll<MAXP_D>(P.h_ll, P.h_flags, FG, mk_tag(P.tag_base, l - 1, PH_DOWN), P.n1 + (size_t)l * D, D, P.eps,
-                            sm, tid_c, wc, l, l == 0, P.prof ? P.prof + ((size_t)b * L + l) * 16 : nullptr);
+                            P.status, P.spin_limit, l, l == 0, P.prof ? P.prof + ((size_t)b * L + l) * 16 : nullptr);
       FB_STAMP(1);
       consume_tiles<CQ, HZ, true>(pipe, q1 - q0, xs_, qs_, cw, lane, wc, l, [&](int row0, float c, int nvalid) {
         // lanes 0/8/16/24 hold rows row0..row0+3: two RoPE pairs (or four v dims)
@@ -961,18 +855,19 @@ __global__ void __launch_bounds__(kThreads, 1) decode_mega2(const __grid_constan
           // columns of the O window that belong to a neighbouring rank (tensor parallel, 8-way split of the 3B-class
           // shape): the O projection must see zeros there, tagged like the real attention output
           const int used = P.n_head * HP, off = P.ao_off >> 1;
+#pragma unroll 1
           for (int i = tid_c; i < KOUT / 2 - used; i += kConsumerThreads)
             ll_store(P.ao_ll + (i < off ? i : used + i), 0u, tg_att);
         }
-        Attn2Args aa{P.q_ll, P.k_ll, P.v_ll, P.ao_ll + (P.ao_off >> 1), kcl, vcl, P.part_ll, P.ao_flags, P.n_kv, P.pos, P.nchunks,
+        const AttnArgs aa{P.q_ll, P.k_ll, P.v_ll, P.ao_ll + (P.ao_off >> 1), P.part_ll, P.ao_flags, P.n_kv, P.pos, P.nchunks,
                      P.maxchunks, P.attn_scale, tg_qkv, mk_tag(P.tag_base, l, PH_PART), tg_att};
         named_bar_sync(kBarConsumers, kConsumerThreads);        // scratch (the activations) is free: every warp left the GEMV
-        attn2_phase<HD, R, LONGKV>(aa, sm.scratch, sm.misc, cw, lane, tid_c, wc, l, &pipe, sm.tdone);
+        attention_phase<HD, R>(aa, sm.scratch, cw, lane, tid_c, wc, l, pipe, sm.tdone);
       }
       FB_STAMP(3);
       // ================= O projection + residual =================
       {
-        stage_plain_ll<MAXP_O>(P.ao_ll, P.ao_flags, FKV, tg_att, KOUT, sm, tid_c, wc, l);
+        stage_plain_ll<imax(MAXP_O, MAXP_F)>(P.ao_ll, P.ao_flags, FKV, tg_att, KOUT, P.status, P.spin_limit, l);
         FB_STAMP(4);
         consume_tiles<CO, HZ, true>(pipe, o1 - o0, xs_, qs_, cw, lane, wc, l,
                                   [&](int row0, float c, int nvalid) { resid_epi(row0, c, nvalid, tg_o, 0); });
@@ -981,7 +876,7 @@ __global__ void __launch_bounds__(kThreads, 1) decode_mega2(const __grid_constan
       }
       FB_STAMP(5);
       // ================= gate/up + SwiGLU =================
-      stage_norm_ll<MAXP_D>(P.h_ll, P.h_flags, FG, tg_o, P.n2 + (size_t)l * D, D, P.eps, sm, tid_c, wc, l, false);
+      stage_norm_ll<MAXP_D>(P.h_ll, P.h_flags, FG, tg_o, P.n2 + (size_t)l * D, D, P.eps, P.status, P.spin_limit, l, false);
       FB_STAMP(6);
       consume_tiles<CG, HZ, true>(pipe, g1 - g0, xs_, qs_, cw, lane, wc, l, [&](int row0, float c, int nvalid) {
         // rows (g_i, u_i, g_{i+1}, u_{i+1}) -> act[i], act[i+1] -> one tagged word
@@ -1000,7 +895,7 @@ __global__ void __launch_bounds__(kThreads, 1) decode_mega2(const __grid_constan
       FB_STAMP(7);
       // ================= down projection + residual =================
       {
-        stage_plain_ll<MAXP_F>(P.act_ll, P.act_flags, FG, tg_gu, FF, sm, tid_c, wc, l);
+        stage_plain_ll<imax(MAXP_O, MAXP_F)>(P.act_ll, P.act_flags, FG, tg_gu, FF, P.status, P.spin_limit, l);
         FB_STAMP(8);
         consume_tiles<CF, HZ, true>(pipe, o1 - o0, xs_, qs_, cw, lane, wc, l,
                                   [&](int row0, float c, int nvalid) { resid_epi(row0, c, nvalid, tg_dn, 1); });
@@ -1011,7 +906,7 @@ __global__ void __launch_bounds__(kThreads, 1) decode_mega2(const __grid_constan
     }
 #undef FB_STAMP
     // ================= final norm + LM head + arg-max =================
-    stage_norm_ll<MAXP_D>(P.h_ll, P.h_flags, FG, mk_tag(P.tag_base, L - 1, PH_DOWN), P.nf, D, P.eps, sm, tid_c, wc, L, false);
+    stage_norm_ll<MAXP_D>(P.h_ll, P.h_flags, FG, mk_tag(P.tag_base, L - 1, PH_DOWN), P.nf, D, P.eps, P.status, P.spin_limit, L, false);
     float bv = -INFINITY;
     int bi = 0x7fffffff;
     consume_tiles<CG, HZ, true>(pipe, l1 - l0, xs_, qs_, cw, lane, wc, L, [&](int row0, float c, int nvalid) {
@@ -1032,6 +927,7 @@ __global__ void __launch_bounds__(kThreads, 1) decode_mega2(const __grid_constan
     named_bar_sync(kBarConsumers, kConsumerThreads);
     const uint32_t tg_lm = mk_tag(P.tag_base, L, PH_LM);
     if (tid_c == 0) {
+#pragma unroll 1
       for (int w = 1; w < kConsumerWarps; w++)
         if (sm.red[w] > bv || (sm.red[w] == bv && sm.misc[w] < bi)) { bv = sm.red[w]; bi = sm.misc[w]; }
       ll_store(P.cand_ll + 2 * b, __float_as_uint(bv), tg_lm);
@@ -1045,6 +941,7 @@ __global__ void __launch_bounds__(kThreads, 1) decode_mega2(const __grid_constan
       if (cw == 0) {
         float v = -INFINITY;
         int ix = 0x7fffffff;
+#pragma unroll 1
         for (int c = lane; c < G; c += 32) {
           const float ov = __uint_as_float(cs[2 * c]);
           const int oi = (int)cs[2 * c + 1];
@@ -1059,12 +956,14 @@ __global__ void __launch_bounds__(kThreads, 1) decode_mega2(const __grid_constan
         if (N > 1 && lane == 0) {
           // every rank holds a slice of the vocabulary: exchange the N (value, index) candidates, reduce in rank order
           uint64_t* mine = P.inbox + (size_t)2 * N * D;
+#pragma unroll 1
           for (int p = 0; p < N; p++) {
             uint64_t* dst = (p == me ? mine : P.peer_inbox[p] + (size_t)2 * N * D) + 2 * me;
             ll_store_sys(dst, __float_as_uint(v), tg_lm);
             ll_store_sys(dst + 1, (uint32_t)ix, tg_lm);
           }
           v = -INFINITY; ix = 0x7fffffff;
+#pragma unroll 1
           for (int s2 = 0; s2 < N; s2++) {
             const float ov = __uint_as_float(ll_poll_sys(mine + 2 * s2, tg_lm, wc, L));
             const int oi = (int)ll_poll_sys(mine + 2 * s2 + 1, tg_lm, wc, L);
@@ -1076,6 +975,7 @@ __global__ void __launch_bounds__(kThreads, 1) decode_mega2(const __grid_constan
     }
     // final residual back to the caller (the reference clobbers its h argument): every CTA writes its own rows
     if (P.d_h)
+#pragma unroll 1
       for (int r = tid_c; r < o1 - o0; r += kConsumerThreads) P.d_h[o0 + r] = f2bf(hown[r]);
   }
   __syncthreads();

@@ -76,27 +76,34 @@ __device__ __forceinline__ void cta_rows(int rows, int unit, int b, int G, int& 
 }
 
 // ------------------------------------------------------------------------------------------------ producer side
+// The number of copies in flight is kept short: with the whole ring in flight (27 MB over 148 SMs) every small
+// latency-critical access of the consumers (flags, tagged words) waits microseconds behind bulk weight traffic. The trailing
+// wait of stage_issued also tells the consumers which loads have landed: one may only wait for load i on a stage's
+// one-bit phase once load i - kStages is known to be complete.
+__device__ __forceinline__ bool stage_slot(const Pipe& p, const WaitCtl& wc, int layer) {
+  return mbar_wait_far(&p.empty[p.it % kStages], ((p.it / kStages) & 1) ^ 1, wc, W_EMPTY, layer);     // p.it counts issued loads only
+}
+__device__ __forceinline__ bool stage_issued(Pipe& p, const WaitCtl& wc, int layer) {
+  p.it++;
+  if (p.it > p.max_fly) {
+    const uint32_t j = p.it - 1 - p.max_fly;
+    if (!mbar_wait_far(&p.full[j % kStages], (j / kStages) & 1, wc, W_FULL, layer)) return false;
+    *p.landed = (int)(j + 1);
+  }
+  return true;
+}
 // `src` points at the tile that holds the first of `nrows` rows; `tile_rows` rows (whole tiles) travel per stage.
 __device__ __forceinline__ bool produce_rows(Pipe& p, const uint8_t* src, int nrows, int tile_rows, int rt, int rec,
                                              const WaitCtl& wc, int layer) {
+#pragma unroll 1
   for (int r = 0; r < nrows; r += tile_rows) {
     const int n = (min(tile_rows, nrows - r) + rt - 1) / rt * rt;             // the last tile may be partly padding
     const uint32_t bytes = (uint32_t)n * rec;
+    if (!stage_slot(p, wc, layer)) return false;
     const int s = p.it % kStages;
-    const uint32_t ph = (p.it / kStages) & 1;
-    if (!mbar_wait(&p.empty[s], ph ^ 1, wc, W_EMPTY, layer)) return false;   // p.it counts issued loads only
     mbar_expect_tx(&p.full[s], bytes);
     bulk_g2s(p.stages + (size_t)s * kStageBytes, src + (size_t)r * rec, bytes, &p.full[s]);
-    p.it++;
-    // Keep the memory system's queues short: with the whole ring in flight (27 MB over 148 SMs) every small
-    // latency-critical access of the consumers (flags, tagged words) waits microseconds behind bulk weight traffic.
-    // The same wait tells the consumers which loads have landed: a consumer may only wait for load i on a stage's
-    // one-bit phase once load i - kStages is known to be complete.
-    if (p.it > p.max_fly) {
-      const uint32_t j = p.it - 1 - p.max_fly;
-      if (!mbar_wait(&p.full[j % kStages], (j / kStages) & 1, wc, W_FULL, layer)) return false;
-      *p.landed = (int)(j + 1);
-    }
+    if (!stage_issued(p, wc, layer)) return false;
   }
   return true;
 }
@@ -106,10 +113,12 @@ __device__ __forceinline__ bool produce_rows(Pipe& p, const uint8_t* src, int nr
 __device__ __forceinline__ void producer_drain(Pipe& p, const WaitCtl& wc) {
   if (*wc.s_abort == 0) return;
   const uint32_t n = p.it < (uint32_t)kStages ? p.it : (uint32_t)kStages;
+#pragma unroll 1
   for (uint32_t k = 0; k < n; k++) {
     const uint32_t it = p.it - 1 - k;
     const int s = it % kStages;
     const uint32_t ph = (it / kStages) & 1;
+#pragma unroll 1
     for (unsigned i = 0; i < wc.limit; i++) {
       if (mbar_try(&p.full[s], ph)) break;
       if ((i & 1023) == 1023) __nanosleep(64);
@@ -123,6 +132,23 @@ struct QueueState {
   int* tdone;
   int* bcnt;
 };
+
+// wait until stage load `it` has landed: on the stage's one-bit phase, once the stage's previous load is known to be complete
+__device__ __forceinline__ bool wait_stage(const Pipe& p, uint32_t it, const WaitCtl& wc, int layer) {
+  if (it >= (uint32_t)kStages) {
+    bool ok = false;
+#pragma unroll 1
+    for (unsigned i = 0; i < wc.limit; i++) {
+      if ((uint32_t)*p.landed > it - kStages) { ok = true; break; }
+      if ((i & 63) == 63 && *wc.s_abort) break;
+    }
+    if (!ok) {
+      if (*wc.s_abort == 0) report_fail_far(wc, W_LANDED, layer, (int)it, *p.landed);
+      return false;
+    }
+  }
+  return mbar_wait_far(&p.full[it % kStages], (it / kStages) & 1, wc, W_FULL, layer);
+}
 
 // GEMV over this CTA's `nrows` rows of one phase (they start on a tile boundary). Warp w takes slice w % KS of tiles
 // w / KS, w / KS + NL, ... in order. Every finished group of up to 4 rows is handed to `epi(row0_local, c, nvalid)` by
@@ -139,22 +165,12 @@ __device__ __forceinline__ void consume_tiles(Pipe& p, int nrows, const XStage& 
   const int nst = (nt + TPS - 1) / TPS;
   if (cw < NL * KS) {
     const int slice = cw % KS;
+#pragma unroll 1
     for (int tl = cw / KS; tl < nt; tl += NL) {
       const int st = tl / TPS, blk = tl % TPS;
       const uint32_t it = p.it + st;
       const int s = it % kStages;
-      if (it >= (uint32_t)kStages) {                 // the stage's previous load must be complete before its phase bit is read
-        bool ok = false;
-        for (unsigned i = 0; i < wc.limit; i++) {
-          if ((uint32_t)*p.landed > it - kStages) { ok = true; break; }
-          if ((i & 63) == 63 && *wc.s_abort) break;
-        }
-        if (!ok) {
-          if (*wc.s_abort == 0) report_fail(wc, W_LANDED, layer, (int)it, *p.landed);
-          break;
-        }
-      }
-      if (!mbar_wait(&p.full[s], (it / kStages) & 1, wc, W_FULL, layer)) break;
+      if (!wait_stage(p, it, wc, layer)) break;
       if (dbg && cw == 0 && lane == 0 && tl == 0) dbg[13] = (long long)globaltimer_ns();
       const uint8_t* tile = p.stages + (size_t)s * kStageBytes + (size_t)blk * TILE;
       const int nvalid_tile = min(RT, nrows - tl * RT);

@@ -1,0 +1,163 @@
+"""GPU: the ends of the ranges that the kernels' dispatch rules cut: chunks and ring stages of the decode attention, token tiles of the
+verify GEMMs and the prompt pass, weight scales too far apart for the short dequantisation, row slices of the token choice,
+row tiles of the draft head. Against the CPU oracle (or, for the token choice, the exact order of the input)."""
+import ctypes
+
+import numpy as np
+import pytest
+import torch
+
+from flint_b200 import _lib, packing
+from flint_b200.config import ModelArgs
+from flint_b200.draft import seeded_draft
+from flint_b200.engine import DecodeEngine
+from oracle import oracle as O
+from oracle.draft_oracle import DraftOracle, sample_probs
+
+pytestmark = pytest.mark.gpu
+
+
+def _tol(ref):
+    """2e-2 at the tiny config's largest |logit| of 2.56, the same relative bar elsewhere: the oracle alone moves by this much
+    when one bf16 ulp of one input element is flipped (tests/test_packer_oracle.py)."""
+    return 2e-2 * max(1.0, float(np.abs(ref).max()) / 2.56)
+
+
+def _f32(t):
+    return O.bf16_to_f32(t.detach().cpu().contiguous().view(torch.int16).numpy().view(np.uint16))
+
+
+def _pair(cfg, max_seq, T0, P=None, seed=7):
+    """Oracle and engine with the same T0 random cache rows; every later row of the device cache is NaN."""
+    P = packing.synth_packed(cfg, 0) if P is None else P
+    orc = O.OracleModel(cfg, P, max_seq)
+    eng = DecodeEngine(cfg, {k: v.cuda() for k, v in P.items()}, max_seq=max_seq)
+    kv = torch.randn(2, cfg.n_layer, T0, cfg.n_local_heads, cfg.head_dim, generator=torch.Generator().manual_seed(seed)).bfloat16()
+    eng.kc.fill_(float("nan"))
+    eng.vc.fill_(float("nan"))
+    for cache, host, rows in ((eng.kc, orc.kc, kv[0]), (eng.vc, orc.vc, kv[1])):
+        cache[:, :T0].copy_(rows)
+        host[:, :T0] = rows.view(torch.int16).numpy().view(np.uint16)
+    return orc, eng
+
+
+# (head_dim, query heads per kv head, positions per ring stage)
+SHAPES = {"llama-1b-class": 64, "granite-4.1-3b": 64, "granite-3b-class": 64, "llama-8b-class": 32}
+
+
+@pytest.mark.parametrize("T0", ["one", "unit", "stage-1", "stage", "chunk-1", "chunk", "chunk+1", "many"])
+@pytest.mark.parametrize("name", sorted(SHAPES))
+def test_decode_attention_at_unit_stage_and_chunk_edges(name, T0):
+    """Cached lengths where this step's own row is the only one, starts a unit of 16, ends or opens a ring stage, a chunk (two stages) or a
+    second chunk, for every head geometry; one layer, 512 tokens of vocabulary."""
+    nps = SHAPES[name]
+    pos = {"one": 0, "unit": 16, "stage-1": nps - 1, "stage": nps, "chunk-1": 2 * nps - 1, "chunk": 2 * nps, "chunk+1": 2 * nps + 1,
+           "many": 39 * nps + 5}[T0]
+    cfg = ModelArgs.from_name(name)
+    cfg.n_layer, cfg.vocab_size = 1, 512
+    orc, eng = _pair(cfg, pos + 4, pos)
+    for i, t in enumerate((17, 400)):
+        ref = orc.decode(t, pos + i)
+        got = eng.decode(t, pos + i).cpu().numpy()
+        eng.check()
+        assert np.abs(got - ref).max() < _tol(ref)
+    eng.close()
+
+
+@pytest.mark.parametrize("asym", [False, True])
+@pytest.mark.parametrize("M", [17, 32, 33, 63, 64])
+def test_verify_token_tile_edges(M, asym):
+    """The token tiles of the tree GEMMs and the row tiles of the attention: one past and exactly full tiles, the largest tree."""
+    cfg = ModelArgs.from_name("tiny")
+    orc, eng = _pair(cfg, 128, 9, packing.synth_packed(cfg, 0, asym=asym))
+    toks = torch.randint(0, cfg.vocab_size, (M,), generator=torch.Generator().manual_seed(M)).tolist()
+    ref, _ = orc.verify(toks, 9)
+    lg, _ = eng.verify(toks, 9)
+    eng.check()
+    assert np.abs(lg.cpu().numpy() - ref).max() < _tol(ref)
+    assert np.abs(_f32(eng.kc[:, 9:9 + M]) - O.bf16_to_f32(orc.kc[:, 9:9 + M])).max() < 0.05
+    eng.close()
+
+
+@pytest.mark.parametrize("M", [5, 40, 70])
+def test_weight_scales_far_apart_take_the_long_dequantisation(M):
+    """Scales of one row 2^12 apart (every third group of every second row shrunk): blocks that the one-fma form cannot hold exactly, next
+    to blocks that it can, in the tree GEMM (5, 40 tokens) and the prompt GEMM (70)."""
+    cfg = ModelArgs.from_name("tiny")
+    P = packing.synth_packed(cfg, 0)
+    for k in ("qkv_s", "o_s", "gu_s", "d_s"):
+        P[k] = P[k].clone()
+        P[k][..., ::2, ::3] *= 2.0 ** -12
+    orc, eng = _pair(cfg, 128, 6, P)
+    toks = torch.randint(0, cfg.vocab_size, (M,), generator=torch.Generator().manual_seed(M)).tolist()
+    ref = np.concatenate([orc.verify(toks[i:i + 40], 6 + i)[0] for i in range(0, M, 40)])
+    lg, _ = (eng.prefill if M > 64 else eng.verify)(toks, 6)
+    eng.check()
+    assert np.abs(lg.cpu().numpy() - ref).max() < _tol(ref)
+    eng.close()
+
+
+@pytest.mark.parametrize("M", [1, 65, 127, 128, 129, 1024, 1025])
+def test_prompt_pass_tile_and_chunk_edges(M):
+    """Prompt passes around the 128-token tile and around the 1024 rows of one pass, behind 3 cached rows: logits of the last
+    rows and every cache row against the oracle, which takes the prompt in pieces of 64."""
+    cfg = ModelArgs.from_name("tiny")
+    cfg.n_layer = 2
+    orc, eng = _pair(cfg, M + 8, 3)
+    toks = torch.randint(0, cfg.vocab_size, (M,), generator=torch.Generator().manual_seed(M)).tolist()
+    for i in range(0, M, 64):
+        ref, _ = orc.verify(toks[i:i + 64], 3 + i)
+    lg, _ = eng.prefill(toks, 3)
+    eng.check()
+    n = len(ref)
+    assert np.abs(lg[M - n:].cpu().numpy() - ref).max() < _tol(ref)
+    for dev, host in ((eng.kc, orc.kc), (eng.vc, orc.vc)):
+        assert np.abs(_f32(dev[:, 3:3 + M]) - O.bf16_to_f32(host[:, 3:3 + M])).max() < 0.05
+    eng.close()
+
+
+@pytest.mark.parametrize("vocab", [1, 31, 4096, 8200, 32768, 49160, 128256, 300001])
+def test_token_choice_over_every_split_of_a_row(vocab):
+    """Rows on one, two, four and eight CTAs, slices that fit the registers and slices that do not, ragged ends: the arg-max
+    (first index on a tie at the two ends of the row), draws confined to the top-k entries, and the k = 1 draw."""
+    cfg = ModelArgs.from_name("tiny")
+    eng = DecodeEngine(cfg, {k: v.cuda() for k, v in packing.synth_packed(cfg, 0).items()}, max_seq=8)
+    lg = torch.randn(3, vocab, generator=torch.Generator().manual_seed(vocab)).cuda()
+    lg[1, 0] = lg[1, vocab - 1] = 9.0
+    lg[2, vocab - 1] = 11.0
+    assert eng.sample(lg, 0.0).tolist() == [int(lg[0].argmax()), 0, vocab - 1]
+    assert eng.sample(lg[2], 0.8, 1, seed=5).tolist() == [vocab - 1]
+    for k in (2, 50):
+        n = 256
+        out = torch.empty(n, dtype=torch.int32, device="cuda")
+        _lib.check(eng.lib.fb_sample(ctypes.c_void_p(lg.data_ptr()), vocab, n, 0, 1.0, k, 3, 0, ctypes.c_void_p(out.data_ptr()), None), "fb_sample")
+        p = sample_probs(lg[0].cpu().numpy(), 1.0, k)
+        assert np.all(p[out.cpu().numpy()] > 0)
+        if vocab > 50:
+            assert len(set(out.tolist())) > 1
+    eng.close()
+
+
+@pytest.mark.parametrize("T", [1, 7, 8, 9, 16, 17, 33])
+def test_draft_row_tile_edges(T):
+    """The draft head's linears take 8 rows per MMA tile: below, at and above one, two and four tiles."""
+    dim, nh, nkv, inter, vocab = 256, 8, 2, 512, 1000
+    m = seeded_draft(dim, nh, inter, seed=5, rope_base=10000.0, n_kv=nkv, fuse=2)
+    g = torch.Generator().manual_seed(T)
+    embed = (torch.randn(vocab, dim, generator=g) * 0.5).bfloat16().cuda()
+    nf = (torch.rand(dim, generator=g) + 0.5).bfloat16().cuda()
+    m.bind_target(embed, nf, logits_scaling=4.0)
+    m.setup_cache(48)
+    orc = DraftOracle({k: _f32(v) for k, v in m._w.items()}, nh, 10000.0, max_roll=48, n_kv=nkv)
+    feat = torch.randn(T, 2 * dim, generator=g).bfloat16().cuda()
+    toks = torch.randint(-1, vocab, (T,), generator=g).to(torch.int32)
+    pos = torch.arange(T, dtype=torch.int32)
+    out = m(feat, None, pos.cuda(), input_pos=pos.cuda(), tokens=toks.cuda())
+    emb = np.stack([_f32(embed[t]) if t >= 0 else np.zeros(dim, np.float32) for t in toks.tolist()])
+    ref = orc.forward(_f32(feat), emb, pos.numpy(), slots=np.arange(T))
+    assert np.abs(_f32(out) - ref).max() <= 2e-2 * np.abs(ref).max()         # as in the rollout test: bf16 between the layers
+    t_dev, s_dev = m.head(out[:16], top_b=3, want_scores=True)          # at most 16 rows a call
+    lg = orc.head_logits(_f32(out[:16]), _f32(nf), _f32(embed), 4.0)              # the head alone: same input rows on both sides
+    top = -np.sort(-lg, axis=1)[:, :3]
+    assert np.abs(s_dev.cpu().numpy() - top).max() <= 2.0 ** -6 * np.abs(lg).max()      # bf16 logits: 2^-9, a near-tie may swap ranks
+    assert np.all(np.take_along_axis(lg, t_dev.cpu().numpy().astype(np.int64), 1) >= top[:, 2:] - 2.0 ** -6 * np.abs(lg).max())
