@@ -235,7 +235,8 @@ int fb_gemv_static(const void* d_q, const void* d_s, const void* d_z, int32_t ro
  *           builds (reference: kernels/megakernel_decode.cu:15-24)
  *   what 4: bulk weight copies one CTA keeps in flight at once (1..4, default 4)
  *   what 5: 1 = consumers poll the tagged activation words directly; 0 = they wait for the producers' arrival flags first
- *   what 8: 0..2, accepted without effect: the decode attention has one implementation (K/V through the weight ring).
+ *   what 7: 0..4, accepted without effect (it selected between several GEMM implementations of fb_verify)
+ *   what 8: 0..2, accepted without effect (it selected between two attention implementations of fb_decode)
  */
 int fb_set_option(fb_ctx* ctx, int32_t what, int64_t value);
 
