@@ -80,6 +80,21 @@ int chunks_for(const fb_ctx* c, int T) {
   return n < c->maxchunks ? n : c->maxchunks;
 }
 
+// Bulk copies a CTA keeps in flight while the layers run. A layer that brings each SM at most two rings of weights and K/V spends far
+// longer on its hand-overs than one copy at a time (about 2.2 TB/s over all SMs) takes, and the flags and tagged words then wait
+// behind less bulk traffic; more bytes need the full rate. Microseconds a token at 4 / 2 / 1 copies: 1B-class (1.2 rings a layer) 394 / 392 /
+// 388, 3B-class (1.5) 1002 / 992 / 983, the same behind 2000 positions (1.7) 1037 / 1031 / 1023, 8B-class (4.5) 1621 / 1667 / 1759. The LM
+// head has no hand-over to disturb: always 4.
+int fly_for(const fb_ctx* c, int T) {
+  if (c->max_fly) return c->max_fly;
+  const fb_model_desc& d = c->d;
+  const int HD = d.head_dim, hz = d.has_zeros ? 1 : 0;
+  const int64_t bytes = (int64_t)(d.n_head + 2 * d.n_kv_head) * HD * rec_bytes_of(d.dim, hz) + (int64_t)d.dim * rec_bytes_of(c->ko, hz) +
+                        (int64_t)2 * d.ffn * rec_bytes_of(d.dim, hz) + (int64_t)d.dim * rec_bytes_of(d.ffn, hz) +
+                        (int64_t)T * d.n_kv_head * HD * 4;
+  return bytes <= (int64_t)2 * kStages * kStageBytes * c->sm_count ? 1 : 4;
+}
+
 // every K the stand-alone entry points (re-layout, dequantise, GEMV) are built for
 #ifndef FB_EXTRA_K
 #define FB_EXTRA_K(X)                             // widths of the build-time extra shapes that this list lacks
@@ -208,7 +223,6 @@ int fb_ctx_create_tp(const fb_model_desc* desc, int device, int32_t tp_rank, int
   c->kernel_id = kid;
   c->rgqa = d.n_head / d.n_kv_head;
   c->spin_limit = 4000000u;
-  c->max_fly = 4;
   c->tp_size = tp_size; c->tp_rank = tp_rank; c->vocab_base = vocab_base; c->ko = ko; c->ao_off = ao_off;
   c->tag_base = 8;
   c->maxchunks = c->sm_count / d.n_kv_head;
@@ -474,7 +488,7 @@ int fb_decode(fb_ctx* c, int32_t token, const int32_t* d_token, void* d_h, int32
   if (c->tag_base > 0xffffffffu - 2 * span) c->tag_base = 8;      // tags never reach 0 (the value of fresh buffers)
   Q.tag_base = c->tag_base; Q.spin_limit = c->spin_limit;
   Q.eps = d.rms_eps; Q.attn_scale = d.attn_scale; Q.resid = d.resid_mult; Q.emb_mult = d.emb_mult;
-  Q.logits_scaling = d.logits_scaling; Q.prof = c->prof; Q.max_fly = (unsigned)c->max_fly; Q.poll_words = c->poll_words;
+  Q.logits_scaling = d.logits_scaling; Q.prof = c->prof; Q.max_fly = (unsigned)fly_for(c, pos + 1); Q.lm_fly = c->max_fly ? Q.max_fly : 4u; Q.poll_words = c->poll_words;
   Q.tp_size = c->tp_size; Q.tp_rank = c->tp_rank; Q.vocab_base = c->vocab_base; Q.inbox = c->inbox; Q.ao_off = c->ao_off;
   for (int p = 0; p < c->tp_size; p++) {
     if (!c->peer_inbox[p]) return FB_ERR_STATE;       /* fb_tp_connect has not been called */

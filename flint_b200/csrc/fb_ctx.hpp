@@ -37,7 +37,7 @@ struct fb_ctx {
   unsigned* vamax;                                                  // per token: bound on the attention output (float bits)
   unsigned* gu_norms;                                               // [n_layer][2] largest squared row norms of gate and up (float bits)
   void* vrope;                                                      // verify: (cos, sin) per (token, rotation pair)
-  int max_fly, poll_words;
+  int max_fly, poll_words;                                          // max_fly 0: chosen by the bytes of a layer (fly_for)
   CUtensorMap kmap, vmap;                                           // the caches as tensors (make_kv_maps)
 };
 

@@ -635,7 +635,7 @@ struct Decode2Params {
   unsigned tag_base, spin_limit;
   float eps, attn_scale, resid, emb_mult, logits_scaling;
   long long* prof;
-  unsigned max_fly;
+  unsigned max_fly, lm_fly;   // bulk copies in flight per CTA while the layers run, and for the LM head
   int32_t poll_words;         // 1: consumers poll the tagged words themselves instead of waiting for arrival flags first
   // tensor parallelism: this GPU holds a slice of every matrix (heads, FFN columns, vocabulary rows); the partial sums
   // of the K-sharded O and down projections are exchanged by peer stores into every rank's inbox
@@ -706,6 +706,7 @@ __global__ void __launch_bounds__(kThreads, 1) decode_mega2(const __grid_constan
              produce_rows(pipe, P.w_gu + l * strG + (size_t)g0 * recD, g1 - g0, CG::TILE_ROWS, CG::RT, recD, wc, l) &&
              produce_rows(pipe, P.w_d + l * strF + (size_t)o0 * recF, o1 - o0, CF::TILE_ROWS, CF::RT, recF, wc, l);
       }
+      pipe.max_fly = P.lm_fly;
       if (ok) produce_rows(pipe, P.w_lm + (size_t)l0 * recD, l1 - l0, CG::TILE_ROWS, CG::RT, recD, wc, L);
       producer_drain(pipe, wc);
     }
