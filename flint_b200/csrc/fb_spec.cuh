@@ -38,6 +38,7 @@ struct SampleParams {
   float temperature;            // <= 0: arg-max (first index of the maximum)
   unsigned long long seed, counter;   // row r draws from stream (seed, counter + r)
   int32_t* out;                 // [rows] token ids
+  int32_t ctas;                 // CTAs (one cluster) of a row
 };
 
 // One cluster of CTAs per row: a CTA keeps its slice of the row in registers (up to 16 values a thread; longer slices are read again),
@@ -76,7 +77,8 @@ __device__ __forceinline__ void warp_best(float& bv, int& bi) {
   }
 }
 
-// grid (CTAs per row = cluster, rows), 1024 threads
+// grid (rows * CTAs per row), clusters of one row's CTAs, 1024 threads. Rows lie on grid.x: grid.y ends at 65535, and a program may
+// draw any number of rows from one vector (stride 0).
 template <bool REG>
 __global__ void __launch_bounds__(1024) sample_rows(const SampleParams P) {
   __shared__ __align__(8) unsigned hist[3][2048];
@@ -85,7 +87,7 @@ __global__ void __launch_bounds__(1024) sample_rows(const SampleParams P) {
   __shared__ int s_i[32];
   __shared__ float c_v[16];                       // the CTAs' candidates, in the first CTA
   __shared__ int c_i[16];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, row = blockIdx.y, C = gridDim.x, rank = blockIdx.x;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, C = P.ctas, row = blockIdx.x / C, rank = blockIdx.x % C;
   const float* lg = P.logits + (long long)row * P.row_stride;
   const int per = (P.vocab + C - 1) / C, i0 = rank * per, i1 = min(P.vocab, i0 + per);
   const bool draw = P.temperature > 0.f, select = draw && P.top_k > 0 && P.top_k < P.vocab;

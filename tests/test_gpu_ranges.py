@@ -138,6 +138,26 @@ def test_token_choice_over_every_split_of_a_row(vocab):
     eng.close()
 
 
+def _sample(eng, lg, vocab, rows, top_k, counter):
+    out = torch.full((rows,), -1, dtype=torch.int32, device="cuda")
+    _lib.check(eng.lib.fb_sample(ctypes.c_void_p(lg.data_ptr()), vocab, rows, 0, 1.0, top_k, 3, counter, ctypes.c_void_p(out.data_ptr()), None),
+               "fb_sample")
+    return out
+
+
+@pytest.mark.parametrize("vocab,top_k", [(300, 0), (300, 7), (8200, 0)])
+def test_token_choice_of_more_rows_than_a_grid_has_in_y(vocab, top_k):
+    """70 000 draws from one vector (stride 0) in one call. Row r draws from stream (seed, counter + r): every row equals a
+    short call that starts at its counter, below, across and above row 65 535."""
+    cfg = ModelArgs.from_name("tiny")
+    eng = DecodeEngine(cfg, {k: v.cuda() for k, v in packing.synth_packed(cfg, 0).items()}, max_seq=8)
+    lg = torch.randn(vocab, generator=torch.Generator().manual_seed(vocab)).cuda()
+    out = _sample(eng, lg, vocab, 70000, top_k, 11)
+    for r0 in (0, 65520, 69970):
+        assert torch.equal(out[r0:r0 + 30], _sample(eng, lg, vocab, 30, top_k, 11 + r0))
+    eng.close()
+
+
 @pytest.mark.parametrize("T", [1, 7, 8, 9, 16, 17, 33])
 def test_draft_row_tile_edges(T):
     """The draft head's linears take 8 rows per MMA tile: below, at and above one, two and four tiles."""
