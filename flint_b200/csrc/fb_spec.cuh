@@ -54,10 +54,11 @@ __device__ __forceinline__ uint32_t sm_map(uint32_t saddr, uint32_t rank) {
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(saddr), "r"(rank));
   return r;
 }
-__device__ __forceinline__ void sm_cluster_sync() {
-  asm volatile("barrier.cluster.arrive.release;" ::: "memory");
-  asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
-}
+__device__ __forceinline__ void sm_cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
+__device__ __forceinline__ void sm_cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
+__device__ __forceinline__ void sm_cluster_sync() { sm_cluster_arrive(); sm_cluster_wait(); }
+// Another CTA's shared memory may be touched only once that CTA is known to run. Every CTA of the cluster arrives at the start of the kernel
+// and waits before its first remote access: the row's loads lie in between and hide the barrier.
 __device__ __forceinline__ void sm_st(uint32_t a, uint32_t v) { asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory"); }
 __device__ __forceinline__ uint2 sm_ld2(uint32_t a) {
   uint2 v;
@@ -91,6 +92,7 @@ __global__ void __launch_bounds__(1024) sample_rows(const SampleParams P) {
   const float* lg = P.logits + (long long)row * P.row_stride;
   const int per = (P.vocab + C - 1) / C, i0 = rank * per, i1 = min(P.vocab, i0 + per);
   const bool draw = P.temperature > 0.f, select = draw && P.top_k > 0 && P.top_k < P.vocab;
+  if (!select) sm_cluster_arrive();               // the selection's own barriers come before its first remote read
   pdl_trigger();
   pdl_wait();
   float v[REG ? kSampleRegs : 1];
@@ -171,6 +173,7 @@ __global__ void __launch_bounds__(1024) sample_rows(const SampleParams P) {
   warp_best(bv, bi);
   if (lane == 0) { s_v[warp] = bv; s_i[warp] = bi; }
   __syncthreads();
+  if (!select) sm_cluster_wait();
   if (warp == 0) {
     bv = s_v[lane]; bi = s_i[lane];
     warp_best(bv, bi);
@@ -200,6 +203,7 @@ __global__ void __launch_bounds__(1024) topb_rows(const float* logits, long long
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, row = blockIdx.y, C = gridDim.x, rank = blockIdx.x;
   const float* lg = logits + (long long)row * row_stride;
   const int per = (vocab + C - 1) / C, i0 = rank * per, i1 = min(vocab, i0 + per);
+  sm_cluster_arrive();
   pdl_trigger();
   pdl_wait();
   float v[REG ? kSampleRegs : 1];
@@ -230,6 +234,7 @@ __global__ void __launch_bounds__(1024) topb_rows(const float* logits, long long
     warp_best(bv, bi);
     if (lane == 0) { s_v[warp] = bv; s_i[warp] = bi; }
     __syncthreads();
+    if (r == 0) sm_cluster_wait();
     if (warp == 0) {
       bv = s_v[lane]; bi = s_i[lane];
       warp_best(bv, bi);

@@ -158,6 +158,61 @@ def test_token_choice_of_more_rows_than_a_grid_has_in_y(vocab, top_k):
     eng.close()
 
 
+@pytest.mark.parametrize("vocab", [8200, 16390, 49160, 300001])
+@pytest.mark.parametrize("temperature,top_k", [(1.0, 0), (0.7, 5), (1.5, 400)])
+def test_sampled_frequencies_of_rows_on_several_ctas(vocab, temperature, top_k):
+    """20 000 draws from one row that 2, 4 or 8 CTAs share, with a run of equal values at the top-k threshold that crosses a slice boundary:
+    nothing outside the support, every frequency within 5 sigma (a threshold that keeps too few entries loses whole tokens)."""
+    cfg = ModelArgs.from_name("tiny")
+    eng = DecodeEngine(cfg, {k: v.cuda() for k, v in packing.synth_packed(cfg, 0).items()}, max_seq=8)
+    lg = torch.randn(vocab, generator=torch.Generator().manual_seed(vocab + top_k)) * 2.0
+    if top_k:
+        kth = torch.topk(lg, top_k).values[-1]
+        lg[vocab // 2 - 3:vocab // 2 + 3] = kth
+    n = 20000
+    lg = lg.cuda()
+    out = torch.empty(n, dtype=torch.int32, device="cuda")
+    _lib.check(eng.lib.fb_sample(ctypes.c_void_p(lg.data_ptr()), vocab, n, 0, temperature, top_k, 123, 0, ctypes.c_void_p(out.data_ptr()), None),
+               "fb_sample")
+    counts = np.bincount(out.cpu().numpy(), minlength=vocab).astype(np.float64)
+    p = sample_probs(lg.cpu().numpy(), temperature, top_k)
+    assert counts.size == vocab and counts[p == 0].sum() == 0
+    sigma = np.sqrt(n * p * (1 - p)) + 1.0
+    assert np.all(np.abs(counts - n * p) < 5 * sigma), float(np.max(np.abs(counts - n * p) / sigma))
+    eng.close()
+
+
+@pytest.mark.parametrize("top_b", [1, 3, 16])
+@pytest.mark.parametrize("vocab", [1000, 8200, 16390, 49160, 140000])
+def test_token_head_order_over_every_split_of_a_row(vocab, top_b):
+    """The B best tokens of rows on 1, 2, 4 and 8 CTAs, slices in registers and slices read again (140 000). One-hot feature rows make
+    the logits exactly 8 x one column of the embedding table, so the order (value descending, first index on ties) is known: a row of normal
+    values, whose bf16 ties are many; one whose winners all lie in one slice; one whose winners are ties on both sides of every slice
+    boundary; a constant row."""
+    dim = 64
+    m = seeded_draft(dim, 1, 64, seed=1, rope_base=10000.0)
+    g = torch.Generator().manual_seed(vocab)
+    embed = torch.randn(vocab, dim, generator=g).bfloat16()
+    ctas = 1
+    while ctas < 8 and vocab >= 8192 * ctas:
+        ctas *= 2
+    per = -(-vocab // ctas)
+    embed[:, 1].clamp_(max=2.0)
+    embed[per * (ctas - 1):per * (ctas - 1) + 20, 1] = torch.arange(20).bfloat16() / 4 + 4
+    for c in range(1, ctas):
+        embed[c * per - 2:c * per + 2, 2] = 6.0
+    embed[:, 3] = 1.0
+    m.bind_target(embed.cuda(), torch.ones(dim, dtype=torch.bfloat16, device="cuda"))
+    m.setup_cache(8)
+    rows = torch.zeros(4, dim, dtype=torch.bfloat16, device="cuda")
+    rows[torch.arange(4), torch.arange(4)] = 8.0              # mean square 1: the norm leaves 8
+    toks, scores = m.head(rows, top_b=top_b, want_scores=True)
+    for r in range(4):
+        v = 8.0 * embed[:, r].float().numpy()
+        order = np.lexsort((np.arange(vocab), -v))[:top_b]
+        assert toks[r].tolist() == order.tolist() and scores[r].tolist() == v[order].tolist()
+
+
 @pytest.mark.parametrize("T", [1, 7, 8, 9, 16, 17, 33])
 def test_draft_row_tile_edges(T):
     """The draft head's linears take 8 rows per MMA tile: below, at and above one, two and four tiles."""
