@@ -323,6 +323,11 @@ __device__ __forceinline__ void ldmatrix_x4_t(uint32_t (&r)[4], uint32_t addr) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
 }
+__device__ __forceinline__ int count_unit(int* n) {
+  int old;
+  asm volatile("atom.acq_rel.cta.shared::cta.add.s32 %0, [%1], 1;" : "=r"(old) : "r"(smem_u32(n)) : "memory");
+  return old;
+}
 
 // Flash-decode of this CTA's (kv head, chunk) items on the tensor pipe, K/V from the ring, at every cached length. Warp w takes units
 // of 16 positions w, w + 14, ...: the R query heads of the group are the rows of a 16-row MMA tile, the positions the N dimension of
@@ -475,7 +480,9 @@ __device__ __forceinline__ void attention_phase(const AttnArgs& a, uint8_t* scra
           }
         }
         __syncwarp();
-        if (lane == 0 && atomicAdd(tdone + sslot, 1) == SPLIT - 1) {   // the stage's last unit hands it back
+        // The stage's last unit hands it back. Stores of other units (the step's own row, the zeroed rows) must not land after the next
+        // copy into the stage: the counter's release and acquire order them before this lane, its proxy fence before the copy.
+        if (lane == 0 && count_unit(tdone + sslot) == SPLIT - 1) {
           tdone[sslot] = 0;
           asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
           mbar_arrive(&pipe.empty[sslot]);

@@ -64,6 +64,24 @@ def test_decode_attention_at_unit_stage_and_chunk_edges(name, T0):
     eng.close()
 
 
+@pytest.mark.parametrize("name", sorted(SHAPES))
+def test_decode_stages_that_warps_wrote_to_are_handed_back_whole(name):
+    """The attention stores this step's own row and zeros into ring stages that the weight stream takes over next: 100 launches at ragged
+    lengths (several units and stages per chunk) give the same bits every time, and the first of them the oracle's values."""
+    cfg = ModelArgs.from_name(name)
+    cfg.n_layer, cfg.vocab_size = 2, 512
+    for pos in (SHAPES[name] + 3, 21 * SHAPES[name] + 9):
+        orc, eng = _pair(cfg, pos + 4, pos)
+        ref, first = orc.decode(17, pos), eng.decode(17, pos).clone()
+        assert np.abs(first.cpu().numpy() - ref).max() < _tol(ref)
+        other = torch.zeros((), dtype=torch.int64, device="cuda")
+        for _ in range(100):
+            other += (eng.decode(17, pos) != first).sum()
+        eng.check()
+        assert int(other) == 0
+        eng.close()
+
+
 @pytest.mark.parametrize("asym", [False, True])
 @pytest.mark.parametrize("M", [17, 32, 33, 63, 64])
 def test_verify_token_tile_edges(M, asym):
