@@ -283,6 +283,14 @@ __device__ __forceinline__ void mma_f16_first(float (&c)[4], const uint32_t (&a)
 // this kernel has called it; pdl_wait() returns when the previous kernel has completed and its writes are visible.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// The kernels of a call read weights before they wait for their predecessor. Those are the caller's tensors, and whatever ran before the
+// call may have written them: the FIRST kernel of a call waits before it lets the next ones start. A draft step (two calls) with early
+// reads from the first kernel on 123.3 us, so 126.2; the first kernel launched in plain stream order instead 128.5, its first weights
+// requested into L2 ahead of the wait 133.8.
+__device__ __forceinline__ void pdl_begin(bool first) {
+  if (first) pdl_wait();
+  pdl_trigger();
+}
 
 // launch with programmatic stream serialisation: the kernel may start while its predecessor drains (see pdl_wait)
 // (`cluster` consecutive CTAs form a thread-block cluster)

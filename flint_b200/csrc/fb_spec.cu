@@ -180,9 +180,9 @@ int fb_draft_forward(fb_draft* r, const void* d_feat, const void* d_emb, const i
   p.W[0] = (const uint16_t*)r->w.merge; p.x0 = (const uint16_t*)d_feat; p.ldx0 = F; p.k0 = F;
   if (d_emb) { p.x1 = (const uint16_t*)d_emb; p.ldx1 = D; }
   else { p.x1 = (const uint16_t*)r->w.embed; p.ldx1 = D; p.x1_tokens = d_tokens; }
-  p.k1 = D; p.N[0] = D; p.T = T; p.y[0] = r->x; p.ldy[0] = D;
+  p.k1 = D; p.N[0] = D; p.T = T; p.y[0] = r->x; p.ldy[0] = D; p.first = true;
   FB_DCUDA(r, launch_linear<DL_STORE>(p, st));
-  FB_DCUDA(r, launch_pdl(d_rmsnorm, dim3(T), dim3(256), 0, st, (const uint16_t*)r->x, D, (const uint16_t*)r->w.n1, r->h, D, D, d.rms_eps));
+  FB_DCUDA(r, launch_pdl(d_rmsnorm, dim3(T), dim3(256), 0, st, (const uint16_t*)r->x, D, (const uint16_t*)r->w.n1, r->h, D, D, d.rms_eps, false));
   // q, k, v in one launch
   memset(&p, 0, sizeof(p));
   const void* qkvw[3] = {r->w.q, r->w.k, r->w.v};
@@ -200,7 +200,7 @@ int fb_draft_forward(fb_draft* r, const void* d_feat, const void* d_emb, const i
   p.W[0] = (const uint16_t*)r->w.o; p.x0 = r->att; p.ldx0 = D; p.k0 = D; p.N[0] = D; p.T = T; p.y[0] = r->x2; p.ldy[0] = D;
   p.resid = r->x; p.ldr = D;
   FB_DCUDA(r, launch_linear<DL_RESID>(p, st));
-  FB_DCUDA(r, launch_pdl(d_rmsnorm, dim3(T), dim3(256), 0, st, (const uint16_t*)r->x2, D, (const uint16_t*)r->w.n2, r->h, D, D, d.rms_eps));
+  FB_DCUDA(r, launch_pdl(d_rmsnorm, dim3(T), dim3(256), 0, st, (const uint16_t*)r->x2, D, (const uint16_t*)r->w.n2, r->h, D, D, d.rms_eps, false));
   // act = silu(gate h) * up h
   memset(&p, 0, sizeof(p));
   p.W[0] = (const uint16_t*)r->w.gate; p.W2 = (const uint16_t*)r->w.up; p.x0 = r->h; p.ldx0 = D; p.k0 = D; p.N[0] = d.inter; p.T = T;
@@ -230,7 +230,7 @@ int fb_draft_head(fb_draft* r, const void* d_feat_rows, int32_t n, int32_t top_b
   const int D = d.dim, F = d.fuse * d.dim;
   // the token head reads the HIGH slice (last dim elements) of the fused feature (reference: spec_mega.py:43-44)
   FB_DCUDA(r, launch_pdl(d_rmsnorm, dim3(n), dim3(256), 0, st, (const uint16_t*)d_feat_rows + (F - D), F, (const uint16_t*)r->w.nf, r->fn, D, D,
-                         d.rms_eps));
+                         d.rms_eps, true));
   DLin p;
   memset(&p, 0, sizeof(p));
   p.W[0] = (const uint16_t*)r->w.embed; p.x0 = r->fn; p.ldx0 = D; p.k0 = D; p.N[0] = d.vocab; p.T = n; p.yf = r->logits; p.ldy[0] = d.vocab;

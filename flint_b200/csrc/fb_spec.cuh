@@ -333,13 +333,14 @@ struct DLin {
   float* yf;                    // DL_LOGITS: f32 [T, N] = bf16(bf16(acc) / scale), rows ldy apart
   int ldy[3], ldr;
   float scale;
+  bool first;                   // the first kernel of a call
 };
 
 // y[t, n] = sum_k W[n, k] x[t, k] for up to 8 NT tokens (t0 ...) on the tensor pipe, weights read once. A CTA takes 16 MT rows of W and
 // its WARPS warps share K: warp w takes the 32-column chunks w, w + WARPS, ... A lane loads 16 bytes of row g (and g + 8) straight into
 // the A fragments of two MMA steps -- the order of columns inside a chunk does not matter as long as x is read the same way, 16 bytes of
 // token g at the same columns -- so nothing goes through shared memory but the warps' partial sums. HBM-bound: a warp keeps AH chunks of
-// weights and activations in flight; the first weights are requested before the previous kernel is waited for. (The CUDA-core form
+// weights and activations in flight; the first weights are requested before the previous kernel is waited for (see pdl_begin). (The CUDA-core form
 // read the weights once per 8 or 16 tokens and took 62 us for a 13 to 50 MB matrix at 32 tokens.)
 template <int NT, int MT, int WARPS, int MODE, bool CAT>
 __global__ void __launch_bounds__(WARPS * 32, NT == 1 ? 3 : 1) d_gemm(const DLin P, int t0) {
@@ -376,7 +377,7 @@ __global__ void __launch_bounds__(WARPS * 32, NT == 1 ? 3 : 1) d_gemm(const DLin
 #pragma unroll
         for (int h = 0; h < 2; h++) d[i][m][h] = ok ? __ldcs(reinterpret_cast<const uint4*>(wr[i][m][h] + c * 32)) : make_uint4(0, 0, 0, 0);
   };
-  pdl_trigger();
+  pdl_begin(P.first && t0 == 0);
 #pragma unroll
   for (int a = 0; a < AH; a++) load_w(warp + WARPS * a, wv[a]);
   pdl_wait();
@@ -476,10 +477,11 @@ __global__ void __launch_bounds__(WARPS * 32, NT == 1 ? 3 : 1) d_gemm(const DLin
 
 // y = bf16(bf16(x * r) * w), r = bf16(rsqrt(bf16(bf16(mean(bf16(x^2))) + eps))): RMSNorm as a bf16 PyTorch expression
 // evaluates it (reference: train/draft_model.py:9-10). One CTA of 256 threads per row.
-__global__ void __launch_bounds__(256) d_rmsnorm(const uint16_t* x, int ldx, const uint16_t* w, uint16_t* y, int ldy, int D, float eps) {
+__global__ void __launch_bounds__(256) d_rmsnorm(const uint16_t* x, int ldx, const uint16_t* w, uint16_t* y, int ldy, int D, float eps,
+                                                 bool first) {
   __shared__ float red[8];
   const int tid = threadIdx.x;
-  pdl_trigger();
+  pdl_begin(first);
   pdl_wait();
   const uint16_t* xr = x + (size_t)blockIdx.x * ldx;
   float ss = 0.f;

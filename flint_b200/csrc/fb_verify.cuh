@@ -19,8 +19,7 @@ __device__ __forceinline__ float2 pow2_for(float a) {
 __global__ void v_embed(const int32_t* tokens, const uint16_t* embed, const uint16_t* h_in, uint16_t* h, int D, int vocab,
                         float mult, int* status_code) {
   const int m = blockIdx.x;
-  pdl_trigger();
-  pdl_wait();
+  pdl_begin(true);
   int tok = 0;
   if (!h_in) {
     tok = tokens[m];

@@ -254,3 +254,39 @@ def test_draft_row_tile_edges(T):
     top = -np.sort(-lg, axis=1)[:, :3]
     assert np.abs(s_dev.cpu().numpy() - top).max() <= 2.0 ** -6 * np.abs(lg).max()      # bf16 logits: 2^-9, a near-tie may swap ranks
     assert np.all(np.take_along_axis(lg, t_dev.cpu().numpy().astype(np.int64), 1) >= top[:, 2:] - 2.0 ** -6 * np.abs(lg).max())
+
+
+def test_weights_written_just_before_a_call_are_the_ones_it_uses():
+    """The caller's weights are bound by pointer. A matrix product that writes the draft's merge matrix or its embedding table, and an
+    elementwise kernel that writes the target's norms, directly before a call on the same stream: the call gives what a call
+    long after them gives, bit for bit."""
+    dim = 512
+    m = seeded_draft(dim, 8, 1024, seed=5, rope_base=10000.0)
+    g = torch.Generator().manual_seed(2)
+    embed = torch.randn(4096, dim, generator=g).bfloat16().cuda()
+    m.bind_target(embed, torch.ones(dim, dtype=torch.bfloat16, device="cuda"))
+    m.setup_cache(48)
+    feat = torch.randn(40, dim, generator=g).bfloat16().cuda()
+    emb, pos = torch.randn(40, dim, generator=g).bfloat16().cuda(), torch.arange(40, dtype=torch.int32, device="cuda")
+    cfg = ModelArgs.from_name("tiny")
+    eng = DecodeEngine(cfg, {k: v.cuda() for k, v in packing.synth_packed(cfg, 0).items()}, max_seq=128)
+    a = [torch.randn(n, 2048, generator=g).bfloat16().cuda() * 0.02 for n in (dim, 4096)]
+    b = [torch.randn(2048, n, generator=g).bfloat16().cuda() for n in (2 * dim, dim)]
+    for i in range(20):
+        torch.mm(a[0], b[0] * (1 + i), out=m._w["merge.weight"])
+        out = m(feat, emb, pos, input_pos=pos)
+        torch.mm(a[1], b[1] * (1 + i), out=embed)
+        toks, scores = m.head(feat[:3], top_b=4, want_scores=True)
+        for k in ("n1", "n2", "nf"):
+            eng._keep[k].fill_(1.0 + 0.25 * i)
+        lg, ft = eng.verify(list(range(i, i + 20)), 0)
+        torch.cuda.synchronize()
+        assert torch.equal(out, m(feat, emb, pos, input_pos=pos))
+        toks2, scores2 = m.head(feat[:3], top_b=4, want_scores=True)
+        assert torch.equal(toks, toks2) and torch.equal(scores, scores2)
+        lg2, ft2 = eng.verify(list(range(i, i + 20)), 0)
+        assert torch.equal(lg, lg2) and torch.equal(ft, ft2)
+        assert i == 0 or not (torch.equal(out, last[0]) or torch.equal(scores, last[1]) or torch.equal(lg, last[2]))
+        last = (out, scores, lg)
+    eng.check()
+    eng.close()
