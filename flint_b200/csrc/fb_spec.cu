@@ -24,6 +24,7 @@ struct fb_draft {
 namespace {
 
 constexpr int kMaxHeadRows = 16;
+constexpr int kAttnSmem = 200 * 1024;            // d_attn holds a score per cache slot and the query: more than the 48 KB that need no asking
 
 template <int NT, int MT, int WARPS, int MODE>
 cudaError_t launch_linear_nt(const DLin& p, int t0, cudaStream_t st) {
@@ -130,6 +131,7 @@ int fb_draft_create(const fb_draft_desc* desc, int device, fb_draft** out) {
   const size_t T = d.max_tokens, D = d.dim, kvd = (size_t)d.n_kv_head * hd, F = (size_t)d.fuse * d.dim;
   cudaError_t e = cudaSuccess;
   auto A = [&](cudaError_t x) { if (e == cudaSuccess) e = x; };
+  A(cudaFuncSetAttribute(d_attn, cudaFuncAttributeMaxDynamicSharedMemorySize, kAttnSmem));
   A(dmalloc(&r->x, T * D * 2)); A(dmalloc(&r->h, T * D * 2)); A(dmalloc(&r->q, T * D * 2));
   A(dmalloc(&r->k, T * kvd * 2)); A(dmalloc(&r->v, T * kvd * 2)); A(dmalloc(&r->att, T * D * 2));
   A(dmalloc(&r->x2, T * D * 2)); A(dmalloc(&r->act, T * (size_t)d.inter * 2)); A(dmalloc(&r->hh, T * D * 2));

@@ -256,6 +256,22 @@ def test_draft_row_tile_edges(T):
     assert np.all(np.take_along_axis(lg, t_dev.cpu().numpy().astype(np.int64), 1) >= top[:, 2:] - 2.0 ** -6 * np.abs(lg).max())
 
 
+@pytest.mark.parametrize("slots", [12284, 20000])
+def test_draft_attention_over_a_large_cache(slots):
+    """A draft head whose score vector alone fills (12 284 slots), or exceeds, the 48 KB of shared memory that a kernel has without asking:
+    the same bits as with a small cache."""
+    dim, outs = 128, []
+    g = torch.Generator().manual_seed(4)
+    feat, emb = (torch.randn(5, dim, generator=g).bfloat16().cuda() for _ in range(2))
+    pos = torch.arange(5, dtype=torch.int32, device="cuda")
+    for n in (8, slots):
+        m = seeded_draft(dim, 2, 256, seed=5, rope_base=10000.0)
+        m.bind_target(torch.zeros(16, dim, dtype=torch.bfloat16, device="cuda"), torch.ones(dim, dtype=torch.bfloat16, device="cuda"))
+        m.setup_cache(n)
+        outs.append(m(feat, emb, pos, input_pos=pos))
+    assert torch.equal(outs[0], outs[1])
+
+
 def test_weights_written_just_before_a_call_are_the_ones_it_uses():
     """The caller's weights are bound by pointer. A matrix product that writes the draft's merge matrix or its embedding table, and an
     elementwise kernel that writes the target's norms, directly before a call on the same stream: the call gives what a call
