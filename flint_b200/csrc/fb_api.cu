@@ -145,21 +145,20 @@ cudaError_t launch_repack(const void* q, const void* s, const void* z, int layer
 
 // The caches as 4-D tensors for the decode kernel's producer: (column, column block of 64, kv head, n_layer * max_seq rows), box =
 // one block x one head x one ring stage of positions; 128-byte blocks are swizzled (AttnCfg). Head dimensions that are no
-// multiple of 64 are one unswizzled block.
-cudaError_t make_kv_maps(fb_ctx* c) {
+// multiple of 64 are one unswizzled block. maps: K, V.
+cudaError_t make_kv_maps(const fb_ctx* c, void* kc, void* vc, int max_seq, CUtensorMap (&maps)[2]) {
   EncodeFn fn = tensor_map_encoder();
   if (!fn) return cudaErrorNotSupported;
   const fb_model_desc& d = c->d;
   const int HD = d.head_dim, bcols = HD % 64 == 0 ? 64 : HD;
   const cuuint64_t row = (cuuint64_t)d.n_kv_head * HD * 2;
-  const cuuint64_t dims[4] = {(cuuint64_t)bcols, (cuuint64_t)(HD / bcols), (cuuint64_t)d.n_kv_head, (cuuint64_t)d.n_layer * (cuuint64_t)c->max_seq};
+  const cuuint64_t dims[4] = {(cuuint64_t)bcols, (cuuint64_t)(HD / bcols), (cuuint64_t)d.n_kv_head, (cuuint64_t)d.n_layer * (cuuint64_t)max_seq};
   const cuuint64_t strides[3] = {(cuuint64_t)bcols * 2, (cuuint64_t)HD * 2, row};
   const cuuint32_t box[4] = {(cuuint32_t)bcols, 1u, 1u, (cuuint32_t)kDecodeKernels[c->kernel_id].nps};
   const cuuint32_t estr[4] = {1u, 1u, 1u, 1u};
-  void* bases[2] = {c->kc, c->vc};
-  CUtensorMap* maps[2] = {&c->kmap, &c->vmap};
+  void* bases[2] = {kc, vc};
   for (int i = 0; i < 2; i++)
-    if (fn(maps[i], CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, bases[i], dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+    if (fn(&maps[i], CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, bases[i], dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
            bcols == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
       return cudaErrorInvalidValue;
@@ -453,9 +452,10 @@ int fb_bind_weights(fb_ctx* c, const fb_weight_ptrs* w, void* stream) {
 int fb_bind_kv(fb_ctx* c, void* d_k, void* d_v, int32_t max_seq) {
   if (!c || !d_k || !d_v || max_seq <= 0) return FB_ERR_ARG;
   if (((uintptr_t)d_k & 15) || ((uintptr_t)d_v & 15)) return FB_ERR_ARG;
-  c->kc = d_k; c->vc = d_v; c->max_seq = max_seq;
   DeviceGuard g(c->device);
-  FB_CUDA(c, make_kv_maps(c));
+  CUtensorMap maps[2];
+  FB_CUDA(c, make_kv_maps(c, d_k, d_v, max_seq, maps));        // refused: the context keeps the cache that it had, or none
+  c->kc = d_k; c->vc = d_v; c->max_seq = max_seq; c->kmap = maps[0]; c->vmap = maps[1];
   return FB_OK;
 }
 

@@ -41,6 +41,23 @@ def _pair(cfg, max_seq, T0, P=None, seed=7):
     return orc, eng
 
 
+def test_a_refused_cache_leaves_the_bound_one_in_place():
+    """fb_bind_kv of a cache that no tensor map can describe (4 layers of 2^31 - 1 positions: more than 2^32 rows) is an error, and the next
+    step runs on the cache that was bound before."""
+    cfg = ModelArgs.from_name("tiny")
+    orc, eng = _pair(cfg, 16, 5)
+    k, v = (torch.zeros_like(eng.kc) for _ in range(2))
+    rc = eng.lib.fb_bind_kv(eng._ctx, ctypes.c_void_p(k.data_ptr()), ctypes.c_void_p(v.data_ptr()), 2 ** 31 - 1)
+    assert rc == _lib.FB_ERR_CUDA
+    ref = orc.decode(17, 5)
+    with pytest.raises(_lib.FlintError):
+        eng.decode(17, 16)                                    # still the bound cache's length
+    got = eng.decode(17, 5).cpu().numpy()
+    eng.check()
+    assert np.abs(got - ref).max() < _tol(ref) and not k.any() and not v.any()
+    eng.close()
+
+
 # (head_dim, query heads per kv head, positions per ring stage)
 SHAPES = {"llama-1b-class": 64, "granite-4.1-3b": 64, "granite-3b-class": 64, "llama-8b-class": 32}
 
