@@ -254,7 +254,7 @@ int fb_verify(fb_ctx* c, const int32_t* d_tokens, const void* d_h, const int32_t
   if (c->tp_size > 1) return FB_ERR_STATE;           /* a tensor-parallel rank holds slices only */
   if (!d_h && !c->embed) return FB_ERR_STATE;
   if (M < 1 || M > 64) return FB_ERR_RANGE;          /* never fall through to another M (reference: result.md:112-113) */
-  if (pos < 0 || pos + M > c->max_seq) return FB_ERR_RANGE;
+  if (pos < 0 || M > c->max_seq - pos) return FB_ERR_RANGE;
   DeviceGuard g(c->device);
   return run_tc_pass(c, d_tokens, d_h, d_depth, d_amask, M, pos, d_logits, d_feat, (cudaStream_t)stream);
 }

@@ -114,6 +114,18 @@ def test_verify_token_tile_edges(M, asym):
     eng.close()
 
 
+def test_positions_near_the_end_of_the_integers_are_out_of_range():
+    """pos + M past 2^31 - 1: refused like every position behind the cache, for trees, prompts and single steps."""
+    cfg = ModelArgs.from_name("tiny")
+    eng = DecodeEngine(cfg, {k: v.cuda() for k, v in packing.synth_packed(cfg, 0).items()}, max_seq=128)
+    for pos in (2 ** 31 - 1, 2 ** 31 - 20, 128, -1):
+        for call in (lambda: eng.verify(list(range(30)), pos), lambda: eng.prefill(list(range(30)), pos), lambda: eng.decode(3, pos)):
+            with pytest.raises(_lib.FlintError) as ei:
+                call()
+            assert ei.value.code == _lib.FB_ERR_RANGE
+    eng.close()
+
+
 @pytest.mark.parametrize("M", [5, 40, 70])
 def test_weight_scales_far_apart_take_the_long_dequantisation(M):
     """Scales of one row 2^12 apart (every third group of every second row shrunk): blocks that the one-fma form cannot hold exactly, next
