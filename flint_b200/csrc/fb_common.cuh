@@ -134,7 +134,27 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* b, uint32_t parity, const Wa
   return false;
 }
 
-// The same out of line, for the decode kernel, whose per-layer code does not fit the instruction cache: what a healthy step
+// Before a CTA may exit, every copy and MMA that it issued has to have completed its barrier phase. In a healthy launch somebody has waited for
+// each of them; after a failure of any role (known for sure only behind the CTA's last barrier) whoever issued them does, with a limit of its
+// own, because a caller may set the limit of the other waits to nothing.
+constexpr unsigned kDrainLimit = 1u << 20;
+__device__ __forceinline__ void drain_phase(uint64_t* b, uint32_t parity) {
+#pragma unroll 1
+  for (unsigned i = 0; i < kDrainLimit; i++) {
+    if (mbar_try(b, parity)) return;
+    if ((i & 1023) == 1023) __nanosleep(64);
+  }
+}
+
+// the same for the last (up to) N of `issued` copies into a ring of N stages
+template <int N>
+__device__ __forceinline__ void drain_ring(uint64_t* full, uint32_t issued) {
+  const uint32_t n = issued < (uint32_t)N ? issued : (uint32_t)N;
+#pragma unroll 1
+  for (uint32_t k = 1; k <= n; k++) drain_phase(&full[(issued - k) % N], ((issued - k) / N) & 1);
+}
+
+// mbar_wait and report_fail out of line, for the decode kernel, whose per-layer code does not fit the instruction cache: what a healthy step
 // never executes stays out of the way.
 inline __device__ __noinline__ void report_fail_far(const WaitCtl c, int where, int layer, int expected, int seen) {
   report_fail(c, where, layer, expected, seen);

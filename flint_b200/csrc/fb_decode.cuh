@@ -715,7 +715,6 @@ __global__ void __launch_bounds__(kThreads, 1) decode_mega2(const __grid_constan
       }
       pipe.max_fly = P.lm_fly;
       if (ok) produce_rows(pipe, P.w_lm + (size_t)l0 * recD, l1 - l0, CG::TILE_ROWS, CG::RT, recD, wc, L);
-      producer_drain(pipe, wc);
     }
   } else {
     const int cw = warp, tid_c = tid;
@@ -987,6 +986,7 @@ __global__ void __launch_bounds__(kThreads, 1) decode_mega2(const __grid_constan
       for (int r = tid_c; r < o1 - o0; r += kConsumerThreads) P.d_h[o0 + r] = f2bf(hown[r]);
   }
   __syncthreads();
+  if (*sm.s_abort && tid == kConsumerThreads) drain_ring<kStages>(pipe.full, pipe.it);
 }
 
 }  // namespace fb

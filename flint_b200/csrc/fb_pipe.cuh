@@ -108,24 +108,6 @@ __device__ __forceinline__ bool produce_rows(Pipe& p, const uint8_t* src, int nr
   return true;
 }
 
-// Before the CTA may exit, every bulk copy it issued must have landed. In a clean run the consumers have already
-// waited for all of them; after a failed wait the last (up to) kStages issued loads may still be in flight.
-__device__ __forceinline__ void producer_drain(Pipe& p, const WaitCtl& wc) {
-  if (*wc.s_abort == 0) return;
-  const uint32_t n = p.it < (uint32_t)kStages ? p.it : (uint32_t)kStages;
-#pragma unroll 1
-  for (uint32_t k = 0; k < n; k++) {
-    const uint32_t it = p.it - 1 - k;
-    const int s = it % kStages;
-    const uint32_t ph = (it / kStages) & 1;
-#pragma unroll 1
-    for (unsigned i = 0; i < wc.limit; i++) {
-      if (mbar_try(&p.full[s], ph)) break;
-      if ((i & 1023) == 1023) __nanosleep(64);
-    }
-  }
-}
-
 // ------------------------------------------------------------------------------------------------ consumer side
 struct QueueState {
   float* qpart;
@@ -260,7 +242,6 @@ __global__ void __launch_bounds__(kThreads, 1) gemv_stream(const GemvParams P) {
   if (warp == kConsumerWarps) {
     if (lane == 0) {
       produce_rows(pipe, P.w + (size_t)r0 * rec, r1 - r0, C::TILE_ROWS, C::RT, rec, wc, 0);
-      producer_drain(pipe, wc);
     }
   } else {
     stage_x_global<C::K>(P.x, sm, tid);
@@ -272,6 +253,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemv_stream(const GemvParams P) {
     });
   }
   __syncthreads();
+  if (*sm.s_abort && tid == kConsumerThreads) drain_ring<kStages>(pipe.full, pipe.it);
 }
 
 // ------------------------------------------------------------------------------------------------ layout kernels

@@ -481,6 +481,18 @@ __device__ __forceinline__ void vtc_epilogue(const VtcParams& P, int srow, int t
   }
 }
 
+// after a failure: the copies and MMAs in flight (see drain_phase); out of line, a healthy launch never comes here
+template <int NRAW, int NS, int NB, int ND>
+inline __device__ __noinline__ void tc_drain(uint64_t* bars, volatile int* s_issued) {
+  uint64_t *raw_full = bars, *b_full = bars + 2 * NRAW + NS, *done = b_full + NB, *acc_full = done + ND;
+  const uint32_t n = s_issued[1];
+  drain_ring<NRAW>(raw_full, s_issued[0]);
+  drain_ring<NB>(b_full, s_issued[2]);
+  if (n) drain_phase(&done[(n - 1) % ND], ((n - 1) / ND) & 1);
+  drain_ring<2>(acc_full, s_issued[3]);
+  __syncwarp();
+}
+
 template <int EPI, bool HZ>
 __global__ void __launch_bounds__(kTcThreads, 1) v_gemm_tc(const __grid_constant__ VtcParams P) {
   using S = VtcSmem<HZ>;
@@ -493,6 +505,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) v_gemm_tc(const __grid_constant
            *acc_full = done + ND, *acc_empty = acc_full + 2;
   uint32_t* s_tmem = reinterpret_cast<uint32_t*>(acc_empty + 2);
   volatile int* s_abort = reinterpret_cast<volatile int*>(s_tmem + 1);
+  volatile int* s_issued = s_abort + 1;                          // [4] copies or MMA groups that warps 0, 1, 2 have issued, whole items of warp 1
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (tid == 0) {
     for (int i = 0; i < NRAW; i++) { mbar_init(&raw_full[i], 1); mbar_init(&raw_empty[i], 8); }
@@ -535,17 +548,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) v_gemm_tc(const __grid_constant
           bulk_g2s(tsm + S::RAW + r.i * REC, blk + (size_t)g * REC, REC, &raw_full[r.i]);
         }
       }
-      // every copy issued must have landed before the CTA may exit: the consumers wait for all of them in a clean run;
-      // after a failure, wait here (bounded)
-      if (*s_abort) {
-        for (int k = 0; k < NRAW && k < (int)gi; k++) {
-          const uint32_t j = gi - 1 - k;
-          for (unsigned i = 0; i < wc.limit; i++) {
-            if (mbar_try(&raw_full[j % NRAW], (j / NRAW) & 1)) break;
-            if ((i & 1023) == 1023) __nanosleep(64);
-          }
-        }
-      }
+      s_issued[0] = gi;
     }
   } else if (warp == 1) {
     // ---------------- MMA issue: the warp waits as one, an elected lane issues eight MMAs per group and one commit. (With the
@@ -555,9 +558,10 @@ __global__ void __launch_bounds__(kTcThreads, 1) v_gemm_tc(const __grid_constant
     Ring<NB> rb;
     Ring<ND> rd;
     Ring<2> ra;
+    uint32_t gi = 0, finished = 0;
     for (TcWalk w(P); w.valid() && ok; w.next(), ra.next()) {
       ok = __all_sync(0xffffffffu, mbar_wait(&acc_empty[ra.i], ra.lap ^ 1u, wc, W_EMPTY, 3));
-      for (int g = 0; g < w.G && ok; g++, rs.next(), rb.next(), rd.next()) {
+      for (int g = 0; g < w.G && ok; g++, gi++, rs.next(), rb.next(), rd.next()) {
         // both are usually there already: test them side by side, a barrier test is a round trip of its own
         bool now = mbar_try(&a_full[rs.i], rs.lap);
         now = mbar_try(&b_full[rb.i], rb.lap) && now;
@@ -579,7 +583,9 @@ __global__ void __launch_bounds__(kTcThreads, 1) v_gemm_tc(const __grid_constant
         }
         __syncwarp();
       }
+      if (ok) finished++;
     }
+    if (lane == 0) { s_issued[1] = gi; s_issued[3] = finished; }
   } else if (warp == 2) {
     // ---------------- activations (the previous kernel's output): two tensor copies per group. Token rows past M are whatever
     // the buffer holds: they only feed accumulator columns that nobody reads.
@@ -598,15 +604,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) v_gemm_tc(const __grid_constant
           tma_load_2d(dst + NT * 128, &P.xmap, g * 128 + 64, w.tt * P.ntok, &b_full[r.i]);
         }
       }
-      if (*s_abort) {
-        for (int k = 0; k < NB && k < (int)gi; k++) {
-          const uint32_t j = gi - 1 - k;
-          for (unsigned i = 0; i < wc.limit; i++) {
-            if (mbar_try(&b_full[j % NB], (j / NB) & 1)) break;
-            if ((i & 1023) == 1023) __nanosleep(64);
-          }
-        }
-      }
+      s_issued[2] = gi;
     }
   } else if (warp >= 4 && warp < 12) {
     // ---------------- dequantise: thread = (row of the block = TMEM lane, half of the group's columns); 8 words -> 32 packed fp16
@@ -695,7 +693,10 @@ __global__ void __launch_bounds__(kTcThreads, 1) v_gemm_tc(const __grid_constant
   }
   tc_fence_before();
   __syncthreads();
-  if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TCOLS));
+  if (warp == 1) {
+    if (*s_abort) tc_drain<NRAW, NS, NB, ND>(bars, s_issued);
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TCOLS));
+  }
 }
 
 }  // namespace fb

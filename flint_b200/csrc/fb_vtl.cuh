@@ -32,6 +32,17 @@ struct VtlSmem {
   static_assert(T_AZ + (HZ ? NS * 8 : 0) <= TCOLS, "tensor memory columns");
 };
 
+// after a failure: the copies and MMAs in flight (see drain_phase); out of line, a healthy launch never comes here
+template <int NRAW, int NS, int NB, int ND>
+inline __device__ __noinline__ void tl_drain(uint64_t* bars, volatile int* s_issued) {
+  uint64_t *raw_full = bars, *b_full = bars + 2 * NRAW + NS, *done = b_full + NB, *acc_full = done + ND;
+  const int n = s_issued[1];
+  drain_ring<NRAW>(raw_full, s_issued[0]);
+  drain_ring<NB>(b_full, s_issued[2]);
+  if (n) drain_phase(n > 0 ? &done[(n - 1) % ND] : acc_full, n > 0 ? ((n - 1) / ND) & 1 : 0);
+  __syncwarp();
+}
+
 template <int NT, int EPI, bool HZ>
 __global__ void __launch_bounds__(kTlThreads, 2) v_gemm_tl(const __grid_constant__ VtcParams P) {
   using S = VtlSmem<NT, HZ>;
@@ -43,6 +54,7 @@ __global__ void __launch_bounds__(kTlThreads, 2) v_gemm_tl(const __grid_constant
            *acc_full = done + ND;
   uint32_t* s_tmem = reinterpret_cast<uint32_t*>(acc_full + 1);
   volatile int* s_abort = reinterpret_cast<volatile int*>(s_tmem + 1);
+  volatile int* s_issued = s_abort + 1;                          // [3] copies or MMA groups (-1: all) that warps 0, 1, 2 have issued
   float* ys = reinterpret_cast<float*>(tsm + S::YS);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (tid == 0) {
@@ -51,7 +63,7 @@ __global__ void __launch_bounds__(kTlThreads, 2) v_gemm_tl(const __grid_constant
     for (int i = 0; i < NB; i++) mbar_init(&b_full[i], 1);
     for (int i = 0; i < ND; i++) mbar_init(&done[i], 1);
     mbar_init(acc_full, 1);
-    *s_abort = 0;
+    *s_abort = s_issued[2] = 0;
     mbar_fence_init();
   }
   if (warp == 1) {
@@ -82,15 +94,7 @@ __global__ void __launch_bounds__(kTlThreads, 2) v_gemm_tl(const __grid_constant
         mbar_expect_tx(&raw_full[r.i], REC);
         bulk_g2s(tsm + S::RAW + r.i * REC, blk + (size_t)(g0 + gi) * REC, REC, &raw_full[r.i]);
       }
-      if (*s_abort) {                                            // after a failure: every copy issued must land before the CTA may exit
-        for (int k = 0; k < NRAW && k < gi; k++) {
-          const int j = gi - 1 - k;
-          for (unsigned i = 0; i < wc.limit; i++) {
-            if (mbar_try(&raw_full[j % NRAW], (j / NRAW) & 1)) break;
-            if ((i & 1023) == 1023) __nanosleep(64);
-          }
-        }
-      }
+      s_issued[0] = gi;
     }
   } else if (warp == 1) {
     // ---------------- MMA issue
@@ -98,7 +102,8 @@ __global__ void __launch_bounds__(kTlThreads, 2) v_gemm_tl(const __grid_constant
     Ring<NS> rs;
     Ring<NB> rb_;
     Ring<ND> rd;
-    for (int gi = 0; gi < ng; gi++, rs.next(), rb_.next(), rd.next()) {
+    int gi = 0;
+    for (; gi < ng; gi++, rs.next(), rb_.next(), rd.next()) {
       bool now = mbar_try(&a_full[rs.i], rs.lap);
       now = mbar_try(&b_full[rb_.i], rb_.lap) && now;
       if (!now) ok = mbar_wait(&a_full[rs.i], rs.lap, wc, W_FULL, 4) && mbar_wait(&b_full[rb_.i], rb_.lap, wc, W_FULL, 4);
@@ -114,11 +119,11 @@ __global__ void __launch_bounds__(kTlThreads, 2) v_gemm_tl(const __grid_constant
           tc_mma_ts(tmem, ta + k * 8, db, idesc, (gi || k) ? 1u : 0u);
           if (HZ) tc_mma_ts(tmem, tz, db, idesc, 1u);
         }
-        tc_commit(&done[rd.i]);
-        if (gi == ng - 1) tc_commit(acc_full);
+        tc_commit(gi == ng - 1 ? acc_full : &done[rd.i]);         // nobody waits for the last group's stages
       }
       __syncwarp();
     }
+    if (lane == 0) s_issued[1] = gi < ng ? gi : -1;
   } else if (warp < 5) {
     // ---------------- activations (the previous kernel's output). Token rows past M only feed accumulator columns that nobody reads.
     if (EPI == EPI_RESID && P.xbf) {
@@ -166,15 +171,7 @@ __global__ void __launch_bounds__(kTlThreads, 2) v_gemm_tl(const __grid_constant
           tma_load_2d(dst, &P.xmap, (g0 + gi) * 128, 0, &b_full[r.i]);
           tma_load_2d(dst + NT * 128, &P.xmap, (g0 + gi) * 128 + 64, 0, &b_full[r.i]);
         }
-        if (*s_abort) {
-          for (int k = 0; k < NB && k < gi; k++) {
-            const int j = gi - 1 - k;
-            for (unsigned i = 0; i < wc.limit; i++) {
-              if (mbar_try(&b_full[j % NB], (j / NB) & 1)) break;
-              if ((i & 1023) == 1023) __nanosleep(64);
-            }
-          }
-        }
+        s_issued[2] = gi;
       }
     }
   } else {
@@ -305,7 +302,10 @@ __global__ void __launch_bounds__(kTlThreads, 2) v_gemm_tl(const __grid_constant
   }
   tc_fence_before();
   __syncthreads();
-  if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(S::TCOLS));
+  if (warp == 1) {
+    if (*s_abort) tl_drain<NRAW, NS, NB, ND>(bars, s_issued);
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(S::TCOLS));
+  }
 }
 
 }  // namespace fb

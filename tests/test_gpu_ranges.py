@@ -114,6 +114,29 @@ def test_verify_token_tile_edges(M, asym):
     eng.close()
 
 
+@pytest.mark.parametrize("asym", [False, True])
+@pytest.mark.parametrize("M", [1, 3, 40, 70, 300])
+def test_passes_that_give_up_leave_nothing_behind(M, asym):
+    """With a wait limit of 0 a pass (one token: a decode step; up to 64 a tree pass; more a prompt pass) gives up at the first wait that is not
+    satisfied already. Every launch ends, after its copies and MMAs in flight (their wait has its own limit), the status says time-out or,
+    if every wait happened to be satisfied, nothing, and the next clean pass gives the bits of the first."""
+    cfg = ModelArgs.from_name("tiny")
+    eng = DecodeEngine(cfg, {k: v.cuda() for k, v in packing.synth_packed(cfg, 0, asym=asym).items()}, max_seq=512)
+    toks = torch.randint(0, cfg.vocab_size, (M,), generator=torch.Generator().manual_seed(M), dtype=torch.int32).cuda()
+    run = (lambda: eng.decode(17, 0).clone()) if M == 1 else (lambda: (eng.verify if M <= 64 else eng.prefill)(toks, 0)[0])
+    ref = run()
+    eng.check()
+    for _ in range(8):
+        eng.set_option(0, 0)
+        run()
+        assert eng.status()["code"] in (_lib.FB_OK, _lib.FB_ERR_TIMEOUT)
+        eng.set_option(0, 4000000)
+        again = run()
+        eng.check()
+        assert torch.equal(ref, again)
+    eng.close()
+
+
 def test_positions_near_the_end_of_the_integers_are_out_of_range():
     """pos + M past 2^31 - 1: refused like every position behind the cache, for trees, prompts and single steps."""
     cfg = ModelArgs.from_name("tiny")
