@@ -42,13 +42,24 @@ def extra_shape_flags(spec: str):
     return flags
 
 
+def extra_shape_header(flags) -> str:
+    """The macros of extra_shape_flags as text to include: nvcc cuts the value of a -D option at its commas."""
+    return "".join("#define %s %s\n" % tuple(f[2:].split("=", 1)) for f in flags)
+
+
 def build(force: bool = False, verbose: bool = False) -> str:
     if not force and not _stale():
         return LIB
     nvcc = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
-    extra = os.environ.get("FLINT_B200_NVCC_FLAGS", "").split() + extra_shape_flags(os.environ.get("FLINT_B200_EXTRA_SHAPES", ""))
+    extra = os.environ.get("FLINT_B200_NVCC_FLAGS", "").split()
     objdir = os.path.join(HERE, "build")
     os.makedirs(objdir, exist_ok=True)
+    shapes = extra_shape_flags(os.environ.get("FLINT_B200_EXTRA_SHAPES", ""))
+    if shapes:
+        header = os.path.join(objdir, "extra_shapes.h")
+        with open(header, "w") as f:
+            f.write(extra_shape_header(shapes))
+        extra += ["-include", header]
     # one object per translation unit, compiled side by side, then one link
     procs, objs = [], []
     for src in SOURCES:

@@ -82,3 +82,32 @@ def test_build_time_extra_shapes_become_kernel_table_macros():
         extra_shape_flags("4096,4096,11000,128,1")
     with pytest.raises(ValueError):
         extra_shape_flags("4096,4096,11008,128")
+
+
+def test_build_time_extra_shapes_reach_the_compiler(monkeypatch):
+    """nvcc cuts the value of a -D option at its commas: the shape macros travel in an included header, which the preprocessor
+    expands to the table entries."""
+    import subprocess
+    from flint_b200.csrc import build as B
+    cmds = []
+
+    class Fake:
+        returncode = 1
+
+        def __init__(self, cmd):
+            cmds.append(cmd)
+
+        def wait(self):
+            return 1
+
+    monkeypatch.setenv("FLINT_B200_EXTRA_SHAPES", "3072,3072,8192,128,3")
+    with monkeypatch.context() as m:
+        m.setattr(B.subprocess, "Popen", Fake)
+        import pytest
+        with pytest.raises(subprocess.CalledProcessError):
+            B.build(force=True)
+    assert cmds and not any(a.startswith("-D") and "," in a for c in cmds for a in c)
+    header = cmds[0][cmds[0].index("-include") + 1]
+    out = subprocess.run(["g++", "-E", "-P", "-x", "c++", "-include", header, "-"], input="FB_EXTRA_DECODE_ENTRIES FB_EXTRA_K(Y)", text=True,
+                         stdout=subprocess.PIPE, check=True).stdout
+    assert out.split() == ["FB_DECODE_ENTRY(3072,3072,8192,128,3),", "Y(3072)"]
