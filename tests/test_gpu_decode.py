@@ -232,19 +232,16 @@ def test_granite3b_shape_two_layers_vs_oracle():
     assert agree == len(toks)
 
 
-@pytest.mark.parametrize("variant", [0, 2])
-def test_long_context_prefilled_cache_vs_oracle(variant):
+def test_long_context_prefilled_cache_vs_oracle():
     """The long-context configuration: K and V caches pre-filled for 32 768 positions with seeded N(0, 1) values (the
     same bf16 bits in the oracle and on the GPU), then decode steps whose attention is split over every CTA and merged.
-    Two layers of the 3B-class shape keep the oracle's run time at a few seconds. Both attention variants: the default
-    at this length (K/V through the weight ring, tensor pipe) and the scalar one (option 8 = 2)."""
+    Two layers of the 3B-class shape keep the oracle's run time at a few seconds."""
     cfg = _granite_shape(2)
     T0, steps = 32768, 3
     W = packing.synth_packed(cfg, 0, device="cuda")
     P = {k: v.cpu() for k, v in W.items()}
     orc = O.OracleModel(cfg, P, T0 + 16)
     eng = DecodeEngine(cfg, W, max_seq=T0 + 16)
-    eng.set_option(8, variant)
     g = torch.Generator().manual_seed(7)
     kv = torch.randn(2, cfg.n_layer, T0, cfg.n_local_heads, cfg.head_dim, generator=g).bfloat16()
     eng.kc[:, :T0].copy_(kv[0])
@@ -265,15 +262,13 @@ def test_long_context_prefilled_cache_vs_oracle(variant):
 
 
 @pytest.mark.parametrize("T0", [3, 57, 64, 300, 5000])
-def test_tiny_long_cache_variant_vs_oracle(T0):
-    """The decode variant whose attention streams K/V through the weight ring as tensor copies and multiplies on the tensor
-    pipe (the default on one GPU), forced at every cached length: a chunk shorter than one stage, exactly one
-    stage, the step's own row inside a stage, many stages per CTA."""
+def test_tiny_decode_attention_at_every_kind_of_cached_length(T0):
+    """The attention streams K/V through the weight ring as tensor copies and multiplies on the tensor pipe: a chunk shorter than one
+    stage, exactly one stage, the step's own row inside a stage, many stages per CTA."""
     cfg = ModelArgs.from_name("tiny")
     P = packing.synth_packed(cfg, 0)
     orc = O.OracleModel(cfg, P, T0 + 8)
     eng = DecodeEngine(cfg, {k: v.cuda() for k, v in P.items()}, max_seq=T0 + 8)
-    eng.set_option(8, 1)
     g = torch.Generator().manual_seed(11)
     kv = torch.randn(2, cfg.n_layer, T0, cfg.n_local_heads, cfg.head_dim, generator=g).bfloat16()
     eng.kc[:, :T0].copy_(kv[0])
@@ -318,18 +313,16 @@ def test_granite3b_class_full_depth_vs_oracle():
     assert agree == len(toks)
 
 
-@pytest.mark.parametrize("variant", [0, 1])
-def test_llama8b_class_shape_two_layers_vs_oracle(variant):
+def test_llama8b_class_shape_two_layers_vs_oracle():
     """The 8B-class shape on ONE GPU (d 4096, 32/8 heads of 128, FFN 14336 = tiles of 2 rows, vocab 128256, untied LM
     head, RoPE base 500000) at a depth of 2 layers against the oracle: the kernel instantiation the tensor-parallel
-    configuration is built from. variant 1 forces the long-cache attention (heads of 128: 32 positions per ring stage)."""
+    configuration is built from (heads of 128: 32 positions per ring stage)."""
     cfg = ModelArgs.from_name("llama-8b-class")
     cfg.n_layer = 2
     W = packing.synth_packed(cfg, 0, device="cuda")
     P = {k: v.cpu() for k, v in W.items()}
     orc = O.OracleModel(cfg, P, 64)
     eng = DecodeEngine(cfg, W, max_seq=64)
-    eng.set_option(8, variant)
     worst, agree = 0.0, 0
     toks = [17, 120000, 123, 4567, 9, 31000]
     for pos, t in enumerate(toks):
@@ -345,8 +338,7 @@ def test_llama8b_class_shape_two_layers_vs_oracle(variant):
 
 def test_llama1b_class_shape_two_layers_decode_and_verify_vs_oracle():
     """A fourth model width (d 2048, 32/8 heads of 64, FFN 8192) at a depth of 2 layers: decode against the oracle, then a
-    16-node tree verify (this width has no bf16 warp-level GEMM instantiation: the library routes it to the kernels that
-    take the width at run time)."""
+    6-node and a 16-node tree verify (the M-token kernels take the width at run time)."""
     from flint_b200.tree import static_tree
     cfg = ModelArgs.from_name("llama-1b-class")
     cfg.n_layer = 2

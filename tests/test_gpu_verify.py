@@ -34,17 +34,13 @@ def _prefix(orc, eng, toks):
         eng.decode(t, p, want_logits=False)
 
 
-@pytest.mark.parametrize("path", [1, 2, 3, 4])
 @pytest.mark.parametrize("asym", [False, True])
 @pytest.mark.parametrize("M", [1, 5, 16, 26, 40])
-def test_tiny_chain_verify_vs_oracle(M, asym, path):
-    """Every GEMM implementation of the verify path (1 = warp-level mma.sync on bf16, 2 = tcgen05 with accumulators in
-    tensor memory, 3 = tcgen05 chains, 4 = warp-level mma.sync on fp16 subnormals for up to 26 tokens) at every padded
-    token count, symmetric and asymmetric weights. A path that does not cover a case runs the library's fallback."""
+def test_tiny_chain_verify_vs_oracle(M, asym):
+    """The tree GEMMs at every padded token count (tiles of 16, 32 and 64), symmetric and asymmetric weights."""
     cfg = ModelArgs.from_name("tiny")
     P = packing.synth_packed(cfg, 0, asym=asym)
     orc, eng = O.OracleModel(cfg, P, 128), DecodeEngine(cfg, _cuda(P), max_seq=128)
-    eng.set_option(7, path)
     _prefix(orc, eng, [3, 1, 4, 1, 5, 9, 2])
     toks = torch.randint(0, cfg.vocab_size, (M,), generator=torch.Generator().manual_seed(M)).tolist()
     ref_lg, ref_ft = orc.verify(toks, 7)
@@ -122,6 +118,24 @@ def test_reference_shaped_verify_launch_and_kv_move():
     assert torch.equal(kc[:, 1], before[:, 2]) and torch.equal(kc[:, 2], before[:, 3]) and torch.equal(kc[:, 3], before[:, 3])
 
 
+def test_options_without_effect_are_accepted_and_change_nothing():
+    """Options 7 and 8 once selected implementations that are gone: their old values are accepted, others refused, and no value changes a
+    bit of a decode step or a tree pass."""
+    cfg = ModelArgs.from_name("tiny")
+    eng = DecodeEngine(cfg, _cuda(packing.synth_packed(cfg, 0)), max_seq=64)
+    toks = [5, 17, 99, 1024, 7]
+    ref = eng.verify(toks, 0)[0].clone(), eng.decode(3, 5).clone()
+    for what, most in ((7, 4), (8, 2)):
+        for v in range(most + 1):
+            eng.set_option(what, v)
+            assert torch.equal(ref[0], eng.verify(toks, 0)[0]) and torch.equal(ref[1], eng.decode(3, 5))
+        for v in (-1, most + 1):
+            with pytest.raises(_lib.FlintError) as ei:
+                eng.set_option(what, v)
+            assert ei.value.code == _lib.FB_ERR_ARG
+    eng.check()
+
+
 def test_verify_bad_m_is_an_error():
     cfg = ModelArgs.from_name("tiny")
     eng = DecodeEngine(cfg, _cuda(packing.synth_packed(cfg, 0)), max_seq=128)
@@ -174,9 +188,8 @@ def _verify_rows_ok(lg, ref_lg, bound=0.02):
     assert _argmax_ok(lg, ref_lg)
 
 
-@pytest.mark.parametrize("path", [1, 2, 3, 4])
 @pytest.mark.parametrize("M", [16, 26, 64])
-def test_granite3b_shape_verify_over_1024_token_cache(M, path):
+def test_granite3b_shape_verify_over_1024_token_cache(M):
     """The benchmark's verify configuration: static trees of 16 / 26 / 64 nodes over a cache of 1024 positions (seeded
     N(0, 1) keys and values), so the attention runs over many spans of positions and the span merge is checked."""
     from flint_b200.tree import static_tree
@@ -186,7 +199,6 @@ def test_granite3b_shape_verify_over_1024_token_cache(M, path):
     P = {k: v.cpu() for k, v in W.items()}
     T0 = 1024
     orc, eng = O.OracleModel(cfg, P, T0 + 64), DecodeEngine(cfg, W, max_seq=T0 + 64)
-    eng.set_option(7, path)
     _prefill_random(orc, eng, cfg, T0)
     parent, depth = static_tree(M)
     amask = O.tree_mask(parent)
