@@ -82,9 +82,13 @@ int chunks_for(const fb_ctx* c, int T) {
 
 // Bulk copies a CTA keeps in flight while the layers run. A layer that brings each SM at most two rings of weights and K/V spends far
 // longer on its hand-overs than one copy at a time (about 2.2 TB/s over all SMs) takes, and the flags and tagged words then wait
-// behind less bulk traffic; more bytes need the full rate. Microseconds a token at 4 / 2 / 1 copies: 1B-class (1.2 rings a layer) 394 / 392 /
-// 388, 3B-class (1.5) 1002 / 992 / 983, the same behind 2000 positions (1.7) 1037 / 1031 / 1023, 8B-class (4.5) 1621 / 1667 / 1759. The LM
-// head has no hand-over to disturb: always 4.
+// behind less bulk traffic; more bytes need the full rate. Microseconds a token at 4 / 2 / 1 copies, by rings a layer:
+//   3B-class   1.5: 1002 / 994 / 985    1.7: 1057 / 1056 / 1040   1.8: 1094 / 1090 / 1084   2.0 (5000 cached): 1149 / 1155 / 1141
+//              2.25: 1206 / 1204 / 1185   2.6: 1287 / 1294 / 1282   3.4: 1452 / 1460 / 1480   4.3: 1623 / 1658 / 1742
+//   40 heads   1.5: 1021 / 1011 / 1003   1.6: 1075 / 1075 / 1067   1.75: 1126 / 1131 / 1132   1.9: 1143 / 1152 / 1151   2.1: 1184 / 1195 / 1188
+//   1B-class   1.2: 394 / 391 / 387   1.4: 422 / 421 / 421   1.75: 441 / 437 / 436         8B-class   4.5: 1621 / 1667 / 1759
+// Up to 1.7 rings one copy gains on every shape, from 3.4 on it loses; in between the shapes differ by up to 1.8 % either way, and two copies
+// are never the best. The LM head has no hand-over to disturb: always 4.
 int fly_for(const fb_ctx* c, int T) {
   if (c->max_fly) return c->max_fly;
   const fb_model_desc& d = c->d;

@@ -10,9 +10,6 @@
 namespace fb {
 
 // ------------------------------------------------------------------------------------------------ constants
-#ifndef FB_ACC2
-#define FB_ACC2 0     // 1: two accumulator sets in the unrolled tile product; measured no faster
-#endif
 #ifndef FB_CW
 #define FB_CW 14      // 14 consumers + 1 producer = 15 warps -> at most 4 per scheduler -> 128 registers per thread
 #endif
@@ -337,20 +334,11 @@ cudaError_t launch_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t sme
   return launch_pdl_cluster(kern, grid, block, smem, st, 1u, args...);
 }
 
-// bf16 tensor-core helpers shared by the verify attention and the long-cache decode attention
+// bf16 tensor-core helpers shared by the attention kernels and the draft head
 __device__ __forceinline__ void mma_bf16(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
   asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
                : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
                : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-__device__ __forceinline__ void mma_bf16_first(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
-               : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3])
-               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.f));
-}
-__device__ __forceinline__ void ldmatrix_x4_trans(uint32_t (&r)[4], const void* smem_row) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(smem_u32(smem_row)));
 }
 __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) { return (uint32_t)f2bf(lo) | ((uint32_t)f2bf(hi) << 16); }
 
@@ -374,18 +362,14 @@ __device__ __forceinline__ void tile_dot_unrolled(const uint8_t* tile, int slice
   const uint32_t ml = tb + C::NIB + (uint32_t)(jl * C::RG * RT + rl) * 2;
   const uint32_t mh = tb + C::NIB + (uint32_t)(jh * C::RG * RT + rh) * 2;
   const uint32_t fl = smem_u32(x.xf) + (uint32_t)(jl * C::RG) * 16, fh = smem_u32(x.xf) + (uint32_t)(jh * C::RG) * 16;
-  float ct[4] = {0.f, 0.f, 0.f, 0.f}, cg[4], ch[4];
+  float ct[4] = {0.f, 0.f, 0.f, 0.f}, cg[4];
   float zl = 0.f, zh = 0.f;
   uint4 w4 = lds128(wa);
   uint2 xb[4];
 #pragma unroll
   for (int i = 0; i < 4; i++) xb[i] = lds64(xa[i]);
   const bool odd0 = (NB % 2 == 0) ? false : (b0 & 1);           // the slice starts in the middle of a round
-#ifdef FB_DOT_UNROLL2
-#pragma unroll 2
-#else
 #pragma unroll
-#endif
   for (int bi = 0; bi < NB; bi++) {
     uint4 wn;
     uint2 xn[4];
@@ -400,13 +384,8 @@ __device__ __forceinline__ void tile_dot_unrolled(const uint8_t* tile, int slice
     for (int i = 0; i < 4; i++) {
       const uint32_t w2 = ws[i] >> 8;
       const uint32_t a[4] = {ws[i] & 0x000F000Fu, ws[i] & 0x00F000F0u, w2 & 0x000F000Fu, w2 & 0x00F000F0u};
-      if (FB_ACC2 && (i & 1)) {
-        if (first && i == 1) mma_f16_first(ch, a, xb[i].x, xb[i].y);
-        else mma_f16(ch, a, xb[i].x, xb[i].y);
-      } else {
-        if (first && i == 0) mma_f16_first(cg, a, xb[i].x, xb[i].y);
-        else mma_f16(cg, a, xb[i].x, xb[i].y);
-      }
+      if (first && i == 0) mma_f16_first(cg, a, xb[i].x, xb[i].y);
+      else mma_f16(cg, a, xb[i].x, xb[i].y);
     }
     const bool closes = (((bi & 1) != 0) != odd0);               // block b0 + bi closes a round
     if (closes || bi == NB - 1) {
@@ -414,7 +393,6 @@ __device__ __forceinline__ void tile_dot_unrolled(const uint8_t* tile, int slice
       const float4 Fl = lds128f(fl + ro * 16), Fh = lds128f(fh + ro * 16);
       const float sl = lds_bf16(ml + ro * RT * 2), sh = lds_bf16(mh + ro * RT * 2);
       const float sl2 = sl * Fl.x, sh2 = sh * Fh.y;
-      if (FB_ACC2) { cg[0] += ch[0]; cg[1] += ch[1]; cg[2] += ch[2]; cg[3] += ch[3]; }
       ct[0] = fmaf(sl2, cg[0], ct[0]); ct[1] = fmaf(sl2, cg[1], ct[1]);
       ct[2] = fmaf(sh2, cg[2], ct[2]); ct[3] = fmaf(sh2, cg[3], ct[3]);
       if (closes) {                                              // once per (row, group): offset and zero point

@@ -128,54 +128,27 @@ __device__ __forceinline__ void st_relaxed_u32(uint32_t* p, uint32_t v) {
   (void)old;
 }
 // all consumer threads call; warp 0 polls flags[0..n) until each equals tag
-#ifndef FB_FLAG_SETS
-#define FB_FLAG_SETS 1       // poll rounds kept in flight (staggered): a posted flag is seen after ~RTT/2 + RTT/(2 sets)
-#endif
-#ifndef FB_FLAG_SLACK_DIV
-#define FB_FLAG_SLACK_DIV 2  // the gather starts when all but n / 2 producers have posted (0: wait for every flag). The tagged
-#endif                       // words of the stragglers are simply polled again by the gather, so the last flags' round trip
-                             // leaves the critical path. Microseconds a token at a third / a half / three quarters: 3B-class
-                             // 1060 / 1020 / 1010, 1B 395 / 390 / 386, 40 / 8 heads of 64 1017 / 1020 / 1042; no flag wait at all
-                             // is slower (every consumer polling words floods L2).
+// The gather starts when all but n / 2 producers have posted. The tagged words of the stragglers are simply polled again by the gather, so
+// the last flags' round trip leaves the critical path. Microseconds a token at a third / a half / three quarters: 3B-class 1060 / 1020 /
+// 1010, 1B 395 / 390 / 386, 40 / 8 heads of 64 1017 / 1020 / 1042; no flag wait at all is slower (every consumer polling words
+// floods L2).
 __device__ __forceinline__ void wait_flags(const uint32_t* flags, int n, uint32_t tag, int cw, int lane, const WaitCtl& wc,
                                            int layer) {
   if (cw == 0) {
-    constexpr int NS = FB_FLAG_SETS;
-    uint32_t v[NS][8];
+    uint32_t v[8];
     // all loads of a round are issued before any is compared (n <= 256: at most 8 per lane)
-    auto issue = [&](uint32_t (&d)[8]) {
+    auto issue = [&]() {
 #pragma unroll
-      for (int j = 0; j < 8; j++) d[j] = (lane + 32 * j < n) ? ld_relaxed_u32(flags + lane + 32 * j) : tag;
+      for (int j = 0; j < 8; j++) v[j] = (lane + 32 * j < n) ? ld_relaxed_u32(flags + lane + 32 * j) : tag;
     };
-    auto all_set = [&](const uint32_t (&d)[8]) {
-      if constexpr (FB_FLAG_SLACK_DIV == 0) {
-        bool ok = true;
-#pragma unroll
-        for (int j = 0; j < 8; j++) ok = ok && (d[j] == tag);
-        return __all_sync(0xffffffffu, ok) != 0;
-      } else {
-        unsigned miss = 0;
-#pragma unroll
-        for (int j = 0; j < 8; j++) miss += (d[j] != tag);
-        return __reduce_add_sync(0xffffffffu, miss) <= (unsigned)(n / FB_FLAG_SLACK_DIV);
-      }
-    };
-#pragma unroll
-    for (int s = 0; s < NS; s++) {
-      if (s) __nanosleep(700 / NS);
-      issue(v[s]);
-    }
-    bool done = false;
+    issue();
 #pragma unroll 1
-    for (unsigned spin = 0; !done; spin++) {
+    for (unsigned spin = 0;; spin++) {
+      unsigned miss = 0;
 #pragma unroll
-      for (int s = 0; s < NS; s++) {
-        if (!done) {
-          if (all_set(v[s])) done = true;
-          else issue(v[s]);
-        }
-      }
-      if (done) break;
+      for (int j = 0; j < 8; j++) miss += (v[j] != tag);
+      if (__reduce_add_sync(0xffffffffu, miss) <= (unsigned)(n / 2)) break;
+      issue();
       int stop = 0;
       if (lane == 0) {
         if (*wc.s_abort) stop = 1;

@@ -204,8 +204,8 @@ __global__ void __launch_bounds__(256) v_norm_f16(const uint16_t* h, const uint1
   }
 }
 
-// Attention output of one token, bf16 -> fp16 times a power of two, in place (the path where the attention CTAs write their rows
-// themselves; v_attn_merge does it on the way otherwise). One CTA of 256 threads per token.
+// Attention output of one token, bf16 -> fp16 times a power of two, in place: prompts, whose GEMM brings its activations by tensor copies (the
+// tree GEMM converts them on the way in). One CTA of 256 threads per token.
 __global__ void __launch_bounds__(256) v_row_f16(uint16_t* x, float* fx, int D) {
   const int m = blockIdx.x, tid = threadIdx.x, nvec = D / 8;
   __shared__ float red[8];
@@ -250,7 +250,7 @@ struct alignas(64) VtcParams {
   CUtensorMap xmap;          // activations fp16 [rows >= M][K] as a 2-D tensor, box 64 columns x NT tokens, 128-byte swizzle
   const uint8_t* w;          // TC layout of this matrix
   int rows, K, M;
-  int nsplit;                // CTAs of a cluster that share one item's K (1, 2 or 4)
+  int nsplit;                // trees: CTAs of a cluster that share one item's K (1, 2, 4 or 8)
   int ntok, ntile;           // tokens of one tile (a multiple of 16, <= NT; one tile unless this is a prompt) and tiles
   DevStatus* status;
   unsigned spin_limit;
@@ -274,7 +274,8 @@ __device__ __forceinline__ uint32_t lds32(uint32_t a) {
   asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a));
   return v;
 }
-// nibble pairs in bits (0..3, 16..19) / (4..7, 20..23) -> fp16 pair (nib - 8) * s: OR-ing in the exponent of 1024 makes 1024 + nib
+// nibble pairs in bits (0..3, 16..19) / (4..7, 20..23) -> fp16 pair (nib - 8) * s, the magic-exponent conversion that is published for int4
+// weights (Kim et al., "Who Says Elephants Can't Run", 2022): OR-ing in the exponent of 1024 makes 1024 + nib
 // (1024 + 16 nib); taking 1032 off (or a sixteenth minus 72) is exact, and so is the product
 __device__ __forceinline__ uint32_t tc_h2(__half2 v) { return *reinterpret_cast<const uint32_t*>(&v); }
 __device__ __forceinline__ __half2 tc_as_h2(uint32_t v) { return *reinterpret_cast<const __half2*>(&v); }
@@ -609,7 +610,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) v_gemm_tc(const __grid_constant
   } else if (warp >= 4 && warp < 12) {
     // ---------------- dequantise: thread = (row of the block = TMEM lane, half of the group's columns); 8 words -> 32 packed fp16
     // pairs per group. (Two warps sharing a group halve the time that a stage is busy; with each warp doing whole groups in turn
-    // the six stages did not cover the round trip to the MMA and back.)
+    // the stages did not cover the round trip to the MMA and back.)
     const uint32_t tl = tmem + ((uint32_t)(quad * 32) << 16) + half * 32;
     uint32_t gi = 0;
     Ring<NRAW> rr;
@@ -658,7 +659,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) v_gemm_tc(const __grid_constant
       }
     }
   } else if (warp >= 12) {
-    // ---------------- epilogue: thread = (row of the block, half of the tokens), eight tokens at a time
+    // ---------------- epilogue: thread = (row of the block, half of the tokens), 8 or 16 tokens at a time
     const uint32_t tlane = tmem + ((uint32_t)(quad * 32) << 16) + half * HC;
     Ring<2> ra;
     pdl_wait();

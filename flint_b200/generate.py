@@ -20,7 +20,7 @@ from .model import Transformer
 
 
 def _prefill(model: Transformer, prompt: torch.Tensor, temperature: float, top_k, seed: int):
-    """Causal chunks of 64 through the verify path; returns (first new token on the device [1], features [T, dim])."""
+    """The whole prompt through the model facade (up to 1024 rows per weight pass); returns (first new token on the device [1], features [T, dim])."""
     eng = model.engine
     T = prompt.numel()
     logits, feats = model(prompt.view(1, -1), torch.arange(T), return_hidden=True)
