@@ -230,7 +230,7 @@ cudaError_t pass_bind_matrix(fb_ctx* c, int which, const void* q, const void* s,
 extern "C" {
 
 int fb_prefill(fb_ctx* c, const int32_t* d_tokens, int32_t n, int32_t pos, float* d_logits, void* d_feat, void* stream) {
-  if (!c || !d_tokens || n < 1) return FB_ERR_ARG;
+  if (!c || !d_tokens || n < 1 || ((uintptr_t)d_feat & 15)) return FB_ERR_ARG;       /* features are stored 16 bytes at a time */
   if (!c->weights_bound || !c->kc) return FB_ERR_STATE;
   if (c->tp_size > 1 || !c->embed) return FB_ERR_STATE;
   if (pos < 0 || n > c->max_seq - pos) return FB_ERR_RANGE;
@@ -249,7 +249,7 @@ int fb_prefill(fb_ctx* c, const int32_t* d_tokens, int32_t n, int32_t pos, float
 
 int fb_verify(fb_ctx* c, const int32_t* d_tokens, const void* d_h, const int32_t* d_depth, const uint8_t* d_amask,
               int32_t M, int32_t pos, float* d_logits, void* d_feat, void* stream) {
-  if (!c || !d_depth || !d_amask || (!d_tokens && !d_h)) return FB_ERR_ARG;
+  if (!c || !d_depth || !d_amask || (!d_tokens && !d_h) || ((uintptr_t)d_feat & 15)) return FB_ERR_ARG;
   if (!c->weights_bound || !c->kc) return FB_ERR_STATE;
   if (c->tp_size > 1) return FB_ERR_STATE;           /* a tensor-parallel rank holds slices only */
   if (!d_h && !c->embed) return FB_ERR_STATE;

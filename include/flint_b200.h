@@ -120,7 +120,8 @@ int fb_decode(fb_ctx* ctx, int32_t token, const int32_t* d_token, void* d_h, int
  * slots j with amask[m*M + j] != 0. M is 1..64 (any value, padded internally to 16/32/64); other M is FB_ERR_RANGE.
  *   d_tokens : device int32[M], or NULL when d_h is given
  *   d_h      : bf16 [M, dim] already multiplied embeddings (the reference's argument), or NULL
- *   d_logits : f32 [M, vocab] or NULL;   d_feat : bf16 [M, dim] post-final-norm feature (the draft head's input) or NULL */
+ *   d_logits : f32 [M, vocab] or NULL;   d_feat : bf16 [M, dim] post-final-norm feature (the draft head's input) or NULL,
+ *              16-byte aligned */
 int fb_verify(fb_ctx* ctx, const int32_t* d_tokens, const void* d_h, const int32_t* d_depth, const uint8_t* d_amask,
               int32_t M, int32_t pos, float* d_logits, void* d_feat, void* stream);
 

@@ -137,6 +137,23 @@ def test_passes_that_give_up_leave_nothing_behind(M, asym):
     eng.close()
 
 
+def test_a_misaligned_feature_buffer_is_an_argument_error():
+    """Features are stored 16 bytes at a time: a buffer that starts 2 bytes later is refused before any launch."""
+    cfg = ModelArgs.from_name("tiny")
+    eng = DecodeEngine(cfg, {k: v.cuda() for k, v in packing.synth_packed(cfg, 0).items()}, max_seq=32)
+    tok, depth = (torch.arange(4, dtype=torch.int32, device="cuda") for _ in range(2))
+    mask = torch.ones(4, 4, dtype=torch.uint8, device="cuda").tril()
+    feat = torch.full((4 * cfg.dim + 8,), 7.0, dtype=torch.bfloat16, device="cuda")
+    p = [ctypes.c_void_p(t.data_ptr()) for t in (tok, depth, mask)]
+    for at in (2, 8):
+        out = ctypes.c_void_p(feat.data_ptr() + at)
+        assert eng.lib.fb_verify(eng._ctx, p[0], None, p[1], p[2], 4, 0, None, out, None) == _lib.FB_ERR_ARG
+        assert eng.lib.fb_prefill(eng._ctx, p[0], 4, 0, None, out, None) == _lib.FB_ERR_ARG
+    torch.cuda.synchronize()
+    assert bool((feat == 7.0).all())
+    eng.close()
+
+
 def test_positions_near_the_end_of_the_integers_are_out_of_range():
     """pos + M past 2^31 - 1: refused like every position behind the cache, for trees, prompts and single steps."""
     cfg = ModelArgs.from_name("tiny")
