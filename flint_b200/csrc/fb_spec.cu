@@ -181,7 +181,7 @@ int fb_draft_forward(fb_draft* r, const void* d_feat, const void* d_emb, const i
   memset(&p, 0, sizeof(p));
   p.W[0] = (const uint16_t*)r->w.merge; p.x0 = (const uint16_t*)d_feat; p.ldx0 = F; p.k0 = F;
   if (d_emb) { p.x1 = (const uint16_t*)d_emb; p.ldx1 = D; }
-  else { p.x1 = (const uint16_t*)r->w.embed; p.ldx1 = D; p.x1_tokens = d_tokens; }
+  else { p.x1 = (const uint16_t*)r->w.embed; p.ldx1 = D; p.x1_tokens = d_tokens; p.x1_rows = d.vocab; }
   p.k1 = D; p.N[0] = D; p.T = T; p.y[0] = r->x; p.ldy[0] = D; p.first = true;
   FB_DCUDA(r, launch_linear<DL_STORE>(p, st));
   FB_DCUDA(r, launch_pdl(d_rmsnorm, dim3(T), dim3(256), 0, st, (const uint16_t*)r->x, D, (const uint16_t*)r->w.n1, r->h, D, D, d.rms_eps, false));

@@ -325,7 +325,8 @@ struct DLin {
   const uint16_t* W2;           // DL_SWIGLU: the `up` matrix, same shape as W[0]
   const uint16_t* x0;           // first input segment: bf16 rows of k0 elements, ldx0 apart
   const uint16_t* x1;           // second segment (k1 elements, ldx1 apart) or nullptr: the input is cat(x0, x1)
-  const int32_t* x1_tokens;     // when set, segment 1 of token t is row x1_tokens[t] of x1 (an embedding table); < 0: zeros
+  const int32_t* x1_tokens;     // when set, segment 1 of token t is row x1_tokens[t] of x1, an embedding table of x1_rows rows; outside: zeros
+  int x1_rows;
   int ldx0, ldx1, k0, k1;
   int N[3], T;
   uint16_t* y[3];               // bf16 [T, N] rows ldy apart (STORE / RESID / SWIGLU)
@@ -389,7 +390,7 @@ __global__ void __launch_bounds__(WARPS * 32, NT == 1 ? 3 : 1) d_gemm(const DLin
     xp0[j] = live ? P.x0 + (size_t)tok * P.ldx0 + 8 * t : nullptr;
     if (CAT) {
       const int id = live ? (P.x1_tokens ? P.x1_tokens[tok] : tok) : -1;
-      xp1[j] = id >= 0 ? P.x1 + (size_t)id * P.ldx1 + 8 * t - P.k0 : nullptr;
+      xp1[j] = id >= 0 && (!P.x1_tokens || id < P.x1_rows) ? P.x1 + (size_t)id * P.ldx1 + 8 * t - P.k0 : nullptr;
     }
   }
   auto load_x = [&](int c, uint4 (&d)[NT]) {

@@ -99,7 +99,7 @@ class DraftHead:
     def forward(self, feat: torch.Tensor, emb: Optional[torch.Tensor] = None, positions: Optional[torch.Tensor] = None,
                 input_pos: Optional[torch.Tensor] = None, tokens: Optional[torch.Tensor] = None) -> torch.Tensor:
         """feat [1, T, fdim] or [T, fdim]; the embeddings either as `emb` (same leading shape, dim wide) or as `tokens`
-        (int32 [T] on the device, a negative id = zero row) looked up on the device. input_pos = cache slots."""
+        (int32 [T] on the device, an id outside the table = zero row) looked up on the device. input_pos = cache slots."""
         if not self._h.value:
             raise RuntimeError("load_state_dict, bind_target and setup_cache first")
         lead = feat.shape[:-1]

@@ -167,7 +167,7 @@ int fb_accept_tree(const int32_t* d_cand, const int32_t* d_parent, const int32_t
  * and of its token head (reference: spec_mega.py:43-44), rounding to bf16 where bf16 PyTorch modules round.
  * fuse * dim is the width of the (fused) feature; n_kv_head == n_head is the reference's multi-head form.
  *   fb_draft_forward: T rows. d_feat bf16 [T, fuse*dim]; the token embedding of row t is d_emb[t] (bf16 [T, dim]) or,
- *                     when d_emb is NULL, row d_tokens[t] of the bound embedding table (a negative id = zeros), read on
+ *                     when d_emb is NULL, row d_tokens[t] of the bound embedding table (an id outside it = zeros), read on
  *                     the device; d_positions int32[T] rotation positions; d_slots int32[T] = cache slot of every row
  *                     (its k/v are written there and row t attends slots 0..d_slots[t]) or NULL (slot t: plain causal
  *                     attention over the T rows); d_out bf16 [T, fuse*dim] = predicted next features

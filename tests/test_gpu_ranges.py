@@ -325,6 +325,25 @@ def test_draft_row_tile_edges(T):
     assert np.all(np.take_along_axis(lg, t_dev.cpu().numpy().astype(np.int64), 1) >= top[:, 2:] - 2.0 ** -6 * np.abs(lg).max())
 
 
+@pytest.mark.parametrize("T", [1, 12, 40])
+def test_draft_token_ids_outside_the_table_are_zero_rows(T):
+    """Ids at and past the vocabulary, like negative ones, read no table row: the bits of a call whose embeddings are zeros there."""
+    dim, vocab = 256, 1000
+    m = seeded_draft(dim, 4, 512, seed=5, rope_base=10000.0)
+    g = torch.Generator().manual_seed(T)
+    embed = torch.randn(vocab, dim, generator=g).bfloat16().cuda()
+    m.bind_target(embed, torch.ones(dim, dtype=torch.bfloat16, device="cuda"))
+    m.setup_cache(48)
+    feat = torch.randn(T, dim, generator=g).bfloat16().cuda()
+    toks = torch.randint(0, vocab, (T,), generator=g, dtype=torch.int32)
+    bad = torch.arange(T) % 3 == 0
+    toks[bad] = torch.tensor([vocab, -1, 2 ** 31 - 1, vocab + 7, -2 ** 31], dtype=torch.int32).repeat(T)[:int(bad.sum())]
+    emb = embed[toks.clamp(0, vocab - 1).long().cuda()]
+    emb[bad.cuda()] = 0
+    pos = torch.arange(T, dtype=torch.int32, device="cuda")
+    assert torch.equal(m(feat, None, pos, input_pos=pos, tokens=toks.cuda()), m(feat, emb, pos, input_pos=pos))
+
+
 @pytest.mark.parametrize("slots", [12284, 20000])
 def test_draft_attention_over_a_large_cache(slots):
     """A draft head whose score vector alone fills (12 284 slots), or exceeds, the 48 KB of shared memory that a kernel has without asking:
