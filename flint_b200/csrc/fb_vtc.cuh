@@ -39,6 +39,7 @@ namespace fb {
 constexpr int kTcThreads = 640;   // warps: 0 weights, 1 MMA issue, 2 activations, 4..11 dequantise, 12..19 epilogue
 constexpr int kTcRowBlock = 128;
 constexpr int kTcTokens = 128;    // most tokens of a prompt's tile
+constexpr int kTcEpiBytes = 2 * 64 * 4 + 16 * 64;
 constexpr int kTcTrailer = kTcRowBlock * 4 + 16;      // a block's row factors, then its flag
 
 __host__ __device__ constexpr int tc_rec_bytes(int has_zeros) { return 8192 + 256 * (has_zeros ? 2 : 1); }
@@ -359,7 +360,8 @@ struct VtcSmem {
   static constexpr int ND = 16;
   static_assert(ND >= NB && ND >= NS, "a retired group must not be overtaken by the next one on its barrier");
   static constexpr int BAR = RAW + NRAW * REC;
-  static constexpr int TOTAL = BAR + 512 + 1024;                   // barriers + slack to align the base
+  static constexpr int EPI = BAR + 512;                            // per epilogue warp: token factors, then 16 tokens x 32 rows of 16 bits
+  static constexpr int TOTAL = EPI + 8 * kTcEpiBytes + 1024;       // + slack to align the base
   static_assert(TOTAL <= 227 * 1024, "prompt GEMM shared memory");
   // tensor memory columns: two accumulators, A stages, A_z (8 columns = one k16 step of the row's zero point, the same for every
   // step of the group)
@@ -392,12 +394,6 @@ struct TcWalk {
   __device__ __forceinline__ void next() { item += step; set(); }
 };
 
-// Tokens whose accumulators an epilogue thread takes together: 16 where an epilogue reads nothing but factors (more independent
-// exponentials and stores in flight), 8 where every token brings an operand from global memory.
-template <int EPI>
-__host__ __device__ constexpr int tc_chunk(int tokens) {
-  return (EPI == EPI_SWIGLU || EPI == EPI_LOGITS) && tokens % 16 == 0 ? 16 : 8;
-}
 // What one chunk of the epilogue reads from global memory (issued early: it does not depend on the GEMM)
 template <int EPI, int CH>
 struct TcOperands {
@@ -432,11 +428,31 @@ struct TcFactors {
   __device__ __forceinline__ float x(int i) const { return __shfl_sync(0xffffffffu, i < 32 ? fx[0] : fx[1], i & 31); }
   __device__ __forceinline__ float a(int i) const { return __shfl_sync(0xffffffffu, i < 32 ? fa[0] : fa[1], i & 31); }
 };
+// The same from a table that the warp keeps in shared memory (prompts: 64 tokens an item; a shuffle per token and factor costs more)
+struct TcFactorTable {
+  float *fx, *fa;
+  template <int EPI>
+  __device__ __forceinline__ void fill(const VtcParams& P, int t0, int tend, int lane) {
+    TcFactors<EPI> f;
+    f.fetch(P, t0, tend, lane);
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+      fx[32 * k + lane] = f.fx[k];
+      if (EPI == EPI_SWIGLU) fa[32 * k + lane] = f.fa[k];
+    }
+    __syncwarp();
+  }
+  __device__ __forceinline__ float x(int i) const { return fx[i]; }
+  __device__ __forceinline__ float a(int i) const { return fa[i]; }
+};
+// silu(g) = g / (1 + e^-g). The division by approximate reciprocal (2 ulp) sits behind an exponential of the same accuracy and ahead of a
+// rounding to bf16; the exact one brings a branch per value, which keeps an epilogue's independent values from overlapping.
+__device__ __forceinline__ float tc_silu(float g) { return __fdividef(g, 1.0f + __expf(-g)); }
 // v[e] = accumulator of (stream row srow, token t0 + e), the i0 + e-th of the warp's tokens; rf = the row's factor. The whole warp
 // calls this together: lanes 2i, 2i + 1 hold the two rows of a RoPE or gate/up pair.
-template <int EPI, int CH>
+template <int EPI, int CH, class F>
 __device__ __forceinline__ void vtc_epilogue(const VtcParams& P, int srow, int t0, int tend, float (&v)[CH], float rf,
-                                             const TcFactors<EPI>& f, int i0, const TcOperands<EPI, CH>& o, int lane) {
+                                             const F& f, int i0, const TcOperands<EPI, CH>& o, int lane) {
   const bool live = srow < P.rows, odd = lane & 1;
 #pragma unroll
   for (int e = 0; e < CH; e++) v[e] = v[e] * rf * f.x(i0 + e);
@@ -456,7 +472,7 @@ __device__ __forceinline__ void vtc_epilogue(const VtcParams& P, int srow, int t
       const float gg = rbf(odd ? got : v[e]), uu = rbf(odd ? v[e + 1] : got);
       const float f0 = f.a(i0 + e), f1 = f.a(i0 + e + 1);
       const int t = t0 + e + (odd ? 1 : 0);
-      const __half a = __float2half_rn(rbf((gg / (1.0f + __expf(-gg))) * uu) * (odd ? f1 : f0));
+      const __half a = __float2half_rn(rbf(tc_silu(gg) * uu) * (odd ? f1 : f0));
       if (live && t < tend) P.act[(size_t)t * P.out_ld + (srow >> 1)] = __half_as_ushort(a);
     }
   } else {
@@ -481,6 +497,68 @@ __device__ __forceinline__ void vtc_epilogue(const VtcParams& P, int srow, int t
     }
   }
 }
+
+// RESID and SWIGLU of 16 tokens by a warp (32 weight rows), through 1 KB of shared memory: the outputs of a token are adjacent there and
+// leave 16 bytes at a time (the residual comes the same way). Thread by thread they are 2-byte accesses, an address and a predicate per
+// value, and with them the epilogue of a 128 x 128 item took as long as its MMAs left idle: prompts of 100 / 250 / 725 tokens of the 3B
+// shape 3710 / 4465 / 7200 us, without any epilogue 3100 / 3630 / 6270.
+template <int EPI>
+struct TcStaged {
+  static constexpr int NV = EPI == EPI_RESID ? 2 : 1;           // 16-byte vectors of a lane: 16 tokens x 64 bytes, or x 32 (SWIGLU halves the rows)
+  static constexpr int LPT = NV * 2;                            // lanes per token
+  uint4 h[NV];
+  __device__ __forceinline__ uint16_t* at(const VtcParams& P, int wrow, int tok, int lane) const {
+    uint16_t* base = EPI == EPI_RESID ? P.h + wrow : P.act + (wrow >> 1);
+    return base + (size_t)tok * P.out_ld + (lane % LPT) * 8;
+  }
+  __device__ __forceinline__ void fetch(const VtcParams& P, int wrow, int t0, int tend, int lane) {
+    if (EPI == EPI_RESID) {
+#pragma unroll
+      for (int i = 0; i < NV; i++) {
+        const int tok = t0 + i * (32 / LPT) + lane / LPT;
+        h[i] = tok < tend ? __ldcg(reinterpret_cast<const uint4*>(at(P, wrow, tok, lane))) : make_uint4(0, 0, 0, 0);
+      }
+    }
+  }
+  // v[e]: accumulator of row wrow + lane and token t0 + e, the i0 + e-th of the warp's tokens
+  __device__ __forceinline__ void run(const VtcParams& P, uint8_t* stage, int wrow, int t0, int tend, float (&v)[16], float rf,
+                                      const TcFactorTable& f, int i0, int lane) {
+    uint16_t* s16 = reinterpret_cast<uint16_t*>(stage);
+    const bool odd = lane & 1;
+    if (EPI == EPI_RESID) {
+#pragma unroll
+      for (int i = 0; i < NV; i++) reinterpret_cast<uint4*>(stage)[i * 32 + lane] = h[i];
+      __syncwarp();
+    }
+#pragma unroll
+    for (int e4 = 0; e4 < 16; e4 += 4) {
+      const float4 fx = *reinterpret_cast<const float4*>(f.fx + i0 + e4);
+      v[e4] = v[e4] * rf * fx.x; v[e4 + 1] = v[e4 + 1] * rf * fx.y; v[e4 + 2] = v[e4 + 2] * rf * fx.z; v[e4 + 3] = v[e4 + 3] * rf * fx.w;
+      if (EPI == EPI_RESID) {
+#pragma unroll
+        for (int e = e4; e < e4 + 4; e++) s16[e * 32 + lane] = f2bf(bf2f(s16[e * 32 + lane]) + v[e] * P.resid);
+      } else {
+        const float4 fa = *reinterpret_cast<const float4*>(f.fa + i0 + e4);
+        // rows (2i, 2i + 1) = (gate_i, up_i): the even lane takes the even tokens of the pair, the odd lane the odd ones
+#pragma unroll
+        for (int e = e4; e < e4 + 4; e += 2) {
+          const float got = __shfl_xor_sync(0xffffffffu, odd ? v[e] : v[e + 1], 1);
+          const float gg = rbf(odd ? got : v[e]), uu = rbf(odd ? v[e + 1] : got);
+          const float a = e == e4 ? (odd ? fa.y : fa.x) : (odd ? fa.w : fa.z);
+          s16[(e + (odd ? 1 : 0)) * 16 + (lane >> 1)] = __half_as_ushort(__float2half_rn(rbf(tc_silu(gg) * uu) * a));
+        }
+      }
+    }
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < NV; i++) {
+      const int tok = t0 + i * (32 / LPT) + lane / LPT;
+      const uint4 o = reinterpret_cast<const uint4*>(stage)[i * 32 + lane];
+      if (tok < tend) *reinterpret_cast<uint4*>(at(P, wrow, tok, lane)) = o;
+    }
+    __syncwarp();
+  }
+};
 
 // after a failure: the copies and MMAs in flight (see drain_phase); out of line, a healthy launch never comes here
 template <int NRAW, int NS, int NB, int ND>
@@ -531,9 +609,6 @@ __global__ void __launch_bounds__(kTcThreads, 1) v_gemm_tc(const __grid_constant
   const int quad = warp & 3, row = quad * 32 + lane;             // warps 4..19: row of the block = TMEM lane
   const int half = ((warp >> 2) & 1) ^ 1;                        // warps 4..11: half of a group's columns; 12..19: of the tokens
   bool ok = true;
-  constexpr int CH = tc_chunk<EPI>(HC);
-  TcOperands<EPI, CH> pre;
-  TcFactors<EPI> fac;
 
   if (warp == 0) {
     // ---------------- producer: the groups' records (weights do not depend on the previous kernel)
@@ -660,7 +735,13 @@ __global__ void __launch_bounds__(kTcThreads, 1) v_gemm_tc(const __grid_constant
     }
   } else if (warp >= 12) {
     // ---------------- epilogue: thread = (row of the block, half of the tokens), 8 or 16 tokens at a time
+    constexpr bool STAGED = EPI == EPI_RESID || EPI == EPI_SWIGLU;
+    constexpr int CH = STAGED || EPI == EPI_LOGITS ? 16 : 8;
     const uint32_t tlane = tmem + ((uint32_t)(quad * 32) << 16) + half * HC;
+    uint8_t* area = tsm + S::EPI + (warp - 12) * kTcEpiBytes;
+    TcFactorTable fac{reinterpret_cast<float*>(area), reinterpret_cast<float*>(area) + 64};
+    TcOperands<EPI, CH> pre;
+    TcStaged<EPI> staged;
     Ring<2> ra;
     pdl_wait();
     for (TcWalk w(P); w.valid() && ok; w.next(), ra.next()) {
@@ -668,8 +749,10 @@ __global__ void __launch_bounds__(kTcThreads, 1) v_gemm_tc(const __grid_constant
       // the row's factor and the first chunk's operands are fetched while the GEMM runs
       const float rf = __ldg(reinterpret_cast<const float*>(P.w + (size_t)(w.rb + 1) * tc_block_bytes(P.K, HZ)) - kTcTrailer / 4 + row);
       const int th0 = tok0 + half * HC, the = min(tend, th0 + HC);
-      pre.fetch(P, srow, th0, the);
-      fac.fetch(P, th0, the, lane);
+      if constexpr (STAGED) staged.fetch(P, srow - lane, th0, the, lane);
+      else pre.fetch(P, srow, th0, the);
+      __syncwarp();
+      fac.fill<EPI>(P, th0, the, lane);
       ok = __all_sync(0xffffffffu, mbar_wait(&acc_full[ra.i], ra.lap, wc, W_FULL, 10));
       if (!ok) break;
       tc_fence_after();
@@ -679,13 +762,20 @@ __global__ void __launch_bounds__(kTcThreads, 1) v_gemm_tc(const __grid_constant
 #pragma unroll
         for (int c8 = 0; c8 < CH / 8; c8++) tc_ld8(tlane + ra.i * NT + (t0 - th0) + c8 * 8, u[c8]);
         TcOperands<EPI, CH> nxt;
-        nxt.fetch(P, srow, t0 + CH, the);
+        TcStaged<EPI> snxt;
+        if constexpr (STAGED) snxt.fetch(P, srow - lane, t0 + CH, the, lane);
+        else nxt.fetch(P, srow, t0 + CH, the);
         tc_ld_wait();
         float v[CH];
 #pragma unroll
         for (int e = 0; e < CH; e++) v[e] = __uint_as_float(u[e >> 3][e & 7]);
-        vtc_epilogue<EPI, CH>(P, srow, t0, the, v, rf, fac, t0 - th0, pre, lane);
-        pre = nxt;
+        if constexpr (STAGED) {
+          staged.run(P, area + 512, srow - lane, t0, the, v, rf, fac, t0 - th0, lane);
+          staged = snxt;
+        } else {
+          vtc_epilogue<EPI, CH>(P, srow, t0, the, v, rf, fac, t0 - th0, pre, lane);
+          pre = nxt;
+        }
       }
       tc_fence_before();
       __syncwarp();

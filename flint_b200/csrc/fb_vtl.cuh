@@ -280,8 +280,20 @@ __global__ void __launch_bounds__(kTlThreads, 2) v_gemm_tl(const __grid_constant
 #pragma unroll
         for (int e = 0; e < CH; e++) {
           v[e] = 0.f;
-          if (t0 + e < HT)
-            for (int r = 0; r < ns; r++) v[e] += yw[(r * TPR + t0 + e) * 128];
+          if (t0 + e < HT) {
+            if constexpr (NT < 64) {                           // four ranks' sums requested together; 64 tokens keep enough loads in flight
+#pragma unroll 1
+              for (int r0 = 0; r0 < ns; r0 += 4) {
+                float y[4];
+#pragma unroll
+                for (int r = 0; r < 4; r++) y[r] = r0 + r < ns ? yw[((r0 + r) * TPR + t0 + e) * 128] : 0.f;
+#pragma unroll
+                for (int r = 0; r < 4; r++) v[e] += y[r];
+              }
+            } else {
+              for (int r = 0; r < ns; r++) v[e] += yw[(r * TPR + t0 + e) * 128];
+            }
+          }
         }
       } else {
         uint32_t u[8];
