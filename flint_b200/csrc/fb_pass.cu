@@ -27,6 +27,15 @@ int tl_splits(int items, int k, int nt, int sms) {
   while (ns < 8 && items * ns * 2 <= 2 * sms && G / (ns * 2) >= 2 && nt / (ns * 2) >= 2) ns *= 2;
   return ns;
 }
+// The same for the tiles of a prompt, one CTA per SM, at least four groups each. Clusters of eight fit only in 120 of 148 SMs: at most four.
+// 1: the persistent kernel, which overlaps an item's epilogue with the next item. In it prompts of 70 / 100 / 128 / 180 / 250 / 300 tokens of the
+// 3B shape took 3200 / 3388 / 3535 / 3684 / 4092 / 4437 us, split in four (one tile) or two 2566 / 2670 / 2750 / 3700 / 3911 / 4150; 100 / 200
+// tokens of the 8B shape 4290 / 5320 -> 3270 / 4725.
+int prompt_splits(int items, int k, int sms) {
+  int ns = 1;
+  while (ns < 4 && items * ns * 2 <= sms && k / 128 / (ns * 2) >= 4) ns *= 2;
+  return ns;
+}
 template <int NT, int EPI, bool HZ>
 cudaError_t launch_vtl_hz(VtcParams& p, int sms, cudaStream_t st) {
   static bool configured[64] = {};
@@ -36,9 +45,9 @@ cudaError_t launch_vtl_hz(VtcParams& p, int sms, cudaStream_t st) {
     FB_TRY(cudaFuncSetAttribute(v_gemm_tl<NT, EPI, HZ>, cudaFuncAttributeMaxDynamicSharedMemorySize, VtlSmem<NT, HZ>::TOTAL));
     configured[dev] = true;
   }
-  if (p.K % 128 || p.M > NT) return cudaErrorInvalidValue;
-  const int items = (p.rows + kTcRowBlock - 1) / kTcRowBlock;
-  p.nsplit = tl_splits(items, p.K, NT, sms);
+  if (p.K % 128 || p.ntok > NT || p.ntok % 16 || (NT < 128 && p.ntile > 1) || (size_t)p.ntok * p.ntile < (size_t)p.M) return cudaErrorInvalidValue;
+  const int items = (p.rows + kTcRowBlock - 1) / kTcRowBlock * p.ntile;
+  p.nsplit = NT == 128 ? prompt_splits(items, p.K, sms) : tl_splits(items, p.K, NT, sms);
   return launch_pdl_cluster(v_gemm_tl<NT, EPI, HZ>, dim3(items * p.nsplit), dim3(kTlThreads), (size_t)VtlSmem<NT, HZ>::TOTAL, st,
                             (unsigned)p.nsplit, p);
 }
@@ -63,7 +72,10 @@ cudaError_t launch_vtc(VtcParams& p, const CUtensorMap* maps, int nt, bool hz, i
     case 16: return hz ? launch_vtl_hz<16, EPI, true>(p, sms, st) : launch_vtl_hz<16, EPI, false>(p, sms, st);
     case 32: return hz ? launch_vtl_hz<32, EPI, true>(p, sms, st) : launch_vtl_hz<32, EPI, false>(p, sms, st);
     case 64: return hz ? launch_vtl_hz<64, EPI, true>(p, sms, st) : launch_vtl_hz<64, EPI, false>(p, sms, st);
-    case 128: return hz ? launch_vtc_hz<EPI, true>(p, sms, st) : launch_vtc_hz<EPI, false>(p, sms, st);
+    case 128:
+      if (prompt_splits((p.rows + kTcRowBlock - 1) / kTcRowBlock * p.ntile, p.K, sms) > 1)
+        return hz ? launch_vtl_hz<128, EPI, true>(p, sms, st) : launch_vtl_hz<128, EPI, false>(p, sms, st);
+      return hz ? launch_vtc_hz<EPI, true>(p, sms, st) : launch_vtc_hz<EPI, false>(p, sms, st);
   }
   return cudaErrorInvalidValue;
 }

@@ -25,9 +25,9 @@
 // reads its words without bank conflicts.
 //
 // Work item = (token tile, row block), round-robin over persistent CTAs; two accumulators, so an item's epilogue overlaps the MMAs of
-// the next. Trees split K over a CLUSTER instead: every CTA sends the sums of a share of the tokens to each CTA of its cluster
-// through distributed shared memory, and each finishes its own tokens (sum in split order: deterministic), so the split costs one
-// cluster barrier instead of a round trip through global memory. Every wait is bounded.
+// the next. Trees and short prompts split K over a CLUSTER instead (fb_vtl.cuh): every CTA sends the sums of a share of the tokens to each CTA of its cluster
+// through distributed shared memory, and each finishes its own tokens (sum in split order: deterministic), so the split costs no
+// round trip through global memory. Every wait is bounded.
 #pragma once
 #include <cuda.h>
 
@@ -251,7 +251,7 @@ struct alignas(64) VtcParams {
   CUtensorMap xmap;          // activations fp16 [rows >= M][K] as a 2-D tensor, box 64 columns x NT tokens, 128-byte swizzle
   const uint8_t* w;          // TC layout of this matrix
   int rows, K, M;
-  int nsplit;                // trees: CTAs of a cluster that share one item's K (1, 2, 4 or 8)
+  int nsplit;                // v_gemm_tl: CTAs of a cluster that share one item's K (1, 2, 4 or 8)
   int ntok, ntile;           // tokens of one tile (a multiple of 16, <= NT; one tile unless this is a prompt) and tiles
   DevStatus* status;
   unsigned spin_limit;
@@ -334,7 +334,7 @@ __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, i
       "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
       ::"r"(smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(smem_u32(bar)) : "memory");
 }
-// cluster of the K splits: barrier over all threads of all its CTAs, and plain stores into a neighbour's shared memory
+// cluster of the K splits: barrier over all threads of all its CTAs, and stores into a neighbour's shared memory
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
 __device__ __forceinline__ uint32_t map_rank(uint32_t saddr, uint32_t rank) {
@@ -432,9 +432,7 @@ struct TcFactors {
 struct TcFactorTable {
   float *fx, *fa;
   template <int EPI>
-  __device__ __forceinline__ void fill(const VtcParams& P, int t0, int tend, int lane) {
-    TcFactors<EPI> f;
-    f.fetch(P, t0, tend, lane);
+  __device__ __forceinline__ void put(const TcFactors<EPI>& f, int lane) {
 #pragma unroll
     for (int k = 0; k < 2; k++) {
       fx[32 * k + lane] = f.fx[k];
@@ -752,7 +750,9 @@ __global__ void __launch_bounds__(kTcThreads, 1) v_gemm_tc(const __grid_constant
       if constexpr (STAGED) staged.fetch(P, srow - lane, th0, the, lane);
       else pre.fetch(P, srow, th0, the);
       __syncwarp();
-      fac.fill<EPI>(P, th0, the, lane);
+      TcFactors<EPI> mine;
+      mine.fetch(P, th0, the, lane);
+      fac.put<EPI>(mine, lane);
       ok = __all_sync(0xffffffffu, mbar_wait(&acc_full[ra.i], ra.lap, wc, W_FULL, 10));
       if (!ok) break;
       tc_fence_after();

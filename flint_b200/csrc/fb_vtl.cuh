@@ -1,11 +1,13 @@
-// The GEMM of fb_vtc.cuh for one tile of up to 64 tokens (tree verification), sized so that TWO CTAs share an SM: at most 113 KB of
-// shared memory, 256 tensor-memory columns and 72 registers a thread. A verify pass is a chain of short dependent launches (4 to 6 us
+// The GEMM of fb_vtc.cuh with one work item per CTA and K split over a cluster: trees, and short prompts, whose tiles alone would leave most
+// SMs without work.
+// One tile of up to 64 tokens (tree verification) is sized so that TWO CTAs share an SM: at most 113 KB of shared memory, 256 tensor-memory columns and 72 registers a thread. A verify pass is a chain of short dependent launches (4 to 6 us
 // of work each); with programmatic dependent launch the next GEMM's CTAs become resident while the previous kernel still runs, so
 // barrier set-up, the tensor-memory allocation, the weight ring and the first dequantised stages are done before the activations
 // exist. The 200 KB form left every launch to ramp up after its predecessor had gone: QKV / O / gate-up / down took
-// 9.7 / 9.4 / 11.1 / 12.1 us at 26 tokens of the 3B shape.
+// 9.7 / 9.4 / 11.1 / 12.1 us at 26 tokens of the 3B shape. The 128-token tiles of a prompt take a whole SM; what their long K needs is the
+// split (64 groups of the down projection in a row are 22 us).
 //
-// One work item (row block) per CTA, K split over a cluster of up to eight CTAs. Warps: 0 weight producer, 1 MMA issue, 2..4
+// One work item (row block of a token tile) per CTA, K split over a cluster of up to eight CTAs (four at 128 tokens). Warps: 0 weight producer, 1 MMA issue, 2..4
 // activations (tensor copies, or the fp16 conversion of the attention output), 5 code warm-up, 6..13 dequantise, then epilogue.
 #pragma once
 #include "fb_vtc.cuh"
@@ -16,9 +18,9 @@ constexpr int kTlThreads = 448;
 template <int NT, bool HZ>
 struct VtlSmem {
   static constexpr int REC = tc_rec_bytes(HZ);
-  static constexpr int NS = NT == 64 && HZ ? 2 : 3;                // dequantised groups (64 tensor-memory columns each)
-  static constexpr int NB = NT == 16 ? 8 : (NT == 32 ? 5 : 3);     // activation stages
-  static constexpr int NRAW = NT == 16 ? 7 : (NT == 32 ? 5 : 3);   // raw int4 groups
+  static constexpr int NS = NT == 128 ? (HZ ? 5 : 6) : (NT == 64 && HZ ? 2 : 3);      // dequantised groups (64 tensor-memory columns each)
+  static constexpr int NB = NT == 16 ? 8 : (NT == 32 ? 5 : (NT == 64 ? 3 : 4));       // activation stages
+  static constexpr int NRAW = NT == 16 ? 7 : (NT == 32 ? 5 : (NT == 64 || HZ ? 3 : 4)); // raw int4 groups
   static constexpr int BSTAGE = NT * 256;
   static constexpr int B = 0;
   static constexpr int RAW = B + NB * BSTAGE;
@@ -27,8 +29,10 @@ struct VtlSmem {
   static constexpr int YS = RAW + NRAW * REC;                      // K splits: [source rank][tokens][128 rows] fp32
   static constexpr int BAR = YS + NT * 512;
   static constexpr int TOTAL = BAR + 512 + 1024;
-  static_assert(TOTAL <= 113 * 1024, "two CTAs per SM");
-  static constexpr int T_A = NT, T_AZ = T_A + NS * 64, TCOLS = 256;
+  static constexpr int CTAS = NT == 128 ? 1 : 2;                   // per SM
+  static_assert(TOTAL <= (CTAS == 2 ? 113 : 227) * 1024, "shared memory of an SM");
+  static_assert(NT < 128 || 8 * kTcEpiBytes <= NB * BSTAGE, "the epilogue of 128 tokens stages in the dead activation ring");
+  static constexpr int T_A = NT, T_AZ = T_A + NS * 64, TCOLS = 512 / CTAS;
   static_assert(T_AZ + (HZ ? NS * 8 : 0) <= TCOLS, "tensor memory columns");
 };
 
@@ -44,7 +48,7 @@ inline __device__ __noinline__ void tl_drain(uint64_t* bars, volatile int* s_iss
 }
 
 template <int NT, int EPI, bool HZ>
-__global__ void __launch_bounds__(kTlThreads, 2) v_gemm_tl(const __grid_constant__ VtcParams P) {
+__global__ void __launch_bounds__(kTlThreads, NT == 128 ? 1 : 2) v_gemm_tl(const __grid_constant__ VtcParams P) {
   using S = VtlSmem<NT, HZ>;
   constexpr int NRAW = S::NRAW, NS = S::NS, NB = S::NB, ND = S::ND, REC = S::REC, HC = NT / 2;
   extern __shared__ __align__(1024) uint8_t tsm_raw[];
@@ -76,7 +80,10 @@ __global__ void __launch_bounds__(kTlThreads, 2) v_gemm_tl(const __grid_constant
   tc_fence_after();
   const uint32_t tmem = *s_tmem;
   WaitCtl wc{P.status, s_abort, P.spin_limit};
-  const int ns = P.nsplit, lg = 31 - __clz(ns), rank = (int)blockIdx.x & (ns - 1), rb = (int)blockIdx.x >> lg, G = P.K / 128;
+  const int ns = P.nsplit, lg = 31 - __clz(ns), rank = (int)blockIdx.x & (ns - 1), item = (int)blockIdx.x >> lg, G = P.K / 128;
+  // a prompt may have several token tiles (NT = 128 only)
+  const int nrb = (P.rows + kTcRowBlock - 1) / kTcRowBlock, rb = NT == 128 ? item % nrb : item, tok0 = NT == 128 ? item / nrb * P.ntok : 0,
+            tend = NT == 128 ? min(P.M, tok0 + P.ntok) : P.M;
   const int g0 = G * rank >> lg, ng = (G * (rank + 1) >> lg) - g0;           // this CTA's groups (ng >= 1)
   const bool split = ns > 1;
   if (split) { cluster_arrive(); cluster_wait(); }               // the neighbours' shared memory exists from here on
@@ -126,7 +133,7 @@ __global__ void __launch_bounds__(kTlThreads, 2) v_gemm_tl(const __grid_constant
     if (lane == 0) s_issued[1] = gi < ng ? gi : -1;
   } else if (warp < 5) {
     // ---------------- activations (the previous kernel's output). Token rows past M only feed accumulator columns that nobody reads.
-    if (EPI == EPI_RESID && P.xbf) {
+    if (NT < 128 && EPI == EPI_RESID && P.xbf) {
       // the attention output in bf16: each of the three warps converts every third group to fp16 times the token's power of two
       pdl_wait();
       float fm[2];
@@ -138,7 +145,7 @@ __global__ void __launch_bounds__(kTlThreads, 2) v_gemm_tl(const __grid_constant
         if (!ok) break;
         uint8_t* dst = tsm + S::B + (li % NB) * S::BSTAGE + (c16 >> 3) * (NT * 128);
         const uint16_t* src = P.xbf + (size_t)(g0 + li) * 128 + c16 * 8;
-#pragma unroll
+#pragma unroll 1                                               // unrolled, the loads of all tokens at once spill: 26 / 61 tokens 2116 / 2735 us, so 2079 / 2637
         for (int k0 = 0; k0 < NT / 2; k0 += 8) {
           uint4 v[8];
 #pragma unroll
@@ -168,30 +175,33 @@ __global__ void __launch_bounds__(kTlThreads, 2) v_gemm_tl(const __grid_constant
           if (!ok) break;
           mbar_expect_tx(&b_full[r.i], S::BSTAGE);
           uint8_t* dst = tsm + S::B + r.i * S::BSTAGE;
-          tma_load_2d(dst, &P.xmap, (g0 + gi) * 128, 0, &b_full[r.i]);
-          tma_load_2d(dst + NT * 128, &P.xmap, (g0 + gi) * 128 + 64, 0, &b_full[r.i]);
+          tma_load_2d(dst, &P.xmap, (g0 + gi) * 128, tok0, &b_full[r.i]);
+          tma_load_2d(dst + NT * 128, &P.xmap, (g0 + gi) * 128 + 64, tok0, &b_full[r.i]);
         }
         s_issued[2] = gi;
       }
     }
-  } else {
+  } else if (NT < 128 || warp > 5) {
     // ---------------- dequantise: thread = (row of the block = TMEM lane, half of the group's columns), then epilogue: thread = (row,
     // half of the tokens). Warp 5 walks through the epilogue first, with every store and remote write switched off, so that its
     // instructions are in the cache when the sums arrive: the code of a dozen kernels passes through that cache every layer, and cold
     // the QKV epilogue took 3.3 us for what is 0.4 us of work.
-    constexpr int CH = 4;
+    constexpr bool STAGED = NT == 128 && (EPI == EPI_RESID || EPI == EPI_SWIGLU);
+    constexpr int CH = STAGED ? 16 : 4;
     const int quad = warp & 3, row = quad * 32 + lane, half = warp >= 10;
     const uint32_t tq = tmem + ((uint32_t)(quad * 32) << 16);
     const int* trailer = reinterpret_cast<const int*>(blk + (size_t)G * REC);
     const bool fast = !HZ && __ldg(trailer + kTcRowBlock) != 0;
-    // splits: this CTA finishes tokens [rank * TPR, (rank + 1) * TPR) of the block
+    // splits: this CTA finishes tokens [rank * TPR, (rank + 1) * TPR) of the tile
     const int TPR = NT >> lg, lgT = 31 - __clz(TPR), HT = split ? TPR >> 1 : HC;
-    const int srow = rb * 128 + row, th0 = (split ? rank * TPR : 0) + half * HT, the = min(P.M, th0 + HT);
-    TcOperands<EPI, CH> pre;
+    const int srow = rb * 128 + row, th0 = tok0 + (split ? rank * TPR : 0) + half * HT, the = min(tend, th0 + HT);
+    TcOperands<EPI, STAGED ? 1 : CH> pre;
+    TcStaged<EPI> staged;
     TcFactors<EPI> fac;
     auto fetch = [&]() {                                         // what the epilogue reads, requested while the last groups run
       pdl_wait();
-      pre.fetch(P, srow, th0, the);
+      if constexpr (STAGED) staged.fetch(P, srow - lane, th0, the, lane);
+      else pre.fetch(P, srow, th0, the);
       fac.fetch(P, th0, the, lane);
     };
     pre.fetch(P, srow, 0, 0);                                    // nothing: defined values for the walk-through
@@ -203,7 +213,7 @@ __global__ void __launch_bounds__(kTlThreads, 2) v_gemm_tl(const __grid_constant
     Ring<NS> rs;
     int gi = 0;
     const bool real = warp > 5;
-    const int gend = real ? ng : 0, tend = real ? the : th0, push_end = real ? P.M : 0;
+    const int gend = real ? ng : 0, tlast = real ? the : th0, push_end = real ? tend - tok0 : 0;
 #pragma unroll 1
     for (; gi < gend; gi++, rr.next(), rs.next()) {
       if (gi == NS) fetch();                                   // the first groups are ready; everything later needs the activations
@@ -276,7 +286,7 @@ __global__ void __launch_bounds__(kTlThreads, 2) v_gemm_tl(const __grid_constant
     if (ok) do {
       float v[CH];
       if (split) {
-        if (t0) pre.fetch(P, srow, th0 + t0, tend);
+        if (!STAGED && t0) pre.fetch(P, srow, th0 + t0, tlast);
 #pragma unroll
         for (int e = 0; e < CH; e++) {
           v[e] = 0.f;
@@ -291,21 +301,31 @@ __global__ void __launch_bounds__(kTlThreads, 2) v_gemm_tl(const __grid_constant
                 for (int r = 0; r < 4; r++) v[e] += y[r];
               }
             } else {
+#pragma unroll 4
               for (int r = 0; r < ns; r++) v[e] += yw[(r * TPR + t0 + e) * 128];
             }
           }
         }
       } else {
-        uint32_t u[8];
-        tc_ld8(tlane + t0, u);
-        if (t0) pre.fetch(P, srow, th0 + t0, tend);
+        uint32_t u[(CH + 7) / 8][8];
+#pragma unroll
+        for (int c8 = 0; c8 < (CH + 7) / 8; c8++) tc_ld8(tlane + t0 + c8 * 8, u[c8]);
+        if (!STAGED && t0) pre.fetch(P, srow, th0 + t0, tlast);
         tc_ld_wait();
 #pragma unroll
-        for (int e = 0; e < CH; e++) v[e] = __uint_as_float(u[e]);
+        for (int e = 0; e < CH; e++) v[e] = __uint_as_float(u[e >> 3][e & 7]);
       }
-      vtc_epilogue<EPI, CH>(P, srow, th0 + t0, tend, v, rf, fac, t0, pre, lane);
+      if constexpr (STAGED) {
+        uint8_t* area = tsm + S::B + (warp - 6) * kTcEpiBytes;
+        TcFactorTable tab{reinterpret_cast<float*>(area), reinterpret_cast<float*>(area) + 64};
+        if (t0 == 0) tab.put<EPI>(fac, lane);
+        else staged.fetch(P, srow - lane, th0 + t0, tlast, lane);
+        staged.run(P, area + 512, srow - lane, th0 + t0, tlast, v, rf, tab, t0, lane);
+      } else {
+        vtc_epilogue<EPI, CH>(P, srow, th0 + t0, tlast, v, rf, fac, t0, pre, lane);
+      }
       t0 += CH;
-    } while (th0 + t0 < tend);
+    } while (th0 + t0 < tlast);
   }
   if (split && warp < 6) {
     __syncwarp();

@@ -203,6 +203,22 @@ def test_prompt_pass_tile_and_chunk_edges(M):
     eng.close()
 
 
+@pytest.mark.parametrize("asym", [False, True])
+@pytest.mark.parametrize("M", [65, 128, 129, 300])
+def test_prompt_tiles_with_split_k(M, asym):
+    """Short prompts on a shape with few row blocks (24 / 16 / 16 of QKV, O, down): one, two and three token tiles run as clusters of four and of
+    two, one of them with tokens in only part of its ranks."""
+    cfg = ModelArgs.from_name("llama-1b-class")
+    cfg.n_layer, cfg.vocab_size = 1, 512
+    orc, eng = _pair(cfg, M + 8, 3, packing.synth_packed(cfg, 0, asym=asym))
+    toks = torch.randint(0, cfg.vocab_size, (M,), generator=torch.Generator().manual_seed(M)).tolist()
+    ref = np.concatenate([orc.verify(toks[i:i + 64], 3 + i)[0] for i in range(0, M, 64)])
+    lg, _ = eng.prefill(toks, 3)
+    eng.check()
+    assert np.abs(lg.cpu().numpy() - ref).max() < _tol(ref)
+    eng.close()
+
+
 @pytest.mark.parametrize("vocab", [1, 31, 4096, 8200, 32768, 49160, 128256, 300001])
 def test_token_choice_over_every_split_of_a_row(vocab):
     """Rows on one, two, four and eight CTAs, slices that fit the registers and slices that do not, ragged ends: the arg-max
