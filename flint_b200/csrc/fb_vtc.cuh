@@ -345,6 +345,10 @@ __device__ __forceinline__ uint32_t map_rank(uint32_t saddr, uint32_t rank) {
 __device__ __forceinline__ void st_cluster_f32(uint32_t addr, float v) {
   asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory");
 }
+// the same, counted on a barrier of that CTA
+__device__ __forceinline__ void st_async(uint32_t addr, uint32_t v, uint32_t bar) {
+  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::"r"(addr), "r"(v), "r"(bar) : "memory");
+}
 
 // Shared-memory plan (bytes). The raw ring keeps HBM busy; a stage of activations is a group's two 64-column tiles.
 template <bool HZ>

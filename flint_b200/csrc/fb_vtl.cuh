@@ -38,25 +38,32 @@ struct VtlSmem {
 
 // after a failure: the copies and MMAs in flight (see drain_phase); out of line, a healthy launch never comes here
 template <int NRAW, int NS, int NB, int ND>
-inline __device__ __noinline__ void tl_drain(uint64_t* bars, volatile int* s_issued) {
+inline __device__ __noinline__ void tl_drain(uint64_t* bars, volatile int* s_issued, bool exchange) {
   uint64_t *raw_full = bars, *b_full = bars + 2 * NRAW + NS, *done = b_full + NB, *acc_full = done + ND;
   const int n = s_issued[1];
   drain_ring<NRAW>(raw_full, s_issued[0]);
   drain_ring<NB>(b_full, s_issued[2]);
   if (n) drain_phase(n > 0 ? &done[(n - 1) % ND] : acc_full, n > 0 ? ((n - 1) / ND) & 1 : 0);
+  // sums on their way here or from here: a neighbour that gave up before it sent any leaves the barrier open, and every neighbour is behind the
+  // cluster barrier by now, so what is under way lands within microseconds
+  if (exchange)
+#pragma unroll 1
+    for (int i = 0; i < 200 && !mbar_test(acc_full + 1, 0); i++) __nanosleep(1000);
   __syncwarp();
 }
 
 template <int NT, int EPI, bool HZ>
 __global__ void __launch_bounds__(kTlThreads, NT == 128 ? 1 : 2) v_gemm_tl(const __grid_constant__ VtcParams P) {
   using S = VtlSmem<NT, HZ>;
+  constexpr bool ASYNC = NT < 64;                                // how a split's sums travel, see below
   constexpr int NRAW = S::NRAW, NS = S::NS, NB = S::NB, ND = S::ND, REC = S::REC, HC = NT / 2;
   extern __shared__ __align__(1024) uint8_t tsm_raw[];
   uint8_t* tsm = tsm_raw + ((1024u - (smem_u32(tsm_raw) & 1023u)) & 1023u);
   uint64_t* bars = reinterpret_cast<uint64_t*>(tsm + S::BAR);
   uint64_t *raw_full = bars, *raw_empty = bars + NRAW, *a_full = bars + 2 * NRAW, *b_full = a_full + NS, *done = b_full + NB,
            *acc_full = done + ND;
-  uint32_t* s_tmem = reinterpret_cast<uint32_t*>(acc_full + 1);
+  uint64_t* xbar = acc_full + 1;                                // K splits: the cluster's sums of this CTA's tokens have arrived
+  uint32_t* s_tmem = reinterpret_cast<uint32_t*>(xbar + 1);
   volatile int* s_abort = reinterpret_cast<volatile int*>(s_tmem + 1);
   volatile int* s_issued = s_abort + 1;                          // [3] copies or MMA groups (-1: all) that warps 0, 1, 2 have issued
   float* ys = reinterpret_cast<float*>(tsm + S::YS);
@@ -67,6 +74,7 @@ __global__ void __launch_bounds__(kTlThreads, NT == 128 ? 1 : 2) v_gemm_tl(const
     for (int i = 0; i < NB; i++) mbar_init(&b_full[i], 1);
     for (int i = 0; i < ND; i++) mbar_init(&done[i], 1);
     mbar_init(acc_full, 1);
+    mbar_init(xbar, 1);
     *s_abort = s_issued[2] = 0;
     mbar_fence_init();
   }
@@ -86,7 +94,12 @@ __global__ void __launch_bounds__(kTlThreads, NT == 128 ? 1 : 2) v_gemm_tl(const
             tend = NT == 128 ? min(P.M, tok0 + P.ntok) : P.M;
   const int g0 = G * rank >> lg, ng = (G * (rank + 1) >> lg) - g0;           // this CTA's groups (ng >= 1)
   const bool split = ns > 1;
-  if (split) { cluster_arrive(); cluster_wait(); }               // the neighbours' shared memory exists from here on
+  const int TPR = NT >> lg;                                      // splits: this CTA finishes tokens [rank * TPR, (rank + 1) * TPR) of the tile
+  if (split) {
+    if (ASYNC && tid == 0) mbar_expect_tx(xbar, (uint32_t)(max(0, min(TPR, P.M - rank * TPR)) * ns * 512));
+    cluster_arrive();                                            // the neighbours' shared memory exists, and expects, from here on
+    cluster_wait();
+  }
   const uint8_t* blk = P.w + (size_t)rb * tc_block_bytes(P.K, HZ);
   bool ok = true;
 
@@ -192,8 +205,7 @@ __global__ void __launch_bounds__(kTlThreads, NT == 128 ? 1 : 2) v_gemm_tl(const
     const uint32_t tq = tmem + ((uint32_t)(quad * 32) << 16);
     const int* trailer = reinterpret_cast<const int*>(blk + (size_t)G * REC);
     const bool fast = !HZ && __ldg(trailer + kTcRowBlock) != 0;
-    // splits: this CTA finishes tokens [rank * TPR, (rank + 1) * TPR) of the tile
-    const int TPR = NT >> lg, lgT = 31 - __clz(TPR), HT = split ? TPR >> 1 : HC;
+    const int lgT = 31 - __clz(TPR), HT = split ? TPR >> 1 : HC;
     const int srow = rb * 128 + row, th0 = tok0 + (split ? rank * TPR : 0) + half * HT, the = min(tend, th0 + HT);
     TcOperands<EPI, STAGED ? 1 : CH> pre;
     TcStaged<EPI> staged;
@@ -260,8 +272,11 @@ __global__ void __launch_bounds__(kTlThreads, NT == 128 ? 1 : 2) v_gemm_tl(const
       if (ok) ok = __all_sync(0xffffffffu, mbar_wait(acc_full, 0, wc, W_FULL, 10));
       tc_fence_after();
     }
+    // K splits: token t's sums go to the CTA that finishes it. Few tokens: an asynchronous store per value, counted on that CTA's barrier, so that
+    // nobody waits for a round trip (4 / 14 / 26 tokens of the 3B shape 1647 / 1802 / 2080 -> 1602 / 1749 / 2046 us against a cluster barrier
+    // behind plain stores). From 64 tokens on the plain stores and the barrier are faster: 61 tokens 2637, asynchronous stores 2658, one bulk
+    // copy per neighbour 2670; a prompt of 100 tokens 2667, 2731, 2767.
     if (split) {
-      // token t of this half goes to the CTA that finishes it
       if (ok) {
 #pragma unroll 1
         for (int c = 0; c < HC; c += 8) {
@@ -271,15 +286,23 @@ __global__ void __launch_bounds__(kTlThreads, NT == 128 ? 1 : 2) v_gemm_tl(const
 #pragma unroll
           for (int e = 0; e < 8; e++) {
             const int tk = half * HC + c + e;
-            if (tk < push_end) st_cluster_f32(map_rank(mine + (uint32_t)(tk & (TPR - 1)) * 512, tk >> lgT), __uint_as_float(u[e]));
+            if (tk < push_end) {
+              const uint32_t to = map_rank(mine + (uint32_t)(tk & (TPR - 1)) * 512, tk >> lgT);
+              if (ASYNC) st_async(to, u[e], map_rank(smem_u32(xbar), tk >> lgT));
+              else st_cluster_f32(to, __uint_as_float(u[e]));
+            }
           }
         }
       }
-      if (real) {
-        __syncwarp();
-        cluster_arrive();
-        cluster_wait();                                        // every rank's sums are in
-        ok = __all_sync(0xffffffffu, ok && *s_abort == 0);
+      if (real) {                                              // every rank's sums are in
+        if (ASYNC) {
+          if (ok) ok = __all_sync(0xffffffffu, mbar_wait(xbar, 0, wc, W_FULL, 11));
+        } else {
+          __syncwarp();
+          cluster_arrive();
+          cluster_wait();
+          ok = __all_sync(0xffffffffu, ok && *s_abort == 0);
+        }
       }
     }
     int t0 = 0;
@@ -327,15 +350,16 @@ __global__ void __launch_bounds__(kTlThreads, NT == 128 ? 1 : 2) v_gemm_tl(const
       t0 += CH;
     } while (th0 + t0 < tlast);
   }
-  if (split && warp < 6) {
+  if (split && (ASYNC || warp < 6)) {                            // nobody leaves before its neighbours have sent what they will send
     __syncwarp();
-    cluster_arrive();
+    if (ASYNC) asm volatile("barrier.cluster.arrive.relaxed;" ::: "memory");
+    else cluster_arrive();
     cluster_wait();
   }
   tc_fence_before();
   __syncthreads();
   if (warp == 1) {
-    if (*s_abort) tl_drain<NRAW, NS, NB, ND>(bars, s_issued);
+    if (*s_abort) tl_drain<NRAW, NS, NB, ND>(bars, s_issued, ASYNC && split);
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(S::TCOLS));
   }
 }
