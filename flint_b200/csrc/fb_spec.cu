@@ -18,7 +18,7 @@ struct fb_draft {
   uint16_t *x, *h, *q, *k, *v, *att, *x2, *act, *hh, *fn;     // [max_tokens] rows of activations
   uint16_t *kc, *vc;                                           // [max_roll, n_kv, hd]
   float* logits;                                               // [max_heads rows, vocab]
-  int last_cuda_error;
+  int last_cuda_error, sm_count;
 };
 
 namespace {
@@ -26,26 +26,30 @@ namespace {
 constexpr int kMaxHeadRows = 16;
 constexpr int kAttnSmem = 200 * 1024;            // d_attn holds a score per cache slot and the query: more than the 48 KB that need no asking
 
-template <int NT, int MT, int WARPS, int MODE>
-cudaError_t launch_linear_nt(const DLin& p, int t0, cudaStream_t st) {
-  int grid = 0;
-  for (int i = 0; i < (MODE == DL_STORE ? 3 : 1) && p.W[i]; i++) grid += (p.N[i] + 16 * MT - 1) / (16 * MT);
-  if (MODE == DL_STORE && p.x1) return launch_pdl(d_gemm<NT, MT, WARPS, MODE, MODE == DL_STORE>, dim3(grid), dim3(WARPS * 32), 0, st, p, t0);
-  return launch_pdl(d_gemm<NT, MT, WARPS, MODE, false>, dim3(grid), dim3(WARPS * 32), 0, st, p, t0);
+template <int NT, int MT, int MODE>
+cudaError_t launch_linear_nt(DLin p, int t0, int sms, cudaStream_t st) {
+  int blocks = 0;
+  for (int i = 0; i < (MODE == DL_STORE ? 3 : 1) && p.W[i]; i++) blocks += (p.N[i] + 16 * MT - 1) / (16 * MT);
+  // K splits while all CTAs are resident at once and every warp keeps two chunks
+  const int slots = sms * (NT == 1 ? 3 : 2), nch = (p.k0 + p.k1 + 31) / 32;
+  p.ks = 1;
+  while (p.ks < kDraftSplits && blocks * (p.ks + 1) <= slots && nch >= 2 * kDraftWarps * (p.ks + 1)) p.ks++;
+  const dim3 grid(blocks * p.ks), block(kDraftWarps * 32);
+  if (MODE == DL_STORE && p.x1) return launch_pdl_cluster(d_gemm<NT, MT, MODE, MODE == DL_STORE>, grid, block, 0, st, (unsigned)p.ks, p, t0);
+  return launch_pdl_cluster(d_gemm<NT, MT, MODE, false>, grid, block, 0, st, (unsigned)p.ks, p, t0);
 }
-// All T tokens, up to 32 per pass over the weights. Up to 8 tokens: 16 rows per CTA (the matrices of a layer then give every SM at least
-// one) and three CTAs per SM. More tokens: 32 rows per CTA (one matrix) or 16 of each of
-// two, so that a CTA reads about as many bytes of activations from L2 as of weights, and 16 warps to share a long K.
+// All T tokens, up to 32 per pass over the weights. Up to 8 tokens: 16 rows per CTA and three CTAs per SM. More tokens: 32 rows per CTA (one
+// matrix) or 16 of each of two, so that a CTA reads about as many bytes of activations from L2 as of weights, and two CTAs per SM.
 template <int MODE>
-cudaError_t launch_linear(const DLin& p, cudaStream_t st) {
+cudaError_t launch_linear(const DLin& p, int sms, cudaStream_t st) {
   if ((p.k0 + p.k1) % 8 || p.k0 % 8 || p.N[0] <= 0 || p.T <= 0) return cudaErrorInvalidValue;
   constexpr int MW = MODE == DL_SWIGLU ? 1 : 2;
   cudaError_t e = cudaSuccess;
   for (int t0 = 0; t0 < p.T && e == cudaSuccess; t0 += 32) {
     const int left = p.T - t0;
-    if (left <= 8) e = launch_linear_nt<1, 1, 8, MODE>(p, t0, st);
-    else if (left <= 16) e = launch_linear_nt<2, MW, 16, MODE>(p, t0, st);
-    else e = launch_linear_nt<4, MW, 16, MODE>(p, t0, st);
+    if (left <= 8) e = launch_linear_nt<1, 1, MODE>(p, t0, sms, st);
+    else if (left <= 16) e = launch_linear_nt<2, MW, MODE>(p, t0, sms, st);
+    else e = launch_linear_nt<4, MW, MODE>(p, t0, sms, st);
   }
   return e;
 }
@@ -131,6 +135,7 @@ int fb_draft_create(const fb_draft_desc* desc, int device, fb_draft** out) {
   const size_t T = d.max_tokens, D = d.dim, kvd = (size_t)d.n_kv_head * hd, F = (size_t)d.fuse * d.dim;
   cudaError_t e = cudaSuccess;
   auto A = [&](cudaError_t x) { if (e == cudaSuccess) e = x; };
+  A(cudaDeviceGetAttribute(&r->sm_count, cudaDevAttrMultiProcessorCount, device));
   A(cudaFuncSetAttribute(d_attn, cudaFuncAttributeMaxDynamicSharedMemorySize, kAttnSmem));
   A(dmalloc(&r->x, T * D * 2)); A(dmalloc(&r->h, T * D * 2)); A(dmalloc(&r->q, T * D * 2));
   A(dmalloc(&r->k, T * kvd * 2)); A(dmalloc(&r->v, T * kvd * 2)); A(dmalloc(&r->att, T * D * 2));
@@ -183,7 +188,7 @@ int fb_draft_forward(fb_draft* r, const void* d_feat, const void* d_emb, const i
   if (d_emb) { p.x1 = (const uint16_t*)d_emb; p.ldx1 = D; }
   else { p.x1 = (const uint16_t*)r->w.embed; p.ldx1 = D; p.x1_tokens = d_tokens; p.x1_rows = d.vocab; }
   p.k1 = D; p.N[0] = D; p.T = T; p.y[0] = r->x; p.ldy[0] = D; p.first = true;
-  FB_DCUDA(r, launch_linear<DL_STORE>(p, st));
+  FB_DCUDA(r, launch_linear<DL_STORE>(p, r->sm_count, st));
   FB_DCUDA(r, launch_pdl(d_rmsnorm, dim3(T), dim3(256), 0, st, (const uint16_t*)r->x, D, (const uint16_t*)r->w.n1, r->h, D, D, d.rms_eps, false));
   // q, k, v in one launch
   memset(&p, 0, sizeof(p));
@@ -192,7 +197,7 @@ int fb_draft_forward(fb_draft* r, const void* d_feat, const void* d_emb, const i
   const int qkvn[3] = {D, kvd, kvd};
   for (int i = 0; i < 3; i++) { p.W[i] = (const uint16_t*)qkvw[i]; p.N[i] = qkvn[i]; p.y[i] = qkvo[i]; p.ldy[i] = qkvn[i]; }
   p.x0 = r->h; p.ldx0 = D; p.k0 = D; p.T = T;
-  FB_DCUDA(r, launch_linear<DL_STORE>(p, st));
+  FB_DCUDA(r, launch_linear<DL_STORE>(p, r->sm_count, st));
   FB_DCUDA(r, launch_pdl(d_rope_store, dim3(T, d.n_head + d.n_kv_head), dim3(64), 0, st, r->q, (const uint16_t*)r->k, (const uint16_t*)r->v, d_positions,
                          d_slots, r->kc, r->vc, d.n_head, d.n_kv_head, hd, d.rope_base, d.max_roll));
   FB_DCUDA(r, launch_pdl(d_attn, dim3(T, d.n_head), dim3(128), (size_t)(d.max_roll + hd) * 4, st, (const uint16_t*)r->q, d_slots,
@@ -201,22 +206,22 @@ int fb_draft_forward(fb_draft* r, const void* d_feat, const void* d_emb, const i
   memset(&p, 0, sizeof(p));
   p.W[0] = (const uint16_t*)r->w.o; p.x0 = r->att; p.ldx0 = D; p.k0 = D; p.N[0] = D; p.T = T; p.y[0] = r->x2; p.ldy[0] = D;
   p.resid = r->x; p.ldr = D;
-  FB_DCUDA(r, launch_linear<DL_RESID>(p, st));
+  FB_DCUDA(r, launch_linear<DL_RESID>(p, r->sm_count, st));
   FB_DCUDA(r, launch_pdl(d_rmsnorm, dim3(T), dim3(256), 0, st, (const uint16_t*)r->x2, D, (const uint16_t*)r->w.n2, r->h, D, D, d.rms_eps, false));
   // act = silu(gate h) * up h
   memset(&p, 0, sizeof(p));
   p.W[0] = (const uint16_t*)r->w.gate; p.W2 = (const uint16_t*)r->w.up; p.x0 = r->h; p.ldx0 = D; p.k0 = D; p.N[0] = d.inter; p.T = T;
   p.y[0] = r->act; p.ldy[0] = d.inter;
-  FB_DCUDA(r, launch_linear<DL_SWIGLU>(p, st));
+  FB_DCUDA(r, launch_linear<DL_SWIGLU>(p, r->sm_count, st));
   // hh = x2 + down(act)
   memset(&p, 0, sizeof(p));
   p.W[0] = (const uint16_t*)r->w.down; p.x0 = r->act; p.ldx0 = d.inter; p.k0 = d.inter; p.N[0] = D; p.T = T; p.y[0] = r->hh; p.ldy[0] = D;
   p.resid = r->x2; p.ldr = D;
-  FB_DCUDA(r, launch_linear<DL_RESID>(p, st));
+  FB_DCUDA(r, launch_linear<DL_RESID>(p, r->sm_count, st));
   // out = fout(hh)
   memset(&p, 0, sizeof(p));
   p.W[0] = (const uint16_t*)r->w.fout; p.x0 = r->hh; p.ldx0 = D; p.k0 = D; p.N[0] = F; p.T = T; p.y[0] = (uint16_t*)d_out; p.ldy[0] = F;
-  FB_DCUDA(r, launch_linear<DL_STORE>(p, st));
+  FB_DCUDA(r, launch_linear<DL_STORE>(p, r->sm_count, st));
   FB_DCUDA(r, cudaGetLastError());
   return FB_OK;
 }
@@ -237,7 +242,7 @@ int fb_draft_head(fb_draft* r, const void* d_feat_rows, int32_t n, int32_t top_b
   memset(&p, 0, sizeof(p));
   p.W[0] = (const uint16_t*)r->w.embed; p.x0 = r->fn; p.ldx0 = D; p.k0 = D; p.N[0] = d.vocab; p.T = n; p.yf = r->logits; p.ldy[0] = d.vocab;
   p.scale = d.logits_scaling;
-  FB_DCUDA(r, launch_linear<DL_LOGITS>(p, st));
+  FB_DCUDA(r, launch_linear<DL_LOGITS>(p, r->sm_count, st));
   const int nc = row_ctas(d.vocab);
   const bool reg = (d.vocab + nc - 1) / nc <= kSampleRegs * 1024;
   FB_DCUDA(r, launch_pdl_cluster(reg ? topb_rows<true> : topb_rows<false>, dim3(nc, n), dim3(1024), 0, st, nc, (const float*)r->logits,

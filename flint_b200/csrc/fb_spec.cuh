@@ -335,6 +335,7 @@ struct DLin {
   int ldy[3], ldr;
   float scale;
   bool first;                   // the first kernel of a call
+  int ks;                       // CTAs of a cluster that share K
 };
 
 // y[t, n] = sum_k W[n, k] x[t, k] for up to 8 NT tokens (t0 ...) on the tensor pipe, weights read once. A CTA takes 16 MT rows of W and
@@ -343,13 +344,21 @@ struct DLin {
 // token g at the same columns -- so nothing goes through shared memory but the warps' partial sums. HBM-bound: a warp keeps AH chunks of
 // weights and activations in flight; the first weights are requested before the previous kernel is waited for (see pdl_begin). (The CUDA-core form
 // read the weights once per 8 or 16 tokens and took 62 us for a 13 to 50 MB matrix at 32 tokens.)
-template <int NT, int MT, int WARPS, int MODE, bool CAT>
-__global__ void __launch_bounds__(WARPS * 32, NT == 1 ? 3 : 1) d_gemm(const DLin P, int t0) {
+// A matrix whose rows give less than the GPU's worth of CTAs is also cut in K over a cluster of ks: the CTAs push their sums into the shared
+// memory of the one that finishes the token, which adds them in rank order. (With 16 warps and no split a 2560-row matrix ran on 80
+// SMs: window of 32 rows 177 -> 153 us, 48 rows of the 40-head shape 290 -> 258; single rows, three CTAs an SM, 123 both ways.)
+constexpr int kDraftSplits = 3;
+constexpr int kDraftWarps = 8;
+template <int NT, int MT, int MODE, bool CAT>
+__global__ void __launch_bounds__(kDraftWarps * 32, NT == 1 ? 3 : 2) d_gemm(const DLin P, int t0) {
+  constexpr int WARPS = kDraftWarps;
   constexpr int NW = MODE == DL_SWIGLU ? 2 : 1, AH = NT == 1 && NW == 1 ? 4 : 2, ROWS = 16 * MT * NW;      // weight matrices per row, chunks in flight
   __shared__ float red[8][ROWS][8 * NT + 1];
+  __shared__ float part[kDraftSplits][8 * NT][ROWS];             // split K: [source rank][token][row]
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
   const int K = P.k0 + P.k1, nch = (K + 31) >> 5;
-  int blk = blockIdx.x, which = 0;
+  const int ks = P.ks, rank = (int)blockIdx.x % ks;
+  int blk = (int)blockIdx.x / ks, which = 0;
   if (MODE == DL_STORE) {
 #pragma unroll
     for (int i = 0; i < 2; i++) {
@@ -359,15 +368,15 @@ __global__ void __launch_bounds__(WARPS * 32, NT == 1 ? 3 : 1) d_gemm(const DLin
     }
   }
   const int N = P.N[which], r0 = blk * 16 * MT;
-  const uint16_t* wr[NW][MT][2];
+  // rows of this lane as 32-bit offsets in units of 8 elements (both matrices of a SwiGLU pair have the same shape)
+  uint32_t wr[MT][2];
 #pragma unroll
   for (int m = 0; m < MT; m++)
 #pragma unroll
-    for (int h = 0; h < 2; h++) {
-      const size_t row = (size_t)min(r0 + m * 16 + h * 8 + g, N - 1) * K + 8 * t;
-      wr[0][m][h] = P.W[which] + row;
-      if (NW > 1) wr[NW - 1][m][h] = P.W2 + row;
-    }
+    for (int h = 0; h < 2; h++) wr[m][h] = (uint32_t)min(r0 + m * 16 + h * 8 + g, N - 1) * (uint32_t)(K >> 3) + t;
+  const uint4* wb[NW];
+  wb[0] = reinterpret_cast<const uint4*>(P.W[which]);
+  if (NW > 1) wb[NW - 1] = reinterpret_cast<const uint4*>(P.W2);
   uint4 wv[AH][NW][MT][2], xv[AH][NT];
   auto load_w = [&](int c, uint4 (&d)[NW][MT][2]) {
     const bool ok = c < nch && c * 32 + 8 * t < K;
@@ -376,33 +385,35 @@ __global__ void __launch_bounds__(WARPS * 32, NT == 1 ? 3 : 1) d_gemm(const DLin
 #pragma unroll
       for (int m = 0; m < MT; m++)
 #pragma unroll
-        for (int h = 0; h < 2; h++) d[i][m][h] = ok ? __ldcs(reinterpret_cast<const uint4*>(wr[i][m][h] + c * 32)) : make_uint4(0, 0, 0, 0);
+        for (int h = 0; h < 2; h++) d[i][m][h] = ok ? __ldcs(wb[i] + (wr[m][h] + c * 4)) : make_uint4(0, 0, 0, 0);
   };
+  if (ks > 1) sm_cluster_arrive();                   // remote stores wait for it below
+  const int c1 = rank * WARPS + warp, step = WARPS * ks;         // this warp's chunks
   pdl_begin(P.first && t0 == 0);
 #pragma unroll
-  for (int a = 0; a < AH; a++) load_w(warp + WARPS * a, wv[a]);
+  for (int a = 0; a < AH; a++) load_w(c1 + step * a, wv[a]);
   pdl_wait();
-  const uint16_t *xp0[NT], *xp1[CAT ? NT : 1];
+  int x1[CAT ? NT : 1];                              // second segment: row of each token, or -1
+  if (CAT) {
 #pragma unroll
-  for (int j = 0; j < NT; j++) {
-    const int tok = t0 + j * 8 + g;
-    const bool live = tok < P.T;
-    xp0[j] = live ? P.x0 + (size_t)tok * P.ldx0 + 8 * t : nullptr;
-    if (CAT) {
-      const int id = live ? (P.x1_tokens ? P.x1_tokens[tok] : tok) : -1;
-      xp1[j] = id >= 0 && (!P.x1_tokens || id < P.x1_rows) ? P.x1 + (size_t)id * P.ldx1 + 8 * t - P.k0 : nullptr;
+    for (int j = 0; j < NT; j++) {
+      const int tok = t0 + j * 8 + g, id = tok < P.T ? (P.x1_tokens ? P.x1_tokens[tok] : tok) : -1;
+      x1[j] = P.x1_tokens && id >= P.x1_rows ? -1 : id;
     }
   }
   auto load_x = [&](int c, uint4 (&d)[NT]) {
     const int col = c * 32 + 8 * t;
+    const bool second = CAT && col >= P.k0;
+    const uint16_t* base = second ? P.x1 + (col - P.k0) : P.x0 + col;
+    const int ld = second ? P.ldx1 : P.ldx0;
 #pragma unroll
     for (int j = 0; j < NT; j++) {
-      const uint16_t* xp = CAT && col >= P.k0 ? xp1[CAT ? j : 0] : xp0[j];
-      d[j] = xp && col < K ? *reinterpret_cast<const uint4*>(xp + c * 32) : make_uint4(0, 0, 0, 0);
+      const int tok = t0 + j * 8 + g, row = second ? x1[CAT ? j : 0] : (tok < P.T ? tok : -1);
+      d[j] = row >= 0 && col < K ? *reinterpret_cast<const uint4*>(base + (size_t)row * ld) : make_uint4(0, 0, 0, 0);
     }
   };
 #pragma unroll
-  for (int a = 0; a < AH; a++) load_x(warp + WARPS * a, xv[a]);
+  for (int a = 0; a < AH; a++) load_x(c1 + step * a, xv[a]);
   float acc[NW][MT][NT][4];
 #pragma unroll
   for (int i = 0; i < NW; i++)
@@ -410,10 +421,10 @@ __global__ void __launch_bounds__(WARPS * 32, NT == 1 ? 3 : 1) d_gemm(const DLin
     for (int m = 0; m < MT; m++)
 #pragma unroll
       for (int j = 0; j < NT; j++) acc[i][m][j][0] = acc[i][m][j][1] = acc[i][m][j][2] = acc[i][m][j][3] = 0.f;
-  for (int c0 = warp; c0 < nch; c0 += WARPS * AH) {
+  for (int c0 = c1; c0 < nch; c0 += step * AH) {
 #pragma unroll
     for (int a = 0; a < AH; a++) {                   // chunks past the end multiply zeros
-      const int c = c0 + WARPS * a;
+      const int c = c0 + step * a;
 #pragma unroll
       for (int i = 0; i < NW; i++)
 #pragma unroll
@@ -426,12 +437,12 @@ __global__ void __launch_bounds__(WARPS * 32, NT == 1 ? 3 : 1) d_gemm(const DLin
             mma_bf16(acc[i][m][j], a1, xv[a][j].z, xv[a][j].w);
           }
         }
-      load_w(c + WARPS * AH, wv[a]);
-      load_x(c + WARPS * AH, xv[a]);
+      load_w(c + step * AH, wv[a]);
+      load_x(c + step * AH, xv[a]);
     }
   }
   auto at = [&](int i, int m, int j, int e) -> float& {
-    return red[warp & 7][(i * MT + m) * 16 + g + 8 * (e >> 1)][j * 8 + 2 * t + (e & 1)];
+    return red[warp][(i * MT + m) * 16 + g + 8 * (e >> 1)][j * 8 + 2 * t + (e & 1)];
   };
   auto each_acc = [&](auto f) {
 #pragma unroll
@@ -443,22 +454,36 @@ __global__ void __launch_bounds__(WARPS * 32, NT == 1 ? 3 : 1) d_gemm(const DLin
 #pragma unroll
           for (int e = 0; e < 4; e++) f(i, m, j, e);
   };
-  if (WARPS > 8) {                                   // the upper eight warps' sums join the lower eight's
-    if (warp >= 8) each_acc([&](int i, int m, int j, int e) { at(i, m, j, e) = acc[i][m][j][e]; });
-    __syncthreads();
-    if (warp < 8) each_acc([&](int i, int m, int j, int e) { acc[i][m][j][e] += at(i, m, j, e); });
-    __syncthreads();
-  }
-  if (warp < 8) each_acc([&](int i, int m, int j, int e) { at(i, m, j, e) = acc[i][m][j][e]; });
+  each_acc([&](int i, int m, int j, int e) { at(i, m, j, e) = acc[i][m][j][e]; });
   __syncthreads();
-  for (int o = tid; o < 16 * MT * 8 * NT; o += WARPS * 32) {
-    const int r = o % (16 * MT), tk = o / (16 * MT), n = r0 + r, tok = t0 + tk;
-    if (n >= N || tok >= P.T) continue;
-    float s = 0.f, s2 = 0.f;
+  constexpr int NO = 16 * MT * 8 * NT;
+  if (ks > 1) {
+    sm_cluster_wait();
+    for (int o = tid; o < NO * NW; o += WARPS * 32) {
+      const int r = o % ROWS, tk = o / ROWS;
+      if (t0 + tk >= P.T) break;
+      float s = 0.f;
 #pragma unroll
-    for (int w = 0; w < 8; w++) {
-      s += red[w][r][tk];
-      if (NW > 1) s2 += red[w][16 * MT * (NW - 1) + r][tk];
+      for (int w = 0; w < 8; w++) s += red[w][r][tk];
+      sm_st(sm_map(smem_u32(&part[rank][tk][r]), tk % ks), __float_as_uint(s));
+    }
+    sm_cluster_sync();
+  }
+  for (int o = tid; o < NO; o += WARPS * 32) {
+    const int r = o % (16 * MT), tk = o / (16 * MT), n = r0 + r, tok = t0 + tk;
+    if (n >= N || tok >= P.T || (ks > 1 && tk % ks != rank)) continue;
+    float s = 0.f, s2 = 0.f;
+    if (ks > 1) {
+      for (int q = 0; q < ks; q++) {
+        s += part[q][tk][r];
+        if (NW > 1) s2 += part[q][tk][16 * MT * (NW - 1) + r];
+      }
+    } else {
+#pragma unroll
+      for (int w = 0; w < 8; w++) {
+        s += red[w][r][tk];
+        if (NW > 1) s2 += red[w][16 * MT * (NW - 1) + r][tk];
+      }
     }
     if (MODE == DL_LOGITS) {
       P.yf[(size_t)tok * P.ldy[0] + n] = rbf(rbf(s) / P.scale);

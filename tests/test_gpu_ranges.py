@@ -341,6 +341,24 @@ def test_draft_row_tile_edges(T):
     assert np.all(np.take_along_axis(lg, t_dev.cpu().numpy().astype(np.int64), 1) >= top[:, 2:] - 2.0 ** -6 * np.abs(lg).max())
 
 
+@pytest.mark.parametrize("T", [1, 8, 16, 33])
+@pytest.mark.parametrize("inter", [1024, 1544, 2048])
+def test_draft_linears_with_split_k(T, inter):
+    """Linears whose K goes over a cluster: the merge (K = 1024) over two CTAs, the down projection over two or three, one of them with a K that
+    is no multiple of a chunk."""
+    dim, nh, nkv, vocab = 256, 8, 2, 1000
+    m = seeded_draft(dim, nh, inter, seed=5, rope_base=10000.0, n_kv=nkv, fuse=3)
+    g = torch.Generator().manual_seed(T)
+    m.bind_target((torch.randn(vocab, dim, generator=g) * 0.5).bfloat16().cuda(), torch.ones(dim, dtype=torch.bfloat16).cuda(), 1.0)
+    m.setup_cache(48)
+    orc = DraftOracle({k: _f32(v) for k, v in m._w.items()}, nh, 10000.0, max_roll=48, n_kv=nkv)
+    feat, emb = (torch.randn(T, n * dim, generator=g).bfloat16().cuda() for n in (3, 1))
+    pos = torch.arange(T, dtype=torch.int32)
+    out = m(feat, emb, pos.cuda(), input_pos=pos.cuda())
+    ref = orc.forward(_f32(feat), _f32(emb), pos.numpy(), slots=np.arange(T))
+    assert np.abs(_f32(out) - ref).max() <= 2e-2 * np.abs(ref).max()         # as above
+
+
 @pytest.mark.parametrize("T", [1, 12, 40])
 def test_draft_token_ids_outside_the_table_are_zero_rows(T):
     """Ids at and past the vocabulary, like negative ones, read no table row: the bits of a call whose embeddings are zeros there."""
