@@ -122,7 +122,8 @@ cudaError_t launch_vattn_tc(const fb_ctx* c, const uint16_t* kc, const uint16_t*
                             cudaStream_t st) {
   const fb_model_desc& d = c->d;
   const int T = pos + M, tiles = (M * c->rgqa + 15) / 16, per4 = c->sm_count / (4 * d.n_kv_head);
-  VattnParams a{c->vq, kc, vc, amask, c->vao, want_max ? c->vamax : nullptr, d.n_head, d.n_kv_head, pos, M, 0, d.attn_scale * 1.4426950408889634f};
+  VattnParams a{c->vq, kc, vc, amask, c->vao, want_max ? c->vamax : nullptr, d.n_head, d.n_kv_head, pos, M, 0, d.attn_scale * 1.4426950408889634f,
+               c->status, c->spin_limit};
   const int rt = tiles <= per4 ? 1 : (tiles <= 2 * per4 ? 2 : 4), mg = (tiles + rt - 1) / rt, groups = d.n_kv_head * mg;
   const int stages = (T + 63) / 64;
   int nspan = 1;

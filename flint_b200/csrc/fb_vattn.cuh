@@ -3,9 +3,11 @@
 // A CTA of eight warps takes, for one kv head, RT row tiles of 16 query rows (row = token * R + head of the group: the R query
 // heads share every K/V row) and one span of positions; its warps are RT tiles x PG = 8 / RT position groups, a group taking every
 // PG-th unit of UP positions. K/V stages come by cp.async. Spans are the CTAs of a CLUSTER: all warps leave their un-normalised
-// partials (acc, running max, denominator) in shared memory and every CTA finishes a share of the rows from its neighbours' shared
-// memory, so there is no merge kernel and no trip of the partials through L2. That pair of kernels took 12.3 + 8.3 us for 26 tokens
-// over 1024 positions (3B shape), mostly latency: one 64-position chunk per CTA, then 4.6 MB of partials written and read back.
+// partials (acc, running max, denominator) in shared memory, the CTA's position groups are merged, and every row's result goes to the CTA of
+// the cluster that finishes it, so there is no merge kernel and no trip of the partials through L2. That pair of kernels took 12.3 + 8.3 us
+// for 26 tokens over 1024 positions (3B shape), mostly latency: one 64-position chunk per CTA, then 4.6 MB of partials written and read
+// back. The partials are pushed: read from the neighbours' memory between two cluster barriers, passes of 4 / 14 / 26 tokens (3B) and 5 / 26 / 61
+// (8B) took 1587 / 1741 / 2020 and 2078 / 2354 / 3370 us, so 1537 / 1727 / 2029 and 2053 / 2339 / 3342.
 // Bound by latency for trees; by instruction issue for prompts (softmax around 16 x 8 MMAs), hence ldmatrix for both operands, packed
 // conversions, base-2 exponentials, and masks only in the units that need one.
 #pragma once
@@ -24,7 +26,9 @@ struct VaCfg {
   static constexpr int PW = HD + 4;                     // floats per partial row: acc[HD], max, denominator
   static constexpr int PART = 8 * 16 * PW * 4;          // partials (over the dead stages)
   static constexpr int RING = NSTG * STAGE > PART ? NSTG * STAGE : PART;
-  static constexpr int TOTAL = RING;
+  static constexpr int INBOX = RING;                    // the spans' partials of this CTA's rows: [span][row][PW]
+  static constexpr int BAR = INBOX + 16 * RT * PW * 4;
+  static constexpr int TOTAL = BAR + 16;
   static_assert(SP / UP == PG || RT == 4, "one unit per warp and stage");
 };
 
@@ -33,15 +37,14 @@ __device__ __forceinline__ uint32_t cluster_map(uint32_t saddr, uint32_t rank) {
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(saddr), "r"(rank));
   return r;
 }
-__device__ __forceinline__ float2 ld_cluster_f2(uint32_t a) {
-  float2 v;
-  asm volatile("ld.shared::cluster.v2.f32 {%0,%1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(a) : "memory");
-  return v;
+// 16 bytes into a CTA of the cluster, counted on that CTA's barrier
+__device__ __forceinline__ void st_async_v4(uint32_t addr, float4 v, uint32_t bar) {
+  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1,%2,%3,%4}, [%5];"
+               ::"r"(addr), "r"(__float_as_uint(v.x)), "r"(__float_as_uint(v.y)), "r"(__float_as_uint(v.z)), "r"(__float_as_uint(v.w)), "r"(bar)
+               : "memory");
 }
-__device__ __forceinline__ float4 ld_cluster_f4(uint32_t a) {
-  float4 v;
-  asm volatile("ld.shared::cluster.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a) : "memory");
-  return v;
+__device__ __forceinline__ void st_cluster_v4(uint32_t addr, float4 v) {
+  asm volatile("st.shared::cluster.v4.f32 [%0], {%1,%2,%3,%4};" ::"r"(addr), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
 }
 __device__ __forceinline__ void cp_async16_zfill(void* dst, const void* src, bool valid) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(valid ? 16 : 0) : "memory");
@@ -75,6 +78,8 @@ struct VattnParams {
   unsigned* amax;          // [M] largest |output| of each token as float bits (cleared by the token's norm), or nullptr
   int n_head, nkv, pos, M, span;
   float scale;             // times log2(e)
+  DevStatus* status;
+  unsigned spin_limit;
 };
 
 // grid (spans = CTAs of a cluster, kv heads, row groups of RT tiles), 256 threads
@@ -94,18 +99,19 @@ __global__ void __launch_bounds__(256) v_attn(const VattnParams P) {
   const int t_begin = rank * P.span, t_end = min(P.amask ? T : P.pos + m_last + 1, t_begin + P.span);
   const int nst = t_end > t_begin ? (t_end - t_begin + SP - 1) / SP : 0;
   pdl_trigger();
-  // the span's old rows do not depend on the previous kernel: bring them into L2 while it runs
-  if (nspan > 1) {
-    constexpr int PER = (HD * 2 + 127) / 128 + 1;
-    const int old_end = min(t_end, P.pos), n = max(0, old_end - t_begin) * 2 * PER;
-    for (int i = tid; i < n; i += 256) {
-      const int tp = t_begin + i / (2 * PER), k = i % (2 * PER);
-      const uint16_t* base = (k < PER ? P.kc : P.vc) + ((size_t)tp * P.nkv + kvh) * HD;
-      const int off = min((k % PER) * 128, HD * 2 - 2);
-      asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const char*>(base) + off));
+  uint64_t* xbar = reinterpret_cast<uint64_t*>(va_sm + S::BAR);                        // spans: all partials of this CTA's rows have arrived
+  volatile int* s_abort = reinterpret_cast<volatile int*>(xbar + 1);
+  constexpr bool ASYNC = RT == 1;                                // how the partials are known to have arrived, see below
+  const bool alone = nspan == 1;
+  if (!alone) {
+    if (ASYNC && tid == 0) {
+      *s_abort = 0;
+      mbar_init(xbar, 1);
+      mbar_fence_init();
+      mbar_expect_tx(xbar, 16 * RT * (HD + 4) * 4);
     }
+    asm volatile("barrier.cluster.arrive.release;" ::: "memory");                      // partials are sent once every neighbour is known to run
   }
-  pdl_wait();
   auto issue = [&](int s) {
     if (s < nst) {
       uint8_t* k_s = va_sm + (s % NSTG) * S::STAGE;
@@ -121,7 +127,27 @@ __global__ void __launch_bounds__(256) v_attn(const VattnParams P) {
     }
     cp_async_commit();
   };
-  for (int s = 0; s < NSTG - 1; s++) issue(s);
+  // Rows below `pos` do not depend on the previous kernel: the first stages that hold no others are requested while it runs, and the rest of
+  // the span is brought into L2 (with all of it only brought into L2, 26 / 61 tokens over 1024 positions took 2049 / 2640 us a pass, so
+  // 2020 / 2617).
+  for (int s = 0, waited = 0;; s++) {
+    if (!waited && (s == NSTG - 1 || min(t_end, t_begin + (s + 1) * SP) > P.pos)) {
+      if (nspan > 1) {
+        constexpr int PER = (HD * 2 + 127) / 128 + 1;
+        const int p0 = t_begin + s * SP, n = max(0, min(t_end, P.pos) - p0) * 2 * PER;
+        for (int i = tid; i < n; i += 256) {
+          const int tp = p0 + i / (2 * PER), k = i % (2 * PER);
+          const uint16_t* base = (k < PER ? P.kc : P.vc) + ((size_t)tp * P.nkv + kvh) * HD;
+          const int off = min((k % PER) * 128, HD * 2 - 2);
+          asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const char*>(base) + off));
+        }
+      }
+      pdl_wait();
+      waited = 1;
+    }
+    if (s == NSTG - 1) break;
+    issue(s);
+  }
   const bool live = tile < ntile;
   const int r_lo = min(tile * 16 + g, rows - 1), r_hi = min(tile * 16 + g + 8, rows - 1);
   const int m_lo = r_lo / R, m_hi = r_hi / R;
@@ -248,7 +274,8 @@ __global__ void __launch_bounds__(256) v_attn(const VattnParams P) {
     }
   }
   __syncthreads();
-  const bool alone = nspan == 1;
+  const int nown = RT * 16 / nspan;                              // this CTA finishes local rows rank, rank + nspan, ...
+  if (!alone) asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
   // the position groups of the CTA meet first: a warp merges 2 RT rows (in place of position group 0's partials), so that the cluster
   // exchanges one partial per row and span
   auto finish = [&](int lr, float4 acc, float den) {             // local row lr, lane = 4 dims: normalise and write
@@ -288,21 +315,32 @@ __global__ void __launch_bounds__(256) v_attn(const VattnParams P) {
     }
     if (alone) {
       finish(lr, acc, den);
-    } else {
-      __syncwarp();
-      if (lane < HD / 4) *reinterpret_cast<float4*>(p0 + lane * 4) = acc;
-      if (lane == 0) *reinterpret_cast<float2*>(p0 + HD) = make_float2(gm, den);
+    } else {                                                     // to the CTA that finishes the row
+      const uint32_t to = lr & (nspan - 1), a = cluster_map(smem_u32(va_sm + S::INBOX) + (uint32_t)((rank * nown + lr / nspan) * PW) * 4, to),
+                     xb = cluster_map(smem_u32(xbar), to);
+      const float4 md = make_float4(gm, den, 0.f, 0.f);
+      if (ASYNC) {
+        if (lane < HD / 4) st_async_v4(a + lane * 16, acc, xb);
+        if (lane == 0) st_async_v4(a + HD * 4, md, xb);
+      } else {
+        if (lane < HD / 4) st_cluster_v4(a + lane * 16, acc);
+        if (lane == 0) st_cluster_v4(a + HD * 4, md);
+      }
     }
   }
   if (!alone) {
-    asm volatile("barrier.cluster.arrive.release;" ::: "memory");
-    asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
-    // this CTA finishes local rows rank, rank + nspan, ...: all spans' partials of a row are requested together
-    const int nown = RT * 16 / nspan;
-    const uint32_t base = smem_u32(va_sm);
-    for (int ri = warp; ri < nown; ri += 8) {
-      const int lr = rank + ri * nspan;
-      const uint32_t a = base + (uint32_t)(((lr >> 4) * 16 + (lr & 15)) * PW) * 4;
+    // One row tile a CTA: asynchronous stores that count on the receiver's barrier, which leaves its neighbours' pace out of it. More: plain
+    // stores and a cluster barrier (26 tokens of the 3B shape 2038 asynchronous, 2029 plain).
+    bool ok = true;
+    if (ASYNC) {
+      const WaitCtl wc{P.status, s_abort, P.spin_limit};
+      ok = __all_sync(0xffffffffu, mbar_wait(xbar, 0, wc, W_FULL, 12));
+    } else {
+      asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+      asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+    }
+    const float* in = reinterpret_cast<const float*>(va_sm + S::INBOX);
+    for (int ri = warp; ok && ri < nown; ri += 8) {
       float2 ml[8];
       float4 v[8];
 #pragma unroll
@@ -310,9 +348,9 @@ __global__ void __launch_bounds__(256) v_attn(const VattnParams P) {
         ml[k] = make_float2(-1e30f, 0.f);
         v[k] = make_float4(0.f, 0.f, 0.f, 0.f);
         if (k < nspan) {
-          const uint32_t ra = cluster_map(a, k);
-          ml[k] = ld_cluster_f2(ra + HD * 4);
-          if (lane < HD / 4) v[k] = ld_cluster_f4(ra + lane * 16);
+          const float* a = in + (k * nown + ri) * PW;
+          ml[k] = *reinterpret_cast<const float2*>(a + HD);
+          if (lane < HD / 4) v[k] = *reinterpret_cast<const float4*>(a + lane * 4);
         }
       }
       float gm = ml[0].x, den = 0.f;
@@ -325,10 +363,18 @@ __global__ void __launch_bounds__(256) v_attn(const VattnParams P) {
         den = fmaf(ml[k].y, e, den);
         acc.x = fmaf(v[k].x, e, acc.x); acc.y = fmaf(v[k].y, e, acc.y); acc.z = fmaf(v[k].z, e, acc.z); acc.w = fmaf(v[k].w, e, acc.w);
       }
-      finish(lr, acc, den);
+      finish(rank + ri * nspan, acc, den);
     }
-    asm volatile("barrier.cluster.arrive.release;" ::: "memory");
-    asm volatile("barrier.cluster.wait.acquire;" ::: "memory");  // nobody leaves while a neighbour reads its shared memory
+    // Nobody leaves before its neighbours have sent what they will send; after a failure (somebody gave up before it sent), not before what is
+    // under way has landed, which takes microseconds.
+    if (ASYNC) {
+      __syncwarp();
+      asm volatile("barrier.cluster.arrive.relaxed;" ::: "memory");
+      asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+      if (!ok && tid == 0)
+#pragma unroll 1
+        for (int i = 0; i < 200 && !mbar_test(xbar, 0); i++) __nanosleep(1000);
+    }
   }
 }
 
