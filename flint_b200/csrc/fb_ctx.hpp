@@ -31,7 +31,7 @@ struct fb_ctx {
   uint64_t* peer_inbox[8];
   bool peers_open[8];
   uint16_t *vh, *vxn, *vq, *vao, *vact;                             // verify / prompt activations, kPromptRows token rows each
-  CUtensorMap m_xn[4], m_ao[4], m_act[4];                           // vxn, vao, vact as tensors: boxes of 16, 32, 64, 128 token rows
+  CUtensorMap m_xn[5], m_ao[5], m_act[5];                           // vxn, vao, vact as tensors: boxes of 16, 32, 64, 128, 192 token rows
   uint8_t *t_qkv, *t_o, *t_gu, *t_d, *t_lm;                          // verify: the matrices in the tensor-core (TC) layout
   float *vfx, *vfao, *vfa, *vfa_inv;                                // per token: inverse powers of two of xn / attention output, that of the SwiGLU output and its inverse
   unsigned* vamax;                                                  // per token: bound on the attention output (float bits)

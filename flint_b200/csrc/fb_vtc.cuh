@@ -1,5 +1,5 @@
 // int4 GEMM of the M-token passes on the 5th-generation tensor cores (tcgen05): a weight row is read once and multiplied with a tile of
-// up to NT tokens. This file: the layout, the arithmetic, the epilogues, and the kernel for prompts (tiles of up to 128 tokens);
+// up to NT tokens. This file: the layout, the arithmetic, the epilogues, and the kernel for prompts (tiles of up to 128 or 192 tokens);
 // fb_vtl.cuh: the kernel for trees (one tile of 16 / 32 / 64).
 //
 // D[128 weight rows][NT tokens] (fp32, in TENSOR MEMORY) += A[128][128] * B[NT][128]^T per group of 128 columns, issued as
@@ -38,8 +38,8 @@ namespace fb {
 
 constexpr int kTcThreads = 640;   // warps: 0 weights, 1 MMA issue, 2 activations, 4..11 dequantise, 12..19 epilogue
 constexpr int kTcRowBlock = 128;
-constexpr int kTcTokens = 128;    // most tokens of a prompt's tile
-constexpr int kTcEpiBytes = 2 * 64 * 4 + 16 * 64;
+constexpr int kTcTable = 96;      // tokens of an epilogue warp, at most
+constexpr int kTcEpiBytes = 2 * kTcTable * 4 + 16 * 64;
 constexpr int kTcTrailer = kTcRowBlock * 4 + 16;      // a block's row factors, then its flag
 
 __host__ __device__ constexpr int tc_rec_bytes(int has_zeros) { return 8192 + 256 * (has_zeros ? 2 : 1); }
@@ -351,11 +351,14 @@ __device__ __forceinline__ void st_async(uint32_t addr, uint32_t v, uint32_t bar
 }
 
 // Shared-memory plan (bytes). The raw ring keeps HBM busy; a stage of activations is a group's two 64-column tiles.
-template <bool HZ>
+// Tiles of 128 tokens, or of 192: an item's groups then take 4/3 of the time for 3/2 of the tokens, because dequantising a group and storing
+// it to tensor memory (which keeps the MMAs out meanwhile) is a cost per item. What is left of tensor memory allows two A stages, and none
+// for zero points.
+template <bool HZ, int NT_>
 struct VtcSmem {
-  static constexpr int NT = kTcTokens, REC = tc_rec_bytes(HZ);
-  static constexpr int NS = HZ ? 3 : 4;                            // A stages (64 columns): what two accumulators leave
-  static constexpr int NB = 5, NRAW = 6;                           // activation stages, raw int4 groups
+  static constexpr int NT = NT_, REC = tc_rec_bytes(HZ);
+  static constexpr int NS = NT == 192 ? 2 : (HZ ? 3 : 4);          // A stages (64 columns): what two accumulators leave
+  static constexpr int NB = NT == 192 ? 3 : 5, NRAW = 6;           // activation stages, raw int4 groups
   static constexpr int BSTAGE = NT * 256;                          // two [NT rows x 128 bytes] swizzled tiles
   static constexpr int B = 0;
   static constexpr int RAW = B + NB * BSTAGE;
@@ -417,13 +420,13 @@ struct TcOperands {
     }
   }
 };
-// The token factors of a warp's (up to 64) tokens, spread over its lanes: one load per item instead of an L2 round trip per chunk
-template <int EPI>
+// The token factors of a warp's (up to 32 NF) tokens, spread over its lanes: one load per item instead of an L2 round trip per chunk
+template <int EPI, int NF = 2>
 struct TcFactors {
-  float fx[2], fa[2];
+  float fx[NF], fa[NF];
   __device__ __forceinline__ void fetch(const VtcParams& P, int t0, int tend, int lane) {
 #pragma unroll
-    for (int k = 0; k < 2; k++) {
+    for (int k = 0; k < NF; k++) {
       const int t = t0 + 32 * k + lane;
       fx[k] = t >= tend ? 0.f : (EPI == EPI_RESID && P.amax) ? pow2_for(__uint_as_float(__ldcg(P.amax + t))).y : __ldcg(P.fx + t);
       if (EPI == EPI_SWIGLU) fa[k] = t < tend ? __ldcg(P.fa + t) : 0.f;
@@ -435,10 +438,10 @@ struct TcFactors {
 // The same from a table that the warp keeps in shared memory (prompts: 64 tokens an item; a shuffle per token and factor costs more)
 struct TcFactorTable {
   float *fx, *fa;
-  template <int EPI>
-  __device__ __forceinline__ void put(const TcFactors<EPI>& f, int lane) {
+  template <int EPI, int NF>
+  __device__ __forceinline__ void put(const TcFactors<EPI, NF>& f, int lane) {
 #pragma unroll
-    for (int k = 0; k < 2; k++) {
+    for (int k = 0; k < NF; k++) {
       fx[32 * k + lane] = f.fx[k];
       if (EPI == EPI_SWIGLU) fa[32 * k + lane] = f.fa[k];
     }
@@ -574,9 +577,9 @@ inline __device__ __noinline__ void tc_drain(uint64_t* bars, volatile int* s_iss
   __syncwarp();
 }
 
-template <int EPI, bool HZ>
+template <int EPI, bool HZ, int NT_>
 __global__ void __launch_bounds__(kTcThreads, 1) v_gemm_tc(const __grid_constant__ VtcParams P) {
-  using S = VtcSmem<HZ>;
+  using S = VtcSmem<HZ, NT_>;
   constexpr int NT = S::NT, NRAW = S::NRAW, NS = S::NS, NB = S::NB, ND = S::ND, REC = S::REC, HC = NT / 2;
   extern __shared__ __align__(1024) uint8_t tsm_raw[];
   // the swizzle pattern is a function of the absolute shared-memory address: tiles must start on 1024-byte boundaries
@@ -741,7 +744,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) v_gemm_tc(const __grid_constant
     constexpr int CH = STAGED || EPI == EPI_LOGITS ? 16 : 8;
     const uint32_t tlane = tmem + ((uint32_t)(quad * 32) << 16) + half * HC;
     uint8_t* area = tsm + S::EPI + (warp - 12) * kTcEpiBytes;
-    TcFactorTable fac{reinterpret_cast<float*>(area), reinterpret_cast<float*>(area) + 64};
+    TcFactorTable fac{reinterpret_cast<float*>(area), reinterpret_cast<float*>(area) + kTcTable};
     TcOperands<EPI, CH> pre;
     TcStaged<EPI> staged;
     Ring<2> ra;
@@ -754,9 +757,9 @@ __global__ void __launch_bounds__(kTcThreads, 1) v_gemm_tc(const __grid_constant
       if constexpr (STAGED) staged.fetch(P, srow - lane, th0, the, lane);
       else pre.fetch(P, srow, th0, the);
       __syncwarp();
-      TcFactors<EPI> mine;
+      TcFactors<EPI, HC / 32> mine;
       mine.fetch(P, th0, the, lane);
-      fac.put<EPI>(mine, lane);
+      fac.put<EPI, HC / 32>(mine, lane);
       ok = __all_sync(0xffffffffu, mbar_wait(&acc_full[ra.i], ra.lap, wc, W_FULL, 10));
       if (!ok) break;
       tc_fence_after();
@@ -774,7 +777,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) v_gemm_tc(const __grid_constant
 #pragma unroll
         for (int e = 0; e < CH; e++) v[e] = __uint_as_float(u[e >> 3][e & 7]);
         if constexpr (STAGED) {
-          staged.run(P, area + 512, srow - lane, t0, the, v, rf, fac, t0 - th0, lane);
+          staged.run(P, area + 2 * kTcTable * 4, srow - lane, t0, the, v, rf, fac, t0 - th0, lane);
           staged = snxt;
         } else {
           vtc_epilogue<EPI, CH>(P, srow, t0, the, v, rf, fac, t0 - th0, pre, lane);

@@ -340,10 +340,10 @@ __global__ void __launch_bounds__(kTlThreads, NT == 128 ? 1 : 2) v_gemm_tl(const
       }
       if constexpr (STAGED) {
         uint8_t* area = tsm + S::B + (warp - 6) * kTcEpiBytes;
-        TcFactorTable tab{reinterpret_cast<float*>(area), reinterpret_cast<float*>(area) + 64};
-        if (t0 == 0) tab.put<EPI>(fac, lane);
+        TcFactorTable tab{reinterpret_cast<float*>(area), reinterpret_cast<float*>(area) + kTcTable};
+        if (t0 == 0) tab.put<EPI, 2>(fac, lane);
         else staged.fetch(P, srow - lane, th0 + t0, tlast, lane);
-        staged.run(P, area + 512, srow - lane, th0 + t0, tlast, v, rf, tab, t0, lane);
+        staged.run(P, area + 2 * kTcTable * 4, srow - lane, th0 + t0, tlast, v, rf, tab, t0, lane);
       } else {
         vtc_epilogue<EPI, CH>(P, srow, th0 + t0, tlast, v, rf, fac, t0, pre, lane);
       }

@@ -219,6 +219,23 @@ def test_prompt_tiles_with_split_k(M, asym):
     eng.close()
 
 
+@pytest.mark.parametrize("M", [161, 192, 193, 385, 900])
+def test_prompt_tiles_of_192_tokens(M):
+    """Prompts whose gate/up (and at 900 tokens QKV) items take fewer rounds as 192-token tiles: one full tile, the first token of a second and
+    a third, tiles cut evenly. Logits of the last rows and every cache row against the oracle."""
+    cfg = ModelArgs.from_name("llama-1b-class")
+    cfg.n_layer, cfg.vocab_size = 1, 512
+    orc, eng = _pair(cfg, M + 8, 3)
+    toks = torch.randint(0, cfg.vocab_size, (M,), generator=torch.Generator().manual_seed(M)).tolist()
+    ref = np.concatenate([orc.verify(toks[i:i + 64], 3 + i)[0] for i in range(0, M, 64)])
+    lg, _ = eng.prefill(toks, 3)
+    eng.check()
+    assert np.abs(lg.cpu().numpy() - ref).max() < _tol(ref)
+    for dev, host in ((eng.kc, orc.kc), (eng.vc, orc.vc)):
+        assert np.abs(_f32(dev[:, 3:3 + M]) - O.bf16_to_f32(host[:, 3:3 + M])).max() < 0.05
+    eng.close()
+
+
 @pytest.mark.parametrize("vocab", [1, 31, 4096, 8200, 32768, 49160, 128256, 300001])
 def test_token_choice_over_every_split_of_a_row(vocab):
     """Rows on one, two, four and eight CTAs, slices that fit the registers and slices that do not, ragged ends: the arg-max
