@@ -346,7 +346,7 @@ struct DLin {
 // read the weights once per 8 or 16 tokens and took 62 us for a 13 to 50 MB matrix at 32 tokens.)
 // A matrix whose rows give less than the GPU's worth of CTAs is also cut in K over a cluster of ks: the CTAs push their sums into the shared
 // memory of the one that finishes the token, which adds them in rank order. (With 16 warps and no split a 2560-row matrix ran on 80
-// SMs: window of 32 rows 177 -> 153 us, 48 rows of the 40-head shape 290 -> 258; single rows, three CTAs an SM, 123 both ways.)
+// SMs: window of 32 rows 177 -> 153 us, 48 rows of the 40-head shape 290 -> 258; single rows, three CTAs an SM, 125.1 without the split, 122.3.)
 constexpr int kDraftSplits = 3;
 constexpr int kDraftWarps = 8;
 template <int NT, int MT, int MODE, bool CAT>

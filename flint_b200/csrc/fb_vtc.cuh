@@ -452,6 +452,7 @@ struct TcFactorTable {
 };
 // silu(g) = g / (1 + e^-g). The division by approximate reciprocal (2 ulp) sits behind an exponential of the same accuracy and ahead of a
 // rounding to bf16; the exact one brings a branch per value, which keeps an epilogue's independent values from overlapping.
+// (Where 1 + e^-g is above 2^126 it returns 0; the quotient is then below 2^-119.)
 __device__ __forceinline__ float tc_silu(float g) { return __fdividef(g, 1.0f + __expf(-g)); }
 // v[e] = accumulator of (stream row srow, token t0 + e), the i0 + e-th of the warp's tokens; rf = the row's factor. The whole warp
 // calls this together: lanes 2i, 2i + 1 hold the two rows of a RoPE or gate/up pair.

@@ -1,14 +1,16 @@
 // The GEMM of fb_vtc.cuh with one work item per CTA and K split over a cluster: trees, and short prompts, whose tiles alone would leave most
 // SMs without work.
-// One tile of up to 64 tokens (tree verification) is sized so that TWO CTAs share an SM: at most 113 KB of shared memory, 256 tensor-memory columns and 72 registers a thread. A verify pass is a chain of short dependent launches (4 to 6 us
-// of work each); with programmatic dependent launch the next GEMM's CTAs become resident while the previous kernel still runs, so
-// barrier set-up, the tensor-memory allocation, the weight ring and the first dequantised stages are done before the activations
-// exist. The 200 KB form left every launch to ramp up after its predecessor had gone: QKV / O / gate-up / down took
-// 9.7 / 9.4 / 11.1 / 12.1 us at 26 tokens of the 3B shape. The 128-token tiles of a prompt take a whole SM; what their long K needs is the
-// split (64 groups of the down projection in a row are 22 us).
 //
-// One work item (row block of a token tile) per CTA, K split over a cluster of up to eight CTAs (four at 128 tokens). Warps: 0 weight producer, 1 MMA issue, 2..4
-// activations (tensor copies, or the fp16 conversion of the attention output), 5 code warm-up, 6..13 dequantise, then epilogue.
+// One tile of up to 64 tokens (tree verification) is sized so that TWO CTAs share an SM: at most 113 KB of shared memory, 256 tensor-memory
+// columns and 72 registers a thread. A verify pass is a chain of short dependent launches (4 to 6 us of work each); with programmatic
+// dependent launch the next GEMM's CTAs become resident while the previous kernel still runs, so barrier set-up, the tensor-memory
+// allocation, the weight ring and the first dequantised stages are done before the activations exist. The 200 KB form left every launch to
+// ramp up after its predecessor had gone: QKV / O / gate-up / down took 9.7 / 9.4 / 11.1 / 12.1 us at 26 tokens of the 3B shape. The 128-token
+// tiles of a prompt take a whole SM; what their long K needs is the split (64 groups of the down projection in a row are 22 us).
+//
+// One work item (row block of a token tile) per CTA, K split over a cluster of up to eight CTAs (four at 128 tokens). Warps: 0 weight
+// producer, 1 MMA issue, 2..4 activations (tensor copies, or the fp16 conversion of the attention output), 5 code warm-up (trees), 6..13
+// dequantise, then epilogue.
 #pragma once
 #include "fb_vtc.cuh"
 
