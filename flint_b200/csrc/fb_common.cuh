@@ -84,19 +84,11 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* b) {
 __device__ __forceinline__ void mbar_expect_tx(uint64_t* b, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(b)), "r"(bytes) : "memory");
 }
-// REMOTE: the phase is completed by stores of other CTAs of the cluster (st.async), whose data the waiter reads: acquire at cluster scope
-// (the default is the CTA's own).
-template <bool REMOTE = false>
 __device__ __forceinline__ bool mbar_try(uint64_t* b, uint32_t parity) {
   uint32_t ok;
-  if (REMOTE)
-    asm volatile(
-        "{ .reg .pred p; mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
-        : "=r"(ok) : "r"(smem_u32(b)), "r"(parity) : "memory");
-  else
-    asm volatile(
-        "{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
-        : "=r"(ok) : "r"(smem_u32(b)), "r"(parity) : "memory");
+  asm volatile(
+      "{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
+      : "=r"(ok) : "r"(smem_u32(b)), "r"(parity) : "memory");
   return ok != 0;
 }
 __device__ __forceinline__ bool mbar_test(uint64_t* b, uint32_t parity) {
@@ -110,33 +102,6 @@ __device__ __forceinline__ bool mbar_test(uint64_t* b, uint32_t parity) {
 __device__ __forceinline__ void bulk_g2s(void* dst_smem, const void* src_gmem, uint32_t bytes, uint64_t* bar) {
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                ::"r"(smem_u32(dst_smem)), "l"(src_gmem), "r"(bytes), "r"(smem_u32(bar)) : "memory");
-}
-
-// ------------------------------------------------------------------------------------------------ clusters
-// Barrier over all threads of all CTAs of a cluster (release / acquire unless said otherwise), and a neighbour's shared memory: the address of the
-// same place there, stores, and stores that count as bytes on a barrier of that CTA.
-__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
-__device__ __forceinline__ void cluster_arrive_relaxed() { asm volatile("barrier.cluster.arrive.relaxed;" ::: "memory"); }
-__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
-__device__ __forceinline__ void cluster_sync() { cluster_arrive(); cluster_wait(); }
-__device__ __forceinline__ uint32_t cluster_map(uint32_t saddr, uint32_t rank) {
-  uint32_t r;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(saddr), "r"(rank));
-  return r;
-}
-__device__ __forceinline__ void st_cluster(uint32_t addr, uint32_t v) {
-  asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
-}
-__device__ __forceinline__ void st_cluster(uint32_t addr, float4 v) {
-  asm volatile("st.shared::cluster.v4.f32 [%0], {%1,%2,%3,%4};" ::"r"(addr), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
-}
-__device__ __forceinline__ void st_async(uint32_t addr, uint32_t v, uint32_t bar) {
-  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::"r"(addr), "r"(v), "r"(bar) : "memory");
-}
-__device__ __forceinline__ void st_async(uint32_t addr, float4 v, uint32_t bar) {
-  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1,%2,%3,%4}, [%5];"
-               ::"r"(addr), "r"(__float_as_uint(v.x)), "r"(__float_as_uint(v.y)), "r"(__float_as_uint(v.z)), "r"(__float_as_uint(v.w)), "r"(bar)
-               : "memory");
 }
 
 // ------------------------------------------------------------------------------------------------ bounded waits
@@ -157,11 +122,10 @@ __device__ __forceinline__ void report_fail(const WaitCtl& c, int where, int lay
   __threadfence();
 }
 
-template <bool REMOTE = false>
 __device__ __forceinline__ bool mbar_wait(uint64_t* b, uint32_t parity, const WaitCtl& c, int where, int layer) {
-  if (mbar_try<REMOTE>(b, parity)) return true;
+  if (mbar_try(b, parity)) return true;
   for (unsigned i = 0; i < c.limit; i++) {
-    if (mbar_try<REMOTE>(b, parity)) return true;
+    if (mbar_try(b, parity)) return true;
     if ((i & 63) == 63) {
       if (*c.s_abort) return false;
       if ((i & 1023) == 1023) {

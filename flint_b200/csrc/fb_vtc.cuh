@@ -32,12 +32,12 @@
 #include <cuda.h>
 
 #include "fb_common.cuh"
-#include "fb_geometry.hpp"
 #include "fb_verify.cuh"
 
 namespace fb {
 
 constexpr int kTcThreads = 640;   // warps: 0 weights, 1 MMA issue, 2 activations, 4..11 dequantise, 12..19 epilogue
+constexpr int kTcRowBlock = 128;
 constexpr int kTcTable = 96;      // tokens of an epilogue warp, at most
 constexpr int kTcEpiBytes = 2 * kTcTable * 4 + 16 * 64;
 constexpr int kTcTrailer = kTcRowBlock * 4 + 16;      // a block's row factors, then its flag
@@ -334,6 +334,22 @@ __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, i
       "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
       ::"r"(smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(smem_u32(bar)) : "memory");
 }
+// cluster of the K splits: barrier over all threads of all its CTAs, and stores into a neighbour's shared memory
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
+__device__ __forceinline__ uint32_t map_rank(uint32_t saddr, uint32_t rank) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(saddr), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ void st_cluster_f32(uint32_t addr, float v) {
+  asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory");
+}
+// the same, counted on a barrier of that CTA
+__device__ __forceinline__ void st_async(uint32_t addr, uint32_t v, uint32_t bar) {
+  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::"r"(addr), "r"(v), "r"(bar) : "memory");
+}
+
 // Shared-memory plan (bytes). The raw ring keeps HBM busy; a stage of activations is a group's two 64-column tiles.
 // Tiles of 128 tokens, or of 192: an item's groups then take 4/3 of the time for 3/2 of the tokens, because dequantising a group and storing
 // it to tensor memory (which keeps the MMAs out meanwhile) is a cost per item. What is left of tensor memory allows two A stages, and none
@@ -434,9 +450,10 @@ struct TcFactorTable {
   __device__ __forceinline__ float x(int i) const { return fx[i]; }
   __device__ __forceinline__ float a(int i) const { return fa[i]; }
 };
-// silu(g) = g / (1 + e^-g) with the exact division, the decode kernel's expression. (The approximate one, off by up to 2 ulp and zero where
-// 1 + e^-g is above 2^126, makes the gate/up epilogue of a prompt cheaper: see the figures at TcStaged.)
-__device__ __forceinline__ float tc_silu(float g) { return g / (1.0f + __expf(-g)); }
+// silu(g) = g / (1 + e^-g). The division by approximate reciprocal (2 ulp) sits behind an exponential of the same accuracy and ahead of a
+// rounding to bf16; the exact one brings a branch per value, which keeps an epilogue's independent values from overlapping.
+// (Where 1 + e^-g is above 2^126 it returns 0; the quotient is then below 2^-119.)
+__device__ __forceinline__ float tc_silu(float g) { return __fdividef(g, 1.0f + __expf(-g)); }
 // v[e] = accumulator of (stream row srow, token t0 + e), the i0 + e-th of the warp's tokens; rf = the row's factor. The whole warp
 // calls this together: lanes 2i, 2i + 1 hold the two rows of a RoPE or gate/up pair.
 template <int EPI, int CH, class F>

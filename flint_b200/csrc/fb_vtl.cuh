@@ -95,7 +95,7 @@ __global__ void __launch_bounds__(kTlThreads, NT == 128 ? 1 : 2) v_gemm_tl(const
   const int nrb = (P.rows + kTcRowBlock - 1) / kTcRowBlock, rb = NT == 128 ? item % nrb : item, tok0 = NT == 128 ? item / nrb * P.ntok : 0,
             tend = NT == 128 ? min(P.M, tok0 + P.ntok) : P.M;
   const int g0 = G * rank >> lg, ng = (G * (rank + 1) >> lg) - g0;           // this CTA's groups (ng >= 1)
-  const bool split = NT == 128 || ns > 1;                        // 128-token tiles come here only to be split
+  const bool split = ns > 1;
   const int TPR = NT >> lg;                                      // splits: this CTA finishes tokens [rank * TPR, (rank + 1) * TPR) of the tile
   if (split) {
     if (ASYNC && tid == 0) mbar_expect_tx(xbar, (uint32_t)(max(0, min(TPR, P.M - rank * TPR)) * ns * 512));
@@ -289,16 +289,16 @@ __global__ void __launch_bounds__(kTlThreads, NT == 128 ? 1 : 2) v_gemm_tl(const
           for (int e = 0; e < 8; e++) {
             const int tk = half * HC + c + e;
             if (tk < push_end) {
-              const uint32_t to = cluster_map(mine + (uint32_t)(tk & (TPR - 1)) * 512, tk >> lgT);
-              if (ASYNC) st_async(to, u[e], cluster_map(smem_u32(xbar), tk >> lgT));
-              else st_cluster(to, u[e]);
+              const uint32_t to = map_rank(mine + (uint32_t)(tk & (TPR - 1)) * 512, tk >> lgT);
+              if (ASYNC) st_async(to, u[e], map_rank(smem_u32(xbar), tk >> lgT));
+              else st_cluster_f32(to, __uint_as_float(u[e]));
             }
           }
         }
       }
       if (real) {                                              // every rank's sums are in
         if (ASYNC) {
-          if (ok) ok = __all_sync(0xffffffffu, mbar_wait<true>(xbar, 0, wc, W_FULL, 11));
+          if (ok) ok = __all_sync(0xffffffffu, mbar_wait(xbar, 0, wc, W_FULL, 11));
         } else {
           __syncwarp();
           cluster_arrive();
@@ -354,7 +354,7 @@ __global__ void __launch_bounds__(kTlThreads, NT == 128 ? 1 : 2) v_gemm_tl(const
   }
   if (split && (ASYNC || warp < 6)) {                            // nobody leaves before its neighbours have sent what they will send
     __syncwarp();
-    if (ASYNC) cluster_arrive_relaxed();
+    if (ASYNC) asm volatile("barrier.cluster.arrive.relaxed;" ::: "memory");
     else cluster_arrive();
     cluster_wait();
   }
