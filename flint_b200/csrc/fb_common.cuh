@@ -84,11 +84,19 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* b) {
 __device__ __forceinline__ void mbar_expect_tx(uint64_t* b, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(b)), "r"(bytes) : "memory");
 }
+// REMOTE: the phase is completed by stores of other CTAs of the cluster (st.async), whose data the waiter reads: acquire at cluster scope
+// (the default is the CTA's own).
+template <bool REMOTE = false>
 __device__ __forceinline__ bool mbar_try(uint64_t* b, uint32_t parity) {
   uint32_t ok;
-  asm volatile(
-      "{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
-      : "=r"(ok) : "r"(smem_u32(b)), "r"(parity) : "memory");
+  if (REMOTE)
+    asm volatile(
+        "{ .reg .pred p; mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
+        : "=r"(ok) : "r"(smem_u32(b)), "r"(parity) : "memory");
+  else
+    asm volatile(
+        "{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
+        : "=r"(ok) : "r"(smem_u32(b)), "r"(parity) : "memory");
   return ok != 0;
 }
 __device__ __forceinline__ bool mbar_test(uint64_t* b, uint32_t parity) {
@@ -122,10 +130,11 @@ __device__ __forceinline__ void report_fail(const WaitCtl& c, int where, int lay
   __threadfence();
 }
 
+template <bool REMOTE = false>
 __device__ __forceinline__ bool mbar_wait(uint64_t* b, uint32_t parity, const WaitCtl& c, int where, int layer) {
-  if (mbar_try(b, parity)) return true;
+  if (mbar_try<REMOTE>(b, parity)) return true;
   for (unsigned i = 0; i < c.limit; i++) {
-    if (mbar_try(b, parity)) return true;
+    if (mbar_try<REMOTE>(b, parity)) return true;
     if ((i & 63) == 63) {
       if (*c.s_abort) return false;
       if ((i & 1023) == 1023) {

@@ -337,7 +337,7 @@ __global__ void __launch_bounds__(256) v_attn(const VattnParams P) {
     bool ok = true;
     if (ASYNC) {
       const WaitCtl wc{P.status, s_abort, P.spin_limit};
-      ok = __all_sync(0xffffffffu, mbar_wait(xbar, 0, wc, W_FULL, 12));
+      ok = __all_sync(0xffffffffu, mbar_wait<true>(xbar, 0, wc, W_FULL, 12));
     } else {
       asm volatile("barrier.cluster.arrive.release;" ::: "memory");
       asm volatile("barrier.cluster.wait.acquire;" ::: "memory");

@@ -298,7 +298,7 @@ __global__ void __launch_bounds__(kTlThreads, NT == 128 ? 1 : 2) v_gemm_tl(const
       }
       if (real) {                                              // every rank's sums are in
         if (ASYNC) {
-          if (ok) ok = __all_sync(0xffffffffu, mbar_wait(xbar, 0, wc, W_FULL, 11));
+          if (ok) ok = __all_sync(0xffffffffu, mbar_wait<true>(xbar, 0, wc, W_FULL, 11));
         } else {
           __syncwarp();
           cluster_arrive();
