@@ -33,7 +33,7 @@ cudaError_t launch_linear_nt(DLin p, int t0, int sms, cudaStream_t st) {
   // K splits while all CTAs are resident at once and every warp keeps two chunks
   const int slots = sms * (NT == 1 ? 3 : 2), nch = (p.k0 + p.k1 + 31) / 32;
   p.ks = 1;
-  while (p.ks < kDraftSplits && blocks * (p.ks + 1) <= slots && nch >= 2 * kDraftWarps * (p.ks + 1)) p.ks++;
+  while (MODE != DL_LOGITS && p.ks < kDraftSplits && blocks * (p.ks + 1) <= slots && nch >= 2 * kDraftWarps * (p.ks + 1)) p.ks++;
   const dim3 grid(blocks * p.ks), block(kDraftWarps * 32);
   if (MODE == DL_STORE && p.x1) return launch_pdl_cluster(d_gemm<NT, MT, MODE, MODE == DL_STORE>, grid, block, 0, st, (unsigned)p.ks, p, t0);
   return launch_pdl_cluster(d_gemm<NT, MT, MODE, false>, grid, block, 0, st, (unsigned)p.ks, p, t0);

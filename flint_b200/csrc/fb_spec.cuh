@@ -357,7 +357,8 @@ __global__ void __launch_bounds__(kDraftWarps * 32, NT == 1 ? 3 : 2) d_gemm(cons
   __shared__ float part[kDraftSplits][8 * NT][ROWS];             // split K: [source rank][token][row]
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
   const int K = P.k0 + P.k1, nch = (K + 31) >> 5;
-  const int ks = P.ks, rank = (int)blockIdx.x % ks;
+  // the token head has CTAs enough
+  const int ks = MODE == DL_LOGITS ? 1 : P.ks, rank = MODE == DL_LOGITS ? 0 : (int)blockIdx.x % ks;
   int blk = (int)blockIdx.x / ks, which = 0;
   if (MODE == DL_STORE) {
 #pragma unroll
@@ -401,8 +402,16 @@ __global__ void __launch_bounds__(kDraftWarps * 32, NT == 1 ? 3 : 2) d_gemm(cons
       x1[j] = P.x1_tokens && id >= P.x1_rows ? -1 : id;
     }
   }
+  // The token head's CTAs are short (ten chunks a warp at 2560 columns), and what each does before its first MMA counts: with the split's divisions and an
+  // address per chunk it took 58.0 / 97 / 92 us for one row of the 3B, 40-head and 1B shapes, so 56.0 / 94 / 89.5. In the longer linears a
+  // pointer per token costs more than it saves (one row, whole block 74.2 -> 75.2).
+  const uint16_t* xrow = MODE == DL_LOGITS && NT == 1 && t0 + g < P.T ? P.x0 + (size_t)(t0 + g) * P.ldx0 + 8 * t : nullptr;
   auto load_x = [&](int c, uint4 (&d)[NT]) {
     const int col = c * 32 + 8 * t;
+    if (MODE == DL_LOGITS && NT == 1) {
+      d[0] = xrow && col < K ? *reinterpret_cast<const uint4*>(xrow + c * 32) : make_uint4(0, 0, 0, 0);
+      return;
+    }
     const bool second = CAT && col >= P.k0;
     const uint16_t* base = second ? P.x1 + (col - P.k0) : P.x0 + col;
     const int ld = second ? P.ldx1 : P.ldx0;
