@@ -4,6 +4,7 @@
 
 #include "../../include/flint_b200.h"
 #include "fb_ctx.hpp"
+#include "fb_geometry.hpp"
 #include "fb_verify.cuh"
 #include "fb_vtc.cuh"
 #include "fb_vtl.cuh"
@@ -19,25 +20,8 @@ using namespace fb;
 
 namespace {
 
-// K splits (CTAs of a cluster) of one GEMM over a single token tile: two CTAs share an SM; matrices with few row blocks are cut while
-// all CTAs are resident at once and each keeps two groups to multiply
-int tl_splits(int items, int k, int nt, int sms) {
-  const int G = k / 128;
-  int ns = 1;
-  while (ns < 8 && items * ns * 2 <= 2 * sms && G / (ns * 2) >= 2 && nt / (ns * 2) >= 2) ns *= 2;
-  return ns;
-}
-// The same for the tiles of a prompt, one CTA per SM, at least four groups each. Clusters of eight fit only in 120 of 148 SMs: at most four.
-// 1: the persistent kernel, which overlaps an item's epilogue with the next item. In it prompts of 70 / 100 / 128 / 180 / 250 / 300 tokens of the
-// 3B shape took 3200 / 3388 / 3535 / 3684 / 4092 / 4437 us, split in four (one tile) or two 2566 / 2670 / 2750 / 3700 / 3911 / 4150; 100 / 200
-// tokens of the 8B shape 4290 / 5320 -> 3270 / 4725.
-int prompt_splits(int items, int k, int sms) {
-  int ns = 1;
-  while (ns < 4 && items * ns * 2 <= sms && k / 128 / (ns * 2) >= 4) ns *= 2;
-  return ns;
-}
 template <int NT, int EPI, bool HZ>
-cudaError_t launch_vtl_hz(VtcParams& p, int sms, cudaStream_t st) {
+cudaError_t launch_vtl_hz(const VtcParams& p, cudaStream_t st) {
   static bool configured[64] = {};
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
@@ -45,14 +29,14 @@ cudaError_t launch_vtl_hz(VtcParams& p, int sms, cudaStream_t st) {
     FB_TRY(cudaFuncSetAttribute(v_gemm_tl<NT, EPI, HZ>, cudaFuncAttributeMaxDynamicSharedMemorySize, VtlSmem<NT, HZ>::TOTAL));
     configured[dev] = true;
   }
-  if (p.K % 128 || p.ntok > NT || p.ntok % 16 || (NT < 128 && p.ntile > 1) || (size_t)p.ntok * p.ntile < (size_t)p.M) return cudaErrorInvalidValue;
+  if (p.K % 128 || p.ntok > NT || p.ntok % 16 || (NT < 128 && p.ntile > 1) || (NT == 128 && p.nsplit < 2) || (size_t)p.ntok * p.ntile < (size_t)p.M)
+    return cudaErrorInvalidValue;
   const int items = (p.rows + kTcRowBlock - 1) / kTcRowBlock * p.ntile;
-  p.nsplit = NT == 128 ? prompt_splits(items, p.K, sms) : tl_splits(items, p.K, NT, sms);
   return launch_pdl_cluster(v_gemm_tl<NT, EPI, HZ>, dim3(items * p.nsplit), dim3(kTlThreads), (size_t)VtlSmem<NT, HZ>::TOTAL, st,
                             (unsigned)p.nsplit, p);
 }
 template <int EPI, bool HZ, int NT>
-cudaError_t launch_vtc_hz(VtcParams& p, int sms, cudaStream_t st) {
+cudaError_t launch_vtc_hz(const VtcParams& p, int sms, cudaStream_t st) {
   static bool configured[64] = {};
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
@@ -64,34 +48,20 @@ cudaError_t launch_vtc_hz(VtcParams& p, int sms, cudaStream_t st) {
   const int items = ((p.rows + kTcRowBlock - 1) / kTcRowBlock) * p.ntile;
   return launch_pdl(v_gemm_tc<EPI, HZ, NT>, dim3(items < sms ? items : sms), dim3(kTcThreads), (size_t)VtcSmem<HZ, NT>::TOTAL, st, p);
 }
-void set_tiles(VtcParams& p, int nt) {                         // tiles of up to nt tokens, cut evenly
-  p.ntile = (p.M + nt - 1) / nt;
-  p.ntok = ((p.M + p.ntile - 1) / p.ntile + 15) / 16 * 16;
-}
-// Prompts: 192-token tiles where they need fewer than 3/4 of the rounds of items that 128-token tiles need (a round of them takes about 4/3 of the
-// time). 180 / 300 / 725 tokens of the 3B shape 3728 / 4164 / 6900 us with 128-token tiles alone, 3558 / 3997 / 6450 with the rule.
-bool wide_tiles(const VtcParams& p, int sms) {
-  const int nrb = (p.rows + kTcRowBlock - 1) / kTcRowBlock;
-  auto rounds = [&](int nt) { return (nrb * ((p.M + nt - 1) / nt) + sms - 1) / sms; };
-  return rounds(192) * 4 < rounds(128) * 3;
-}
 // `maps`: the activation buffer as a tensor, one map per token tile height (16, 32, 64, 128, 192)
 template <int EPI>
-cudaError_t launch_vtc(VtcParams& p, const CUtensorMap* maps, int nt, bool hz, int sms, cudaStream_t st) {
-  p.xmap = maps[nt == 16 ? 0 : (nt == 32 ? 1 : (nt == 64 ? 2 : 3))];
-  switch (nt) {
-    case 16: return hz ? launch_vtl_hz<16, EPI, true>(p, sms, st) : launch_vtl_hz<16, EPI, false>(p, sms, st);
-    case 32: return hz ? launch_vtl_hz<32, EPI, true>(p, sms, st) : launch_vtl_hz<32, EPI, false>(p, sms, st);
-    case 64: return hz ? launch_vtl_hz<64, EPI, true>(p, sms, st) : launch_vtl_hz<64, EPI, false>(p, sms, st);
+cudaError_t launch_vtc(VtcParams& p, const CUtensorMap* maps, bool hz, int sms, cudaStream_t st) {
+  const GemmGeometry g = gemm_geometry(p.M, p.rows, p.K, hz, sms);
+  p.ntok = g.ntok; p.ntile = g.ntile; p.nsplit = g.nsplit;
+  p.xmap = maps[g.nt == 16 ? 0 : (g.nt == 32 ? 1 : (g.nt == 64 ? 2 : (g.nt == 128 ? 3 : 4)))];
+  switch (g.nt) {
+    case 16: return hz ? launch_vtl_hz<16, EPI, true>(p, st) : launch_vtl_hz<16, EPI, false>(p, st);
+    case 32: return hz ? launch_vtl_hz<32, EPI, true>(p, st) : launch_vtl_hz<32, EPI, false>(p, st);
+    case 64: return hz ? launch_vtl_hz<64, EPI, true>(p, st) : launch_vtl_hz<64, EPI, false>(p, st);
     case 128:
-      if (prompt_splits((p.rows + kTcRowBlock - 1) / kTcRowBlock * p.ntile, p.K, sms) > 1)
-        return hz ? launch_vtl_hz<128, EPI, true>(p, sms, st) : launch_vtl_hz<128, EPI, false>(p, sms, st);
-      if (hz) return launch_vtc_hz<EPI, true, 128>(p, sms, st);
-      if (!wide_tiles(p, sms)) return launch_vtc_hz<EPI, false, 128>(p, sms, st);
-      VtcParams w = p;
-      set_tiles(w, 192);
-      w.xmap = maps[4];
-      return launch_vtc_hz<EPI, false, 192>(w, sms, st);
+      if (g.nsplit > 1) return hz ? launch_vtl_hz<128, EPI, true>(p, st) : launch_vtl_hz<128, EPI, false>(p, st);
+      return hz ? launch_vtc_hz<EPI, true, 128>(p, sms, st) : launch_vtc_hz<EPI, false, 128>(p, sms, st);
+    case 192: return launch_vtc_hz<EPI, false, 192>(p, sms, st);
   }
   return cudaErrorInvalidValue;
 }
@@ -131,25 +101,17 @@ template <int HD, int R>
 cudaError_t launch_vattn_hd(const VattnParams& a, int rt, dim3 grid, cudaStream_t st) {
   return rt == 1 ? launch_vattn_rt<HD, R, 1>(a, grid, st) : (rt == 2 ? launch_vattn_rt<HD, R, 2>(a, grid, st) : launch_vattn_rt<HD, R, 4>(a, grid, st));
 }
-// Geometry. Few row tiles: one or two a CTA, its warps share the span's positions instead; four where that many CTAs would not fit the
-// GPU with four spans each. Spans: a power of two up to 8 while there is a stage for each and all CTAs are resident at once (with one
-// CTA per SM the GPU holds 15 clusters of 8 -- the 16th waited for a second wave, 22 us instead of 12 -- but 36 of 4).
 cudaError_t launch_vattn_tc(const fb_ctx* c, const uint16_t* kc, const uint16_t* vc, const uint8_t* amask, int pos, int M, bool want_max,
                             cudaStream_t st) {
   const fb_model_desc& d = c->d;
-  const int T = pos + M, tiles = (M * c->rgqa + 15) / 16, per4 = c->sm_count / (4 * d.n_kv_head);
-  VattnParams a{c->vq, kc, vc, amask, c->vao, want_max ? c->vamax : nullptr, d.n_head, d.n_kv_head, pos, M, 0, d.attn_scale * 1.4426950408889634f,
-               c->status, c->spin_limit};
-  const int rt = tiles <= per4 ? 1 : (tiles <= 2 * per4 ? 2 : 4), mg = (tiles + rt - 1) / rt, groups = d.n_kv_head * mg;
-  const int stages = (T + 63) / 64;
-  int nspan = 1;
-  while (nspan < 8 && nspan * 2 <= stages && groups * nspan * 2 <= (nspan == 4 ? c->sm_count * 2 / 3 : c->sm_count)) nspan *= 2;
-  a.span = (stages + nspan - 1) / nspan * 64;
-  const dim3 grid(nspan, d.n_kv_head, mg);
-  if (d.head_dim == 64 && c->rgqa == 4) return launch_vattn_hd<64, 4>(a, rt, grid, st);
-  if (d.head_dim == 80 && c->rgqa == 4) return launch_vattn_hd<80, 4>(a, rt, grid, st);
-  if (d.head_dim == 64 && c->rgqa == 5) return launch_vattn_hd<64, 5>(a, rt, grid, st);
-  if (d.head_dim == 128 && c->rgqa == 4) return launch_vattn_hd<128, 4>(a, rt, grid, st);
+  const AttnGeometry a = attn_geometry(M, pos, d.n_kv_head, c->rgqa, c->sm_count);
+  const VattnParams p{c->vq, kc, vc, amask, c->vao, want_max ? c->vamax : nullptr, d.n_head, d.n_kv_head, pos, M, a.span,
+                      d.attn_scale * 1.4426950408889634f, c->status, c->spin_limit};
+  const dim3 grid(a.nspan, d.n_kv_head, a.groups);
+  if (d.head_dim == 64 && c->rgqa == 4) return launch_vattn_hd<64, 4>(p, a.rt, grid, st);
+  if (d.head_dim == 80 && c->rgqa == 4) return launch_vattn_hd<80, 4>(p, a.rt, grid, st);
+  if (d.head_dim == 64 && c->rgqa == 5) return launch_vattn_hd<64, 5>(p, a.rt, grid, st);
+  if (d.head_dim == 128 && c->rgqa == 4) return launch_vattn_hd<128, 4>(p, a.rt, grid, st);
   return cudaErrorInvalidValue;
 }
 
@@ -160,8 +122,7 @@ int run_tc_pass(fb_ctx* c, const int32_t* d_tokens, const void* d_h, const int32
   const fb_model_desc& d = c->d;
   const int D = d.dim, FF = d.ffn, HD = d.head_dim, QD = d.n_head * HD, QKV = (d.n_head + 2 * d.n_kv_head) * HD, sms = c->sm_count;
   const bool hz = d.has_zeros != 0;
-  // token tile: the smallest that holds the tokens; prompts go in tiles of up to 128, cut evenly
-  const int nt = M <= 16 ? 16 : (M <= 32 ? 32 : (M <= 64 ? 64 : 128));
+  const bool tree = token_tile(M) <= 64;
   const size_t tQ = tc_matrix_bytes(QKV, D, hz), tO = tc_matrix_bytes(D, QD, hz), tG = tc_matrix_bytes(2 * FF, D, hz),
                tF = tc_matrix_bytes(D, FF, hz);
   FB_CUDA(c, launch_pdl(v_embed, dim3(M), dim3(256), 0, st, d_tokens, (const uint16_t*)c->embed, (const uint16_t*)d_h, c->vh,
@@ -170,7 +131,6 @@ int run_tc_pass(fb_ctx* c, const int32_t* d_tokens, const void* d_h, const int32
   VtcParams t;
   memset(&t, 0, sizeof(t));
   t.M = M; t.status = c->status; t.spin_limit = c->spin_limit;
-  set_tiles(t, nt);
   t.rope = (const float2*)c->vrope; t.n_head = d.n_head; t.nkv = d.n_kv_head; t.pos = pos; t.head_dim = HD;
   t.resid = d.resid_mult; t.logits_scaling = d.logits_scaling; t.h = c->vh; t.q = c->vq; t.act = c->vact; t.fa = c->vfa;
   t.logits = d_logits;
@@ -186,26 +146,26 @@ int run_tc_pass(fb_ctx* c, const int32_t* d_tokens, const void* d_h, const int32
     uint16_t* vcl = (uint16_t*)c->vc + (size_t)l * c->max_seq * d.n_kv_head * HD;
     FB_CUDA(c, norm((const uint16_t*)c->n1 + (size_t)l * D, nullptr, nullptr));
     t.w = c->t_qkv + l * tQ; t.rows = QKV; t.K = D; t.kc = kcl; t.vc = vcl; t.fx = c->vfx;
-    FB_CUDA(c, launch_vtc<EPI_QKV>(t, c->m_xn, nt, hz, sms, st));
+    FB_CUDA(c, launch_vtc<EPI_QKV>(t, c->m_xn, hz, sms, st));
     // trees: the O GEMM converts the attention output to fp16 on its way in; prompts, whose activations come by tensor copies, have it
     // converted in place
-    FB_CUDA(c, launch_vattn_tc(c, kcl, vcl, d_amask, pos, M, nt <= 64, st));
-    if (nt > 64) FB_CUDA(c, launch_pdl(v_row_f16, dim3(M), dim3(256), 0, st, c->vao, c->vfao, QD));
+    FB_CUDA(c, launch_vattn_tc(c, kcl, vcl, d_amask, pos, M, tree, st));
+    if (!tree) FB_CUDA(c, launch_pdl(v_row_f16, dim3(M), dim3(256), 0, st, c->vao, c->vfao, QD));
     t.w = c->t_o + l * tO; t.rows = D; t.K = QD; t.out_ld = D; t.fx = c->vfao;
-    t.xbf = nt <= 64 ? c->vao : nullptr; t.amax = nt <= 64 ? c->vamax : nullptr;
-    FB_CUDA(c, launch_vtc<EPI_RESID>(t, c->m_ao, nt, hz, sms, st));
+    t.xbf = tree ? c->vao : nullptr; t.amax = tree ? c->vamax : nullptr;
+    FB_CUDA(c, launch_vtc<EPI_RESID>(t, c->m_ao, hz, sms, st));
     t.xbf = nullptr; t.amax = nullptr;
     FB_CUDA(c, norm((const uint16_t*)c->n2 + (size_t)l * D, nullptr, c->gu_norms + 2 * l));
     t.w = c->t_gu + l * tG; t.rows = 2 * FF; t.K = D; t.out_ld = FF; t.fx = c->vfx;
-    FB_CUDA(c, launch_vtc<EPI_SWIGLU>(t, c->m_xn, nt, hz, sms, st));
+    FB_CUDA(c, launch_vtc<EPI_SWIGLU>(t, c->m_xn, hz, sms, st));
     t.w = c->t_d + l * tF; t.rows = D; t.K = FF; t.out_ld = D; t.fx = c->vfa_inv;
-    FB_CUDA(c, launch_vtc<EPI_RESID>(t, c->m_act, nt, hz, sms, st));
+    FB_CUDA(c, launch_vtc<EPI_RESID>(t, c->m_act, hz, sms, st));
   }
   // the feature goes to the caller; the LM head reads the context's copy
   FB_CUDA(c, norm(c->nf, (uint16_t*)d_feat, nullptr));
   if (d_logits) {
     t.w = c->t_lm; t.rows = d.vocab; t.K = D; t.out_ld = d.vocab; t.fx = c->vfx;
-    FB_CUDA(c, launch_vtc<EPI_LOGITS>(t, c->m_xn, nt, hz, sms, st));
+    FB_CUDA(c, launch_vtc<EPI_LOGITS>(t, c->m_xn, hz, sms, st));
   }
   FB_CUDA(c, cudaGetLastError());
   return FB_OK;

@@ -6,6 +6,7 @@
 
 #include "../../include/flint_b200.h"
 #include "fb_ctx.hpp"
+#include "fb_geometry.hpp"
 #include "fb_spec.cuh"
 
 using namespace fb;
@@ -30,10 +31,7 @@ template <int NT, int MT, int MODE>
 cudaError_t launch_linear_nt(DLin p, int t0, int sms, cudaStream_t st) {
   int blocks = 0;
   for (int i = 0; i < (MODE == DL_STORE ? 3 : 1) && p.W[i]; i++) blocks += (p.N[i] + 16 * MT - 1) / (16 * MT);
-  // K splits while all CTAs are resident at once and every warp keeps two chunks
-  const int slots = sms * (NT == 1 ? 3 : 2), nch = (p.k0 + p.k1 + 31) / 32;
-  p.ks = 1;
-  while (MODE != DL_LOGITS && p.ks < kDraftSplits && blocks * (p.ks + 1) <= slots && nch >= 2 * kDraftWarps * (p.ks + 1)) p.ks++;
+  p.ks = MODE == DL_LOGITS ? 1 : draft_splits(blocks, (p.k0 + p.k1 + 31) / 32, NT, sms);
   const dim3 grid(blocks * p.ks), block(kDraftWarps * 32);
   if (MODE == DL_STORE && p.x1) return launch_pdl_cluster(d_gemm<NT, MT, MODE, MODE == DL_STORE>, grid, block, 0, st, (unsigned)p.ks, p, t0);
   return launch_pdl_cluster(d_gemm<NT, MT, MODE, false>, grid, block, 0, st, (unsigned)p.ks, p, t0);

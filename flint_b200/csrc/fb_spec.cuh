@@ -7,6 +7,7 @@
 // activation and residual addition rounds its result to bf16; accumulation inside a layer is fp32.
 #pragma once
 #include "fb_common.cuh"
+#include "fb_geometry.hpp"
 
 namespace fb {
 
@@ -347,8 +348,6 @@ struct DLin {
 // A matrix whose rows give less than the GPU's worth of CTAs is also cut in K over a cluster of ks: the CTAs push their sums into the shared
 // memory of the one that finishes the token, which adds them in rank order. (With 16 warps and no split a 2560-row matrix ran on 80
 // SMs: window of 32 rows 177 -> 153 us, 48 rows of the 40-head shape 290 -> 258; single rows, three CTAs an SM, 125.1 without the split, 122.3.)
-constexpr int kDraftSplits = 3;
-constexpr int kDraftWarps = 8;
 template <int NT, int MT, int MODE, bool CAT>
 __global__ void __launch_bounds__(kDraftWarps * 32, NT == 1 ? 3 : 2) d_gemm(const DLin P, int t0) {
   constexpr int WARPS = kDraftWarps;

@@ -32,12 +32,12 @@
 #include <cuda.h>
 
 #include "fb_common.cuh"
+#include "fb_geometry.hpp"
 #include "fb_verify.cuh"
 
 namespace fb {
 
 constexpr int kTcThreads = 640;   // warps: 0 weights, 1 MMA issue, 2 activations, 4..11 dequantise, 12..19 epilogue
-constexpr int kTcRowBlock = 128;
 constexpr int kTcTable = 96;      // tokens of an epilogue warp, at most
 constexpr int kTcEpiBytes = 2 * kTcTable * 4 + 16 * 64;
 constexpr int kTcTrailer = kTcRowBlock * 4 + 16;      // a block's row factors, then its flag

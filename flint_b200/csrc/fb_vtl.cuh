@@ -95,7 +95,7 @@ __global__ void __launch_bounds__(kTlThreads, NT == 128 ? 1 : 2) v_gemm_tl(const
   const int nrb = (P.rows + kTcRowBlock - 1) / kTcRowBlock, rb = NT == 128 ? item % nrb : item, tok0 = NT == 128 ? item / nrb * P.ntok : 0,
             tend = NT == 128 ? min(P.M, tok0 + P.ntok) : P.M;
   const int g0 = G * rank >> lg, ng = (G * (rank + 1) >> lg) - g0;           // this CTA's groups (ng >= 1)
-  const bool split = ns > 1;
+  const bool split = NT == 128 || ns > 1;                        // 128-token tiles come here only to be split
   const int TPR = NT >> lg;                                      // splits: this CTA finishes tokens [rank * TPR, (rank + 1) * TPR) of the tile
   if (split) {
     if (ASYNC && tid == 0) mbar_expect_tx(xbar, (uint32_t)(max(0, min(TPR, P.M - rank * TPR)) * ns * 512));

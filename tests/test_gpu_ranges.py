@@ -3,6 +3,7 @@ verify GEMMs and the prompt pass, weight scales too far apart for the short dequ
 row tiles of the draft head. Against the CPU oracle (or, for the token choice, the exact order of the input)."""
 import ctypes
 
+import geometry
 import numpy as np
 import pytest
 import torch
@@ -10,7 +11,8 @@ import torch
 from flint_b200 import _lib, packing
 from flint_b200.config import ModelArgs
 from flint_b200.draft import seeded_draft
-from flint_b200.engine import DecodeEngine
+from flint_b200.engine import DecodeEngine, query
+from flint_b200.tree import tree_mask
 from oracle import oracle as O
 from oracle.draft_oracle import DraftOracle, sample_probs
 
@@ -115,15 +117,21 @@ def test_verify_token_tile_edges(M, asym):
 
 
 @pytest.mark.parametrize("asym", [False, True])
-@pytest.mark.parametrize("M", [1, 3, 40, 70, 300])
-def test_passes_that_give_up_leave_nothing_behind(M, asym):
+@pytest.mark.parametrize("M,pos", [(1, 0), (3, 0), (40, 0), (70, 0), (300, 0), (3, 600), (16, 600)])
+def test_passes_that_give_up_leave_nothing_behind(M, pos, asym):
     """With a wait limit of 0 a pass (one token: a decode step; up to 64 a tree pass; more a prompt pass) gives up at the first wait that is not
-    satisfied already. Every launch ends, after its copies and MMAs in flight (their wait has its own limit), the status says time-out or,
-    if every wait happened to be satisfied, nothing, and the next clean pass gives the bits of the first."""
+    satisfied already. Every launch ends, after its copies, MMAs and remote stores in flight (their wait has its own limit), the status says
+    time-out or, if every wait happened to be satisfied, nothing, and the next clean pass gives the bits of the first. Behind 600 positions the
+    attention of 3 and 16 tokens runs as clusters of eight whose partials are asynchronous stores; at position 0 it is one CTA."""
     cfg = ModelArgs.from_name("tiny")
-    eng = DecodeEngine(cfg, {k: v.cuda() for k, v in packing.synth_packed(cfg, 0, asym=asym).items()}, max_seq=512)
+    if pos:
+        rt, _, nspan, _ = geometry.attn(M, pos, cfg.n_local_heads, cfg.n_head // cfg.n_local_heads, query()["sm_count"])
+        assert (rt, nspan) == (1, 8)
+    eng = DecodeEngine(cfg, {k: v.cuda() for k, v in packing.synth_packed(cfg, 0, asym=asym).items()}, max_seq=640)
+    eng.kc.normal_()
+    eng.vc.normal_()
     toks = torch.randint(0, cfg.vocab_size, (M,), generator=torch.Generator().manual_seed(M), dtype=torch.int32).cuda()
-    run = (lambda: eng.decode(17, 0).clone()) if M == 1 else (lambda: (eng.verify if M <= 64 else eng.prefill)(toks, 0)[0])
+    run = (lambda: eng.decode(17, 0).clone()) if M == 1 else (lambda: (eng.verify if M <= 64 else eng.prefill)(toks, pos)[0])
     ref = run()
     eng.check()
     for _ in range(8):
@@ -203,29 +211,9 @@ def test_prompt_pass_tile_and_chunk_edges(M):
     eng.close()
 
 
-@pytest.mark.parametrize("asym", [False, True])
-@pytest.mark.parametrize("M", [65, 128, 129, 300])
-def test_prompt_tiles_with_split_k(M, asym):
-    """Short prompts on a shape with few row blocks (24 / 16 / 16 of QKV, O, down): one, two and three token tiles run as clusters of four and of
-    two, one of them with tokens in only part of its ranks."""
-    cfg = ModelArgs.from_name("llama-1b-class")
-    cfg.n_layer, cfg.vocab_size = 1, 512
+def _prompt_against_oracle(cfg, M, asym=False):
+    """Logits of all rows and every cache row of a prompt behind 3 cached rows; the oracle takes it in pieces of 64."""
     orc, eng = _pair(cfg, M + 8, 3, packing.synth_packed(cfg, 0, asym=asym))
-    toks = torch.randint(0, cfg.vocab_size, (M,), generator=torch.Generator().manual_seed(M)).tolist()
-    ref = np.concatenate([orc.verify(toks[i:i + 64], 3 + i)[0] for i in range(0, M, 64)])
-    lg, _ = eng.prefill(toks, 3)
-    eng.check()
-    assert np.abs(lg.cpu().numpy() - ref).max() < _tol(ref)
-    eng.close()
-
-
-@pytest.mark.parametrize("M", [161, 192, 193, 385, 900])
-def test_prompt_tiles_of_192_tokens(M):
-    """Prompts whose gate/up (and at 900 tokens QKV) items take fewer rounds as 192-token tiles: one full tile, the first token of a second and
-    a third, tiles cut evenly. Logits of the last rows and every cache row against the oracle."""
-    cfg = ModelArgs.from_name("llama-1b-class")
-    cfg.n_layer, cfg.vocab_size = 1, 512
-    orc, eng = _pair(cfg, M + 8, 3)
     toks = torch.randint(0, cfg.vocab_size, (M,), generator=torch.Generator().manual_seed(M)).tolist()
     ref = np.concatenate([orc.verify(toks[i:i + 64], 3 + i)[0] for i in range(0, M, 64)])
     lg, _ = eng.prefill(toks, 3)
@@ -233,6 +221,75 @@ def test_prompt_tiles_of_192_tokens(M):
     assert np.abs(lg.cpu().numpy() - ref).max() < _tol(ref)
     for dev, host in ((eng.kc, orc.kc), (eng.vc, orc.vc)):
         assert np.abs(_f32(dev[:, 3:3 + M]) - O.bf16_to_f32(host[:, 3:3 + M])).max() < 0.05
+    eng.close()
+
+
+@pytest.mark.parametrize("asym", [False, True])
+@pytest.mark.parametrize("M,splits", [(65, (4, 4, 4)), (128, (4, 4, 4)), (129, (2, 4, 4)), (300, (2, 2, 2))])
+def test_prompt_tiles_with_split_k(M, splits, asym):
+    """Short prompts on a shape with few row blocks (24 / 16 / 16 of QKV, O, down; 4 of the LM head): one, two and three token tiles run as clusters
+    of four and of two, one of them with tokens in only part of its ranks."""
+    cfg = ModelArgs.from_name("llama-1b-class")
+    cfg.n_layer, cfg.vocab_size = 1, 512
+    g = geometry.matrices(cfg, M, asym, query()["sm_count"])
+    assert tuple(g[n][3] for n in ("qkv", "o", "d")) == splits and g["lm"][3] == 4 and g["o"][2] == -(-M // 128)
+    _prompt_against_oracle(cfg, M, asym)
+
+
+@pytest.mark.parametrize("asym", [False, True])
+def test_prompt_tiles_with_split_k_of_gate_and_up(asym):
+    """A model whose 32 gate/up row blocks are few enough for a prompt's SwiGLU to run over a cluster. No built-in shape is one: this runs on a library
+    built with FLINT_B200_EXTRA_SHAPES="2048,2048,2048,64,4"."""
+    cfg = ModelArgs(block_size=256, vocab_size=512, n_layer=1, n_head=32, n_local_heads=8, dim=2048, intermediate_size=2048)
+    try:
+        DecodeEngine(cfg, {k: v.cuda() for k, v in packing.synth_packed(cfg, 0, asym=asym).items()}, max_seq=8).close()
+    except _lib.FlintError as e:
+        assert e.code == _lib.FB_ERR_SHAPE
+        pytest.skip("library built without the shape 2048,2048,2048,64,4")
+    for M, splits in ((65, 4), (81, 4), (128, 4), (129, 2)):
+        assert geometry.matrices(cfg, M, asym, query()["sm_count"])["gu"][2:] == (-(-M // 128), splits)
+        _prompt_against_oracle(cfg, M, asym)
+
+
+@pytest.mark.parametrize("name,vocab,M,wide", [
+    ("llama-1b-class", 512, 161, "gu"), ("llama-1b-class", 512, 192, "gu"), ("llama-1b-class", 512, 257, "gu"), ("llama-1b-class", 512, 384, "gu"),
+    ("llama-1b-class", 512, 513, "gu"), ("llama-1b-class", 512, 900, "qkv gu"), ("llama-1b-class", 20000, 161, "gu lm"),
+    ("llama-1b-class", 20000, 700, "gu lm"), ("granite-3b-class", 10000, 900, "o gu d lm"), ("granite-3b-class", 512, 1000, "o d"),
+    ("llama-8b-class", 512, 520, "qkv o gu d")])
+def test_prompt_tiles_of_192_tokens(name, vocab, M, wide):
+    """Prompts some of whose matrices take fewer rounds as 192-token tiles, every epilogue among them: a tile not quite and just full, the first
+    tokens of a second and a third tile, tiles cut evenly into halves of 96 and less; the LM head with a last row block that is not full."""
+    cfg = ModelArgs.from_name(name)
+    cfg.n_layer, cfg.vocab_size = 1, vocab
+    g = geometry.matrices(cfg, M, sms=query()["sm_count"])
+    assert [n for n in g if g[n][0] == 192] == wide.split()
+    _prompt_against_oracle(cfg, M)
+
+
+@pytest.mark.parametrize("pos,Ms", [(127, (4,)), (128, (14,)), (129, (26,)), (1000, (4, 14, 26, 61)), (3001, (4, 26))])
+@pytest.mark.parametrize("name", sorted(SHAPES))
+def test_verify_attention_over_spans_of_every_geometry(name, pos, Ms):
+    """Trees behind cached prefixes for every head geometry, 40 / 8 heads (whose row tiles cut a token's heads) and heads of 128 among them: one, two
+    and four row tiles a CTA, clusters of two to eight, the first stages requested ahead of the wait and, at 3001, more than those; a random
+    ancestor mask."""
+    cfg = ModelArgs.from_name(name)
+    cfg.n_layer, cfg.vocab_size = 1, 512
+    if pos == 1000:
+        r = cfg.n_head // cfg.n_local_heads
+        geo = [geometry.attn(M, pos, cfg.n_local_heads, r, query()["sm_count"]) for M in Ms]
+        assert [(g[0], g[2]) for g in geo] == ([(1, 8), (1, 4), (2, 4), (4, 4)] if r == 4 else [(1, 4), (2, 4), (4, 4), (4, 2)])
+    orc, eng = _pair(cfg, pos + 64, pos)
+    for M in Ms:
+        g = torch.Generator().manual_seed(M)
+        toks = torch.randint(0, cfg.vocab_size, (M,), generator=g).tolist()
+        parent = [-1] + [int(torch.randint(0, i, (1,), generator=g)) for i in range(1, M)]
+        mask = tree_mask(parent)
+        depth = mask.sum(1).astype(np.int32) - 1
+        ref, _ = orc.verify(toks, pos, depth, mask)
+        lg, _ = eng.verify(toks, pos, torch.from_numpy(depth), torch.from_numpy(mask))
+        eng.check()
+        assert np.abs(lg.cpu().numpy() - ref).max() < _tol(ref)
+        assert np.abs(_f32(eng.kc[:, pos:pos + M]) - O.bf16_to_f32(orc.kc[:, pos:pos + M])).max() < 0.05
     eng.close()
 
 
@@ -359,11 +416,15 @@ def test_draft_row_tile_edges(T):
 
 
 @pytest.mark.parametrize("T", [1, 8, 16, 33])
-@pytest.mark.parametrize("inter", [1024, 1544, 2048])
-def test_draft_linears_with_split_k(T, inter):
-    """Linears whose K goes over a cluster: the merge (K = 1024) over two CTAs, the down projection over two or three, one of them with a K that
-    is no multiple of a chunk."""
-    dim, nh, nkv, vocab = 256, 8, 2, 1000
+@pytest.mark.parametrize("dim,inter", [(256, 1024), (256, 1544), (256, 2048), (1024, 1032), (1536, 1032)])
+def test_draft_linears_with_split_k(T, dim, inter):
+    """Linears whose K goes over a cluster. 256 wide: the merge (K = 1024) over two CTAs, the down projection over two or three, one of them with a K that
+    is no multiple of a chunk. 1024 and 1536 wide: q, k and v in one grid, the SwiGLU pair, O and the last linear too, over two and three CTAs."""
+    nh, nkv, vocab, sms = dim // 128 * 4, dim // 128, 1000, query()["sm_count"]
+    kv = nkv * (dim // nh)
+    for n in {min(T, 32), T - 32 if T > 32 else T}:
+        ks = [geometry.draft(rows, k, n, pair, sms) for rows, k, pair in (((dim,), 4 * dim, False), ((dim, kv, kv), dim, False), ((inter,), dim, True))]
+        assert ks == ([2, 1, 1] if dim == 256 else [3, 2, 2] if dim == 1024 else [3, 3, 3])
     m = seeded_draft(dim, nh, inter, seed=5, rope_base=10000.0, n_kv=nkv, fuse=3)
     g = torch.Generator().manual_seed(T)
     m.bind_target((torch.randn(vocab, dim, generator=g) * 0.5).bfloat16().cuda(), torch.ones(dim, dtype=torch.bfloat16).cuda(), 1.0)
