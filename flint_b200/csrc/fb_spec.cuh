@@ -50,18 +50,9 @@ struct SampleParams {
 // engine/generate.py:37-39). Bound by latency: four cluster barriers and three scans. (One CTA per row took 83 us for a row of 128256
 // values and k = 50: five passes of 512 KB through one SM, most of the first digit's atomics on a handful of bins.)
 constexpr int kSampleRegs = 16;
-__device__ __forceinline__ uint32_t sm_map(uint32_t saddr, uint32_t rank) {
-  uint32_t r;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(saddr), "r"(rank));
-  return r;
-}
-__device__ __forceinline__ void sm_cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
-__device__ __forceinline__ void sm_cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
-__device__ __forceinline__ void sm_cluster_sync() { sm_cluster_arrive(); sm_cluster_wait(); }
 // Another CTA's shared memory may be touched only once that CTA is known to run. Every CTA of the cluster arrives at the start of the kernel
 // and waits before its first remote access: the row's loads lie in between and hide the barrier.
-__device__ __forceinline__ void sm_st(uint32_t a, uint32_t v) { asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory"); }
-__device__ __forceinline__ uint2 sm_ld2(uint32_t a) {
+__device__ __forceinline__ uint2 ld_cluster(uint32_t a) {
   uint2 v;
   asm volatile("ld.shared::cluster.v2.u32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(a) : "memory");
   return v;
@@ -93,7 +84,7 @@ __global__ void __launch_bounds__(1024) sample_rows(const SampleParams P) {
   const float* lg = P.logits + (long long)row * P.row_stride;
   const int per = (P.vocab + C - 1) / C, i0 = rank * per, i1 = min(P.vocab, i0 + per);
   const bool draw = P.temperature > 0.f, select = draw && P.top_k > 0 && P.top_k < P.vocab;
-  if (!select) sm_cluster_arrive();               // the selection's own barriers come before its first remote read
+  if (!select) cluster_arrive();               // the selection's own barriers come before its first remote read
   pdl_trigger();
   pdl_wait();
   float v[REG ? kSampleRegs : 1];
@@ -124,14 +115,14 @@ __global__ void __launch_bounds__(1024) sample_rows(const SampleParams P) {
         const uint32_t key = fkey(x);
         if ((key & mask) == prefix) atomicAdd(&hist[d][(key >> shift) & dmask], 1u);
       });
-      sm_cluster_sync();
+      cluster_sync();
       // thread t holds bins 2047 - 2t and 2046 - 2t: an inclusive scan in thread order counts from the largest key down
       const uint32_t h = (uint32_t)__cvta_generic_to_shared(&hist[d][2046 - 2 * tid]);
       unsigned b0 = 0u, b1 = 0u;
 #pragma unroll
       for (int c = 0; c < 8; c++)
         if (c < C) {
-          const uint2 u = sm_ld2(sm_map(h, c));
+          const uint2 u = ld_cluster(cluster_map(h, c));
           b0 += u.x;
           b1 += u.y;
         }
@@ -174,16 +165,16 @@ __global__ void __launch_bounds__(1024) sample_rows(const SampleParams P) {
   warp_best(bv, bi);
   if (lane == 0) { s_v[warp] = bv; s_i[warp] = bi; }
   __syncthreads();
-  if (!select) sm_cluster_wait();
+  if (!select) cluster_wait();
   if (warp == 0) {
     bv = s_v[lane]; bi = s_i[lane];
     warp_best(bv, bi);
     if (lane == 0) {
-      sm_st(sm_map((uint32_t)__cvta_generic_to_shared(c_v + rank), 0), __float_as_uint(bv));
-      sm_st(sm_map((uint32_t)__cvta_generic_to_shared(c_i + rank), 0), (uint32_t)bi);
+      st_cluster(cluster_map((uint32_t)__cvta_generic_to_shared(c_v + rank), 0), __float_as_uint(bv));
+      st_cluster(cluster_map((uint32_t)__cvta_generic_to_shared(c_i + rank), 0), (uint32_t)bi);
     }
   }
-  sm_cluster_sync();
+  cluster_sync();
   if (rank == 0 && warp == 0) {
     bv = lane < C ? c_v[lane] : -INFINITY;
     bi = lane < C ? c_i[lane] : 0x7fffffff;
@@ -204,7 +195,7 @@ __global__ void __launch_bounds__(1024) topb_rows(const float* logits, long long
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, row = blockIdx.y, C = gridDim.x, rank = blockIdx.x;
   const float* lg = logits + (long long)row * row_stride;
   const int per = (vocab + C - 1) / C, i0 = rank * per, i1 = min(vocab, i0 + per);
-  sm_cluster_arrive();
+  cluster_arrive();
   pdl_trigger();
   pdl_wait();
   float v[REG ? kSampleRegs : 1];
@@ -235,15 +226,15 @@ __global__ void __launch_bounds__(1024) topb_rows(const float* logits, long long
     warp_best(bv, bi);
     if (lane == 0) { s_v[warp] = bv; s_i[warp] = bi; }
     __syncthreads();
-    if (r == 0) sm_cluster_wait();
+    if (r == 0) cluster_wait();
     if (warp == 0) {
       bv = s_v[lane]; bi = s_i[lane];
       warp_best(bv, bi);
       if (lane == 0) {
         s_pick = bi;
         s_v[0] = bv;
-        sm_st(sm_map((uint32_t)__cvta_generic_to_shared(c_v + rank * B + r), 0), __float_as_uint(bv));
-        sm_st(sm_map((uint32_t)__cvta_generic_to_shared(c_i + rank * B + r), 0), (uint32_t)bi);
+        st_cluster(cluster_map((uint32_t)__cvta_generic_to_shared(c_v + rank * B + r), 0), __float_as_uint(bv));
+        st_cluster(cluster_map((uint32_t)__cvta_generic_to_shared(c_i + rank * B + r), 0), (uint32_t)bi);
       }
     }
     __syncthreads();
@@ -253,7 +244,7 @@ __global__ void __launch_bounds__(1024) topb_rows(const float* logits, long long
     if (REG && pi != 0x7fffffff && loc >= 0 && (loc & 1023) == 0) taken |= 1u << (loc >> 10);
     __syncthreads();
   }
-  sm_cluster_sync();
+  cluster_sync();
   if (rank == 0 && warp == 0) {
     unsigned used = 0u;                           // lane l looks at candidates l, l + 32, ... (at most 256: 8 each)
     for (int r = 0; r < B; r++) {
@@ -387,7 +378,7 @@ __global__ void __launch_bounds__(kDraftWarps * 32, NT == 1 ? 3 : 2) d_gemm(cons
 #pragma unroll
         for (int h = 0; h < 2; h++) d[i][m][h] = ok ? __ldcs(wb[i] + (wr[m][h] + c * 4)) : make_uint4(0, 0, 0, 0);
   };
-  if (ks > 1) sm_cluster_arrive();                   // remote stores wait for it below
+  if (ks > 1) cluster_arrive();                   // remote stores wait for it below
   const int c1 = rank * WARPS + warp, step = WARPS * ks;         // this warp's chunks
   pdl_begin(P.first && t0 == 0);
 #pragma unroll
@@ -466,16 +457,16 @@ __global__ void __launch_bounds__(kDraftWarps * 32, NT == 1 ? 3 : 2) d_gemm(cons
   __syncthreads();
   constexpr int NO = 16 * MT * 8 * NT;
   if (ks > 1) {
-    sm_cluster_wait();
+    cluster_wait();
     for (int o = tid; o < NO * NW; o += WARPS * 32) {
       const int r = o % ROWS, tk = o / ROWS;
       if (t0 + tk >= P.T) break;
       float s = 0.f;
 #pragma unroll
       for (int w = 0; w < 8; w++) s += red[w][r][tk];
-      sm_st(sm_map(smem_u32(&part[rank][tk][r]), tk % ks), __float_as_uint(s));
+      st_cluster(cluster_map(smem_u32(&part[rank][tk][r]), tk % ks), __float_as_uint(s));
     }
-    sm_cluster_sync();
+    cluster_sync();
   }
   for (int o = tid; o < NO; o += WARPS * 32) {
     const int r = o % (16 * MT), tk = o / (16 * MT), n = r0 + r, tok = t0 + tk;

@@ -32,20 +32,6 @@ struct VaCfg {
   static_assert(SP / UP == PG || RT == 4, "one unit per warp and stage");
 };
 
-__device__ __forceinline__ uint32_t cluster_map(uint32_t saddr, uint32_t rank) {
-  uint32_t r;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(saddr), "r"(rank));
-  return r;
-}
-// 16 bytes into a CTA of the cluster, counted on that CTA's barrier
-__device__ __forceinline__ void st_async_v4(uint32_t addr, float4 v, uint32_t bar) {
-  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1,%2,%3,%4}, [%5];"
-               ::"r"(addr), "r"(__float_as_uint(v.x)), "r"(__float_as_uint(v.y)), "r"(__float_as_uint(v.z)), "r"(__float_as_uint(v.w)), "r"(bar)
-               : "memory");
-}
-__device__ __forceinline__ void st_cluster_v4(uint32_t addr, float4 v) {
-  asm volatile("st.shared::cluster.v4.f32 [%0], {%1,%2,%3,%4};" ::"r"(addr), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
-}
 __device__ __forceinline__ void cp_async16_zfill(void* dst, const void* src, bool valid) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(valid ? 16 : 0) : "memory");
 }
@@ -110,7 +96,7 @@ __global__ void __launch_bounds__(256) v_attn(const VattnParams P) {
       mbar_fence_init();
       mbar_expect_tx(xbar, 16 * RT * (HD + 4) * 4);
     }
-    asm volatile("barrier.cluster.arrive.release;" ::: "memory");                      // partials are sent once every neighbour is known to run
+    cluster_arrive();                      // partials are sent once every neighbour is known to run
   }
   auto issue = [&](int s) {
     if (s < nst) {
@@ -275,7 +261,7 @@ __global__ void __launch_bounds__(256) v_attn(const VattnParams P) {
   }
   __syncthreads();
   const int nown = RT * 16 / nspan;                              // this CTA finishes local rows rank, rank + nspan, ...
-  if (!alone) asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+  if (!alone) cluster_wait();
   // the position groups of the CTA meet first: a warp merges 2 RT rows (in place of position group 0's partials), so that the cluster
   // exchanges one partial per row and span
   auto finish = [&](int lr, float4 acc, float den) {             // local row lr, lane = 4 dims: normalise and write
@@ -323,11 +309,11 @@ __global__ void __launch_bounds__(256) v_attn(const VattnParams P) {
                      xb = cluster_map(smem_u32(xbar), to);
       const float4 md = make_float4(gm, den, 0.f, 0.f);
       if (ASYNC) {
-        if (lane < HD / 4) st_async_v4(a + lane * 16, acc, xb);
-        if (lane == 0) st_async_v4(a + HD * 4, md, xb);
+        if (lane < HD / 4) st_async(a + lane * 16, acc, xb);
+        if (lane == 0) st_async(a + HD * 4, md, xb);
       } else {
-        if (lane < HD / 4) st_cluster_v4(a + lane * 16, acc);
-        if (lane == 0) st_cluster_v4(a + HD * 4, md);
+        if (lane < HD / 4) st_cluster(a + lane * 16, acc);
+        if (lane == 0) st_cluster(a + HD * 4, md);
       }
     }
   }
@@ -339,8 +325,8 @@ __global__ void __launch_bounds__(256) v_attn(const VattnParams P) {
       const WaitCtl wc{P.status, s_abort, P.spin_limit};
       ok = __all_sync(0xffffffffu, mbar_wait<true>(xbar, 0, wc, W_FULL, 12));
     } else {
-      asm volatile("barrier.cluster.arrive.release;" ::: "memory");
-      asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+      cluster_arrive();
+      cluster_wait();
     }
     const float* in = reinterpret_cast<const float*>(va_sm + S::INBOX);
     for (int ri = warp; ok && ri < nown; ri += 8) {
@@ -372,8 +358,8 @@ __global__ void __launch_bounds__(256) v_attn(const VattnParams P) {
     // under way has landed, which takes microseconds.
     if (ASYNC) {
       __syncwarp();
-      asm volatile("barrier.cluster.arrive.relaxed;" ::: "memory");
-      asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+      cluster_arrive_relaxed();
+      cluster_wait();
       if (!ok && tid == 0)
 #pragma unroll 1
         for (int i = 0; i < 200 && !mbar_test(xbar, 0); i++) __nanosleep(1000);

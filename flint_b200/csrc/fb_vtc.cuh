@@ -334,22 +334,6 @@ __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, i
       "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
       ::"r"(smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(smem_u32(bar)) : "memory");
 }
-// cluster of the K splits: barrier over all threads of all its CTAs, and stores into a neighbour's shared memory
-__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
-__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
-__device__ __forceinline__ uint32_t map_rank(uint32_t saddr, uint32_t rank) {
-  uint32_t r;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(saddr), "r"(rank));
-  return r;
-}
-__device__ __forceinline__ void st_cluster_f32(uint32_t addr, float v) {
-  asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory");
-}
-// the same, counted on a barrier of that CTA
-__device__ __forceinline__ void st_async(uint32_t addr, uint32_t v, uint32_t bar) {
-  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::"r"(addr), "r"(v), "r"(bar) : "memory");
-}
-
 // Shared-memory plan (bytes). The raw ring keeps HBM busy; a stage of activations is a group's two 64-column tiles.
 // Tiles of 128 tokens, or of 192: an item's groups then take 4/3 of the time for 3/2 of the tokens, because dequantising a group and storing
 // it to tensor memory (which keeps the MMAs out meanwhile) is a cost per item. What is left of tensor memory allows two A stages, and none

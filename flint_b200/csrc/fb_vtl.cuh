@@ -289,9 +289,9 @@ __global__ void __launch_bounds__(kTlThreads, NT == 128 ? 1 : 2) v_gemm_tl(const
           for (int e = 0; e < 8; e++) {
             const int tk = half * HC + c + e;
             if (tk < push_end) {
-              const uint32_t to = map_rank(mine + (uint32_t)(tk & (TPR - 1)) * 512, tk >> lgT);
-              if (ASYNC) st_async(to, u[e], map_rank(smem_u32(xbar), tk >> lgT));
-              else st_cluster_f32(to, __uint_as_float(u[e]));
+              const uint32_t to = cluster_map(mine + (uint32_t)(tk & (TPR - 1)) * 512, tk >> lgT);
+              if (ASYNC) st_async(to, u[e], cluster_map(smem_u32(xbar), tk >> lgT));
+              else st_cluster(to, u[e]);
             }
           }
         }
@@ -354,7 +354,7 @@ __global__ void __launch_bounds__(kTlThreads, NT == 128 ? 1 : 2) v_gemm_tl(const
   }
   if (split && (ASYNC || warp < 6)) {                            // nobody leaves before its neighbours have sent what they will send
     __syncwarp();
-    if (ASYNC) asm volatile("barrier.cluster.arrive.relaxed;" ::: "memory");
+    if (ASYNC) cluster_arrive_relaxed();
     else cluster_arrive();
     cluster_wait();
   }
