@@ -84,7 +84,7 @@ __global__ void __launch_bounds__(1024) sample_rows(const SampleParams P) {
   const float* lg = P.logits + (long long)row * P.row_stride;
   const int per = (P.vocab + C - 1) / C, i0 = rank * per, i1 = min(P.vocab, i0 + per);
   const bool draw = P.temperature > 0.f, select = draw && P.top_k > 0 && P.top_k < P.vocab;
-  if (!select) cluster_arrive();               // the selection's own barriers come before its first remote read
+  if (!select) cluster_arrive();                  // the selection's own barriers come before its first remote read
   pdl_trigger();
   pdl_wait();
   float v[REG ? kSampleRegs : 1];
@@ -338,7 +338,7 @@ struct DLin {
 // read the weights once per 8 or 16 tokens and took 62 us for a 13 to 50 MB matrix at 32 tokens.)
 // A matrix whose rows give less than the GPU's worth of CTAs is also cut in K over a cluster of ks: the CTAs push their sums into the shared
 // memory of the one that finishes the token, which adds them in rank order. (With 16 warps and no split a 2560-row matrix ran on 80
-// SMs: window of 32 rows 177 -> 153 us, 48 rows of the 40-head shape 290 -> 258; single rows, three CTAs an SM, 125.1 without the split, 122.3.)
+// SMs: block over 32 rows 130.6 -> 105.9 us, 48 rows 202 -> 167; one row, three CTAs an SM, 77.2 without the split, 74.0 with it.)
 template <int NT, int MT, int MODE, bool CAT>
 __global__ void __launch_bounds__(kDraftWarps * 32, NT == 1 ? 3 : 2) d_gemm(const DLin P, int t0) {
   constexpr int WARPS = kDraftWarps;
@@ -378,7 +378,7 @@ __global__ void __launch_bounds__(kDraftWarps * 32, NT == 1 ? 3 : 2) d_gemm(cons
 #pragma unroll
         for (int h = 0; h < 2; h++) d[i][m][h] = ok ? __ldcs(wb[i] + (wr[m][h] + c * 4)) : make_uint4(0, 0, 0, 0);
   };
-  if (ks > 1) cluster_arrive();                   // remote stores wait for it below
+  if (ks > 1) cluster_arrive();                      // remote stores wait for it below
   const int c1 = rank * WARPS + warp, step = WARPS * ks;         // this warp's chunks
   pdl_begin(P.first && t0 == 0);
 #pragma unroll

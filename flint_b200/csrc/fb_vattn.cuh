@@ -96,7 +96,7 @@ __global__ void __launch_bounds__(256) v_attn(const VattnParams P) {
       mbar_fence_init();
       mbar_expect_tx(xbar, 16 * RT * (HD + 4) * 4);
     }
-    cluster_arrive();                      // partials are sent once every neighbour is known to run
+    cluster_arrive();                                            // partials are sent once every neighbour is known to run
   }
   auto issue = [&](int s) {
     if (s < nst) {

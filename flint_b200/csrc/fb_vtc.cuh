@@ -1,6 +1,6 @@
 // int4 GEMM of the M-token passes on the 5th-generation tensor cores (tcgen05): a weight row is read once and multiplied with a tile of
 // up to NT tokens. This file: the layout, the arithmetic, the epilogues, and the kernel for prompts (tiles of up to 128 or 192 tokens);
-// fb_vtl.cuh: the kernel for trees (one tile of 16 / 32 / 64).
+// fb_vtl.cuh: the kernel with one work item per CTA and K split over clusters, for trees (one tile of 16 / 32 / 64) and short prompts (tiles of 128).
 //
 // D[128 weight rows][NT tokens] (fp32, in TENSOR MEMORY) += A[128][128] * B[NT][128]^T per group of 128 columns, issued as
 // eight tcgen05.mma (K = 16 each) into ONE accumulator for the whole K range. A is the group's weights with their scale,
@@ -25,9 +25,9 @@
 // reads its words without bank conflicts.
 //
 // Work item = (token tile, row block), round-robin over persistent CTAs; two accumulators, so an item's epilogue overlaps the MMAs of
-// the next. Trees and short prompts split K over a CLUSTER instead (fb_vtl.cuh): every CTA sends the sums of a share of the tokens to each CTA of its cluster
-// through distributed shared memory, and each finishes its own tokens (sum in split order: deterministic), so the split costs no
-// round trip through global memory. Every wait is bounded.
+// the next. Trees and short prompts split K over a CLUSTER instead (fb_vtl.cuh): every CTA sends the sums of a share of the tokens to each CTA
+// of its cluster through distributed shared memory, and each finishes its own tokens (sum in split order: deterministic), so the split costs
+// no round trip through global memory. Every wait is bounded.
 #pragma once
 #include <cuda.h>
 
@@ -335,9 +335,9 @@ __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, i
       ::"r"(smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(smem_u32(bar)) : "memory");
 }
 // Shared-memory plan (bytes). The raw ring keeps HBM busy; a stage of activations is a group's two 64-column tiles.
-// Tiles of 128 tokens, or of 192: an item's groups then take 4/3 of the time for 3/2 of the tokens, because dequantising a group and storing
-// it to tensor memory (which keeps the MMAs out meanwhile) is a cost per item. What is left of tensor memory allows two A stages, and none
-// for zero points.
+// Tiles of 128 tokens, or of 192: an item's groups then take about 4/3 of the time for 3/2 of the tokens (680 cycles a group at 128, 950
+// at 192), because dequantising a group and storing it to tensor memory (which keeps the MMAs out meanwhile) is a cost per item. What is
+// left of tensor memory allows two A stages, and none for zero points.
 template <bool HZ, int NT_>
 struct VtcSmem {
   static constexpr int NT = NT_, REC = tc_rec_bytes(HZ);
@@ -419,7 +419,7 @@ struct TcFactors {
   __device__ __forceinline__ float x(int i) const { return __shfl_sync(0xffffffffu, i < 32 ? fx[0] : fx[1], i & 31); }
   __device__ __forceinline__ float a(int i) const { return __shfl_sync(0xffffffffu, i < 32 ? fa[0] : fa[1], i & 31); }
 };
-// The same from a table that the warp keeps in shared memory (prompts: 64 tokens an item; a shuffle per token and factor costs more)
+// The same from a table that the warp keeps in shared memory (prompts: up to 96 tokens of an item; a shuffle per token and factor costs more)
 struct TcFactorTable {
   float *fx, *fa;
   template <int EPI, int NF>
@@ -436,7 +436,8 @@ struct TcFactorTable {
 };
 // silu(g) = g / (1 + e^-g) with the exact division, the decode kernel's expression. (The approximate one, off by up to 2 ulp and zero where 1 + e^-g is
 // above 2^126, rounds bf16(silu(g) u) the other way at 386 of the 65280 x 128 pairs of a finite bf16 g and a mantissa of u, all but two of them
-// at g = -87.5 .. -88.5. Without its branches a prompt of 725 tokens of the 3B shape takes 6185 us instead of 6349, a 26-node tree 0.8 % less.)
+// at g = -87.5 .. -88.5. Without its branches a prompt of 725 tokens of the 3B shape takes 6185 us instead of 6349, engine calls back to back, a
+// 26-node tree 0.5 % less.)
 __device__ __forceinline__ float tc_silu(float g) { return g / (1.0f + __expf(-g)); }
 // v[e] = accumulator of (stream row srow, token t0 + e), the i0 + e-th of the warp's tokens; rf = the row's factor. The whole warp
 // calls this together: lanes 2i, 2i + 1 hold the two rows of a RoPE or gate/up pair.
@@ -491,7 +492,7 @@ __device__ __forceinline__ void vtc_epilogue(const VtcParams& P, int srow, int t
 // RESID and SWIGLU of 16 tokens by a warp (32 weight rows), through 1 KB of shared memory: the outputs of a token are adjacent there and
 // leave 16 bytes at a time (the residual comes the same way). Thread by thread they are 2-byte accesses, an address and a predicate per
 // value, and with them the epilogue of a 128 x 128 item took as long as its MMAs left idle: prompts of 100 / 250 / 725 tokens of the 3B
-// shape 3710 / 4465 / 7200 us, without any epilogue 3100 / 3630 / 6270.
+// shape 3710 / 4465 / 7200 us, without any epilogue 3100 / 3630 / 6270, staged (with the approximate silu) 3380 / 4062 / 6840.
 template <int EPI>
 struct TcStaged {
   static constexpr int NV = EPI == EPI_RESID ? 2 : 1;           // 16-byte vectors of a lane: 16 tokens x 64 bytes, or x 32 (SWIGLU halves the rows)

@@ -331,14 +331,13 @@ __global__ void __launch_bounds__(kTlThreads, NT == 128 ? 1 : 2) v_gemm_tl(const
             }
           }
         }
-      } else {
-        uint32_t u[(CH + 7) / 8][8];
-#pragma unroll
-        for (int c8 = 0; c8 < (CH + 7) / 8; c8++) tc_ld8(tlane + t0 + c8 * 8, u[c8]);
-        if (!STAGED && t0) pre.fetch(P, srow, th0 + t0, tlast);
+      } else if constexpr (!STAGED) {
+        uint32_t u[8];
+        tc_ld8(tlane + t0, u);
+        if (t0) pre.fetch(P, srow, th0 + t0, tlast);
         tc_ld_wait();
 #pragma unroll
-        for (int e = 0; e < CH; e++) v[e] = __uint_as_float(u[e >> 3][e & 7]);
+        for (int e = 0; e < CH; e++) v[e] = __uint_as_float(u[e]);
       }
       if constexpr (STAGED) {
         uint8_t* area = tsm + S::B + (warp - 6) * kTcEpiBytes;

@@ -117,17 +117,23 @@ def test_verify_token_tile_edges(M, asym):
 
 
 @pytest.mark.parametrize("asym", [False, True])
-@pytest.mark.parametrize("M,pos", [(1, 0), (3, 0), (40, 0), (70, 0), (300, 0), (3, 600), (16, 600)])
-def test_passes_that_give_up_leave_nothing_behind(M, pos, asym):
+@pytest.mark.parametrize("name,M,pos", [("tiny", 1, 0), ("tiny", 3, 0), ("tiny", 40, 0), ("tiny", 70, 0), ("tiny", 300, 0), ("tiny", 3, 600),
+                                        ("tiny", 16, 600), ("llama-1b-class", 26, 1000), ("llama-1b-class", 70, 0)])
+def test_passes_that_give_up_leave_nothing_behind(name, M, pos, asym):
     """With a wait limit of 0 a pass (one token: a decode step; up to 64 a tree pass; more a prompt pass) gives up at the first wait that is not
     satisfied already. Every launch ends, after its copies, MMAs and remote stores in flight (their wait has its own limit), the status says
     time-out or, if every wait happened to be satisfied, nothing, and the next clean pass gives the bits of the first. Behind 600 positions the
-    attention of 3 and 16 tokens runs as clusters of eight whose partials are asynchronous stores; at position 0 it is one CTA."""
-    cfg = ModelArgs.from_name("tiny")
-    if pos:
-        rt, _, nspan, _ = geometry.attn(M, pos, cfg.n_local_heads, cfg.n_head // cfg.n_local_heads, query()["sm_count"])
+    attention of 3 and 16 tokens runs as clusters of eight whose partials are asynchronous stores, at position 0 as one CTA; the larger model's
+    prompt runs as clusters of four that share K."""
+    cfg = ModelArgs.from_name(name)
+    if name != "tiny":
+        cfg.n_layer, cfg.vocab_size = 1, 512
+    sms = query()["sm_count"]
+    if pos == 600:
+        rt, _, nspan, _ = geometry.attn(M, pos, cfg.n_local_heads, cfg.n_head // cfg.n_local_heads, sms)
         assert (rt, nspan) == (1, 8)
-    eng = DecodeEngine(cfg, {k: v.cuda() for k, v in packing.synth_packed(cfg, 0, asym=asym).items()}, max_seq=640)
+    assert name == "tiny" or M < 64 or geometry.matrices(cfg, M, asym, sms)["qkv"][3] == 4
+    eng = DecodeEngine(cfg, {k: v.cuda() for k, v in packing.synth_packed(cfg, 0, asym=asym).items()}, max_seq=pos + 512)
     eng.kc.normal_()
     eng.vc.normal_()
     toks = torch.randint(0, cfg.vocab_size, (M,), generator=torch.Generator().manual_seed(M), dtype=torch.int32).cuda()
