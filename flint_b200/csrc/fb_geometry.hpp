@@ -1,7 +1,6 @@
 // Launch geometry as plain functions of the sizes: what fb_pass.cu and fb_spec.cu launch, and what a host-side test can ask. No CUDA here.
 // Times: engine calls back to back.
 #pragma once
-#include <stdint.h>
 
 namespace fb {
 
@@ -32,7 +31,8 @@ inline GemmGeometry gemm_geometry(int M, int rows, int k, bool zeros, int sms) {
   // The same for the tiles of a prompt, one CTA per SM, at least four groups each. Clusters of eight fit only in 120 of 148 SMs: at most four.
   // Not split: the persistent kernel, which overlaps an item's epilogue with the next item. All prompts in it / split: 70 / 100 / 128 / 180 / 250 / 300 / 384
   // tokens of the 3B shape 3214 / 3411 / 3579 / 3594 / 4153 / 4282 / 4603 -> 2592 / 2678 / 2773 / 3612 / 3936 / 4036 / 4303 us, 100 / 180 / 250 of the 8B shape
-  // 4300 / 4605 / 5569 -> 3239 / 4075 / 5023. Two and more tiles gain least just above 128 tokens: 0 to 2 % at 129 to 190 tokens of the 3B shapes.
+  // 4300 / 4605 / 5569 -> 3239 / 4075 / 5023. Two tiles gain least just above 128 tokens: -0.7 to +2 % at 129 to 190 tokens
+  // of the 3B shapes.
   while (g.nsplit < 4 && items * g.nsplit * 2 <= sms && groups / (g.nsplit * 2) >= 4) g.nsplit *= 2;
   if (g.nsplit > 1 || zeros) return g;                           // no 192-token tiles for zero points: tensor memory is full
   // 192-token tiles where they need fewer than 3/4 of the rounds of items that 128-token tiles need (a round of them takes about 4/3 of the time).
