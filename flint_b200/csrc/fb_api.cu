@@ -491,7 +491,7 @@ int fb_decode(fb_ctx* c, int32_t token, const int32_t* d_token, void* d_h, int32
   const unsigned span = (unsigned)(d.n_layer + 1) * 8u;
   if (c->tag_base > 0xffffffffu - 2 * span) c->tag_base = 8;      // tags never reach 0 (the value of fresh buffers)
   Q.tag_base = c->tag_base; Q.spin_limit = c->spin_limit;
-  Q.eps = d.rms_eps; Q.attn_scale = d.attn_scale; Q.resid = d.resid_mult; Q.emb_mult = d.emb_mult;
+  Q.eps = d.rms_eps; Q.attn_scale = d.attn_scale * 1.4426950408889634f; Q.resid = d.resid_mult; Q.emb_mult = d.emb_mult;
   Q.logits_scaling = d.logits_scaling; Q.prof = c->prof; Q.max_fly = (unsigned)fly_for(c, pos + 1); Q.lm_fly = c->max_fly ? Q.max_fly : 4u; Q.poll_words = c->poll_words;
   Q.tp_size = c->tp_size; Q.tp_rank = c->tp_rank; Q.vocab_base = c->vocab_base; Q.inbox = c->inbox; Q.ao_off = c->ao_off;
   for (int p = 0; p < c->tp_size; p++) {

@@ -277,7 +277,7 @@ struct AttnArgs {
   uint64_t* part_ll;        // [NKV][maxchunks][R*HD + 2R] tagged chunk partials (acc, then m, then d per head)
   uint32_t* ao_flags;       // [NKV * nchunks] arrival flags of the attention output, one per (kv head, chunk) CTA
   int nkv, pos, nchunks, maxchunks;
-  float scale;
+  float scale;              // times log2(e)
   uint32_t tag_in, tag_part, tag_out;
 };
 
@@ -421,14 +421,14 @@ __device__ __forceinline__ void attention_phase(const AttnArgs& a, uint8_t* scra
               }
             mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
             mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
-            const float corr = __expf(mrun[h] - mx);
+            const float corr = ex2(mrun[h] - mx);
             mrun[h] = mx;
             lrun[h] *= corr;
 #pragma unroll
             for (int j = 0; j < NTD; j++) { o[j][2 * h] *= corr; o[j][2 * h + 1] *= corr; }
 #pragma unroll
             for (int nt = 0; nt < 2; nt++) {                       // A columns 2t (+ 1) of positions 8 nt ..
-              float p0 = __expf(sc[nt][2 * h] - mx), p1 = __expf(sc[nt][2 * h + 1] - mx);
+              float p0 = ex2(sc[nt][2 * h] - mx), p1 = ex2(sc[nt][2 * h + 1] - mx);
               lrun[h] += p0 + p1;                                  // this lane's columns; the quad is summed at the end
 #pragma unroll
               for (int e = 0; e < 3; e++) {
@@ -489,7 +489,7 @@ __device__ __forceinline__ void attention_phase(const AttnArgs& a, uint8_t* scra
       float Dn = 0.f, A0 = 0.f, A1 = 0.f;
 #pragma unroll 2
       for (int w = 0; w < nact; w++) {
-        const float e = __expf(wm[w * R + r] - gm);
+        const float e = ex2(wm[w * R + r] - gm);
         const float2 v = *reinterpret_cast<const float2*>(wacc + (w * R + r) * HD + d);
         Dn += wd[w * R + r] * e;
         A0 += v.x * e;
@@ -547,7 +547,7 @@ __device__ __forceinline__ void attention_phase(const AttnArgs& a, uint8_t* scra
         float Dn = 0.f, A0 = 0.f, A1 = 0.f;
 #pragma unroll 4
         for (int cc = 0; cc < a.nchunks; cc++) {
-          const float e = __expf(pf[cc * per * 2 + r] - gm);
+          const float e = ex2(pf[cc * per * 2 + r] - gm);
           const float2 v = *reinterpret_cast<const float2*>(pf + (cc * per + R + tid_c) * 2);
           Dn += pf[cc * per * 2 + R + r] * e;
           A0 += v.x * e;
