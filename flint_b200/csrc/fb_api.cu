@@ -23,8 +23,8 @@ struct KernelEntry {
 
 // KD: model width, KO: attention output width of this rank, KF: FFN width of this rank
 #define FB_DECODE_ENTRY(KD, KO, KF, HD, R)                                                        \
-  {KD, KO, KF, HD, R, 0, (const void*)decode_mega2<KD, KO, KF, HD, R, false>, AttnCfg<HD>::NPS},   \
-  {KD, KO, KF, HD, R, 1, (const void*)decode_mega2<KD, KO, KF, HD, R, true>, AttnCfg<HD>::NPS}
+  {KD, KO, KF, HD, R, 0, (const void*)decode_mega2<KD, KO, KF, HD, R, false>, AttnCfg<HD, DecodePlan<KD, KO, KF>::STAGE>::NPS},   \
+  {KD, KO, KF, HD, R, 1, (const void*)decode_mega2<KD, KO, KF, HD, R, true>, AttnCfg<HD, DecodePlan<KD, KO, KF>::STAGE>::NPS}
 
 const KernelEntry kDecodeKernels[] = {
     FB_DECODE_ENTRY(512, 512, 1408, 64, 4),  // tiny test decoder
@@ -89,6 +89,7 @@ int chunks_for(const fb_ctx* c, int T) {
 //   1B-class   1.2: 394 / 391 / 387   1.4: 422 / 421 / 421   1.75: 441 / 437 / 436         8B-class   4.5: 1621 / 1667 / 1759
 // Up to 1.7 rings one copy gains on every shape, from 3.4 on it loses; in between the shapes differ by up to 1.8 % either way, and two copies
 // are never the best. The LM head has no hand-over to disturb: always 4.
+constexpr int64_t kRingBytes = 184320;      // a ring of eight 22.5 KB stages
 int fly_for(const fb_ctx* c, int T) {
   if (c->max_fly) return c->max_fly;
   const fb_model_desc& d = c->d;
@@ -96,7 +97,7 @@ int fly_for(const fb_ctx* c, int T) {
   const int64_t bytes = (int64_t)(d.n_head + 2 * d.n_kv_head) * HD * rec_bytes_of(d.dim, hz) + (int64_t)d.dim * rec_bytes_of(c->ko, hz) +
                         (int64_t)2 * d.ffn * rec_bytes_of(d.dim, hz) + (int64_t)d.dim * rec_bytes_of(d.ffn, hz) +
                         (int64_t)T * d.n_kv_head * HD * 4;
-  return bytes <= (int64_t)2 * kStages * kStageBytes * c->sm_count ? 1 : 4;
+  return bytes <= (int64_t)2 * kRingBytes * c->sm_count ? 1 : 4;
 }
 
 // every K the stand-alone entry points (re-layout, dequantise, GEMV) are built for
@@ -109,13 +110,13 @@ template <int K>
 int launch_gemv_k(bool hz, const GemvParams& p, int grid, cudaStream_t st) {
   cudaError_t e;
   if (hz) {
-    e = cudaFuncSetAttribute(gemv_stream<TCfg<K>, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
+    e = cudaFuncSetAttribute(gemv_stream<K, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
     if (e != cudaSuccess) return (int)e;
-    gemv_stream<TCfg<K>, true><<<grid, kThreads, kSmemBytes, st>>>(p);
+    gemv_stream<K, true><<<grid, kThreads, kSmemBytes, st>>>(p);
   } else {
-    e = cudaFuncSetAttribute(gemv_stream<TCfg<K>, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
+    e = cudaFuncSetAttribute(gemv_stream<K, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
     if (e != cudaSuccess) return (int)e;
-    gemv_stream<TCfg<K>, false><<<grid, kThreads, kSmemBytes, st>>>(p);
+    gemv_stream<K, false><<<grid, kThreads, kSmemBytes, st>>>(p);
   }
   return (int)cudaGetLastError();
 }
@@ -258,13 +259,11 @@ int fb_ctx_create_tp(const fb_model_desc* desc, int device, int32_t tp_rank, int
     if (e == cudaSuccess) A(cudaMemset(*ll_ptrs[i], 0, 8 * ll_words[i] + 16));
   }
   if (e == cudaSuccess) e = pass_alloc(c);
-  A(dmalloc(&c->flags, 3 * 256 * 4));
-  if (e == cudaSuccess) A(cudaMemset(c->flags, 0, 3 * 256 * 4));
   if (c->sm_count > 256) e = cudaErrorInvalidValue;
   {  // rows of the residual stream one CTA owns (whole tiles of the O and the down matrix)
     const int uo = tile_rt(ko) > tile_rt(d.ffn) ? tile_rt(ko) : tile_rt(d.ffn);
     const int units = (d.dim + uo - 1) / uo;
-    if (((units + c->sm_count - 1) / c->sm_count + 1) * uo > kMaxOwnRows || (2 * d.ffn) % 4) e = cudaErrorInvalidValue;
+    if ((units + c->sm_count - 1) / c->sm_count * uo > kMaxOwnRows || (2 * d.ffn) % 4) e = cudaErrorInvalidValue;
   }
   if (e == cudaSuccess) {
     float invf[128];
@@ -287,7 +286,7 @@ int fb_ctx_destroy(fb_ctx* c) {
   for (int p = 0; p < 8; p++)
     if (c->peers_open[p] && c->peer_inbox[p]) cudaIpcCloseMemHandle(c->peer_inbox[p]);
   void* ptrs[] = {c->w_qkv, c->w_o, c->w_gu, c->w_d, c->w_lm, c->invf,
-                  c->status, c->h_ll, c->q_ll, c->k_ll, c->v_ll, c->ao_ll, c->act_ll, c->cand_ll, c->flags,
+                  c->status, c->h_ll, c->q_ll, c->k_ll, c->v_ll, c->ao_ll, c->act_ll, c->cand_ll,
                   c->part_ll, c->inbox};
   for (void* p : ptrs)
     if (p) cudaFree(p);
@@ -300,8 +299,8 @@ int fb_set_option(fb_ctx* c, int32_t what, int64_t value) {
   if (!c) return FB_ERR_ARG;
   if (what == 0) { c->spin_limit = (unsigned)value; return FB_OK; }       // spin limit of every device-side wait
   if (what == 1) { c->force_chunks = (int)value; return FB_OK; }          // attention chunks per kv head (0 = auto)
-  if (what == 5) { c->poll_words = value != 0; return FB_OK; }
-  if (what == 8) return value < 0 || value > 2 ? FB_ERR_ARG : FB_OK;     // 7, 8: accepted, without effect: one implementation
+  if (what == 5) return FB_OK;                                             // 5, 7, 8: accepted, without effect: one implementation
+  if (what == 8) return value < 0 || value > 2 ? FB_ERR_ARG : FB_OK;
   if (what == 7) return value < 0 || value > 4 ? FB_ERR_ARG : FB_OK;
   if (what == 4) { if (value < 1 || value > kStages / 2) return FB_ERR_ARG; c->max_fly = (int)value; return FB_OK; }
   if (what == 2) { c->prof = (long long*)(uintptr_t)value; return FB_OK; } // device int64[sm_count * n_layer * 16] phase stamps (ns), 0 = off
@@ -481,7 +480,6 @@ int fb_decode(fb_ctx* c, int32_t token, const int32_t* d_token, void* d_h, int32
   Q.kc = (uint16_t*)c->kc; Q.vc = (uint16_t*)c->vc;
   Q.kmap = c->kmap; Q.vmap = c->vmap;
   Q.h_ll = c->h_ll; Q.q_ll = c->q_ll; Q.k_ll = c->k_ll; Q.v_ll = c->v_ll; Q.ao_ll = c->ao_ll; Q.act_ll = c->act_ll;
-  Q.h_flags = c->flags; Q.act_flags = c->flags + 256; Q.ao_flags = c->flags + 512;
   Q.cand_ll = c->cand_ll; Q.part_ll = c->part_ll; Q.status = c->status;
   Q.d_token = d_token; Q.d_h = (uint16_t*)d_h; Q.d_logits = d_logits; Q.d_next = d_next;
   Q.token = token; Q.pos = pos; Q.max_seq = c->max_seq;
@@ -492,7 +490,7 @@ int fb_decode(fb_ctx* c, int32_t token, const int32_t* d_token, void* d_h, int32
   if (c->tag_base > 0xffffffffu - 2 * span) c->tag_base = 8;      // tags never reach 0 (the value of fresh buffers)
   Q.tag_base = c->tag_base; Q.spin_limit = c->spin_limit;
   Q.eps = d.rms_eps; Q.attn_scale = d.attn_scale * 1.4426950408889634f; Q.resid = d.resid_mult; Q.emb_mult = d.emb_mult;
-  Q.logits_scaling = d.logits_scaling; Q.prof = c->prof; Q.max_fly = (unsigned)fly_for(c, pos + 1); Q.lm_fly = c->max_fly ? Q.max_fly : 4u; Q.poll_words = c->poll_words;
+  Q.logits_scaling = d.logits_scaling; Q.prof = c->prof; Q.max_fly = (unsigned)fly_for(c, pos + 1); Q.lm_fly = c->max_fly ? Q.max_fly : 4u;
   Q.tp_size = c->tp_size; Q.tp_rank = c->tp_rank; Q.vocab_base = c->vocab_base; Q.inbox = c->inbox; Q.ao_off = c->ao_off;
   for (int p = 0; p < c->tp_size; p++) {
     if (!c->peer_inbox[p]) return FB_ERR_STATE;       /* fb_tp_connect has not been called */

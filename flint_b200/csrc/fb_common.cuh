@@ -1,6 +1,6 @@
 // Shared device-side building blocks of the sm_100a decode path: PTX wrappers (mbarrier, 1-D bulk copies,
 // coherent loads), bounded waits that report instead of hanging, the tiled streaming weight layout and the int4 tile x
-// vector product (fp16 mma.sync) that every GEMV phase uses.
+// vector product (integer mma.sync) that every GEMV phase uses.
 #pragma once
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
@@ -16,11 +16,10 @@ namespace fb {
 constexpr int kConsumerWarps = FB_CW;
 constexpr int kConsumerThreads = kConsumerWarps * 32;
 constexpr int kThreads = kConsumerThreads + 32;    // + one producer warp (lane 0 issues the bulk copies)
-constexpr int kStages = 8;                         // ring depth: 8 x 22.5 KB = 180 KB of weights in flight per SM
-constexpr int kStageBytes = 23040;                 // a stage holds whole tiles (4 tiles of K = 2560, 1 of K = 8192 ...)
-constexpr int kScratchBytes = 40960;               // activations of the phase (<= 14336 fp16), then attention scratch
-constexpr int kTailBytes = 6144;                   // mbarriers, flags, reductions, slice partials, owned rows, group factors
-constexpr int kSmemBytes = kStages * kStageBytes + kScratchBytes + kTailBytes;
+constexpr int kStages = 8;                         // ring depth
+constexpr int kTailBytes = 6144;                   // mbarriers, flags, reductions, unit table, slice partials, owned rows, group factors
+constexpr int kSmemBytes = 231424;                 // 226 KB: with the static variables what a CTA may have
+constexpr int kAttnScratch = 40960;                // attention scratch, which shares its place with the activations
 constexpr int kMaxOwnRows = 64;                    // rows of the residual stream one CTA may own
 constexpr int kMaxGroups = 112;                    // K <= 14336
 
@@ -207,41 +206,57 @@ __device__ __forceinline__ bool mbar_wait_far(uint64_t* b, uint32_t parity, cons
 }
 
 // ------------------------------------------------------------------------------------------------ streaming layout
-// Weights are stored as TILES of RT consecutive stream rows x all K columns, laid out for the tensor pipe: a tile is
-// a sequence of "steps", 128 bytes each = one 32-bit word per lane of a warp, and a step is exactly the A operand of one
-// mma.m16n8k16. Batch-1 decode has no second matrix dimension to fill the 16 MMA rows with, so the 16 rows of a step
-// are RT weight rows x NJ = 16/RT column ranges of K/NJ columns each: MMA row i = (tile row i % RT, range i / RT), and
-// column n of the B operand carries the activations of range n. Output C[i][i / RT] is then the partial dot product
-// of tile row i % RT over range i / RT; the other columns are ignored.
+// Weights are stored as TILES of RT consecutive stream rows x all K columns, cut into CHUNKS of KC columns (tiles of long rows do not fit a ring stage), and
+// a chunk is laid out for the tensor pipe. Batch-1 decode has no second matrix dimension to fill the 16 rows of an mma.m16n8k32 with, so
+// these are RT weight rows x NJ = 16/RT column ranges of KC/NJ columns each: MMA row i = (tile row i % RT, range i / RT).
 //
-// Inside a word the eight nibbles are placed so that no arithmetic is needed to turn them into fp16 operands:
-//   w & 0x000F000F        -> (nib0, nib4) as fp16 SUBNORMALS nib * 2^-24   = A[g  ][2t], A[g  ][2t+1]
-//   w & 0x00F000F0        -> (nib1, nib5) as 16 * nib * 2^-24              = A[g+8][2t], A[g+8][2t+1]
-//   (w >> 8) & the same   -> (nib2, nib6), (nib3, nib7)                    = A[g][2t+8..], A[g+8][2t+8..]
-// for lane (g = lane / 4, t = lane % 4). The tensor pipe multiplies subnormals exactly, so C = 2^-24 * sum nib * x for
-// the first eight MMA rows and 16 times that for the last eight; the per-group flush folds 2^24 (or 2^20), the group's
-// bf16 scale and the activations' power-of-two factor into one fp32 multiply, and removes the nibble offset with
-// -8 * scale * sum(x) (and adds zero * sum(x) for the asymmetric layout). Products and the subtraction are exact in
-// fp32 terms: the arithmetic is the reference's sum (nib - 8) * s * x with a different summation order.
+// The product is exact integer arithmetic: weights as s8 16 (nib - 8), activations as s8 digits. A group of 128 activations is brought by a power of two to
+// [2^28, 2^29) and rounded to integers (exact for every bf16 element down to 2^-21 of the group's largest magnitude, off by at most 2^-29 of
+// that magnitude below), and four signed digits of a number, of weights 2^23, 2^15, 2^8 and 1, go to four COLUMNS of the B operand, which a
+// matrix-vector product leaves idle anyway: with two ranges all eight are in use. Lane t of a quad holds columns 2t and 2t + 1, two digits of one range.
+// The group's flush joins them and multiplies by the power of two and the bf16 scale in fp32: the reference's sum (nib - 8) * s * x in
+// another order of summation.
 //
-// Steps are stored four to a block: block bq holds, for every lane, the words of steps 4bq..4bq+3 as one 16-byte
-// vector. Range j walks its columns with its steps rotated inside each block (local step (s & ~3) | ((s + j) & 3)),
-// which spreads the ranges' activation loads over different shared-memory banks. After the nibble area come the
-// tile's scales as bf16 [K/128][RT], then (asymmetric layout) the zeros in the same shape.
-__host__ __device__ constexpr int tile_rt(int k) {
-  const int g = k / 128;
-  if (g % 4 == 0 && 4 * (k / 2 + g * 4) <= 23040) return 4;
-  if (g % 8 == 0) return 2;
-  if (g % 2 == 0) return 8;
-  return 16;
+// A block of 64 columns of every range is 512 bytes: 16 per lane (g = lane / 4, t = lane % 4). Byte b of word i holds columns 16t + 4i + b of MMA row g (high
+// nibble) and row g + 8 (low nibble), as nib - 8 in two's complement: words 2s and 2s + 1 are the A operand of MMA step s after w & 0xF0F0F0F0 and
+// (w << 4) & 0xF0F0F0F0. The columns of a step are not the ones that the instruction numbers so, but B is read in the same order. After a chunk's
+// nibble area come its scales as bf16 [KC/128][RT], then (asymmetric layout) its zeros in the same shape.
+//
+// This replaced fp16 operands (m16n8k16, nibbles as fp16 subnormals, four ranges of four rows): five ALU operations and one MMA per eight weights of a lane
+// against three and a half, half the shared-memory reads of activations, and a flush per group of eight rows instead of four. (e4m3 operands need
+// the same operations, but sm_100a runs mma.sync on them at less than half of the integer rate: 7.2 against 3.0 cycles an instruction and SM, operands
+// from shared memory.) Gate/up of the 3B / 1B / 8B-class shapes, 16384 x 2560, 16384 x 2048, 28672 x 4096, in the decode kernel: 4.4 / 3.9 / 11.8 us before,
+// 2.5 / 2.2 / 7.3 now; the stand-alone product over 400000 x 2560 5.3 -> 5.8 TB/s. Against a 64-bit sum the logits of two layers are closer than
+// before (mean distance in units of the test's tolerance: 0.61 -> 0.35 at 3B, 0.50 -> 0.15 at 1B, 0.66 -> 0.51 at 8B): the products round only in the flush.
+__host__ __device__ constexpr int tile_rt(int k) { return (k / 128) % 2 == 0 ? 8 : 16; }
+__host__ __device__ constexpr int chunk_bytes(int rt, int kc, int has_zeros) { return rt * (kc / 2 + (kc / 128) * 2 * (has_zeros ? 2 : 1)); }
+constexpr int kChunkFit = 20992;                   // the smallest ring stage (SmemPlan of K = 14336)
+// Columns of a chunk: all of K where that fits a stage; else 4096 or 2048 where they divide K (8192 in 2, 14336 in 7: with 28 rows a CTA two chunks a warp), else
+// the longest whole number of groups per range that divides K and fits.
+__host__ __device__ constexpr int chunk_k(int k) {
+  const int rt = tile_rt(k), unit = 128 * (16 / rt);
+  if (chunk_bytes(rt, k, 1) <= kChunkFit) return k;
+  if (k % 4096 == 0) return 4096;
+  if (k % 2048 == 0) return 2048;
+  int best = unit;
+  for (int c = unit; c < k; c += unit)
+    if (k % c == 0 && chunk_bytes(rt, c, 1) <= kChunkFit) best = c;
+  return best;
 }
-__host__ __device__ constexpr int tile_bytes(int k, int has_zeros) {
-  return tile_rt(k) * (k / 2 + (k / 128) * 2 * (has_zeros ? 2 : 1));
-}
+__host__ __device__ constexpr int tile_bytes(int k, int has_zeros) { return k / chunk_k(k) * chunk_bytes(tile_rt(k), chunk_k(k), has_zeros); }
 // bytes per stream row (a tile is RT of these; only whole tiles are addressable)
 __host__ __device__ constexpr int rec_bytes_of(int k, int has_zeros) { return tile_bytes(k, has_zeros) / tile_rt(k); }
 __host__ __device__ constexpr int pad_rows(int rows, int k) { return (rows + tile_rt(k) - 1) / tile_rt(k) * tile_rt(k); }
-__host__ __device__ __forceinline__ int local_step(int s, int j) { return (s & ~3) | ((s + j) & 3); }
+
+// Shared memory of a kernel whose longest K is MAXK: the tail (fixed offsets), the activations (4 bytes each) or the attention's scratch, and what is left
+// in eight ring stages.
+template <int MAXK>
+struct SmemPlan {
+  static constexpr int SCRATCH = 4 * MAXK > kAttnScratch ? 4 * MAXK : kAttnScratch;
+  static constexpr int RING = kTailBytes + SCRATCH;
+  static constexpr int STAGE = (kSmemBytes - RING) / kStages / 128 * 128;
+  static_assert(MAXK / 128 <= 112, "group factors");
+};
 
 // stream row j of a matrix holds source row perm(j)
 //   order 0: identity
@@ -258,52 +273,86 @@ __host__ __device__ __forceinline__ int perm_row(int j, int order, int arg, int 
   return j;
 }
 
-// Compile-time schedule of one matrix shape. KS > 1 cuts a tile's blocks into KS slices that different warps take
-// (phases that give a CTA only a handful of tiles); TPS tiles travel in one bulk copy / ring stage.
-template <int K_, int KS_ = 1, int TPS_ = 0>
+constexpr int kPartBytes = 1024;                   // partial sums of units: [32][8 rows] or [16][16 rows]
+// Compile-time schedule of one matrix shape over ring stages of STAGE bytes: CPS chunks travel in one bulk copy. A chunk is RPC rounds (one group of every
+// range, two blocks); the warps of a CTA that has few chunks share one by rounds (unit_entry).
+template <int K_, int STAGE>
 struct TCfg {
-  static constexpr int K = K_, KS = KS_, RT = tile_rt(K_);
-  static constexpr int NJ = 16 / RT, G = K / 128, RG = G / NJ, BQ = RG * 2;     // rounds (8 steps) per range; 4-step blocks
-  static constexpr int NB = BQ / KS;                                             // blocks per slice
-  static constexpr int NIB = RT * K / 2;
-  static constexpr int tile(bool hz) { return tile_bytes(K_, hz); }
-  static constexpr int TPS_FIT = kStageBytes / tile_bytes(K_, 1);
-  static constexpr int TPS = TPS_ > 0 ? TPS_ : (KS_ > 1 ? (TPS_FIT > 2 ? 2 : TPS_FIT) : (TPS_FIT > 8 ? 8 : TPS_FIT));
-  static constexpr int TILE_ROWS = TPS * RT;                                      // rows per ring stage
-  static_assert(K % 128 == 0 && G % NJ == 0 && BQ % KS == 0, "columns must split into whole groups per range and slice");
-  static_assert(TPS >= 1 && TPS * tile_bytes(K_, 1) <= kStageBytes, "a stage holds whole tiles");
-  static_assert(KS == 1 || (RT <= 4 && TPS <= 2 && KS <= 4), "slice partials: 4 rows x 4 slices x 2 tiles per stage");
-  static_assert(tile_bytes(K_, 0) % 16 == 0 && tile_bytes(K_, 1) % 16 == 0, "bulk copies move multiples of 16 bytes");
+  static constexpr int K = K_, RT = tile_rt(K_), NJ = 16 / RT, KC = chunk_k(K_), NC = K / KC;
+  static constexpr int G = KC / 128, RPC = G / NJ;
+  static constexpr int NIB = RT * KC / 2;
+  static constexpr int chunk(bool hz) { return chunk_bytes(RT, KC, hz); }
+  static constexpr int FIT = STAGE / chunk_bytes(RT, KC, 1), CPS = NC > 1 ? (RT == 8 && FIT > 1 ? 2 : 1) : (FIT > 8 ? 8 : FIT);
+  static_assert(K % KC == 0 && G % NJ == 0, "columns must split into chunks and whole groups per range");
+  static_assert(CPS >= 1 && CPS * chunk_bytes(RT, KC, 1) <= STAGE, "a stage holds whole chunks");
+  // partial sums are kept in a ring of SLOTS units: the oldest unfinished chunk holds its stage, so younger ones are at most a ring ahead
+  static constexpr int SLOTS = kPartBytes / (RT * 4);
+  static_assert(FIT >= 1 && (NC == 1 || (kStages + 1) * CPS + NC <= SLOTS) && SLOTS >= kConsumerWarps, "partial sums");
+  static_assert(chunk_bytes(RT, KC, 0) % 16 == 0, "bulk copies move multiples of 16 bytes");
 };
+// Which chunks of a phase a warp takes: chunk, first round, rounds, slices per chunk, a byte each. Few chunks: each is cut in `ks` slices so that as
+// many warps as possible have one; else the warps take whole chunks w, w + 14, ...
+__device__ __forceinline__ uint32_t unit_entry(int nch, int rpc, int warp) {
+  int ks = nch > 0 && nch <= kConsumerWarps / 2 ? kConsumerWarps / nch : 1;
+  if (ks > rpc) ks = rpc;
+  const int ci = warp / ks, sl = warp - ci * ks, r0 = rpc * sl / ks, r1 = rpc * (sl + 1) / ks;
+  return (uint32_t)(ci < nch ? ci : 255) | (uint32_t)r0 << 8 | (uint32_t)(r1 - r0) << 16 | (uint32_t)ks << 24;
+}
 
-// activations of the current phase in shared memory: fp16 in B-operand order (inside every 16 columns the halves are
-// [2t, 2t+1, 2t+8, 2t+9] for t = 0..3) and, per group of 128 columns, {2^24 / m, 2^20 / m, -8 * sum x, sum x} where m is
-// the power of two the group was multiplied by before the conversion to fp16
+// activations of the current phase in shared memory: per 64 columns their lowest digits [64], then the next ones, in column order; and per group of
+// 128 columns {2^-e, sum x} for the lanes that hold the two low digits, {2^15 2^-e, 0} for those of the two high ones (sum x: asymmetric layout only)
 struct XStage {
-  const __half* xh;
+  const uint8_t* x8;
   const float4* xf;
 };
 
-// Convert 4 consecutive bf16 activations (elements 4*lane .. 4*lane+3 of one group of 128, one group per warp) and
-// store them; lane 0 also writes the group's factors. The whole warp must call this together.
-__device__ __forceinline__ void stage_group_fp16(uint32_t p01, uint32_t p23, __half* xh_group, float4* xf_group, int lane) {
-  const uint32_t e0 = (p01 >> 7) & 255, e1 = (p01 >> 23) & 255, e2 = (p23 >> 7) & 255, e3 = (p23 >> 23) & 255;
-  const uint32_t em = __reduce_max_sync(0xffffffffu, max(max(e0, e1), max(e2, e3)));
-  uint32_t mf = 268u - em;                    // exponent field of m: the group's largest magnitude lands in [2^14, 2^15)
-  mf = mf > 253u ? 253u : (mf < 24u ? 24u : mf);
-  const float mult = __uint_as_float(mf << 23), inv = __uint_as_float((254u - mf) << 23);
-  const float f0 = bflo(p01), f1 = bfhi(p01), f2 = bflo(p23), f3 = bfhi(p23);
-  const __half2 h01 = __floats2half2_rn(f0 * mult, f1 * mult), h23 = __floats2half2_rn(f2 * mult, f3 * mult);
-  float sx = (f0 + f1) + (f2 + f3);
+// Convert bf16 activations for the tensor pipe: v[k] holds elements 4 lane .. 4 lane + 3 of group first + k * step, which a warp converts together if it is
+// below `groups`. Every CTA converts the whole vector in every phase, and the phase waits for it: no branch but the stores' predicates, so that
+// the groups of a thread run side by side. The two halves of a number come out of the mantissas of sums with 1.5 * 2^23 + 128 (the 128 makes the
+// low byte's digit signed), on the FMA pipe.
+template <bool SUM, int N>
+__device__ __forceinline__ void stage_groups(const uint2 (&v)[N], int first, int step, int groups, uint8_t* x8, float4* xf, int lane) {
+  uint32_t em[N];
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) sx += __shfl_xor_sync(0xffffffffu, sx, o);
-  // element c = 4 * (lane % 4) + e of its 16-block: the pair (c, c+1) goes to half2 slot 2 * ((c % 8) / 2) + c / 8
-  const int c = (lane & 3) * 4;
-  __half2* dst = reinterpret_cast<__half2*>(xh_group + (lane >> 2) * 16);
-  __syncwarp();                               // in-place use: every lane has read its source words
-  dst[((c % 8) / 2) * 2 + (c / 8)] = h01;
-  dst[(((c + 2) % 8) / 2) * 2 + ((c + 2) / 8)] = h23;
-  if (lane == 0) *xf_group = make_float4(inv * 16777216.f, inv * 1048576.f, -8.f * sx, sx);
+  for (int k = 0; k < N; k++) {
+    const uint32_t mm = __vmaxu2(v[k].x & 0x7fff7fffu, v[k].y & 0x7fff7fffu);
+    em[k] = __reduce_max_sync(0xffffffffu, max(mm >> 16, mm & 0xffffu)) >> 7;
+  }
+  float sx[N];
+#pragma unroll
+  for (int k = 0; k < N; k++) sx[k] = SUM ? (bflo(v[k].x) + bfhi(v[k].x)) + (bflo(v[k].y) + bfhi(v[k].y)) : 0.f;
+  if (SUM)
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+      for (int k = 0; k < N; k++) sx[k] += __shfl_xor_sync(0xffffffffu, sx[k], o);
+#pragma unroll
+  for (int k = 0; k < N; k++) {
+    const uint32_t mf = min(267u - em[k], 253u);                // exponent field of the multiplier: largest magnitude in [2^13, 2^14)
+    const float mult = __uint_as_float(mf << 23), magic = 12583040.f;
+    const float x[4] = {bflo(v[k].x), bfhi(v[k].x), bflo(v[k].y), bfhi(v[k].y)};
+    uint32_t hi[4], lo[4];
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      const float h = fmaf(x[i], mult, magic);                  // the nearest integer, in the low bits
+      const float r = fmaf(x[i], mult, magic - h);              // exact: what is left, |r| <= 1/2
+      hi[i] = __float_as_uint(h);
+      lo[i] = __float_as_uint(fmaf(r, 32768.f, magic));
+    }
+    // 4 x 4 bytes transposed: a word holds one digit of the four elements
+    const uint32_t a = __byte_perm(lo[0], lo[1], 0x5140), b = __byte_perm(lo[2], lo[3], 0x5140), c = __byte_perm(hi[0], hi[1], 0x5140),
+                   d = __byte_perm(hi[2], hi[3], 0x5140);
+    const int grp = first + k * step;
+    const float inv = em[k] == 255u ? __uint_as_float(0x7fc00000u) : __uint_as_float((254u - mf) << 23);      // infinities and NaN: the group's products are NaN
+    if (grp < groups) {
+      uint32_t* dst = reinterpret_cast<uint32_t*>(x8 + grp * 512 + (lane >> 4) * 256) + (lane & 15);
+      dst[0] = __byte_perm(a, b, 0x5410) ^ 0x80808080u;
+      dst[16] = __byte_perm(a, b, 0x7632);
+      dst[32] = __byte_perm(c, d, 0x5410) ^ 0x80808080u;
+      dst[48] = __byte_perm(c, d, 0x7632);
+      if (lane == 0) xf[grp] = make_float4(inv * 0.0625f * (1.f / 32768.f), sx[k], inv * 0.0625f, 0.f);
+    }
+  }
 }
 
 // ------------------------------------------------------------------------------------------------ tile x vector
@@ -312,14 +361,9 @@ __device__ __forceinline__ uint4 lds128(uint32_t a) {
   asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a));
   return v;
 }
-__device__ __forceinline__ float4 lds128f(uint32_t a) {
-  float4 v;
-  asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a));
-  return v;
-}
-__device__ __forceinline__ uint2 lds64(uint32_t a) {
-  uint2 v;
-  asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(a));
+__device__ __forceinline__ float2 lds64f(uint32_t a) {
+  float2 v;
+  asm volatile("ld.shared.v2.f32 {%0,%1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(a));
   return v;
 }
 __device__ __forceinline__ float lds_bf16(uint32_t a) {
@@ -327,15 +371,10 @@ __device__ __forceinline__ float lds_bf16(uint32_t a) {
   asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(a));
   return __uint_as_float(((uint32_t)v) << 16);
 }
-__device__ __forceinline__ void mma_f16(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+__device__ __forceinline__ void mma_s8(int (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+               : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3])
                : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-__device__ __forceinline__ void mma_f16_first(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
-               : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3])
-               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.f));
 }
 
 // Programmatic dependent launch: every kernel of the verify chain is launched with the stream-serialisation attribute.
@@ -391,219 +430,67 @@ __device__ __forceinline__ float ex2(float x) {
 }
 __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) { return (uint32_t)f2bf(lo) | ((uint32_t)f2bf(hi) << 16); }
 
-// Fully unrolled form of the tile product (same contract as tile_dot_rolled below): every block's flags and offsets
-// are compile-time constants. Fastest per tile (5.3 TB/s on the stand-alone GEMV against 4.7 for the rolled form), but
-// ~10 KB of straight-line code per call site.
+// Rounds [r0, r0 + n) of a chunk (its `ci`-th of the tile) against the staged activations. RT 8: on return every lane of quad g holds the total of tile
+// row g in out_lo. RT 16: row g in out_lo and row g + 8 in out_hi.
+// The loop is ROLLED (two rounds per iteration): the decode kernel's per-layer code does not fit the instruction cache, and every phase of every
+// layer runs through its own copy of this one. Bound by shared-memory reads (16 of 64 cycles a round of 2048 weights per SM) and the ALU.
 template <class C, bool HZ>
-__device__ __forceinline__ void tile_dot_unrolled(const uint8_t* tile, int slice, const XStage& x, int lane, float& out_lo,
-                                         float& out_hi) {
-  constexpr int RT = C::RT, NB = C::NB;
+__device__ __forceinline__ void chunk_dot(const uint8_t* chunk, int ci, int r0, int n, const XStage& x, int lane, float& out_lo, float& out_hi) {
+  constexpr int RT = C::RT, NJ = C::NJ;
+  constexpr uint32_t META = RT * 2;                              // bytes of a group's scales
   const int g = lane >> 2, t = lane & 3;
-  const int jl = g / RT, jh = (g + 8) / RT, jb = g % C::NJ;
-  const int rl = g % RT, rh = (g + 8) % RT;
-  const int b0 = C::KS == 1 ? 0 : slice * NB;
-  const uint32_t tb = smem_u32(tile);
-  const uint32_t wa = tb + (uint32_t)(b0 * 32 + lane) * 16;
-  const uint32_t xbase = smem_u32(x.xh) + (uint32_t)(jb * (C::K / C::NJ) + 4 * t) * 2 + (uint32_t)b0 * 128;
-  uint32_t xa[4];
+  const int j = NJ == 2 ? t >> 1 : 0;                            // the range of this lane's accumulator columns
+  const bool up = NJ == 2 && t >= 2;                             // ... and with two ranges the MMA rows: g or g + 8
+  const uint32_t tb = smem_u32(chunk);
+  uint32_t wa = tb + (uint32_t)(r0 * 64 + lane) * 16;
+  // B: lane (g, t) reads column g, digit g & 3 of range g >> 2 (one range: again). Eight lanes read 128 bytes in a row: no bank twice.
+  uint32_t xa = smem_u32(x.x8) + (uint32_t)(ci * C::KC + (NJ == 2 ? (g >> 2) * (C::KC / NJ) : 0)) * 4 + (uint32_t)(r0 * 512 + (g & 3) * 64 + 16 * t);
+  uint32_t ma = tb + C::NIB + (uint32_t)(j * C::RPC + r0) * META + (uint32_t)g * 2;
+  uint32_t fa = smem_u32(x.xf) + (uint32_t)(ci * C::G + j * C::RPC + r0) * 16 + (t & 1) * 8;
+  float ct = 0.f, ct2 = 0.f;
+  uint4 w0 = lds128(wa), w1 = lds128(wa + 512), x0 = lds128(xa), x1 = lds128(xa + 256);
+  auto round = [&](bool more) {
+    const uint32_t wstep = more ? 1024u : 0u, xstep = more ? 512u : 0u;      // the last round reads its own operands again
+    wa += wstep;
+    xa += xstep;
+    const uint4 wn0 = lds128(wa), wn1 = lds128(wa + 512), xn0 = lds128(xa), xn1 = lds128(xa + 256);
+    const float2 F = lds64f(fa);
+    const float s = lds_bf16(ma);
+    int c[4] = {0, 0, 0, 0};
+    const uint32_t ws[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w}, xs[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
 #pragma unroll
-  for (int i = 0; i < 4; i++) xa[i] = xbase + 32 * ((i + jb) & 3);
-  const uint32_t ml = tb + C::NIB + (uint32_t)(jl * C::RG * RT + rl) * 2;
-  const uint32_t mh = tb + C::NIB + (uint32_t)(jh * C::RG * RT + rh) * 2;
-  const uint32_t fl = smem_u32(x.xf) + (uint32_t)(jl * C::RG) * 16, fh = smem_u32(x.xf) + (uint32_t)(jh * C::RG) * 16;
-  float ct[4] = {0.f, 0.f, 0.f, 0.f}, cg[4];
-  float zl = 0.f, zh = 0.f;
-  uint4 w4 = lds128(wa);
-  uint2 xb[4];
-#pragma unroll
-  for (int i = 0; i < 4; i++) xb[i] = lds64(xa[i]);
-  const bool odd0 = (NB % 2 == 0) ? false : (b0 & 1);           // the slice starts in the middle of a round
-#pragma unroll
-  for (int bi = 0; bi < NB; bi++) {
-    uint4 wn;
-    uint2 xn[4];
-    if (bi + 1 < NB) {                                           // next block's operands are in flight during this one
-      wn = lds128(wa + (bi + 1) * 512);
-#pragma unroll
-      for (int i = 0; i < 4; i++) xn[i] = lds64(xa[i] + (bi + 1) * 128);
+    for (int k = 0; k < 8; k += 2) {
+      const uint32_t a[4] = {ws[k] & 0xF0F0F0F0u, (ws[k] << 4) & 0xF0F0F0F0u, ws[k + 1] & 0xF0F0F0F0u, (ws[k + 1] << 4) & 0xF0F0F0F0u};
+      mma_s8(c, a, xs[k], xs[k + 1]);
     }
-    const uint32_t ws[4] = {w4.x, w4.y, w4.z, w4.w};
-    const bool first = (bi == 0) || (((bi & 1) != 0) == odd0);   // block b0 + bi opens a round
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-      const uint32_t w2 = ws[i] >> 8;
-      const uint32_t a[4] = {ws[i] & 0x000F000Fu, ws[i] & 0x00F000F0u, w2 & 0x000F000Fu, w2 & 0x00F000F0u};
-      if (first && i == 0) mma_f16_first(cg, a, xb[i].x, xb[i].y);
-      else mma_f16(cg, a, xb[i].x, xb[i].y);
+    const float v = __int2float_rn((up ? c[2] : c[0]) + 256 * (up ? c[3] : c[1]));
+    ct = fmaf(s, F.x * v, ct);                                  // in this order: F.x alone may be subnormal
+    if (HZ) ct = fmaf(lds_bf16(ma + C::G * META), F.y, ct);
+    if (RT == 16) {
+      ct2 = fmaf(lds_bf16(ma + 16), F.x * __int2float_rn(c[2] + 256 * c[3]), ct2);
+      if (HZ) ct2 = fmaf(lds_bf16(ma + C::G * META + 16), F.y, ct2);
     }
-    const bool closes = (((bi & 1) != 0) != odd0);               // block b0 + bi closes a round
-    if (closes || bi == NB - 1) {
-      const uint32_t ro = (NB % 2 == 0) ? (uint32_t)(b0 >> 1) + (bi >> 1) : (uint32_t)((b0 + bi) >> 1);
-      const float4 Fl = lds128f(fl + ro * 16), Fh = lds128f(fh + ro * 16);
-      const float sl = lds_bf16(ml + ro * RT * 2), sh = lds_bf16(mh + ro * RT * 2);
-      const float sl2 = sl * Fl.x, sh2 = sh * Fh.y;
-      ct[0] = fmaf(sl2, cg[0], ct[0]); ct[1] = fmaf(sl2, cg[1], ct[1]);
-      ct[2] = fmaf(sh2, cg[2], ct[2]); ct[3] = fmaf(sh2, cg[3], ct[3]);
-      if (closes) {                                              // once per (row, group): offset and zero point
-        zl = fmaf(sl, Fl.z, zl);
-        zh = fmaf(sh, Fh.z, zh);
-        if (HZ) {
-          zl = fmaf(lds_bf16(ml + C::G * RT * 2 + ro * RT * 2), Fl.w, zl);
-          zh = fmaf(lds_bf16(mh + C::G * RT * 2 + ro * RT * 2), Fh.w, zh);
-        }
-      }
-    }
-    if (bi + 1 < NB) {
-      w4 = wn;
-#pragma unroll
-      for (int i = 0; i < 4; i++) xb[i] = xn[i];
-    }
-  }
-  // valid outputs: MMA row g -> column jl, MMA row g + 8 -> column jh
-  const float vl = (jl == 2 * t) ? ct[0] + zl : ((jl == 2 * t + 1) ? ct[1] + zl : 0.f);
-  const float vh = (jh == 2 * t) ? ct[2] + zh : ((jh == 2 * t + 1) ? ct[3] + zh : 0.f);
-  if (RT <= 8) {
-    float v = vl + vh;
-    v += __shfl_xor_sync(0xffffffffu, v, 1);
-    v += __shfl_xor_sync(0xffffffffu, v, 2);
-#pragma unroll
-    for (int o = 4 * RT; o < 32; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    out_lo = v;
-    out_hi = 0.f;
-  } else {
-    out_lo = vl;
-    out_hi = vh;
-  }
-}
-
-// One slice (NB blocks) of one tile against the staged activations. RT <= 8: on return every lane with lane / 4 % RT == r
-// holds the slice's total of tile row r in out_lo. RT == 16: lane 4g holds row g in out_lo and row g + 8 in out_hi.
-// The block loop is ROLLED over rounds (two rounds = four blocks of four MMA steps and two group flushes per iteration): the
-// product of a tile is ~4 KB of code that every block of every tile reuses, instead of NB fully unrolled blocks (~10 KB per call
-// site, executed once per tile) streaming through the instruction cache.
-template <class C, bool HZ>
-__device__ __forceinline__ void tile_dot_rolled(const uint8_t* tile, int slice, const XStage& x, int lane, float& out_lo,
-                                         float& out_hi) {
-  constexpr int RT = C::RT, NB = C::NB;
-  const int g = lane >> 2, t = lane & 3;
-  const int jl = g / RT, jh = (g + 8) / RT, jb = g % C::NJ;
-  const int rl = g % RT, rh = (g + 8) % RT;
-  const int b0 = C::KS == 1 ? 0 : slice * NB;
-  const uint32_t tb = smem_u32(tile);
-  uint32_t wa = tb + (uint32_t)(b0 * 32 + lane) * 16;
-  const uint32_t xbase = smem_u32(x.xh) + (uint32_t)(jb * (C::K / C::NJ) + 4 * t) * 2 + (uint32_t)b0 * 128;
-  uint32_t xa[4];
-#pragma unroll
-  for (int i = 0; i < 4; i++) xa[i] = xbase + 32 * ((i + jb) & 3);
-  uint32_t ml = tb + C::NIB + (uint32_t)(jl * C::RG * RT + rl) * 2;
-  uint32_t mh = tb + C::NIB + (uint32_t)(jh * C::RG * RT + rh) * 2;
-  uint32_t fl = smem_u32(x.xf) + (uint32_t)(jl * C::RG) * 16, fh = smem_u32(x.xf) + (uint32_t)(jh * C::RG) * 16;
-  float ct[4] = {0.f, 0.f, 0.f, 0.f}, cg[4];
-  float zl = 0.f, zh = 0.f;
-  const bool odd0 = (NB % 2 == 0) ? false : (b0 & 1);           // the slice starts in the middle of a round
-  {                                                              // first round of the slice
-    const uint32_t ro0 = (uint32_t)(b0 >> 1);
-    ml += ro0 * RT * 2; mh += ro0 * RT * 2; fl += ro0 * 16; fh += ro0 * 16;
-  }
-  uint4 w4 = lds128(wa);
-  uint2 xb[4];
-#pragma unroll
-  for (int i = 0; i < 4; i++) xb[i] = lds64(xa[i]);
-  // one block: four MMA steps; the next block's operands are requested before this block's MMAs
-  auto block = [&](bool first, bool more) {
-    uint4 wn = w4;
-    uint2 xn[4];
-#pragma unroll
-    for (int i = 0; i < 4; i++) xn[i] = xb[i];
-    if (more) {
-      wn = lds128(wa + 512);
-#pragma unroll
-      for (int i = 0; i < 4; i++) xn[i] = lds64(xa[i] + 128);
-    }
-    const uint32_t ws[4] = {w4.x, w4.y, w4.z, w4.w};
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-      const uint32_t w2 = ws[i] >> 8;
-      const uint32_t a[4] = {ws[i] & 0x000F000Fu, ws[i] & 0x00F000F0u, w2 & 0x000F000Fu, w2 & 0x00F000F0u};
-      if (first && i == 0) mma_f16_first(cg, a, xb[i].x, xb[i].y);
-      else mma_f16(cg, a, xb[i].x, xb[i].y);
-    }
-    wa += 512;
-#pragma unroll
-    for (int i = 0; i < 4; i++) xa[i] += 128;
-    w4 = wn;
-#pragma unroll
-    for (int i = 0; i < 4; i++) xb[i] = xn[i];
+    ma += META;
+    fa += 16;
+    w0 = wn0; w1 = wn1; x0 = xn0; x1 = xn1;
   };
-  // the group's flush; `whole`: this slice closes the round (offset and zero point once per (row, group))
-  auto flush = [&](bool whole) {
-    const float4 Fl = lds128f(fl), Fh = lds128f(fh);
-    const float sl = lds_bf16(ml), sh = lds_bf16(mh);
-    const float sl2 = sl * Fl.x, sh2 = sh * Fh.y;
-    ct[0] = fmaf(sl2, cg[0], ct[0]); ct[1] = fmaf(sl2, cg[1], ct[1]);
-    ct[2] = fmaf(sh2, cg[2], ct[2]); ct[3] = fmaf(sh2, cg[3], ct[3]);
-    if (whole) {
-      zl = fmaf(sl, Fl.z, zl);
-      zh = fmaf(sh, Fh.z, zh);
-      if (HZ) {
-        zl = fmaf(lds_bf16(ml + C::G * RT * 2), Fl.w, zl);
-        zh = fmaf(lds_bf16(mh + C::G * RT * 2), Fh.w, zh);
-      }
-    }
-    ml += RT * 2; mh += RT * 2; fl += 16; fh += 16;
-  };
-  int left = NB;                                                 // blocks still to do
-  if (odd0) {                                                    // second half of a round another slice opened
-    block(true, left > 1);
-    flush(true);
-    left--;
-  }
 #pragma unroll 1
-  for (; left >= 4; left -= 4) {                                 // two rounds per iteration (+1.8 % tokens/s over one)
-    block(true, true);
-    block(false, true);
-    flush(true);
-    block(true, true);
-    block(false, left > 4);
-    flush(true);
+  for (; n >= 2; n -= 2) {
+    round(true);
+    round(n > 2);
   }
-  if (NB % 4 != 0)
-#pragma unroll 1
-  for (; left >= 2; left -= 2) {
-    block(true, true);
-    block(false, left > 2);
-    flush(true);
-  }
-  if (NB % 2 != 0 && left) {                                     // first half of a round the next slice closes
-    block(true, false);
-    flush(false);
-  }
-  // valid outputs: MMA row g -> column jl, MMA row g + 8 -> column jh
-  const float vl = (jl == 2 * t) ? ct[0] + zl : ((jl == 2 * t + 1) ? ct[1] + zl : 0.f);
-  const float vh = (jh == 2 * t) ? ct[2] + zh : ((jh == 2 * t + 1) ? ct[3] + zh : 0.f);
-  if (RT <= 8) {
-    float v = vl + vh;
-    v += __shfl_xor_sync(0xffffffffu, v, 1);
-    v += __shfl_xor_sync(0xffffffffu, v, 2);
-#pragma unroll
-    for (int o = 4 * RT; o < 32; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    out_lo = v;
+  if (n) round(false);
+  if (RT == 8) {
+    ct += __shfl_xor_sync(0xffffffffu, ct, 1);
+    ct += __shfl_xor_sync(0xffffffffu, ct, 2);
+    out_lo = ct;
     out_hi = 0.f;
-  } else {
-    out_lo = vl;
-    out_hi = vh;
+  } else {                                                       // lanes 2 and 3 of a quad hold nothing
+    ct += __shfl_xor_sync(0xffffffffu, ct, 1);
+    ct2 += __shfl_xor_sync(0xffffffffu, ct2, 1);
+    out_lo = __shfl_sync(0xffffffffu, ct, lane & 28);
+    out_hi = __shfl_sync(0xffffffffu, ct2, lane & 28);
   }
-}
-
-// ROLL selects the form. The decode megakernel runs the rolled one in every phase: its per-layer code does not fit the
-// instruction cache, and with ~10 KB of straight-line code per phase less to fetch the whole layer got faster (QKV
-// 2.14 -> 1.81 µs, O 2.21 -> 1.85 µs, attention 4.4 -> 4.0 µs, gate/up 4.42 -> 4.77 µs; 862 -> 897 tok/s; rolling only the
-// small phases gave nothing back: 868 tok/s). The stand-alone GEMV, a small kernel, keeps the unrolled form.
-template <class C, bool HZ, bool ROLL = false>
-__device__ __forceinline__ void tile_dot(const uint8_t* tile, int slice, const XStage& x, int lane, float& out_lo,
-                                         float& out_hi) {
-  if constexpr (ROLL) tile_dot_rolled<C, HZ>(tile, slice, x, lane, out_lo, out_hi);
-  else tile_dot_unrolled<C, HZ>(tile, slice, x, lane, out_lo, out_hi);
 }
 
 }  // namespace fb

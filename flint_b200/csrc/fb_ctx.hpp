@@ -24,7 +24,6 @@ struct fb_ctx {
   int force_chunks;
   long long* prof;
   uint64_t *h_ll, *q_ll, *k_ll, *v_ll, *ao_ll, *act_ll, *cand_ll, *part_ll;   // tagged vectors of the data-flow kernel
-  uint32_t* flags;                                                  // [3][256] arrival flags: h, act, ao
   unsigned tag_base;
   int tp_size, tp_rank, vocab_base, ko, ao_off;                     // tensor parallelism (1 GPU: tp_size 1, ko = dim)
   uint64_t* inbox;                                                  // [2][tp][dim] partial words + [tp][2] candidates
@@ -37,7 +36,7 @@ struct fb_ctx {
   unsigned* vamax;                                                  // per token: bound on the attention output (float bits)
   unsigned* gu_norms;                                               // [n_layer][2] largest squared row norms of gate and up (float bits)
   void* vrope;                                                      // verify: (cos, sin) per (token, rotation pair)
-  int max_fly, poll_words;                                          // max_fly 0: chosen by the bytes of a layer (fly_for)
+  int max_fly;                                                      // max_fly 0: chosen by the bytes of a layer (fly_for)
   CUtensorMap kmap, vmap;                                           // the caches as tensors (make_kv_maps)
 };
 

@@ -3,12 +3,13 @@
 // Phases of one token are chained by DATA, not by grid barriers: every vector that crosses CTAs (residual h, q / new
 // k / new v, attention output, SwiGLU activations, arg-max candidates) lives in global memory as 8-byte words that
 // carry their payload (two bf16 values or one fp32/int32) together with a 32-bit tag unique to (launch, layer,
-// phase). A producer stores the word once; a consumer polls the word itself until the tag matches, so the value
+// phase). A producer publishes the word once; a consumer polls the word itself until the tag matches, so the value
 // arrives with the same L2 round trip that a barrier would only have announced. Each hop costs about one L2 round
-// trip instead of three (barrier arrive, barrier poll, data fetch).
+// trip instead of three (barrier arrive, barrier poll, data fetch). (Arrival flags that were waited for ahead of the words gained as long as words were
+// stored, see ll_store; with exchanges they cost 847 us a token of the 3B-class shape at 200 positions against 808 without.)
 //
-// Why single buffers are enough: every phase consumes a vector that ALL CTAs contributed to, so a CTA can only be
-// one full phase ahead of the slowest one; a buffer is rewritten two phases after its last reader at the earliest.
+// Why single buffers are enough: a CTA reads a phase's input only if it owns rows of that phase, the next phase needs every such CTA's words, and an
+// input is overwritten in the next phase at the earliest. (A CTA without rows skips the input: it might find it overwritten.)
 #pragma once
 #include <cuda.h>
 
@@ -20,20 +21,23 @@ namespace fb {
 // multiples of 64 are cut into column blocks of 64 (128 bytes, the swizzle width), [block][position][64] each, so that the eight
 // rows of an 8x8 matrix load lie in different banks (unswizzled rows of 128 or 256 bytes all start in the same bank: 8 times
 // the shared-memory cycles); other head dimensions keep whole rows (160 bytes for 80: two rows per bank group).
-template <int HD>
+template <int HD, int STG>
 struct AttnCfg {
-  static constexpr int NPS = 2 * 64 * HD * 2 <= kStageBytes ? 64 : 32;
+  static constexpr int NPS = 2 * 64 * HD * 2 <= STG ? 64 : 32;
   static constexpr int MATRIX_BYTES = NPS * HD * 2, KV_STAGE_BYTES = 2 * MATRIX_BYTES;
   static constexpr bool SPLIT = HD % 64 == 0;
   static constexpr int BLKS = SPLIT ? HD / 64 : 1, BCOLS = SPLIT ? 64 : HD, ROWB = BCOLS * 2;
   static_assert(HD % 8 == 0 && HD <= 128, "head_dim must be a multiple of 8 and <= 128");
-  static_assert(KV_STAGE_BYTES <= kStageBytes && MATRIX_BYTES % 128 == 0, "a ring stage holds one sweep of K and V rows");
+  static_assert(KV_STAGE_BYTES <= STG && MATRIX_BYTES % 128 == 0, "a ring stage holds one sweep of K and V rows");
 };
 
 // ------------------------------------------------------------------------------------------------ tagged words
+// Words are published by atomic exchanges, whose result nobody wants: an exchange is performed at L2 at once, a store waits in the SM's store path until
+// something pushes it out (200 cached positions of the 3B-class shape: 882 us a token with stores, 784 with exchanges; with stores and an exchange per
+// CTA and phase behind them, the arrival flags that this kernel once had, 809).
 __device__ __forceinline__ void ll_store(uint64_t* p, uint32_t payload, uint32_t tag) {
   const uint64_t v = ((uint64_t)tag << 32) | payload;
-  asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+  asm volatile("{ .reg .b64 old;\n atom.relaxed.gpu.global.exch.b64 old, [%0], %1; }" ::"l"(p), "l"(v) : "memory");
 }
 __device__ __forceinline__ void ll_load2(const uint64_t* p, uint64_t& a, uint64_t& b) {
   asm volatile("ld.relaxed.gpu.global.v2.u64 {%0,%1}, [%2];" : "=l"(a), "=l"(b) : "l"(p) : "memory");
@@ -71,27 +75,27 @@ __device__ __forceinline__ uint32_t ll_poll_sys(const uint64_t* p, uint32_t tag,
 // 16 bytes = two tagged words in one store (each word carries its own tag)
 __device__ __forceinline__ void ll_store2(uint64_t* p, uint32_t pay0, uint32_t pay1, uint32_t tag) {
   const uint64_t a = ((uint64_t)tag << 32) | pay0, b = ((uint64_t)tag << 32) | pay1;
-  asm volatile("st.relaxed.gpu.global.v2.u64 [%0], {%1, %2};" ::"l"(p), "l"(a), "l"(b) : "memory");
+  asm volatile("{ .reg .b128 v, old;\n mov.b128 v, {%1, %2};\n atom.relaxed.gpu.global.exch.b128 old, [%0], v; }" ::"l"(p), "l"(a), "l"(b) : "memory");
 }
 // one round of a bounded poll went by without the word: true = give up (abort seen or limit reached)
 inline __device__ __noinline__ bool poll_again(unsigned spin, const WaitCtl wc, int layer, int expected, int seen) {
   if (*wc.s_abort) return true;
-  if (spin > 16) __nanosleep(40);
   if ((spin & 255) == 255 && ld_volatile_s32(&wc.st->abort)) { *wc.s_abort = 1; return true; }
   if (spin >= wc.limit) { report_fail_far(wc, W_FLAG, layer, expected, seen); return true; }
   return false;
 }
 
-// Poll `nwords` (even, 16-byte aligned base) tagged words into 32-bit payloads dst[0..nwords). Threads
-// tid, tid+nthreads, ... each own word pairs; all of a thread's loads are issued before any is checked.
+// Poll tagged words, 16-byte aligned: pair k of a thread is words 2 (tid + k * nthreads) and the one behind it, `npairs` pairs in all; their payloads go to
+// v[k] (zero where there is no such pair). All of a thread's loads are issued before any is checked.
 template <int MAXP>
-__device__ __forceinline__ void ll_gather(const uint64_t* src, int nwords, uint32_t tag, uint32_t* dst, int tid,
-                                          int nthreads, const WaitCtl& wc, int layer) {
-  const int npairs = nwords >> 1;
+__device__ __forceinline__ void ll_gather(const uint64_t* src, int npairs, uint32_t tag, uint2 (&v)[MAXP], int tid, int nthreads,
+                                          const WaitCtl& wc, int layer) {
   uint32_t pending = 0;
 #pragma unroll
-  for (int k = 0; k < MAXP; k++)
+  for (int k = 0; k < MAXP; k++) {
+    v[k] = make_uint2(0, 0);
     if (tid + k * nthreads < npairs) pending |= 1u << k;
+  }
 #pragma unroll 1
   for (unsigned spin = 0; pending; spin++) {
     uint64_t a[MAXP], b[MAXP];
@@ -102,9 +106,7 @@ __device__ __forceinline__ void ll_gather(const uint64_t* src, int nwords, uint3
     for (int k = 0; k < MAXP; k++)
       if (pending & (1u << k)) {
         if ((uint32_t)(a[k] >> 32) == tag && (uint32_t)(b[k] >> 32) == tag) {
-          const int j = 2 * (tid + k * nthreads);
-          dst[j] = (uint32_t)a[k];
-          dst[j + 1] = (uint32_t)b[k];
+          v[k] = make_uint2((uint32_t)a[k], (uint32_t)b[k]);
           pending &= ~(1u << k);
         }
       }
@@ -112,87 +114,22 @@ __device__ __forceinline__ void ll_gather(const uint64_t* src, int nwords, uint3
   }
 }
 
-// Arrival flags: polling the tagged data words directly from 75 000 threads floods the few L2 lines that hold a
-// vector, so a CTA first waits (one warp, a handful of coalesced loads per round) until every producer CTA has posted
-// its arrival flag, and only then gathers the words. The flag is posted without a fence, so the tags in the words
-// stay the correctness check: a word that lags behind its flag is simply polled again.
-__device__ __forceinline__ uint32_t ld_relaxed_u32(const uint32_t* p) {
-  uint32_t v;
-  asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-  return v;
-}
-// flags are posted with an atomic exchange: it is performed at L2 at once instead of waiting in the SM's store path
-__device__ __forceinline__ void st_relaxed_u32(uint32_t* p, uint32_t v) {
-  uint32_t old;
-  asm volatile("atom.relaxed.gpu.global.exch.b32 %0, [%1], %2;" : "=r"(old) : "l"(p), "r"(v) : "memory");
-  (void)old;
-}
-// all consumer threads call; warp 0 polls flags[0..n) until each equals tag
-// The gather starts when all but n / 2 producers have posted. The tagged words of the stragglers are simply polled again by the gather, so
-// the last flags' round trip leaves the critical path. Microseconds a token at a third / a half / three quarters: 3B-class 1060 / 1020 /
-// 1010, 1B 395 / 390 / 386, 40 / 8 heads of 64 1017 / 1020 / 1042; no flag wait at all is slower (every consumer polling words
-// floods L2).
-__device__ __forceinline__ void wait_flags(const uint32_t* flags, int n, uint32_t tag, int cw, int lane, const WaitCtl& wc,
-                                           int layer) {
-  if (cw == 0) {
-    uint32_t v[8];
-    // all loads of a round are issued before any is compared (n <= 256: at most 8 per lane)
-    auto issue = [&]() {
-#pragma unroll
-      for (int j = 0; j < 8; j++) v[j] = (lane + 32 * j < n) ? ld_relaxed_u32(flags + lane + 32 * j) : tag;
-    };
-    issue();
-#pragma unroll 1
-    for (unsigned spin = 0;; spin++) {
-      unsigned miss = 0;
-#pragma unroll
-      for (int j = 0; j < 8; j++) miss += (v[j] != tag);
-      if (__reduce_add_sync(0xffffffffu, miss) <= (unsigned)(n / 2)) break;
-      issue();
-      int stop = 0;
-      if (lane == 0) {
-        if (*wc.s_abort) stop = 1;
-        else if ((spin & 63) == 63 && ld_volatile_s32(&wc.st->abort)) { *wc.s_abort = 1; stop = 1; }
-        else if (spin >= wc.limit) { report_fail_far(wc, W_FLAG, layer, (int)tag, n); stop = 1; }
-      }
-      if (__shfl_sync(0xffffffffu, stop, 0)) break;
-    }
-  }
-  named_bar_sync(kBarConsumers, kConsumerThreads);
-}
-// a warp that has finished its part of a phase calls this; the CTA's last warp posts the flag
-__device__ __forceinline__ void post_when_cta_done(int* s_done, uint32_t* flag, uint32_t tag, int lane,
-                                                   long long* dbg = nullptr) {
-  __syncwarp();
-  if (lane == 0) {
-    const int old = atomicAdd(s_done, 1);
-    if (old == kConsumerWarps - 1) {
-      *s_done = 0;
-      st_relaxed_u32(flag, tag);
-      if (dbg) dbg[12] = (long long)globaltimer_ns();
-    }
-  }
-}
-
 // ------------------------------------------------------------------------------------------------ staging from tagged vectors
-// Both are real functions, one instance per kernel, not inlined at their five call sites: the layer loop's code is larger than
-// the instruction cache, and every kilobyte less shortens all phases (inlined copies of one generic staging function 1187 us a token of
-// the 3B-class shape; one shared copy 1051; templated on the widths and shared as here 1001). For the same reason the conversion
-// after the plain gather is a rolled loop and both plain phases share the instance of the wider one. The tile products stay
-// inlined per phase: one shared product costs more in calls than it saves (1125).
-// Both leave the phase's activations in sm.xh / sm.xf (fp16 in B-operand order + per-group factors) and end
-// with a consumer-wide barrier. A thread owns the 4 elements 4*pr .. 4*pr+3 for pr = tid_c, tid_c + kConsumerThreads, ...
-// so a warp owns whole groups of 128 and converts them in place.
+// Both are real functions, one instance per kernel, not inlined at their five call sites: every kilobyte of the layer loop shortens all phases (inlined
+// copies of one generic staging function 1187 us a token of the 3B-class shape; one shared copy 1051; templated on the widths and shared
+// as here 1001). Both plain phases share the instance of the wider one. The tile products stay inlined per phase: one shared product costs more in
+// calls than it saves (1125).
+// Both leave the phase's activations in sm.x8 / sm.xf (digits + per-group factors) and end with a consumer-wide barrier. A thread owns the 4
+// elements 4*pr .. 4*pr+3 for pr = tid_c, tid_c + kConsumerThreads, ... and keeps them in registers, so a warp owns whole groups of 128. (As a rolled
+// loop over shared memory the conversion of 8192 elements was a chain of five groups; side by side it takes 0.4 us less.)
 // xn = bf16( (float(h) * r) * float(w) ) from the tagged residual vector (dim/2 words)
-template <int MAXP>
-inline __device__ __noinline__ void stage_norm_ll(const uint64_t* hll, const uint32_t* flags, int nflags, uint32_t tag,
-                                                  const uint16_t* gw, int D, float eps, DevStatus* status, unsigned limit, int layer,
+template <int MAXP, bool SUM>
+inline __device__ __noinline__ void stage_norm_ll(const uint64_t* hll, uint32_t tag, const uint16_t* gw, int D, float eps, DevStatus* status, unsigned limit, int layer,
                                                   bool have_h, long long* dbg = nullptr) {
   extern __shared__ __align__(128) uint8_t smem_raw[];
   const Smem sm = carve_smem(smem_raw);
   const WaitCtl wc{status, sm.s_abort, limit};
   const int tid_c = threadIdx.x;
-  uint32_t* xs32 = reinterpret_cast<uint32_t*>(sm.xh);
   float* red = sm.red;
   const int npairs = D / 4, lane = tid_c & 31;
   uint2 wv[MAXP];                       // norm weights do not depend on the wait: fetch them first
@@ -201,26 +138,27 @@ inline __device__ __noinline__ void stage_norm_ll(const uint64_t* hll, const uin
     const int pr = tid_c + k * kConsumerThreads;
     wv[k] = pr < npairs ? __ldg(reinterpret_cast<const uint2*>(gw) + pr) : make_uint2(0, 0);
   }
-  if (!have_h) {      // layer 0 finds the raw residual (bf16, natural order) already in place
-    if (nflags > 0) wait_flags(flags, nflags, tag, tid_c >> 5, lane, wc, layer);
-    else named_bar_sync(kBarConsumers, kConsumerThreads);     // every warp has left the phase that read the activations
-    if (dbg && tid_c == 0) dbg[10] = (long long)globaltimer_ns();
-    ll_gather<MAXP>(hll, D / 2, tag, xs32, tid_c, kConsumerThreads, wc, layer);
-    if (dbg && tid_c == 0) dbg[11] = (long long)globaltimer_ns();
-  }
-  // each thread squares the pairs it gathered itself: no barrier needed before this
   uint2 raw[MAXP];
+  if (!have_h) {
+    // Every warp has left the phase before (and whose activations it read): polling that starts while slow warps still multiply costs them
+    // more than it gains.
+    named_bar_sync(kBarConsumers, kConsumerThreads);
+    ll_gather<MAXP>(hll, npairs, tag, raw, tid_c, kConsumerThreads, wc, layer);
+    if (dbg && tid_c == 0) dbg[11] = (long long)globaltimer_ns();
+  } else {            // layer 0 finds the raw residual (bf16, natural order) in place; the barrier below comes before anybody overwrites it
+    const uint2* h0 = reinterpret_cast<const uint2*>(sm.x8);
+#pragma unroll
+    for (int k = 0; k < MAXP; k++) {
+      const int pr = tid_c + k * kConsumerThreads;
+      raw[k] = pr < npairs ? h0[pr] : make_uint2(0, 0);
+    }
+  }
   float ss = 0.f;
 #pragma unroll
   for (int k = 0; k < MAXP; k++) {
-    const int pr = tid_c + k * kConsumerThreads;
-    raw[k] = make_uint2(0, 0);
-    if (pr < npairs) {
-      const uint32_t a = xs32[2 * pr], b = xs32[2 * pr + 1];
-      raw[k] = make_uint2(a, b);
-      ss = fmaf(bflo(a), bflo(a), ss); ss = fmaf(bfhi(a), bfhi(a), ss);
-      ss = fmaf(bflo(b), bflo(b), ss); ss = fmaf(bfhi(b), bfhi(b), ss);
-    }
+    const uint32_t a = raw[k].x, b = raw[k].y;
+    ss = fmaf(bflo(a), bflo(a), ss); ss = fmaf(bfhi(a), bfhi(a), ss);
+    ss = fmaf(bflo(b), bflo(b), ss); ss = fmaf(bfhi(b), bfhi(b), ss);
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
@@ -228,41 +166,34 @@ inline __device__ __noinline__ void stage_norm_ll(const uint64_t* hll, const uin
   named_bar_sync(kBarConsumers, kConsumerThreads);
   float tot = 0.f;
 #pragma unroll
-  for (int w = 0; w < kConsumerWarps; w++) tot += red[w];
+  for (int w = 0; w < kConsumerWarps; w += 2) {
+    const float2 v = *reinterpret_cast<const float2*>(red + w);
+    tot += v.x;
+    tot += v.y;
+  }
   const float r = 1.0f / sqrtf(tot / (float)D + eps);
 #pragma unroll
   for (int k = 0; k < MAXP; k++) {
-    const int pr = tid_c + k * kConsumerThreads;      // warp-uniform bound: npairs is a multiple of 32
-    if (pr < npairs) {
-      const uint32_t a = raw[k].x, b = raw[k].y;
-      const uint32_t o0 = (uint32_t)f2bf(bflo(a) * r * bflo(wv[k].x)) | ((uint32_t)f2bf(bfhi(a) * r * bfhi(wv[k].x)) << 16);
-      const uint32_t o1 = (uint32_t)f2bf(bflo(b) * r * bflo(wv[k].y)) | ((uint32_t)f2bf(bfhi(b) * r * bfhi(wv[k].y)) << 16);
-      const int grp = pr >> 5;
-      stage_group_fp16(o0, o1, sm.xh + grp * 128, sm.xf + grp, lane);
-    }
+    const uint32_t a = raw[k].x, b = raw[k].y;
+    raw[k].x = (uint32_t)f2bf(bflo(a) * r * bflo(wv[k].x)) | ((uint32_t)f2bf(bfhi(a) * r * bfhi(wv[k].x)) << 16);
+    raw[k].y = (uint32_t)f2bf(bflo(b) * r * bflo(wv[k].y)) | ((uint32_t)f2bf(bfhi(b) * r * bfhi(wv[k].y)) << 16);
   }
+  stage_groups<SUM, MAXP>(raw, tid_c >> 5, kConsumerWarps, D / 128, sm.x8, sm.xf, lane);
   named_bar_sync(kBarConsumers, kConsumerThreads);
 }
 
-template <int MAXP>
-inline __device__ __noinline__ void stage_plain_ll(const uint64_t* src, const uint32_t* flags, int nflags, uint32_t tag, int K,
+template <int MAXP, bool SUM>
+inline __device__ __noinline__ void stage_plain_ll(const uint64_t* src, uint32_t tag, int K,
                                                    DevStatus* status, unsigned limit, int layer) {
   extern __shared__ __align__(128) uint8_t smem_raw[];
   const Smem sm = carve_smem(smem_raw);
   const WaitCtl wc{status, sm.s_abort, limit};
   const int tid_c = threadIdx.x;
-  uint32_t* xs32 = reinterpret_cast<uint32_t*>(sm.xh);
   const int npairs = K / 4, lane = tid_c & 31;
-  if (nflags > 0) wait_flags(flags, nflags, tag, tid_c >> 5, lane, wc, layer);
-  else named_bar_sync(kBarConsumers, kConsumerThreads);
-  ll_gather<MAXP>(src, K / 2, tag, xs32, tid_c, kConsumerThreads, wc, layer);
-  // a thread converts exactly the words it gathered itself
-#pragma unroll 1
-  for (int pr = tid_c; pr < npairs; pr += kConsumerThreads) {
-    const uint2 v = *reinterpret_cast<const uint2*>(xs32 + 2 * pr);
-    const int grp = pr >> 5;
-    stage_group_fp16(v.x, v.y, sm.xh + grp * 128, sm.xf + grp, lane);
-  }
+  named_bar_sync(kBarConsumers, kConsumerThreads);            // every warp has left the phase that read the activations
+  uint2 raw[MAXP];
+  ll_gather<MAXP>(src, npairs, tag, raw, tid_c, kConsumerThreads, wc, layer);
+  stage_groups<SUM, MAXP>(raw, tid_c >> 5, kConsumerWarps, K / 128, sm.x8, sm.xf, lane);
   named_bar_sync(kBarConsumers, kConsumerThreads);
 }
 
@@ -275,16 +206,15 @@ struct AttnArgs {
   const uint64_t* v_ll;     // [NKV * HD/2] new value, natural order
   uint64_t* ao_ll;          // [NH * HD/2] natural order
   uint64_t* part_ll;        // [NKV][maxchunks][R*HD + 2R] tagged chunk partials (acc, then m, then d per head)
-  uint32_t* ao_flags;       // [NKV * nchunks] arrival flags of the attention output, one per (kv head, chunk) CTA
   int nkv, pos, nchunks, maxchunks;
   float scale;              // times log2(e)
   uint32_t tag_in, tag_part, tag_out;
 };
 
 // byte offset of 8-column block `c` of row `row` of a K or V matrix in a ring stage at shared address `base`
-template <int HD>
+template <int HD, int STG>
 __device__ __forceinline__ uint32_t kv_addr(uint32_t base, int row, int c) {
-  using C = AttnCfg<HD>;
+  using C = AttnCfg<HD, STG>;
   if constexpr (!C::SPLIT) return base + (uint32_t)(row * C::ROWB + c * 16);
   const uint32_t a = base + (uint32_t)((c >> 3) * (C::NPS * 128) + row * 128);
   return a + ((((uint32_t)c & 7) ^ ((a >> 7) & 7)) << 4);       // the tensor copy's 128-byte swizzle: address bits 4..6 ^ 7..9
@@ -309,13 +239,13 @@ __device__ __forceinline__ int count_unit(int* n) {
 // with K/V loaded by the warps themselves: 40 / 8 heads of 64, 604 positions 1240 -> 1014 us a token (24 us a layer in all), 32 / 8 heads
 // of 64, 22 positions 433 -> 397. Against the earlier ring form (unswizzled 256-byte rows, 8-way bank conflicts on K and V, all 14 warps
 // merged whether they had a unit or not) heads of 128, 1778 positions: attention 9.8 -> 7.9 us a layer.
-template <int HD, int R>
+template <int HD, int R, int STG>
 __device__ __forceinline__ void attention_phase(const AttnArgs& a, uint8_t* scratch, int cw, int lane, int tid_c, const WaitCtl& wc, int layer,
                                                 Pipe& pipe, int* tdone) {
-  using C = AttnCfg<HD>;
+  using C = AttnCfg<HD, STG>;
   constexpr int HP = HD / 2, KSTEPS = (HD + 15) / 16, NTD = HD / 8, NPS = C::NPS, UP = 16, SPLIT = NPS / UP, RH = R > 8 ? 2 : 1;
   static_assert(R <= 16 && NPS % UP == 0, "the query heads of a group are the rows of one MMA tile");
-  static_assert(kConsumerWarps * R * (HD + 2) * 4 + (R + 2) * HD * 2 <= kScratchBytes, "attention scratch");
+  static_assert(kConsumerWarps * R * (HD + 2) * 4 + (R + 2) * HD * 2 <= kAttnScratch, "attention scratch");
   float* wacc = reinterpret_cast<float*>(scratch);                 // [CW][R][HD]
   float* wm = wacc + kConsumerWarps * R * HD;                      // [CW][R]
   float* wd = wm + kConsumerWarps * R;                             // [CW][R]
@@ -382,20 +312,20 @@ __device__ __forceinline__ void attention_phase(const AttnArgs& a, uint8_t* scra
         const uint32_t it = pipe.it + st;
         const int sslot = it % kStages;
         if (!wait_stage(pipe, it, wc, layer)) break;
-        uint8_t* stage = pipe.stages + (size_t)sslot * kStageBytes;
+        uint8_t* stage = pipe.stages + (size_t)sslot * STG;
         const uint32_t k_s = smem_u32(stage), v_s = k_s + C::MATRIX_BYTES;
         const int row0 = part * UP, base = t0 + st * NPS + row0, nvalid = min(UP, t1 - base);
         if (nvalid > 0) {
           const int own = a.pos - base;
           if (own >= 0 && own < UP && lane < NTD) {                // this step's own row: from the tagged words, not the cache
             const uint4 kn = reinterpret_cast<const uint4*>(qs + R * HP)[lane], vn = reinterpret_cast<const uint4*>(qs + (R + 1) * HP)[lane];
-            *reinterpret_cast<uint4*>(stage + (kv_addr<HD>(k_s, row0 + own, lane) - k_s)) = kn;
-            *reinterpret_cast<uint4*>(stage + (kv_addr<HD>(v_s, row0 + own, lane) - k_s)) = vn;
+            *reinterpret_cast<uint4*>(stage + (kv_addr<HD, STG>(k_s, row0 + own, lane) - k_s)) = kn;
+            *reinterpret_cast<uint4*>(stage + (kv_addr<HD, STG>(v_s, row0 + own, lane) - k_s)) = vn;
           }
           // rows past the chunk are other cache rows (or never written): their V must not meet a zero probability as NaN
 #pragma unroll 1
           for (int i = lane; i < (UP - nvalid) * NTD; i += 32)
-            *reinterpret_cast<uint4*>(stage + (kv_addr<HD>(v_s, row0 + nvalid + i / NTD, i % NTD) - k_s)) = make_uint4(0, 0, 0, 0);
+            *reinterpret_cast<uint4*>(stage + (kv_addr<HD, STG>(v_s, row0 + nvalid + i / NTD, i % NTD) - k_s)) = make_uint4(0, 0, 0, 0);
           __syncwarp();
           float sc[2][4];
 #pragma unroll
@@ -403,7 +333,7 @@ __device__ __forceinline__ void attention_phase(const AttnArgs& a, uint8_t* scra
 #pragma unroll
           for (int ks = 0; ks < KSTEPS; ks++) {
             uint32_t bk[4];                                        // (positions 0..7, columns 0..7), (.., 8..15), (8..15, 0..7), (8..15, 8..15)
-            ldmatrix_x4(bk, kv_addr<HD>(k_s, row0 + (mat >> 1) * 8 + (lane & 7), min(2 * ks + (mat & 1), NTD - 1)));
+            ldmatrix_x4(bk, kv_addr<HD, STG>(k_s, row0 + (mat >> 1) * 8 + (lane & 7), min(2 * ks + (mat & 1), NTD - 1)));
             mma_bf16(sc[0], aq[ks], bk[0], bk[1]);
             mma_bf16(sc[1], aq[ks], bk[2], bk[3]);
           }
@@ -444,7 +374,7 @@ __device__ __forceinline__ void attention_phase(const AttnArgs& a, uint8_t* scra
 #pragma unroll
           for (int j = 0; j < NTD; j += 2) {
             uint32_t bv[4];
-            ldmatrix_x4_t(bv, kv_addr<HD>(v_s, row0 + (mat & 1) * 8 + (lane & 7), min(j + (mat >> 1), NTD - 1)));
+            ldmatrix_x4_t(bv, kv_addr<HD, STG>(v_s, row0 + (mat & 1) * 8 + (lane & 7), min(j + (mat >> 1), NTD - 1)));
 #pragma unroll
             for (int e = 0; e < 3; e++) {
               mma_bf16(o[j], ap[e], bv[0], bv[1]);
@@ -556,8 +486,7 @@ __device__ __forceinline__ void attention_phase(const AttnArgs& a, uint8_t* scra
         ll_store(a.ao_ll + (size_t)(kvh * R + r) * HP + (d >> 1), (uint32_t)f2bf(A0 / Dn) | ((uint32_t)f2bf(A1 / Dn) << 16), a.tag_out);
       }
     }
-    named_bar_sync(kBarConsumers, kConsumerThreads);
-    if (tid_c == 0) st_relaxed_u32(a.ao_flags + kvh * a.nchunks + c, a.tag_out);
+    named_bar_sync(kBarConsumers, kConsumerThreads);          // the scratch is free for the next item
   }
 }
 
@@ -570,10 +499,10 @@ __device__ __forceinline__ void tma_load_4d(void* dst, const CUtensorMap* map, i
       "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];"
       ::"r"(smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(z), "r"(w), "r"(smem_u32(bar)) : "memory");
 }
-template <int HD>
+template <int HD, int STG>
 __device__ __forceinline__ bool produce_kv(Pipe& p, const CUtensorMap* kmap, const CUtensorMap* vmap, int row0, int nkv, int nchunks,
                                            int T, int b, int G, const WaitCtl& wc, int layer) {
-  using C = AttnCfg<HD>;
+  using C = AttnCfg<HD, STG>;
   const int items = nkv * nchunks, chunk_len = (T + nchunks - 1) / nchunks;
 #pragma unroll 1
   for (int item = b; item < items; item += G) {
@@ -583,7 +512,7 @@ __device__ __forceinline__ bool produce_kv(Pipe& p, const CUtensorMap* kmap, con
       if (!stage_slot(p, wc, layer)) return false;
       const int s = (int)(p.it % kStages);
       mbar_expect_tx(&p.full[s], (uint32_t)C::KV_STAGE_BYTES);
-      uint8_t* dst = p.stages + (size_t)s * kStageBytes;
+      uint8_t* dst = p.stages + (size_t)s * STG;
 #pragma unroll
       for (int bl = 0; bl < C::BLKS; bl++) {
         tma_load_4d(dst + bl * (C::NPS * C::ROWB), kmap, 0, bl, kvh, row0 + ts, &p.full[s]);
@@ -604,7 +533,6 @@ struct Decode2Params {
   uint16_t *kc, *vc;
   uint64_t *h_ll, *q_ll, *k_ll, *v_ll, *ao_ll, *act_ll, *cand_ll;   // tagged vectors
   uint64_t* part_ll;
-  uint32_t *h_flags, *act_flags, *ao_flags;                          // arrival flags: [G], [G], [NKV]
   DevStatus* status;
   const int32_t* d_token;
   uint16_t* d_h;
@@ -616,7 +544,6 @@ struct Decode2Params {
   float eps, attn_scale, resid, emb_mult, logits_scaling;
   long long* prof;
   unsigned max_fly, lm_fly;   // bulk copies in flight per CTA while the layers run, and for the LM head
-  int32_t poll_words;         // 1: consumers poll the tagged words themselves instead of waiting for arrival flags first
   // tensor parallelism: this GPU holds a slice of every matrix (heads, FFN columns, vocabulary rows); the partial sums
   // of the K-sharded O and down projections are exchanged by peer stores into every rank's inbox
   int32_t tp_size, tp_rank, vocab_base;
@@ -629,15 +556,16 @@ struct Decode2Params {
 enum { PH_QKV = 1, PH_ATT = 2, PH_O = 3, PH_GU = 4, PH_DOWN = 5, PH_LM = 6, PH_PART = 7 };
 __device__ __forceinline__ uint32_t mk_tag(unsigned base, int layer, int ph) { return base + (unsigned)(layer * 8 + ph); }
 
-// small phases (QKV, O, down give a CTA a handful of tiles): cut long tiles in two so that more warps share them
-__host__ __device__ constexpr int small_ks(int k) {
-  const int rt = tile_rt(k), bq = (k / 128) / (16 / rt) * 2;
-  return (rt <= 4 && bq >= 16 && bq % 2 == 0) ? 2 : 1;
-}
 __host__ __device__ constexpr int imax(int a, int b) { return a > b ? a : b; }
+
+// the ring stage of a kernel of these widths
+template <int KDIM, int KOUT, int KFFN>
+using DecodePlan = SmemPlan<imax(KDIM, imax(KOUT, KFFN))>;
 
 template <int KDIM, int KOUT, int KFFN, int HD, int R, bool HZ>
 __global__ void __launch_bounds__(kThreads, 1) decode_mega2(const __grid_constant__ Decode2Params P) {
+  using S = DecodePlan<KDIM, KOUT, KFFN>;
+  constexpr int STG = S::STAGE;
   extern __shared__ __align__(128) uint8_t smem_raw[];
   Smem sm = carve_smem(smem_raw);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -653,82 +581,77 @@ __global__ void __launch_bounds__(kThreads, 1) decode_mega2(const __grid_constan
   }
   __syncthreads();
   WaitCtl wc{P.status, sm.s_abort, P.spin_limit};
-  Pipe pipe{sm.stages, sm.full, sm.empty, sm.landed, 0u, P.max_fly};
+  Pipe pipe{smem_raw + S::RING, sm.full, sm.empty, sm.landed, 0u, P.max_fly, STG};
   constexpr int HP = HD / 2;
-  using CQ = TCfg<KDIM, small_ks(KDIM)>;      // QKV: few rows per CTA
-  using CG = TCfg<KDIM>;                      // gate/up and LM head: many rows per CTA
-  using CO = TCfg<KOUT, small_ks(KOUT)>;      // O projection (K = this rank's attention output width)
-  using CF = TCfg<KFFN, small_ks(KFFN)>;      // down projection
+  using CD = TCfg<KDIM, STG>;                 // QKV, gate/up, LM head
+  using CO = TCfg<KOUT, STG>;                 // O projection (K = this rank's attention output width)
+  using CF = TCfg<KFFN, STG>;                 // down projection
   constexpr int UO = imax(CO::RT, CF::RT);    // O and down give a CTA the same rows of the residual stream
-  static_assert(CG::RT % 4 == 0, "the SwiGLU epilogue packs rows (g, u, g', u') into one tagged word");
   const int D = P.dim, FF = P.ffn, L = P.n_layer, V = P.vocab;
   const int QKV = (P.n_head + 2 * P.n_kv) * HD;
-  const int FG = P.poll_words ? 0 : G, FKV = P.poll_words ? 0 : P.n_kv * P.nchunks;     // arrival flags to wait for
   constexpr int recD = rec_bytes_of(KDIM, HZ), recO = rec_bytes_of(KOUT, HZ), recF = rec_bytes_of(KFFN, HZ);
   const size_t strQ = (size_t)pad_rows(QKV, KDIM) * recD, strO = (size_t)pad_rows(D, KOUT) * recO,
                strG = (size_t)pad_rows(2 * FF, KDIM) * recD, strF = (size_t)pad_rows(D, KFFN) * recF;
   const int N = P.tp_size, me = P.tp_rank;
   int q0, q1, o0, o1, g0, g1, l0, l1;
-  cta_rows(QKV, CQ::RT, b, G, q0, q1);
+  cta_rows(QKV, CD::RT, b, G, q0, q1);
   cta_rows(D, UO, b, G, o0, o1);         // the same rows of h belong to this CTA in the O and the down phase
-  cta_rows(2 * FF, CG::RT, b, G, g0, g1);   // (g_i, u_i, g_i+1, u_i+1) stay together: one tagged word of activations
-  cta_rows(V, CG::RT, b, G, l0, l1);
+  cta_rows(2 * FF, CD::RT, b, G, g0, g1);   // (g_i, u_i, g_i+1, u_i+1) stay together: one tagged word of activations
+  cta_rows(V, CD::RT, b, G, l0, l1);
 
   if (warp == kConsumerWarps) {
     if (lane == 0) {
       bool ok = true;
 #pragma unroll 1
       for (int l = 0; l < L && ok; l++) {
-        ok = produce_rows(pipe, P.w_qkv + l * strQ + (size_t)q0 * recD, q1 - q0, CQ::TILE_ROWS, CQ::RT, recD, wc, l);
-        ok = ok && produce_kv<HD>(pipe, &P.kmap, &P.vmap, l * P.max_seq, P.n_kv, P.nchunks, P.pos + 1, b, G, wc, l);
-        ok = ok &&
-             produce_rows(pipe, P.w_o + l * strO + (size_t)o0 * recO, o1 - o0, CO::TILE_ROWS, CO::RT, recO, wc, l) &&
-             produce_rows(pipe, P.w_gu + l * strG + (size_t)g0 * recD, g1 - g0, CG::TILE_ROWS, CG::RT, recD, wc, l) &&
-             produce_rows(pipe, P.w_d + l * strF + (size_t)o0 * recF, o1 - o0, CF::TILE_ROWS, CF::RT, recF, wc, l);
+        ok = produce_rows<CD, HZ>(pipe, P.w_qkv + l * strQ, q0, q1, wc, l);
+        ok = ok && produce_kv<HD, STG>(pipe, &P.kmap, &P.vmap, l * P.max_seq, P.n_kv, P.nchunks, P.pos + 1, b, G, wc, l);
+        ok = ok && produce_rows<CO, HZ>(pipe, P.w_o + l * strO, o0, o1, wc, l) && produce_rows<CD, HZ>(pipe, P.w_gu + l * strG, g0, g1, wc, l) &&
+             produce_rows<CF, HZ>(pipe, P.w_d + l * strF, o0, o1, wc, l);
       }
       pipe.max_fly = P.lm_fly;
-      if (ok) produce_rows(pipe, P.w_lm + (size_t)l0 * recD, l1 - l0, CG::TILE_ROWS, CG::RT, recD, wc, L);
+      if (ok) produce_rows<CD, HZ>(pipe, P.w_lm, l0, l1, wc, L);
     }
   } else {
     const int cw = warp, tid_c = tid;
     float* hown = sm.hown;                                      // this CTA's rows of the residual stream (exact bf16 values)
-    int* s_done = sm.misc + 20;                                 // warps of this CTA that finished the current producing phase
-    if (tid_c == 0) *s_done = 0;
+    // what this warp takes of every phase (its own entries: no barrier needed beyond the warp)
+    uint32_t* units = sm.units + cw;
+    if (lane == 0) {
+      units[0] = unit_entry((q1 - q0 + CD::RT - 1) / CD::RT * CD::NC, CD::RPC, cw);
+      units[16] = unit_entry((o1 - o0 + CO::RT - 1) / CO::RT * CO::NC, CO::RPC, cw);
+      units[32] = unit_entry((g1 - g0 + CD::RT - 1) / CD::RT * CD::NC, CD::RPC, cw);
+      units[48] = unit_entry((o1 - o0 + CF::RT - 1) / CF::RT * CF::NC, CF::RPC, cw);
+    }
+    __syncwarp();
     const QueueState qs_{sm.qpart, sm.tdone, sm.bcnt};
-    const XStage xs_{sm.xh, sm.xf};
+    const XStage xs_{sm.x8, sm.xf};
     float* ypart = sm.hown + kMaxOwnRows;                       // tensor parallel: this rank's partial sums of its rows
     constexpr int MAXP_O = (KOUT / 4 + kConsumerThreads - 1) / kConsumerThreads;
     // O / down epilogue. One GPU: h = bf16(h + y * resid) at once. Tensor parallel: y is a partial sum over this
     // rank's K slice: keep it, push it to every peer's inbox, finish in resid_finish once all rows are done.
     auto resid_epi = [&](int row0, float c, int nvalid, uint32_t tag, int par) {
-      const int r = row0 + (lane >> 3);
+      const int r = row0 + (lane >> 2);
       if (N > 1) {
-        // lanes 0/8/16/24 hold the partial sums of rows row0..row0+3; lane j < N-1 pushes all four to one peer as two
-        // 16-byte stores, so the N-1 transfers of a tile leave the SM side by side instead of one after the other
-        const float c0 = __shfl_sync(0xffffffffu, c, 0), c1 = __shfl_sync(0xffffffffu, c, 8),
-                    c2 = __shfl_sync(0xffffffffu, c, 16), c3 = __shfl_sync(0xffffffffu, c, 24);
-        if ((lane & 7) == 0 && (lane >> 3) < nvalid) ypart[r] = c;
-        if (lane < N - 1) {
-          const int p = lane >= me ? lane + 1 : lane;
-          uint64_t* dst = P.peer_inbox[p] + ((size_t)(par * N + me)) * D + o0 + row0;     // 32-byte aligned: row0 % 4 == 0
-          if (nvalid == 4) {
-            ll_store2_sys(dst, __float_as_uint(c0), __float_as_uint(c1), tag);
-            ll_store2_sys(dst + 2, __float_as_uint(c2), __float_as_uint(c3), tag);
-          } else {
-            const float cc[4] = {c0, c1, c2, c3};
-#pragma unroll 1
-            for (int i = 0; i < nvalid; i++) ll_store_sys(dst + i, __float_as_uint(cc[i]), tag);
-          }
+        // quad r holds the partial sum of row row0 + r; lane j < N-1 pushes all eight to one peer, 16 bytes a store, so the N-1 transfers of a tile
+        // leave the SM side by side instead of one after the other
+        if ((lane & 3) == 0 && (lane >> 2) < nvalid) ypart[r] = c;
+        const int p = lane >= me ? lane + 1 : lane;
+        uint64_t* dst = P.peer_inbox[lane < N - 1 ? p : me] + ((size_t)(par * N + me)) * D + o0 + row0;     // 64-byte aligned: row0 % 8 == 0
+#pragma unroll
+        for (int i = 0; i < 8; i += 2) {
+          const float c0 = __shfl_sync(0xffffffffu, c, 4 * i), c1 = __shfl_sync(0xffffffffu, c, 4 * i + 4);
+          if (lane < N - 1 && i < nvalid) ll_store2_sys(dst + i, __float_as_uint(c0), __float_as_uint(c1), tag);      // whole pairs: dim is even
         }
         return;
       }
       float hn = 0.f;
-      if ((lane & 7) == 0 && (lane >> 3) < nvalid) {
+      if ((lane & 3) == 0 && (lane >> 2) < nvalid) {
         hn = rbf(hown[r] + c * P.resid);
         hown[r] = hn;
       }
-      const float hn1 = __shfl_down_sync(0xffffffffu, hn, 8);
-      if ((lane & 15) == 0 && (lane >> 3) < nvalid)
+      const float hn1 = __shfl_down_sync(0xffffffffu, hn, 4);
+      if ((lane & 7) == 0 && (lane >> 2) < nvalid)
         ll_store(P.h_ll + ((o0 + r) >> 1), (uint32_t)f2bf(hn) | ((uint32_t)f2bf(hn1) << 16), tag);
     };
     // tensor parallel only: collect the peers' partials of this CTA's rows (one 16-byte load per thread and poll round,
@@ -768,7 +691,6 @@ __global__ void __launch_bounds__(kThreads, 1) decode_mega2(const __grid_constan
         ll_store(P.h_ll + ((o0 >> 1) + pr), (uint32_t)f2bf(h0) | ((uint32_t)f2bf(h1) << 16), tag);
       }
       named_bar_sync(kBarConsumers, kConsumerThreads);
-      if (tid_c == 0) st_relaxed_u32(P.h_flags + b, tag);
     };
     constexpr int MAXP_D = (KDIM / 4 + kConsumerThreads - 1) / kConsumerThreads;
     constexpr int MAXP_F = (KFFN / 4 + kConsumerThreads - 1) / kConsumerThreads;
@@ -782,7 +704,7 @@ __global__ void __launch_bounds__(kThreads, 1) decode_mega2(const __grid_constan
 #pragma unroll 1
       for (int i = tid_c; i < D; i += kConsumerThreads) {
         const uint16_t v = P.d_h ? ld_cg_u16(P.d_h + i) : f2bf(bf2f(__ldg(P.embed + (size_t)tok * D + i)) * P.emb_mult);
-        reinterpret_cast<uint16_t*>(sm.xh)[i] = v;
+        reinterpret_cast<uint16_t*>(sm.x8)[i] = v;
         if (i >= o0 && i < o1) hown[i - o0] = bf2f(v);
       }
       named_bar_sync(kBarConsumers, kConsumerThreads);
@@ -797,14 +719,14 @@ __global__ void __launch_bounds__(kThreads, 1) decode_mega2(const __grid_constan
                      tg_dn = mk_tag(P.tag_base, l, PH_DOWN);
       // ================= QKV: norm1 -> GEMV -> RoPE -> tagged q / new k / new v, cache append =================
       FB_STAMP(0);
-      stage_norm_ll<MAXP_D>(P.h_ll, P.h_flags, FG, mk_tag(P.tag_base, l - 1, PH_DOWN), P.n1 + (size_t)l * D, D, P.eps,
+      if (q1 > q0) stage_norm_ll<MAXP_D, HZ>(P.h_ll, mk_tag(P.tag_base, l - 1, PH_DOWN), P.n1 + (size_t)l * D, D, P.eps,
                             P.status, P.spin_limit, l, l == 0, P.prof ? P.prof + ((size_t)b * L + l) * 16 : nullptr);
       FB_STAMP(1);
-      consume_tiles<CQ, HZ, true>(pipe, q1 - q0, xs_, qs_, cw, lane, wc, l, [&](int row0, float c, int nvalid) {
-        // lanes 0/8/16/24 hold rows row0..row0+3: two RoPE pairs (or four v dims)
-        const float c1 = __shfl_down_sync(0xffffffffu, c, 8);
-        if ((lane & 15) == 0 && (lane >> 3) < nvalid) {
-          const int rs = q0 + row0 + (lane >> 3);              // stream row of the pair's first element (even)
+      consume_tiles<CD, HZ>(pipe, q1 - q0, units[0], xs_, qs_, cw, lane, wc, l, [&](int row0, float c, int nvalid) {
+        // quad r holds row row0 + r: four RoPE pairs (or eight v dims)
+        const float c1 = __shfl_down_sync(0xffffffffu, c, 4);
+        if ((lane & 7) == 0 && (lane >> 2) < nvalid) {
+          const int rs = q0 + row0 + (lane >> 2);              // stream row of the pair's first element (even)
           const int head = rs / HD, within = rs % HD;
           if (head < P.n_head + P.n_kv) {
             const int i = within >> 1;
@@ -839,59 +761,55 @@ __global__ void __launch_bounds__(kThreads, 1) decode_mega2(const __grid_constan
           for (int i = tid_c; i < KOUT / 2 - used; i += kConsumerThreads)
             ll_store(P.ao_ll + (i < off ? i : used + i), 0u, tg_att);
         }
-        const AttnArgs aa{P.q_ll, P.k_ll, P.v_ll, P.ao_ll + (P.ao_off >> 1), P.part_ll, P.ao_flags, P.n_kv, P.pos, P.nchunks,
+        const AttnArgs aa{P.q_ll, P.k_ll, P.v_ll, P.ao_ll + (P.ao_off >> 1), P.part_ll, P.n_kv, P.pos, P.nchunks,
                      P.maxchunks, P.attn_scale, tg_qkv, mk_tag(P.tag_base, l, PH_PART), tg_att};
         named_bar_sync(kBarConsumers, kConsumerThreads);        // scratch (the activations) is free: every warp left the GEMV
-        attention_phase<HD, R>(aa, sm.scratch, cw, lane, tid_c, wc, l, pipe, sm.tdone);
+        attention_phase<HD, R, STG>(aa, sm.scratch, cw, lane, tid_c, wc, l, pipe, sm.tdone);
       }
       FB_STAMP(3);
       // ================= O projection + residual =================
       {
-        stage_plain_ll<imax(MAXP_O, MAXP_F)>(P.ao_ll, P.ao_flags, FKV, tg_att, KOUT, P.status, P.spin_limit, l);
+        if (o1 > o0) stage_plain_ll<imax(MAXP_O, MAXP_F), HZ>(P.ao_ll, tg_att, KOUT, P.status, P.spin_limit, l);
         FB_STAMP(4);
-        consume_tiles<CO, HZ, true>(pipe, o1 - o0, xs_, qs_, cw, lane, wc, l,
+        consume_tiles<CO, HZ>(pipe, o1 - o0, units[16], xs_, qs_, cw, lane, wc, l,
                                   [&](int row0, float c, int nvalid) { resid_epi(row0, c, nvalid, tg_o, 0); });
         if (N > 1) resid_finish(tg_o, 0, l);
-        else post_when_cta_done(s_done, P.h_flags + b, tg_o, lane);
       }
       FB_STAMP(5);
       // ================= gate/up + SwiGLU =================
-      stage_norm_ll<MAXP_D>(P.h_ll, P.h_flags, FG, tg_o, P.n2 + (size_t)l * D, D, P.eps, P.status, P.spin_limit, l, false);
+      if (g1 > g0) stage_norm_ll<MAXP_D, HZ>(P.h_ll, tg_o, P.n2 + (size_t)l * D, D, P.eps, P.status, P.spin_limit, l, false);
       FB_STAMP(6);
-      consume_tiles<CG, HZ, true>(pipe, g1 - g0, xs_, qs_, cw, lane, wc, l, [&](int row0, float c, int nvalid) {
-        // rows (g_i, u_i, g_{i+1}, u_{i+1}) -> act[i], act[i+1] -> one tagged word
-        const float u = __shfl_down_sync(0xffffffffu, c, 8);
+      consume_tiles<CD, HZ>(pipe, g1 - g0, units[32], xs_, qs_, cw, lane, wc, l, [&](int row0, float c, int nvalid) {
+        // rows (g_i, u_i, ...) -> act[i] .. act[i + 3] -> two tagged words
+        const float u = __shfl_down_sync(0xffffffffu, c, 4);
         float av = 0.f;
-        if ((lane & 15) == 0 && (lane >> 3) < nvalid) {
+        if ((lane & 7) == 0 && (lane >> 2) < nvalid) {
           const float gg = rbf(c), uu = rbf(u);
           av = rbf((gg / (1.0f + __expf(-gg))) * uu);
         }
-        const float av1 = __shfl_down_sync(0xffffffffu, av, 16);
-        const int i = (g0 + row0) >> 1;                          // act index of lane 0's value: even, g0 % 4 == 0
-        if (lane == 0 && nvalid == 4)
-          ll_store(P.act_ll + (i >> 1), (uint32_t)f2bf(av) | ((uint32_t)f2bf(av1) << 16), tg_gu);
+        const float av1 = __shfl_down_sync(0xffffffffu, av, 8);
+        if ((lane & 15) == 0 && (lane >> 2) + 4 <= nvalid)
+          ll_store(P.act_ll + ((g0 + row0) >> 2) + (lane >> 4), (uint32_t)f2bf(av) | ((uint32_t)f2bf(av1) << 16), tg_gu);
       });
-      post_when_cta_done(s_done, P.act_flags + b, tg_gu, lane);
       FB_STAMP(7);
       // ================= down projection + residual =================
       {
-        stage_plain_ll<imax(MAXP_O, MAXP_F)>(P.act_ll, P.act_flags, FG, tg_gu, FF, P.status, P.spin_limit, l);
+        if (o1 > o0) stage_plain_ll<imax(MAXP_O, MAXP_F), HZ>(P.act_ll, tg_gu, FF, P.status, P.spin_limit, l);
         FB_STAMP(8);
-        consume_tiles<CF, HZ, true>(pipe, o1 - o0, xs_, qs_, cw, lane, wc, l,
+        consume_tiles<CF, HZ>(pipe, o1 - o0, units[48], xs_, qs_, cw, lane, wc, l,
                                   [&](int row0, float c, int nvalid) { resid_epi(row0, c, nvalid, tg_dn, 1); });
         if (N > 1) resid_finish(tg_dn, 1, l);
-        else post_when_cta_done(s_done, P.h_flags + b, tg_dn, lane, P.prof ? P.prof + ((size_t)b * L + l) * 16 : nullptr);
       }
       FB_STAMP(9);
     }
 #undef FB_STAMP
     // ================= final norm + LM head + arg-max =================
-    stage_norm_ll<MAXP_D>(P.h_ll, P.h_flags, FG, mk_tag(P.tag_base, L - 1, PH_DOWN), P.nf, D, P.eps, P.status, P.spin_limit, L, false);
+    stage_norm_ll<MAXP_D, HZ>(P.h_ll, mk_tag(P.tag_base, L - 1, PH_DOWN), P.nf, D, P.eps, P.status, P.spin_limit, L, false);
     float bv = -INFINITY;
     int bi = 0x7fffffff;
-    consume_tiles<CG, HZ, true>(pipe, l1 - l0, xs_, qs_, cw, lane, wc, L, [&](int row0, float c, int nvalid) {
-      if ((lane & 7) == 0 && (lane >> 3) < nvalid) {
-        const int row = P.vocab_base + l0 + row0 + (lane >> 3);     // index in the full vocabulary
+    consume_tiles<CD, HZ>(pipe, l1 - l0, unit_entry((l1 - l0 + CD::RT - 1) / CD::RT * CD::NC, CD::RPC, cw), xs_, qs_, cw, lane, wc, L, [&](int row0, float c, int nvalid) {
+      if ((lane & 3) == 0 && (lane >> 2) < nvalid) {
+        const int row = P.vocab_base + l0 + row0 + (lane >> 2);     // index in the full vocabulary
         const float y = c / P.logits_scaling;
         if (P.d_logits) P.d_logits[row] = y;
         if (y > bv || (y == bv && row < bi)) { bv = y; bi = row; }
@@ -914,9 +832,11 @@ __global__ void __launch_bounds__(kThreads, 1) decode_mega2(const __grid_constan
       ll_store(P.cand_ll + 2 * b + 1, (uint32_t)bi, tg_lm);
     }
     if (b == 0) {
-      uint32_t* cs = reinterpret_cast<uint32_t*>(sm.xh);
+      uint32_t* cs = reinterpret_cast<uint32_t*>(sm.x8);
       named_bar_sync(kBarConsumers, kConsumerThreads);
-      ll_gather<2>(P.cand_ll, 2 * G, tg_lm, cs, tid_c, kConsumerThreads, wc, L);
+      uint2 cand[1];
+      ll_gather<1>(P.cand_ll, G, tg_lm, cand, tid_c, kConsumerThreads, wc, L);
+      if (tid_c < G) *reinterpret_cast<uint2*>(cs + 2 * tid_c) = cand[0];
       named_bar_sync(kBarConsumers, kConsumerThreads);
       if (cw == 0) {
         float v = -INFINITY;
