@@ -6,7 +6,7 @@ import sys
 HERE = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(os.path.dirname(HERE))
 LIB = os.environ.get("FLINT_B200_BUILD_OUT") or os.path.join(os.path.dirname(HERE), "libflintb200.so")
-SOURCES = ["fb_api.cu", "fb_pass.cu", "fb_spec.cu"]
+SOURCES = ["fb_api.cu", "fb_decode_tp.cu", "fb_pass.cu", "fb_spec.cu"]
 HEADERS = sorted(f for f in os.listdir(HERE) if f.endswith((".cuh", ".h", ".hpp"))) + [os.path.join(ROOT, "include", "flint_b200.h")]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-lineinfo", "-std=c++17",
               "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr"]

@@ -17,36 +17,21 @@ namespace {
 
 struct KernelEntry {
   int dim, ko, ffn, head_dim, rgqa, hz;
-  const void* fn;
+  const void* fn;          // the kernel of a single GPU; none where the attention output is not as wide as the model
   int nps;                 // K/V positions per ring stage (the box of the cache tensors)
 };
 
-// KD: model width, KO: attention output width of this rank, KF: FFN width of this rank
-#define FB_DECODE_ENTRY(KD, KO, KF, HD, R)                                                        \
-  {KD, KO, KF, HD, R, 0, (const void*)decode_mega2<KD, KO, KF, HD, R, false>, AttnCfg<HD, DecodePlan<KD, KO, KF>::STAGE>::NPS},   \
-  {KD, KO, KF, HD, R, 1, (const void*)decode_mega2<KD, KO, KF, HD, R, true>, AttnCfg<HD, DecodePlan<KD, KO, KF>::STAGE>::NPS}
+template <int KD, int KO, int KF, int HD, int R, bool HZ>
+const void* single_gpu_kernel() {
+  if constexpr (KO == KD) return (const void*)decode_mega2<KD, KO, KF, HD, R, HZ, false>;
+  else return nullptr;
+}
+#define FB_DECODE_ENTRY(KD, KO, KF, HD, R)                                                                                      \
+  {KD, KO, KF, HD, R, 0, single_gpu_kernel<KD, KO, KF, HD, R, false>(), AttnCfg<HD, DecodePlan<KD, KO, KF>::STAGE>::NPS},        \
+  {KD, KO, KF, HD, R, 1, single_gpu_kernel<KD, KO, KF, HD, R, true>(), AttnCfg<HD, DecodePlan<KD, KO, KF>::STAGE>::NPS}
 
 const KernelEntry kDecodeKernels[] = {
-    FB_DECODE_ENTRY(512, 512, 1408, 64, 4),  // tiny test decoder
-    FB_DECODE_ENTRY(512, 512, 1536, 64, 4),       // tiny decoder whose FFN splits into whole groups over 2 ranks
-    FB_DECODE_ENTRY(512, 256, 768, 64, 4),        // ... and its 2-rank slice
-    FB_DECODE_ENTRY(640, 640, 1024, 80, 4),       // small decoder with heads of 80 ...
-    FB_DECODE_ENTRY(640, 384, 512, 80, 4),        // ... whose 2-rank slice reads a widened O window (320 columns in 3 groups)
-    FB_DECODE_ENTRY(2560, 2560, 8192, 80, 4),   // 3B-class (32 q / 8 kv heads of 80)
-#ifndef FB_KERNELS_MINIMAL                        // (a build for kernel experiments keeps only the shapes above)
-    FB_DECODE_ENTRY(2560, 2560, 8192, 64, 5),     // the reference's native Granite shape (40 q / 8 kv heads of 64)
-    FB_DECODE_ENTRY(4096, 4096, 14336, 128, 4),   // 8B-class
-    FB_DECODE_ENTRY(2560, 1280, 4096, 80, 4),     // 3B-class over 2 GPUs
-    FB_DECODE_ENTRY(2560, 640, 2048, 80, 4),      // 3B-class over 4 GPUs
-    FB_DECODE_ENTRY(2560, 384, 1024, 80, 4),      // 3B-class over 8 GPUs (320 attention columns inside 3 whole groups)
-    FB_DECODE_ENTRY(4096, 2048, 7168, 128, 4),    // 8B-class over 2 GPUs
-    FB_DECODE_ENTRY(4096, 1024, 3584, 128, 4),    // 8B-class over 4 GPUs
-    FB_DECODE_ENTRY(4096, 512, 1792, 128, 4),     // 8B-class over 8 GPUs
-    FB_DECODE_ENTRY(2048, 2048, 8192, 64, 4),     // 1B-class (32 q / 8 kv heads of 64)
-#endif
-#ifdef FB_EXTRA_DECODE_ENTRIES                    // further shapes named at build time (csrc/build.py: FLINT_B200_EXTRA_SHAPES)
-    FB_EXTRA_DECODE_ENTRIES
-#endif
+#include "fb_decode_shapes.h"
 };
 constexpr int kNumDecodeKernels = sizeof(kDecodeKernels) / sizeof(kDecodeKernels[0]);
 
@@ -57,6 +42,8 @@ void o_window(int width, int rank, int* ko, int* off) {
   *ko = hi - lo;
   *off = start - lo;
 }
+
+const void* kernel_of(int id, int tp_size) { return tp_size > 1 ? decode_tp_kernel(id) : kDecodeKernels[id].fn; }
 
 int find_kernel(const fb_model_desc& d, int ko) {
   if (d.n_kv_head <= 0 || d.n_head % d.n_kv_head) return -1;
@@ -80,15 +67,14 @@ int chunks_for(const fb_ctx* c, int T) {
   return n < c->maxchunks ? n : c->maxchunks;
 }
 
-// Bulk copies a CTA keeps in flight while the layers run. A layer that brings each SM at most two rings of weights and K/V spends far
-// longer on its hand-overs than one copy at a time (about 2.2 TB/s over all SMs) takes, and the flags and tagged words then wait
-// behind less bulk traffic; more bytes need the full rate. Microseconds a token at 4 / 2 / 1 copies, by rings a layer:
-//   3B-class   1.5: 1002 / 994 / 985    1.7: 1057 / 1056 / 1040   1.8: 1094 / 1090 / 1084   2.0 (5000 cached): 1149 / 1155 / 1141
-//              2.25: 1206 / 1204 / 1185   2.6: 1287 / 1294 / 1282   3.4: 1452 / 1460 / 1480   4.3: 1623 / 1658 / 1742
-//   40 heads   1.5: 1021 / 1011 / 1003   1.6: 1075 / 1075 / 1067   1.75: 1126 / 1131 / 1132   1.9: 1143 / 1152 / 1151   2.1: 1184 / 1195 / 1188
-//   1B-class   1.2: 394 / 391 / 387   1.4: 422 / 421 / 421   1.75: 441 / 437 / 436         8B-class   4.5: 1621 / 1667 / 1759
-// Up to 1.7 rings one copy gains on every shape, from 3.4 on it loses; in between the shapes differ by up to 1.8 % either way, and two copies
-// are never the best. The LM head has no hand-over to disturb: always 4.
+// Bulk copies a CTA keeps in flight while the layers run. A layer that brings each SM less than two rings of weights and K/V spends far
+// longer on its hand-overs than on the copies, and the tagged words then wait behind less bulk traffic; more bytes, or copies of less than 20 KB, need
+// the full rate. Microseconds a token at 1 / 2 / 3 / 4 copies (cached positions, rings a layer):
+//   3B-class   20, 1.6: 739 / 730 / 734 / 733   200, 1.6: 804 / 794 / 799 / 798   2000, 1.8: 830 / 819 / 820 / 819   4000, 2.0: 900 / 883 / 877 / 875
+//              8000, 2.3: 960 / 953 / 949 / 946   32700, 4.7: 1589 / 1473 / 1438 / 1431
+//   40 heads   600, 1.7: 794 / 788 / 794 / 796   1500, 1.75: 810 / 802 / 809 / 809   3900, 1.9: 876 / 864 / 859 / 860
+//   1B-class (copies of 17 KB)   22, 1.2: 289 / 284 / 281 / 280   3900, 1.6: 348 / 343 / 341 / 340        8B-class, 200: 1409 / 1326 / 1292 / 1287
+// The LM head has no hand-over to disturb: always 4.
 constexpr int64_t kRingBytes = 184320;      // a ring of eight 22.5 KB stages
 int fly_for(const fb_ctx* c, int T) {
   if (c->max_fly) return c->max_fly;
@@ -97,7 +83,8 @@ int fly_for(const fb_ctx* c, int T) {
   const int64_t bytes = (int64_t)(d.n_head + 2 * d.n_kv_head) * HD * rec_bytes_of(d.dim, hz) + (int64_t)d.dim * rec_bytes_of(c->ko, hz) +
                         (int64_t)2 * d.ffn * rec_bytes_of(d.dim, hz) + (int64_t)d.dim * rec_bytes_of(d.ffn, hz) +
                         (int64_t)T * d.n_kv_head * HD * 4;
-  return bytes <= (int64_t)2 * kRingBytes * c->sm_count ? 1 : 4;
+  const int chunk = chunk_bytes(tile_rt(d.dim), chunk_k(d.dim), hz), copy = kRingBytes / kStages / chunk * chunk;
+  return bytes * 10 <= (int64_t)18 * kRingBytes * c->sm_count && copy >= 20000 ? 2 : 4;
 }
 
 // every K the stand-alone entry points (re-layout, dequantise, GEMV) are built for
@@ -270,7 +257,7 @@ int fb_ctx_create_tp(const fb_model_desc* desc, int device, int32_t tp_rank, int
     for (int i = 0; i < d.head_dim / 2; i++) invf[i] = (float)pow((double)d.rope_base, -2.0 * i / d.head_dim);
     A(cudaMemcpy(c->invf, invf, sizeof(float) * (d.head_dim / 2), cudaMemcpyHostToDevice));
     A(cudaMemset(c->status, 0, sizeof(DevStatus)));
-    A(cudaFuncSetAttribute(kDecodeKernels[kid].fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes));
+    A(cudaFuncSetAttribute(kernel_of(kid, tp_size), cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes));
   }
   if (e != cudaSuccess) {
     fb_ctx_destroy(c);
@@ -302,7 +289,7 @@ int fb_set_option(fb_ctx* c, int32_t what, int64_t value) {
   if (what == 5) return FB_OK;                                             // 5, 7, 8: accepted, without effect: one implementation
   if (what == 8) return value < 0 || value > 2 ? FB_ERR_ARG : FB_OK;
   if (what == 7) return value < 0 || value > 4 ? FB_ERR_ARG : FB_OK;
-  if (what == 4) { if (value < 1 || value > kStages / 2) return FB_ERR_ARG; c->max_fly = (int)value; return FB_OK; }
+  if (what == 4) { if (value < 1 || value > kStages - 1) return FB_ERR_ARG; c->max_fly = (int)value; return FB_OK; }
   if (what == 2) { c->prof = (long long*)(uintptr_t)value; return FB_OK; } // device int64[sm_count * n_layer * 16] phase stamps (ns), 0 = off
   return FB_ERR_ARG;
 }
@@ -497,7 +484,7 @@ int fb_decode(fb_ctx* c, int32_t token, const int32_t* d_token, void* d_h, int32
     Q.peer_inbox[p] = c->peer_inbox[p];
   }
   void* args2[] = {&Q};
-  FB_CUDA(c, cudaLaunchCooperativeKernel(kDecodeKernels[c->kernel_id].fn, dim3(c->sm_count), dim3(kThreads), args2, (size_t)kSmemBytes,
+  FB_CUDA(c, cudaLaunchCooperativeKernel(kernel_of(c->kernel_id, c->tp_size), dim3(c->sm_count), dim3(kThreads), args2, (size_t)kSmemBytes,
                                          (cudaStream_t)stream));
   c->tag_base += span;
   return FB_OK;

@@ -82,3 +82,6 @@ void pass_free(fb_ctx* c);
 // one stacked weight matrix in the layouts the passes read (order / arg / orows as in fb_repack)
 cudaError_t pass_bind_matrix(fb_ctx* c, int which, const void* q, const void* s, const void* z, int layers, int rows, int k, int order,
                              int arg, int orows, cudaStream_t st);
+
+// ---- the decode kernels of tensor-parallel ranks (fb_decode_tp.cu), by index into fb_api.cu's table
+const void* decode_tp_kernel(int id);

@@ -16,7 +16,7 @@ struct Pipe {
   uint64_t* empty;
   volatile int* landed;  // stage loads that are known to be complete (written by the producer, read by consumers)
   uint32_t it;           // running stage-load counter; producer and consumers walk the same sequence
-  uint32_t max_fly;      // producer only: bulk copies allowed in flight at once (1..kStages/2)
+  uint32_t max_fly;      // producer only: bulk copies allowed in flight at once (1..kStages - 1)
   uint32_t stage_bytes;  // SmemPlan::STAGE
 };
 
