@@ -77,13 +77,14 @@ int fb_sample(const float* d_logits, int32_t vocab, int32_t rows, int64_t row_st
   if (!d_logits || !d_out || vocab <= 0 || rows <= 0 || row_stride < 0) return FB_ERR_ARG;
   const int c = row_ctas(vocab);
   const bool reg = (vocab + c - 1) / c <= kSampleRegs * 1024;
+  const bool select = temperature > 0.f && top_k > 0 && top_k < vocab;
+  const auto kern = select ? (reg ? sample_rows<true, true> : sample_rows<false, true>) : (reg ? sample_rows<true, false> : sample_rows<false, false>);
   const int64_t most = 0x7fffffff / c;              // rows of one launch: grid.x holds every CTA of every row
   for (int64_t r0 = 0; r0 < rows; r0 += most) {
     const int64_t n = rows - r0 < most ? rows - r0 : most;
     const SampleParams p{d_logits + r0 * row_stride, (long long)row_stride, vocab, top_k, temperature, (unsigned long long)seed,
                          (unsigned long long)counter + (unsigned long long)r0, d_out + r0, c};
-    const cudaError_t e = launch_pdl_cluster(reg ? sample_rows<true> : sample_rows<false>, dim3((unsigned)(n * c)), dim3(1024), 0,
-                                             (cudaStream_t)stream, c, p);
+    const cudaError_t e = launch_pdl_cluster(kern, dim3((unsigned)(n * c)), dim3(1024), 0, (cudaStream_t)stream, c, p);
     if (e != cudaSuccess) return FB_ERR_CUDA;
   }
   return FB_OK;

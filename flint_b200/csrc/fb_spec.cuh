@@ -30,6 +30,7 @@ __device__ __forceinline__ uint32_t fkey(float f) {
   const uint32_t u = __float_as_uint(f);
   return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
 }
+__device__ __forceinline__ float fkey_value(uint32_t k) { return __uint_as_float((k & 0x80000000u) ? k & 0x7fffffffu : ~k); }
 
 // ------------------------------------------------------------------------------------------------ sampling
 struct SampleParams {
@@ -44,14 +45,28 @@ struct SampleParams {
 
 // One cluster of CTAs per row: a CTA keeps its slice of the row in registers (up to 16 values a thread; longer slices are read again),
 // so a row is read once, by several SMs. top-k keeps every entry >= the k-th largest value (ties included, as `logits < v[-1] -> -inf`
-// does, reference: engine/generate.py:41-45); the k-th largest is found exactly by a radix select on order-preserving keys in three
-// digits of 11, 11 and 10 bits: every CTA counts its own slice and reads the others' counts from their shared memory. The draw is arg-max of logit / T + Gumbel noise,
-// which is a sample of softmax(logits / T) over the kept entries: the same distribution as arg-max(p / Exponential(1)) (reference:
-// engine/generate.py:37-39). Bound by latency: four cluster barriers and three scans. (One CTA per row took 83 us for a row of 128256
-// values and k = 50: five passes of 512 KB through one SM, most of the first digit's atomics on a handful of bins.)
+// does, reference: engine/generate.py:41-45). The draw is arg-max of logit / T + Gumbel noise, which is a sample of softmax(logits / T) over the kept
+// entries: the same distribution as arg-max(p / Exponential(1)) (reference: engine/generate.py:37-39).
+// Up to 4/5 as many kept entries as the row has warps (256 for a row of 8 CTAs): the k-th largest of the warps' maxima bounds the k-th largest value from
+// below, and few values lie above it (about 60 for k = 50 of 128256 normal values, 400 for k = 200). They go to the first CTA's list, where an entry
+// is kept if fewer than k entries are larger: two cluster barriers and no histogram. More kept entries, or so many ties that the list is
+// full: radix select on order-preserving keys in three digits of 11, 11 and 10 bits; every CTA counts its own slice and reads the others'
+// counts from their shared memory: four cluster barriers, three scans, and most of the first digit's atomics on a handful of bins.
+// Logits of 128256 entries, one row, k = 50: 16.4 us with the radix select, 7.5 with the list (a call back to back: 10, the host's part); 16 rows of k = 50 / 200 33.6 / 34.4
+// -> 14.4 / 17.9, 64 rows 87 / 89 -> 37 / 42. Without top-k, in a kernel without the selection: 64 rows arg-max 24.2 -> 19.3, draw 53 -> 47. (One CTA per row and five passes took 83 us for one row.)
 constexpr int kSampleRegs = 16;
 // Another CTA's shared memory may be touched only once that CTA is known to run. Every CTA of the cluster arrives at the start of the kernel
 // and waits before its first remote access: the row's loads lie in between and hide the barrier.
+__device__ __forceinline__ uint32_t ld_cluster_u32(uint32_t a) {
+  uint32_t v;
+  asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
+  return v;
+}
+__device__ __forceinline__ uint32_t add_cluster(uint32_t a, uint32_t n) {
+  uint32_t old;
+  asm volatile("atom.relaxed.cluster.shared::cluster.add.u32 %0, [%1], %2;" : "=r"(old) : "r"(a), "r"(n) : "memory");
+  return old;
+}
 __device__ __forceinline__ uint2 ld_cluster(uint32_t a) {
   uint2 v;
   asm volatile("ld.shared::cluster.v2.u32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(a) : "memory");
@@ -72,10 +87,12 @@ __device__ __forceinline__ void warp_best(float& bv, int& bi) {
 
 // grid (rows * CTAs per row), clusters of one row's CTAs, 1024 threads. Rows lie on grid.x: grid.y ends at 65535, and a program may
 // draw any number of rows from one vector (stride 0).
-template <bool REG>
+constexpr int kSampleList = 1024;                 // candidates of the short selection: one per thread
+// SELECT: a draw with top-k
+template <bool REG, bool SELECT>
 __global__ void __launch_bounds__(1024) sample_rows(const SampleParams P) {
-  __shared__ __align__(8) unsigned hist[3][2048];
-  __shared__ unsigned s_warp[32], s_bin, s_k;
+  __shared__ __align__(16) unsigned hist[SELECT ? 3 : 1][SELECT ? 2048 : 4];                 // radix select; the short selection: keys of the warps' maxima, of the list, indices of the list
+  __shared__ unsigned s_warp[32], s_bin, s_k, s_cnt;
   __shared__ float s_v[32];
   __shared__ int s_i[32];
   __shared__ float c_v[16];                       // the CTAs' candidates, in the first CTA
@@ -83,8 +100,9 @@ __global__ void __launch_bounds__(1024) sample_rows(const SampleParams P) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, C = P.ctas, row = blockIdx.x / C, rank = blockIdx.x % C;
   const float* lg = P.logits + (long long)row * P.row_stride;
   const int per = (P.vocab + C - 1) / C, i0 = rank * per, i1 = min(P.vocab, i0 + per);
-  const bool draw = P.temperature > 0.f, select = draw && P.top_k > 0 && P.top_k < P.vocab;
-  if (!select) cluster_arrive();                  // the selection's own barriers come before its first remote read
+  const bool draw = SELECT || P.temperature > 0.f, brief = SELECT && P.top_k <= C * 32 * 4 / 5;
+  if (tid == 0) s_cnt = 0u;
+  if (!SELECT || brief) cluster_arrive();         // the radix select's own barriers come before its first remote read
   pdl_trigger();
   pdl_wait();
   float v[REG ? kSampleRegs : 1];
@@ -101,8 +119,103 @@ __global__ void __launch_bounds__(1024) sample_rows(const SampleParams P) {
       for (int i = i0 + tid; i < i1; i += 1024) f(i, lg[i]);
     }
   };
+  const float inv_t = draw ? 1.0f / P.temperature : 1.0f;
+  auto score = [&](int i, float x) { return draw ? x * inv_t + gumbel(mix32(P.seed, P.counter + (unsigned long long)row, (uint32_t)i)) : x; };
+  float bv = -INFINITY;
+  int bi = 0x7fffffff;
+  if (SELECT && brief) {
+    unsigned *wkey = hist[0], *lkey = hist[SELECT], *lidx = hist[SELECT] + kSampleList;
+    uint32_t top = 0u;
+    each([&](int, float x) { top = max(top, fkey(x)); });
+    top = __reduce_max_sync(0xffffffffu, top);
+    cluster_wait();
+    if (lane < C) st_cluster(cluster_map((uint32_t)__cvta_generic_to_shared(wkey + rank * 32 + warp), lane), top);
+    cluster_sync();
+    if (warp == 0) {
+      // the largest 16-bit prefix that at least k of the maxima reach
+      uint32_t w[8], lo = 0xffffu, hi = 0u;
+#pragma unroll
+      for (int c = 0; c < 8; c++) {
+        w[c] = c < C ? wkey[c * 32 + lane] >> 16 : 0u;
+        if (c < C) { lo = min(lo, w[c]); hi = max(hi, w[c]); }
+      }
+      lo = __reduce_min_sync(0xffffffffu, lo);
+      hi = __reduce_max_sync(0xffffffffu, hi);
+      while (lo < hi) {                                          // at least k reach lo
+        const uint32_t mid = (lo + hi + 1) / 2;
+        unsigned n = 0;
+#pragma unroll
+        for (int c = 0; c < 8; c++) n += w[c] >= mid;
+        if (__reduce_add_sync(0xffffffffu, n) >= (unsigned)P.top_k) lo = mid;
+        else hi = mid - 1;
+      }
+      if (lane == 0) s_bin = lo << 16;
+    }
+    __syncthreads();
+    const uint32_t floor = s_bin;
+    unsigned own = 0;
+    each([&](int, float x) { own += fkey(x) >= floor; });
+    const unsigned all = __reduce_add_sync(0xffffffffu, own);
+    if (all) {
+      unsigned at = own;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const unsigned u = __shfl_up_sync(0xffffffffu, at, o);
+        if (lane >= o) at += u;
+      }
+      unsigned base = 0;
+      if (lane == 0) base = add_cluster(cluster_map((uint32_t)__cvta_generic_to_shared(&s_cnt), 0), all);
+      at += __shfl_sync(0xffffffffu, base, 0) - own;
+      if (own) {
+        const uint32_t k0 = cluster_map((uint32_t)__cvta_generic_to_shared(lkey), 0), x0 = cluster_map((uint32_t)__cvta_generic_to_shared(lidx), 0);
+        each([&](int i, float x) {
+          if (fkey(x) >= floor) {
+            if (at < kSampleList) {
+              st_cluster(k0 + at * 4, fkey(x));
+              st_cluster(x0 + at * 4, (uint32_t)i);
+            }
+            at++;
+          }
+        });
+      }
+    }
+    cluster_sync();
+    const unsigned n = ld_cluster_u32(cluster_map((uint32_t)__cvta_generic_to_shared(&s_cnt), 0));
+    cluster_arrive();                             // the first CTA stays until the others have read its count
+    if (n <= kSampleList) {
+      if (rank == 0) {
+        const unsigned n4 = (n + 3) / 4 * 4;
+        if (tid >= (int)n && tid < (int)n4) lkey[tid] = 0u;
+        __syncthreads();
+        if (tid < (int)n) {
+          const uint32_t mine = lkey[tid];
+          unsigned larger = 0;
+#pragma unroll 4
+          for (unsigned c = 0; c < n4; c += 4) {
+            const uint4 o = *reinterpret_cast<const uint4*>(lkey + c);
+            larger += (o.x > mine) + (o.y > mine) + (o.z > mine) + (o.w > mine);
+          }
+          if (larger < (unsigned)P.top_k) {
+            const int i = (int)lidx[tid];
+            take_best(bv, bi, score(i, fkey_value(mine)), i);
+          }
+        }
+        warp_best(bv, bi);
+        if (lane == 0) { s_v[warp] = bv; s_i[warp] = bi; }
+        __syncthreads();
+        if (warp == 0) {
+          bv = s_v[lane]; bi = s_i[lane];
+          warp_best(bv, bi);
+          if (lane == 0) P.out[row] = bi == 0x7fffffff ? 0 : bi;
+        }
+      }
+      cluster_wait();
+      return;
+    }
+    cluster_wait();
+  }
   uint32_t thr = 0u;
-  if (select) {
+  if constexpr (SELECT) {
     for (int i = tid; i < 2048; i += 1024) { hist[0][i] = hist[1][i] = hist[2][i] = 0u; }
     __syncthreads();
     uint32_t prefix = 0u, mask = 0u;
@@ -154,18 +267,13 @@ __global__ void __launch_bounds__(1024) sample_rows(const SampleParams P) {
     }
     thr = prefix;                                 // key of the k-th largest value
   }
-  float bv = -INFINITY;
-  int bi = 0x7fffffff;
-  const float inv_t = draw ? 1.0f / P.temperature : 1.0f;
   each([&](int i, float x) {
-    if (fkey(x) < thr) return;
-    const float sc = draw ? x * inv_t + gumbel(mix32(P.seed, P.counter + (unsigned long long)row, (uint32_t)i)) : x;
-    take_best(bv, bi, sc, i);
+    if (!SELECT || fkey(x) >= thr) take_best(bv, bi, score(i, x), i);
   });
   warp_best(bv, bi);
   if (lane == 0) { s_v[warp] = bv; s_i[warp] = bi; }
   __syncthreads();
-  if (!select) cluster_wait();
+  if (!SELECT) cluster_wait();
   if (warp == 0) {
     bv = s_v[lane]; bi = s_i[lane];
     warp_best(bv, bi);
