@@ -25,7 +25,8 @@ struct fb_draft {
 namespace {
 
 constexpr int kMaxHeadRows = 16;
-constexpr int kAttnSmem = 200 * 1024;            // d_attn holds a score per cache slot and the query: more than the 48 KB that need no asking
+constexpr int kAttnSmem = 200 * 1024;            // d_attn's scores of every cache slot and the query (more than the 48 KB that need no asking) ...
+constexpr int kAttnSmemNew = 8 * 1024;           // ... and the new k and v of a single token (d_attn_one)
 
 template <int NT, int MT, int MODE>
 cudaError_t launch_linear_nt(DLin p, int t0, int sms, cudaStream_t st) {
@@ -33,8 +34,10 @@ cudaError_t launch_linear_nt(DLin p, int t0, int sms, cudaStream_t st) {
   for (int i = 0; i < (MODE == DL_STORE ? 3 : 1) && p.W[i]; i++) blocks += (p.N[i] + 16 * MT - 1) / (16 * MT);
   p.ks = MODE == DL_LOGITS ? 1 : draft_splits(blocks, (p.k0 + p.k1 + 31) / 32, NT, sms);
   const dim3 grid(blocks * p.ks), block(kDraftWarps * 32);
-  if (MODE == DL_STORE && p.x1) return launch_pdl_cluster(d_gemm<NT, MT, MODE, MODE == DL_STORE>, grid, block, 0, st, (unsigned)p.ks, p, t0);
-  return launch_pdl_cluster(d_gemm<NT, MT, MODE, false>, grid, block, 0, st, (unsigned)p.ks, p, t0);
+  constexpr bool FOLDS = NT == 1 && (MODE == DL_STORE || MODE == DL_SWIGLU);
+  if (MODE == DL_STORE && p.x1) return launch_pdl_cluster(d_gemm<NT, MT, MODE, MODE == DL_STORE, false>, grid, block, 0, st, (unsigned)p.ks, p, t0);
+  if (FOLDS && p.norm_w) return launch_pdl_cluster(d_gemm<NT, MT, MODE, false, FOLDS>, grid, block, 0, st, (unsigned)p.ks, p, t0);
+  return launch_pdl_cluster(d_gemm<NT, MT, MODE, false, false>, grid, block, 0, st, (unsigned)p.ks, p, t0);
 }
 // All T tokens, up to 32 per pass over the weights. Up to 8 tokens: 16 rows per CTA and three CTAs per SM. More tokens: 32 rows per CTA (one
 // matrix) or 16 of each of two, so that a CTA reads about as many bytes of activations from L2 as of weights, and two CTAs per SM.
@@ -50,6 +53,11 @@ cudaError_t launch_linear(const DLin& p, int sms, cudaStream_t st) {
     else e = launch_linear_nt<4, MW, MODE>(p, t0, sms, st);
   }
   return e;
+}
+// RMSNorm of n rows, `first`: the first kernel of a call, which nothing hides: in registers (one row, step and token head 118.5 -> 117.2 us at 3B, 136.6 -> 135.4 at 1B;
+// inside the block no faster at 3B and 1 us slower at 1B)
+cudaError_t launch_norm(const uint16_t* x, int ldx, const void* w, uint16_t* y, int n, int D, float eps, bool first, cudaStream_t st) {
+  return launch_pdl(first && D <= kNormRegs * 256 ? d_rmsnorm_regs : d_rmsnorm, dim3(n), dim3(256), 0, st, x, ldx, (const uint16_t*)w, y, D, D, eps, first);
 }
 // CTAs per row of the token choice: slices of at least 4096 values, at most 8 CTAs (the portable cluster)
 int row_ctas(int vocab) {
@@ -136,6 +144,7 @@ int fb_draft_create(const fb_draft_desc* desc, int device, fb_draft** out) {
   auto A = [&](cudaError_t x) { if (e == cudaSuccess) e = x; };
   A(cudaDeviceGetAttribute(&r->sm_count, cudaDevAttrMultiProcessorCount, device));
   A(cudaFuncSetAttribute(d_attn, cudaFuncAttributeMaxDynamicSharedMemorySize, kAttnSmem));
+  A(cudaFuncSetAttribute(d_attn_one, cudaFuncAttributeMaxDynamicSharedMemorySize, kAttnSmem + kAttnSmemNew));
   A(dmalloc(&r->x, T * D * 2)); A(dmalloc(&r->h, T * D * 2)); A(dmalloc(&r->q, T * D * 2));
   A(dmalloc(&r->k, T * kvd * 2)); A(dmalloc(&r->v, T * kvd * 2)); A(dmalloc(&r->att, T * D * 2));
   A(dmalloc(&r->x2, T * D * 2)); A(dmalloc(&r->act, T * (size_t)d.inter * 2)); A(dmalloc(&r->hh, T * D * 2));
@@ -188,28 +197,36 @@ int fb_draft_forward(fb_draft* r, const void* d_feat, const void* d_emb, const i
   else { p.x1 = (const uint16_t*)r->w.embed; p.ldx1 = D; p.x1_tokens = d_tokens; p.x1_rows = d.vocab; }
   p.k1 = D; p.N[0] = D; p.T = T; p.y[0] = r->x; p.ldy[0] = D; p.first = true;
   FB_DCUDA(r, launch_linear<DL_STORE>(p, r->sm_count, st));
-  FB_DCUDA(r, launch_pdl(d_rmsnorm, dim3(T), dim3(256), 0, st, (const uint16_t*)r->x, D, (const uint16_t*)r->w.n1, r->h, D, D, d.rms_eps, false));
+  const bool fold = draft_folds_norm(T, D);
+  if (!fold) FB_DCUDA(r, launch_norm(r->x, D, r->w.n1, r->h, T, D, d.rms_eps, false, st));
   // q, k, v in one launch
   memset(&p, 0, sizeof(p));
   const void* qkvw[3] = {r->w.q, r->w.k, r->w.v};
   uint16_t* qkvo[3] = {r->q, r->k, r->v};
   const int qkvn[3] = {D, kvd, kvd};
   for (int i = 0; i < 3; i++) { p.W[i] = (const uint16_t*)qkvw[i]; p.N[i] = qkvn[i]; p.y[i] = qkvo[i]; p.ldy[i] = qkvn[i]; }
-  p.x0 = r->h; p.ldx0 = D; p.k0 = D; p.T = T;
+  p.x0 = fold ? r->x : r->h; p.ldx0 = D; p.k0 = D; p.T = T; p.norm_w = fold ? (const uint16_t*)r->w.n1 : nullptr; p.norm_eps = d.rms_eps;
   FB_DCUDA(r, launch_linear<DL_STORE>(p, r->sm_count, st));
-  FB_DCUDA(r, launch_pdl(d_rope_store, dim3(T, d.n_head + d.n_kv_head), dim3(64), 0, st, r->q, (const uint16_t*)r->k, (const uint16_t*)r->v, d_positions,
-                         d_slots, r->kc, r->vc, d.n_head, d.n_kv_head, hd, d.rope_base, d.max_roll));
-  FB_DCUDA(r, launch_pdl(d_attn, dim3(T, d.n_head), dim3(128), (size_t)(d.max_roll + hd) * 4, st, (const uint16_t*)r->q, d_slots,
-                         (const uint16_t*)r->kc, (const uint16_t*)r->vc, r->att, d.n_head, d.n_kv_head, hd, d.max_roll));
+  const size_t asmem = (size_t)(d.max_roll + hd) * 4, news = (size_t)hd * 8;
+  if (T == 1 && news <= kAttnSmemNew && asmem <= kAttnSmem) {
+    FB_DCUDA(r, launch_pdl(d_attn_one, dim3(d.n_head), dim3(128), asmem + news, st, (const uint16_t*)r->q, (const uint16_t*)r->k, (const uint16_t*)r->v,
+                           d_positions, d_slots, r->kc, r->vc, r->att, d.n_head, d.n_kv_head, hd, d.rope_base, d.max_roll));
+  } else {
+    FB_DCUDA(r, launch_pdl(d_rope_store, dim3(T, d.n_head + d.n_kv_head), dim3(64), 0, st, r->q, (const uint16_t*)r->k, (const uint16_t*)r->v, d_positions,
+                           d_slots, r->kc, r->vc, d.n_head, d.n_kv_head, hd, d.rope_base, d.max_roll));
+    FB_DCUDA(r, launch_pdl(d_attn, dim3(T, d.n_head), dim3(128), asmem, st, (const uint16_t*)r->q, d_slots, (const uint16_t*)r->kc,
+                           (const uint16_t*)r->vc, r->att, d.n_head, d.n_kv_head, hd, d.max_roll));
+  }
   // x2 = x + o(att)
   memset(&p, 0, sizeof(p));
   p.W[0] = (const uint16_t*)r->w.o; p.x0 = r->att; p.ldx0 = D; p.k0 = D; p.N[0] = D; p.T = T; p.y[0] = r->x2; p.ldy[0] = D;
   p.resid = r->x; p.ldr = D;
   FB_DCUDA(r, launch_linear<DL_RESID>(p, r->sm_count, st));
-  FB_DCUDA(r, launch_pdl(d_rmsnorm, dim3(T), dim3(256), 0, st, (const uint16_t*)r->x2, D, (const uint16_t*)r->w.n2, r->h, D, D, d.rms_eps, false));
+  if (!fold) FB_DCUDA(r, launch_norm(r->x2, D, r->w.n2, r->h, T, D, d.rms_eps, false, st));
   // act = silu(gate h) * up h
   memset(&p, 0, sizeof(p));
-  p.W[0] = (const uint16_t*)r->w.gate; p.W2 = (const uint16_t*)r->w.up; p.x0 = r->h; p.ldx0 = D; p.k0 = D; p.N[0] = d.inter; p.T = T;
+  p.W[0] = (const uint16_t*)r->w.gate; p.W2 = (const uint16_t*)r->w.up; p.x0 = fold ? r->x2 : r->h; p.ldx0 = D;
+  p.norm_w = fold ? (const uint16_t*)r->w.n2 : nullptr; p.norm_eps = d.rms_eps; p.k0 = D; p.N[0] = d.inter; p.T = T;
   p.y[0] = r->act; p.ldy[0] = d.inter;
   FB_DCUDA(r, launch_linear<DL_SWIGLU>(p, r->sm_count, st));
   // hh = x2 + down(act)
@@ -235,8 +252,8 @@ int fb_draft_head(fb_draft* r, const void* d_feat_rows, int32_t n, int32_t top_b
   cudaStream_t st = (cudaStream_t)stream;
   const int D = d.dim, F = d.fuse * d.dim;
   // the token head reads the HIGH slice (last dim elements) of the fused feature (reference: spec_mega.py:43-44)
-  FB_DCUDA(r, launch_pdl(d_rmsnorm, dim3(n), dim3(256), 0, st, (const uint16_t*)d_feat_rows + (F - D), F, (const uint16_t*)r->w.nf, r->fn, D, D,
-                         d.rms_eps, true));
+  const uint16_t* rows = (const uint16_t*)d_feat_rows + (F - D);
+  FB_DCUDA(r, launch_norm(rows, F, r->w.nf, r->fn, n, D, d.rms_eps, true, st));
   DLin p;
   memset(&p, 0, sizeof(p));
   p.W[0] = (const uint16_t*)r->w.embed; p.x0 = r->fn; p.ldx0 = D; p.k0 = D; p.N[0] = d.vocab; p.T = n; p.yf = r->logits; p.ldy[0] = d.vocab;

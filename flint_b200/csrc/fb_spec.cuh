@@ -436,7 +436,39 @@ struct DLin {
   float scale;
   bool first;                   // the first kernel of a call
   int ks;                       // CTAs of a cluster that share K
+  const uint16_t* norm_w;       // when set (draft_folds_norm): x0 is normalised by every CTA (d_norm_row), weights bf16 [k0]
+  float norm_eps;
 };
+// RMSNorm inside the linear behind it, for a single token whose row fits the registers: every CTA normalises it (an L2 round trip and a block reduction) instead
+// of waiting for a kernel that does (one row, step and token head, with d_attn_one: 120.4 -> 118.5 us at 3B, 140.0 -> 136.6 at 1B, 157.7 -> 155.3 with 40 heads).
+constexpr int kNormRegs = 16;                     // elements of a thread
+__host__ __device__ constexpr bool draft_folds_norm(int T, int D) { return T == 1 && D <= kNormRegs * 256; }
+
+// d_rmsnorm's arithmetic, in its order, with the row in registers (D <= kNormRegs * 256), by a CTA of 256 threads that has yet to wait for the row.
+__device__ __forceinline__ void d_norm_row(const uint16_t* xr, const uint16_t* w, uint16_t* y, int D, float eps, float* red) {
+  const int tid = threadIdx.x;
+  uint16_t wv[kNormRegs], xv[kNormRegs];
+#pragma unroll
+  for (int k = 0; k < kNormRegs; k++) wv[k] = tid + 256 * k < D ? w[tid + 256 * k] : (uint16_t)0;
+  pdl_wait();
+#pragma unroll
+  for (int k = 0; k < kNormRegs; k++) xv[k] = tid + 256 * k < D ? xr[tid + 256 * k] : (uint16_t)0;
+  float ss = 0.f;
+#pragma unroll
+  for (int k = 0; k < kNormRegs; k++) ss += rbf(bf2f(xv[k]) * bf2f(xv[k]));
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+  if ((tid & 31) == 0) red[tid >> 5] = ss;
+  __syncthreads();
+  float tot = 0.f;
+#pragma unroll
+  for (int i = 0; i < 8; i++) tot += red[i];
+  const float r = rbf(rsqrtf(rbf(rbf(tot / (float)D) + eps)));
+#pragma unroll
+  for (int k = 0; k < kNormRegs; k++)
+    if (tid + 256 * k < D) y[tid + 256 * k] = f2bf(rbf(bf2f(xv[k]) * r) * bf2f(wv[k]));
+  __syncthreads();
+}
 
 // y[t, n] = sum_k W[n, k] x[t, k] for up to 8 NT tokens (t0 ...) on the tensor pipe, weights read once. A CTA takes 16 MT rows of W and
 // its WARPS warps share K: warp w takes the 32-column chunks w, w + WARPS, ... A lane loads 16 bytes of row g (and g + 8) straight into
@@ -447,12 +479,13 @@ struct DLin {
 // A matrix whose rows give less than the GPU's worth of CTAs is also cut in K over a cluster of ks: the CTAs push their sums into the shared
 // memory of the one that finishes the token, which adds them in rank order. (With 16 warps and no split a 2560-row matrix ran on 80
 // SMs: block over 32 rows 130.6 -> 105.9 us, 48 rows 202 -> 167; one row, three CTAs an SM, 77.2 without the split, 74.0 with it.)
-template <int NT, int MT, int MODE, bool CAT>
+template <int NT, int MT, int MODE, bool CAT, bool FOLD>
 __global__ void __launch_bounds__(kDraftWarps * 32, NT == 1 ? 3 : 2) d_gemm(const DLin P, int t0) {
   constexpr int WARPS = kDraftWarps;
   constexpr int NW = MODE == DL_SWIGLU ? 2 : 1, AH = NT == 1 && NW == 1 ? 4 : 2, ROWS = 16 * MT * NW;      // weight matrices per row, chunks in flight
   __shared__ float red[8][ROWS][8 * NT + 1];
   __shared__ float part[kDraftSplits][8 * NT][ROWS];             // split K: [source rank][token][row]
+  __shared__ __align__(16) uint16_t xs[FOLD ? kNormRegs * 256 : 8];      // FOLD: the normalised row
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
   const int K = P.k0 + P.k1, nch = (K + 31) >> 5;
   // the token head has CTAs enough
@@ -491,7 +524,9 @@ __global__ void __launch_bounds__(kDraftWarps * 32, NT == 1 ? 3 : 2) d_gemm(cons
   pdl_begin(P.first && t0 == 0);
 #pragma unroll
   for (int a = 0; a < AH; a++) load_w(c1 + step * a, wv[a]);
-  pdl_wait();
+  if constexpr (FOLD) d_norm_row(P.x0, P.norm_w, xs, P.k0, P.norm_eps, &red[0][0][0]);
+  else pdl_wait();
+  const uint16_t* x0 = FOLD ? xs : P.x0;
   int x1[CAT ? NT : 1];                              // second segment: row of each token, or -1
   if (CAT) {
 #pragma unroll
@@ -511,7 +546,7 @@ __global__ void __launch_bounds__(kDraftWarps * 32, NT == 1 ? 3 : 2) d_gemm(cons
       return;
     }
     const bool second = CAT && col >= P.k0;
-    const uint16_t* base = second ? P.x1 + (col - P.k0) : P.x0 + col;
+    const uint16_t* base = second ? P.x1 + (col - P.k0) : x0 + col;
     const int ld = second ? P.ldx1 : P.ldx0;
 #pragma unroll
     for (int j = 0; j < NT; j++) {
@@ -634,6 +669,13 @@ __global__ void __launch_bounds__(256) d_rmsnorm(const uint16_t* x, int ldx, con
     y[(size_t)blockIdx.x * ldy + i] = f2bf(rbf(bf2f(xr[i]) * r) * bf2f(w[i]));
 }
 
+// The same with the row in registers
+__global__ void __launch_bounds__(256) d_rmsnorm_regs(const uint16_t* x, int ldx, const uint16_t* w, uint16_t* y, int ldy, int D, float eps, bool first) {
+  __shared__ float red[8];
+  pdl_begin(first);
+  d_norm_row(x + (size_t)blockIdx.x * ldx, w, y + (size_t)blockIdx.x * ldy, D, eps, red);
+}
+
 // Half-split rotation of q and k (bf16 cos / sin tables as the reference casts them, reference:
 // train/draft_model.py:12-22) and the cache write: token t's rotated k and its v go to cache slot slots[t].
 // grid (T, n_head + n_kv), 64 threads: one CTA per (token, head), a thread per rotation pair (the angle's powf / cosf / sinf are the
@@ -727,6 +769,94 @@ __global__ void __launch_bounds__(128) d_attn(const uint16_t* q, const int32_t* 
 #pragma unroll 8
     for (int s = 0; s <= last; s++) a = fmaf(d_sc[s], bf2f(vc[((size_t)s * nkv + kh) * hd + i]), a);
     out[((size_t)t * nh + head) * hd + i] = f2bf(a / den);
+  }
+}
+
+// d_rope_store and d_attn of a single token in one launch: every query head's CTA rotates its own q and the group's new k, the first of the group
+// writes k and v to the cache, and nobody reads the new rows from there. The same operations in the same order. grid (nh), 128 threads.
+__global__ void __launch_bounds__(128) d_attn_one(const uint16_t* q, const uint16_t* k, const uint16_t* v, const int32_t* positions, const int32_t* slots,
+                                                  uint16_t* kc, uint16_t* vc, uint16_t* out, int nh, int nkv, int hd, float rope_base, int max_roll) {
+  extern __shared__ float d_sc[];                  // [max_roll] scores, [hd] the query, [hd] the new k, [hd] the new v
+  __shared__ float red[4];
+  float *qs = d_sc + max_roll, *ks = qs + hd, *vs = ks + hd;
+  const int head = blockIdx.x, kh = head / (nh / nkv), tid = threadIdx.x;
+  pdl_trigger();
+  pdl_wait();
+  const int slot = slots ? slots[0] : 0, last = min(slot, max_roll - 1);
+  if (last < 0) return;
+  const bool fresh = slot < max_roll;              // else the cache keeps its rows and q stays as it is, as in d_rope_store
+  const uint16_t* qh = q + (size_t)head * hd;
+  if (fresh) {
+    const float pos = (float)positions[0];
+    const bool writes = head % (nh / nkv) == 0;
+    const size_t row = ((size_t)slot * nkv + kh) * hd;
+    const int half = hd >> 1;
+    for (int i = tid; i < half; i += 128) {
+      const float ang = pos * (1.0f / powf(rope_base, (float)(2 * i) / (float)hd));
+      const float c = rbf(cosf(ang)), s = rbf(sinf(ang));
+      const float a = bf2f(qh[i]), b = bf2f(qh[i + half]), e = bf2f(k[kh * hd + i]), f = bf2f(k[kh * hd + i + half]);
+      qs[i] = rbf(rbf(a * c) + rbf(-b * s));
+      qs[i + half] = rbf(rbf(b * c) + rbf(a * s));
+      const uint16_t k0 = f2bf(rbf(e * c) + rbf(-f * s)), k1 = f2bf(rbf(f * c) + rbf(e * s));
+      ks[i] = bf2f(k0);
+      ks[i + half] = bf2f(k1);
+      if (writes) { kc[row + i] = k0; kc[row + i + half] = k1; }
+    }
+    for (int i = tid; i < hd; i += 128) {
+      const uint16_t x = v[kh * hd + i];
+      vs[i] = bf2f(x);
+      if (writes) vc[row + i] = x;
+    }
+  } else {
+    for (int i = tid; i < hd; i += 128) qs[i] = bf2f(qh[i]);
+  }
+  __syncthreads();
+  const float scale = rsqrtf((float)hd);
+  const int cached = fresh ? slot : last + 1;      // rows that come from the cache
+  float mx = -INFINITY;
+  for (int s = tid; s <= last; s += 128) {
+    float d = 0.f;
+    if (s == cached) {
+      for (int i = 0; i < hd; i++) d = fmaf(qs[i], ks[i], d);
+    } else if (hd % 8 == 0) {                        // rows start on 16-byte boundaries
+      const uint16_t* kr = kc + ((size_t)s * nkv + kh) * hd;
+#pragma unroll 4
+      for (int i = 0; i < hd; i += 8) {
+        const uint4 kv = *reinterpret_cast<const uint4*>(kr + i);
+        const uint32_t p[4] = {kv.x, kv.y, kv.z, kv.w};
+#pragma unroll
+        for (int e = 0; e < 4; e++) { d = fmaf(qs[i + 2 * e], bflo(p[e]), d); d = fmaf(qs[i + 2 * e + 1], bfhi(p[e]), d); }
+      }
+    } else {
+      for (int i = 0; i < hd; i++) d = fmaf(qs[i], bf2f(kc[((size_t)s * nkv + kh) * hd + i]), d);
+    }
+    d *= scale;
+    d_sc[s] = d;
+    mx = fmaxf(mx, d);
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+  if ((tid & 31) == 0) red[tid >> 5] = mx;
+  __syncthreads();
+  mx = fmaxf(fmaxf(red[0], red[1]), fmaxf(red[2], red[3]));
+  __syncthreads();
+  float den = 0.f;
+  for (int s = tid; s <= last; s += 128) {
+    const float e = expf(d_sc[s] - mx);
+    d_sc[s] = e;
+    den += e;
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) den += __shfl_xor_sync(0xffffffffu, den, o);
+  if ((tid & 31) == 0) red[tid >> 5] = den;
+  __syncthreads();
+  den = red[0] + red[1] + red[2] + red[3];
+  for (int i = tid; i < hd; i += 128) {
+    float a = 0.f;
+#pragma unroll 8
+    for (int s = 0; s < cached; s++) a = fmaf(d_sc[s], bf2f(vc[((size_t)s * nkv + kh) * hd + i]), a);
+    if (fresh) a = fmaf(d_sc[slot], vs[i], a);
+    out[(size_t)head * hd + i] = f2bf(a / den);
   }
 }
 
