@@ -14,6 +14,7 @@ from typing import Dict, Optional
 import torch
 
 from . import _lib
+from .engine import _stream_ptr
 
 _KEYS = {"merge": "merge.weight", "n1": "n1", "n2": "n2", "q": "q.weight", "k": "k.weight", "v": "v.weight", "o": "o.weight",
          "gate": "gate.weight", "up": "up.weight", "down": "down.weight", "fout": "fout.weight"}
@@ -111,7 +112,7 @@ class DraftHead:
         e2 = None if emb is None else emb.reshape(-1, self.dim).to(torch.bfloat16).contiguous()
         tk = None if tokens is None else tokens.to(device=dev, dtype=torch.int32).contiguous()
         out = torch.empty(T, self.fdim, dtype=torch.bfloat16, device=dev)
-        st = ctypes.c_void_p(torch.cuda.current_stream(dev).cuda_stream)
+        st = _stream_ptr(dev)
         _lib.check(self.lib.fb_draft_forward(self._h, _p(f2), _p(e2), _p(tk), _p(pos), _p(slots), T, _p(out), st),
                    "fb_draft_forward")
         self._keep = (f2, e2, tk, pos, slots)
@@ -125,7 +126,7 @@ class DraftHead:
         n = f2.shape[0]
         toks = torch.empty(n, top_b, dtype=torch.int32, device=f2.device)
         sc = torch.empty(n, top_b, dtype=torch.float32, device=f2.device) if want_scores else None
-        st = ctypes.c_void_p(torch.cuda.current_stream(f2.device).cuda_stream)
+        st = _stream_ptr(f2.device)
         _lib.check(self.lib.fb_draft_head(self._h, _p(f2), n, top_b, _p(toks), _p(sc), st), "fb_draft_head")
         self._keep_h = f2
         return (toks, sc) if want_scores else toks

@@ -21,7 +21,9 @@ def _ptr(t: Optional[torch.Tensor]):
 
 
 def _stream_ptr(device) -> int:
-    return torch.cuda.current_stream(device).cuda_stream
+    """The current stream of a CUDA device, as torch.cuda.current_stream(device).cuda_stream gives it, without the Stream object (2.2 us a call)."""
+    index = device.index
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if index is None else index)
 
 
 def query(device: int = 0) -> Dict[str, int]:
