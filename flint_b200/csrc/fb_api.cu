@@ -289,7 +289,7 @@ int fb_set_option(fb_ctx* c, int32_t what, int64_t value) {
   if (what == 5) return FB_OK;                                             // 5, 7, 8: accepted, without effect: one implementation
   if (what == 8) return value < 0 || value > 2 ? FB_ERR_ARG : FB_OK;
   if (what == 7) return value < 0 || value > 4 ? FB_ERR_ARG : FB_OK;
-  if (what == 4) { if (value < 1 || value > kStages - 1) return FB_ERR_ARG; c->max_fly = (int)value; return FB_OK; }
+  if (what == 4) { if (value < 1 || value > kStages / 2) return FB_ERR_ARG; c->max_fly = (int)value; return FB_OK; }
   if (what == 2) { c->prof = (long long*)(uintptr_t)value; return FB_OK; } // device int64[sm_count * n_layer * 16] phase stamps (ns), 0 = off
   return FB_ERR_ARG;
 }

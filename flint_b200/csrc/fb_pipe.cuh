@@ -16,7 +16,7 @@ struct Pipe {
   uint64_t* empty;
   volatile int* landed;  // stage loads that are known to be complete (written by the producer, read by consumers)
   uint32_t it;           // running stage-load counter; producer and consumers walk the same sequence
-  uint32_t max_fly;      // producer only: bulk copies allowed in flight at once (1..kStages - 1)
+  uint32_t max_fly;      // producer only: bulk copies allowed in flight at once (1..kStages/2)
   uint32_t stage_bytes;  // SmemPlan::STAGE
 };
 
@@ -77,7 +77,7 @@ __device__ __forceinline__ void cta_rows(int rows, int unit, int b, int G, int& 
 
 // ------------------------------------------------------------------------------------------------ producer side
 // The number of copies in flight is kept short: with the whole ring in flight (27 MB over 148 SMs) every small
-// latency-critical access of the consumers (flags, tagged words) waits microseconds behind bulk weight traffic. The trailing
+// latency-critical access of the consumers (tagged words) waits microseconds behind bulk weight traffic. The trailing
 // wait of stage_issued also tells the consumers which loads have landed: one may only wait for load i on a stage's
 // one-bit phase once load i - kStages is known to be complete.
 __device__ __forceinline__ bool stage_slot(const Pipe& p, const WaitCtl& wc, int layer) {

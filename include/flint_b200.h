@@ -24,7 +24,7 @@ enum {
   FB_ERR_SHAPE = 2,        /* model shape this build has no kernel for */
   FB_ERR_CUDA = 3,         /* a CUDA runtime call failed; fb_last_status() carries the cudaError_t */
   FB_ERR_STATE = 4,        /* weights / KV cache not bound yet, or context poisoned by an earlier device error */
-  FB_ERR_TIMEOUT = 5,      /* a bounded device-side wait ran out (copy barrier, arrival flag, tagged word, peer word) */
+  FB_ERR_TIMEOUT = 5,      /* a bounded device-side wait ran out (copy barrier, tagged word, peer word) */
   FB_ERR_RANGE = 6         /* pos / M / token outside the bound cache or vocabulary */
 };
 
@@ -234,8 +234,8 @@ int fb_gemv_static(const void* d_q, const void* d_s, const void* d_z, int32_t ro
  *   what 2: value = device pointer to int64[sm_count * n_layer * 16] (0 = off): %globaltimer stamps (ns) of every CTA
  *           at the phase boundaries of every layer, the run-time replacement of the reference's -DNOSYNC/-DNOATTN diagnostic
  *           builds (reference: kernels/megakernel_decode.cu:15-24)
- *   what 4: bulk copies one CTA keeps in flight at once (1..4; default: 1 while layers of few bytes run, else 4)
- *   what 5: 1 = consumers poll the tagged activation words directly; 0 = they wait for the producers' arrival flags first
+ *   what 4: bulk copies one CTA keeps in flight at once (1..4; default: 2 while layers of few bytes run, else 4)
+ *   what 5: accepted without effect (it selected whether consumers wait for arrival flags ahead of the tagged words; there are none)
  *   what 7: 0..4, accepted without effect (it selected between several GEMM implementations of fb_verify)
  *   what 8: 0..2, accepted without effect (it selected between two attention implementations of fb_decode)
  */
