@@ -320,7 +320,8 @@ int fb_last_status(fb_ctx* c, fb_status* out) {
 
 size_t fb_stream_bytes(int32_t rows, int32_t k, int32_t has_zeros) {
   if (rows < 0 || !supported_k(k)) return 0;
-  return (size_t)pad_rows(rows, k) * rec_bytes_of(k, has_zeros);
+  const int u = stream_row_unit(k);
+  return (size_t)((rows + u - 1) / u * u) * rec_bytes_of(k, has_zeros);
 }
 
 int fb_repack(const void* d_q, const void* d_s, const void* d_z, int32_t rows, int32_t k, int32_t order, int32_t order_arg,
@@ -329,25 +330,33 @@ int fb_repack(const void* d_q, const void* d_s, const void* d_z, int32_t rows, i
   if (order == 1 && (order_arg <= 0 || order_arg % 2 || order_rows % order_arg || order_rows > rows)) return FB_ERR_ARG;
   if (order == 2 && (order_arg * 2 != rows)) return FB_ERR_ARG;
   if (!supported_k(k)) return FB_ERR_SHAPE;
-  return launch_repack(d_q, d_s, d_z, 1, rows, k, order, order_arg, order_rows, (uint8_t*)d_out, (cudaStream_t)stream) ==
-                 cudaSuccess
-             ? FB_OK
-             : FB_ERR_CUDA;
+  const int full = rows / tile_rt(k) * tile_rt(k);
+  cudaStream_t st = (cudaStream_t)stream;
+  if (full && launch_repack(d_q, d_s, d_z, 1, full, k, order, order_arg, order_rows, (uint8_t*)d_out, st) != cudaSuccess) return FB_ERR_CUDA;
+  if (rows > full)
+    repack_plain<<<rows - full, 128, 0, st>>>((const uint32_t*)d_q, (const uint16_t*)d_s, (const uint16_t*)d_z, full, k, order, order_arg, order_rows,
+                                              (uint8_t*)d_out + (size_t)full * rec_bytes_of(k, d_z != nullptr));
+  return cudaGetLastError() == cudaSuccess ? FB_OK : FB_ERR_CUDA;
 }
 
 int fb_dequant(const void* d_in, int32_t rows, int32_t k, int32_t has_zeros, int32_t order, int32_t order_arg,
                int32_t order_rows, float* d_out, void* stream) {
   if (!d_in || !d_out || rows <= 0 || k <= 0 || k % 128 || order < 0 || order > 2) return FB_ERR_ARG;
+  const int full = k % 128 ? 0 : rows / tile_rt(k) * tile_rt(k);
+  cudaStream_t st = (cudaStream_t)stream;
   switch (k) {
 #define X(K_)                                                                                                         \
   case K_:                                                                                                            \
-    dequant_tiles<K_><<<rows, 256, 0, (cudaStream_t)stream>>>((const uint8_t*)d_in, rows, has_zeros, order, order_arg, \
+    if (full) dequant_tiles<K_><<<full, 256, 0, st>>>((const uint8_t*)d_in, full, has_zeros, order, order_arg, \
                                                               order_rows, d_out);                                     \
     break;
     FB_FOR_EACH_K(X)
 #undef X
     default: return FB_ERR_SHAPE;
   }
+  if (rows > full)
+    dequant_plain<<<rows - full, 256, 0, st>>>((const uint8_t*)d_in + (size_t)full * rec_bytes_of(k, has_zeros), full, k, has_zeros, order, order_arg,
+                                               order_rows, d_out);
   return cudaGetLastError() == cudaSuccess ? FB_OK : FB_ERR_CUDA;
 }
 

@@ -248,6 +248,13 @@ __host__ __device__ constexpr int tile_bytes(int k, int has_zeros) { return k / 
 __host__ __device__ constexpr int rec_bytes_of(int k, int has_zeros) { return tile_bytes(k, has_zeros) / tile_rt(k); }
 __host__ __device__ constexpr int pad_rows(int rows, int k) { return (rows + tile_rt(k) - 1) / tile_rt(k) * tile_rt(k); }
 
+// A matrix on its own (fb_repack, fb_gemv, fb_dequant) holds whole tiles only; the rows behind the last one follow plainly, [rows][K/8] words in the caller's
+// order, then their scales [rows][K/128] (and zeros), so that a matrix of few rows is not padded to a tile. Its buffer: rows in multiples of these.
+__host__ __device__ constexpr int stream_row_unit(int k) {
+  const int g = k / 128;
+  return g % 4 == 0 && 4 * (k / 2 + g * 4) <= 23040 ? 4 : (g % 8 == 0 ? 2 : (g % 2 == 0 ? 8 : 16));
+}
+
 // Shared memory of a kernel whose longest K is MAXK: the tail (fixed offsets), the activations (4 bytes each) or the attention's scratch, and what is left
 // in eight ring stages.
 template <int MAXK>
@@ -432,8 +439,9 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) { return (uint
 
 // Rounds [r0, r0 + n) of a chunk (its `ci`-th of the tile) against the staged activations. RT 8: on return every lane of quad g holds the total of tile
 // row g in out_lo. RT 16: row g in out_lo and row g + 8 in out_hi.
-// The loop is ROLLED (two rounds per iteration): the decode kernel's per-layer code does not fit the instruction cache, and every phase of every
-// layer runs through its own copy of this one. Bound by shared-memory reads (16 of 64 cycles a round of 2048 weights per SM) and the ALU.
+// The loop is ROLLED (two rounds per iteration): every phase of the decode kernel has its own copy of it, and they share the instruction cache. Per round of 2048
+// weights a warp issues 24 half-rate ALU operations, 4 MMAs and 4 loads of 16 bytes a lane (16 cycles of an SM's shared memory); on its own the loop
+// streams at 0.99 of the copy bandwidth.
 template <class C, bool HZ>
 __device__ __forceinline__ void chunk_dot(const uint8_t* chunk, int ci, int r0, int n, const XStage& x, int lane, float& out_lo, float& out_hi) {
   constexpr int RT = C::RT, NJ = C::NJ;

@@ -120,8 +120,7 @@ __device__ __forceinline__ void ll_gather(const uint64_t* src, int npairs, uint3
 // as here 1001). Both plain phases share the instance of the wider one. The tile products stay inlined per phase: one shared product costs more in
 // calls than it saves (1125).
 // Both leave the phase's activations in sm.x8 / sm.xf (digits + per-group factors) and end with a consumer-wide barrier. A thread owns the 4
-// elements 4*pr .. 4*pr+3 for pr = tid_c, tid_c + kConsumerThreads, ... and keeps them in registers, so a warp owns whole groups of 128. (As a rolled
-// loop over shared memory the conversion of 8192 elements was a chain of five groups; side by side it takes 0.4 us less.)
+// elements 4*pr .. 4*pr+3 for pr = tid_c, tid_c + kConsumerThreads, ... and keeps them in registers, so a warp owns whole groups of 128.
 // xn = bf16( (float(h) * r) * float(w) ) from the tagged residual vector (dim/2 words)
 template <int MAXP, bool SUM>
 inline __device__ __noinline__ void stage_norm_ll(const uint64_t* hll, uint32_t tag, const uint16_t* gw, int D, float eps, DevStatus* status, unsigned limit, int layer,

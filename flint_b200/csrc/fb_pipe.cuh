@@ -223,6 +223,27 @@ __device__ __forceinline__ void stage_x_global(const uint16_t* gx, const Smem& s
   named_bar_sync(kBarConsumers, kConsumerThreads);
 }
 
+// row r of `n` plain rows times x (a warp; every lane returns the sum)
+inline __device__ __noinline__ float plain_row_dot(const uint8_t* base, int n, int r, int k, bool hz, const uint16_t* x, int lane) {
+  const int nw = k / 8, G = k / 128;
+  const uint32_t* q = reinterpret_cast<const uint32_t*>(base) + (size_t)r * nw;
+  const uint16_t *sc = reinterpret_cast<const uint16_t*>(base + (size_t)n * nw * 4) + (size_t)r * G, *zr = sc + (size_t)n * G;
+  float acc = 0.f;
+  for (int w = lane; w < nw; w += 32) {
+    const uint32_t v = __ldg(q + w);
+    float dot = 0.f, xs = 0.f;
+    for (int e = 0; e < 8; e++) {
+      const float xv = bf2f(__ldg(x + w * 8 + e));
+      dot = fmaf((float)(v >> (4 * e) & 15u) - 8.0f, xv, dot);
+      xs += xv;
+    }
+    acc = fmaf(bf2f(__ldg(sc + (w >> 4))), dot, acc);
+    if (hz) acc = fmaf(bf2f(__ldg(zr + (w >> 4))), xs, acc);
+  }
+  for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+  return acc;
+}
+
 template <int K, bool HZ>
 __global__ void __launch_bounds__(kThreads, 1) gemv_stream(const GemvParams P) {
   using S = SmemPlan<K>;
@@ -235,10 +256,17 @@ __global__ void __launch_bounds__(kThreads, 1) gemv_stream(const GemvParams P) {
   WaitCtl wc{P.status, sm.s_abort, P.spin_limit};
   Pipe pipe{smem_raw + S::RING, sm.full, sm.empty, sm.landed, 0u, 4u, S::STAGE};
   int r0, r1;
-  cta_rows(P.rows, C::RT, blockIdx.x, gridDim.x, r0, r1);
+  const int full = P.rows / C::RT * C::RT;
+  cta_rows(full, C::RT, blockIdx.x, gridDim.x, r0, r1);
   if (warp == kConsumerWarps) {
     if (lane == 0) produce_rows<C, HZ>(pipe, P.w, r0, r1, wc, 0);
   } else {
+    // the rows behind the last whole tile: a warp each, of the last CTA
+    if (blockIdx.x == gridDim.x - 1)
+      for (int r = warp; r < P.rows - full; r += kConsumerWarps) {
+        const float v = plain_row_dot(P.w + (size_t)full * rec_bytes_of(K, HZ), P.rows - full, r, K, HZ, P.x, lane);
+        if (lane == 0) P.y[perm_row(full + r, P.order, P.order_arg, P.order_rows)] = v;
+      }
     stage_x_global<K, HZ>(P.x, sm, tid);
     const XStage xs{sm.x8, sm.xf};
     const QueueState qs{sm.qpart, sm.tdone, sm.bcnt};
@@ -287,6 +315,28 @@ __global__ void repack_tiles(const uint32_t* q, const uint16_t* sc, const uint16
     uint16_t* meta = reinterpret_cast<uint16_t*>(tile + (size_t)k * C::chunk(hz) + C::NIB);
     meta[at] = row >= 0 ? sc[(size_t)row * (K / 128) + grp] : 0;
     if (hz) meta[RT * C::G + at] = row >= 0 ? zr[(size_t)row * (K / 128) + grp] : 0;
+  }
+}
+
+// The rows from `full` on, plainly (see stream_row_unit). One CTA per row.
+inline __global__ void repack_plain(const uint32_t* q, const uint16_t* sc, const uint16_t* zr, int full, int k, int order, int order_arg, int order_rows, uint8_t* out) {
+  const int n = gridDim.x, r = blockIdx.x, nw = k / 8, G = k / 128, row = perm_row(full + r, order, order_arg, order_rows);
+  uint32_t* dq = reinterpret_cast<uint32_t*>(out) + (size_t)r * nw;
+  uint16_t *ds = reinterpret_cast<uint16_t*>(out + (size_t)n * nw * 4) + (size_t)r * G, *dz = ds + (size_t)n * G;
+  for (int w = threadIdx.x; w < nw; w += blockDim.x) dq[w] = q[(size_t)row * nw + w];
+  for (int g = threadIdx.x; g < G; g += blockDim.x) {
+    ds[g] = sc[(size_t)row * G + g];
+    if (zr) dz[g] = zr[(size_t)row * G + g];
+  }
+}
+inline __global__ void dequant_plain(const uint8_t* in, int full, int k, int has_zeros, int order, int order_arg, int order_rows, float* out) {
+  const int n = gridDim.x, r = blockIdx.x, nw = k / 8, G = k / 128, row = perm_row(full + r, order, order_arg, order_rows);
+  const uint32_t* q = reinterpret_cast<const uint32_t*>(in) + (size_t)r * nw;
+  const uint16_t *sc = reinterpret_cast<const uint16_t*>(in + (size_t)n * nw * 4) + (size_t)r * G, *zr = sc + (size_t)n * G;
+  for (int c = threadIdx.x; c < k; c += blockDim.x) {
+    float v = ((float)(q[c >> 3] >> (4 * (c & 7)) & 15u) - 8.0f) * bf2f(sc[c >> 7]);
+    if (has_zeros) v = v + bf2f(zr[c >> 7]);
+    out[(size_t)row * k + c] = v;
   }
 }
 
