@@ -334,7 +334,7 @@ int fb_repack(const void* d_q, const void* d_s, const void* d_z, int32_t rows, i
   cudaStream_t st = (cudaStream_t)stream;
   if (full && launch_repack(d_q, d_s, d_z, 1, full, k, order, order_arg, order_rows, (uint8_t*)d_out, st) != cudaSuccess) return FB_ERR_CUDA;
   if (rows > full)
-    repack_plain<<<rows - full, 128, 0, st>>>((const uint32_t*)d_q, (const uint16_t*)d_s, (const uint16_t*)d_z, full, k, order, order_arg, order_rows,
+    repack_plain<><<<rows - full, 128, 0, st>>>((const uint32_t*)d_q, (const uint16_t*)d_s, (const uint16_t*)d_z, full, k, order, order_arg, order_rows,
                                               (uint8_t*)d_out + (size_t)full * rec_bytes_of(k, d_z != nullptr));
   return cudaGetLastError() == cudaSuccess ? FB_OK : FB_ERR_CUDA;
 }
@@ -355,7 +355,7 @@ int fb_dequant(const void* d_in, int32_t rows, int32_t k, int32_t has_zeros, int
     default: return FB_ERR_SHAPE;
   }
   if (rows > full)
-    dequant_plain<<<rows - full, 256, 0, st>>>((const uint8_t*)d_in + (size_t)full * rec_bytes_of(k, has_zeros), full, k, has_zeros, order, order_arg,
+    dequant_plain<><<<rows - full, 256, 0, st>>>((const uint8_t*)d_in + (size_t)full * rec_bytes_of(k, has_zeros), full, k, has_zeros, order, order_arg,
                                                order_rows, d_out);
   return cudaGetLastError() == cudaSuccess ? FB_OK : FB_ERR_CUDA;
 }

@@ -319,7 +319,8 @@ __global__ void repack_tiles(const uint32_t* q, const uint16_t* sc, const uint16
 }
 
 // The rows from `full` on, plainly (see stream_row_unit). One CTA per row.
-inline __global__ void repack_plain(const uint32_t* q, const uint16_t* sc, const uint16_t* zr, int full, int k, int order, int order_arg, int order_rows, uint8_t* out) {
+template <int UNIT = 0>      // (a template so that several translation units may include it)
+__global__ void repack_plain(const uint32_t* q, const uint16_t* sc, const uint16_t* zr, int full, int k, int order, int order_arg, int order_rows, uint8_t* out) {
   const int n = gridDim.x, r = blockIdx.x, nw = k / 8, G = k / 128, row = perm_row(full + r, order, order_arg, order_rows);
   uint32_t* dq = reinterpret_cast<uint32_t*>(out) + (size_t)r * nw;
   uint16_t *ds = reinterpret_cast<uint16_t*>(out + (size_t)n * nw * 4) + (size_t)r * G, *dz = ds + (size_t)n * G;
@@ -329,7 +330,8 @@ inline __global__ void repack_plain(const uint32_t* q, const uint16_t* sc, const
     if (zr) dz[g] = zr[(size_t)row * G + g];
   }
 }
-inline __global__ void dequant_plain(const uint8_t* in, int full, int k, int has_zeros, int order, int order_arg, int order_rows, float* out) {
+template <int UNIT = 0>
+__global__ void dequant_plain(const uint8_t* in, int full, int k, int has_zeros, int order, int order_arg, int order_rows, float* out) {
   const int n = gridDim.x, r = blockIdx.x, nw = k / 8, G = k / 128, row = perm_row(full + r, order, order_arg, order_rows);
   const uint32_t* q = reinterpret_cast<const uint32_t*>(in) + (size_t)r * nw;
   const uint16_t *sc = reinterpret_cast<const uint16_t*>(in + (size_t)n * nw * 4) + (size_t)r * G, *zr = sc + (size_t)n * G;

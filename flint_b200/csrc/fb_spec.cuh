@@ -123,8 +123,8 @@ __global__ void __launch_bounds__(1024) sample_rows(const SampleParams P) {
   auto score = [&](int i, float x) { return draw ? x * inv_t + gumbel(mix32(P.seed, P.counter + (unsigned long long)row, (uint32_t)i)) : x; };
   float bv = -INFINITY;
   int bi = 0x7fffffff;
-  if (SELECT && brief) {
-    unsigned *wkey = hist[0], *lkey = hist[SELECT], *lidx = hist[SELECT] + kSampleList;
+  if constexpr (SELECT) if (brief) {
+    unsigned *wkey = hist[0], *lkey = hist[1], *lidx = hist[1] + kSampleList;
     uint32_t top = 0u;
     each([&](int, float x) { top = max(top, fkey(x)); });
     top = __reduce_max_sync(0xffffffffu, top);
