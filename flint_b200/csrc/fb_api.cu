@@ -35,14 +35,6 @@ const KernelEntry kDecodeKernels[] = {
 };
 constexpr int kNumDecodeKernels = sizeof(kDecodeKernels) / sizeof(kDecodeKernels[0]);
 
-// columns of the O projection a rank reads: its heads' columns widened to whole int4 groups (a rank of the 3B-class
-// model split 8 ways owns 320 columns = 2.5 groups: it reads 384 and feeds zeros for its neighbour's 64)
-void o_window(int width, int rank, int* ko, int* off) {
-  const int start = rank * width, lo = start / 128 * 128, hi = (start + width + 127) / 128 * 128;
-  *ko = hi - lo;
-  *off = start - lo;
-}
-
 const void* kernel_of(int id, int tp_size) { return tp_size > 1 ? decode_tp_kernel(id) : kDecodeKernels[id].fn; }
 
 int find_kernel(const fb_model_desc& d, int ko) {
@@ -195,8 +187,8 @@ int fb_ctx_create_tp(const fb_model_desc* desc, int device, int32_t tp_rank, int
   if (tp_size < 1 || tp_size > 8 || tp_rank < 0 || tp_rank >= tp_size) return FB_ERR_ARG;
   if (d.n_layer <= 0 || d.vocab <= 0 || d.dim % 128 || d.ffn % 128 || d.n_head <= 0 || d.head_dim <= 0) return FB_ERR_SHAPE;
   if (tp_size == 1 && d.n_head * d.head_dim != d.dim) return FB_ERR_SHAPE;
-  int ko = 0, ao_off = 0;
-  o_window(d.n_head * d.head_dim, tp_rank, &ko, &ao_off);
+  const OWindow win = o_window(d.n_head * d.head_dim, tp_rank);
+  const int ko = win.ko, ao_off = win.off;
   if (tp_size == 1 && ao_off) return FB_ERR_SHAPE;
   const int kid = find_kernel(d, ko);
   if (kid < 0) return FB_ERR_SHAPE;

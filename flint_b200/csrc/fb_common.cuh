@@ -7,6 +7,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "fb_geometry.hpp"
+
 namespace fb {
 
 // ------------------------------------------------------------------------------------------------ constants
@@ -228,7 +230,6 @@ __device__ __forceinline__ bool mbar_wait_far(uint64_t* b, uint32_t parity, cons
 // from shared memory.) Gate/up of the 3B / 1B / 8B-class shapes, 16384 x 2560, 16384 x 2048, 28672 x 4096, in the decode kernel: 4.4 / 3.9 / 11.8 us before,
 // 2.5 / 2.2 / 7.3 now; the stand-alone product over 400000 x 2560 5.3 -> 5.8 TB/s. Against a 64-bit sum the logits of two layers are closer than
 // before (mean distance in units of the test's tolerance: 0.61 -> 0.35 at 3B, 0.50 -> 0.15 at 1B, 0.66 -> 0.51 at 8B): the products round only in the flush.
-__host__ __device__ constexpr int tile_rt(int k) { return (k / 128) % 2 == 0 ? 8 : 16; }
 __host__ __device__ constexpr int chunk_bytes(int rt, int kc, int has_zeros) { return rt * (kc / 2 + (kc / 128) * 2 * (has_zeros ? 2 : 1)); }
 constexpr int kChunkFit = 20992;                   // the smallest ring stage (SmemPlan of K = 14336)
 // Columns of a chunk: all of K where that fits a stage; else 4096 or 2048 where they divide K (8192 in 2, 14336 in 7: with 28 rows a CTA two chunks a warp), else
@@ -298,8 +299,9 @@ struct TCfg {
   static_assert(chunk_bytes(RT, KC, 0) % 16 == 0, "bulk copies move multiples of 16 bytes");
 };
 // Which chunks of a phase a warp takes: chunk, first round, rounds, slices per chunk, a byte each. Few chunks: each is cut in `ks` slices so that as
-// many warps as possible have one; else the warps take whole chunks w, w + 14, ...
-__device__ __forceinline__ uint32_t unit_entry(int nch, int rpc, int warp) {
+// many warps as possible have one; else the warps take whole chunks w, w + 14, ... Called once per phase and launch, so out of line: five copies with their
+// divisions are code that the layer loop has to share the instruction cache with (3B-class 794 -> 784 us a token, 8B 1409 -> 1417, others as before).
+inline __device__ __noinline__ uint32_t unit_entry(int nch, int rpc, int warp) {
   int ks = nch > 0 && nch <= kConsumerWarps / 2 ? kConsumerWarps / nch : 1;
   if (ks > rpc) ks = rpc;
   const int ci = warp / ks, sl = warp - ci * ks, r0 = rpc * sl / ks, r1 = rpc * (sl + 1) / ks;

@@ -8,8 +8,11 @@
 // trip instead of three (barrier arrive, barrier poll, data fetch). (Arrival flags that were waited for ahead of the words gained as long as words were
 // stored, see ll_store; with exchanges they cost 847 us a token of the 3B-class shape at 200 positions against 808 without.)
 //
-// Why single buffers are enough: a CTA reads a phase's input only if it owns rows of that phase, the next phase needs every such CTA's words, and an
-// input is overwritten in the next phase at the earliest. (A CTA without rows skips the input: it might find it overwritten.)
+// Why single buffers are enough: a CTA publishes words only behind its own reads of the phase's input, a phase's words are made from all words of the phase before
+// (of the attention: of the queries of all heads), so whoever publishes a buffer's next words knows, through the phases in between, that all readers of the last ones
+// are done. That holds for words whose writer has waited, and only for those: nobody publishes anything else (columns that nobody computes are not
+// published as zeros but left out of the reading, see o_words). A CTA without rows of a phase skips its input: nothing of its own would hold the next words
+// back, and it might find the input overwritten. tests/test_decode_order.py follows all shapes through.
 #pragma once
 #include <cuda.h>
 
@@ -85,16 +88,16 @@ inline __device__ __noinline__ bool poll_again(unsigned spin, const WaitCtl wc, 
   return false;
 }
 
-// Poll tagged words, 16-byte aligned: pair k of a thread is words 2 (tid + k * nthreads) and the one behind it, `npairs` pairs in all; their payloads go to
+// Poll tagged words, 16-byte aligned: pair k of a thread is words 2 (tid + k * nthreads) and the one behind it, pairs [first, end) in all; their payloads go to
 // v[k] (zero where there is no such pair). All of a thread's loads are issued before any is checked.
 template <int MAXP>
-__device__ __forceinline__ void ll_gather(const uint64_t* src, int npairs, uint32_t tag, uint2 (&v)[MAXP], int tid, int nthreads,
-                                          const WaitCtl& wc, int layer) {
+__device__ __forceinline__ void ll_gather(const uint64_t* src, int end, uint32_t tag, uint2 (&v)[MAXP], int tid, int nthreads,
+                                          const WaitCtl& wc, int layer, int first = 0) {
   uint32_t pending = 0;
 #pragma unroll
   for (int k = 0; k < MAXP; k++) {
     v[k] = make_uint2(0, 0);
-    if (tid + k * nthreads < npairs) pending |= 1u << k;
+    if (tid + k * nthreads >= first && tid + k * nthreads < end) pending |= 1u << k;
   }
 #pragma unroll 1
   for (unsigned spin = 0; pending; spin++) {
@@ -181,9 +184,11 @@ inline __device__ __noinline__ void stage_norm_ll(const uint64_t* hll, uint32_t 
   named_bar_sync(kBarConsumers, kConsumerThreads);
 }
 
-template <int MAXP, bool SUM>
+// `only`, in the kernels of ranks: first and end pair of the words that somebody publishes; the other elements are zero. (A parameter pack: the kernels of one GPU
+// have no such argument.)
+template <int MAXP, bool SUM, class... Only>
 inline __device__ __noinline__ void stage_plain_ll(const uint64_t* src, uint32_t tag, int K,
-                                                   DevStatus* status, unsigned limit, int layer) {
+                                                   DevStatus* status, unsigned limit, int layer, Only... only) {
   extern __shared__ __align__(128) uint8_t smem_raw[];
   const Smem sm = carve_smem(smem_raw);
   const WaitCtl wc{status, sm.s_abort, limit};
@@ -191,7 +196,12 @@ inline __device__ __noinline__ void stage_plain_ll(const uint64_t* src, uint32_t
   const int npairs = K / 4, lane = tid_c & 31;
   named_bar_sync(kBarConsumers, kConsumerThreads);            // every warp has left the phase that read the activations
   uint2 raw[MAXP];
-  ll_gather<MAXP>(src, npairs, tag, raw, tid_c, kConsumerThreads, wc, layer);
+  if constexpr (sizeof...(Only) > 0) {
+    const WordPairs w{only...};
+    ll_gather<MAXP>(src, w.end, tag, raw, tid_c, kConsumerThreads, wc, layer, w.first);
+  } else {
+    ll_gather<MAXP>(src, npairs, tag, raw, tid_c, kConsumerThreads, wc, layer);
+  }
   stage_groups<SUM, MAXP>(raw, tid_c >> 5, kConsumerWarps, K / 128, sm.x8, sm.xf, lane);
   named_bar_sync(kBarConsumers, kConsumerThreads);
 }
@@ -770,15 +780,7 @@ __global__ void __launch_bounds__(kThreads, 1) decode_mega2(const __grid_constan
       FB_STAMP(2);
       // ================= attention =================
       {
-        if (b == 0 && KOUT != 0) {
-          // columns of the O window that belong to a neighbouring rank (tensor parallel, 8-way split of the 3B-class
-          // shape): the O projection must see zeros there, tagged like the real attention output
-          const int used = P.n_head * HP, off = P.ao_off >> 1;
-#pragma unroll 1
-          for (int i = tid_c; i < KOUT / 2 - used; i += kConsumerThreads)
-            ll_store(P.ao_ll + (i < off ? i : used + i), 0u, tg_att);
-        }
-        const AttnArgs aa{P.q_ll, P.k_ll, P.v_ll, P.ao_ll + (P.ao_off >> 1), P.part_ll, P.n_kv, P.pos, P.nchunks,
+        const AttnArgs aa{P.q_ll, P.k_ll, P.v_ll, TP ? P.ao_ll + (P.ao_off >> 1) : P.ao_ll, P.part_ll, P.n_kv, P.pos, P.nchunks,
                      P.maxchunks, P.attn_scale, tg_qkv, mk_tag(P.tag_base, l, PH_PART), tg_att};
         named_bar_sync(kBarConsumers, kConsumerThreads);        // scratch (the activations) is free: every warp left the GEMV
         attention_phase<HD, R, STG>(aa, sm.scratch, cw, lane, tid_c, wc, l, pipe, sm.tdone);
@@ -786,7 +788,13 @@ __global__ void __launch_bounds__(kThreads, 1) decode_mega2(const __grid_constan
       FB_STAMP(3);
       // ================= O projection + residual =================
       {
-        if (o1 > o0) stage_plain_ll<imax(MAXP_O, MAXP_F), HZ>(P.ao_ll, tg_att, KOUT, P.status, P.spin_limit, l);
+        // a rank of several: the window's other columns belong to a neighbour, whose O projection sees them; this one sees zeros there
+        if constexpr (TP) {
+          const WordPairs own = o_words(P.n_head * HD, P.ao_off);
+          if (o1 > o0) stage_plain_ll<imax(MAXP_O, MAXP_F), HZ>(P.ao_ll, tg_att, KOUT, P.status, P.spin_limit, l, own.first, own.end);
+        } else {
+          if (o1 > o0) stage_plain_ll<imax(MAXP_O, MAXP_F), HZ>(P.ao_ll, tg_att, KOUT, P.status, P.spin_limit, l);
+        }
         FB_STAMP(4);
         consume_tiles<CO, HZ>(pipe, o1 - o0, units[16], xs_, qs_, cw, lane, wc, l,
                                   [&](int row0, float c, int nvalid) { resid_epi(row0, c, nvalid, tg_o, 0); });
@@ -811,7 +819,11 @@ __global__ void __launch_bounds__(kThreads, 1) decode_mega2(const __grid_constan
       FB_STAMP(7);
       // ================= down projection + residual =================
       {
-        if (o1 > o0) stage_plain_ll<imax(MAXP_O, MAXP_F), HZ>(P.act_ll, tg_gu, FF, P.status, P.spin_limit, l);
+        if constexpr (TP) {
+          if (o1 > o0) stage_plain_ll<imax(MAXP_O, MAXP_F), HZ>(P.act_ll, tg_gu, FF, P.status, P.spin_limit, l, 0, FF / 4);
+        } else {
+          if (o1 > o0) stage_plain_ll<imax(MAXP_O, MAXP_F), HZ>(P.act_ll, tg_gu, FF, P.status, P.spin_limit, l);
+        }
         FB_STAMP(8);
         consume_tiles<CF, HZ>(pipe, o1 - o0, units[48], xs_, qs_, cw, lane, wc, l,
                                   [&](int row0, float c, int nvalid) { resid_epi(row0, c, nvalid, tg_dn, 1); });

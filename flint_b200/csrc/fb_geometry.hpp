@@ -1,8 +1,27 @@
-// Launch geometry as plain functions of the sizes: what fb_pass.cu and fb_spec.cu launch, and what a host-side test can ask. No CUDA here.
+// Launch geometry as plain functions of the sizes: what fb_pass.cu and fb_spec.cu launch, how the decode kernel cuts its phases, and what a host-side test can
+// ask. No CUDA here (the device code uses the constexpr ones).
 // Times: engine calls back to back.
 #pragma once
 
 namespace fb {
+
+// rows of a tile of the streaming layout
+constexpr int tile_rt(int k) { return (k / 128) % 2 == 0 ? 8 : 16; }
+// the first of the rows of a phase that CTA b of G owns (they end where those of b + 1 start); `unit` rows stay together
+constexpr int cta_first_row(int rows, int unit, int b, int G) {
+  const int r = (int)((long long)((rows + unit - 1) / unit) * b / G) * unit;
+  return r < rows ? r : rows;
+}
+// Columns of the O projection a rank reads: its heads' columns widened to whole int4 groups (a rank of the 3B-class
+// model split 8 ways owns 320 columns = 2.5 groups: it reads 384 and takes zeros for its neighbour's 64). off: where its own start.
+struct OWindow { int ko, off; };
+constexpr OWindow o_window(int width, int rank) {
+  const int start = rank * width, lo = start / 128 * 128, hi = (start + width + 127) / 128 * 128;
+  return OWindow{hi - lo, start - lo};
+}
+// ... as pairs of tagged words (four columns a pair; a head is a multiple of eight): the only ones that this rank's attention publishes
+struct WordPairs { int first, end; };
+constexpr WordPairs o_words(int width, int off) { return WordPairs{off / 4, (off + width) / 4}; }
 
 constexpr int kTcRowBlock = 128;  // weight rows of a GEMM's work item
 

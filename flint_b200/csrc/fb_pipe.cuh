@@ -70,9 +70,8 @@ __device__ __forceinline__ void pipe_init(const Smem& sm) {
 
 // rows [r0, r1) of a phase that CTA b of G owns; `unit` rows stay together (the tile height of the matrix)
 __device__ __forceinline__ void cta_rows(int rows, int unit, int b, int G, int& r0, int& r1) {
-  const long long nu = (rows + unit - 1) / unit;
-  r0 = min(rows, (int)((nu * b) / G) * unit);
-  r1 = min(rows, (int)((nu * (b + 1)) / G) * unit);
+  r0 = cta_first_row(rows, unit, b, G);
+  r1 = cta_first_row(rows, unit, b + 1, G);
 }
 
 // ------------------------------------------------------------------------------------------------ producer side

@@ -16,6 +16,18 @@ extern "C" void attn(int M, int pos, int n_kv, int r, int sms, int* o) {
   const fb::AttnGeometry a = fb::attn_geometry(M, pos, n_kv, r, sms);
   o[0] = a.rt; o[1] = a.groups; o[2] = a.nspan; o[3] = a.span;
 }
+extern "C" int tile_rt(int k) { return fb::tile_rt(k); }
+extern "C" int cta_first_row(int rows, int unit, int b, int G) { return fb::cta_first_row(rows, unit, b, G); }
+extern "C" void window(int width, int rank, int* o) {
+  const fb::OWindow w = fb::o_window(width, rank);
+  const fb::WordPairs p = fb::o_words(width, w.off);
+  o[0] = w.ko; o[1] = w.off; o[2] = p.first; o[3] = p.end;
+}
+static const int kShapes[][5] = {
+#define FB_DECODE_ENTRY(KD, KO, KF, HD, R) {KD, KO, KF, HD, R}
+#include "fb_decode_shapes.h"
+};
+extern "C" int shapes(const int** o) { *o = &kShapes[0][0]; return (int)(sizeof(kShapes) / sizeof(kShapes[0])); }
 extern "C" int draft(int blocks, int chunks, int nt, int sms) { return fb::draft_splits(blocks, chunks, nt, sms); }
 """
 _lib = None
@@ -61,3 +73,25 @@ def draft(rows, k, T, pair=False, sms=148):
     nt = 1 if T <= 8 else (2 if T <= 16 else 4)
     per = 16 if nt == 1 or pair else 32
     return _load().draft(sum(-(-r // per) for r in rows), -(-k // 32), nt, sms)
+
+
+def decode_shapes():
+    """(model width, O columns of a rank, FFN width of a rank, head dimension, query heads per kv head) of every decode kernel"""
+    p = ctypes.POINTER(ctypes.c_int)()
+    n = _load().shapes(ctypes.byref(p))
+    return [tuple(p[5 * i:5 * i + 5]) for i in range(n)]
+
+
+def tile_rt(k):
+    return _load().tile_rt(k)
+
+
+def cta_rows(rows, unit, sms=148):
+    """First and end row of every CTA's share of a decode phase"""
+    at = [_load().cta_first_row(rows, unit, b, sms) for b in range(sms + 1)]
+    return list(zip(at[:-1], at[1:]))
+
+
+def o_window(width, rank):
+    """(columns of the O projection that a rank reads, where its own start in them, first and end pair of tagged words of its own)"""
+    return _four(_load().window, width, rank)
