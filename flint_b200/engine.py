@@ -20,10 +20,17 @@ def _ptr(t: Optional[torch.Tensor]):
     return None if t is None else t.data_ptr()          # the prototypes say void*: ctypes takes the integer
 
 
+# private, but what torch's own code generators call; the public way where a later torch lacks it
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None) or (lambda index: torch.cuda.current_stream(index).cuda_stream)
+
+
 def _stream_ptr(device) -> int:
-    """The current stream of a CUDA device, as torch.cuda.current_stream(device).cuda_stream gives it, without the Stream object (2.2 us a call)."""
+    """The current stream of a CUDA device, as torch.cuda.current_stream(device).cuda_stream gives it (ValueError for any other device: what follows is a
+    launch on that device's pointers), without the Stream object (2.2 us a call)."""
+    if device.type != "cuda":
+        raise ValueError(f"Expected a cuda device, but got: {device}")
     index = device.index
-    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if index is None else index)
+    return _raw_stream(torch.cuda.current_device() if index is None else index)
 
 
 def query(device: int = 0) -> Dict[str, int]:
