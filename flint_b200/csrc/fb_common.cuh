@@ -299,14 +299,16 @@ struct TCfg {
   static_assert(chunk_bytes(RT, KC, 0) % 16 == 0, "bulk copies move multiples of 16 bytes");
 };
 // Which chunks of a phase a warp takes: chunk, first round, rounds, slices per chunk, a byte each. Few chunks: each is cut in `ks` slices so that as
-// many warps as possible have one; else the warps take whole chunks w, w + 14, ... Called once per phase and launch, so out of line: five copies with their
-// divisions are code that the layer loop has to share the instruction cache with (3B-class 794 -> 784 us a token, 8B 1409 -> 1417, others as before).
-inline __device__ __noinline__ uint32_t unit_entry(int nch, int rpc, int warp) {
+// many warps as possible have one; else the warps take whole chunks w, w + 14, ...
+__device__ __forceinline__ uint32_t unit_entry(int nch, int rpc, int warp) {
   int ks = nch > 0 && nch <= kConsumerWarps / 2 ? kConsumerWarps / nch : 1;
   if (ks > rpc) ks = rpc;
   const int ci = warp / ks, sl = warp - ci * ks, r0 = rpc * sl / ks, r1 = rpc * (sl + 1) / ks;
   return (uint32_t)(ci < nch ? ci : 255) | (uint32_t)r0 << 8 | (uint32_t)(r1 - r0) << 16 | (uint32_t)ks << 24;
 }
+// ... out of line, for the decode kernel, which asks once per phase and launch: five copies with their divisions are code that its layer loop has to share the
+// instruction cache with (3B-class 794 -> 784 us a token, 8B 1409 -> 1417, others as before)
+inline __device__ __noinline__ uint32_t unit_entry_far(int nch, int rpc, int warp) { return unit_entry(nch, rpc, warp); }
 
 // activations of the current phase in shared memory: per 64 columns their lowest digits [64], then the next ones, in column order; and per group of
 // 128 columns {2^-e, sum x} for the lanes that hold the two low digits, {2^15 2^-e, 0} for those of the two high ones (sum x: asymmetric layout only)

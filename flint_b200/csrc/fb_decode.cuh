@@ -645,10 +645,10 @@ __global__ void __launch_bounds__(kThreads, 1) decode_mega2(const __grid_constan
     // what this warp takes of every phase (its own entries: no barrier needed beyond the warp)
     uint32_t* units = sm.units + cw;
     if (lane == 0) {
-      units[0] = unit_entry((q1 - q0 + CD::RT - 1) / CD::RT * CD::NC, CD::RPC, cw);
-      units[16] = unit_entry((o1 - o0 + CO::RT - 1) / CO::RT * CO::NC, CO::RPC, cw);
-      units[32] = unit_entry((g1 - g0 + CD::RT - 1) / CD::RT * CD::NC, CD::RPC, cw);
-      units[48] = unit_entry((o1 - o0 + CF::RT - 1) / CF::RT * CF::NC, CF::RPC, cw);
+      units[0] = unit_entry_far((q1 - q0 + CD::RT - 1) / CD::RT * CD::NC, CD::RPC, cw);
+      units[16] = unit_entry_far((o1 - o0 + CO::RT - 1) / CO::RT * CO::NC, CO::RPC, cw);
+      units[32] = unit_entry_far((g1 - g0 + CD::RT - 1) / CD::RT * CD::NC, CD::RPC, cw);
+      units[48] = unit_entry_far((o1 - o0 + CF::RT - 1) / CF::RT * CF::NC, CF::RPC, cw);
     }
     __syncwarp();
     const QueueState qs_{sm.qpart, sm.tdone, sm.bcnt};
@@ -836,7 +836,7 @@ __global__ void __launch_bounds__(kThreads, 1) decode_mega2(const __grid_constan
     stage_norm_ll<MAXP_D, HZ>(P.h_ll, mk_tag(P.tag_base, L - 1, PH_DOWN), P.nf, D, P.eps, P.status, P.spin_limit, L, false);
     float bv = -INFINITY;
     int bi = 0x7fffffff;
-    consume_tiles<CD, HZ>(pipe, l1 - l0, unit_entry((l1 - l0 + CD::RT - 1) / CD::RT * CD::NC, CD::RPC, cw), xs_, qs_, cw, lane, wc, L, [&](int row0, float c, int nvalid) {
+    consume_tiles<CD, HZ>(pipe, l1 - l0, unit_entry_far((l1 - l0 + CD::RT - 1) / CD::RT * CD::NC, CD::RPC, cw), xs_, qs_, cw, lane, wc, L, [&](int row0, float c, int nvalid) {
       if ((lane & 3) == 0 && (lane >> 2) < nvalid) {
         const int row = P.vocab_base + l0 + row0 + (lane >> 2);     // index in the full vocabulary
         const float y = c / P.logits_scaling;

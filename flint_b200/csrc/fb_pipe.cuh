@@ -211,34 +211,52 @@ struct GemvParams {
   unsigned spin_limit;
 };
 
-// every consumer thread calls; ends with a consumer-wide barrier
+// every consumer thread calls; ends with a consumer-wide barrier. A warp's groups are loaded and converted side by side (one after the other 2560 rows of K =
+// 8192 / 14336 5.5 / 8.6 us a launch instead of 5.0 / 7.6).
 template <int K, bool HZ>
 __device__ __forceinline__ void stage_x_global(const uint16_t* gx, const Smem& sm, int tid_c) {
+  constexpr int G = K / 128, N = (G + kConsumerWarps - 1) / kConsumerWarps;
   const int warp = tid_c >> 5, lane = tid_c & 31;
-  for (int grp = warp; grp < K / 128; grp += kConsumerWarps) {
-    const uint2 v[1] = {__ldg(reinterpret_cast<const uint2*>(gx + grp * 128) + lane)};
-    stage_groups<HZ, 1>(v, grp, 0, K / 128, sm.x8, sm.xf, lane);
+  uint2 v[N];
+#pragma unroll
+  for (int k = 0; k < N; k++) {
+    const int grp = warp + k * kConsumerWarps;
+    v[k] = grp < G ? __ldg(reinterpret_cast<const uint2*>(gx + grp * 128) + lane) : make_uint2(0, 0);
   }
+  stage_groups<HZ, N>(v, warp, kConsumerWarps, G, sm.x8, sm.xf, lane);
   named_bar_sync(kBarConsumers, kConsumerThreads);
 }
 
-// row r of `n` plain rows times x (a warp; every lane returns the sum)
-inline __device__ __noinline__ float plain_row_dot(const uint8_t* base, int n, int r, int k, bool hz, const uint16_t* x, int lane) {
-  const int nw = k / 8, G = k / 128;
-  const uint32_t* q = reinterpret_cast<const uint32_t*>(base) + (size_t)r * nw;
-  const uint16_t *sc = reinterpret_cast<const uint16_t*>(base + (size_t)n * nw * 4) + (size_t)r * G, *zr = sc + (size_t)n * G;
+// Row r of `n` plain rows times x: what a thread's columns add, summed over its warp. All consumer threads of a CTA share a row, 32 columns (16 bytes) each: up to K =
+// 14336 one load of weights and four of x a thread, side by side.
+inline __device__ __noinline__ float plain_row_part(const uint8_t* base, int n, int r, int k, bool hz, const uint16_t* x, int tid_c) {
+  const int G = k / 128;
+  const uint4* q = reinterpret_cast<const uint4*>(base + (size_t)r * (k / 2));
+  const uint16_t *sc = reinterpret_cast<const uint16_t*>(base + (size_t)n * (k / 2)) + (size_t)r * G, *zr = sc + (size_t)n * G;
   float acc = 0.f;
-  for (int w = lane; w < nw; w += 32) {
-    const uint32_t v = __ldg(q + w);
-    float dot = 0.f, xs = 0.f;
-    for (int e = 0; e < 8; e++) {
-      const float xv = bf2f(__ldg(x + w * 8 + e));
-      dot = fmaf((float)(v >> (4 * e) & 15u) - 8.0f, xv, dot);
-      xs += xv;
+#pragma unroll 1
+  for (int c = tid_c; c < k / 32; c += kConsumerThreads) {
+    const uint4 w = __ldg(q + c);
+    const uint4* xp = reinterpret_cast<const uint4*>(x) + 4 * c;
+    const uint4 x0 = __ldg(xp), x1 = __ldg(xp + 1), x2 = __ldg(xp + 2), x3 = __ldg(xp + 3);
+    const float s = bf2f(__ldg(sc + (c >> 2))), z = hz ? bf2f(__ldg(zr + (c >> 2))) : 0.f;
+    const uint32_t ws[4] = {w.x, w.y, w.z, w.w};
+    const uint4 xs[4] = {x0, x1, x2, x3};
+    float dot = 0.f, sum = 0.f;
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      const uint32_t p[4] = {xs[i].x, xs[i].y, xs[i].z, xs[i].w};
+#pragma unroll
+      for (int e = 0; e < 8; e++) {
+        const float v = e & 1 ? bfhi(p[e >> 1]) : bflo(p[e >> 1]);
+        dot = fmaf((float)(ws[i] >> (4 * e) & 15u) - 8.0f, v, dot);
+        sum += v;
+      }
     }
-    acc = fmaf(bf2f(__ldg(sc + (w >> 4))), dot, acc);
-    if (hz) acc = fmaf(bf2f(__ldg(zr + (w >> 4))), xs, acc);
+    acc = fmaf(s, dot, acc);
+    if (hz) acc = fmaf(z, sum, acc);
   }
+#pragma unroll
   for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
   return acc;
 }
@@ -260,13 +278,23 @@ __global__ void __launch_bounds__(kThreads, 1) gemv_stream(const GemvParams P) {
   if (warp == kConsumerWarps) {
     if (lane == 0) produce_rows<C, HZ>(pipe, P.w, r0, r1, wc, 0);
   } else {
-    // the rows behind the last whole tile: a warp each, of the last CTA
-    if (blockIdx.x == gridDim.x - 1)
-      for (int r = warp; r < P.rows - full; r += kConsumerWarps) {
-        const float v = plain_row_dot(P.w + (size_t)full * rec_bytes_of(K, HZ), P.rows - full, r, K, HZ, P.x, lane);
-        if (lane == 0) P.y[perm_row(full + r, P.order, P.order_arg, P.order_rows)] = v;
-      }
+    // The rows behind the last whole tile, a CTA each from the first one on (cta_rows gives the first CTAs the fewest tiles), ahead of the staging: the tiles are on
+    // their way meanwhile. 37 / 2567 / 16389 rows of K = 14336, 300 / 2563 / 16389 of K = 2560, a launch of a graph: 5.2 / 8.4 / 23.6 and 3.9 / 4.0 / 5.2 us; as scalar
+    // loops of a warp each in one CTA 18.9 / 21.9 / 55.9 and 5.8 / 6.0 / 7.4. (Loading them beside the activations and multiplying behind the staging: no faster.)
+    const int plain = P.rows - full;
+    float* part = sm.yin;                                       // [row of this CTA][warp]
+    int mine = 0;
+    for (int r = blockIdx.x; r < plain; r += gridDim.x, mine++) {
+      const float v = plain_row_part(P.w + (size_t)full * rec_bytes_of(K, HZ), plain, r, K, HZ, P.x, tid);
+      if (lane == 0) part[16 * mine + warp] = v;
+    }
     stage_x_global<K, HZ>(P.x, sm, tid);
+    for (int i = warp; i < mine; i += kConsumerWarps) {
+      float v = lane < kConsumerWarps ? part[16 * i + lane] : 0.f;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+      if (lane == 0) P.y[perm_row(full + (int)blockIdx.x + i * (int)gridDim.x, P.order, P.order_arg, P.order_rows)] = v;
+    }
     const XStage xs{sm.x8, sm.xf};
     const QueueState qs{sm.qpart, sm.tdone, sm.bcnt};
     const uint32_t entry = unit_entry((r1 - r0 + C::RT - 1) / C::RT * C::NC, C::RPC, warp);

@@ -116,6 +116,26 @@ def test_gemv_power_of_two_activations_are_exact(e):
     assert np.abs(ys[0] - ref).max() < 2e-5 * (np.abs(ref).max() + 1e-6)
 
 
+@pytest.mark.parametrize("k,rt", [(256, 8), (640, 16), (1408, 16), (8192, 8), (14336, 8)])
+@pytest.mark.parametrize("asym", [False, True])
+def test_gemv_rows_behind_the_last_whole_tile(k, rt, asym):
+    """Every number of rows that a last tile can lack, with and without whole tiles before them: a row is shared by all warps of a CTA (fewer columns than
+    threads, and exactly as many). A thread's 32 products and the sums over lanes and warps: fewer than 64 roundings of 2^-24, the bar of the other rows."""
+    lib = _lib.load()
+    for left in range(1, rt):
+        for rows in (left, 3 * rt + left):
+            q, s, z = _mat(rows, k, 31 + left, asym)
+            x = torch.randn(k, generator=torch.Generator().manual_seed(left)).bfloat16()
+            st = _repack(lib, q.cuda(), s.cuda(), z.cuda() if z is not None else None)
+            y = torch.full((rows,), float("nan"), device="cuda")
+            status = torch.zeros(8, dtype=torch.int32, device="cuda")
+            _lib.check(lib.fb_gemv(_p(st), rows, k, int(asym), 0, 0, 0, _p(x.cuda()), _p(y), _p(status), None), "fb_gemv")
+            torch.cuda.synchronize()
+            assert int(status[0]) == 0
+            ref = O.c_gemv(q, s, z, x)[0]
+            assert np.abs(y.cpu().numpy() - ref).max() < 2e-5 * (np.abs(ref).max() + 1e-6), rows
+
+
 def test_gemv_permuted_rows_land_in_source_order():
     lib = _lib.load()
     rows, k = 768, 512           # tiny-config QKV: 8 q + 2 k heads of 64 paired, 2 v heads plain
