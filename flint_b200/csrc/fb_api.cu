@@ -19,6 +19,7 @@ struct KernelEntry {
   int dim, ko, ffn, head_dim, rgqa, hz;
   const void* fn;          // the kernel of a single GPU; none where the attention output is not as wide as the model
   int nps;                 // K/V positions per ring stage (the box of the cache tensors)
+  int copy, ring;          // bytes of a bulk copy of the matrices that read the model width, and of the whole ring
 };
 
 template <int KD, int KO, int KF, int HD, int R, bool HZ>
@@ -26,9 +27,13 @@ const void* single_gpu_kernel() {
   if constexpr (KO == KD) return (const void*)decode_mega2<KD, KO, KF, HD, R, HZ, false>;
   else return nullptr;
 }
-#define FB_DECODE_ENTRY(KD, KO, KF, HD, R)                                                                                      \
-  {KD, KO, KF, HD, R, 0, single_gpu_kernel<KD, KO, KF, HD, R, false>(), AttnCfg<HD, DecodePlan<KD, KO, KF>::STAGE>::NPS},        \
-  {KD, KO, KF, HD, R, 1, single_gpu_kernel<KD, KO, KF, HD, R, true>(), AttnCfg<HD, DecodePlan<KD, KO, KF>::STAGE>::NPS}
+template <int KD, int KO, int KF, int HD, int R, bool HZ>
+constexpr KernelEntry kernel_entry() {
+  constexpr int stage = DecodePlan<KD, KO, KF>::STAGE;
+  using C = TCfg<KD, stage>;
+  return {KD, KO, KF, HD, R, HZ, single_gpu_kernel<KD, KO, KF, HD, R, HZ>(), AttnCfg<HD, stage>::NPS, C::CPS * C::chunk(HZ), kStages * stage};
+}
+#define FB_DECODE_ENTRY(KD, KO, KF, HD, R) kernel_entry<KD, KO, KF, HD, R, false>(), kernel_entry<KD, KO, KF, HD, R, true>()
 
 const KernelEntry kDecodeKernels[] = {
 #include "fb_decode_shapes.h"
@@ -59,24 +64,24 @@ int chunks_for(const fb_ctx* c, int T) {
   return n < c->maxchunks ? n : c->maxchunks;
 }
 
-// Bulk copies a CTA keeps in flight while the layers run. A layer that brings each SM less than two rings of weights and K/V spends far
-// longer on its hand-overs than on the copies, and the tagged words then wait behind less bulk traffic; more bytes, or copies of less than 20 KB, need
-// the full rate. Microseconds a token at 1 / 2 / 3 / 4 copies (cached positions, rings a layer):
+// Bulk copies a CTA keeps in flight while the layers run. A layer that brings each SM at most 1.8 rings of weights and K/V spends far
+// longer on its hand-overs than on the copies, and the tagged words then wait behind less bulk traffic; more bytes, or copies of less than 20 KB (two of them
+// are then too little to stream with), need the full rate. Measured are copies of 21.1 KB (width 2560) and 16.9 KB (2048; 4096 in layers of more than
+// 1.8 rings); the line lies between the two, and widths of 512 and 640 make no difference. Microseconds a token at 1 / 2 / 3 / 4 copies (cached positions, rings a layer):
 //   3B-class   20, 1.6: 739 / 730 / 734 / 733   200, 1.6: 804 / 794 / 799 / 798   2000, 1.8: 830 / 819 / 820 / 819   4000, 2.0: 900 / 883 / 877 / 875
 //              8000, 2.3: 960 / 953 / 949 / 946   32700, 4.7: 1589 / 1473 / 1438 / 1431
 //   40 heads   600, 1.7: 794 / 788 / 794 / 796   1500, 1.75: 810 / 802 / 809 / 809   3900, 1.9: 876 / 864 / 859 / 860
 //   1B-class (copies of 17 KB)   22, 1.2: 289 / 284 / 281 / 280   3900, 1.6: 348 / 343 / 341 / 340        8B-class, 200: 1409 / 1326 / 1292 / 1287
 // The LM head has no hand-over to disturb: always 4.
-constexpr int64_t kRingBytes = 184320;      // a ring of eight 22.5 KB stages
 int fly_for(const fb_ctx* c, int T) {
   if (c->max_fly) return c->max_fly;
   const fb_model_desc& d = c->d;
+  const KernelEntry& e = kDecodeKernels[c->kernel_id];
   const int HD = d.head_dim, hz = d.has_zeros ? 1 : 0;
   const int64_t bytes = (int64_t)(d.n_head + 2 * d.n_kv_head) * HD * rec_bytes_of(d.dim, hz) + (int64_t)d.dim * rec_bytes_of(c->ko, hz) +
                         (int64_t)2 * d.ffn * rec_bytes_of(d.dim, hz) + (int64_t)d.dim * rec_bytes_of(d.ffn, hz) +
                         (int64_t)T * d.n_kv_head * HD * 4;
-  const int chunk = chunk_bytes(tile_rt(d.dim), chunk_k(d.dim), hz), copy = kRingBytes / kStages / chunk * chunk;
-  return bytes * 10 <= (int64_t)18 * kRingBytes * c->sm_count && copy >= 20000 ? 2 : 4;
+  return bytes * 10 <= (int64_t)18 * e.ring * c->sm_count && e.copy >= 20000 ? 2 : 4;
 }
 
 // every K the stand-alone entry points (re-layout, dequantise, GEMV) are built for
