@@ -28,7 +28,7 @@ const void* single_gpu_kernel() {
   else return nullptr;
 }
 template <int KD, int KO, int KF, int HD, int R, bool HZ>
-constexpr KernelEntry kernel_entry() {
+KernelEntry kernel_entry() {
   constexpr int stage = DecodePlan<KD, KO, KF>::STAGE;
   using C = TCfg<KD, stage>;
   return {KD, KO, KF, HD, R, HZ, single_gpu_kernel<KD, KO, KF, HD, R, HZ>(), AttnCfg<HD, stage>::NPS, C::CPS * C::chunk(HZ), kStages * stage};
@@ -339,7 +339,7 @@ int fb_repack(const void* d_q, const void* d_s, const void* d_z, int32_t rows, i
 int fb_dequant(const void* d_in, int32_t rows, int32_t k, int32_t has_zeros, int32_t order, int32_t order_arg,
                int32_t order_rows, float* d_out, void* stream) {
   if (!d_in || !d_out || rows <= 0 || k <= 0 || k % 128 || order < 0 || order > 2) return FB_ERR_ARG;
-  const int full = k % 128 ? 0 : rows / tile_rt(k) * tile_rt(k);
+  const int full = rows / tile_rt(k) * tile_rt(k);
   cudaStream_t st = (cudaStream_t)stream;
   switch (k) {
 #define X(K_)                                                                                                         \

@@ -52,10 +52,10 @@ def test_streaming_layout_dequant_bit_exact(asym, order):
     assert np.array_equal(out.cpu().numpy().view(np.uint32), ref.view(np.uint32))
 
 
-@pytest.mark.parametrize("k", [512, 640, 1280, 14336])          # tile heights 4, 16, 8, 2
+@pytest.mark.parametrize("k", [512, 640, 1280, 14336])          # tiles of 8, 16, 8 and 8 rows, the last in seven chunks
 @pytest.mark.parametrize("asym", [False, True])
 def test_streaming_layout_every_tile_height(k, asym):
-    """Rows that do not fill the last tile: the padding rows must not leak into the rows that exist."""
+    """Whole tiles, and the rows behind them, which a matrix on its own keeps plainly."""
     lib = _lib.load()
     rows = 37
     q, s, z = _mat(rows, k, 11, asym)
@@ -93,8 +93,8 @@ def test_gemv_vs_oracle(k, asym):
 
 @pytest.mark.parametrize("e", [-100, 60, 100])
 def test_gemv_power_of_two_activations_are_exact(e):
-    """The kernel multiplies fp16 copies of the activations; a power of two per group of 128 columns keeps that exact
-    over the whole bf16 range: scaling x by 2^e (one group by a different power) scales y by exactly 2^e."""
+    """The kernel multiplies integers; a power of two per group of 128 columns keeps the activations exact over the whole bf16
+    range: scaling x by 2^e (one group by a different power) scales y by exactly 2^e."""
     lib = _lib.load()
     rows, k = 300, 2560
     q, s, z = _mat(rows, k, 21, True)

@@ -39,9 +39,9 @@ def _matrix(rows, k, asym, seed):
 @pytest.mark.parametrize("tiles", [1, 2, 3, 4, 7, 8, 15])
 @pytest.mark.parametrize("k,asym", [(2048, False), (2560, True), (8192, False), (14336, True), (1408, False)])
 def test_every_number_of_tiles_a_cta(k, asym, tiles):
-    """1 .. 15 tiles of a CTA (8 rows; 16 where k has an odd number of groups), the last ragged: tiles in 14, 7, 4, 3, 2 and no slices, tiles of 2 and 7
-    chunks, more chunks than warps. fp32 sums of k exact products in any order differ from the oracle's by less than 2e-5 of the largest
-    result (64 roundings of 2^-24 each and the oracle's own)."""
+    """1 .. 15 tiles of a CTA (8 rows; 16 where k has an odd number of groups): tiles in 14, 7, 4, 3, 2 and no slices, tiles of 2 and 7 chunks, more chunks
+    than warps. The rows behind the last whole tile are plain ones here (tiles with padding: the vocabulary test of the decode step). fp32 sums of k
+    exact products in any order differ from the oracle's by less than 2e-5 of the largest result (64 roundings of 2^-24 each and the oracle's own)."""
     rt = 8 if (k // 128) % 2 == 0 else 16
     rows = query(torch.cuda.current_device())["sm_count"] * rt * tiles - 3
     q, s, z = _matrix(rows, k, asym, k + tiles)

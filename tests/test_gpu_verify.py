@@ -237,7 +237,7 @@ def test_tiny_tree_verify_long_cache(pos, M):
 
 
 def test_llama8b_class_shape_verify_two_layers():
-    """Heads of 128 and the 14336-wide FFN (tiles of 2 rows) through the verify path: 16-node tree, 2 layers."""
+    """Heads of 128 and the 14336-wide FFN through the verify path: 16-node tree, 2 layers."""
     from flint_b200.tree import static_tree
     cfg = ModelArgs.from_name("llama-8b-class")
     cfg.n_layer = 2
