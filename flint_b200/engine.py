@@ -20,13 +20,14 @@ def _ptr(t: Optional[torch.Tensor]):
     return None if t is None else t.data_ptr()          # the prototypes say void*: ctypes takes the integer
 
 
-# private, but what torch's own code generators call; the public way where a later torch lacks it
+# The current stream of the GPU with this index as torch.cuda.current_stream(index).cuda_stream gives it, without the Stream object (2.2 us a call). Private, but what
+# torch's own code generators call; the public way where a later torch lacks it.
 _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None) or (lambda index: torch.cuda.current_stream(index).cuda_stream)
 
 
 def _stream_ptr(device) -> int:
-    """The current stream of a CUDA device, as torch.cuda.current_stream(device).cuda_stream gives it (ValueError for any other device: what follows is a
-    launch on that device's pointers), without the Stream object (2.2 us a call)."""
+    """... of a caller's device: ValueError for any but a GPU, as what follows is a launch on that device's pointers. (An engine's device was looked at when
+    it was made.)"""
     if device.type != "cuda":
         raise ValueError(f"Expected a cuda device, but got: {device}")
     index = device.index
@@ -81,7 +82,7 @@ class DecodeEngine:
                 if t.device != self.device or not t.is_contiguous():
                     raise ValueError(f"{name}: must be a contiguous tensor on {self.device}")
                 setattr(w, name, t.data_ptr())
-        _lib.check(self.lib.fb_bind_weights(self._ctx, ctypes.byref(w), _stream_ptr(self.device)), "fb_bind_weights")
+        _lib.check(self.lib.fb_bind_weights(self._ctx, ctypes.byref(w), _raw_stream(self.dev_index)), "fb_bind_weights")
         torch.cuda.synchronize(self.device)
         shape = (cfg.n_layer, self.max_seq, self.n_kv_local, cfg.head_dim)
         self.kc = kc if kc is not None else torch.zeros(shape, dtype=torch.bfloat16, device=self.device)
@@ -144,20 +145,20 @@ class DecodeEngine:
         lg = logits if logits is not None else (self._logits if want_logits else None)
         nx = next_token if next_token is not None else self._next
         _lib.check(self.lib.fb_decode(self._ctx, int(token), None, None, int(pos), _ptr(lg), _ptr(nx),
-                                      _stream_ptr(self.device)), "fb_decode")
+                                      _raw_stream(self.dev_index)), "fb_decode")
         return lg
 
     def decode_chained(self, token_dev: torch.Tensor, pos: int, next_token: torch.Tensor,
                        logits: Optional[torch.Tensor] = None):
         """One step whose input token is read from device memory (the previous step's argmax): no host sync."""
         _lib.check(self.lib.fb_decode(self._ctx, 0, _ptr(token_dev), None, int(pos), _ptr(logits), _ptr(next_token),
-                                      _stream_ptr(self.device)), "fb_decode")
+                                      _raw_stream(self.dev_index)), "fb_decode")
 
     def decode_h(self, h: torch.Tensor, pos: int, logits: Optional[torch.Tensor] = None) -> torch.Tensor:
         """One step from an already multiplied embedding h bf16 [dim] (clobbered, as the reference does)."""
         lg = logits if logits is not None else torch.empty(self.cfg.vocab_size, dtype=torch.float32, device=self.device)
         _lib.check(self.lib.fb_decode(self._ctx, 0, None, _ptr(h), int(pos), _ptr(lg), _ptr(self._next),
-                                      _stream_ptr(self.device)), "fb_decode")
+                                      _raw_stream(self.dev_index)), "fb_decode")
         return lg
 
     @property
@@ -185,7 +186,7 @@ class DecodeEngine:
         logits = torch.empty(M, self.cfg.vocab_size, dtype=torch.float32, device=self.device) if want_logits else None
         feat = torch.empty(M, self.cfg.dim, dtype=torch.bfloat16, device=self.device)
         _lib.check(self.lib.fb_verify(self._ctx, _ptr(tok), None, _ptr(depth), _ptr(amask), M, int(pos), _ptr(logits),
-                                      _ptr(feat), _stream_ptr(self.device)), "fb_verify")
+                                      _ptr(feat), _raw_stream(self.dev_index)), "fb_verify")
         self._keepalive = (tok, depth, amask)
         return logits, feat
 
@@ -196,7 +197,7 @@ class DecodeEngine:
         n = tok.numel()
         logits = torch.empty(n, self.cfg.vocab_size, dtype=torch.float32, device=self.device) if want_logits else None
         feat = torch.empty(n, self.cfg.dim, dtype=torch.bfloat16, device=self.device)
-        _lib.check(self.lib.fb_prefill(self._ctx, _ptr(tok), n, int(pos), _ptr(logits), _ptr(feat), _stream_ptr(self.device)),
+        _lib.check(self.lib.fb_prefill(self._ctx, _ptr(tok), n, int(pos), _ptr(logits), _ptr(feat), _raw_stream(self.dev_index)),
                    "fb_prefill")
         self._keepalive = (tok,)
         return logits, feat
@@ -209,7 +210,7 @@ class DecodeEngine:
         feat = torch.empty(M, self.cfg.dim, dtype=torch.bfloat16, device=self.device)
         hc = h.contiguous()
         _lib.check(self.lib.fb_verify(self._ctx, None, _ptr(hc), _ptr(depth), _ptr(amask), M, int(pos), _ptr(logits),
-                                      _ptr(feat), _stream_ptr(self.device)), "fb_verify")
+                                      _ptr(feat), _raw_stream(self.dev_index)), "fb_verify")
         self._keepalive = (hc, depth, amask)
         return logits, feat
 
@@ -225,14 +226,14 @@ class DecodeEngine:
         if out is None:
             out = torch.empty(rows, dtype=torch.int32, device=lg.device)
         _lib.check(self.lib.fb_sample(_ptr(lg), vocab, rows, lg.stride(0) if rows > 1 else 0, float(temperature),
-                                      int(top_k or 0), int(seed), int(counter), _ptr(out), _stream_ptr(self.device)), "fb_sample")
+                                      int(top_k or 0), int(seed), int(counter), _ptr(out), _raw_stream(self.dev_index)), "fb_sample")
         return out
 
     def accept_chain(self, target: torch.Tensor, draft: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch.Tensor:
         """Device int32 [2]: accepted count and the target's next token (reference: spec_mega.py:106-113)."""
         out = out if out is not None else torch.empty(2, dtype=torch.int32, device=self.device)
         _lib.check(self.lib.fb_accept_chain(_ptr(target), _ptr(draft), int(draft.numel()), _ptr(out),
-                                            _stream_ptr(self.device)), "fb_accept_chain")
+                                            _raw_stream(self.dev_index)), "fb_accept_chain")
         return out
 
     def accept_tree(self, cand: torch.Tensor, parent: torch.Tensor, target: torch.Tensor,
@@ -241,20 +242,20 @@ class DecodeEngine:
         (reference: spec_tree.py:108-118)."""
         M = int(cand.numel())
         out = out if out is not None else torch.zeros(2 + M, dtype=torch.int32, device=self.device)
-        _lib.check(self.lib.fb_accept_tree(_ptr(cand), _ptr(parent), _ptr(target), M, _ptr(out), _stream_ptr(self.device)),
+        _lib.check(self.lib.fb_accept_tree(_ptr(cand), _ptr(parent), _ptr(target), M, _ptr(out), _raw_stream(self.dev_index)),
                    "fb_accept_tree")
         return out
 
     def kv_compact(self, accept: torch.Tensor, pos: int):
         """Moves the accepted path's cache rows to slots pos+1.. on the device, from accept_tree's output."""
-        _lib.check(self.lib.fb_kv_compact(self._ctx, _ptr(accept), int(pos), _stream_ptr(self.device)), "fb_kv_compact")
+        _lib.check(self.lib.fb_kv_compact(self._ctx, _ptr(accept), int(pos), _raw_stream(self.dev_index)), "fb_kv_compact")
 
     def kv_move(self, src, dst):
         """cache[:, dst[i]] = cache[:, src[i]] in order, K and V, every layer (reference: spec_tree.py:126-128)."""
         n = len(src)
         a = (ctypes.c_int32 * n)(*[int(x) for x in src])
         b = (ctypes.c_int32 * n)(*[int(x) for x in dst])
-        _lib.check(self.lib.fb_kv_move(self._ctx, a, b, n, _stream_ptr(self.device)), "fb_kv_move")
+        _lib.check(self.lib.fb_kv_move(self._ctx, a, b, n, _raw_stream(self.dev_index)), "fb_kv_move")
 
 
 # --------------------------------------------------------------------------------------------------
