@@ -228,8 +228,9 @@ __device__ __forceinline__ bool mbar_wait_far(uint64_t* b, uint32_t parity, cons
 // against three and a half, half the shared-memory reads of activations, and a flush per group of eight rows instead of four. (e4m3 operands need
 // the same operations, but sm_100a runs mma.sync on them at less than half of the integer rate: 7.2 against 3.0 cycles an instruction and SM, operands
 // from shared memory.) Gate/up of the 3B / 1B / 8B-class shapes, 16384 x 2560, 16384 x 2048, 28672 x 4096, in the decode kernel: 4.4 / 3.9 / 11.8 us before,
-// 2.5 / 2.2 / 7.3 now; the stand-alone product over 400000 x 2560 5.3 -> 5.8 TB/s. Against a 64-bit sum the logits of two layers are closer than
-// before (mean distance in units of the test's tolerance: 0.61 -> 0.35 at 3B, 0.50 -> 0.15 at 1B, 0.66 -> 0.51 at 8B): the products round only in the flush.
+// 2.5 / 2.2 / 7.3 now; the stand-alone product over 400000 x 2560 5.3 -> 5.8 TB/s. The products are off from 64-bit ones by 3.4e-7
+// (normal activations) to 1.5e-5 (outliers, SwiGLU outputs) before and by 5e-8 to 9.4e-8 now, whatever the activations: they round only in the flush. Elements below
+// 2^-21 of their group's largest, which the fp16 form held exactly, were lost there to the fp32 sums of nibble times the largest.
 __host__ __device__ constexpr int chunk_bytes(int rt, int kc, int has_zeros) { return rt * (kc / 2 + (kc / 128) * 2 * (has_zeros ? 2 : 1)); }
 constexpr int kChunkFit = 20992;                   // the smallest ring stage (SmemPlan of K = 14336)
 // Columns of a chunk: all of K where that fits a stage; else 4096 or 2048 where they divide K (8192 in 2, 14336 in 7: with 28 rows a CTA two chunks a warp), else

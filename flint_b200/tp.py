@@ -3,7 +3,7 @@
 Megatron-style sharding of every int4 matrix: QKV by heads (rows), O by this rank's heads (columns = K), gate/up by
 FFN rows, down by FFN columns (K), LM head by vocabulary rows; norms and the embedding table are replicated. Where a
 rank's attention width is not a multiple of the int4 group (the 3B-class model over 8 ranks: 320 columns), its O slice
-is widened to the enclosing group boundaries and the kernel feeds zeros for the neighbour's columns (`o_window`). The two
+is widened to the enclosing group boundaries and the kernel takes zeros for the neighbour's columns (`o_window`). The two
 K-sharded projections leave partial sums that the kernel exchanges itself (peer stores into every rank's inbox,
 tagged words, summed in rank order so every rank holds bit-identical residuals); this module only slices the packed
 tensors, creates one engine per process and passes the IPC handles of the inboxes around once, through
@@ -27,7 +27,7 @@ def o_window(cfg: ModelArgs, rank: int, size: int):
     """Columns of the O projection rank `rank` reads: its heads' columns widened to whole int4 groups.
 
     Returns (lo, hi, off): the rank holds columns [lo, hi) of every O row and its own attention output starts `off`
-    columns into that window; the kernel feeds zeros for the columns of the window that belong to a neighbour, so no
+    columns into that window; the kernel takes zeros for the columns of the window that belong to a neighbour, so no
     weight is re-quantised and every rank's dequantised values stay bit-exact. For shapes whose per-rank width is a
     multiple of 128 the window is exactly the rank's columns (off = 0)."""
     w = (cfg.n_head // size) * cfg.head_dim
