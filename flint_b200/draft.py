@@ -110,6 +110,8 @@ class DraftHead:
         pos = (torch.arange(T, device=dev) if positions is None else positions).to(device=dev, dtype=torch.int32).contiguous()
         slots = None if input_pos is None else input_pos.to(device=dev, dtype=torch.int32).contiguous()
         e2 = None if emb is None else emb.reshape(-1, self.dim).to(torch.bfloat16).contiguous()
+        if e2 is not None and not (e2.is_cuda or e2.is_pinned()):      # the kernels read it where it lies
+            raise ValueError(f"emb must be on the GPU, not on {e2.device}")
         tk = None if tokens is None else tokens.to(device=dev, dtype=torch.int32).contiguous()
         out = torch.empty(T, self.fdim, dtype=torch.bfloat16, device=dev)
         st = _stream_ptr(dev)

@@ -4,7 +4,7 @@ import ctypes
 import pytest
 import torch
 
-from flint_b200 import engine
+from flint_b200 import draft, engine
 from flint_b200.draft import DraftHead
 
 
@@ -31,6 +31,12 @@ def head():
 def test_draft_forward_refuses_features_on_the_cpu(head):
     with pytest.raises(ValueError, match="cuda device"):
         head(torch.zeros(2, 512, dtype=torch.bfloat16), tokens=torch.zeros(2, dtype=torch.int32))
+
+
+def test_draft_forward_refuses_embeddings_on_the_cpu(head, monkeypatch):
+    monkeypatch.setattr(draft, "_stream_ptr", lambda device: 0)          # as if the features were where they should be
+    with pytest.raises(ValueError, match="emb"):
+        head(torch.zeros(2, 512, dtype=torch.bfloat16), torch.zeros(2, 512, dtype=torch.bfloat16))
 
 
 def test_draft_head_refuses_rows_on_the_cpu(head):
